@@ -227,7 +227,6 @@ struct ConvTileParams {
     unsigned long long* probe_out;
     int* status;
     int probe;
-    long long* dbg;      // optional per-role cycle counters of CTA 0 (profiling aid), else null
     // fused epilogue (all optional): y = relu?(conv + bias[k] + residual) in fp32, quantised once
     // with the output's exponent; stored as int16 and / or as the byte planes the next
     // convolution reads
@@ -341,7 +340,7 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap mapI0,
     const unsigned tmem_base = *tmem_holder;
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             // the filter planes of this CTA's output channels: once, resident
             mbar_expect_tx(filt_bar, p.npanels * panel_bytes);
             for (int j = 0; j < p.npanels; ++j)
@@ -350,8 +349,6 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap mapI0,
             const int n_mma = p.n_mma;
             unsigned empty_parity = 1;         // the first pass over the ring finds every stage free
             bool ok = true;
-            const long long t_start = clock64();
-            long long t_wait = 0;
             for (int tile = blockIdx.x; tile < p.num_tiles && ok; tile += gridDim.x, ++ti) {
                 unsigned long long* fb = full_bar + (ti % n_mma) * kConvMaxStages;   // its consumer's
                 const int pq = tile / p.nblk, nb = tile - pq * p.nblk;
@@ -359,11 +356,9 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap mapI0,
                 const int n0 = nb * 128;
                 const int h0 = pp * p.str_h - p.pad_h, w0 = q * p.str_w - p.pad_w;
                 for (int cc = 0; cc < p.cchunks; ++cc) {
-                    const long long tw = clock64();
                     if (!mbar_wait_relaxed(&empty_bar[s], empty_parity)) {
                         atomicExch(fail_flag, 1); ok = false; break;
                     }
-                    t_wait += clock64() - tw;
                     unsigned char* sa = ring + (size_t)s * 2 * act_stage;
                     mbar_expect_tx(&fb[s], 2 * p.box_bytes);
                     tma_load_4d(sa, &mapI0, n0, w0, h0, cc * p.cu, &fb[s]);
@@ -371,21 +366,16 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap mapI0,
                     if (++s == p.nstages) { s = 0; empty_parity ^= 1u; }
                 }
             }
-            if (p.dbg && blockIdx.x == 0 && blockIdx.y == 0) {
-                p.dbg[0] = clock64() - t_start; p.dbg[1] = t_wait;
-            }
         }
     } else if (warp == 1 || warp >= 18) {
         // up to three MMA-issuing threads take the tiles in turn (when there are accumulator sets
-        // for them): an MMA instruction costs its issuing thread about a hundred cycles whatever
-        // its N and whatever the operand layout (a K-major, channel-innermost variant of this
-        // kernel was measured slower), and at 16..64 output channels that latency is what bounds
-        // a tile.  Three keep up with the operand fetch; a fourth would need a 21st warp, and at
-        // 672 threads the register file leaves the epilogue 80 registers (it spills and the
-        // kernel is slower than with two).
+        // for them), so that the waits of one tile's chunks overlap the next tile's instructions.
+        // The issuing thread is picked with elect.sync: under `lane == 0` the compiler cannot
+        // see that one thread runs and wraps every instruction in a loop over the active threads
+        // (22 launches of a batch-256 pass 364 -> 328 us, the update kernel 622 -> 471 us).
         const int mma_id = warp == 1 ? 0 : warp - 17;
         const int n_mma = p.n_mma;
-        if (lane == 0) {
+        if (elect_one()) {
             // bit 15: A is MN-major.  A_hi is signed, A_lo unsigned, both filter planes signed.
             const unsigned mn = 1u << 15;
             const unsigned id_s2 = make_idesc_n(2, 1, 1, 2 * bn) | mn, id_u2 = make_idesc_n(2, 0, 1, 2 * bn) | mn;
@@ -407,8 +397,6 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap mapI0,
             unsigned phase_bits = 0, stage_lo = ring_lo;       // bit s: parity of my next phase of stage s
             unsigned empty_bits = 0;                           // bit b: the same for set b's "drained" barrier
             unsigned long long* fb = full_bar + mma_id * kConvMaxStages;
-            const long long t_start = clock64();
-            long long t_wait_e = 0, t_wait_f = 0, t_mma = 0, t_commit = 0;
             for (int tile = blockIdx.x; tile < p.num_tiles && ok; tile += gridDim.x, ++ti) {
                 if (ti % n_mma != mma_id) {
                     // the other issuing thread's tile: step over its stages (their "filled"
@@ -421,26 +409,21 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap mapI0,
                 }
                 const int buf = ti % p.nbuf;
                 const unsigned acc_base = tmem_base + buf * acc_cols;
-                const long long tw = clock64();
                 if (ti >= p.nbuf) {
                     if (!mbar_wait(&tmem_empty[mma_id * 4 + buf], (empty_bits >> buf) & 1u)) {
                         atomicExch(fail_flag, 1); ok = false; break;
                     }
                     empty_bits ^= 1u << buf;
                 }
-                t_wait_e += clock64() - tw;
                 tc_fence_after();
                 int idx = 0;                                   // 32-byte column block of the filter planes
                 for (int cc = 0; cc < p.cchunks; ++cc) {
-                    const long long tw2 = clock64();
                     if (!mbar_wait(&fb[s], (phase_bits >> s) & 1u)) {
                         atomicExch(fail_flag, 1); ok = false; break;
                     }
                     phase_bits ^= 1u << s;
-                    t_wait_f += clock64() - tw2;
                     tc_fence_after();
                     unsigned a_lo = stage_lo;
-                    const long long tm0 = clock64();
                     for (int k = 0; k < ksteps; ++k, ++idx, a_lo += 256u) {
                         const unsigned boff = (unsigned)(idx >> 2) * panel_units + (unsigned)(idx & 3) * 2u;
                         const unsigned long long dB = desc_hi | (filt_lo + boff);
@@ -458,19 +441,11 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap mapI0,
                             tc_mma<MODE_FLEX16>(acc_base + 2 * bn, dA1, dBl, id_u1, 0u);
                         }
                     }
-                    const long long tm1 = clock64();
                     tc_commit(&empty_bar[s]);
                     stage_lo += stage_units;
                     if (++s == p.nstages) { s = 0; stage_lo = ring_lo; }
-                    t_mma += tm1 - tm0; t_commit += clock64() - tm1;
                 }
-                const long long tc0 = clock64();
                 tc_commit(&tmem_full[buf]);
-                t_commit += clock64() - tc0;
-            }
-            if (p.dbg && blockIdx.x == 0 && blockIdx.y == 0 && mma_id == 0) {
-                p.dbg[2] = clock64() - t_start; p.dbg[3] = t_wait_e; p.dbg[4] = t_wait_f;
-                p.dbg[8] = t_mma; p.dbg[9] = t_commit;
             }
         }
     } else {
@@ -500,8 +475,6 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap mapI0,
         const unsigned rmask = fast ? (1u << sh) - 1u : 0u, rhalf = fast ? 1u << (sh - 1) : 0u;
         int ti = 0;
         bool ok = true;
-        const long long t_start = clock64();
-        long long t_wait = 0, t_ld = 0, t_arr = 0, t_all = 0;
         for (int tile = blockIdx.x; tile < p.num_tiles; tile += gridDim.x, ++ti) {
             const int buf = ti % p.nbuf;
             if (buf != set) continue;
@@ -515,13 +488,10 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap mapI0,
                 for (int j = 0; j < 8; ++j)
                     rz[j] = cc0 + j < kt ? p.residual[base + (long long)j * p.ldc] : (short)0;
             }
-            const long long tw = clock64();
             if (ok && !mbar_wait_relaxed(&tmem_full[buf], (ti / p.nbuf) & 1)) { atomicExch(fail_flag, 1); ok = false; }
-            t_wait += clock64() - tw;
             tc_fence_after();
             const unsigned lane_addr = tmem_base + buf * acc_cols + ((unsigned)(quarter * 32) << 16);
             // 128 * (sum of this row's activations), from the extra column p.kt
-            const long long te0 = clock64();
             const int s_hi = (int)tmem_ld1(lane_addr + bn + p.kt);
             const int s_lo = (int)tmem_ld1(lane_addr + 2 * bn + p.kt);
             tmem_ld_wait();
@@ -623,7 +593,6 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap mapI0,
                 tmem_ld16(lane_addr + bn + c0, xx);
                 tmem_ld16(lane_addr + 2 * bn + c0, ll);
                 tmem_ld_wait();
-                t_ld += clock64() - te0;
                 if (!ok) continue;
                 short* out = (short*)p.O + (long long)(ncol0 + c0) * p.ldc + row;
                 long long v[16];
@@ -659,18 +628,11 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap mapI0,
                 }
             }
             // this warp has read its part of the accumulator set
-            const long long te1 = clock64();
             tc_fence_before();
             __syncwarp();
             // tell the thread that fills this set next (tile ti + nbuf of this CTA, if there is one)
             if (lane == 0 && ti + p.nbuf < n_my)
                 mbar_arrive(&tmem_empty[((ti + p.nbuf) % n_mma_e) * 4 + buf]);
-            t_arr += clock64() - te1;
-            t_all += clock64() - te0;
-        }
-        if (p.dbg && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 64) {
-            p.dbg[5] = clock64() - t_start; p.dbg[6] = t_wait; p.dbg[7] = ti;
-            p.dbg[10] = t_ld; p.dbg[11] = t_arr; p.dbg[12] = t_all;
         }
         if (p.probe) {
             // fused: the bit pattern of max |y| (fp32); plain: max |integer sum|
@@ -979,11 +941,6 @@ int implicit_tiles(const void* act_planes, const void* filt_planes, void* O, con
         p.write_i16 = epi->write_int16 ? 1 : 0;
         p.out_planes = (unsigned char*)epi->out_planes;
         p.out_plane_bytes = (long long)epi->plane_bytes;
-    }
-    {
-        // profiling aid: B2_CONV_DBG=<device address> makes CTA 0 write 8 cycle counters there
-        const char* e = getenv("B2_CONV_DBG");
-        p.dbg = e ? (long long*)strtoull(e, nullptr, 0) : nullptr;
     }
     static bool attr_set = false;
     if (!attr_set) {
@@ -1316,7 +1273,7 @@ conv_update_kernel(const __grid_constant__ CUtensorMap mapI0, const __grid_const
     const unsigned tmem_base = *tmem_holder;
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             int s = 0;
             unsigned empty_parity = 1;
             for (int i = 0; i < mine; ++i) {
@@ -1338,7 +1295,7 @@ conv_update_kernel(const __grid_constant__ CUtensorMap mapI0, const __grid_const
         }
     } else if (warp == 1 || warp == 2) {
         const int id = warp - 1;
-        if (lane == 0) {
+        if (elect_one()) {
             const unsigned id_s = make_idesc_n(2, 1, 1, 2 * bn), id_u = make_idesc_n(2, 0, 1, 2 * bn);
             const unsigned acc = tmem_base + id * 4 * bn;
             unsigned long long* fb = full_bar + id * kUpdMaxStages;

@@ -100,6 +100,12 @@ __device__ __forceinline__ bool mbar_try_wait(unsigned long long* bar, unsigned 
         : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
     return ok != 0;
 }
+// one thread of the (converged) warp
+__device__ __forceinline__ bool elect_one() {
+    unsigned ok;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok));
+    return ok != 0;
+}
 // bounded wait: gives up after `limit` polls (each poll suspends up to a hardware time limit)
 __device__ __forceinline__ bool mbar_wait_limit(unsigned long long* bar, unsigned parity, int limit) {
     for (int i = 0; i < limit; ++i)
@@ -285,7 +291,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constant__ C
     const unsigned tmem_base = *tmem_holder;
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             for (int kb = 0; kb < nkb; ++kb) {
                 const int s = kb % kStages;
                 if (kb >= kStages && !mbar_wait(&empty_bar[s], ((kb / kStages) - 1) & 1)) {
@@ -302,7 +308,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constant__ C
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (elect_one()) {
             // flex16: planes are (hi = signed, lo = unsigned) bytes; accumulators HH | X | LL
             const unsigned id_ss = make_idesc(2, 1, 1, BN), id_su = make_idesc(2, 1, 0, BN),
                            id_us = make_idesc(2, 0, 1, BN), id_uu = make_idesc(2, 0, 0, BN);
