@@ -231,6 +231,7 @@ struct ConvTileParams {
     // with the output's exponent; stored as int16 and / or as the byte planes the next
     // convolution reads
     int fused;                    // 0: plain integer rescale of the convolution
+    int short_sum;                // |256*HH + X| < 2^31 for every operand (see implicit_tiles)
     const short* bias; int slot_bias;
     const short* residual; int slot_res;      // same K,P,Q,N layout as the output
     int relu;
@@ -345,18 +346,25 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap mapI0,
             mbar_expect_tx(filt_bar, p.npanels * panel_bytes);
             for (int j = 0; j < p.npanels; ++j)
                 tma_load_2d(filt + j * panel_bytes, &mapB, j * kKBytes, blockIdx.y * 2 * bn, filt_bar);
-            int s = 0, ti = 0;
+            // Every role of this kernel is a single chain of instructions per tile, so nothing in
+            // the loops divides: the tile's image block, column and row advance by the fixed step
+            // of gridDim.x tiles with carries, and ring positions are counters (the divisions
+            // alone cost this thread more than the copies of a small tile take).
+            int s = 0, mma = 0;
             const int n_mma = p.n_mma;
             unsigned empty_parity = 1;         // the first pass over the ring finds every stage free
             bool ok = true;
-            for (int tile = blockIdx.x; tile < p.num_tiles && ok; tile += gridDim.x, ++ti) {
-                unsigned long long* fb = full_bar + (ti % n_mma) * kConvMaxStages;   // its consumer's
-                const int pq = tile / p.nblk, nb = tile - pq * p.nblk;
-                const int pp = pq / p.Q, q = pq - pp * p.Q;
+            const int Q = p.Q, nblk = p.nblk;
+            int nb = (int)blockIdx.x % nblk, pq = (int)blockIdx.x / nblk, q = pq % Q, pp = pq / Q;
+            const int d_nb = (int)gridDim.x % nblk, d_pq = (int)gridDim.x / nblk, d_q = d_pq % Q,
+                      d_p = d_pq / Q;
+            for (int tile = blockIdx.x; tile < p.num_tiles && ok; tile += gridDim.x) {
+                unsigned long long* fb = full_bar + mma * kConvMaxStages;            // its consumer's
+                if (++mma == n_mma) mma = 0;
                 const int n0 = nb * 128;
                 const int h0 = pp * p.str_h - p.pad_h, w0 = q * p.str_w - p.pad_w;
                 for (int cc = 0; cc < p.cchunks; ++cc) {
-                    if (!mbar_wait_relaxed(&empty_bar[s], empty_parity)) {
+                    if (!mbar_wait(&empty_bar[s], empty_parity)) {
                         atomicExch(fail_flag, 1); ok = false; break;
                     }
                     unsigned char* sa = ring + (size_t)s * 2 * act_stage;
@@ -365,6 +373,9 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap mapI0,
                     tma_load_4d(sa + act_stage, &mapI1, n0, w0, h0, cc * p.cu, &fb[s]);
                     if (++s == p.nstages) { s = 0; empty_parity ^= 1u; }
                 }
+                nb += d_nb; q += d_q; pp += d_p;
+                if (nb >= nblk) { nb -= nblk; ++q; }
+                if (q >= Q) { q -= Q; ++pp; }
             }
         }
     } else if (warp == 1 || warp >= 18) {
@@ -380,7 +391,6 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap mapI0,
             const unsigned mn = 1u << 15;
             const unsigned id_s2 = make_idesc_n(2, 1, 1, 2 * bn) | mn, id_u2 = make_idesc_n(2, 0, 1, 2 * bn) | mn;
             const unsigned id_s1 = make_idesc_n(2, 1, 1, bn) | mn, id_u1 = make_idesc_n(2, 0, 1, bn) | mn;
-            int ti = 0;
             bool ok = mma_id < n_mma && mbar_wait(filt_bar, 0);
             if (!ok && mma_id < n_mma) atomicExch(fail_flag, 1);
             const int ksteps = p.kc_pad >> 5;
@@ -397,8 +407,13 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap mapI0,
             unsigned phase_bits = 0, stage_lo = ring_lo;       // bit s: parity of my next phase of stage s
             unsigned empty_bits = 0;                           // bit b: the same for set b's "drained" barrier
             unsigned long long* fb = full_bar + mma_id * kConvMaxStages;
-            for (int tile = blockIdx.x; tile < p.num_tiles && ok; tile += gridDim.x, ++ti) {
-                if (ti % n_mma != mma_id) {
+            int turn = 0, buf = -1;
+            bool first_use = true;                             // the sets start out empty
+            for (int tile = blockIdx.x; tile < p.num_tiles && ok; tile += gridDim.x) {
+                if (++buf == p.nbuf) { buf = 0; first_use = false; }
+                const bool my_turn = turn == mma_id;
+                if (++turn == n_mma) turn = 0;
+                if (!my_turn) {
                     // the other issuing thread's tile: step over its stages (their "filled"
                     // barriers are the other thread's own)
                     for (int cc = 0; cc < p.cchunks; ++cc) {
@@ -407,9 +422,8 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap mapI0,
                     }
                     continue;
                 }
-                const int buf = ti % p.nbuf;
                 const unsigned acc_base = tmem_base + buf * acc_cols;
-                if (ti >= p.nbuf) {
+                if (!first_use) {
                     if (!mbar_wait(&tmem_empty[mma_id * 4 + buf], (empty_bits >> buf) & 1u)) {
                         atomicExch(fail_flag, 1); ok = false; break;
                     }
@@ -471,24 +485,32 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap mapI0,
         const float f_conv = p.table[p.slotA].scale * p.table[p.slotB].scale * q_out;
         const float s_res = p.residual ? p.table[p.slot_res].scale * q_out : 0.0f;
         float fmax_probe = 0.0f, fstat = 0.0f;
+        const unsigned ldc32 = (unsigned)p.ldc;                // (the host checks that K*ldc fits)
+        unsigned char* const out_lo = p.out_planes + p.out_plane_bytes;
         const bool fast = sh >= 1 && sh <= 31;
         const unsigned rmask = fast ? (1u << sh) - 1u : 0u, rhalf = fast ? 1u << (sh - 1) : 0u;
-        int ti = 0;
         bool ok = true;
-        for (int tile = blockIdx.x; tile < p.num_tiles; tile += gridDim.x, ++ti) {
-            const int buf = ti % p.nbuf;
-            if (buf != set) continue;
+        // this warp's tiles: every nbuf-th one of the CTA; `next` is the issuing thread of the
+        // tile that follows in the same accumulator set
+        const int buf = set, nbuf = p.nbuf, d_next = nbuf % n_mma_e;
+        int next = (set + nbuf) % n_mma_e;
+        unsigned full_parity = 0;
+        // (with three sets the warps of the fourth slot have none)
+        for (int ti = set < nbuf ? set : n_my; ti < n_my; ti += nbuf) {
+            const int tile = (int)blockIdx.x + ti * (int)gridDim.x;
             const long long row = (long long)tile * 128 + quarter * 32 + lane;   // (pq*N + n)
             // the residual of the first piece is fetched while the tile is still being multiplied
             short rz[8];
-            if (p.fused && p.residual) {
-                const int cc0 = part * 8;
-                const long long base = (long long)(ncol0 + cc0) * p.ldc + row;
+            const unsigned row32 = (unsigned)row;
+            auto load_res = [&](int cc0) {
+                const unsigned off = (unsigned)(ncol0 + cc0) * ldc32 + row32;
 #pragma unroll
                 for (int j = 0; j < 8; ++j)
-                    rz[j] = cc0 + j < kt ? p.residual[base + (long long)j * p.ldc] : (short)0;
-            }
-            if (ok && !mbar_wait_relaxed(&tmem_full[buf], (ti / p.nbuf) & 1)) { atomicExch(fail_flag, 1); ok = false; }
+                    rz[j] = cc0 + j < kt ? p.residual[off + (unsigned)j * ldc32] : (short)0;
+            };
+            if (p.fused && p.residual) load_res(part * 8);
+            if (ok && !mbar_wait(&tmem_full[buf], full_parity)) { atomicExch(fail_flag, 1); ok = false; }
+            full_parity ^= 1u;
             tc_fence_after();
             const unsigned lane_addr = tmem_base + buf * acc_cols + ((unsigned)(quarter * 32) << 16);
             // 128 * (sum of this row's activations), from the extra column p.kt
@@ -500,87 +522,97 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap mapI0,
             if (p.fused) {
                 // fp32 epilogue: the exact integer sum scaled to a real value, bias and residual
                 // added, ReLU, ONE quantisation with the output's exponent.  Eight columns at a
-                // time (the register budget of a 608-thread CTA), loads first, then arithmetic,
-                // then stores: eight independent chains.
-                {
-                    // the warps that share a lane quarter take the 8-column pieces in turn
-                    for (int cc0 = part * 8; cc0 < kt; cc0 += 8 * epi_w) {
-                        unsigned hh[8], xx[8], ll[8];
-                        tmem_ld8(lane_addr + cc0, hh);
-                        tmem_ld8(lane_addr + bn + cc0, xx);
-                        tmem_ld8(lane_addr + 2 * bn + cc0, ll);
-                        const long long base = (long long)(ncol0 + cc0) * p.ldc + row;
-                        const int live = kt - cc0;
-                        float y[8];
-                        if (p.residual) {
+                // time, loads first, then arithmetic, then stores: eight independent chains.  The
+                // warps that share a lane quarter take the 8-column pieces in turn.
+                // What bounds it is instruction issue (68 % of the slots in the form before this
+                // one: a flag test per stored value, 64-bit addresses), so every choice is made
+                // once per piece and addresses are a uniform base plus a 32-bit offset.
+                for (int cc0 = part * 8; cc0 < kt; cc0 += 8 * epi_w) {
+                    unsigned hh[8], xx[8], ll[8];
+                    tmem_ld8(lane_addr + cc0, hh);
+                    tmem_ld8(lane_addr + bn + cc0, xx);
+                    tmem_ld8(lane_addr + 2 * bn + cc0, ll);
+                    const int live = kt - cc0;
+                    float y[8];
+                    if (p.residual) {
 #pragma unroll
-                            for (int j = 0; j < 8; ++j) y[j] = (float)rz[j] * s_res;
-                            // and the next piece's, one piece ahead of its use
-                            const int nx = cc0 + 8 * epi_w;
-                            if (nx < kt) {
-                                const long long nbase = (long long)(ncol0 + nx) * p.ldc + row;
+                        for (int j = 0; j < 8; ++j) y[j] = fmaf((float)rz[j], s_res, bias_s[cc0 + j]);
+                        // and the next piece's, one piece ahead of its use
+                        const int nx = cc0 + 8 * epi_w;
+                        if (nx < kt) load_res(nx);
+                    } else {
 #pragma unroll
-                                for (int j = 0; j < 8; ++j)
-                                    rz[j] = nx + j < kt ? p.residual[nbase + (long long)j * p.ldc] : (short)0;
-                            }
-                        } else {
-#pragma unroll
-                            for (int j = 0; j < 8; ++j) y[j] = 0.0f;
-                        }
-                        tmem_ld_wait();
-                        if (!ok) continue;
+                        for (int j = 0; j < 8; ++j) y[j] = bias_s[cc0 + j];
+                    }
+                    tmem_ld_wait();
+                    if (!ok) continue;
+                    if (p.short_sum) {
+                        // 256*HH + X fits 32 bits: two conversions a value instead of three (they
+                        // run at a quarter of the rate of the rest)
 #pragma unroll
                         for (int j = 0; j < 8; ++j) {
-                            // three exact-or-correctly-rounded conversions instead of a 64-bit sum:
-                            // the fp32 result is quantised to 16 bits right after
+                            const float t = (float)((int)(hh[j] << 8) + (int)xx[j]);
+                            y[j] = fmaf(fmaf(t, 256.0f, (float)(int)ll[j] + fixf), f_conv, y[j]);
+                        }
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) {
+                            // correctly rounded conversions instead of a 64-bit sum: the fp32
+                            // result is quantised to 16 bits right after
                             const float acc = fmaf((float)(int)hh[j], 65536.0f,
                                                    fmaf((float)(int)xx[j], 256.0f, (float)(int)ll[j] + fixf));
-                            y[j] += fmaf(acc, f_conv, bias_s[cc0 + j]);
+                            y[j] = fmaf(acc, f_conv, y[j]);
                         }
-                        if (p.relu) {
+                    }
+                    if (p.relu) {
 #pragma unroll
-                            for (int j = 0; j < 8; ++j) y[j] = fmaxf(y[j], 0.0f);      // also NaN -> 0
-                        } else if (!p.probe) {
+                        for (int j = 0; j < 8; ++j) y[j] = fmaxf(y[j], 0.0f);      // also NaN -> 0
+                    } else if (!p.probe) {
 #pragma unroll
-                            for (int j = 0; j < 8; ++j) y[j] = (y[j] != y[j]) ? 0.0f : fmaxf(y[j], -32768.0f);
-                        }
-                        if (p.probe) {
+                        for (int j = 0; j < 8; ++j) y[j] = (y[j] != y[j]) ? 0.0f : fmaxf(y[j], -32768.0f);
+                    }
+                    if (p.probe) {
 #pragma unroll
-                            for (int j = 0; j < 8; ++j)
-                                if (j < live) fmax_probe = fmaxf(fmax_probe, fabsf(y[j]));
-                            continue;
-                        }
-                        // y is already in units of the output's step (see f_conv): clamp, round to
-                        // nearest even by the magic-number add; the low 16 bits of the sum are the
-                        // mantissa, so the bytes are stored straight from it
-                        int m[8];
+                        for (int j = 0; j < 8; ++j)
+                            if (j < live) fmax_probe = fmaxf(fmax_probe, fabsf(y[j]));
+                        continue;
+                    }
+                    // y is already in units of the output's step (see f_conv): clamp, round to
+                    // nearest even by the magic-number add; the low 16 bits of the sum are the
+                    // mantissa, so the bytes are stored straight from it
+                    int m[8];
 #pragma unroll
-                        for (int j = 0; j < 8; ++j) {
-                            y[j] = fminf(y[j], 32767.0f);
-                            m[j] = __float_as_int(y[j] + 12582912.0f);
-                        }
-                        if (live >= 8) {
+                    for (int j = 0; j < 8; ++j) {
+                        y[j] = fminf(y[j], 32767.0f);
+                        m[j] = __float_as_int(y[j] + 12582912.0f);
+                    }
+                    const unsigned off = (unsigned)(ncol0 + cc0) * ldc32 + row32;
+                    if (live >= 8) {
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) fstat = fmaxf(fstat, fabsf(y[j]));
+                        if (p.out_planes) {
 #pragma unroll
                             for (int j = 0; j < 8; ++j) {
+                                const unsigned at = off + (unsigned)j * ldc32;
+                                p.out_planes[at] = (unsigned char)(m[j] >> 8);
+                                out_lo[at] = (unsigned char)m[j];
+                            }
+                        }
+                        if (p.write_i16) {
+#pragma unroll
+                            for (int j = 0; j < 8; ++j)
+                                ((short*)p.O)[off + (unsigned)j * ldc32] = (short)m[j];
+                        }
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) {
+                            if (j < live) {
                                 fstat = fmaxf(fstat, fabsf(y[j]));
-                                const long long at = base + (long long)j * p.ldc;
+                                const unsigned at = off + (unsigned)j * ldc32;
                                 if (p.write_i16) ((short*)p.O)[at] = (short)m[j];
                                 if (p.out_planes) {
                                     p.out_planes[at] = (unsigned char)(m[j] >> 8);
-                                    p.out_planes[p.out_plane_bytes + at] = (unsigned char)m[j];
-                                }
-                            }
-                        } else {
-#pragma unroll
-                            for (int j = 0; j < 8; ++j) {
-                                if (j < live) {
-                                    fstat = fmaxf(fstat, fabsf(y[j]));
-                                    const long long at = base + (long long)j * p.ldc;
-                                    if (p.write_i16) ((short*)p.O)[at] = (short)m[j];
-                                    if (p.out_planes) {
-                                        p.out_planes[at] = (unsigned char)(m[j] >> 8);
-                                        p.out_planes[p.out_plane_bytes + at] = (unsigned char)m[j];
-                                    }
+                                    out_lo[at] = (unsigned char)m[j];
                                 }
                             }
                         }
@@ -631,8 +663,9 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap mapI0,
             tc_fence_before();
             __syncwarp();
             // tell the thread that fills this set next (tile ti + nbuf of this CTA, if there is one)
-            if (lane == 0 && ti + p.nbuf < n_my)
-                mbar_arrive(&tmem_empty[((ti + p.nbuf) % n_mma_e) * 4 + buf]);
+            if (lane == 0 && ti + nbuf < n_my) mbar_arrive(&tmem_empty[next * 4 + buf]);
+            next += d_next;
+            if (next >= n_mma_e) next -= n_mma_e;
         }
         if (p.probe) {
             // fused: the bit pattern of max |y| (fp32); plain: max |integer sum|
@@ -928,6 +961,8 @@ int implicit_tiles(const void* act_planes, const void* filt_planes, void* O, con
     p.O = O; p.table = table; p.slotA = slotI; p.slotB = slotF; p.slotC = slotO;
     p.stats = stats; p.probe_out = probe_out; p.status = status; p.probe = probe;
     p.fused = 0; p.bias = nullptr; p.residual = nullptr; p.slot_bias = p.slot_res = 0; p.relu = 0;
+    // per K row |HH| <= 2^14 and |X| <= 2 * 2^14 + 2^15, padding rows included
+    p.short_sum = (long long)s.cchunks * s.kc_pad * ((1 << 22) + (1 << 16)) < (1LL << 31);
     p.write_i16 = 1; p.out_planes = nullptr; p.out_plane_bytes = 0;
     if (epi) {
         B2_REQUIRE(!epi->bias || epi->slot_bias >= 0, "bias needs its scale slot");
@@ -935,6 +970,7 @@ int implicit_tiles(const void* act_planes, const void* filt_planes, void* O, con
         B2_REQUIRE(epi->write_int16 || epi->out_planes, "the fused epilogue stores nothing");
         B2_REQUIRE(!epi->out_planes || ((uintptr_t)epi->out_planes & 15) == 0, "planes alignment");
         p.fused = 1;
+        B2_REQUIRE((long long)g.K * p.ldc < (1LL << 32), "output tensor too large");
         p.bias = epi->bias; p.slot_bias = epi->slot_bias;
         p.residual = epi->residual; p.slot_res = epi->slot_residual;
         p.relu = epi->relu ? 1 : 0;
