@@ -210,10 +210,11 @@ struct ConvTileParams {
     int cu;                       // channels per chunk
     int cchunks;                  // chunks per tile = stages per tile
     int kc_pad;                   // K rows per chunk, padded to a multiple of 32
-    int box_bytes;                // bytes one activation box delivers (cu*R*S*128)
+    int box_bytes;                // bytes one activation box delivers (cu * window * 128)
+    int gh, gw, tq;               // output pixels a tile covers (gh x gw), tiles along a row
     int npanels;                  // 128-byte K panels of the resident filter planes
     int nstages;                  // ring depth
-    int bn;                       // columns per accumulator: kt output channels + the sum column
+    int bn;                       // columns per accumulator: gh*gw * (kt channels + a sum column)
     int kt;                       // output channels per CTA column (blockIdx.y)
     int nbuf;                     // accumulator sets in tensor memory: 1, 2, 3 (or 4)
     int n_mma;                    // MMA-issuing threads: 1..3, at most nbuf
@@ -230,12 +231,11 @@ struct ConvTileParams {
     // fused epilogue (all optional): y = relu?(conv + bias[k] + residual) in fp32, quantised once
     // with the output's exponent; stored as int16 and / or as the byte planes the next
     // convolution reads
-    int fused;                    // 0: plain integer rescale of the convolution
-    int short_sum;                // |256*HH + X| < 2^31 for every operand (see implicit_tiles)
     const short* bias; int slot_bias;
     const short* residual; int slot_res;      // same K,P,Q,N layout as the output
     int relu;
     int write_i16;
+    int vec;                      // tensors aligned for eight images at a time
     unsigned char* out_planes; long long out_plane_bytes;
 };
 
@@ -246,6 +246,39 @@ __device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* map, i
         "[%0], [%1, {%2, %3, %4, %5}], [%6];"
         ::"r"(smem_u32(dst)), "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(smem_u32(bar))
         : "memory");
+}
+// two fp32 values in one 64-bit register, and the packed arithmetic on them
+__device__ __forceinline__ unsigned long long pack2(float a, float b) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void unpack2(unsigned long long v, float& a, float& b) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b,
+                                                   unsigned long long c) {
+    unsigned long long r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
+    unsigned long long r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+// max(m, |a|, |b|)
+__device__ __forceinline__ float max3_abs(float m, float a, float b) {
+    float r;
+    asm("max.abs.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(m), "f"(a), "f"(b));
+    return r;
+}
+// eight consecutive int16, as one load where the alignment allows it
+__device__ __forceinline__ uint4 load8(const short* p, int vec) {
+    if (vec) return *reinterpret_cast<const uint4*>(p);
+    const unsigned short* q = reinterpret_cast<const unsigned short*>(p);
+    return make_uint4(q[0] | (unsigned)q[1] << 16, q[2] | (unsigned)q[3] << 16,
+                      q[4] | (unsigned)q[5] << 16, q[6] | (unsigned)q[7] << 16);
 }
 // one 32-bit column of this thread's TMEM lane
 __device__ __forceinline__ unsigned tmem_ld1(unsigned taddr) {
@@ -274,8 +307,15 @@ __device__ __forceinline__ unsigned make_idesc_n(unsigned dfmt, unsigned afmt, u
 constexpr int kConvMaxStages = 8;
 constexpr int kConvThreads = 640;           // producer, MMA, sixteen epilogue warps, two more MMA warps
 constexpr int kConvSmemMax = 232448;        // 227 KB: the most one CTA can have
-constexpr int kConvSmemFixed = 1024 /*alignment*/ + 1024 /*barriers, bias*/;
+constexpr int kConvSmemFixed = 1024 /*alignment*/ + 1024 /*barriers, bias*/ + 16 * 1024 /*epilogue staging*/;
 
+// OFF: 32-bit element offsets into the output where they reach, 64-bit ones for larger tensors.
+// EPI: 0 plain integer rescale, 1 fused tail, 2 fused tail with a residual.  SHORT: 256*HH + X fits 32
+// bits.  EVEN: eight images and eight channels at a time throughout -- aligned tensors, channel
+// counts that are multiples of eight -- and not a measuring launch.  (Template parameters because a tested-and-skipped block of the epilogue is not free: the
+// compiler predicates it, and its instructions are issued all the same -- 60 of 330 per piece.)
+enum { EPI_INT = 0, EPI_FUSED = 1, EPI_RESIDUAL = 2 };
+template <typename OFF, int EPI, bool SHORT, bool EVEN>
 __global__ void __launch_bounds__(kConvThreads, 1)
 conv_implicit_kernel(const __grid_constant__ CUtensorMap mapI0,
                      const __grid_constant__ CUtensorMap mapI1,
@@ -301,9 +341,11 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap mapI0,
     unsigned long long* filt_bar = tmem_empty + 16;
     unsigned* tmem_holder = (unsigned*)(filt_bar + 1);
     int* fail_flag = (int*)(tmem_holder + 1);
-    float* bias_s = (float*)(fail_flag + 2);                      // [bn] bias of this CTA's channels, real values
+    // [bn] bias of this CTA's channels in units of the output's step; then the epilogue's staging
+    float* bias_s = (float*)((unsigned char*)full_bar + 512);
+    unsigned char* epi_smem = (unsigned char*)full_bar + 1024;    // 1 KB per epilogue warp
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
     const int epi_w = p.nbuf == 3 ? 1 : 4 / p.nbuf;   // epilogue warps per lane quarter and accumulator set
 
     // Programmatic dependent launch: the next kernel of the stream, if it was launched the same
@@ -329,8 +371,8 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap mapI0,
     // completed work of all earlier kernels of the stream
     asm volatile("griddepcontrol.wait;" ::: "memory");
     if (threadIdx.x >= 64 && threadIdx.x < 64 + bn) {
-        const int col = blockIdx.y * p.kt + (threadIdx.x - 64);
-        bias_s[threadIdx.x - 64] = (p.fused && p.bias && (threadIdx.x - 64) < p.kt && col < p.K)
+        const int col = blockIdx.y * p.kt + (int)(threadIdx.x - 64) % p.kt;
+        bias_s[threadIdx.x - 64] = (EPI != EPI_INT && p.bias && (int)(threadIdx.x - 64) < p.gh * p.gw * p.kt && col < p.K)
                                        ? (float)p.bias[col] * p.table[p.slot_bias].scale *
                                              (p.probe ? 1.0f : p.table[p.slotC].inv_scale)
                                        : 0.0f;
@@ -338,7 +380,7 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap mapI0,
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const unsigned tmem_base = *tmem_holder;
+    const unsigned tmem_base = (unsigned)warp_uniform((int)*tmem_holder);
 
     if (warp == 0) {
         if (elect_one()) {
@@ -354,15 +396,16 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap mapI0,
             const int n_mma = p.n_mma;
             unsigned empty_parity = 1;         // the first pass over the ring finds every stage free
             bool ok = true;
-            const int Q = p.Q, nblk = p.nblk;
-            int nb = (int)blockIdx.x % nblk, pq = (int)blockIdx.x / nblk, q = pq % Q, pp = pq / Q;
-            const int d_nb = (int)gridDim.x % nblk, d_pq = (int)gridDim.x / nblk, d_q = d_pq % Q,
-                      d_p = d_pq / Q;
+            const int tq = p.tq, nblk = p.nblk;
+            int nb = (int)blockIdx.x % nblk, pq = (int)blockIdx.x / nblk, q = pq % tq, pp = pq / tq;
+            const int d_nb = (int)gridDim.x % nblk, d_pq = (int)gridDim.x / nblk, d_q = d_pq % tq,
+                      d_p = d_pq / tq;
+            const int step_h = p.gh * p.str_h, step_w = p.gw * p.str_w;
             for (int tile = blockIdx.x; tile < p.num_tiles && ok; tile += gridDim.x) {
                 unsigned long long* fb = full_bar + mma * kConvMaxStages;            // its consumer's
                 if (++mma == n_mma) mma = 0;
                 const int n0 = nb * 128;
-                const int h0 = pp * p.str_h - p.pad_h, w0 = q * p.str_w - p.pad_w;
+                const int h0 = pp * step_h - p.pad_h, w0 = q * step_w - p.pad_w;
                 for (int cc = 0; cc < p.cchunks; ++cc) {
                     if (!mbar_wait(&empty_bar[s], empty_parity)) {
                         atomicExch(fail_flag, 1); ok = false; break;
@@ -375,7 +418,7 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap mapI0,
                 }
                 nb += d_nb; q += d_q; pp += d_p;
                 if (nb >= nblk) { nb -= nblk; ++q; }
-                if (q >= Q) { q -= Q; ++pp; }
+                if (q >= tq) { q -= tq; ++pp; }
             }
         }
     } else if (warp == 1 || warp >= 18) {
@@ -470,8 +513,11 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap mapI0,
         const int slot = (warp - 2) >> 2;
         const int set = slot / epi_w, part = slot % epi_w;
         const int ncol0 = blockIdx.y * p.kt;                  // first output channel of this CTA
-        int kt = p.K - ncol0;                                  // output channels this CTA owns
-        if (kt > p.kt) kt = p.kt;
+        // columns of the accumulators: gh*gw pixels x kt channels, then one sum column per pixel.
+        // (a tile of several pixels has kt a multiple of 16, so no piece of columns straddles two
+        // pixels; kt > channels left only where K is cut into CTA columns, and then G is 1)
+        const int G = p.gh * p.gw, kt = p.kt, ncols = G * kt;
+        const int left = p.K - ncol0 < kt ? p.K - ncol0 : kt;  // output channels this CTA owns
         int stat = 0;
         unsigned long long pmax = 0;
         const int n_mma_e = p.n_mma;
@@ -483,182 +529,253 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap mapI0,
         // sum is the real-valued sum times that power, bit for bit); the probe keeps real values
         const float q_out = p.probe ? 1.0f : p.table[p.slotC].inv_scale;
         const float f_conv = p.table[p.slotA].scale * p.table[p.slotB].scale * q_out;
-        const float s_res = p.residual ? p.table[p.slot_res].scale * q_out : 0.0f;
-        float fmax_probe = 0.0f, fstat = 0.0f;
-        const unsigned ldc32 = (unsigned)p.ldc;                // (the host checks that K*ldc fits)
+        const float s_res = EPI == EPI_RESIDUAL ? p.table[p.slot_res].scale * q_out : 0.0f;
+        const unsigned long long s_res2 = pack2(s_res, s_res), f_conv2 = pack2(f_conv, f_conv),
+                                 k256 = pack2(256.0f, 256.0f), k65536 = pack2(65536.0f, 65536.0f),
+                                 kmagic = pack2(12582912.0f, 12582912.0f);
+        float fstat = 0.0f;
+        const OFF ldc = (OFF)p.ldc;
         unsigned char* const out_lo = p.out_planes + p.out_plane_bytes;
         const bool fast = sh >= 1 && sh <= 31;
         const unsigned rmask = fast ? (1u << sh) - 1u : 0u, rhalf = fast ? 1u << (sh - 1) : 0u;
         bool ok = true;
         // this warp's tiles: every nbuf-th one of the CTA; `next` is the issuing thread of the
-        // tile that follows in the same accumulator set
+        // tile that follows in the same accumulator set.  Coordinates advance with carries, as in
+        // the producer.
         const int buf = set, nbuf = p.nbuf, d_next = nbuf % n_mma_e;
         int next = (set + nbuf) % n_mma_e;
         unsigned full_parity = 0;
+        const int tq = p.tq, nblk = p.nblk;
+        const int first = (int)blockIdx.x + set * (int)gridDim.x, step = nbuf * (int)gridDim.x;
+        int nb = first % nblk, pq = first / nblk, tx = pq % tq, ty = pq / tq;
+        const int d_nb = step % nblk, d_pq = step / nblk, d_x = d_pq % tq, d_y = d_pq / tq;
+        // Stores and the residual go through 512 bytes of shared memory of this warp each: a
+        // thread computes one image of eight channels, but stores eight images of one channel --
+        // one 8-byte store per plane (16 bytes for int16) in place of eight of one byte.
+        // Two halves used in turn, so that one __syncwarp between writing and reading is enough.
+        unsigned char* const stage_smem = epi_smem + (warp - 2) * 1024;
+        unsigned stage = 0;
+        const int epi_mask = epi_w - 1, kt8 = (kt + 7) >> 3 & epi_mask;
+        const bool probing = !EVEN && p.probe;
+        const float z_lo = p.relu ? 0.0f : (probing ? -INFINITY : -32768.0f),
+                    z_hi = probing ? INFINITY : 32767.0f;
+        const int scol = lane >> 2;                            // channel of the piece this lane stores
+        const int simg = quarter * 32 + (lane & 3) * 8;        // and its first image in the tile
         // (with three sets the warps of the fourth slot have none)
         for (int ti = set < nbuf ? set : n_my; ti < n_my; ti += nbuf) {
-            const int tile = (int)blockIdx.x + ti * (int)gridDim.x;
-            const long long row = (long long)tile * 128 + quarter * 32 + lane;   // (pq*N + n)
-            // the residual of the first piece is fetched while the tile is still being multiplied
-            short rz[8];
-            const unsigned row32 = (unsigned)row;
-            auto load_res = [&](int cc0) {
-                const unsigned off = (unsigned)(ncol0 + cc0) * ldc32 + row32;
-#pragma unroll
-                for (int j = 0; j < 8; ++j)
-                    rz[j] = cc0 + j < kt ? p.residual[off + (unsigned)j * ldc32] : (short)0;
+            const int p0 = ty * p.gh, q0 = tx * p.gw;
+            // a pixel of the tile: inside the image or not, and its offset within a channel
+            auto pixel = [&](int g, OFF& off) -> bool {
+                const int gy = p.gw == 1 ? g : g >> 1, gx = p.gw == 1 ? 0 : g & 1;
+                off = (OFF)((p0 + gy) * p.Q + q0 + gx) * (OFF)p.N + (OFF)(nb * 128);
+                return p0 + gy < p.P && q0 + gx < p.Q;
             };
-            if (p.fused && p.residual) load_res(part * 8);
-            if (ok && !mbar_wait(&tmem_full[buf], full_parity)) { atomicExch(fail_flag, 1); ok = false; }
-            full_parity ^= 1u;
-            tc_fence_after();
-            const unsigned lane_addr = tmem_base + buf * acc_cols + ((unsigned)(quarter * 32) << 16);
-            // 128 * (sum of this row's activations), from the extra column p.kt
-            const int s_hi = (int)tmem_ld1(lane_addr + bn + p.kt);
-            const int s_lo = (int)tmem_ld1(lane_addr + 2 * bn + p.kt);
-            tmem_ld_wait();
-            const long long fix = 128LL * (256LL * (long long)s_hi + (long long)s_lo);
-            const float fixf = (float)fix;
-            if (p.fused) {
+            if (EPI != EPI_INT) {
                 // fp32 epilogue: the exact integer sum scaled to a real value, bias and residual
                 // added, ReLU, ONE quantisation with the output's exponent.  Eight columns at a
                 // time, loads first, then arithmetic, then stores: eight independent chains.  The
                 // warps that share a lane quarter take the 8-column pieces in turn.
-                // What bounds it is instruction issue (68 % of the slots in the form before this
-                // one: a flag test per stored value, 64-bit addresses), so every choice is made
-                // once per piece and addresses are a uniform base plus a 32-bit offset.
-                for (int cc0 = part * 8; cc0 < kt; cc0 += 8 * epi_w) {
-                    unsigned hh[8], xx[8], ll[8];
-                    tmem_ld8(lane_addr + cc0, hh);
-                    tmem_ld8(lane_addr + bn + cc0, xx);
-                    tmem_ld8(lane_addr + 2 * bn + cc0, ll);
-                    const int live = kt - cc0;
-                    float y[8];
-                    if (p.residual) {
-#pragma unroll
-                        for (int j = 0; j < 8; ++j) y[j] = fmaf((float)rz[j], s_res, bias_s[cc0 + j]);
-                        // and the next piece's, one piece ahead of its use
-                        const int nx = cc0 + 8 * epi_w;
-                        if (nx < kt) load_res(nx);
-                    } else {
-#pragma unroll
-                        for (int j = 0; j < 8; ++j) y[j] = bias_s[cc0 + j];
-                    }
+                // Instruction issue bounds it, so choices are made once per pixel or piece, sums
+                // are formed two at a time (fma.f32x2), and addresses once per pixel.
+                uint4 rq = make_uint4(0, 0, 0, 0);
+                OFF off;
+                bool inside = pixel(0, off);
+                off += (OFF)(ncol0 + scol) * ldc + (OFF)simg;
+                // the residual of the first piece is fetched while the tile is being multiplied
+                int c = (part & epi_mask) * 8;
+                if (EPI == EPI_RESIDUAL && inside && c < kt && (EVEN || c + scol < left))
+                    rq = load8(p.residual + off + (OFF)c * ldc, EVEN || p.vec);
+                if (ok && !mbar_wait(&tmem_full[buf], full_parity)) { atomicExch(fail_flag, 1); ok = false; }
+                tc_fence_after();
+                const unsigned lane_addr = tmem_base + buf * acc_cols + ((unsigned)(quarter * 32) << 16);
+                bool ahead = false;
+                for (int g = 0, start = part; g < G; ++g) {
+                    // 128 * (sum of the activations under the pixel's window), from its sum column
+                    // (|sum of activations| < 2^30: exact in 32 bits)
+                    const unsigned s_hi = tmem_ld1(lane_addr + bn + ncols + g);
+                    const unsigned s_lo = tmem_ld1(lane_addr + 2 * bn + ncols + g);
                     tmem_ld_wait();
-                    if (!ok) continue;
-                    if (p.short_sum) {
-                        // 256*HH + X fits 32 bits: two conversions a value instead of three (they
-                        // run at a quarter of the rate of the rest)
-#pragma unroll
-                        for (int j = 0; j < 8; ++j) {
-                            const float t = (float)((int)(hh[j] << 8) + (int)xx[j]);
-                            y[j] = fmaf(fmaf(t, 256.0f, (float)(int)ll[j] + fixf), f_conv, y[j]);
+                    const float fixf = 128.0f * (float)(int)(s_hi * 256u + s_lo);
+                    const unsigned long long fix2 = pack2(fixf, fixf);
+                    const unsigned col0 = lane_addr + g * kt;
+                    const bool here = inside && ok;
+                    const OFF at_g = off;
+                    start = (start + epi_w - kt8) & epi_mask;     // first piece of this warp in pixel g+1
+                    for (; c < kt; c += 8 * epi_w) {
+                        unsigned hh[8], xx[8], ll[8];
+                        tmem_ld8(col0 + c, hh);
+                        tmem_ld8(col0 + bn + c, xx);
+                        tmem_ld8(col0 + 2 * bn + c, ll);
+                        const int live = left - c;
+                        const OFF at = at_g + (OFF)c * ldc;
+                        unsigned long long y[4];
+                        {
+                            const ulonglong2 b0 = *reinterpret_cast<const ulonglong2*>(bias_s + c);
+                            const ulonglong2 b1 = *reinterpret_cast<const ulonglong2*>(bias_s + c + 4);
+                            y[0] = b0.x; y[1] = b0.y; y[2] = b1.x; y[3] = b1.y;
                         }
-                    } else {
+                        stage ^= 512;
+                        if (EPI == EPI_RESIDUAL) {
+                            *reinterpret_cast<uint4*>(stage_smem + stage + lane * 16) = rq;
+                            __syncwarp();
+                            const short* rs = reinterpret_cast<const short*>(stage_smem + stage + lane * 2);
 #pragma unroll
-                        for (int j = 0; j < 8; ++j) {
+                            for (int j = 0; j < 4; ++j)
+                                y[j] = fma2(pack2((float)rs[64 * j], (float)rs[64 * j + 32]), s_res2, y[j]);
+                            stage ^= 512;
+                            // the residual of the next piece, one piece ahead of its use
+                            int cn = c + 8 * epi_w;
+                            OFF offn = at_g;
+                            bool in = inside;
+                            if (cn >= kt && g + 1 < G) {
+                                in = pixel(g + 1, offn);
+                                offn += (OFF)(ncol0 + scol) * ldc + (OFF)simg;
+                                cn = start * 8;
+                                ahead = true;
+                            }
+                            if (in && cn < kt && (EVEN || cn + scol < left))
+                                rq = load8(p.residual + offn + (OFF)cn * ldc, EVEN || p.vec);
+                        }
+                        tmem_ld_wait();
+                        if (!here) continue;
+                        if (SHORT) {
+                            // 256*HH + X fits 32 bits: two conversions a value instead of three
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) {
+                                const unsigned long long t =
+                                    pack2((float)(int)((hh[2 * j] << 8) + xx[2 * j]),
+                                          (float)(int)((hh[2 * j + 1] << 8) + xx[2 * j + 1]));
+                                const unsigned long long l =
+                                    add2(pack2((float)(int)ll[2 * j], (float)(int)ll[2 * j + 1]), fix2);
+                                y[j] = fma2(fma2(t, k256, l), f_conv2, y[j]);
+                            }
+                        } else {
                             // correctly rounded conversions instead of a 64-bit sum: the fp32
                             // result is quantised to 16 bits right after
-                            const float acc = fmaf((float)(int)hh[j], 65536.0f,
-                                                   fmaf((float)(int)xx[j], 256.0f, (float)(int)ll[j] + fixf));
-                            y[j] = fmaf(acc, f_conv, y[j]);
-                        }
-                    }
-                    if (p.relu) {
 #pragma unroll
-                        for (int j = 0; j < 8; ++j) y[j] = fmaxf(y[j], 0.0f);      // also NaN -> 0
-                    } else if (!p.probe) {
-#pragma unroll
-                        for (int j = 0; j < 8; ++j) y[j] = (y[j] != y[j]) ? 0.0f : fmaxf(y[j], -32768.0f);
-                    }
-                    if (p.probe) {
-#pragma unroll
-                        for (int j = 0; j < 8; ++j)
-                            if (j < live) fmax_probe = fmaxf(fmax_probe, fabsf(y[j]));
-                        continue;
-                    }
-                    // y is already in units of the output's step (see f_conv): clamp, round to
-                    // nearest even by the magic-number add; the low 16 bits of the sum are the
-                    // mantissa, so the bytes are stored straight from it
-                    int m[8];
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) {
-                        y[j] = fminf(y[j], 32767.0f);
-                        m[j] = __float_as_int(y[j] + 12582912.0f);
-                    }
-                    const unsigned off = (unsigned)(ncol0 + cc0) * ldc32 + row32;
-                    if (live >= 8) {
-#pragma unroll
-                        for (int j = 0; j < 8; ++j) fstat = fmaxf(fstat, fabsf(y[j]));
-                        if (p.out_planes) {
-#pragma unroll
-                            for (int j = 0; j < 8; ++j) {
-                                const unsigned at = off + (unsigned)j * ldc32;
-                                p.out_planes[at] = (unsigned char)(m[j] >> 8);
-                                out_lo[at] = (unsigned char)m[j];
+                            for (int j = 0; j < 4; ++j) {
+                                const unsigned long long l =
+                                    add2(pack2((float)(int)ll[2 * j], (float)(int)ll[2 * j + 1]), fix2);
+                                const unsigned long long x =
+                                    fma2(pack2((float)(int)xx[2 * j], (float)(int)xx[2 * j + 1]), k256, l);
+                                const unsigned long long h = pack2((float)(int)hh[2 * j], (float)(int)hh[2 * j + 1]);
+                                y[j] = fma2(fma2(h, k65536, x), f_conv2, y[j]);
                             }
                         }
-                        if (p.write_i16) {
+                        // in units of the output's step (see f_conv): ReLU and clamp, round to
+                        // nearest even by the magic-number add; the low 16 bits of the sum are the
+                        // mantissa.  (No NaN can arise: every term is finite.)
+                        float z[8];
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) unpack2(y[j], z[2 * j], z[2 * j + 1]);
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) z[j] = fminf(fmaxf(z[j], z_lo), z_hi);
+                        if (EVEN || live >= 8) {
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) fstat = max3_abs(fstat, z[2 * j], z[2 * j + 1]);
+                        } else {
 #pragma unroll
                             for (int j = 0; j < 8; ++j)
-                                ((short*)p.O)[off + (unsigned)j * ldc32] = (short)m[j];
+                                if (j < live) fstat = fmaxf(fstat, fabsf(z[j]));
                         }
-                    } else {
+                        if (!EVEN && p.probe) { __syncwarp(); continue; }
+                        unsigned short* so = reinterpret_cast<unsigned short*>(stage_smem + stage + lane * 2);
 #pragma unroll
-                        for (int j = 0; j < 8; ++j) {
-                            if (j < live) {
-                                fstat = fmaxf(fstat, fabsf(y[j]));
-                                const unsigned at = off + (unsigned)j * ldc32;
-                                if (p.write_i16) ((short*)p.O)[at] = (short)m[j];
+                        for (int j = 0; j < 4; ++j) {
+                            float a, b;
+                            unpack2(add2(pack2(z[2 * j], z[2 * j + 1]), kmagic), a, b);
+                            so[64 * j] = (unsigned short)__float_as_uint(a);
+                            so[64 * j + 32] = (unsigned short)__float_as_uint(b);
+                        }
+                        __syncwarp();
+                        const uint4 w = *reinterpret_cast<const uint4*>(stage_smem + stage + lane * 16);
+                        if (EVEN || (scol < live && p.vec)) {
+                            if (p.out_planes) {
+                                *reinterpret_cast<uint2*>(p.out_planes + at) =
+                                    make_uint2(__byte_perm(w.x, w.y, 0x7531), __byte_perm(w.z, w.w, 0x7531));
+                                *reinterpret_cast<uint2*>(out_lo + at) =
+                                    make_uint2(__byte_perm(w.x, w.y, 0x6420), __byte_perm(w.z, w.w, 0x6420));
+                            }
+                            if (p.write_i16) *reinterpret_cast<uint4*>((short*)p.O + at) = w;
+                        } else if (scol < live) {
+                            const unsigned v[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll 1
+                            for (int j = 0; j < 8; ++j) {
+                                const unsigned m = (j & 4 ? (j & 2 ? v[3] : v[2]) : (j & 2 ? v[1] : v[0])) >> 16 * (j & 1);
                                 if (p.out_planes) {
-                                    p.out_planes[at] = (unsigned char)(m[j] >> 8);
-                                    out_lo[at] = (unsigned char)m[j];
+                                    p.out_planes[at + j] = (unsigned char)(m >> 8);
+                                    out_lo[at + j] = (unsigned char)m;
                                 }
+                                if (p.write_i16) ((short*)p.O)[at + j] = (short)m;
                             }
                         }
                     }
+                    if (g + 1 < G) {
+                        inside = pixel(g + 1, off);
+                        off += (OFF)(ncol0 + scol) * ldc + (OFF)simg;
+                        c = start * 8;
+                        // (a pixel in which this warp had no piece has fetched nothing ahead)
+                        if (EPI == EPI_RESIDUAL && !ahead && inside && c < kt && (EVEN || c + scol < left))
+                            rq = load8(p.residual + off + (OFF)c * ldc, EVEN || p.vec);
+                        ahead = false;
+                    }
                 }
-            } else
-            for (int c0 = part * 16; c0 < kt; c0 += 16 * epi_w) {
-                unsigned hh[16], xx[16], ll[16];
-                tmem_ld16(lane_addr + c0, hh);
-                tmem_ld16(lane_addr + bn + c0, xx);
-                tmem_ld16(lane_addr + 2 * bn + c0, ll);
-                tmem_ld_wait();
-                if (!ok) continue;
-                short* out = (short*)p.O + (long long)(ncol0 + c0) * p.ldc + row;
-                long long v[16];
+            } else {
+                if (ok && !mbar_wait(&tmem_full[buf], full_parity)) { atomicExch(fail_flag, 1); ok = false; }
+                tc_fence_after();
+                const unsigned lane_addr = tmem_base + buf * acc_cols + ((unsigned)(quarter * 32) << 16);
+                for (int c0 = part * 16; c0 < ncols; c0 += 16 * epi_w) {
+                    unsigned hh[16], xx[16], ll[16];
+                    const int g = G == 1 ? 0 : c0 / kt, chan = c0 - g * kt;
+                    OFF off;
+                    const bool inside = pixel(g, off);
+                    off += (OFF)(ncol0 + chan) * ldc + (OFF)(quarter * 32 + lane);
+                    const unsigned s_hi = tmem_ld1(lane_addr + bn + ncols + g);
+                    const unsigned s_lo = tmem_ld1(lane_addr + 2 * bn + ncols + g);
+                    tmem_ld16(lane_addr + c0, hh);
+                    tmem_ld16(lane_addr + bn + c0, xx);
+                    tmem_ld16(lane_addr + 2 * bn + c0, ll);
+                    tmem_ld_wait();
+                    const int live = left - chan;
+                    if (!ok || !inside) continue;
+                    short* out = (short*)p.O + off;
+                    const long long fix = 128LL * (long long)(int)(s_hi * 256u + s_lo);
+                    long long v[16];
 #pragma unroll
-                for (int j = 0; j < 16; ++j)
-                    v[j] = ((long long)(int)hh[j] << 16) + ((long long)(int)xx[j] << 8) +
-                           (long long)(int)ll[j] + fix;
-                if (p.probe) {
+                    for (int j = 0; j < 16; ++j)
+                        v[j] = ((long long)(int)hh[j] << 16) + ((long long)(int)xx[j] << 8) +
+                               (long long)(int)ll[j] + fix;
+                    if (p.probe) {
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) {
+                            const unsigned long long a = (unsigned long long)(v[j] < 0 ? -v[j] : v[j]);
+                            if (j < live) pmax = a > pmax ? a : pmax;
+                        }
+                        continue;
+                    }
+                    // all sixteen values first, then the stores: independent chains for the scheduler
+                    int q[16];
+                    if (fast) {
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) q[j] = rescale_i64_fast(v[j], sh, rmask, rhalf);
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) q[j] = rescale_i64(v[j], sh);
+                    }
 #pragma unroll
                     for (int j = 0; j < 16; ++j) {
-                        const unsigned long long a = (unsigned long long)(v[j] < 0 ? -v[j] : v[j]);
-                        if (c0 + j < kt) pmax = a > pmax ? a : pmax;
-                    }
-                    continue;
-                }
-                // all sixteen values first, then the stores: independent chains for the scheduler
-                int q[16];
-                if (fast) {
-#pragma unroll
-                    for (int j = 0; j < 16; ++j) q[j] = rescale_i64_fast(v[j], sh, rmask, rhalf);
-                } else {
-#pragma unroll
-                    for (int j = 0; j < 16; ++j) q[j] = rescale_i64(v[j], sh);
-                }
-                const int live = kt - c0;
-#pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                    if (j < live) {
-                        const int a = q[j] < 0 ? -q[j] : q[j];
-                        stat = a > stat ? a : stat;
-                        out[(long long)j * p.ldc] = (short)q[j];
+                        if (j < live) {
+                            const int a = q[j] < 0 ? -q[j] : q[j];
+                            stat = a > stat ? a : stat;
+                            out[(long long)j * p.ldc] = (short)q[j];
+                        }
                     }
                 }
             }
+            full_parity ^= 1u;
+            nb += d_nb; tx += d_x; ty += d_y;
+            if (nb >= nblk) { nb -= nblk; ++tx; }
+            if (tx >= tq) { tx -= tq; ++ty; }
             // this warp has read its part of the accumulator set
             tc_fence_before();
             __syncwarp();
@@ -669,7 +786,7 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap mapI0,
         }
         if (p.probe) {
             // fused: the bit pattern of max |y| (fp32); plain: max |integer sum|
-            if (p.fused) pmax = (unsigned long long)__float_as_uint(fmax_probe);
+            if (EPI != EPI_INT) pmax = (unsigned long long)__float_as_uint(fstat);
             for (int o = 16; o > 0; o >>= 1) {
                 const unsigned long long t = __shfl_xor_sync(0xffffffffu, pmax, o);
                 pmax = t > pmax ? t : pmax;
@@ -740,51 +857,58 @@ split_same_layout_kernel(const T* __restrict__ src, long long n, void* __restric
 }
 
 // filters C,R,S,K -> ONE array [ntn][2*bn rows][kp] for the implicit kernel: for every CTA column
-// the high bytes of its kt output channels (rows 0..bn-1) and, behind them, the low bytes minus
-// 128 as signed bytes (rows bn..2bn-1).  Row kt of either half is the sum column: 0 in the high
-// half, +1 in the low half, on every K position the MMAs touch.  The K positions of chunk cc start
-// at cc*kc_pad and run over (channel within the chunk, r, s); padding positions and channels
-// beyond C hold the filter value 0 (bytes 0 and -128).
+// the high bytes of its output channels (rows 0..bn-1) and, behind them, the low bytes minus 128 as
+// signed bytes (rows bn..2bn-1).  A tile covers gh x gw output pixels: row g*kt + k holds output
+// channel k as pixel g sees it, that is, shifted by (g/gw)*str_h, (g%gw)*str_w inside the common
+// window of wh x ww taps; row gh*gw*kt + g is pixel g's sum column: 0 in the high half, +1 in the
+// low half on the taps of its own R x S window.  Everything else -- taps of the common window that
+// are not the pixel's, channels beyond C, padding -- is zero in both halves, so it adds nothing
+// whatever the operand holds there.  The K positions of chunk cc start at cc*kc_pad and run over
+// (channel within the chunk, tap row, tap column).
+struct FilterLayout {
+    int C, R, S, K, cu, cchunks, kc_pad, ntn, bn, kt, kp, gh, gw, str_h, str_w, wh, ww;
+};
+
 template <typename T>
 __global__ void __launch_bounds__(256)
-filter_planes_kernel(const T* __restrict__ F, int C, int RS, int K, int cu, int cchunks, int kc_pad,
-                     int ntn, int bn, int kt, int kp, int bprop, unsigned char* __restrict__ planes) {
-    const long long total = (long long)ntn * 2 * bn * kp;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
-         i += (long long)gridDim.x * blockDim.x) {
-        const int kc = (int)(i % kp);
-        const int r2 = (int)((i / kp) % (2 * bn)), tile = (int)(i / ((long long)kp * 2 * bn));
-        const bool low = r2 >= bn;
-        const int col = low ? r2 - bn : r2;
-        const int cc = kc / kc_pad, within = kc - cc * kc_pad;
-        int m = 0;                                           // the filter mantissa at this position
-        bool sum_col = false;
-        if (col == kt) {
-            sum_col = cc < cchunks;
-        } else if (col < kt && tile * kt + col < K && cc < cchunks && within < cu * RS) {
-            const int cl = within / RS, tap = within - cl * RS;
-            const int c = cc * cu + cl;
-            // bprop: the filter tensor is that of the FORWARD convolution, [K outputs here = its
-            // input channels][R][S][C reduced here = its output channels], read flipped
-            if (c < C)
-                m = bprop ? (int)F[((long long)(tile * kt + col) * RS + (RS - 1 - tap)) * C + c]
-                          : (int)F[((long long)c * RS + tap) * K + tile * kt + col];
-        }
-        unsigned char v;
-        if (sum_col) v = low ? 1 : 0;
-        else {
-            const int lo = m & 0xff;
-            v = low ? (unsigned char)(lo ^ 0x80) : (unsigned char)(((m - lo) >> 8) & 0xff);
+filter_planes_kernel(const T* __restrict__ F, const FilterLayout f, int bprop,
+                     unsigned char* __restrict__ planes) {
+    const int total = f.ntn * 2 * f.bn * f.kp, G = f.gh * f.gw, RS = f.R * f.S;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+        const int kc = i % f.kp;
+        const int r2 = (i / f.kp) % (2 * f.bn), tile = i / f.kp / (2 * f.bn);
+        const bool low = r2 >= f.bn;
+        const int col = low ? r2 - f.bn : r2;
+        const int cc = kc / f.kc_pad, within = kc - cc * f.kc_pad;
+        const int cl = within / (f.wh * f.ww), tap = within - cl * f.wh * f.ww;
+        const int th = tap / f.ww, tw = tap - th * f.ww;
+        const bool sum_col = col >= G * f.kt;
+        const int g = sum_col ? col - G * f.kt : col / f.kt, k = tile * f.kt + (sum_col ? 0 : col % f.kt);
+        const int r = th - g / f.gw * f.str_h, s = tw - g % f.gw * f.str_w, c = cc * f.cu + cl;
+        unsigned char v = 0;
+        if (g < G && r >= 0 && r < f.R && s >= 0 && s < f.S && cl < f.cu && cc < f.cchunks && c < f.C &&
+            k < f.K) {
+            if (sum_col) {
+                v = low ? 1 : 0;
+            } else {
+                // bprop: the filter tensor is that of the FORWARD convolution, [K outputs here =
+                // its input channels][R][S][C reduced here = its output channels], read flipped
+                const int at = r * f.S + s;
+                const int m = bprop ? (int)F[((long long)k * RS + (RS - 1 - at)) * f.C + c]
+                                    : (int)F[((long long)c * RS + at) * f.K + k];
+                const int lo = m & 0xff;
+                v = low ? (unsigned char)(lo ^ 0x80) : (unsigned char)(((m - lo) >> 8) & 0xff);
+            }
         }
         planes[i] = v;
     }
 }
 
-// int8 plane in C,H,W,N layout; box = [cu][R][S][128 images]
-int make_map_4d(CUtensorMap* map, void* base, const ConvGeom& g, int cu) {
+// int8 plane in C,H,W,N layout; box = [cu][wh][ww][128 images]
+int make_map_4d(CUtensorMap* map, void* base, const ConvGeom& g, int cu, int wh, int ww) {
     cuuint64_t dims[4] = {(cuuint64_t)g.N, (cuuint64_t)g.W, (cuuint64_t)g.H, (cuuint64_t)g.C};
     cuuint64_t strides[3] = {(cuuint64_t)g.N, (cuuint64_t)g.W * g.N, (cuuint64_t)g.H * g.W * g.N};
-    cuuint32_t box[4] = {(cuuint32_t)kKBytes, (cuuint32_t)g.S, (cuuint32_t)g.R, (cuuint32_t)cu};
+    cuuint32_t box[4] = {(cuuint32_t)kKBytes, (cuuint32_t)ww, (cuuint32_t)wh, (cuuint32_t)cu};
     cuuint32_t estr[4] = {1, 1, 1, 1};
     CUresult r = g_encode(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, base, dims, strides, box, estr,
                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
@@ -795,38 +919,74 @@ int make_map_4d(CUtensorMap* map, void* base, const ConvGeom& g, int cu) {
 
 struct ImplicitShape {
     int ntn, kt, bn, nbuf, tmem_cols, cu, cchunks, kc_pad, npanels, kp, nstages, smem;
+    int gh, gw, wh, ww, tiles;
     size_t act_plane, filt_bytes, bytes;
 };
 
-ImplicitShape implicit_shape(const ConvGeom& g) {
+// the shape with tiles of gh x gw output pixels; nstages < 2 where it does not fit
+ImplicitShape implicit_shape_for(const ConvGeom& g, int gh, int gw) {
     ImplicitShape s;
-    // output channels per CTA column: at most 127, so that with the sum column the two filter
+    s.gh = gh; s.gw = gw;
+    s.wh = (gh - 1) * g.str_h + g.R; s.ww = (gw - 1) * g.str_w + g.S;
+    const int G = gh * gw, taps = s.wh * s.ww;
+    s.tiles = ((g.P + gh - 1) / gh) * ((g.Q + gw - 1) / gw) * (g.N / 128);
+    // output channels per CTA column: at most 127, so that with the sum columns the two filter
     // planes make one operand of at most 256 rows
     s.ntn = (g.K + 126) / 127;
     s.kt = (g.K + s.ntn - 1) / s.ntn;
-    s.bn = round_up(s.kt + 1, 16);
+    s.bn = round_up(G * (s.kt + 1), 16);
     const int sets = 512 / (3 * s.bn);
     s.nbuf = sets >= 4 ? 4 : sets >= 3 ? 3 : sets >= 2 ? 2 : 1;
     s.tmem_cols = 32;
     while (s.tmem_cols < 3 * s.bn * s.nbuf) s.tmem_cols *= 2;
-    const int RS = g.R * g.S;
-    // 16 channels per chunk for real windows (a 3x3 chunk is 144 rows = 18 KB per plane); a 1x1
-    // filter takes up to 128 channels per chunk
-    s.cu = RS > 1 ? 16 : (g.C >= 128 ? 128 : round_up(g.C, 32));
+    // channels per chunk: about 36 KB for the two planes of a stage (a 3x3 chunk of 16 channels is
+    // 144 rows of 128 bytes), so that several stages are in flight; 1x1 filters on single pixels
+    // take up to 128 channels
+    if (taps == 1) s.cu = g.C >= 128 ? 128 : round_up(g.C, 32);
+    else s.cu = taps > 64 ? 2 : taps > 20 ? 4 : taps > 10 ? 8 : taps > 4 ? 16 : 32;
     s.cchunks = (g.C + s.cu - 1) / s.cu;
-    s.kc_pad = round_up(s.cu * RS, 32);
+    s.kc_pad = round_up(s.cu * taps, 32);
     s.kp = round_up(s.cchunks * s.kc_pad, kKBytes);
     s.npanels = s.kp / kKBytes;
     const int filt_smem = s.npanels * 2 * s.bn * kKBytes;
     const int stage = 2 * s.kc_pad * 128;
     int nst = (kConvSmemMax - kConvSmemFixed - filt_smem) / stage;
     if (nst > kConvMaxStages) nst = kConvMaxStages;
-    s.nstages = nst;
+    s.nstages = s.bn > 128 || s.wh > 256 || s.ww > 256 ? 0 : nst;
     s.smem = kConvSmemFixed + filt_smem + (nst > 0 ? nst : 0) * stage;
     s.act_plane = (((size_t)g.C * g.H * g.W * g.N) + 1023) / 1024 * 1024;
     s.filt_bytes = (((size_t)s.ntn * 2 * s.bn * s.kp) + 1023) / 1024 * 1024;
     s.bytes = 2 * s.act_plane + s.filt_bytes;
     return s;
+}
+
+// Cycles of a launch with that shape, from the costs measured on the kernel with parts of it taken
+// out: an MMA instruction takes the tensor pipe bn cycles (N = 2*bn) but its issuer at least 46;
+// the operand fetch runs at 64 bytes a clock and SM; a column costs the sixteen epilogue warps 27;
+// and every tile about 300 for the hand-overs between the roles, whatever it holds.
+long long implicit_cost(const ImplicitShape& s) {
+    const long long mma = (long long)s.cchunks * (s.kc_pad / 32) * 2 * (s.bn > 46 ? s.bn : 46);
+    const long long fetch = (long long)s.cchunks * s.cu * s.wh * s.ww * 2 * 128 / 64;
+    const long long epi = 27LL * s.gh * s.gw * s.kt;
+    long long t = mma > fetch ? mma : fetch;
+    if (epi > t) t = epi;
+    return (long long)((s.tiles * s.ntn + 147) / 148) * (t + 300);
+}
+
+// How many output pixels a tile covers: few channels leave the tensor pipe and the hand-overs
+// between the roles mostly idle on one pixel (a 16-channel 3x3 layer spends 550 cycles of a tile on
+// twelve narrow instructions and as many on waiting), and neighbouring pixels share most of their
+// window.  One pixel where the channels fill the operand, where a group would leave SMs without
+// a tile, or where the window grows too much (strides).
+ImplicitShape implicit_shape(const ConvGeom& g) {
+    ImplicitShape best = implicit_shape_for(g, 1, 1);
+    if (best.ntn > 1 || best.kt % 16 != 0) return best;
+    static const int cand[3][2] = {{1, 2}, {2, 1}, {2, 2}};
+    for (int i = 0; i < 3; ++i) {
+        const ImplicitShape s = implicit_shape_for(g, cand[i][0], cand[i][1]);
+        if (s.nstages >= 3 && s.bn <= 80 && implicit_cost(s) < implicit_cost(best)) best = s;
+    }
+    return best;
 }
 
 // flex16 only: an MN-major tf32 operand needs the 32-byte-atom variant of the 128-byte swizzle
@@ -926,11 +1086,12 @@ template <typename T, int MODE>
 int implicit_filter_planes(const T* F, const ConvGeom& g, const ImplicitShape& s, void* planes,
                            cudaStream_t st, int bprop = 0) {
     const long long n_f = (long long)s.ntn * 2 * s.bn * s.kp;
+    B2_REQUIRE(n_f < (1LL << 30), "filter tensor too large");
     long long fb = (n_f + 255) / 256;
     if (fb > 148 * 8) fb = 148 * 8;
-    filter_planes_kernel<T><<<(unsigned)fb, 256, 0, st>>>(F, g.C, g.R * g.S, g.K, s.cu, s.cchunks,
-                                                        s.kc_pad, s.ntn, s.bn, s.kt, s.kp, bprop,
-                                                        (unsigned char*)planes);
+    const FilterLayout f = {g.C, g.R, g.S, g.K, s.cu, s.cchunks, s.kc_pad, s.ntn, s.bn, s.kt, s.kp,
+                            s.gh, s.gw, g.str_h, g.str_w, s.wh, s.ww};
+    filter_planes_kernel<T><<<(unsigned)fb, 256, 0, st>>>(F, f, bprop, (unsigned char*)planes);
     B2_CUDA(cudaGetLastError());
     return B2_OK;
 }
@@ -945,44 +1106,37 @@ int implicit_tiles(const void* act_planes, const void* filt_planes, void* O, con
                "operand planes must be 1024-byte aligned");
     void* A0 = (void*)act_planes; void* A1 = (unsigned char*)act_planes + s.act_plane;
     CUtensorMap mI0, mI1, mB;
-    if ((rc = make_map_4d(&mI0, A0, g, s.cu))) return rc;
-    if ((rc = make_map_4d(&mI1, A1, g, s.cu))) return rc;
+    if ((rc = make_map_4d(&mI0, A0, g, s.cu, s.wh, s.ww))) return rc;
+    if ((rc = make_map_4d(&mI1, A1, g, s.cu, s.wh, s.ww))) return rc;
     if ((rc = make_map(&mB, (void*)filt_planes, s.ntn * 2 * s.bn, s.kp, 1, 2 * s.bn))) return rc;
     ConvTileParams p;
     p.P = g.P; p.Q = g.Q; p.N = g.N; p.K = g.K;
     p.pad_h = g.pad_h; p.pad_w = g.pad_w; p.str_h = g.str_h; p.str_w = g.str_w;
     p.cu = s.cu; p.cchunks = s.cchunks; p.kc_pad = s.kc_pad;
-    p.box_bytes = s.cu * g.R * g.S * 128;
+    p.box_bytes = s.cu * s.wh * s.ww * 128;
+    p.gh = s.gh; p.gw = s.gw; p.tq = (g.Q + s.gw - 1) / s.gw;
     p.npanels = s.npanels; p.nstages = s.nstages;
     p.bn = s.bn; p.kt = s.kt; p.nbuf = s.nbuf; p.tmem_cols = s.tmem_cols;
     p.nblk = g.N / 128;
-    p.num_tiles = g.P * g.Q * p.nblk;
+    p.num_tiles = s.tiles;
     p.ldc = (long long)g.P * g.Q * g.N;
     p.O = O; p.table = table; p.slotA = slotI; p.slotB = slotF; p.slotC = slotO;
     p.stats = stats; p.probe_out = probe_out; p.status = status; p.probe = probe;
-    p.fused = 0; p.bias = nullptr; p.residual = nullptr; p.slot_bias = p.slot_res = 0; p.relu = 0;
-    // per K row |HH| <= 2^14 and |X| <= 2 * 2^14 + 2^15, padding rows included
-    p.short_sum = (long long)s.cchunks * s.kc_pad * ((1 << 22) + (1 << 16)) < (1LL << 31);
+    p.vec = 0; p.bias = nullptr; p.residual = nullptr; p.slot_bias = p.slot_res = 0; p.relu = 0;
     p.write_i16 = 1; p.out_planes = nullptr; p.out_plane_bytes = 0;
     if (epi) {
         B2_REQUIRE(!epi->bias || epi->slot_bias >= 0, "bias needs its scale slot");
         B2_REQUIRE(!epi->residual || epi->slot_residual >= 0, "residual needs its scale slot");
         B2_REQUIRE(epi->write_int16 || epi->out_planes, "the fused epilogue stores nothing");
         B2_REQUIRE(!epi->out_planes || ((uintptr_t)epi->out_planes & 15) == 0, "planes alignment");
-        p.fused = 1;
-        B2_REQUIRE((long long)g.K * p.ldc < (1LL << 32), "output tensor too large");
         p.bias = epi->bias; p.slot_bias = epi->slot_bias;
         p.residual = epi->residual; p.slot_res = epi->slot_residual;
         p.relu = epi->relu ? 1 : 0;
         p.write_i16 = epi->write_int16 ? 1 : 0;
         p.out_planes = (unsigned char*)epi->out_planes;
         p.out_plane_bytes = (long long)epi->plane_bytes;
-    }
-    static bool attr_set = false;
-    if (!attr_set) {
-        B2_CUDA(cudaFuncSetAttribute(conv_implicit_kernel,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, kConvSmemMax));
-        attr_set = true;
+        p.vec = (((uintptr_t)epi->residual | (epi->write_int16 ? (uintptr_t)O : 0)) & 15) == 0 &&
+                (epi->plane_bytes & 7) == 0;
     }
     dim3 grid(p.num_tiles < 148 ? p.num_tiles : 148, s.ntn);
     // a CTA with one or two tiles has no use for more accumulator sets than tiles: with fewer
@@ -1000,7 +1154,33 @@ int implicit_tiles(const void* act_planes, const void* filt_planes, void* O, con
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr; cfg.numAttrs = getenv("B2_CONV_NO_PDL") ? 0 : 1;
-    B2_CUDA(cudaLaunchKernelEx(&cfg, conv_implicit_kernel, mI0, mI1, mB, p));
+    typedef void (*Kernel)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const ConvTileParams);
+    typedef unsigned long long U64;
+    static const Kernel kernels[] = {
+        conv_implicit_kernel<unsigned, EPI_INT, false, false>,
+        conv_implicit_kernel<unsigned, EPI_FUSED, false, false>,
+        conv_implicit_kernel<unsigned, EPI_RESIDUAL, false, false>,
+        conv_implicit_kernel<U64, EPI_INT, false, false>,
+        conv_implicit_kernel<U64, EPI_FUSED, false, false>,
+        conv_implicit_kernel<U64, EPI_RESIDUAL, false, false>,
+        conv_implicit_kernel<unsigned, EPI_FUSED, false, true>,
+        conv_implicit_kernel<unsigned, EPI_RESIDUAL, false, true>,
+        conv_implicit_kernel<unsigned, EPI_FUSED, true, true>,
+        conv_implicit_kernel<unsigned, EPI_RESIDUAL, true, true>};
+    // per product |HH| <= 2^14 and |X| <= 2^14 + 2^15
+    const bool short_sum = (long long)g.C * g.R * g.S * ((1 << 22) + (1 << 16)) < (1LL << 31);
+    const bool wide = (long long)g.K * p.ldc >= (1LL << 32);
+    const bool even = epi && !wide && !probe && p.vec && g.K % 8 == 0 && s.kt % 8 == 0;
+    const int tail = !epi ? EPI_INT : p.residual ? EPI_RESIDUAL : EPI_FUSED;
+    const int which = even ? (short_sum ? 7 : 5) + tail : wide ? 3 + tail : tail;
+    static bool attr_set = false;
+    if (!attr_set) {
+        for (size_t i = 0; i < sizeof(kernels) / sizeof(kernels[0]); ++i)
+            B2_CUDA(cudaFuncSetAttribute(kernels[i], cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         kConvSmemMax));
+        attr_set = true;
+    }
+    B2_CUDA(cudaLaunchKernelEx(&cfg, kernels[which], mI0, mI1, mB, p));
     return B2_OK;
 }
 
@@ -1272,7 +1452,7 @@ conv_update_kernel(const __grid_constant__ CUtensorMap mapI0, const __grid_const
     unsigned* tmem_holder = (unsigned*)(tmem_full + 2);
     int* fail_flag = (int*)(tmem_holder + 1);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
     const int chunk = blockIdx.y / p.ntn, ktile = blockIdx.y - chunk * p.ntn;
     const int kb0 = blockIdx.x * p.per;
     int mine = p.nkb - kb0;
@@ -1306,7 +1486,7 @@ conv_update_kernel(const __grid_constant__ CUtensorMap mapI0, const __grid_const
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const unsigned tmem_base = *tmem_holder;
+    const unsigned tmem_base = (unsigned)warp_uniform((int)*tmem_holder);
 
     if (warp == 0) {
         if (elect_one()) {
@@ -1478,8 +1658,8 @@ int run_update_implicit(const T* I, const T* E, void* U, const ConvGeom& g, cons
         E, n_err, eplanes, eplanes + u.err_plane, 0x80808080u);
     B2_CUDA(cudaGetLastError());
     CUtensorMap mI0, mI1, mE0, mE1;
-    if ((rc = make_map_4d(&mI0, base, g, u.cu))) return rc;
-    if ((rc = make_map_4d(&mI1, base + u.act_plane, g, u.cu))) return rc;
+    if ((rc = make_map_4d(&mI0, base, g, u.cu, g.R, g.S))) return rc;
+    if ((rc = make_map_4d(&mI1, base + u.act_plane, g, u.cu, g.R, g.S))) return rc;
     const int cols = g.P * g.Q * g.N;
     if ((rc = make_map(&mE0, eplanes, g.K, cols, 1, u.kt))) return rc;
     if ((rc = make_map(&mE1, eplanes + u.err_plane, g.K, cols, 1, u.kt))) return rc;

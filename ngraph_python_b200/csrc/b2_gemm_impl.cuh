@@ -100,6 +100,10 @@ __device__ __forceinline__ bool mbar_try_wait(unsigned long long* bar, unsigned 
         : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
     return ok != 0;
 }
+// A value that is the same in the whole warp, in a form the compiler knows to be: tensor-memory
+// addresses and the like live in uniform registers, and for a value it cannot prove uniform the
+// compiler emits a loop over the distinct values of the warp around every instruction that needs it.
+__device__ __forceinline__ int warp_uniform(int v) { return __shfl_sync(0xffffffffu, v, 0); }
 // one thread of the (converged) warp
 __device__ __forceinline__ bool elect_one() {
     unsigned ok;
@@ -272,7 +276,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constant__ C
     unsigned* tmem_holder = (unsigned*)(tmem_empty + 2);
     int* fail_flag = (int*)(tmem_holder + 1);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
     const int m0 = blockIdx.y * kBlockM, n0 = blockIdx.x * BN;
     const int kElems = MODE == MODE_FLEX16 ? kKBytes : kKBytes / 4;   // elements of K per k-block
     const int kb0 = p.partial ? blockIdx.z * p.kb_per_split : 0;
@@ -288,7 +292,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constant__ C
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const unsigned tmem_base = *tmem_holder;
+    const unsigned tmem_base = (unsigned)warp_uniform((int)*tmem_holder);
 
     if (warp == 0) {
         if (elect_one()) {
