@@ -183,6 +183,57 @@ int b2_flex_publish(int32_t* stats, int32_t n, const int32_t* status, int32_t* h
                     int32_t* host_status, void* stream);
 
 /* ------------------------------------------------------------------------------------------
+ * The two ends of a recorded step list, and the host work between calls.
+ * b2_call_inputs launches the kernel that takes a call's arguments in: for every input k whose
+ * address in the block is not NULL, dst[0..n) <- the fp32 values there (flex_slot >= 0: quantised
+ * as b2_flex_host_quantize does, with the block's inv_scale, statistic in stats[flex_slot]).  The
+ * block lies in pinned host memory that the device can address and is read when the kernel runs, so
+ * one recorded launch serves every call; so may be the arguments.  table_rows > 0 copies that many
+ * rows of the block's scale table to `table` first.
+ * b2_call_outputs is b2_flex_publish with results: dst[k] (pinned host memory) <- bytes[k] bytes of
+ * src[k], both 16-byte aligned.
+ * b2_call_stage: the address at which the device can read `bytes` bytes of host memory at src:
+ * src itself where it is page-locked, else `pinned`, to which they are copied.
+ * Replace FlexGPUDeviceTensor.__setitem__ / get and the per-kernel statistics read of the reference
+ * (ngraph/transformers/flexgputransform.py:178-208, 347-371).
+ * ------------------------------------------------------------------------------------------ */
+#define B2_CALL_MAX_INPUTS 16
+#define B2_CALL_MAX_OUTPUTS 16
+typedef struct b2_call_arg { const void* src; float inv_scale; int32_t reserved; } b2_call_arg;
+typedef struct b2_call_block {
+    const b2_flex_scale* table; int32_t table_rows; int32_t reserved;
+    b2_call_arg arg[B2_CALL_MAX_INPUTS];
+} b2_call_block;
+typedef struct b2_call_input { void* dst; int64_t n; int32_t flex_slot; int32_t reserved; } b2_call_input;
+typedef struct b2_call_output { const void* src; void* dst; int64_t bytes; } b2_call_output;
+int b2_call_inputs(const b2_call_input* inputs, int32_t n, const b2_call_block* block,
+                   b2_flex_scale* table, int32_t* stats, void* stream);
+int b2_call_outputs(const b2_call_output* outputs, int32_t n, int32_t* stats, int32_t n_stats,
+                    const int32_t* status, int32_t* host_stats, int32_t* host_status, void* stream);
+int b2_call_stage(const void* src, size_t bytes, void* pinned, const void** visible);
+/* Exponent bookkeeping of a whole call over the state arrays of all entries (one row per entry; the
+ * rule is ngraph_python_b200/flex.py's, FlexEntry.begin_write / end_write).
+ *   begin: every initialised entry ids[k] adopts its pending exponent; row slot_write[k] of the host
+ *          table gets it, row slot_read[k] (where it is another one) the exponent of the data stored
+ *          so far.  uploaded[row] holds the exponent each row has; *changed tells whether any moved.
+ *   end:   records maxima[slots[k]] (maxima[k] without slots) for ids[k], no id twice, and chooses
+ *          the next exponents.  undecided[0..*n_undecided) lists the k whose choice lies so close to
+ *          a boundary that it needs exactly rounded sums; *settled: every entry has seen the same
+ *          maximum for longer than its history window and keeps its exponent.
+ * Replace manage_before_computation / manage_after_computation (flexgputransform.py:347-371). */
+#define B2_FLEX_HISTORY 16
+typedef struct b2_flex_state {
+    int64_t *dec, *pending; uint8_t* initialized; int64_t* overflows;
+    double* hist; int64_t *hist_len, *hist_pos; double* run_value; int64_t *run_length, *run_choice;
+} b2_flex_state;
+int b2_flex_begin_call(const b2_flex_state* s, int32_t n, const int64_t* ids,
+                       const int64_t* slot_write, const int64_t* slot_read, int64_t* uploaded,
+                       b2_flex_scale* host_table, int32_t* changed);
+int b2_flex_end_call(const b2_flex_state* s, int32_t n, const int64_t* ids, const int64_t* slots,
+                     const int32_t* maxima, int32_t* undecided, int32_t* n_undecided,
+                     int32_t* settled);
+
+/* ------------------------------------------------------------------------------------------
  * Dense GEMM on tcgen05 tensor cores: C[M,N] = op(A)[M,K] * op(B)[K,N], C row-major (ldc).
  * Replaces: GEMMKernel and the sgemm / fgemm SASS kernels (ngraph/transformers/gpu/gemm.py:26-263,
  * gpu/kernels/sass/fgemm_common_128x128.sass).  op() is given by element strides, as the

@@ -1,0 +1,325 @@
+// What a call of a compiled computation does around its kernels: taking the arguments in, handing
+// the results out, and the exponent bookkeeping of every tensor it writes.
+//
+// Replaces the per-tensor host work of the reference's flex transformer -- one conversion and one
+// upload per argument (ngraph/transformers/flexgputransform.py:178-208), one statistics read per
+// kernel and manage_before / manage_after_computation per tensor (flexgputransform.py:347-371) --
+// by one kernel at each end of a recorded step list and one pass over plain arrays on the host.
+//
+// k_call_inputs is the first node of a recorded step list.  The addresses of a call's arguments
+// stand in a block of pinned host memory that it reads; the values are read from wherever they lie
+// (the caller's own device tensor, the caller's pinned array, or the pinned block into which
+// b2_call_stage copied pageable memory) and stored once, quantised where the tensor is flex16.
+// Bound by what it reads: PCIe for host arguments, HBM for device tensors.  A flex16 argument of
+// 8192 x 16384 values: copy to a staging tensor 173 us + conversion 167 us before, one pass of
+// 6 bytes a value now.
+#include <cmath>
+#include <cstring>
+#if defined(__x86_64__)
+#include <immintrin.h>
+#endif
+
+#include "b2_common.h"
+#include "b2_ew_device.cuh"
+
+namespace {
+
+const int kThreads = 256;
+const int kPerThread = 16;                       // values a thread takes from a chunk
+const int kChunk = kThreads * kPerThread;        // 4096 values
+
+struct Inputs {
+    int n;
+    b2_call_input in[B2_CALL_MAX_INPUTS];
+    long long first_chunk[B2_CALL_MAX_INPUTS + 1];
+};
+
+__device__ __forceinline__ short quant1(float x, float inv, int& stat) {
+    const float v = fminf(fmaxf(x * inv, -32768.0f), 32767.0f);   // power-of-two scaling: exact
+    const int m = (int)v;                                         // truncation toward zero
+    stat = b2_absmax(stat, m);
+    return (short)m;
+}
+
+__global__ void __launch_bounds__(kThreads)
+k_call_inputs(const Inputs a, const b2_call_block* __restrict__ blk, b2_flex_scale* __restrict__ table,
+              int* __restrict__ stats) {
+    __shared__ int ismem[32];
+    __shared__ const float* src_s[B2_CALL_MAX_INPUTS];
+    __shared__ float inv_s[B2_CALL_MAX_INPUTS];
+    if (threadIdx.x < a.n) {
+        src_s[threadIdx.x] = (const float*)blk->arg[threadIdx.x].src;
+        inv_s[threadIdx.x] = blk->arg[threadIdx.x].inv_scale;
+    }
+    // the scale table, when a row of it has changed
+    if (blockIdx.x == gridDim.x - 1 && table && blk->table_rows > 0) {
+        const b2_flex_scale* h = blk->table;
+        for (int i = threadIdx.x; i < blk->table_rows; i += kThreads) table[i] = h[i];
+    }
+    __syncthreads();
+    int stat = 0, cur = 0;
+    for (long long c = blockIdx.x; c < a.first_chunk[a.n]; c += gridDim.x) {
+        int k = cur;
+        while (c >= a.first_chunk[k + 1]) ++k;
+        if (k != cur) {
+            if (a.in[cur].flex_slot >= 0) b2_block_stat(stat, stats + a.in[cur].flex_slot, ismem);
+            stat = 0;
+            cur = k;
+        }
+        const float* src = src_s[k];
+        if (!src) continue;                       // not an argument of this call: keep what is there
+        const long long base = (c - a.first_chunk[k]) * kChunk;
+        const long long left = a.in[k].n - base;
+        const bool flex = a.in[k].flex_slot >= 0;
+        const float inv = inv_s[k];
+        if (left >= kChunk && (((uintptr_t)src | (uintptr_t)a.in[k].dst) & 15) == 0) {
+            float4 v[kPerThread / 4];
+            const float4* s4 = reinterpret_cast<const float4*>(src + base);
+#pragma unroll
+            for (int j = 0; j < kPerThread / 4; ++j) v[j] = __ldcs(s4 + j * kThreads + threadIdx.x);
+            if (flex) {
+                uint2* d = reinterpret_cast<uint2*>((short*)a.in[k].dst + base);
+#pragma unroll
+                for (int j = 0; j < kPerThread / 4; ++j) {
+                    const unsigned short q0 = quant1(v[j].x, inv, stat), q1 = quant1(v[j].y, inv, stat),
+                                         q2 = quant1(v[j].z, inv, stat), q3 = quant1(v[j].w, inv, stat);
+                    d[j * kThreads + threadIdx.x] = make_uint2(q0 | (unsigned)q1 << 16, q2 | (unsigned)q3 << 16);
+                }
+            } else {
+                float4* d = reinterpret_cast<float4*>((float*)a.in[k].dst + base);
+#pragma unroll
+                for (int j = 0; j < kPerThread / 4; ++j) d[j * kThreads + threadIdx.x] = v[j];
+            }
+        } else {
+            // the last chunk of a tensor, or an address that is not 16-byte aligned
+            const long long end = left < kChunk ? left : kChunk;
+#pragma unroll 4
+            for (long long i = threadIdx.x; i < end; i += kThreads) {
+                const float x = __ldcs(src + base + i);
+                if (flex) ((short*)a.in[k].dst)[base + i] = quant1(x, inv, stat);
+                else ((float*)a.in[k].dst)[base + i] = x;
+            }
+        }
+    }
+    if (a.n && a.in[cur].flex_slot >= 0) b2_block_stat(stat, stats + a.in[cur].flex_slot, ismem);
+}
+
+struct Outputs {
+    int n;
+    b2_call_output out[B2_CALL_MAX_OUTPUTS];
+};
+
+// End of a call: results, flex statistics and status word into pinned host memory the device can
+// address, statistics cleared.  Block 0 takes statistics and status, the others the results.
+__global__ void __launch_bounds__(kThreads)
+k_call_outputs(const Outputs o, int* __restrict__ stats, int n_stats, const int* __restrict__ status,
+               int* __restrict__ host_stats, int* __restrict__ host_status) {
+    if (blockIdx.x == 0) {
+        for (int i = threadIdx.x; i < n_stats; i += kThreads) {
+            host_stats[i] = stats[i];
+            stats[i] = 0;
+        }
+        if (threadIdx.x == 0 && status) *host_status = *status;
+    } else {
+        const long long first = (long long)(blockIdx.x - 1) * kThreads + threadIdx.x;
+        const long long stride = (long long)(gridDim.x - 1) * kThreads;
+        for (int k = 0; k < o.n; ++k) {
+            const long long n16 = o.out[k].bytes >> 4;       // (allocations are 16-byte aligned)
+            const uint4* s = reinterpret_cast<const uint4*>(o.out[k].src);
+            uint4* d = reinterpret_cast<uint4*>(o.out[k].dst);
+            for (long long i = first; i < n16; i += stride) d[i] = s[i];
+            const long long tail = (n16 << 4) + first * 2;   // (elements are 2 or 4 bytes)
+            if (tail < o.out[k].bytes)
+                *(unsigned short*)((char*)o.out[k].dst + tail) = *(const unsigned short*)((const char*)o.out[k].src + tail);
+        }
+    }
+}
+
+#if defined(__x86_64__)
+// Pageable memory to the pinned block: streaming stores, so that the lines the GPU is about to read
+// are not first fetched and then left dirty in the cache.
+__attribute__((target("avx2"))) void copy_streaming(void* dst, const void* src, size_t n) {
+    char* d = (char*)dst;
+    const char* s = (const char*)src;
+    size_t i = 0;
+    for (; i + 128 <= n; i += 128) {
+        const __m256i a = _mm256_loadu_si256((const __m256i*)(s + i));
+        const __m256i b = _mm256_loadu_si256((const __m256i*)(s + i + 32));
+        const __m256i c = _mm256_loadu_si256((const __m256i*)(s + i + 64));
+        const __m256i e = _mm256_loadu_si256((const __m256i*)(s + i + 96));
+        _mm256_stream_si256((__m256i*)(d + i), a);
+        _mm256_stream_si256((__m256i*)(d + i + 32), b);
+        _mm256_stream_si256((__m256i*)(d + i + 64), c);
+        _mm256_stream_si256((__m256i*)(d + i + 96), e);
+    }
+    if (i < n) memcpy(d + i, s + i, n - i);
+    _mm_sfence();
+}
+#endif
+
+// largest dec in [0, 31] with a * 2^dec <= 32767; -1 for a <= 0
+int largest_dec(double a) {
+    if (!(a > 0.0)) return -1;
+    if (std::isinf(a)) return 0;
+    int e;
+    (void)std::frexp(a, &e);
+    int dec = 15 - e;
+    if (std::ldexp(a, dec + 1) <= 32767.0) dec += 1;
+    while (std::ldexp(a, dec) > 32767.0) dec -= 1;
+    return dec < 0 ? 0 : dec > 31 ? 31 : dec;
+}
+
+}  // namespace
+
+extern "C" int b2_call_inputs(const b2_call_input* inputs, int32_t n, const b2_call_block* block,
+                              b2_flex_scale* table, int32_t* stats, void* stream) {
+    B2_REQUIRE(n >= 0 && n <= B2_CALL_MAX_INPUTS && (n == 0 || inputs) && block, "bad argument");
+    Inputs a;
+    a.n = n;
+    long long chunks = 0;
+    for (int i = 0; i < n; ++i) {
+        B2_REQUIRE(inputs[i].dst && inputs[i].n >= 0 && (inputs[i].flex_slot < 0 || stats), "bad argument");
+        a.in[i] = inputs[i];
+        a.first_chunk[i] = chunks;
+        chunks += (inputs[i].n + kChunk - 1) / kChunk;
+    }
+    a.first_chunk[n] = chunks;
+    long long grid = chunks < 1 ? 1 : chunks > 148 * 8 ? 148 * 8 : chunks;
+    k_call_inputs<<<(unsigned)grid, kThreads, 0, (cudaStream_t)stream>>>(a, block, table, stats);
+    B2_CUDA(cudaGetLastError());
+    return B2_OK;
+}
+
+extern "C" int b2_call_outputs(const b2_call_output* outputs, int32_t n, int32_t* stats,
+                               int32_t n_stats, const int32_t* status, int32_t* host_stats,
+                               int32_t* host_status, void* stream) {
+    B2_REQUIRE(n >= 0 && n <= B2_CALL_MAX_OUTPUTS && (n == 0 || outputs), "bad argument");
+    B2_REQUIRE(n_stats >= 0 && (n_stats == 0 || (stats && host_stats)), "bad argument");
+    B2_REQUIRE((status == nullptr) == (host_status == nullptr), "status source and destination go together");
+    Outputs o;
+    o.n = n;
+    long long most = 0;
+    for (int i = 0; i < n; ++i) {
+        B2_REQUIRE(outputs[i].src && outputs[i].dst && outputs[i].bytes >= 0 &&
+                   (((uintptr_t)outputs[i].src | (uintptr_t)outputs[i].dst) & 15) == 0,
+                   "results must be 16-byte aligned");
+        o.out[i] = outputs[i];
+        if (outputs[i].bytes > most) most = outputs[i].bytes;
+    }
+    long long grid = n == 0 ? 1 : 1 + (most / 16 + kThreads - 1) / kThreads;
+    if (n && grid < 2) grid = 2;
+    if (grid > 65) grid = 65;
+    k_call_outputs<<<(unsigned)grid, kThreads, 0, (cudaStream_t)stream>>>(o, stats, n_stats, status,
+                                                                          host_stats, host_status);
+    B2_CUDA(cudaGetLastError());
+    return B2_OK;
+}
+
+extern "C" int b2_call_stage(const void* src, size_t bytes, void* pinned, const void** visible) {
+    B2_REQUIRE(src && visible, "null argument");
+    cudaPointerAttributes at;
+    const cudaError_t e = cudaPointerGetAttributes(&at, src);
+    if (e == cudaSuccess && at.type == cudaMemoryTypeHost && at.devicePointer) {
+        *visible = at.devicePointer;              // page-locked: the kernel reads it where it is
+        return B2_OK;
+    }
+    (void)cudaGetLastError();                     // (not a CUDA address: no error of the caller's)
+    B2_REQUIRE(pinned, "pageable memory needs a pinned block to copy to");
+#if defined(__x86_64__)
+    static const bool avx2 = __builtin_cpu_supports("avx2");
+    if (avx2 && ((uintptr_t)pinned & 31) == 0) copy_streaming(pinned, src, bytes);
+    else memcpy(pinned, src, bytes);
+#else
+    memcpy(pinned, src, bytes);
+#endif
+    *visible = pinned;
+    return B2_OK;
+}
+
+extern "C" int b2_flex_begin_call(const b2_flex_state* s, int32_t n, const int64_t* ids,
+                                  const int64_t* slot_write, const int64_t* slot_read,
+                                  int64_t* uploaded, b2_flex_scale* host_table, int32_t* changed) {
+    B2_REQUIRE(s && n >= 0 && (n == 0 || (ids && slot_write && slot_read)) && uploaded && host_table &&
+               changed, "null argument");
+    int ch = 0;
+    auto row = [&](int64_t slot, int64_t dec) {
+        if (uploaded[slot] == dec) return;
+        uploaded[slot] = dec;
+        host_table[slot].scale = std::ldexp(1.0f, (int)-dec);
+        host_table[slot].inv_scale = std::ldexp(1.0f, (int)dec);
+        ch = 1;
+    };
+    for (int32_t k = 0; k < n; ++k) {
+        const int64_t i = ids[k], stored = s->dec[i];
+        if (s->initialized[i] && s->pending[i] >= 0) {
+            s->dec[i] = s->pending[i];
+            s->pending[i] = -1;
+        }
+        row(slot_write[k], s->dec[i]);
+        if (slot_read[k] != slot_write[k]) row(slot_read[k], stored);
+    }
+    *changed = ch;
+    return B2_OK;
+}
+
+extern "C" int b2_flex_end_call(const b2_flex_state* s, int32_t n, const int64_t* ids,
+                                const int64_t* slots, const int32_t* maxima, int32_t* undecided,
+                                int32_t* n_undecided, int32_t* settled) {
+    B2_REQUIRE(s && n >= 0 && (n == 0 || (ids && maxima && undecided)) && n_undecided && settled,
+               "null argument");
+    const int H = B2_FLEX_HISTORY;
+    int open = 0, all = 1;
+    for (int32_t k = 0; k < n; ++k) {
+        const int64_t i = ids[k];
+        const int64_t m = maxima[slots ? slots[k] : k];
+        const double scale = std::ldexp(1.0, (int)-s->dec[i]);
+        auto push = [&](double v) {
+            int64_t& pos = s->hist_pos[i];
+            s->hist[i * H + pos] = v;
+            pos = (pos + 1) % H;
+            if (s->hist_len[i] < H) s->hist_len[i] += 1;
+        };
+        if (m >= 32767) {
+            s->overflows[i] += 1;
+            s->run_length[i] = 0;
+            push(2.0 * (double)m * scale);
+            s->pending[i] = s->dec[i] - 2 < 0 ? 0 : s->dec[i] - 2;
+            all = 0;
+            continue;
+        }
+        const double value = (double)m * scale;
+        if (value == s->run_value[i]) {
+            s->run_length[i] += 1;
+            if (s->run_length[i] > H) {
+                // the window already holds nothing but this value: the same choice as before
+                s->pending[i] = s->run_choice[i];
+                if (s->pending[i] >= 0 && s->pending[i] != s->dec[i]) all = 0;
+                continue;
+            }
+        } else {
+            s->run_value[i] = value;
+            s->run_length[i] = 1;
+        }
+        all = 0;
+        push(value);
+        const double* h = s->hist + i * H;
+        const int len = (int)s->hist_len[i];
+        double sum = 0.0, var = 0.0, top = h[0];
+        for (int j = 0; j < len; ++j) { sum += h[j]; if (h[j] > top) top = h[j]; }
+        const double mean = sum / len;
+        for (int j = 0; j < len; ++j) var += (h[j] - mean) * (h[j] - mean);
+        const double predicted = top + 3.0 * std::sqrt(var / len);
+        const int choice = largest_dec(predicted);
+        // these sums are not the exactly rounded ones of the rule: where the value lies within a
+        // hair of the point at which the choice changes, the caller decides with exact sums
+        if (choice >= 0 && !std::isinf(predicted) &&
+            (std::fabs(std::ldexp(predicted, choice) - 32767.0) < 1e-6 * 32767.0 ||
+             std::fabs(std::ldexp(predicted, choice + 1) - 32767.0) < 1e-6 * 32767.0))
+            undecided[open++] = k;
+        s->pending[i] = choice;
+        s->run_choice[i] = choice;
+    }
+    *n_undecided = open;
+    *settled = all;
+    return B2_OK;
+}

@@ -85,28 +85,8 @@ extern "C" int b2_absmax_bits_f32(const float* src, int64_t n, int32_t* out, voi
     return B2_OK;
 }
 
-// End of a call: the statistics array and the status word go to the host in ONE small kernel that
-// stores them into pinned host memory the device can address (zero-copy), and the statistics are
-// cleared for the next call.  Replaces two device-to-host copies and a memset per call -- inside
-// a replayed CUDA graph those are three more serialised nodes, each with its own latency.
-namespace {
-__global__ void __launch_bounds__(kThreads)
-k_publish(int* __restrict__ stats, int n, const int* __restrict__ status,
-          volatile int* __restrict__ host_stats, volatile int* __restrict__ host_status) {
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        host_stats[i] = stats[i];
-        stats[i] = 0;
-    }
-    if (threadIdx.x == 0 && status && host_status) *host_status = *status;
-    __threadfence_system();
-}
-}  // namespace
-
+// End of a call without results: see b2_call_outputs.
 extern "C" int b2_flex_publish(int32_t* stats, int32_t n, const int32_t* status,
                                int32_t* host_stats, int32_t* host_status, void* stream) {
-    B2_REQUIRE(n >= 0 && (n == 0 || (stats && host_stats)), "bad argument");
-    B2_REQUIRE((status == nullptr) == (host_status == nullptr), "status source and destination go together");
-    k_publish<<<1, kThreads, 0, (cudaStream_t)stream>>>(stats, n, status, host_stats, host_status);
-    B2_CUDA(cudaGetLastError());
-    return B2_OK;
+    return b2_call_outputs(nullptr, 0, stats, n, status, host_stats, host_status, stream);
 }

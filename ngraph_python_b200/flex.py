@@ -90,9 +90,10 @@ _NONE = -1          # "no exponent chosen" in the integer arrays below
 class FlexManager(object):
     """Creates entries, hands out rows of the device scale table / statistics array, and holds
     the exponent state of ALL entries in arrays, so that the bookkeeping of a computation with
-    hundreds of written tensors (a training step) is a handful of numpy operations per call
-    (`begin_write_batch`, `end_write_batch`) instead of a Python loop over entries -- that loop
-    took 1.2 ms per ResNet-20 training step, with the GPU idle.  A FlexEntry is a view on one
+    hundreds of written tensors (a training step) is one native pass before and one after a call
+    (`begin_call`, `end_call`) instead of a Python loop over entries (1.2 ms per ResNet-20 training
+    step, with the GPU idle) or a few dozen numpy operations (0.16 ms even for 24 tensors: their
+    fixed cost).  A FlexEntry is a view on one
     row of these arrays; its own methods apply the same rules one entry at a time (first writes,
     host writes, tests) and the two paths make the same choices."""
 
@@ -108,6 +109,10 @@ class FlexManager(object):
         self.flex_entries = {}
         self.autoflex_count = 0
         self.n_slots = 0
+        import ctypes
+        import numpy as np
+        self._undecided = np.empty((64,), dtype=np.int32)
+        self._n_open, self._settled = ctypes.c_int32(0), ctypes.c_int32(0)
         self._alloc(64)
 
     def _alloc(self, cap):
@@ -130,6 +135,7 @@ class FlexManager(object):
         grow("run_value", np.float64, np.nan)              # nan: no value recorded yet
         grow("run_length", np.int64, 0)
         grow("run_choice", np.int64, _NONE)
+        self._state = None
 
     def make_flex_entry(self, name=""):
         i = len(self.flex_entries)
@@ -176,66 +182,51 @@ class FlexManager(object):
         """FlexEntry.end_write for the entries `ids` (int array, no duplicates) with the max
         |mantissa| each of them recorded."""
         import numpy as np
-        if self.fixed_point or len(ids) == 0:
-            return
-        ids = np.asarray(ids, dtype=np.int64)
-        m = np.asarray(maxima, dtype=np.int64)
-        dec = self.dec[ids]
-        scale = np.ldexp(1.0, (-dec).astype(np.int32))
-        value = m * scale
-        ovf = m >= MANT_MAX
-        if ovf.any():
-            sel = ids[ovf]
-            self.overflows[sel] += 1
-            self.run_length[sel] = 0
-            self._push_many(sel, 2.0 * value[ovf])
-            self.pending[sel] = np.maximum(dec[ovf] - 2, DEC_MIN)
-        ok = ~ovf
-        same = ok & (value == self.run_value[ids])
-        if same.any():
-            self.run_length[ids[same]] += 1
-        # the window already holds nothing but this value: same choice as after the previous write
-        early = same & (self.run_length[ids] > HISTORY_LEN)
-        if early.any():
-            sel = ids[early]
-            self.pending[sel] = self.run_choice[sel]
-        fresh = ok & ~same
-        if fresh.any():
-            sel = ids[fresh]
-            self.run_value[sel] = value[fresh]
-            self.run_length[sel] = 1
-        rest = ok & ~early
-        if not rest.any():
-            return
-        sel = ids[rest]
-        self._push_many(sel, value[rest])
-        H = self.hist[sel]
-        n = self.hist_len[sel]
-        mask = np.arange(HISTORY_LEN)[None, :] < n[:, None]     # rows fill from slot 0
-        mean = H.sum(axis=1) / n                                 # unused slots hold 0
-        d = np.where(mask, H - mean[:, None], 0.0)
-        var = (d * d).sum(axis=1) / n
-        predicted = np.where(mask, H, -np.inf).max(axis=1) + HEADROOM_SIGMAS * np.sqrt(var)
-        choice = _largest_dec_holding_many(predicted)
-        # numpy's sums are not the exactly rounded ones of the one-entry rule: where the value
-        # lies within a hair of the point at which the choice changes, decide with that rule
-        with np.errstate(over="ignore", invalid="ignore"):
-            c = np.where(choice < 0, 0, choice).astype(np.int32)
-            t0 = np.ldexp(predicted, c)
-            t1 = np.ldexp(predicted, c + 1)
-        near = (choice >= 0) & ((np.abs(t0 - MANT_MAX) < 1e-6 * MANT_MAX) |
-                                (np.abs(t1 - MANT_MAX) < 1e-6 * MANT_MAX))
-        for k in np.nonzero(near)[0]:
-            exact = _choose_dec_scalar(self.history_of(int(sel[k])))
-            choice[k] = _NONE if exact is None else exact
-        self.pending[sel] = choice
-        self.run_choice[sel] = choice
+        ids = np.ascontiguousarray(ids, dtype=np.int64)
+        self.end_call(ids, None, np.ascontiguousarray(maxima, dtype=np.int32))
 
-    def _push_many(self, sel, values):
-        pos = self.hist_pos[sel]
-        self.hist[sel, pos] = values
-        self.hist_pos[sel] = (pos + 1) % HISTORY_LEN
-        self.hist_len[sel] = builtin_min_arr(self.hist_len[sel] + 1)
+    def end_call(self, ids, slots, maxima):
+        """end_write of every entry of the int64 array `ids` in one native pass, entry k with
+        maxima[slots[k]] (maxima[k] when slots is None; int32).  True when every entry has seen the
+        same maximum for longer than the history window and will keep its exponent."""
+        import numpy as np
+        from . import lib
+        n = len(ids)
+        if self.fixed_point or n == 0:
+            return True
+        if len(self._undecided) < n:
+            self._undecided = np.empty((2 * n,), dtype=np.int32)
+        state, n_open, settled = self._native_state(), self._n_open, self._settled
+        lib.check(lib.raw().b2_flex_end_call(
+            state, n, ids.ctypes.data, None if slots is None else slots.ctypes.data,
+            maxima.ctypes.data, self._undecided.ctypes.data, n_open, settled))
+        for k in self._undecided[:n_open.value]:
+            # plain sums are not the exactly rounded ones of the one-entry rule: where the value
+            # lies within a hair of the point at which the choice changes, that rule decides
+            i = int(ids[k])
+            exact = _choose_dec_scalar(self.history_of(i))
+            self.pending[i] = self.run_choice[i] = _NONE if exact is None else exact
+        return bool(settled.value)
+
+    def begin_call(self, ids, slots_written, slots_read, uploaded, table):
+        """begin_write of every initialised entry of `ids`, and the rows of the host scale table
+        (float32 [rows][2]) that follow from it, in one native pass.  `uploaded` (int64) holds the
+        exponent each row has.  True when a row changed."""
+        import ctypes
+        from . import lib
+        changed = ctypes.c_int32(0)
+        lib.check(lib.raw().b2_flex_begin_call(
+            self._native_state(), len(ids), ids.ctypes.data, slots_written.ctypes.data,
+            slots_read.ctypes.data, uploaded.ctypes.data, table.ctypes.data, changed))
+        return bool(changed.value)
+
+    def _native_state(self):
+        """The arrays as the native library takes them."""
+        if self._state is None:
+            from . import lib
+            self._state = lib.FlexState(*[getattr(self, n).ctypes.data
+                                          for n, _ in lib.FlexState._fields_])
+        return self._state
 
     def settled(self, ids):
         """True when every one of the entries has seen the same maximum for longer than the
@@ -244,34 +235,6 @@ class FlexManager(object):
             return True
         p, d = self.pending[ids], self.dec[ids]
         return bool(((self.run_length[ids] > HISTORY_LEN) & ((p < 0) | (p == d))).all())
-
-
-def builtin_min_arr(a):
-    import numpy as np
-    return np.minimum(a, HISTORY_LEN)
-
-
-def _largest_dec_holding_many(a):
-    """largest_dec_holding over an array of non-negative finite values; -1 where it gives None."""
-    import numpy as np
-    a = np.asarray(a, dtype=np.float64)
-    out = np.full(a.shape, _NONE, dtype=np.int64)
-    pos = a > 0.0
-    if not pos.any():
-        return out
-    x = a[pos]
-    _, e = np.frexp(x)
-    dec = 15 - e.astype(np.int64)
-    with np.errstate(over="ignore"):
-        up = np.ldexp(x, (dec + 1).astype(np.int32)) <= MANT_MAX
-        dec = np.where(up, dec + 1, dec)
-        for _ in range(2):
-            down = np.ldexp(x, dec.astype(np.int32)) > MANT_MAX
-            dec = np.where(down, dec - 1, dec)
-    dec = np.clip(dec, DEC_MIN, DEC_MAX)
-    dec = np.where(np.isinf(x), DEC_MIN, dec)
-    out[pos] = dec
-    return out
 
 
 class FlexEntry(object):

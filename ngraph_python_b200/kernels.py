@@ -87,6 +87,7 @@ class _PlaneUser(object):
         self.plane_arg = stream_arg          # index of the streamed tensor in op.args / in_views
         self.filter_arg = filter_arg
         self.filter_bytes = filt_bytes
+        self.in_views[filter_arg].buffer.watched = True
         # the input gradient of a strided convolution streams the error tensor with zeros between
         # its elements: planes of its own, written by one extra launch of this step
         self.own_plane_bytes = 0

@@ -69,6 +69,33 @@ class FlexScale(C.Structure):
     _fields_ = [("scale", C.c_float), ("inv_scale", C.c_float)]
 
 
+CALL_MAX_INPUTS, CALL_MAX_OUTPUTS = 16, 16
+
+
+class CallArg(C.Structure):
+    _fields_ = [("src", C.c_void_p), ("inv_scale", C.c_float), ("reserved", C.c_int32)]
+
+
+class CallBlock(C.Structure):
+    _fields_ = [("table", C.c_void_p), ("table_rows", C.c_int32), ("reserved", C.c_int32),
+                ("arg", CallArg * CALL_MAX_INPUTS)]
+
+
+class CallInput(C.Structure):
+    _fields_ = [("dst", C.c_void_p), ("n", C.c_int64), ("flex_slot", C.c_int32),
+                ("reserved", C.c_int32)]
+
+
+class CallOutput(C.Structure):
+    _fields_ = [("src", C.c_void_p), ("dst", C.c_void_p), ("bytes", C.c_int64)]
+
+
+class FlexState(C.Structure):
+    _fields_ = [(n, C.c_void_p) for n in
+                ("dec", "pending", "initialized", "overflows", "hist", "hist_len", "hist_pos",
+                 "run_value", "run_length", "run_choice")]
+
+
 def _load():
     if not os.path.exists(LIB_PATH):
         raise ImportError(
@@ -141,6 +168,13 @@ def _load():
         "b2_flex_dequantize": (C.c_int, [vp, vp, i64, vp, i32, vp]),
         "b2_absmax_bits_f32": (C.c_int, [vp, i64, vp, vp]),
         "b2_flex_publish": (C.c_int, [vp, i32, vp, vp, vp, vp]),
+        "b2_call_inputs": (C.c_int, [C.POINTER(CallInput), i32, vp, vp, vp, vp]),
+        "b2_call_outputs": (C.c_int, [C.POINTER(CallOutput), i32, vp, i32, vp, vp, vp, vp]),
+        "b2_call_stage": (C.c_int, [vp, sz, vp, C.POINTER(vp)]),
+        "b2_flex_begin_call": (C.c_int, [C.POINTER(FlexState), i32, vp, vp, vp, vp, vp,
+                                         C.POINTER(i32)]),
+        "b2_flex_end_call": (C.c_int, [C.POINTER(FlexState), i32, vp, vp, vp, vp, C.POINTER(i32),
+                                       C.POINTER(i32)]),
     }
     for name, (res, args) in sigs.items():
         fn = getattr(lib, name)

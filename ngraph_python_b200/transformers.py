@@ -12,6 +12,7 @@ There is no CPU path: constructing the transformer without the shared library or
 device raises.
 """
 import collections
+import ctypes
 import math
 import numbers
 
@@ -155,6 +156,7 @@ class Computation(object):
         self.steps = None
         self.executor = None
         self.launches_per_call = 0
+        self._io = None             # argument and result handling of the recorded step list
         self._comm_steps = []       # this computation's exchanges, in production order
         self._allreduce = None      # their arena and bucket plan (one per computation)
 
@@ -205,6 +207,8 @@ class Computation(object):
         if len(args) != len(self.parameters):
             raise ValueError("Computation was expecting %d arguments, but was called with %d" %
                              (len(self.parameters), len(args)))
+        if self._io is not None and t.tracer is None and self._io.ready():
+            return self._io.call(args)
         views = [t._view_of(p) for p in self.parameters]
         for v, value in zip(views, args):
             t._stage(v, value)             # the input copies run while the host does the rest
@@ -222,7 +226,9 @@ class Computation(object):
         t._end_call(self)
         if traced is not None:
             t._collect_trace(self, traced)
-        results = [t._finish_host(p) for p in pending]
+        return self._results([t._finish_host(p) for p in pending])
+
+    def _results(self, results):
         if self.returns_kind is Op:
             return results[0]
         if self.returns_kind is None:
@@ -307,12 +313,15 @@ class Computation(object):
             t._allreduce.begin_call()
         t._recording = has_comm          # comm steps and waits: kernels only, no NCCL, no bookkeeping
         io_in_graph = False
+        io = _CallIO.of(self, exchanged_apart=has_comm)
         try:
             for seg in segments:
                 if all(s.launches == 0 for s in seg["steps"]):
                     continue             # nothing to record (fp32 exchange markers)
                 g = torch.cuda.CUDAGraph()
                 with torch.cuda.graph(g):
+                    if io is not None and seg is segments[0]:
+                        io.record_inputs()       # the call's arguments are the first node
                     for s in seg["steps"]:
                         t._launch_step(s)
                     if in_graph:
@@ -321,13 +330,14 @@ class Computation(object):
                         # the call's read-back rides in the graph: status word and flex
                         # statistics to pinned host memory, then the statistics cleared for the
                         # next call -- one graph launch and one synchronisation per call
-                        t._publish()
+                        t._publish(io.outputs if io is not None else ())
                         io_in_graph = True
                 seg["graph"] = g
         finally:
             t._recording = False
         per_call = t.kernel_launches - before
         self._graphs = [seg["graph"] for seg in segments]
+        self._io = io if io_in_graph and segments and segments[0]["graph"] is not None else None
 
         def replay():
             for s in refreshable:
@@ -352,6 +362,133 @@ class Computation(object):
 
 
 builtin_sum = sum
+
+
+# ---------------------------------------------------------------------------------------------
+class _CallIO(object):
+    """Arguments and results of a recorded step list: its first node reads the arguments from
+    wherever they lie and its last one stores small results into pinned memory, so that a call is
+    one graph launch and one synchronisation.  Per argument the host only writes an address into a
+    pinned block; pageable memory is first copied to a pinned buffer."""
+
+    STAGED_MOST = 4 << 20       # pageable arguments up to this size go through a pinned buffer
+    RESULTS_MOST = 1 << 20      # results up to this many bytes are stored by the last node
+
+    @classmethod
+    def of(cls, comp, exchanged_apart):
+        """The handler for `comp`, or None where a call needs more than that (strided arguments,
+        more of them than the kernel takes)."""
+        t = comp.transformer
+        views = [t._view_of(p) for p in comp.parameters]
+        if len(views) > lib.CALL_MAX_INPUTS or not all(v.is_dense() for v in views):
+            return None
+        return cls(comp, views, exchanged_apart)
+
+    def __init__(self, comp, views, exchanged_apart):
+        t = self.t = comp.transformer
+        torch = t.torch
+        self.comp, self.views = comp, views
+        self.lengths = [tuple(v.axes.lengths) for v in views]
+        self.flex_views = [v for v in views if v.buffer.flex]
+        self.block_mem = torch.zeros((ctypes.sizeof(lib.CallBlock),), dtype=torch.uint8).pin_memory()
+        self.block = lib.CallBlock.from_address(self.block_mem.data_ptr())
+        self.table_rows = t._table_host.shape[0] if t.flex else 0
+        if t.flex:
+            self.block.table = t._table_host.data_ptr()
+        self.pinned = [None] * len(views)
+        for k, v in enumerate(views):
+            if 4 * v.buffer.size <= 1 << 20:
+                self._pinned_buffer(k)
+        self.visible = ctypes.c_void_p()
+        # results: small dense ones ride in the last node, the others are copied after it
+        self.outputs, self.later, budget = [], [], self.RESULTS_MOST
+        self.results = []               # (pinned array, view) or None, in the order of the returns
+        for v in comp.return_views:
+            buf = v.buffer
+            n = max(buf.size, 1) * (2 if buf.flex else 4)
+            apart = exchanged_apart and getattr(buf, "comm_key", None) is not None
+            if v.is_dense() and not apart and n <= budget and buf.ptr() % 16 == 0 and \
+                    len(self.outputs) < lib.CALL_MAX_OUTPUTS:
+                budget -= n
+                host = torch.empty((max(buf.size, 1),), dtype=buf.tensor.dtype).pin_memory()
+                self.outputs.append((buf.ptr(), host.data_ptr(), n))
+                self.results.append((host, v))
+            else:
+                self.results.append(None)
+
+    def _pinned_buffer(self, k):
+        if self.pinned[k] is None:
+            n = max(self.views[k].buffer.size, 1)
+            self.pinned[k] = self.t.torch.empty((n,), dtype=self.t.torch.float32).pin_memory()
+        return self.pinned[k].data_ptr()
+
+    def record_inputs(self):
+        t = self.t
+        ins = (lib.CallInput * max(1, len(self.views)))()
+        for k, v in enumerate(self.views):
+            ins[k].dst, ins[k].n = v.buffer.ptr(), v.buffer.size
+            ins[k].flex_slot = v.buffer.slot if v.buffer.flex else -1
+        lib.check(lib.raw().b2_call_inputs(
+            ins, len(self.views), self.block_mem.data_ptr(),
+            t._table.data_ptr() if t.flex else None, t._stats.data_ptr() if t.flex else None,
+            t.stream.cuda_stream))
+        t.kernel_launches += 1
+
+    def ready(self):
+        """False while an argument has no exponent yet: its range has to be measured first."""
+        return all(v.buffer.entry.initialized for v in self.flex_views)
+
+    def _source(self, k, value):
+        """(address the device can read argument k's fp32 values from, object to keep alive);
+        address 0 when the values are already in place."""
+        t, view = self.t, self.views[k]
+        buf = view.buffer
+        torch = t.torch
+        if isinstance(value, torch.Tensor) and value.is_cuda:
+            src = t._device_argument(view, value)
+            if src.device == t.device:
+                return src.data_ptr(), src
+            src = src.to(t.device)
+            return src.data_ptr(), src
+        if type(value) is np.ndarray and value.dtype == np.float32 and \
+                value.shape == self.lengths[k] and value.flags.c_contiguous:
+            arr = value
+        else:
+            arr = t._host_argument(view, value)
+        if arr.nbytes > self.STAGED_MOST and not torch.from_numpy(
+                arr if arr.flags.writeable else arr.copy()).is_pinned():
+            # the driver's own pipelined copy
+            t._stage(view, arr)
+            return (buf.staging.data_ptr() if buf.flex else 0), arr
+        lib.check(lib.raw().b2_call_stage(
+            arr.__array_interface__["data"][0], arr.nbytes,
+            self._pinned_buffer(k) if arr.nbytes <= self.STAGED_MOST else None, self.visible))
+        return self.visible.value, arr
+
+    def call(self, args):
+        t, comp, block = self.t, self.comp, self.block
+        keep = []
+        try:
+            for k, value in enumerate(args):
+                self.views[k].buffer.version += 1
+                address, obj = self._source(k, value)
+                block.arg[k].src = address
+                keep.append(obj)
+            t._begin_call(comp, self)
+            for k, v in enumerate(self.views):
+                if v.buffer.flex:
+                    block.arg[k].inv_scale = math.ldexp(1.0, v.buffer.entry.dec)
+                    t._inputs_written.append(v.buffer)
+            comp.executor()
+            pending = [None if r is not None else t._device_to_host_async(v)
+                       for r, v in zip(self.results, comp.return_views)]
+            t._end_call(comp)
+        finally:
+            for k in range(len(args)):
+                block.arg[k].src = None
+            block.table_rows = 0
+        return comp._results([t._finish_host(p or r)
+                              for p, r in zip(pending, self.results)])
 
 
 # ---------------------------------------------------------------------------------------------
@@ -1613,13 +1750,7 @@ class B200Transformer(object):
         if not view.is_dense():
             raise ValueError("host writes need a dense tensor")
         if isinstance(value, torch.Tensor) and value.is_cuda:
-            # a tensor that already lives on the device (the reference's DeviceTensor.__setitem__
-            # takes a GPUArray the same way, gputransform.py:806-854): device-to-device copy
-            if tuple(value.shape) != tuple(view.axes.lengths) and \
-                    tuple(value.shape) != (buf.size,):
-                raise ValueError("value shape %s does not match tensor axes %s"
-                                 % (tuple(value.shape), view.axes))
-            src = value.to(torch.float32).reshape(-1)
+            src = self._device_argument(view, value)
             if not buf.flex:
                 buf.tensor.copy_(src, non_blocking=True)
                 return
@@ -1628,17 +1759,7 @@ class B200Transformer(object):
                                           device=self.device)
             buf.staging.copy_(src, non_blocking=True)
             return
-        arr = np.asarray(value, dtype=np.float32)
-        # a scalar broadcasts; otherwise the shape must be the tensor's, or flat with its size
-        # (a transposed or otherwise differently shaped array of the right size is an error, as
-        # it is for the reference's DeviceTensor.__setitem__)
-        if arr.shape not in ((), tuple(view.axes.lengths), (buf.size,)):
-            squeezed = tuple(n for n in arr.shape if n != 1)
-            if squeezed != tuple(n for n in view.axes.lengths if n != 1):
-                raise ValueError("value shape %s does not match tensor axes %s"
-                                 % (arr.shape, view.axes))
-        arr = np.ascontiguousarray(np.broadcast_to(arr, view.axes.lengths)
-                                   if arr.shape == () else arr.reshape(view.axes.lengths))
+        arr = self._host_argument(view, value)
         src = torch.from_numpy(np.array(arr.reshape(-1), copy=not arr.flags.writeable))
         async_ok = src.is_pinned()
         if not buf.flex:
@@ -1647,6 +1768,28 @@ class B200Transformer(object):
         if buf.staging is None:
             buf.staging = torch.empty((max(buf.size, 1),), dtype=torch.float32, device=self.device)
         buf.staging.copy_(src, non_blocking=async_ok)
+
+    def _device_argument(self, view, value):
+        """A tensor that already lives on the device (the reference's DeviceTensor.__setitem__
+        takes a GPUArray the same way, gputransform.py:806-854), as flat fp32."""
+        if tuple(value.shape) != tuple(view.axes.lengths) and tuple(value.shape) != (view.buffer.size,):
+            raise ValueError("value shape %s does not match tensor axes %s"
+                             % (tuple(value.shape), view.axes))
+        return value.to(self.torch.float32).reshape(-1)
+
+    def _host_argument(self, view, value):
+        """A host value as a contiguous fp32 array of the view's shape.  A scalar broadcasts;
+        otherwise the shape must be the tensor's, or flat with its size (a transposed or otherwise
+        differently shaped array of the right size is an error, as it is for the reference's
+        DeviceTensor.__setitem__)."""
+        arr = np.asarray(value, dtype=np.float32)
+        if arr.shape not in ((), tuple(view.axes.lengths), (view.buffer.size,)):
+            squeezed = tuple(n for n in arr.shape if n != 1)
+            if squeezed != tuple(n for n in view.axes.lengths if n != 1):
+                raise ValueError("value shape %s does not match tensor axes %s"
+                                 % (arr.shape, view.axes))
+        return np.ascontiguousarray(np.broadcast_to(arr, view.axes.lengths)
+                                    if arr.shape == () else arr.reshape(view.axes.lengths))
 
     def _host_to_device(self, view, value, init=False, in_call=False, staged=False):
         """DeviceTensor.__setitem__ (ngraph/transformers/gputransform.py:806-854); flex:
@@ -1835,26 +1978,17 @@ class B200Transformer(object):
             self._table_np[slot, 1] = math.ldexp(1.0, dec)
             self._table_dirty = True
 
-    def _set_table_rows_host(self, slots, decs):
-        """_set_table_row_host for arrays of rows and exponents."""
-        changed = self._dec_uploaded[slots] != decs
-        if changed.any():
-            rows, d = slots[changed], decs[changed]
-            self._flex_epoch += 1
-            self._dec_uploaded[rows] = d
-            self._table_np[rows, 0] = np.ldexp(1.0, (-d).astype(np.int32))
-            self._table_np[rows, 1] = np.ldexp(1.0, d.astype(np.int32))
-            self._table_dirty = True
-
-    def _begin_call(self, comp):
+    def _begin_call(self, comp, io=None):
+        """io: the recorded step list's argument handling; its first node then uploads the scale
+        table."""
         self._ensure_scratch()
         self._allreduce = comp._allreduce
         if self._allreduce is not None:
             self._allreduce.begin_call()
         if self.flex:
-            self._begin_call_flex(comp)
+            self._begin_call_flex(comp, io)
 
-    def _begin_call_flex(self, comp):
+    def _begin_call_flex(self, comp, io=None):
         """Exponent bookkeeping before a call (manage_before_computation of every tensor the call
         writes, flexgputransform.py:347-358): host work only, plus the upload of the scale table
         when a row changed."""
@@ -1892,34 +2026,32 @@ class B200Transformer(object):
                           np.array([b.slot_write for b in bufs], dtype=np.int64),
                           np.array([b.slot for b in bufs], dtype=np.int64))
                 comp._flex_buf_arrays = arrays
-            ids, slot_w, slot_r = arrays
-            fm = self.flex_manager
-            dec_stored = fm.dec[ids].copy()
             # tensors this call overwrites adopt the exponent chosen after their previous write
-            dec_w = dec_stored.copy()
-            init = fm.initialized[ids]
-            if init.any():
-                dec_w[init] = fm.begin_write_batch(ids[init])
-            self._set_table_rows_host(slot_w, dec_w)
-            two = slot_r != slot_w
-            if two.any():
-                self._set_table_rows_host(slot_r[two], dec_stored[two])
+            if self.flex_manager.begin_call(arrays[0], arrays[1], arrays[2], self._dec_uploaded,
+                                            self._table_np):
+                self._flex_epoch += 1
+                self._table_dirty = True
         if self._table_dirty:
-            self._table.copy_(self._table_host, non_blocking=True)
+            if io is not None:
+                io.block.table_rows = io.table_rows
+            else:
+                self._table.copy_(self._table_host, non_blocking=True)
             self._table_dirty = False
         if self._stats_clean:
             self._stats_clean = False
         else:
             self._stats.zero_()
 
-    def _publish(self):
-        """Status word and flex statistics into pinned host memory, statistics cleared: one
-        small launch (lib: b2_flex_publish)."""
+    def _publish(self, outputs=()):
+        """Status word, flex statistics and small results into pinned host memory, statistics
+        cleared: one small launch (lib: b2_call_outputs).  outputs: (device address, pinned
+        address, bytes)."""
         n = self._stats.numel() if self.flex else 0
-        lib.check(lib.raw().b2_flex_publish(
-            self._stats.data_ptr() if self.flex else None, n, self._status.data_ptr(),
-            self._stats_host.data_ptr() if self.flex else None, self._status_host.data_ptr(),
-            self.stream.cuda_stream))
+        outs = (lib.CallOutput * max(1, len(outputs)))(*[lib.CallOutput(*o) for o in outputs])
+        lib.check(lib.raw().b2_call_outputs(
+            outs, len(outputs), self._stats.data_ptr() if self.flex else None, n,
+            self._status.data_ptr(), self._stats_host.data_ptr() if self.flex else None,
+            self._status_host.data_ptr(), self.stream.cuda_stream))
         self.kernel_launches += 1
 
     def _end_call(self, comp):
@@ -1936,9 +2068,14 @@ class B200Transformer(object):
         torch.cuda.current_stream(self.device).synchronize()
         if exchanging:
             self._allreduce.after_sync()
-        for b in comp.written:
+        watched = getattr(comp, "_watched", None)
+        if watched is None:
+            # (the tensors whose changes somebody follows: convolution filters with cached planes)
+            watched = comp._watched = [b for b in comp.written if getattr(b, "watched", False)]
+            self._status_np = self._status_host.numpy()
+        for b in watched:
             b.version += 1
-        if int(self._status_host[0]) != 0:
+        if self._status_np[0] != 0:
             self._status.zero_()
             raise lib.B200Error("a device-side wait ran out during the computation")
         if self.flex:
@@ -1966,12 +2103,13 @@ class B200Transformer(object):
             comp._flex_written_arrays = arrays
         ids, slots, distinct = arrays
         if distinct:
-            fm.end_write_batch(ids, stats[slots])      # all written tensors in a few array ops
+            settled = fm.end_call(ids, slots, stats)   # all written tensors in one native pass
         else:
             for b in comp.written:                     # an entry written twice: one at a time
                 b.entry.end_write(int(stats[b.slot_write]))
+            settled = fm.settled(ids)
         in_ids = np.array([b.entry.i for b in self._inputs_written], dtype=np.int64)
-        if fm.settled(ids) and fm.settled(in_ids):
+        if settled and fm.settled(in_ids):
             idx = np.concatenate([np.array([b.slot for b in self._inputs_written], dtype=np.int64),
                                   slots])
             comp._steady = (self._flex_epoch, idx, stats[idx].copy(), len(self._inputs_written))
