@@ -243,6 +243,10 @@ int b2_flex_end_call(const b2_flex_state* s, int32_t n, const int64_t* ids, cons
  * the K-major operand planes the kernel streams with TMA.
  * ------------------------------------------------------------------------------------------ */
 int b2_gemm_scratch_bytes(int32_t flex, int32_t M, int32_t N, int32_t K, size_t* bytes);
+/* Kernels one product launches: 1 where its operands are converted on the way in, else the operand
+ * planes and the tile kernel (K strides as below). */
+int b2_gemm_launches(int32_t flex, int64_t a_k_stride, int64_t b_k_stride, int32_t M, int32_t N,
+                     int32_t K, int32_t* launches);
 /* fp32 via 3xTF32 (relative error ~2^-21). */
 int b2_gemm_f32(const float* A, int64_t a_row_stride, int64_t a_k_stride, const float* B,
                 int64_t b_k_stride, int64_t b_col_stride, float* C, int64_t ldc, int32_t M,

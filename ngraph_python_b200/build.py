@@ -7,7 +7,8 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libb200ng.so")
 
-SOURCES = ["b2_api.cu", "b2_ew_codegen.cu", "b2_flex.cu", "b2_call.cu", "b2_gemm.cu", "b2_conv.cu",
+SOURCES = ["b2_api.cu", "b2_ew_codegen.cu", "b2_flex.cu", "b2_call.cu", "b2_direct.cu", "b2_direct_flex.cu",
+           "b2_gemm.cu", "b2_conv.cu",
            "b2_dimshuffle.cu", "b2_rng.cu", "b2_comm.cu"]
 
 
@@ -38,7 +39,7 @@ def build(force=False, verbose=False):
     if not force and not _stale():
         return LIB
     nvcc = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
-    cmd = [nvcc, "-shared", "-Xcompiler", "-fPIC", "-O3", "-std=c++17", "-lineinfo",
+    cmd = [nvcc, "-shared", "--threads", "0", "-Xcompiler", "-fPIC", "-O3", "-std=c++17", "-lineinfo",
            "-gencode", "arch=compute_100a,code=sm_100a", "-fmad=false",
            "-o", LIB] + [os.path.join(CSRC, s) for s in SOURCES] + ["-ldl"]
     if verbose:

@@ -286,14 +286,6 @@ __device__ __forceinline__ unsigned tmem_ld1(unsigned taddr) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(r) : "r"(taddr) : "memory");
     return r;
 }
-// 8 consecutive 32-bit columns of this thread's TMEM lane
-__device__ __forceinline__ void tmem_ld8(unsigned taddr, unsigned* r) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-          "=r"(r[7])
-        : "r"(taddr) : "memory");
-}
 __device__ __forceinline__ void prefetch_map(const CUtensorMap* m) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(m) : "memory");
 }
@@ -348,10 +340,6 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap mapI0,
     const int warp = warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
     const int epi_w = p.nbuf == 3 ? 1 : 4 / p.nbuf;   // epilogue warps per lane quarter and accumulator set
 
-    // Programmatic dependent launch: the next kernel of the stream, if it was launched the same
-    // way, may take the SMs this grid leaves while its last CTAs still work, and do its set-up;
-    // it reads and writes global memory only after its own griddepcontrol.wait below.
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (threadIdx.x == 0) {
         prefetch_map(&mapI0); prefetch_map(&mapI1); prefetch_map(&mapB);
         for (int s = 0; s < kConvMaxStages; ++s) {
@@ -366,7 +354,14 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap mapI0,
         *fail_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 1) tmem_alloc(tmem_holder, p.tmem_cols);
+    if (warp == 1) {
+        tmem_alloc(tmem_holder, p.tmem_cols);
+        // Programmatic dependent launch: the next kernel of the stream, if it was launched the same
+        // way, may take the SMs this grid leaves while its last CTAs still work, and do its set-up;
+        // it reads and writes global memory only after its own griddepcontrol.wait below.  (Not
+        // before this CTA holds its tensor memory, or the two could each wait for what the other has.)
+        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    }
     // everything before this line touches no global memory; everything after it sees the
     // completed work of all earlier kernels of the stream
     asm volatile("griddepcontrol.wait;" ::: "memory");

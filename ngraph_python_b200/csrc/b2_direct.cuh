@@ -1,0 +1,706 @@
+// Tensor-core product with the operands converted on the way in: C[M,N] = A[M,K] * B[N,K]^T in one
+// launch, for problems where the pre-pass of the plane kernel (b2_gemm_impl.cuh) and its launches
+// cost as much as the product, and for convolutions that would otherwise be unrolled in memory.
+//
+// One CTA per 128 x BN tile (times a slice of K), 288 threads:
+//   warps 0-7: producers -- load a k-block of both operands from wherever it lies (K contiguous,
+//              rows contiguous, or rows gathered from a C,H,W,N tensor through a table of column
+//              offsets), split it into its two planes and store them K-major, 128-byte swizzled,
+//              into a ring of stages; afterwards the epilogue;
+//   warp 8:    tensor memory, tcgen05.mma issue.
+// A k-block is 128 bytes of plane: 32 fp32 or 128 int16 values.
+//   fp32:   3xTF32.  B's planes lie behind one another and make one operand of 2*BN rows:
+//           A_hi x [B_hi | B_lo] -> [hh | x], A_lo x B_hi -> x.  The two sums are kept apart until the
+//           end; a chain runs over at most 16 k-blocks (the tensor core's fp32 sum truncates), longer
+//           K is cut into slices.
+//   flex16: four exact int8 products, HH | X | LL as in b2_gemm_impl.cuh.
+// Slices of K: the CTAs of a cluster (up to 8) take one each; partial sums meet in distributed shared
+// memory, every CTA adds a share of the columns in slice order (deterministic, fp32 adds rounded to
+// nearest, flex16 exact in int64) and finishes them.
+//
+// What bounds it: at the sizes it is chosen for, latency -- launch, first loads, one pass through the
+// ring, the exchange in the cluster -- so the split is taken to give every SM a CTA; for unrolled
+// convolutions the producers' issue slots.
+#ifndef B2_DIRECT_CUH
+#define B2_DIRECT_CUH
+#include "b2_direct.h"
+#include "b2_gemm_impl.cuh"
+
+namespace {
+
+constexpr int kDirThreads = 288;
+constexpr int kDirMaxK = 4608;            // columns of the gather table
+__host__ __device__ constexpr int dir_stages(int bn) { return bn == 128 ? 3 : 2; }
+__host__ __device__ constexpr int dir_stage_bytes(int bn) { return 2 * (128 + bn) * 128; }
+__host__ __device__ constexpr int dir_ring_bytes(int bn) { return dir_stages(bn) * dir_stage_bytes(bn); }
+__host__ __device__ constexpr int dir_tmem_cols(int mode, int bn) {
+    int need = (mode == MODE_FLEX16 ? 3 : 2) * bn, c = 32;
+    while (c < need) c *= 2;
+    return c;
+}
+
+struct DirectParams {
+    b2_direct_args a;
+    int num_kb, kb_per_split, splits;
+    int a_vec, b_vec;                     // 16-byte loads (K contiguous) / row pairs (flex16, others)
+};
+
+__device__ __forceinline__ void dir_split_tf32(float a, float& hi, float& lo) {
+    unsigned hb;
+    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(hb) : "f"(a));
+    hi = __uint_as_float(hb);
+    lo = a - hi;
+}
+__device__ __forceinline__ unsigned swz(int row, int chunk) {
+    return (unsigned)(row * 128 + ((chunk ^ (row & 7)) << 4));
+}
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ unsigned peer_addr(const void* p, int rank) {
+    unsigned r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_u32(p)), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ long long ld_peer(unsigned a, long long) {
+    long long v;
+    asm volatile("ld.shared::cluster.b64 %0, [%1];" : "=l"(v) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ float ld_peer(unsigned a, float) {
+    float v;
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+    return v;
+}
+
+// ---- operand tiles ---------------------------------------------------------------------------
+// Registers of one thread's share of an operand's k-block, loaded in one go so that all loads are
+// in flight together, and stored a k-block later.
+//
+// fp32, K contiguous: unit = 4 rows x 8 chunks of 16 bytes, a lane holds one chunk; else unit = 32 rows
+// x 1 chunk, a lane holds four columns of its row.  flex16: the same with 16 columns to a chunk; with
+// rows contiguous a lane takes two neighbouring rows (one 4-byte load brings both).
+template <int MODE, int ROWS>
+struct OperandTile {
+    static constexpr int kUnits = MODE == MODE_FLEX16 ? (ROWS >= 64 ? ROWS / 64 : 1) : (ROWS >= 32 ? ROWS / 32 : 1);
+    static constexpr int kRegs = MODE == MODE_FLEX16 ? 16 * kUnits : 4 * kUnits;
+    static constexpr int kKUnits = ROWS / 4 >= 8 ? ROWS / 32 : 1;      // units per warp, K contiguous
+    unsigned r[kRegs];
+
+    // -- K contiguous
+    __device__ __forceinline__ void load_k(const void* src, long long rs, int row0, int rows, int K,
+                                           int k0, int vec, int warp, int lane) {
+        const int chunk = lane & 7;
+        constexpr int per = MODE == MODE_FLEX16 ? 16 : 4, regs = MODE == MODE_FLEX16 ? 8 : 4;
+#pragma unroll
+        for (int i = 0; i < kKUnits; ++i) {
+            const int lr = (warp + 8 * i) * 4 + (lane >> 3), row = row0 + lr, k = k0 + chunk * per;
+#pragma unroll
+            for (int j = 0; j < regs; ++j) r[regs * i + j] = 0;
+            if (lr >= ROWS || row >= rows || k >= K) continue;
+            if (MODE == MODE_FLEX16) {
+                const short* p = (const short*)src + (long long)row * rs + k;
+                if (vec && k + 16 <= K) {
+                    const uint4 a = __ldg((const uint4*)p), b = __ldg((const uint4*)p + 1);
+                    r[8 * i + 0] = a.x; r[8 * i + 1] = a.y; r[8 * i + 2] = a.z; r[8 * i + 3] = a.w;
+                    r[8 * i + 4] = b.x; r[8 * i + 5] = b.y; r[8 * i + 6] = b.z; r[8 * i + 7] = b.w;
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 16; ++j)
+                        if (k + j < K) r[8 * i + (j >> 1)] |= (unsigned)(unsigned short)p[j] << ((j & 1) * 16);
+                }
+            } else {
+                const float* p = (const float*)src + (long long)row * rs + k;
+                if (vec && k + 4 <= K) {
+                    const float4 v = __ldg((const float4*)p);
+                    r[4 * i + 0] = __float_as_uint(v.x); r[4 * i + 1] = __float_as_uint(v.y);
+                    r[4 * i + 2] = __float_as_uint(v.z); r[4 * i + 3] = __float_as_uint(v.w);
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        if (k + j < K) r[4 * i + j] = __float_as_uint(p[j]);
+                }
+            }
+        }
+    }
+    __device__ __forceinline__ void store_k(unsigned char* p0, unsigned char* p1, int warp, int lane) const {
+        const int chunk = lane & 7;
+#pragma unroll
+        for (int i = 0; i < kKUnits; ++i) {
+            const int lr = (warp + 8 * i) * 4 + (lane >> 3);
+            if (lr >= ROWS) continue;
+            const unsigned at = swz(lr, chunk);
+            if (MODE == MODE_FLEX16) {
+                const unsigned* w = r + 8 * i;
+                uint4 h, l;
+                h.x = __byte_perm(w[0], w[1], 0x7531); l.x = __byte_perm(w[0], w[1], 0x6420);
+                h.y = __byte_perm(w[2], w[3], 0x7531); l.y = __byte_perm(w[2], w[3], 0x6420);
+                h.z = __byte_perm(w[4], w[5], 0x7531); l.z = __byte_perm(w[4], w[5], 0x6420);
+                h.w = __byte_perm(w[6], w[7], 0x7531); l.w = __byte_perm(w[6], w[7], 0x6420);
+                *(uint4*)(p0 + at) = h;
+                *(uint4*)(p1 + at) = l;
+            } else {
+                store_f4(p0, p1, at, r + 4 * i);
+            }
+        }
+    }
+    __device__ __forceinline__ static void store_f4(unsigned char* p0, unsigned char* p1, unsigned at,
+                                                    const unsigned* v) {
+        float4 h, l;
+        dir_split_tf32(__uint_as_float(v[0]), h.x, l.x); dir_split_tf32(__uint_as_float(v[1]), h.y, l.y);
+        dir_split_tf32(__uint_as_float(v[2]), h.z, l.z); dir_split_tf32(__uint_as_float(v[3]), h.w, l.w);
+        *(float4*)(p0 + at) = h;
+        *(float4*)(p1 + at) = l;
+    }
+    // rows of this lane in a group of 32 (fp32) or 64 (flex16): a pair of rows for flex16.  Four
+    // lanes of eight start with the odd row, which keeps the 16-byte stores of a phase apart.
+    __device__ __forceinline__ static void store_pair(unsigned char* p0, unsigned char* p1, int lr, int chunk,
+                                                      int lane, const unsigned* w) {
+        uint4 h[2], l[2];
+        unsigned* hp[2] = {(unsigned*)&h[0], (unsigned*)&h[1]};
+        unsigned* lp[2] = {(unsigned*)&l[0], (unsigned*)&l[1]};
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            // words hold (row | next row << 16) of four columns
+            const unsigned a = __byte_perm(w[4 * q], w[4 * q + 1], 0x5140), b = __byte_perm(w[4 * q + 2], w[4 * q + 3], 0x5140);
+            const unsigned c = __byte_perm(w[4 * q], w[4 * q + 1], 0x7362), d = __byte_perm(w[4 * q + 2], w[4 * q + 3], 0x7362);
+            lp[0][q] = __byte_perm(a, b, 0x5410); hp[0][q] = __byte_perm(a, b, 0x7632);
+            lp[1][q] = __byte_perm(c, d, 0x5410); hp[1][q] = __byte_perm(c, d, 0x7632);
+        }
+        const bool odd = (lane >> 2) & 1;
+        const unsigned at0 = swz(lr + (odd ? 1 : 0), chunk), at1 = swz(lr + (odd ? 0 : 1), chunk);
+        *(uint4*)(p0 + at0) = odd ? h[1] : h[0];
+        *(uint4*)(p0 + at1) = odd ? h[0] : h[1];
+        *(uint4*)(p1 + at0) = odd ? l[1] : l[0];
+        *(uint4*)(p1 + at1) = odd ? l[0] : l[1];
+    }
+};
+
+template <int MODE, int BN, int AK>
+__global__ void __launch_bounds__(kDirThreads, (BN == 128 ? 1 : 2))
+direct_kernel(const __grid_constant__ DirectParams p) {
+    extern __shared__ unsigned char smem_raw[];
+    unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    constexpr int NST = dir_stages(BN), STAGE = dir_stage_bytes(BN);
+    constexpr int KB = MODE == MODE_FLEX16 ? 128 : 32;            // columns of a k-block
+    constexpr int PER = KB / 8;                                   // columns of a 16-byte chunk
+    constexpr int kCols = dir_tmem_cols(MODE, BN);
+    typedef OperandTile<MODE, 128> ATile;
+    typedef OperandTile<MODE, BN> BTile;
+    unsigned long long* full_bar = (unsigned long long*)(smem + NST * STAGE);     // [NST]
+    unsigned long long* empty_bar = full_bar + NST;                               // [NST]
+    unsigned long long* tmem_full = empty_bar + NST;
+    unsigned* tmem_holder = (unsigned*)(tmem_full + 1);
+    int* fail_flag = (int*)(tmem_holder + 1);
+    int2* tab = (int2*)((unsigned char*)full_bar + 128);                          // [K of the slice] gather table
+
+    const int warp = warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
+    const b2_direct_args& a = p.a;
+    const int m0 = blockIdx.y * 128, n0 = blockIdx.x * BN;
+    const int rank = blockIdx.z, kb0 = rank * p.kb_per_split;
+    const int nkb = min(p.kb_per_split, p.num_kb - kb0);
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < NST; ++s) { mbar_init(&full_bar[s], 8); mbar_init(&empty_bar[s], 1); }
+        mbar_init(tmem_full, 1);
+        *fail_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 8) {
+        tmem_alloc(tmem_holder, kCols);
+        // the next kernel may start its set-up now: not before this CTA holds its tensor memory, or
+        // the two could each wait for what the other has
+        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    }
+    if (AK == B2_OPERAND_GATHER) {
+        // offset and tap of every column of this slice
+        const b2_gather& g = a.g;
+        const int RS = g.R * g.S;
+        for (int i = threadIdx.x; i < nkb * KB; i += kDirThreads) {
+            const int k = kb0 * KB + i;
+            int2 e = make_int2(0, 31);
+            if (k < a.K) {
+                const int c = g.bprop ? k % g.channels : k / RS, rs = g.bprop ? k / g.channels : k % RS;
+                const int r = rs / g.S, s = rs - r * g.S;
+                const int dh = g.bprop ? -(r * g.dil_h / g.str_h) : r * g.dil_h;
+                const int dw = g.bprop ? -(s * g.dil_w / g.str_w) : s * g.dil_w;
+                e = make_int2(((c * g.H + dh) * g.W + dw) * g.N, rs);
+            }
+            tab[i] = e;
+        }
+    }
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const unsigned tmem_base = (unsigned)warp_uniform((int)*tmem_holder);
+
+    if (warp < 8) {
+        // ---- producers
+        // fp32 loads a k-block ahead; a flex16 k-block is 128 columns, few of them make a problem, and a
+        // second set of registers would spill
+        constexpr bool AHEAD = MODE != MODE_FLEX16;
+        ATile ta[AHEAD ? 2 : 1];
+        BTile tb[AHEAD ? 2 : 1];
+        // gathered rows: fixed for the whole CTA.  fp32: one row of a group of 32; flex16: two of 64.
+        constexpr int GR = MODE == MODE_FLEX16 ? 2 : 1;
+        const int a_lr = MODE == MODE_FLEX16 ? (warp & 1) * 64 + 2 * lane : (warp & 3) * 32 + lane;
+        const int a_c0 = MODE == MODE_FLEX16 ? warp >> 1 : warp >> 2;              // first chunk
+        constexpr int a_cs = MODE == MODE_FLEX16 ? 4 : 2;                          // chunk step
+        constexpr int A_UNITS = 8 / a_cs;                                          // 2 or 4
+        const void* a_row[GR];
+        unsigned mask[GR];                                                         // bit t: tap t inside
+        bool pair = GR == 2 && p.a_vec;
+        if (AK != B2_OPERAND_K) {
+#pragma unroll
+            for (int e = 0; e < GR; ++e) {
+                const int row = m0 + a_lr + e;
+                mask[e] = 0;
+                long long base = row;
+                if (AK == B2_OPERAND_GATHER) {
+                    const b2_gather& g = a.g;
+                    base = 0;
+                    if (row < a.M) {
+                        const int n = row % g.N, pq = row / g.N, q = pq % g.Q, pp = pq / g.Q;
+                        int h0, w0;
+                        if (g.bprop) {
+                            const int th = pp + g.pad_h, tw = q + g.pad_w;
+                            h0 = th / g.str_h; w0 = tw / g.str_w;
+                            for (int t = 0; t < g.R * g.S; ++t) {
+                                const int r = t / g.S * g.dil_h, s = t % g.S * g.dil_w;
+                                const int hh = h0 - r / g.str_h, ww = w0 - s / g.str_w;
+                                if (th >= r && tw >= s && (th - r) % g.str_h == 0 && (tw - s) % g.str_w == 0 &&
+                                    hh < g.H && ww < g.W)
+                                    mask[e] |= 1u << t;
+                            }
+                        } else {
+                            h0 = pp * g.str_h - g.pad_h; w0 = q * g.str_w - g.pad_w;
+                            for (int t = 0; t < g.R * g.S; ++t) {
+                                const int hh = h0 + t / g.S * g.dil_h, ww = w0 + t % g.S * g.dil_w;
+                                if (hh >= 0 && hh < g.H && ww >= 0 && ww < g.W) mask[e] |= 1u << t;
+                            }
+                        }
+                        base = ((long long)h0 * g.W + w0) * g.N + n;
+                    }
+                } else if (row < a.M) {
+                    mask[e] = 1u;
+                }
+                a_row[e] = (const char*)a.A + base * (MODE == MODE_FLEX16 ? 2 : 4);
+            }
+            if (GR == 2) pair = pair && (mask[GR - 1] == mask[0]) && m0 + a_lr + 1 < a.M;
+        }
+        auto load = [&](int kb, ATile& A, BTile& B) {
+            const int kt = kb * KB, k0 = kb0 * KB + kt;
+            if (AK == B2_OPERAND_K) {
+                A.load_k(a.A, a.a_rs, m0, a.M, a.K, k0, p.a_vec, warp, lane);
+            } else {
+#pragma unroll
+                for (int i = 0; i < A_UNITS; ++i) {
+                    const int kc = (a_c0 + a_cs * i) * PER;
+#pragma unroll
+                    for (int j = 0; j < PER; ++j) {
+                        unsigned v = 0;
+                        long long o;
+                        bool in0, in1 = false;
+                        if (AK == B2_OPERAND_GATHER) {
+                            const int2 t = tab[kt + kc + j];
+                            o = t.x;
+                            in0 = (mask[0] >> t.y) & 1u;
+                            if (GR == 2) in1 = (mask[GR - 1] >> t.y) & 1u;
+                            if (k0 + kc + j >= a.K) in0 = in1 = false;
+                        } else {
+                            o = (long long)(k0 + kc + j) * a.a_ks;
+                            in0 = mask[0] && k0 + kc + j < a.K;
+                            if (GR == 2) in1 = mask[GR - 1] && k0 + kc + j < a.K;
+                        }
+                        if (MODE == MODE_FLEX16) {
+                            if (pair) {
+                                if (in0) v = __ldg((const unsigned*)((const short*)a_row[0] + o));
+                            } else {
+                                if (in0) v = __ldg((const unsigned short*)a_row[0] + o);
+                                if (in1) v |= (unsigned)__ldg((const unsigned short*)a_row[GR - 1] + o) << 16;
+                            }
+                        } else if (in0) {
+                            v = __float_as_uint(__ldg((const float*)a_row[0] + o));
+                        }
+                        A.r[PER * i + j] = v;
+                    }
+                }
+            }
+            if (a.b_kind == B2_OPERAND_K) {
+                B.load_k(a.B, a.b_rs, n0, a.N, a.K, k0, p.b_vec, warp, lane);
+            } else {
+                // chunk = warp, groups of 32 (64) rows
+#pragma unroll
+                for (int i = 0; i < BTile::kUnits; ++i) {
+                    const int lr = MODE == MODE_FLEX16 ? i * 64 + 2 * lane : i * 32 + lane, row = n0 + lr;
+                    const bool in0 = lr < BN && row < a.N, in1 = lr + 1 < BN && row + 1 < a.N;
+#pragma unroll
+                    for (int j = 0; j < PER; ++j) {
+                        const int k = k0 + warp * PER + j;
+                        unsigned v = 0;
+                        if (k < a.K) {
+                            if (MODE == MODE_FLEX16) {
+                                const unsigned short* s = (const unsigned short*)a.B + row + (long long)k * a.b_ks;
+                                if (p.b_vec && in1) v = __ldg((const unsigned*)s);
+                                else {
+                                    if (in0) v = __ldg(s);
+                                    if (in1) v |= (unsigned)__ldg(s + 1) << 16;
+                                }
+                            } else if (in0) {
+                                v = __float_as_uint(__ldg((const float*)a.B + row + (long long)k * a.b_ks));
+                            }
+                        }
+                        B.r[PER * i + j] = v;
+                    }
+                }
+            }
+        };
+        auto store = [&](int s, const ATile& A, const BTile& B) {
+            unsigned char* st = smem + s * STAGE;
+            unsigned char* b0 = st + 2 * 128 * 128;
+            if (AK == B2_OPERAND_K) {
+                A.store_k(st, st + 128 * 128, warp, lane);
+            } else {
+#pragma unroll
+                for (int i = 0; i < A_UNITS; ++i) {
+                    if (MODE == MODE_FLEX16)
+                        ATile::store_pair(st, st + 128 * 128, a_lr, a_c0 + a_cs * i, lane, A.r + PER * i);
+                    else
+                        ATile::store_f4(st, st + 128 * 128, swz(a_lr, a_c0 + a_cs * i), A.r + PER * i);
+                }
+            }
+            if (a.b_kind == B2_OPERAND_K) {
+                B.store_k(b0, b0 + BN * 128, warp, lane);
+            } else {
+#pragma unroll
+                for (int i = 0; i < BTile::kUnits; ++i) {
+                    const int lr = MODE == MODE_FLEX16 ? i * 64 + 2 * lane : i * 32 + lane;
+                    if (lr >= BN) continue;
+                    if (MODE == MODE_FLEX16) BTile::store_pair(b0, b0 + BN * 128, lr, warp, lane, B.r + PER * i);
+                    else BTile::store_f4(b0, b0 + BN * 128, swz(lr, warp), B.r + PER * i);
+                }
+            }
+        };
+        if (AHEAD) load(0, ta[0], tb[0]);
+        int s = 0;
+        unsigned parity = 1;
+        bool ok = true;
+        auto put = [&](int kb, ATile& A, BTile& B, ATile& An, BTile& Bn) {
+            if (!AHEAD) load(kb, A, B);
+            else if (kb + 1 < nkb) load(kb + 1, An, Bn);          // in flight while this one is stored
+            if (ok && !mbar_wait(&empty_bar[s], parity)) { atomicExch(fail_flag, 1); ok = false; }
+            store(s, A, B);
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&full_bar[s]);
+            if (++s == NST) { s = 0; parity ^= 1u; }
+        };
+        constexpr int kNext = AHEAD ? 1 : 0;
+        for (int kb = 0; kb < nkb; kb += 2) {
+            put(kb, ta[0], tb[0], ta[kNext], tb[kNext]);
+            if (kb + 1 < nkb) put(kb + 1, ta[kNext], tb[kNext], ta[0], tb[0]);
+        }
+    } else if (elect_one()) {
+        // ---- MMA issue
+        const unsigned id_ss = make_idesc(2, 1, 1, BN), id_su = make_idesc(2, 1, 0, BN),
+                       id_us = make_idesc(2, 0, 1, BN), id_uu = make_idesc(2, 0, 0, BN);
+        const unsigned id_t1 = make_idesc(1, 2, 2, BN), id_t2 = make_idesc(1, 2, 2, 2 * BN);
+        int s = 0;
+        unsigned parity = 0;
+        for (int kb = 0; kb < nkb; ++kb) {
+            if (!mbar_wait(&full_bar[s], parity)) { atomicExch(fail_flag, 1); break; }
+            tc_fence_after();
+            unsigned char* st = smem + s * STAGE;
+            const unsigned long long dA0 = make_smem_desc(st), dA1 = make_smem_desc(st + 128 * 128);
+            const unsigned long long dB0 = make_smem_desc(st + 2 * 128 * 128);
+            const unsigned long long dB1 = make_smem_desc(st + 2 * 128 * 128 + BN * 128);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const unsigned long long adv = (unsigned long long)(2 * k);
+                const unsigned acc = (kb > 0 || k > 0) ? 1u : 0u;
+                if (MODE == MODE_FLEX16) {
+                    tc_mma<MODE>(tmem_base, dA0 + adv, dB0 + adv, id_ss, acc);               // HH
+                    tc_mma<MODE>(tmem_base + BN, dA0 + adv, dB1 + adv, id_su, acc);          // X += ah*bl
+                    tc_mma<MODE>(tmem_base + BN, dA1 + adv, dB0 + adv, id_us, 1u);           // X += al*bh
+                    tc_mma<MODE>(tmem_base + 2 * BN, dA1 + adv, dB1 + adv, id_uu, acc);      // LL
+                } else {
+                    tc_mma<MODE>(tmem_base, dA0 + adv, dB0 + adv, id_t2, acc);               // hh | x
+                    tc_mma<MODE>(tmem_base + BN, dA1 + adv, dB0 + adv, id_t1, 1u);           // x += lo*hi
+                }
+            }
+            tc_commit(&empty_bar[s]);
+            if (++s == NST) { s = 0; parity ^= 1u; }
+        }
+        tc_commit(tmem_full);
+    }
+    __syncwarp();
+
+    // ---- epilogue: warps 0-7, lane quarter = warp % 4, the two warps of a quarter take the 8-column
+    // pieces in turn
+    typedef typename std::conditional<MODE == MODE_FLEX16, long long, float>::type Sum;
+    Sum* red = (Sum*)smem;                                        // [BN][128], slices only
+    const int quarter = warp & 3, half = warp >> 2;
+    const int lrow = quarter * 32 + lane, row = m0 + lrow;
+    const int splits = p.splits;
+    bool ok = true;
+    int stat = 0;
+    unsigned long long pmax = 0;
+    float fstat = 0.0f;
+    int sh = 0;
+    float f_prod = 0.f, s_bias = 0.f, s_res = 0.f;
+    if (MODE == MODE_FLEX16 && warp < 8) {
+        const float q_out = a.probe ? 1.0f : a.table[a.slotC].inv_scale;
+        f_prod = a.table[a.slotA].scale * a.table[a.slotB].scale * q_out;
+        sh = -ilogbf(f_prod);
+        if (a.tail && a.bias) s_bias = a.table[a.slot_bias].scale * q_out;
+        if (a.tail && a.residual) s_res = a.table[a.slot_res].scale * q_out;
+    }
+    auto finish = [&](int c0, Sum* v) {
+        // eight results of one row: tail, rescale, statistics, store
+        if (row >= a.M) return;
+        const int col = n0 + c0, live = a.N - col;
+        const long long at = a.colmajor ? (long long)col * a.ldc + row : (long long)row * a.ldc + col;
+        const long long dc = a.colmajor ? a.ldc : 1;
+        if (MODE == MODE_FLEX16) {
+            int q[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                q[j] = 0;
+                if (j >= live) continue;
+                const long long x = (long long)v[j];
+                if (a.tail) {
+                    float y = (float)x * f_prod;
+                    if (a.bias) y += (float)((const short*)a.bias)[col + j] * s_bias;
+                    if (a.residual) y += (float)((const short*)a.residual)[at + j * dc] * s_res;
+                    if (a.relu) y = fmaxf(y, 0.0f);
+                    if (a.probe) { fstat = fmaxf(fstat, fabsf(y)); continue; }
+                    y = fminf(fmaxf(y, -32768.0f), 32767.0f);
+                    fstat = fmaxf(fstat, fabsf(y));
+                    q[j] = __float2int_rn(y);
+                } else if (a.probe) {
+                    const unsigned long long m = (unsigned long long)(x < 0 ? -x : x);
+                    pmax = m > pmax ? m : pmax;
+                } else {
+                    q[j] = rescale_i64(x, sh);
+                    const int m = q[j] < 0 ? -q[j] : q[j];
+                    stat = m > stat ? m : stat;
+                }
+            }
+            if (a.probe) return;
+            short* out = (short*)a.C + at;
+            if (!a.colmajor && live >= 8 && ((uintptr_t)out & 15) == 0) {
+                uint4 w;
+                w.x = (q[0] & 0xffff) | (q[1] << 16); w.y = (q[2] & 0xffff) | (q[3] << 16);
+                w.z = (q[4] & 0xffff) | (q[5] << 16); w.w = (q[6] & 0xffff) | (q[7] << 16);
+                *(uint4*)out = w;
+            } else {
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+                    if (j < live) out[j * dc] = (short)q[j];
+            }
+        } else {
+            float y[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                y[j] = (float)v[j];
+                if (j >= live || !a.tail) continue;
+                if (a.bias) y[j] += ((const float*)a.bias)[col + j];
+                if (a.residual) y[j] += ((const float*)a.residual)[at + j * dc];
+                if (a.relu) y[j] = y[j] < 0.0f ? 0.0f : y[j];      // (keeps NaN, as max(x, 0) does)
+            }
+            float* out = (float*)a.C + at;
+            if (!a.colmajor && live >= 8 && ((uintptr_t)out & 15) == 0) {
+                *(float4*)out = make_float4(y[0], y[1], y[2], y[3]);
+                *(float4*)(out + 4) = make_float4(y[4], y[5], y[6], y[7]);
+            } else {
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+                    if (j < live) out[j * dc] = y[j];
+            }
+        }
+    };
+    if (warp < 8) {
+        ok = mbar_wait(tmem_full, 0);
+        if (!ok) atomicExch(fail_flag, 1);
+        tc_fence_after();
+        const unsigned lane_addr = tmem_base + ((unsigned)(quarter * 32) << 16);
+        for (int c0 = half * 8; c0 < BN; c0 += 16) {
+            if (n0 + c0 >= a.N) break;
+            Sum v[8];
+            if (MODE == MODE_FLEX16) {
+                unsigned hh[8], xx[8], ll[8];
+                tmem_ld8(lane_addr + c0, hh);
+                tmem_ld8(lane_addr + BN + c0, xx);
+                tmem_ld8(lane_addr + 2 * BN + c0, ll);
+                tmem_ld_wait();
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+                    v[j] = (Sum)(((long long)(int)hh[j] << 16) + ((long long)(int)xx[j] << 8) + (long long)(int)ll[j]);
+            } else {
+                unsigned hh[8], xx[8];
+                tmem_ld8(lane_addr + c0, hh);
+                tmem_ld8(lane_addr + BN + c0, xx);
+                tmem_ld_wait();
+#pragma unroll
+                for (int j = 0; j < 8; ++j) v[j] = (Sum)(__uint_as_float(hh[j]) + __uint_as_float(xx[j]));
+            }
+            if (splits == 1) {
+                if (ok) finish(c0, v);
+            } else {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) red[(c0 + j) * 128 + lrow] = v[j];
+            }
+        }
+    }
+    if (splits > 1) {
+        cluster_sync();
+        if (warp < 8) {
+            // this CTA's share of the pieces: every splits-th, dealt to the warps of a quarter
+            for (int c0 = (rank + half * splits) * 8; c0 < BN; c0 += 16 * splits) {
+                if (n0 + c0 >= a.N) break;
+                Sum v[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j) v[j] = 0;
+                for (int z = 0; z < splits; ++z) {
+                    const unsigned at = peer_addr(red + c0 * 128 + lrow, z);
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) v[j] += ld_peer(at + j * 128 * (unsigned)sizeof(Sum), (Sum)0);
+                }
+                if (ok) finish(c0, v);
+            }
+        }
+        cluster_sync();                                           // peers may still be reading
+    }
+    if (MODE == MODE_FLEX16 && warp < 8) {
+        if (a.tail) {
+            if (a.probe) pmax = (unsigned long long)__float_as_uint(fstat);
+            else stat = (int)rintf(fstat);
+        }
+        if (a.probe) {
+            for (int o = 16; o > 0; o >>= 1) {
+                const unsigned long long t = __shfl_xor_sync(0xffffffffu, pmax, o);
+                pmax = t > pmax ? t : pmax;
+            }
+            if (lane == 0 && pmax) atomicMax(a.probe_out, pmax);
+        } else {
+            for (int o = 16; o > 0; o >>= 1) {
+                const int t = __shfl_xor_sync(0xffffffffu, stat, o);
+                stat = t > stat ? t : stat;
+            }
+            if (lane == 0 && stat) atomicMax(a.stats + a.slotC, stat);
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 8) {
+        tc_fence_after();
+        tmem_dealloc(tmem_base, kCols);
+    }
+    if (threadIdx.x == 0 && *fail_flag && a.status) atomicExch(a.status, 1);
+}
+
+// ---- host ------------------------------------------------------------------------------------
+struct DirectShape { int bn, splits, kb_per_split; long long cost; };
+
+template <int MODE>
+DirectShape direct_shape(const b2_direct_args& a) {
+    const int KB = MODE == MODE_FLEX16 ? 128 : 32;
+    const int num_kb = (a.K + KB - 1) / KB;
+    // fp32: 16 k-blocks to a chain; flex16: exact int32 sums up to 32768 columns
+    const int most = MODE == MODE_FLEX16 ? 256 : 16;
+    DirectShape best = {0, 0, 0, -1};
+    const long long tm = (a.M + 127) / 128;
+    for (int bn = 16; bn <= 128; bn *= 2) {
+        if (bn > 16 && bn / 2 >= a.N) break;
+        const long long tiles = tm * ((a.N + bn - 1) / bn);
+        for (int want = 1; want <= 8 && want <= num_kb; ++want) {
+            const int per = (num_kb + want - 1) / want, splits = (num_kb + per - 1) / per;
+            if (splits != want || per > most) continue;
+            if (a.a_kind == B2_OPERAND_GATHER && 1152 + dir_ring_bytes(bn) + per * KB * 8 > 232448) continue;
+            // cycles of a k-block: the MMAs (N columns of a K step take N/2 cycles of the pipe, 46 at
+            // least), and the producers' instructions at about two a cycle
+            const int n1 = bn / 2 > 46 ? bn / 2 : 46, n2 = bn > 46 ? bn : 46;
+            const long long mma = MODE == MODE_FLEX16 ? 16 * n1 : 4 * (n1 + n2);
+            const double ia = a.a_kind == B2_OPERAND_K ? 1.0 : a.a_kind == B2_OPERAND_ROWS ? 1.6 : 3.0;
+            const double ib = a.b_kind == B2_OPERAND_K ? 1.0 : 1.6;
+            const long long prod = (long long)((128 * ia + bn * ib) * (MODE == MODE_FLEX16 ? 3.2 : 2.5));
+            const long long kb = mma > prod ? mma : prod;
+            const long long one = 3500 + per * kb + per * 120 + bn * (splits > 1 ? 24 : 12) + (splits > 1 ? 1500 : 0);
+            const long long ctas = tiles * splits, slots = 148LL * (bn == 128 ? 1 : 2);
+            long long cost = (ctas + slots - 1) / slots * one;
+            const long long work = (ctas * (per * kb + bn * 12 + 600) + 147) / 148;
+            if (work > cost) cost = work;
+            if (best.cost < 0 || cost < best.cost) best = {bn, splits, per, cost};
+        }
+    }
+    return best;
+}
+
+template <int MODE, int BN, int AK>
+int direct_launch_as(const DirectParams& p, cudaStream_t st) {
+    const int KB = MODE == MODE_FLEX16 ? 128 : 32;
+    int ring = dir_ring_bytes(BN);
+    const int red = p.splits > 1 ? BN * 128 * (MODE == MODE_FLEX16 ? 8 : 4) : 0;
+    static_assert(dir_ring_bytes(BN) >= BN * 128 * 8, "the slices' sums are exchanged through the ring");
+    (void)red;
+    const int smem = 1024 + ring + 128 + (AK == B2_OPERAND_GATHER ? p.kb_per_split * KB * 8 : 0);
+    static bool attr_set = false;
+    if (!attr_set) {
+        B2_CUDA(cudaFuncSetAttribute(direct_kernel<MODE, BN, AK>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     1024 + ring + 128 + (AK == B2_OPERAND_GATHER ? kDirMaxK * 8 < 232448 - 1152 - ring ? kDirMaxK * 8 : 232448 - 1152 - ring : 0)));
+        attr_set = true;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((p.a.N + BN - 1) / BN, (p.a.M + 127) / 128, p.splits);
+    cfg.blockDim = dim3(kDirThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = 1; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = p.splits;
+    cfg.attrs = attr;
+    cfg.numAttrs = p.splits > 1 ? 2 : 1;
+    B2_CUDA(cudaLaunchKernelEx(&cfg, direct_kernel<MODE, BN, AK>, p));
+    return B2_OK;
+}
+
+template <int MODE, int BN>
+int direct_launch_bn(const DirectParams& p, cudaStream_t st) {
+    switch (p.a.a_kind) {
+        case B2_OPERAND_K: return direct_launch_as<MODE, BN, B2_OPERAND_K>(p, st);
+        case B2_OPERAND_ROWS: return direct_launch_as<MODE, BN, B2_OPERAND_ROWS>(p, st);
+        default: return direct_launch_as<MODE, BN, B2_OPERAND_GATHER>(p, st);
+    }
+}
+
+template <int MODE>
+int direct_launch_mode(const b2_direct_args& a, cudaStream_t st) {
+    const DirectShape s = direct_shape<MODE>(a);
+    B2_REQUIRE(s.cost >= 0, "K is too long for this kernel");
+    DirectParams p;
+    p.a = a;
+    const int KB = MODE == MODE_FLEX16 ? 128 : 32, vec = MODE == MODE_FLEX16 ? 8 : 4;
+    p.num_kb = (a.K + KB - 1) / KB;
+    p.kb_per_split = s.kb_per_split;
+    p.splits = s.splits;
+    auto aligned = [&](int kind, const void* x, long long rs, long long ks) {
+        if (kind == B2_OPERAND_K) return ((uintptr_t)x & 15) == 0 && rs % vec == 0;
+        if (kind == B2_OPERAND_ROWS) return ((uintptr_t)x & 3) == 0 && ks % 2 == 0;
+        return ((uintptr_t)x & 3) == 0 && a.g.N % 2 == 0;         // pairs of images of one pixel
+    };
+    p.a_vec = aligned(a.a_kind, a.A, a.a_rs, a.a_ks);
+    p.b_vec = aligned(a.b_kind, a.B, a.b_rs, a.b_ks);
+    switch (s.bn) {
+        case 16: return direct_launch_bn<MODE, 16>(p, st);
+        case 32: return direct_launch_bn<MODE, 32>(p, st);
+        case 64: return direct_launch_bn<MODE, 64>(p, st);
+        default: return direct_launch_bn<MODE, 128>(p, st);
+    }
+}
+
+}  // namespace
+#endif  // B2_DIRECT_CUH

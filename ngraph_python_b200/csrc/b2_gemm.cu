@@ -19,6 +19,16 @@ extern "C" int b2_gemm_scratch_bytes(int32_t flex, int32_t M, int32_t N, int32_t
     return B2_OK;
 }
 
+extern "C" int b2_gemm_launches(int32_t flex, int64_t a_k_stride, int64_t b_k_stride, int32_t M,
+                                int32_t N, int32_t K, int32_t* launches) {
+    B2_REQUIRE(launches && M > 0 && N > 0 && K > 0, "bad argument");
+    const int mode = flex ? MODE_FLEX16 : MODE_F32X3;
+    b2_direct_args d;
+    *launches = gemm_goes_direct(mode, nullptr, 1, a_k_stride, nullptr, b_k_stride, 1, M, N, K, &d) ? 1
+                : pick_splits(mode, shapes_for(mode, M, N, K), false) > 1 ? 4 : 3;
+    return B2_OK;
+}
+
 extern "C" int b2_gemm_f32(const float* A, int64_t a_row_stride, int64_t a_k_stride, const float* B,
                            int64_t b_k_stride, int64_t b_col_stride, float* C, int64_t ldc,
                            int32_t M, int32_t N, int32_t K, void* scratch, size_t scratch_bytes,

@@ -44,8 +44,10 @@
 #include <cuda.h>
 
 #include <mutex>
+#include <type_traits>
 
 #include "b2_common.h"
+#include "b2_direct.h"
 
 // The tile kernel is compiled once, in the translation unit that defines B2_GEMM_OWNS_TILE_KERNEL
 // (b2_gemm.cu); every other includer reaches it through this function.  Shapes and GemmParams
@@ -177,6 +179,14 @@ __device__ __forceinline__ void tmem_ld16(unsigned taddr, unsigned* r) {
         : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
           "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
           "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr) : "memory");
+}
+// 8 consecutive 32-bit columns of this thread's TMEM lane
+__device__ __forceinline__ void tmem_ld8(unsigned taddr, unsigned* r) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+          "=r"(r[7])
         : "r"(taddr) : "memory");
 }
 __device__ __forceinline__ void tmem_ld_wait() {
@@ -989,55 +999,35 @@ int launch_on_planes(unsigned char* base, const Shapes& s, GemmParams p, cudaStr
 }
 #endif
 
-// A flex16 product far smaller than one wave of tensor-core tiles (the 10 x 64 x 256 classifier
-// of a small network): one thread per result, exact int64 sum, the tile kernel's rescale -- one
-// launch instead of the operand pre-passes and a mostly empty 128-row tile.
-__global__ void __launch_bounds__(256)
-small_gemm_flex16_kernel(const short* __restrict__ A, long long a_rs, long long a_cs,
-                         const short* __restrict__ B, long long b_ks, long long b_ns,
-                         short* __restrict__ C, long long ldc, int M, int N, int K,
-                         const b2_flex_scale* __restrict__ table, int slotA, int slotB, int slotC,
-                         int* stats, unsigned long long* probe_out, int probe) {
-    const float f = table[slotA].scale * table[slotB].scale * (probe ? 1.0f : table[slotC].inv_scale);
-    const int sh = -ilogbf(f);
-    int stat = 0;
-    unsigned long long pmax = 0;
-    const long long total = (long long)M * N;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
-         i += (long long)gridDim.x * blockDim.x) {
-        const int m = (int)(i / N), n = (int)(i - (long long)m * N);
-        const short* a = A + m * a_rs;
-        const short* b = B + n * b_ns;
-        long long acc = 0;
-#pragma unroll 4
-        for (int k = 0; k < K; ++k) acc += (long long)((int)a[k * a_cs] * (int)b[k * b_ks]);
-        if (probe) {
-            const unsigned long long v = (unsigned long long)(acc < 0 ? -acc : acc);
-            pmax = v > pmax ? v : pmax;
-        } else {
-            const int q = rescale_i64(acc, sh);
-            const int v = q < 0 ? -q : q;
-            stat = v > stat ? v : stat;
-            C[m * ldc + n] = (short)q;
-        }
-    }
-    if (probe) {
-        for (int o = 16; o > 0; o >>= 1) {
-            const unsigned long long t = __shfl_xor_sync(0xffffffffu, pmax, o);
-            pmax = t > pmax ? t : pmax;
-        }
-        if ((threadIdx.x & 31) == 0 && pmax) atomicMax(probe_out, pmax);
-    } else {
-        for (int o = 16; o > 0; o >>= 1) {
-            const int t = __shfl_xor_sync(0xffffffffu, stat, o);
-            stat = t > stat ? t : stat;
-        }
-        if ((threadIdx.x & 31) == 0 && stat) atomicMax(stats + slotC, stat);
-    }
+// Cycles of the plane path: two pre-pass launches (and a memset), their traffic, and the tile kernel
+// with one CTA per SM -- 1100 (fp32) or 1430 (flex16) cycles a k-block at BN = 128, both measured.
+inline long long plane_cost(int mode, const Shapes& s, int M, int N, int K) {
+    const long long prepass = ((long long)M + N) * K * (mode == MODE_FLEX16 ? 4 : 12) / 2600;
+    const long long kb = (mode == MODE_FLEX16 ? 1430LL : 1100LL) * (128 + s.bn) / 256;
+    const long long tiles = (long long)(s.Mp / kBlockM) * (s.Np / s.bn), num_kb = s.Kp / (kKBytes / s.esize);
+    return 13000 + prepass + (tiles + 147) / 148 * (3500 + num_kb * kb);
 }
 
-inline bool small_gemm(int mode, int M, int N, int K) {
-    return mode == MODE_FLEX16 && (long long)M * N <= 8192 && K <= 1024;
+// Whether a product takes the kernel that converts its operands on the way in (one launch), and its
+// arguments: the cheaper of C and its transpose, so that a product with few rows does not pad them to
+// a whole tile.
+inline bool gemm_goes_direct(int mode, const void* A, long long a_rs, long long a_cs, const void* B,
+                             long long b_ks, long long b_ns, int M, int N, int K, b2_direct_args* out) {
+    b2_direct_args d = {};
+    d.flex = mode == MODE_FLEX16;
+    d.A = A; d.a_rs = a_rs; d.a_ks = a_cs; d.a_kind = a_cs == 1 ? B2_OPERAND_K : B2_OPERAND_ROWS;
+    d.B = B; d.b_rs = b_ns; d.b_ks = b_ks; d.b_kind = b_ks == 1 ? B2_OPERAND_K : B2_OPERAND_ROWS;
+    d.M = M; d.N = N; d.K = K;
+    b2_direct_args t = d;
+    t.A = d.B; t.a_rs = d.b_rs; t.a_ks = d.b_ks; t.a_kind = d.b_kind;
+    t.B = d.A; t.b_rs = d.a_rs; t.b_ks = d.a_ks; t.b_kind = d.a_kind;
+    t.M = N; t.N = M; t.colmajor = 1;
+    const long long cd = b2_direct_cost(d), ct = b2_direct_cost(t);
+    const long long plane = plane_cost(mode, shapes_for(mode, M, N, K), M, N, K);
+    const bool swap = ct >= 0 && (cd < 0 || ct < cd);
+    *out = swap ? t : d;
+    const long long best = swap ? ct : cd;
+    return best >= 0 && best < plane;
 }
 
 template <typename T, int MODE>
@@ -1048,13 +1038,12 @@ int run_gemm(const T* A, long long a_rs, long long a_cs, const T* B, long long b
     B2_REQUIRE(A && B && C && M > 0 && N > 0 && K > 0, "bad GEMM argument");
     B2_REQUIRE(a_rs == 1 || a_cs == 1, "A must be contiguous along M or K");
     B2_REQUIRE(b_ks == 1 || b_ns == 1, "B must be contiguous along K or N");
-    if (small_gemm(MODE, M, N, K)) {
-        const int blocks = (int)(((long long)M * N + 255) / 256);
-        small_gemm_flex16_kernel<<<blocks, 256, 0, st>>>(
-            (const short*)A, a_rs, a_cs, (const short*)B, b_ks, b_ns, (short*)C, ldc, M, N, K, table,
-            slotA, slotB, slotC, stats, probe_out, probe);
-        B2_CUDA(cudaGetLastError());
-        return B2_OK;
+    b2_direct_args d;
+    if (gemm_goes_direct(MODE, A, a_rs, a_cs, B, b_ks, b_ns, M, N, K, &d)) {
+        d.C = C; d.ldc = ldc; d.table = table; d.slotC = slotC;
+        d.slotA = d.colmajor ? slotB : slotA; d.slotB = d.colmajor ? slotA : slotB;
+        d.stats = stats; d.probe_out = probe_out; d.status = status; d.probe = probe;
+        return b2_direct_launch(d, st);
     }
     const Shapes s = shapes_for(MODE, M, N, K);
     const int splits = pick_splits(MODE, s, false);     // > 1 only for flex16 with K > 32768

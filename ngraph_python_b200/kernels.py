@@ -178,7 +178,7 @@ class _PlaneUser(object):
 class GemmStep(_Step):
     """C[M,N] = op(A)[M,K] * op(B)[K,N] for a DotOp."""
     kind = "gemm"
-    launches = 3          # two operand-plane kernels + the tensor-core kernel
+    launches = 3
 
     def __init__(self, index, op, t):
         super(GemmStep, self).__init__(index, op)
@@ -190,8 +190,6 @@ class GemmStep(_Step):
         if None in (am, ak, bk, bn):
             raise ValueError("Unhandled op: dot operands must be 2-d collapsible: {}".format(op))
         self.M, self.K, self.N = am[0], ak[0], bn[0]
-        if t.flex and self.M * self.N <= 8192 and self.K <= 1024:
-            self.launches = 1         # the library's one-launch form for very small products
         if bk[0] != self.K:
             raise ValueError("Unhandled op: reduction axes of the dot operands disagree")
         # extents of 1 carry no stride of their own: describe them as row-major
@@ -207,6 +205,7 @@ class GemmStep(_Step):
         self.out_views = [t._view_of(op)]
         self.flex = t.flex
         self.scratch_bytes = lib.gemm_scratch_bytes(self.flex, self.M, self.N, self.K) + 1024
+        self.launches = lib.gemm_launches(self.flex, a_cs, b_ks, self.M, self.N, self.K)
 
     def launch(self, t):
         xv, yv = self.in_views

@@ -118,6 +118,7 @@ def _load():
         "b2_ew_source": (C.c_char_p, [vp]),
         "b2_ew_launch_count": (C.c_int, [vp]),
         "b2_gemm_scratch_bytes": (C.c_int, [i32, i32, i32, i32, C.POINTER(sz)]),
+        "b2_gemm_launches": (C.c_int, [i32, i64, i64, i32, i32, i32, C.POINTER(i32)]),
         "b2_gemm_f32": (C.c_int, [vp, i64, i64, vp, i64, i64, vp, i64, i32, i32, i32, vp, sz, vp,
                                   vp]),
         "b2_gemm_flex16": (C.c_int, [vp, i64, i64, vp, i64, i64, vp, i64, i32, i32, i32, vp, i32,
@@ -321,6 +322,12 @@ class PlannedKernel(object):
 def gemm_scratch_bytes(flex, M, N, K):
     n = C.c_size_t()
     check(_lib.b2_gemm_scratch_bytes(int(bool(flex)), M, N, K, C.byref(n)))
+    return n.value
+
+
+def gemm_launches(flex, a_k_stride, b_k_stride, M, N, K):
+    n = C.c_int32()
+    check(_lib.b2_gemm_launches(int(bool(flex)), a_k_stride, b_k_stride, M, N, K, C.byref(n)))
     return n.value
 
 
