@@ -45,10 +45,10 @@ struct DirectParams {
     int a_vec, b_vec;                     // 16-byte loads (K contiguous) / row pairs (flex16, others)
 };
 
+// a = hi + lo with hi rounded to tf32, ties away from zero: what cvt.rna.tf32 gives for every finite a
+// (infinities and NaN end as NaN in the product either way), on the full-rate integer pipe
 __device__ __forceinline__ void dir_split_tf32(float a, float& hi, float& lo) {
-    unsigned hb;
-    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(hb) : "f"(a));
-    hi = __uint_as_float(hb);
+    hi = __uint_as_float((__float_as_uint(a) + 0x1000u) & 0xffffe000u);
     lo = a - hi;
 }
 __device__ __forceinline__ unsigned swz(int row, int chunk) {
@@ -88,38 +88,45 @@ struct OperandTile {
     static constexpr int kKUnits = ROWS / 4 >= 8 ? ROWS / 32 : 1;      // units per warp, K contiguous
     unsigned r[kRegs];
 
-    // -- K contiguous
-    __device__ __forceinline__ void load_k(const void* src, long long rs, int row0, int rows, int K,
-                                           int k0, int vec, int warp, int lane) {
-        const int chunk = lane & 7;
-        constexpr int per = MODE == MODE_FLEX16 ? 16 : 4, regs = MODE == MODE_FLEX16 ? 8 : 4;
+    // -- K contiguous: byte offsets of this lane's chunk in each of its rows (-1: no such row)
+    __device__ __forceinline__ static void offsets_k(long long (&at)[kKUnits], long long rs, int row0, int rows,
+                                                     int warp, int lane) {
+        constexpr int per = MODE == MODE_FLEX16 ? 16 : 4, size = MODE == MODE_FLEX16 ? 2 : 4;
 #pragma unroll
         for (int i = 0; i < kKUnits; ++i) {
-            const int lr = (warp + 8 * i) * 4 + (lane >> 3), row = row0 + lr, k = k0 + chunk * per;
+            const int lr = (warp + 8 * i) * 4 + (lane >> 3), row = row0 + lr;
+            at[i] = lr < ROWS && row < rows ? ((long long)row * rs + (lane & 7) * per) * size : -1;
+        }
+    }
+    // `left`: columns from k0 to the end of K
+    __device__ __forceinline__ void load_k(const void* src, const long long (&at)[kKUnits], int k0, int left,
+                                           int vec, int lane) {
+        constexpr int per = MODE == MODE_FLEX16 ? 16 : 4, regs = MODE == MODE_FLEX16 ? 8 : 4,
+                      size = MODE == MODE_FLEX16 ? 2 : 4;
+        const char* base = (const char*)src + (long long)k0 * size;
+        const bool whole = vec && (lane & 7) * per + per <= left;
+#pragma unroll
+        for (int i = 0; i < kKUnits; ++i) {
 #pragma unroll
             for (int j = 0; j < regs; ++j) r[regs * i + j] = 0;
-            if (lr >= ROWS || row >= rows || k >= K) continue;
-            if (MODE == MODE_FLEX16) {
-                const short* p = (const short*)src + (long long)row * rs + k;
-                if (vec && k + 16 <= K) {
-                    const uint4 a = __ldg((const uint4*)p), b = __ldg((const uint4*)p + 1);
-                    r[8 * i + 0] = a.x; r[8 * i + 1] = a.y; r[8 * i + 2] = a.z; r[8 * i + 3] = a.w;
-                    r[8 * i + 4] = b.x; r[8 * i + 5] = b.y; r[8 * i + 6] = b.z; r[8 * i + 7] = b.w;
-                } else {
-#pragma unroll
-                    for (int j = 0; j < 16; ++j)
-                        if (k + j < K) r[8 * i + (j >> 1)] |= (unsigned)(unsigned short)p[j] << ((j & 1) * 16);
+            if (at[i] < 0) continue;
+            const char* p = base + at[i];
+            if (whole) {
+                const uint4 a = __ldg((const uint4*)p);
+                r[regs * i + 0] = a.x; r[regs * i + 1] = a.y; r[regs * i + 2] = a.z; r[regs * i + 3] = a.w;
+                if (MODE == MODE_FLEX16) {
+                    const uint4 b = __ldg((const uint4*)p + 1);
+                    r[regs * i + regs - 4] = b.x; r[regs * i + regs - 3] = b.y;
+                    r[regs * i + regs - 2] = b.z; r[regs * i + regs - 1] = b.w;
                 }
             } else {
-                const float* p = (const float*)src + (long long)row * rs + k;
-                if (vec && k + 4 <= K) {
-                    const float4 v = __ldg((const float4*)p);
-                    r[4 * i + 0] = __float_as_uint(v.x); r[4 * i + 1] = __float_as_uint(v.y);
-                    r[4 * i + 2] = __float_as_uint(v.z); r[4 * i + 3] = __float_as_uint(v.w);
-                } else {
 #pragma unroll
-                    for (int j = 0; j < 4; ++j)
-                        if (k + j < K) r[4 * i + j] = __float_as_uint(p[j]);
+                for (int j = 0; j < per; ++j) {
+                    if ((lane & 7) * per + j >= left) continue;
+                    if (MODE == MODE_FLEX16)
+                        r[regs * i + (j >> 1)] |= (unsigned)((const unsigned short*)p)[j] << ((j & 1) * 16);
+                    else
+                        r[regs * i + j % regs] = ((const unsigned*)p)[j];
                 }
             }
         }
@@ -290,10 +297,13 @@ direct_kernel(const __grid_constant__ DirectParams p) {
             }
             if (GR == 2) pair = pair && (mask[GR - 1] == mask[0]) && m0 + a_lr + 1 < a.M;
         }
+        long long a_at[ATile::kKUnits], b_at[BTile::kKUnits];
+        if (AK == B2_OPERAND_K) ATile::offsets_k(a_at, a.a_rs, m0, a.M, warp, lane);
+        BTile::offsets_k(b_at, a.b_rs, n0, a.N, warp, lane);
         auto load = [&](int kb, ATile& A, BTile& B) {
             const int kt = kb * KB, k0 = kb0 * KB + kt;
             if (AK == B2_OPERAND_K) {
-                A.load_k(a.A, a.a_rs, m0, a.M, a.K, k0, p.a_vec, warp, lane);
+                A.load_k(a.A, a_at, k0, a.K - k0, p.a_vec, lane);
             } else {
 #pragma unroll
                 for (int i = 0; i < A_UNITS; ++i) {
@@ -329,7 +339,7 @@ direct_kernel(const __grid_constant__ DirectParams p) {
                 }
             }
             if (a.b_kind == B2_OPERAND_K) {
-                B.load_k(a.B, a.b_rs, n0, a.N, a.K, k0, p.b_vec, warp, lane);
+                B.load_k(a.B, b_at, k0, a.K - k0, p.b_vec, lane);
             } else {
                 // chunk = warp, groups of 32 (64) rows
 #pragma unroll
@@ -619,19 +629,18 @@ DirectShape direct_shape(const b2_direct_args& a) {
             const int per = (num_kb + want - 1) / want, splits = (num_kb + per - 1) / per;
             if (splits != want || per > most) continue;
             if (a.a_kind == B2_OPERAND_GATHER && 1152 + dir_ring_bytes(bn) + per * KB * 8 > 232448) continue;
-            // cycles of a k-block: the MMAs (N columns of a K step take N/2 cycles of the pipe, 46 at
-            // least), and the producers' instructions at about two a cycle
-            const int n1 = bn / 2 > 46 ? bn / 2 : 46, n2 = bn > 46 ? bn : 46;
-            const long long mma = MODE == MODE_FLEX16 ? 16 * n1 : 4 * (n1 + n2);
-            const double ia = a.a_kind == B2_OPERAND_K ? 1.0 : a.a_kind == B2_OPERAND_ROWS ? 1.6 : 3.0;
-            const double ib = a.b_kind == B2_OPERAND_K ? 1.0 : 1.6;
-            const long long prod = (long long)((128 * ia + bn * ib) * (MODE == MODE_FLEX16 ? 3.2 : 2.5));
-            const long long kb = mma > prod ? mma : prod;
-            const long long one = 3500 + per * kb + per * 120 + bn * (splits > 1 ? 24 : 12) + (splits > 1 ? 1500 : 0);
+            // Measured on one B200 (cycles at 1.9 GHz): the producers set the pace, 7 (fp32) or 22
+            // (flex16) cycles an operand row of a k-block when they keep an SM busy, and a k-block
+            // takes 1000 + 6 bn or 4000 cycles from load to commit when they do not; the two CTAs of
+            // an SM overlap.  Gathered rows cost their address and bounds.
+            const double ra = a.a_kind == B2_OPERAND_GATHER ? 1.5 : 1.0;
+            const long long pace = (long long)((128 * ra + bn) * (MODE == MODE_FLEX16 ? (bn == 128 ? 33 : 22) : 7));
+            const long long lat = MODE == MODE_FLEX16 ? 4000 : 1000 + 6 * bn;
             const long long ctas = tiles * splits, slots = 148LL * (bn == 128 ? 1 : 2);
-            long long cost = (ctas + slots - 1) / slots * one;
-            const long long work = (ctas * (per * kb + bn * 12 + 600) + 147) / 148;
-            if (work > cost) cost = work;
+            const long long together = ctas <= 148 || bn == 128 ? 1 : 2;
+            const long long kb = together * pace > lat ? together * pace : lat;
+            const long long one = 7000 + per * kb + together * bn * (splits > 1 ? 24 : 12) + (splits > 1 ? 3000 : 0);
+            const long long cost = (ctas + slots - 1) / slots * one;
             if (best.cost < 0 || cost < best.cost) best = {bn, splits, per, cost};
         }
     }

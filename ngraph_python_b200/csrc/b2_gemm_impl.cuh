@@ -47,7 +47,6 @@
 #include <type_traits>
 
 #include "b2_common.h"
-#include "b2_direct.h"
 
 // The tile kernel is compiled once, in the translation unit that defines B2_GEMM_OWNS_TILE_KERNEL
 // (b2_gemm.cu); every other includer reaches it through this function.  Shapes and GemmParams
@@ -998,82 +997,6 @@ int launch_on_planes(unsigned char* base, const Shapes& s, GemmParams p, cudaStr
     return b2_gemm_launch_on_planes(MODE, base, &s, &p, st, splits, workspace);
 }
 #endif
-
-// Cycles of the plane path: two pre-pass launches (and a memset), their traffic, and the tile kernel
-// with one CTA per SM -- 1100 (fp32) or 1430 (flex16) cycles a k-block at BN = 128, both measured.
-inline long long plane_cost(int mode, const Shapes& s, int M, int N, int K) {
-    const long long prepass = ((long long)M + N) * K * (mode == MODE_FLEX16 ? 4 : 12) / 2600;
-    const long long kb = (mode == MODE_FLEX16 ? 1430LL : 1100LL) * (128 + s.bn) / 256;
-    const long long tiles = (long long)(s.Mp / kBlockM) * (s.Np / s.bn), num_kb = s.Kp / (kKBytes / s.esize);
-    return 13000 + prepass + (tiles + 147) / 148 * (3500 + num_kb * kb);
-}
-
-// Whether a product takes the kernel that converts its operands on the way in (one launch), and its
-// arguments: the cheaper of C and its transpose, so that a product with few rows does not pad them to
-// a whole tile.
-inline bool gemm_goes_direct(int mode, const void* A, long long a_rs, long long a_cs, const void* B,
-                             long long b_ks, long long b_ns, int M, int N, int K, b2_direct_args* out) {
-    b2_direct_args d = {};
-    d.flex = mode == MODE_FLEX16;
-    d.A = A; d.a_rs = a_rs; d.a_ks = a_cs; d.a_kind = a_cs == 1 ? B2_OPERAND_K : B2_OPERAND_ROWS;
-    d.B = B; d.b_rs = b_ns; d.b_ks = b_ks; d.b_kind = b_ks == 1 ? B2_OPERAND_K : B2_OPERAND_ROWS;
-    d.M = M; d.N = N; d.K = K;
-    b2_direct_args t = d;
-    t.A = d.B; t.a_rs = d.b_rs; t.a_ks = d.b_ks; t.a_kind = d.b_kind;
-    t.B = d.A; t.b_rs = d.a_rs; t.b_ks = d.a_ks; t.b_kind = d.a_kind;
-    t.M = N; t.N = M; t.colmajor = 1;
-    const long long cd = b2_direct_cost(d), ct = b2_direct_cost(t);
-    const long long plane = plane_cost(mode, shapes_for(mode, M, N, K), M, N, K);
-    const bool swap = ct >= 0 && (cd < 0 || ct < cd);
-    *out = swap ? t : d;
-    const long long best = swap ? ct : cd;
-    return best >= 0 && best < plane;
-}
-
-template <typename T, int MODE>
-int run_gemm(const T* A, long long a_rs, long long a_cs, const T* B, long long b_ks, long long b_ns,
-             void* C, long long ldc, int M, int N, int K, const b2_flex_scale* table, int slotA,
-             int slotB, int slotC, int* stats, void* scratch, size_t scratch_bytes,
-             unsigned long long* probe_out, int* status, int probe, cudaStream_t st) {
-    B2_REQUIRE(A && B && C && M > 0 && N > 0 && K > 0, "bad GEMM argument");
-    B2_REQUIRE(a_rs == 1 || a_cs == 1, "A must be contiguous along M or K");
-    B2_REQUIRE(b_ks == 1 || b_ns == 1, "B must be contiguous along K or N");
-    b2_direct_args d;
-    if (gemm_goes_direct(MODE, A, a_rs, a_cs, B, b_ks, b_ns, M, N, K, &d)) {
-        d.C = C; d.ldc = ldc; d.table = table; d.slotC = slotC;
-        d.slotA = d.colmajor ? slotB : slotA; d.slotB = d.colmajor ? slotA : slotB;
-        d.stats = stats; d.probe_out = probe_out; d.status = status; d.probe = probe;
-        return b2_direct_launch(d, st);
-    }
-    const Shapes s = shapes_for(MODE, M, N, K);
-    const int splits = pick_splits(MODE, s, false);     // > 1 only for flex16 with K > 32768
-    const size_t need = gemm_scratch_need(MODE, s);
-    B2_REQUIRE(scratch && scratch_bytes >= need && ((uintptr_t)scratch & 1023) == 0,
-               "GEMM needs %zu bytes of 1024-byte aligned scratch, got %zu", need, scratch_bytes);
-    unsigned char* base = (unsigned char*)scratch;
-    const size_t a_plane = (size_t)s.Mp * s.Kp * s.esize, b_plane = (size_t)s.Np * s.Kp * s.esize;
-    void* A0 = base; void* A1 = base + a_plane;
-    void* B0 = base + 2 * a_plane; void* B1 = base + 2 * a_plane + b_plane;
-    int* rowsum = nullptr;
-    unsigned lo_xor = 0;
-    if (MODE == MODE_FLEX16) {
-        rowsum = (int*)(base + s.rowsum_off);
-        lo_xor = 0x80;
-        B2_CUDA(cudaMemsetAsync(rowsum, 0, (size_t)s.Mp * sizeof(int), st));
-    }
-    int rc = split_operand<T, MODE>(A, a_rs, a_cs, M, K, s.Mp, s.Kp, A0, A1, 0, rowsum, st);
-    if (rc) return rc;
-    // op(B)^T: rows = N, element (n, k) = B[k * b_ks + n * b_ns]
-    rc = split_operand<T, MODE>(B, b_ns, b_ks, N, K, s.Np, s.Kp, B0, B1, lo_xor, nullptr, st);
-    if (rc) return rc;
-    GemmParams p;
-    p.M = M; p.N = N; p.num_kb = 0;
-    p.ldc = ldc; p.C = C; p.table = table; p.slotA = slotA; p.slotB = slotB; p.slotC = slotC;
-    p.stats = stats; p.probe_out = probe_out; p.status = status; p.probe = probe;
-    p.c_colmajor = 0;
-    p.rowsum = rowsum;
-    return launch_on_planes<MODE>(base, s, p, st, splits, base + align1k(s.bytes));
-}
 
 }  // namespace
 
