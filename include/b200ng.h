@@ -289,12 +289,13 @@ int b2_conv_fprop_flex16(const int16_t* I, const int16_t* F, int16_t* O, const b
                          int32_t* status, int32_t probe, void* stream);
 /* The flex16 convolution in parts, for callers that keep operand planes around: the tile kernel
  * reads its streamed tensor (pass 0: the activations I; pass 1, the input gradient of a
- * unit-stride convolution: the error tensor E) and the filters as byte planes -- high and low
- * bytes of the int16 mantissas, the streamed tensor in its own C,H,W,N (K,P,Q,N) order with the
- * low plane act_plane_bytes after the high plane, 1024-byte aligned.  A fused elementwise kernel
+ * convolution: the error tensor E) and the filters as byte planes -- high and low
+ * bytes of the int16 mantissas, the streamed tensor in its own C,H,W,N (K,P,Q,N) order, every row
+ * of N images padded to a multiple of 16 bytes, the low plane act_plane_bytes after the high
+ * plane, 1024-byte aligned.  A fused elementwise kernel
  * can emit such planes directly (B2_FLEX16_PLANES) and the filter planes of constant weights can
  * be built once, which leaves ONE launch per convolution.  `supported` is 0 where the plane path
- * does not apply (batch not a multiple of 128, dilation, very large windows; pass 1: strides);
+ * does not apply (dilation, very large windows; pass 1: strides whose product exceeds 4);
  * use b2_conv_fprop_flex16 / b2_conv_bprop_flex16 there.  `d` always describes the FORWARD
  * convolution.  No counterpart in the reference, whose kernels read int16 tensors directly. */
 enum b2_conv_pass { B2_CONV_FPROP = 0, B2_CONV_BPROP = 1 };

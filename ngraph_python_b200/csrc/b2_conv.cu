@@ -39,11 +39,17 @@ struct ConvGeom {
     // depth (the reference's D / T / M axes): handled by the gather + GEMM path only; the tile
     // kernels take convolutions with D = T = M = 1
     int D, T, M, pad_d, str_d, dil_d;
-    // the streamed tensor of an implicit-GEMM pass may be a zero-dilated view of a smaller one
-    // (the input gradient of a strided convolution): element (h, w) is source (h/up_h, w/up_w)
-    // where both divide and the quotient is inside src_h x src_w, zero elsewhere
-    int up_h, up_w, src_h, src_w;
+    // the tile kernel's view of an input gradient: C, H, W are the error tensor's, K, P, Q the input's,
+    // the rest the forward convolution's
+    int bprop;
 };
+
+// Byte planes have their rows of N images padded to a multiple of 16 bytes (what TMA strides need).
+inline int plane_pitch(int n) { return (n + 15) / 16 * 16; }
+inline size_t plane_size(int c, int h, int w, int n) {
+    return ((size_t)c * h * w * plane_pitch(n) + 1023) / 1024 * 1024;
+}
+inline int image_blocks(int n) { return (n + 127) / 128; }
 
 int geom_from(const b2_conv_dims* d, ConvGeom* g) {
     B2_REQUIRE(d, "null dims");
@@ -57,7 +63,7 @@ int geom_from(const b2_conv_dims* d, ConvGeom* g) {
     g->C = d->C; g->H = d->H; g->W = d->W; g->N = d->N; g->K = d->K; g->R = d->R; g->S = d->S;
     g->P = d->P; g->Q = d->Q; g->pad_h = d->pad_h; g->pad_w = d->pad_w; g->str_h = d->str_h;
     g->str_w = d->str_w; g->dil_h = d->dil_h; g->dil_w = d->dil_w;
-    g->up_h = g->up_w = 1; g->src_h = g->H; g->src_w = g->W;
+    g->bprop = 0;
     g->D = d->D; g->T = d->T; g->M = d->M; g->pad_d = d->pad_d; g->str_d = d->str_d;
     g->dil_d = d->dil_d;
     return B2_OK;
@@ -206,12 +212,12 @@ im2col_planes_kernel(const T* __restrict__ I, ConvGeom g, int rows, int kg, int 
 // ================================================================================================
 struct ConvTileParams {
     int P, Q, N, K;
-    int pad_h, pad_w, str_h, str_w;
+    int off_h, off_w, step_h, step_w;   // a tile's window starts at tile * step + off
     int cu;                       // channels per chunk
     int cchunks;                  // chunks per tile = stages per tile
     int kc_pad;                   // K rows per chunk, padded to a multiple of 32
     int box_bytes;                // bytes one activation box delivers (cu * window * 128)
-    int gh, gw, tq;               // output pixels a tile covers (gh x gw), tiles along a row
+    int gh, gw, gw_log, tq;       // output pixels a tile covers (gh x gw), tiles along a row
     int npanels;                  // 128-byte K panels of the resident filter planes
     int nstages;                  // ring depth
     int bn;                       // columns per accumulator: gh*gw * (kt channels + a sum column)
@@ -235,7 +241,9 @@ struct ConvTileParams {
     const short* residual; int slot_res;      // same K,P,Q,N layout as the output
     int relu;
     int write_i16;
-    int vec;                      // tensors aligned for eight images at a time
+    int vec;                      // int16 tensors aligned for eight images at a time
+    int NP;                       // images per row of the byte planes
+    long long ldc_planes;
     unsigned char* out_planes; long long out_plane_bytes;
 };
 
@@ -273,12 +281,15 @@ __device__ __forceinline__ float max3_abs(float m, float a, float b) {
     asm("max.abs.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(m), "f"(a), "f"(b));
     return r;
 }
-// eight consecutive int16, as one load where the alignment allows it
-__device__ __forceinline__ uint4 load8(const short* p, int vec) {
+// eight consecutive int16, as one load where the alignment allows it; only the first n exist
+__device__ __forceinline__ uint4 load8(const short* p, int vec, int n) {
+    if (n <= 0) return make_uint4(0, 0, 0, 0);
     if (vec) return *reinterpret_cast<const uint4*>(p);
     const unsigned short* q = reinterpret_cast<const unsigned short*>(p);
-    return make_uint4(q[0] | (unsigned)q[1] << 16, q[2] | (unsigned)q[3] << 16,
-                      q[4] | (unsigned)q[5] << 16, q[6] | (unsigned)q[7] << 16);
+    unsigned v[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] = j < n ? q[j] : 0;
+    return make_uint4(v[0] | v[1] << 16, v[2] | v[3] << 16, v[4] | v[5] << 16, v[6] | v[7] << 16);
 }
 // one 32-bit column of this thread's TMEM lane
 __device__ __forceinline__ unsigned tmem_ld1(unsigned taddr) {
@@ -395,12 +406,12 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap mapI0,
             int nb = (int)blockIdx.x % nblk, pq = (int)blockIdx.x / nblk, q = pq % tq, pp = pq / tq;
             const int d_nb = (int)gridDim.x % nblk, d_pq = (int)gridDim.x / nblk, d_q = d_pq % tq,
                       d_p = d_pq / tq;
-            const int step_h = p.gh * p.str_h, step_w = p.gw * p.str_w;
+            const int step_h = p.step_h, step_w = p.step_w;
             for (int tile = blockIdx.x; tile < p.num_tiles && ok; tile += gridDim.x) {
                 unsigned long long* fb = full_bar + mma * kConvMaxStages;            // its consumer's
                 if (++mma == n_mma) mma = 0;
                 const int n0 = nb * 128;
-                const int h0 = pp * step_h - p.pad_h, w0 = q * step_w - p.pad_w;
+                const int h0 = pp * step_h + p.off_h, w0 = q * step_w + p.off_w;
                 for (int cc = 0; cc < p.cchunks; ++cc) {
                     if (!mbar_wait(&empty_bar[s], empty_parity)) {
                         atomicExch(fail_flag, 1); ok = false; break;
@@ -529,7 +540,7 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap mapI0,
                                  k256 = pack2(256.0f, 256.0f), k65536 = pack2(65536.0f, 65536.0f),
                                  kmagic = pack2(12582912.0f, 12582912.0f);
         float fstat = 0.0f;
-        const OFF ldc = (OFF)p.ldc;
+        const OFF ldc = (OFF)p.ldc, ldc_p = (OFF)p.ldc_planes;
         unsigned char* const out_lo = p.out_planes + p.out_plane_bytes;
         const bool fast = sh >= 1 && sh <= 31;
         const unsigned rmask = fast ? (1u << sh) - 1u : 0u, rhalf = fast ? 1u << (sh - 1) : 0u;
@@ -559,12 +570,20 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap mapI0,
         // (with three sets the warps of the fourth slot have none)
         for (int ti = set < nbuf ? set : n_my; ti < n_my; ti += nbuf) {
             const int p0 = ty * p.gh, q0 = tx * p.gw;
-            // a pixel of the tile: inside the image or not, and its offset within a channel
+            // a pixel of the tile: inside the image or not, and its offset within a channel (of the
+            // int16 tensors; the planes' where their rows are padded)
+            OFF poff = 0;
             auto pixel = [&](int g, OFF& off) -> bool {
-                const int gy = p.gw == 1 ? g : g >> 1, gx = p.gw == 1 ? 0 : g & 1;
-                off = (OFF)((p0 + gy) * p.Q + q0 + gx) * (OFF)p.N + (OFF)(nb * 128);
+                const int gy = g >> p.gw_log, gx = g & (p.gw - 1);
+                const OFF pix = (OFF)((p0 + gy) * p.Q + q0 + gx);
+                off = pix * (OFF)p.N + (OFF)(nb * 128);
+                if (!EVEN) poff = pix * (OFF)p.NP + (OFF)(nb * 128);
                 return p0 + gy < p.P && q0 + gx < p.Q;
             };
+            // images beyond N in the last block of a ragged batch: this thread's own, and how many of
+            // the eight that it loads and stores exist
+            const bool live_img = EVEN || nb * 128 + quarter * 32 + lane < p.N;
+            const int n_img = EVEN ? 8 : p.N - (nb * 128 + simg);
             if (EPI != EPI_INT) {
                 // fp32 epilogue: the exact integer sum scaled to a real value, bias and residual
                 // added, ReLU, ONE quantisation with the output's exponent.  Eight columns at a
@@ -579,7 +598,7 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap mapI0,
                 // the residual of the first piece is fetched while the tile is being multiplied
                 int c = (part & epi_mask) * 8;
                 if (EPI == EPI_RESIDUAL && inside && c < kt && (EVEN || c + scol < left))
-                    rq = load8(p.residual + off + (OFF)c * ldc, EVEN || p.vec);
+                    rq = load8(p.residual + off + (OFF)c * ldc, EVEN || p.vec, n_img);
                 if (ok && !mbar_wait(&tmem_full[buf], full_parity)) { atomicExch(fail_flag, 1); ok = false; }
                 tc_fence_after();
                 const unsigned lane_addr = tmem_base + buf * acc_cols + ((unsigned)(quarter * 32) << 16);
@@ -594,7 +613,7 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap mapI0,
                     const unsigned long long fix2 = pack2(fixf, fixf);
                     const unsigned col0 = lane_addr + g * kt;
                     const bool here = inside && ok;
-                    const OFF at_g = off;
+                    const OFF at_g = off, poff_g = poff + (OFF)(ncol0 + scol) * ldc_p + (OFF)simg;
                     start = (start + epi_w - kt8) & epi_mask;     // first piece of this warp in pixel g+1
                     for (; c < kt; c += 8 * epi_w) {
                         unsigned hh[8], xx[8], ll[8];
@@ -621,6 +640,7 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap mapI0,
                             // the residual of the next piece, one piece ahead of its use
                             int cn = c + 8 * epi_w;
                             OFF offn = at_g;
+                            const OFF keep = poff;
                             bool in = inside;
                             if (cn >= kt && g + 1 < G) {
                                 in = pixel(g + 1, offn);
@@ -628,8 +648,9 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap mapI0,
                                 cn = start * 8;
                                 ahead = true;
                             }
+                            poff = keep;
                             if (in && cn < kt && (EVEN || cn + scol < left))
-                                rq = load8(p.residual + offn + (OFF)cn * ldc, EVEN || p.vec);
+                                rq = load8(p.residual + offn + (OFF)cn * ldc, EVEN || p.vec, n_img);
                         }
                         tmem_ld_wait();
                         if (!here) continue;
@@ -665,13 +686,13 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap mapI0,
                         for (int j = 0; j < 4; ++j) unpack2(y[j], z[2 * j], z[2 * j + 1]);
 #pragma unroll
                         for (int j = 0; j < 8; ++j) z[j] = fminf(fmaxf(z[j], z_lo), z_hi);
-                        if (EVEN || live >= 8) {
+                        if (EVEN || (live >= 8 && live_img)) {
 #pragma unroll
                             for (int j = 0; j < 4; ++j) fstat = max3_abs(fstat, z[2 * j], z[2 * j + 1]);
                         } else {
 #pragma unroll
                             for (int j = 0; j < 8; ++j)
-                                if (j < live) fstat = fmaxf(fstat, fabsf(z[j]));
+                                if (j < live && live_img) fstat = fmaxf(fstat, fabsf(z[j]));
                         }
                         if (!EVEN && p.probe) { __syncwarp(); continue; }
                         unsigned short* so = reinterpret_cast<unsigned short*>(stage_smem + stage + lane * 2);
@@ -684,24 +705,23 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap mapI0,
                         }
                         __syncwarp();
                         const uint4 w = *reinterpret_cast<const uint4*>(stage_smem + stage + lane * 16);
-                        if (EVEN || (scol < live && p.vec)) {
+                        if (EVEN || (scol < live && n_img > 0)) {
                             if (p.out_planes) {
-                                *reinterpret_cast<uint2*>(p.out_planes + at) =
+                                // (rows of the planes are padded to 16 images: all eight have a place)
+                                const OFF pat = EVEN ? at : poff_g + (OFF)c * ldc_p;
+                                *reinterpret_cast<uint2*>(p.out_planes + pat) =
                                     make_uint2(__byte_perm(w.x, w.y, 0x7531), __byte_perm(w.z, w.w, 0x7531));
-                                *reinterpret_cast<uint2*>(out_lo + at) =
+                                *reinterpret_cast<uint2*>(out_lo + pat) =
                                     make_uint2(__byte_perm(w.x, w.y, 0x6420), __byte_perm(w.z, w.w, 0x6420));
                             }
-                            if (p.write_i16) *reinterpret_cast<uint4*>((short*)p.O + at) = w;
-                        } else if (scol < live) {
-                            const unsigned v[4] = {w.x, w.y, w.z, w.w};
+                            if (EVEN || p.vec) {
+                                if (p.write_i16) *reinterpret_cast<uint4*>((short*)p.O + at) = w;
+                            } else if (p.write_i16) {
+                                const unsigned v[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll 1
-                            for (int j = 0; j < 8; ++j) {
-                                const unsigned m = (j & 4 ? (j & 2 ? v[3] : v[2]) : (j & 2 ? v[1] : v[0])) >> 16 * (j & 1);
-                                if (p.out_planes) {
-                                    p.out_planes[at + j] = (unsigned char)(m >> 8);
-                                    out_lo[at + j] = (unsigned char)m;
-                                }
-                                if (p.write_i16) ((short*)p.O)[at + j] = (short)m;
+                                for (int j = 0; j < 8 && j < n_img; ++j)
+                                    ((short*)p.O)[at + j] = (short)((j & 4 ? (j & 2 ? v[3] : v[2])
+                                                                           : (j & 2 ? v[1] : v[0])) >> 16 * (j & 1));
                             }
                         }
                     }
@@ -711,7 +731,7 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap mapI0,
                         c = start * 8;
                         // (a pixel in which this warp had no piece has fetched nothing ahead)
                         if (EPI == EPI_RESIDUAL && !ahead && inside && c < kt && (EVEN || c + scol < left))
-                            rq = load8(p.residual + off + (OFF)c * ldc, EVEN || p.vec);
+                            rq = load8(p.residual + off + (OFF)c * ldc, EVEN || p.vec, n_img);
                         ahead = false;
                     }
                 }
@@ -732,7 +752,7 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap mapI0,
                     tmem_ld16(lane_addr + 2 * bn + c0, ll);
                     tmem_ld_wait();
                     const int live = left - chan;
-                    if (!ok || !inside) continue;
+                    if (!ok || !inside || !live_img) continue;
                     short* out = (short*)p.O + off;
                     const long long fix = 128LL * (long long)(int)(s_hi * 256u + s_lo);
                     long long v[16];
@@ -851,23 +871,62 @@ split_same_layout_kernel(const T* __restrict__ src, long long n, void* __restric
     }
 }
 
+// the same into planes whose rows of n images are padded to np
+__global__ void __launch_bounds__(256)
+split_padded_kernel(const short* __restrict__ src, long long rows, int n, int np,
+                    unsigned char* __restrict__ plane0, unsigned char* __restrict__ plane1) {
+    const int g8 = np / 8;
+    const long long total = rows * g8, stride = (long long)gridDim.x * blockDim.x;
+    for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < total; v += stride) {
+        const long long row = v / g8;
+        const int i0 = (int)(v - row * g8) * 8;
+        const unsigned short* q = (const unsigned short*)src + row * n + i0;
+        unsigned w[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) w[j] = i0 + j < n ? q[j] : 0u;
+        uint2 h, l;
+        l.x = (w[0] & 0xff) | (w[1] & 0xff) << 8 | (w[2] & 0xff) << 16 | w[3] << 24;
+        l.y = (w[4] & 0xff) | (w[5] & 0xff) << 8 | (w[6] & 0xff) << 16 | w[7] << 24;
+        h.x = w[0] >> 8 | (w[1] >> 8) << 8 | (w[2] >> 8) << 16 | (w[3] >> 8) << 24;
+        h.y = w[4] >> 8 | (w[5] >> 8) << 8 | (w[6] >> 8) << 16 | (w[7] >> 8) << 24;
+        *(uint2*)(plane0 + row * np + i0) = h;
+        *(uint2*)(plane1 + row * np + i0) = l;
+    }
+}
+
+// int16 tensor [c][h][w][n] -> its two byte planes, the low one plane_bytes behind the high one
+int split_to_planes(const short* x, int c, int h, int w, int n, void* planes, size_t plane_bytes,
+                    cudaStream_t st) {
+    const int np = plane_pitch(n);
+    const long long rows = (long long)c * h * w, units = rows * np / 8;
+    long long blocks = (units + 255) / 256;
+    if (blocks > 148 * 16) blocks = 148 * 16;
+    unsigned char* lo = (unsigned char*)planes + plane_bytes;
+    if (np == n)
+        split_same_layout_kernel<short, MODE_FLEX16><<<(unsigned)blocks, 256, 0, st>>>(x, rows * n, planes, lo);
+    else
+        split_padded_kernel<<<(unsigned)blocks, 256, 0, st>>>(x, rows, n, np, (unsigned char*)planes, lo);
+    B2_CUDA(cudaGetLastError());
+    return B2_OK;
+}
+
 // filters C,R,S,K -> ONE array [ntn][2*bn rows][kp] for the implicit kernel: for every CTA column
 // the high bytes of its output channels (rows 0..bn-1) and, behind them, the low bytes minus 128 as
 // signed bytes (rows bn..2bn-1).  A tile covers gh x gw output pixels: row g*kt + k holds output
-// channel k as pixel g sees it, that is, shifted by (g/gw)*str_h, (g%gw)*str_w inside the common
-// window of wh x ww taps; row gh*gw*kt + g is pixel g's sum column: 0 in the high half, +1 in the
+// channel k as pixel g sees it inside the common window of wh x ww taps (forward: shifted by
+// (g/gw)*str_h, (g%gw)*str_w; input gradient: the taps of its own residue modulo the stride, flipped); row gh*gw*kt + g is pixel g's sum column: 0 in the high half, +1 in the
 // low half on the taps of its own R x S window.  Everything else -- taps of the common window that
 // are not the pixel's, channels beyond C, padding -- is zero in both halves, so it adds nothing
 // whatever the operand holds there.  The K positions of chunk cc start at cc*kc_pad and run over
 // (channel within the chunk, tap row, tap column).
 struct FilterLayout {
     int C, R, S, K, cu, cchunks, kc_pad, ntn, bn, kt, kp, gh, gw, str_h, str_w, wh, ww;
+    int bprop, off_h, off_w, pad_h, pad_w;
 };
 
 template <typename T>
 __global__ void __launch_bounds__(256)
-filter_planes_kernel(const T* __restrict__ F, const FilterLayout f, int bprop,
-                     unsigned char* __restrict__ planes) {
+filter_planes_kernel(const T* __restrict__ F, const FilterLayout f, unsigned char* __restrict__ planes) {
     const int total = f.ntn * 2 * f.bn * f.kp, G = f.gh * f.gw, RS = f.R * f.S;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
         const int kc = i % f.kp;
@@ -879,7 +938,9 @@ filter_planes_kernel(const T* __restrict__ F, const FilterLayout f, int bprop,
         const int th = tap / f.ww, tw = tap - th * f.ww;
         const bool sum_col = col >= G * f.kt;
         const int g = sum_col ? col - G * f.kt : col / f.kt, k = tile * f.kt + (sum_col ? 0 : col % f.kt);
-        const int r = th - g / f.gw * f.str_h, s = tw - g % f.gw * f.str_w, c = cc * f.cu + cl;
+        const int gy = g / f.gw, gx = g - gy * f.gw, c = cc * f.cu + cl;
+        const int r = f.bprop ? gy + f.pad_h - f.str_h * (f.off_h + th) : th - gy * f.str_h;
+        const int s = f.bprop ? gx + f.pad_w - f.str_w * (f.off_w + tw) : tw - gx * f.str_w;
         unsigned char v = 0;
         if (g < G && r >= 0 && r < f.R && s >= 0 && s < f.S && cl < f.cu && cc < f.cchunks && c < f.C &&
             k < f.K) {
@@ -887,10 +948,10 @@ filter_planes_kernel(const T* __restrict__ F, const FilterLayout f, int bprop,
                 v = low ? 1 : 0;
             } else {
                 // bprop: the filter tensor is that of the FORWARD convolution, [K outputs here =
-                // its input channels][R][S][C reduced here = its output channels], read flipped
+                // its input channels][R][S][C reduced here = its output channels]
                 const int at = r * f.S + s;
-                const int m = bprop ? (int)F[((long long)k * RS + (RS - 1 - at)) * f.C + c]
-                                    : (int)F[((long long)c * RS + at) * f.K + k];
+                const int m = f.bprop ? (int)F[((long long)k * RS + at) * f.C + c]
+                                      : (int)F[((long long)c * RS + at) * f.K + k];
                 const int lo = m & 0xff;
                 v = low ? (unsigned char)(lo ^ 0x80) : (unsigned char)(((m - lo) >> 8) & 0xff);
             }
@@ -902,7 +963,8 @@ filter_planes_kernel(const T* __restrict__ F, const FilterLayout f, int bprop,
 // int8 plane in C,H,W,N layout; box = [cu][wh][ww][128 images]
 int make_map_4d(CUtensorMap* map, void* base, const ConvGeom& g, int cu, int wh, int ww) {
     cuuint64_t dims[4] = {(cuuint64_t)g.N, (cuuint64_t)g.W, (cuuint64_t)g.H, (cuuint64_t)g.C};
-    cuuint64_t strides[3] = {(cuuint64_t)g.N, (cuuint64_t)g.W * g.N, (cuuint64_t)g.H * g.W * g.N};
+    const cuuint64_t np = plane_pitch(g.N);
+    cuuint64_t strides[3] = {np, (cuuint64_t)g.W * np, (cuuint64_t)g.H * g.W * np};
     cuuint32_t box[4] = {(cuuint32_t)kKBytes, (cuuint32_t)ww, (cuuint32_t)wh, (cuuint32_t)cu};
     cuuint32_t estr[4] = {1, 1, 1, 1};
     CUresult r = g_encode(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, base, dims, strides, box, estr,
@@ -914,29 +976,51 @@ int make_map_4d(CUtensorMap* map, void* base, const ConvGeom& g, int cu, int wh,
 
 struct ImplicitShape {
     int ntn, kt, bn, nbuf, tmem_cols, cu, cchunks, kc_pad, npanels, kp, nstages, smem;
-    int gh, gw, wh, ww, tiles;
+    int gh, gw, wh, ww, off_h, off_w, step_h, step_w, tiles;
     size_t act_plane, filt_bytes, bytes;
 };
+
+inline int floor_div(int a, int b) { return a >= 0 ? a / b : -((-a + b - 1) / b); }
+
+// One direction of a tile's window: output positions tile*g .. tile*g + g-1, filter extent r.
+//   forward:        input = out * str - pad + tap
+//   input gradient: error = (out + pad - tap) / str where that divides; g is a multiple of str, so every
+//                   tile has the same residues and steps g / str errors further
+inline void window(int bprop, int g, int r, int pad, int str, int* extent, int* off, int* step) {
+    if (!bprop) {
+        *extent = (g - 1) * str + r; *off = -pad; *step = g * str;
+    } else {
+        const int lo = -floor_div(-(pad - r + 1), str), hi = floor_div(g - 1 + pad, str);
+        *extent = hi - lo + 1 > 1 ? hi - lo + 1 : 1; *off = lo; *step = g / str;
+    }
+}
 
 // the shape with tiles of gh x gw output pixels; nstages < 2 where it does not fit
 ImplicitShape implicit_shape_for(const ConvGeom& g, int gh, int gw) {
     ImplicitShape s;
     s.gh = gh; s.gw = gw;
-    s.wh = (gh - 1) * g.str_h + g.R; s.ww = (gw - 1) * g.str_w + g.S;
+    window(g.bprop, gh, g.R, g.pad_h, g.str_h, &s.wh, &s.off_h, &s.step_h);
+    window(g.bprop, gw, g.S, g.pad_w, g.str_w, &s.ww, &s.off_w, &s.step_w);
     const int G = gh * gw, taps = s.wh * s.ww;
-    s.tiles = ((g.P + gh - 1) / gh) * ((g.Q + gw - 1) / gw) * (g.N / 128);
-    // output channels per CTA column: at most 127, so that with the sum columns the two filter
-    // planes make one operand of at most 256 rows
-    s.ntn = (g.K + 126) / 127;
-    s.kt = (g.K + s.ntn - 1) / s.ntn;
+    s.tiles = ((g.P + gh - 1) / gh) * ((g.Q + gw - 1) / gw) * image_blocks(g.N);
+    // output channels per CTA column: with the sum columns the two filter planes make one operand
+    // of at most 256 rows; in a tile of several pixels a multiple of 16 (no piece of columns
+    // straddles two pixels)
+    const int most = G == 1 ? 127 : (128 / G - 1) / 16 * 16;
+    if (G == 1) {
+        s.ntn = (g.K + most - 1) / most;
+        s.kt = (g.K + s.ntn - 1) / s.ntn;
+    } else {
+        s.kt = round_up(g.K, 16) < most ? round_up(g.K, 16) : most;
+        s.ntn = (g.K + s.kt - 1) / s.kt;
+    }
     s.bn = round_up(G * (s.kt + 1), 16);
     const int sets = 512 / (3 * s.bn);
     s.nbuf = sets >= 4 ? 4 : sets >= 3 ? 3 : sets >= 2 ? 2 : 1;
     s.tmem_cols = 32;
     while (s.tmem_cols < 3 * s.bn * s.nbuf) s.tmem_cols *= 2;
     // channels per chunk: about 36 KB for the two planes of a stage (a 3x3 chunk of 16 channels is
-    // 144 rows of 128 bytes), so that several stages are in flight; 1x1 filters on single pixels
-    // take up to 128 channels
+    // 144 rows of 128 bytes), so that several stages are in flight; 1x1 windows take up to 128 channels
     if (taps == 1) s.cu = g.C >= 128 ? 128 : round_up(g.C, 32);
     else s.cu = taps > 64 ? 2 : taps > 20 ? 4 : taps > 10 ? 8 : taps > 4 ? 16 : 32;
     s.cchunks = (g.C + s.cu - 1) / s.cu;
@@ -947,9 +1031,9 @@ ImplicitShape implicit_shape_for(const ConvGeom& g, int gh, int gw) {
     const int stage = 2 * s.kc_pad * 128;
     int nst = (kConvSmemMax - kConvSmemFixed - filt_smem) / stage;
     if (nst > kConvMaxStages) nst = kConvMaxStages;
-    s.nstages = s.bn > 128 || s.wh > 256 || s.ww > 256 ? 0 : nst;
+    s.nstages = s.bn > 128 || s.wh > 256 || s.ww > 256 || s.kt < 1 ? 0 : nst;
     s.smem = kConvSmemFixed + filt_smem + (nst > 0 ? nst : 0) * stage;
-    s.act_plane = (((size_t)g.C * g.H * g.W * g.N) + 1023) / 1024 * 1024;
+    s.act_plane = plane_size(g.C, g.H, g.W, g.N);
     s.filt_bytes = (((size_t)s.ntn * 2 * s.bn * s.kp) + 1023) / 1024 * 1024;
     s.bytes = 2 * s.act_plane + s.filt_bytes;
     return s;
@@ -973,14 +1057,21 @@ long long implicit_cost(const ImplicitShape& s) {
 // twelve narrow instructions and as many on waiting), and neighbouring pixels share most of their
 // window.  One pixel where the channels fill the operand, where a group would leave SMs without
 // a tile, or where the window grows too much (strides).
+//
+// The input gradient of a strided convolution needs tiles that are multiples of the stride: then every
+// pixel of a tile reads its own residue class of taps from the error tensor as it lies, without the
+// zeros that dilating it would put between its elements.
 ImplicitShape implicit_shape(const ConvGeom& g) {
-    ImplicitShape best = implicit_shape_for(g, 1, 1);
-    if (best.ntn > 1 || best.kt % 16 != 0) return best;
-    static const int cand[3][2] = {{1, 2}, {2, 1}, {2, 2}};
-    for (int i = 0; i < 3; ++i) {
-        const ImplicitShape s = implicit_shape_for(g, cand[i][0], cand[i][1]);
-        if (s.nstages >= 3 && s.bn <= 80 && implicit_cost(s) < implicit_cost(best)) best = s;
-    }
+    const int sh = g.bprop ? g.str_h : 1, sw = g.bprop ? g.str_w : 1;
+    ImplicitShape best = implicit_shape_for(g, sh, sw);
+    if (g.K % 16 != 0) return best;
+    for (int a = 1; a <= 2; ++a)
+        for (int b = 1; b <= 2; ++b) {
+            const int gh = sh * a, gw = sw * b;
+            if (a * b == 1 || gh * gw > 4 || gw == 3) continue;
+            const ImplicitShape s = implicit_shape_for(g, gh, gw);
+            if (s.nstages >= 3 && s.bn <= 80 && implicit_cost(s) < implicit_cost(best)) best = s;
+        }
     return best;
 }
 
@@ -989,104 +1080,45 @@ ImplicitShape implicit_shape(const ConvGeom& g) {
 // tensor core reads zeros.  fp32 convolutions therefore stay on the gather + K-major path, and so
 // do dilated filters and windows too large for two stages of shared memory.
 bool implicit_ok(int mode, const ConvGeom& g) {
-    if (mode != MODE_FLEX16 || g.N % 128 != 0 || g.dil_h != 1 || g.dil_w != 1) return false;
+    if (mode != MODE_FLEX16 || g.dil_h != 1 || g.dil_w != 1 || getenv("B2_CONV_IM2COL")) return false;
     if (!flat_depth(g)) return false;
-    if (g.R > 256 || g.S > 256 || (long long)g.P * g.Q * (g.N / 128) >= (1LL << 30)) return false;
+    if (g.R > 256 || g.S > 256 || (long long)g.P * g.Q * image_blocks(g.N) >= (1LL << 30)) return false;
+    if (g.bprop && (g.str_h * g.str_w > 4 || g.str_w == 3)) return false;
     // the exact int32 sums: |X| <= 2*128*255 per K row
     if ((long long)g.C * g.R * g.S + 32 > 32768) return false;
     return implicit_shape(g).nstages >= 2;
 }
 
-// The input gradient of a convolution is itself a unit-stride convolution: of the error tensor
-// (K channels, P x Q), with zeros put between its elements when the forward pass was strided,
-// with the filters flipped and transposed, padded by R-1-pad.  The dilated tensor is H+2pad-R+1
-// high (for unit stride that is P), so that the result is exactly H high.  Returns false where
-// this does not hold or does not pay (filter dilation, padding larger than the window allows,
-// strides whose zero-filling would multiply the work by more than four).
-bool bprop_as_fprop(const ConvGeom& f, ConvGeom* g) {
-    if (f.dil_h != 1 || f.dil_w != 1 || f.str_h * f.str_w > 4 || !flat_depth(f)) return false;
-    if (f.pad_h > f.R - 1 || f.pad_w > f.S - 1) return false;
-    const int he = f.H + 2 * f.pad_h - f.R + 1, we = f.W + 2 * f.pad_w - f.S + 1;
-    if (he < (f.P - 1) * f.str_h + 1 || we < (f.Q - 1) * f.str_w + 1) return false;
-    *g = f;
-    g->C = f.K; g->H = he; g->W = we; g->K = f.C; g->P = f.H; g->Q = f.W;
-    g->pad_h = f.R - 1 - f.pad_h; g->pad_w = f.S - 1 - f.pad_w;
-    g->str_h = g->str_w = 1;
-    g->up_h = f.str_h; g->up_w = f.str_w; g->src_h = f.P; g->src_w = f.Q;
-    return true;
-}
-
-// geometry of the implicit kernel for a pass (0 forward, 1 input gradient); false if unsupported
+// geometry of the implicit kernel for a pass (0 forward, 1 input gradient); false if unsupported.
+// The input gradient streams the error tensor (K channels, P x Q) and writes the input's shape.
 bool pass_geom(const ConvGeom& f, int pass, ConvGeom* g) {
-    if (pass == 0) { *g = f; return implicit_ok(MODE_FLEX16, f); }
-    return pass == 1 && bprop_as_fprop(f, g) && implicit_ok(MODE_FLEX16, *g);
-}
-
-// The three parts of an implicit-GEMM forward convolution: the two operand pre-passes (which a
-// caller can skip when it already holds the planes) and the tile kernel.
-// int16 tensor [C][src_h][src_w][N] -> the two byte planes of its zero-dilated form
-// [C][H][W][N]; eight images per thread (N is a multiple of 128 on this path).
-__global__ void __launch_bounds__(256)
-dilate_planes_kernel(const short* __restrict__ src, ConvGeom g, long long n8,
-                     void* __restrict__ plane0, void* __restrict__ plane1) {
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    const int nv = g.N / 8;
-    for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < n8; v += stride) {
-        const int n = (int)(v % nv);
-        long long r = v / nv;
-        const int w = (int)(r % g.W); r /= g.W;
-        const int h = (int)(r % g.H);
-        const int c = (int)(r / g.H);
-        const int sh = h / g.up_h, sw = w / g.up_w;
-        unsigned hi[2] = {0, 0}, lo[2] = {0, 0};
-        if (sh * g.up_h == h && sw * g.up_w == w && sh < g.src_h && sw < g.src_w) {
-            const long long at = (((long long)c * g.src_h + sh) * g.src_w + sw) * nv + n;
-            const int4 q = __ldcs(reinterpret_cast<const int4*>(src) + at);
-            const unsigned x[4] = {(unsigned)q.x, (unsigned)q.y, (unsigned)q.z, (unsigned)q.w};
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const unsigned l2 = __byte_perm(x[j], 0, 0x4420);   // low bytes of the two int16
-                const unsigned h2 = __byte_perm(x[j], 0, 0x4431);   // high bytes
-                lo[j >> 1] |= (l2 & 0xffffu) << (16 * (j & 1));
-                hi[j >> 1] |= (h2 & 0xffffu) << (16 * (j & 1));
-            }
-        }
-        reinterpret_cast<uint2*>(plane0)[v] = make_uint2(hi[0], hi[1]);
-        reinterpret_cast<uint2*>(plane1)[v] = make_uint2(lo[0], lo[1]);
+    *g = f;
+    if (pass == 1) {
+        g->bprop = 1;
+        g->C = f.K; g->H = f.P; g->W = f.Q; g->K = f.C; g->P = f.H; g->Q = f.W;
     }
+    return (pass == 0 || pass == 1) && implicit_ok(MODE_FLEX16, *g);
 }
 
+// The three parts of an implicit-GEMM convolution: the two operand pre-passes (which a caller can skip
+// when it already holds the planes) and the tile kernel.
 template <typename T, int MODE>
 int implicit_split_activations(const T* I, const ConvGeom& g, const ImplicitShape& s, void* planes,
                                cudaStream_t st) {
-    const long long n_act = (long long)g.C * g.H * g.W * g.N;
-    long long blocks = (n_act / 8 + 255) / 256;
-    if (blocks > 148 * 16) blocks = 148 * 16;
-    if (blocks < 1) blocks = 1;
-    if (g.up_h != 1 || g.up_w != 1 || g.src_h != g.H || g.src_w != g.W) {
-        B2_REQUIRE(MODE == MODE_FLEX16 && g.N % 8 == 0 && ((uintptr_t)I & 15) == 0,
-                   "the dilated planes need int16 data, 16-byte aligned, N a multiple of 8");
-        dilate_planes_kernel<<<(unsigned)blocks, 256, 0, st>>>(
-            (const short*)I, g, n_act / 8, planes, (unsigned char*)planes + s.act_plane);
-        B2_CUDA(cudaGetLastError());
-        return B2_OK;
-    }
-    split_same_layout_kernel<T, MODE><<<(unsigned)blocks, 256, 0, st>>>(
-        I, n_act, planes, (unsigned char*)planes + s.act_plane);
-    B2_CUDA(cudaGetLastError());
-    return B2_OK;
+    return split_to_planes((const short*)I, g.C, g.H, g.W, g.N, planes, s.act_plane, st);
 }
 
 template <typename T, int MODE>
 int implicit_filter_planes(const T* F, const ConvGeom& g, const ImplicitShape& s, void* planes,
-                           cudaStream_t st, int bprop = 0) {
+                           cudaStream_t st) {
     const long long n_f = (long long)s.ntn * 2 * s.bn * s.kp;
     B2_REQUIRE(n_f < (1LL << 30), "filter tensor too large");
     long long fb = (n_f + 255) / 256;
     if (fb > 148 * 8) fb = 148 * 8;
     const FilterLayout f = {g.C, g.R, g.S, g.K, s.cu, s.cchunks, s.kc_pad, s.ntn, s.bn, s.kt, s.kp,
-                            s.gh, s.gw, g.str_h, g.str_w, s.wh, s.ww};
-    filter_planes_kernel<T><<<(unsigned)fb, 256, 0, st>>>(F, f, bprop, (unsigned char*)planes);
+                            s.gh, s.gw, g.str_h, g.str_w, s.wh, s.ww,
+                            g.bprop, s.off_h, s.off_w, g.pad_h, g.pad_w};
+    filter_planes_kernel<T><<<(unsigned)fb, 256, 0, st>>>(F, f, (unsigned char*)planes);
     B2_CUDA(cudaGetLastError());
     return B2_OK;
 }
@@ -1106,15 +1138,17 @@ int implicit_tiles(const void* act_planes, const void* filt_planes, void* O, con
     if ((rc = make_map(&mB, (void*)filt_planes, s.ntn * 2 * s.bn, s.kp, 1, 2 * s.bn))) return rc;
     ConvTileParams p;
     p.P = g.P; p.Q = g.Q; p.N = g.N; p.K = g.K;
-    p.pad_h = g.pad_h; p.pad_w = g.pad_w; p.str_h = g.str_h; p.str_w = g.str_w;
+    p.off_h = s.off_h; p.off_w = s.off_w; p.step_h = s.step_h; p.step_w = s.step_w;
     p.cu = s.cu; p.cchunks = s.cchunks; p.kc_pad = s.kc_pad;
     p.box_bytes = s.cu * s.wh * s.ww * 128;
     p.gh = s.gh; p.gw = s.gw; p.tq = (g.Q + s.gw - 1) / s.gw;
+    p.gw_log = s.gw == 4 ? 2 : s.gw == 2 ? 1 : 0;
     p.npanels = s.npanels; p.nstages = s.nstages;
     p.bn = s.bn; p.kt = s.kt; p.nbuf = s.nbuf; p.tmem_cols = s.tmem_cols;
-    p.nblk = g.N / 128;
+    p.nblk = image_blocks(g.N);
     p.num_tiles = s.tiles;
     p.ldc = (long long)g.P * g.Q * g.N;
+    p.NP = plane_pitch(g.N); p.ldc_planes = (long long)g.P * g.Q * p.NP;
     p.O = O; p.table = table; p.slotA = slotI; p.slotB = slotF; p.slotC = slotO;
     p.stats = stats; p.probe_out = probe_out; p.status = status; p.probe = probe;
     p.vec = 0; p.bias = nullptr; p.residual = nullptr; p.slot_bias = p.slot_res = 0; p.relu = 0;
@@ -1130,8 +1164,9 @@ int implicit_tiles(const void* act_planes, const void* filt_planes, void* O, con
         p.write_i16 = epi->write_int16 ? 1 : 0;
         p.out_planes = (unsigned char*)epi->out_planes;
         p.out_plane_bytes = (long long)epi->plane_bytes;
+        B2_REQUIRE(!epi->out_planes || (epi->plane_bytes & 7) == 0, "planes alignment");
         p.vec = (((uintptr_t)epi->residual | (epi->write_int16 ? (uintptr_t)O : 0)) & 15) == 0 &&
-                (epi->plane_bytes & 7) == 0;
+                g.N % 8 == 0;
     }
     dim3 grid(p.num_tiles < 148 ? p.num_tiles : 148, s.ntn);
     // a CTA with one or two tiles has no use for more accumulator sets than tiles: with fewer
@@ -1164,8 +1199,9 @@ int implicit_tiles(const void* act_planes, const void* filt_planes, void* O, con
         conv_implicit_kernel<unsigned, EPI_RESIDUAL, true, true>};
     // per product |HH| <= 2^14 and |X| <= 2^14 + 2^15
     const bool short_sum = (long long)g.C * g.R * g.S * ((1 << 22) + (1 << 16)) < (1LL << 31);
-    const bool wide = (long long)g.K * p.ldc >= (1LL << 32);
-    const bool even = epi && !wide && !probe && p.vec && g.K % 8 == 0 && s.kt % 8 == 0;
+    const bool wide = (long long)g.K * p.ldc_planes >= (1LL << 32);
+    const bool even = epi && !wide && !probe && p.vec && g.N % 128 == 0 && g.K % 8 == 0 && s.kt % 8 == 0 &&
+                      g.K % s.kt == 0;
     const int tail = !epi ? EPI_INT : p.residual ? EPI_RESIDUAL : EPI_FUSED;
     const int which = even ? (short_sum ? 7 : 5) + tail : wide ? 3 + tail : tail;
     static bool attr_set = false;
@@ -1204,7 +1240,7 @@ int run_fprop(const T* I, const T* F, void* O, const b2_conv_dims* d, const b2_f
     int rc = geom_from(d, &g);
     if (rc) return rc;
     B2_REQUIRE(I && F && O, "null tensor");
-    if (implicit_ok(MODE, g) && !getenv("B2_CONV_IM2COL"))
+    if (implicit_ok(MODE, g))
         return run_fprop_implicit<T, MODE>(I, F, O, g, table, slotI, slotF, slotO, stats, scratch,
                                            scratch_bytes, probe_out, status, probe, st);
     const long long rows_ll = (long long)g.M * g.P * g.Q * g.N;
@@ -1371,14 +1407,14 @@ int run_bprop(const T* E, const T* F, void* GI, const b2_conv_dims* d, const b2_
     if (rc) return rc;
     B2_REQUIRE(E && F && GI, "null tensor");
     ConvGeom gb;
-    if (MODE == MODE_FLEX16 && pass_geom(g, 1, &gb) && !getenv("B2_CONV_IM2COL")) {
+    if (MODE == MODE_FLEX16 && pass_geom(g, 1, &gb)) {
         const ImplicitShape si = implicit_shape(gb);
         B2_REQUIRE(scratch && scratch_bytes >= si.bytes && ((uintptr_t)scratch & 1023) == 0,
                    "convolution bprop needs %zu bytes of 1024-byte aligned scratch, got %zu",
                    si.bytes, scratch_bytes);
         unsigned char* base = (unsigned char*)scratch;
         if ((rc = implicit_split_activations<T, MODE>(E, gb, si, base, st))) return rc;
-        if ((rc = implicit_filter_planes<T, MODE>(F, gb, si, base + 2 * si.act_plane, st, 1))) return rc;
+        if ((rc = implicit_filter_planes<T, MODE>(F, gb, si, base + 2 * si.act_plane, st))) return rc;
         return implicit_tiles(base, base + 2 * si.act_plane, GI, gb, si, table, slotE, slotF, slotG,
                               stats, probe_out, status, probe, st);
     }
@@ -1856,7 +1892,7 @@ extern "C" int b2_conv_filter_planes(const int16_t* F, const b2_conv_dims* d, in
     if (rc) return rc;
     B2_REQUIRE(F && planes && pass_geom(f, pass, &g), "planes are not available for this convolution");
     return implicit_filter_planes<short, MODE_FLEX16>(F, g, implicit_shape(g), planes,
-                                                      (cudaStream_t)stream, pass);
+                                                      (cudaStream_t)stream);
 }
 
 extern "C" int b2_conv_flex16_planes(int32_t pass, const void* act_planes,

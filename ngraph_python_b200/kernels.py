@@ -88,15 +88,10 @@ class _PlaneUser(object):
         self.filter_arg = filter_arg
         self.filter_bytes = filt_bytes
         self.in_views[filter_arg].buffer.watched = True
-        # the input gradient of a strided convolution streams the error tensor with zeros between
-        # its elements: planes of its own, written by one extra launch of this step
-        self.own_plane_bytes = 0
-        if conv_pass == lib.CONV_BPROP and (self.dims.str_h > 1 or self.dims.str_w > 1):
-            self.own_plane_bytes = act_bytes
-            self.launches = 2
-            return
         buf = self.in_views[stream_arg].buffer
         buf.plane_bytes = act_bytes
+        # (planes whose rows of images are padded are written by the convolutions only)
+        buf.plane_dense = self.dims.N % 16 == 0
         buf.plane_steps = getattr(buf, "plane_steps", []) + [self]
         self.launches = 1
 
@@ -105,10 +100,6 @@ class _PlaneUser(object):
             self.filter_planes = t.torch.zeros((self.filter_bytes + 1024,), dtype=t.torch.uint8,
                                                device=t.device)
             self.filter_ptr = self.filter_planes.data_ptr() + (-self.filter_planes.data_ptr()) % 1024
-            if self.own_plane_bytes:
-                self.own_planes = t.torch.zeros((2 * self.own_plane_bytes + 1024,),
-                                                dtype=t.torch.uint8, device=t.device)
-                self.own_planes_ptr = self.own_planes.data_ptr() + (-self.own_planes.data_ptr()) % 1024
 
     def _build_filter_planes(self, t):
         fv = self.in_views[self.filter_arg]
@@ -132,8 +123,8 @@ class _PlaneUser(object):
         raw = lib.raw()
         st = t.stream.cuda_stream
         xbuf, fbuf = xv.buffer, fv.buffer
-        planes_ptr = self.own_planes_ptr if self.own_plane_bytes else xbuf.planes_ptr
-        if self.own_plane_bytes or not xbuf.planes_by_producer:
+        planes_ptr = xbuf.planes_ptr
+        if not xbuf.planes_by_producer:
             lib.check(raw.b2_conv_split_activations(self._ptr(xv), C.byref(self.dims),
                                                     self.conv_pass, planes_ptr, st))
             t.kernel_launches += 1

@@ -1356,7 +1356,8 @@ class _Planner(object):
             else:
                 d["reg"] = reg[m]
                 buf = v.buffer
-                wants = (buf.flex and buf.plane_bytes > 0 and not isinstance(m, AssignOp) and
+                wants = (buf.flex and buf.plane_bytes > 0 and getattr(buf, "plane_dense", True) and
+                         not isinstance(m, AssignOp) and
                          v.is_dense() and len(outs) + len(red_outs) + 2 <= fusion.MAX_OUT)
                 if wants:
                     # the convolutions that read this tensor take it as two byte planes: write
