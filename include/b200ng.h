@@ -324,6 +324,8 @@ typedef struct b2_conv_epilogue {
     int32_t relu;
     int32_t write_int16;
     void* out_planes;        size_t plane_bytes;
+    const int16_t* mask;     /* int16 tensor in the output's layout: y = mask > 0 ? y : 0 (the
+                              * gradient of a ReLU, taken from its activation); NULL = absent */
 } b2_conv_epilogue;
 int b2_conv_flex16_planes_fused(int32_t pass, const void* act_planes, const void* filter_planes,
                                 int16_t* out, const b2_conv_dims* d, const b2_flex_scale* table,

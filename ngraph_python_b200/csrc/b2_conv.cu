@@ -239,6 +239,7 @@ struct ConvTileParams {
     // convolution reads
     const short* bias; int slot_bias;
     const short* residual; int slot_res;      // same K,P,Q,N layout as the output
+    const short* mask;                        // likewise: y = mask > 0 ? y : 0
     int relu;
     int write_i16;
     int vec;                      // int16 tensors aligned for eight images at a time
@@ -275,12 +276,6 @@ __device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigne
     asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
     return r;
 }
-// max(m, |a|, |b|)
-__device__ __forceinline__ float max3_abs(float m, float a, float b) {
-    float r;
-    asm("max.abs.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(m), "f"(a), "f"(b));
-    return r;
-}
 // eight consecutive int16, as one load where the alignment allows it; only the first n exist
 __device__ __forceinline__ uint4 load8(const short* p, int vec, int n) {
     if (n <= 0) return make_uint4(0, 0, 0, 0);
@@ -313,12 +308,12 @@ constexpr int kConvSmemMax = 232448;        // 227 KB: the most one CTA can have
 constexpr int kConvSmemFixed = 1024 /*alignment*/ + 1024 /*barriers, bias*/ + 16 * 1024 /*epilogue staging*/;
 
 // OFF: 32-bit element offsets into the output where they reach, 64-bit ones for larger tensors.
-// EPI: 0 plain integer rescale, 1 fused tail, 2 fused tail with a residual.  SHORT: 256*HH + X fits 32
-// bits.  EVEN: eight images and eight channels at a time throughout -- aligned tensors, channel
+// EPI: 0 plain integer rescale, 1 fused tail, 2 fused tail with a residual.  MASK: the result is kept
+// where another tensor is positive (the gradient of a ReLU).  SHORT: 256*HH + X fits 32 bits.  EVEN: eight images and eight channels at a time throughout -- aligned tensors, channel
 // counts that are multiples of eight -- and not a measuring launch.  (Template parameters because a tested-and-skipped block of the epilogue is not free: the
 // compiler predicates it, and its instructions are issued all the same -- 60 of 330 per piece.)
 enum { EPI_INT = 0, EPI_FUSED = 1, EPI_RESIDUAL = 2 };
-template <typename OFF, int EPI, bool SHORT, bool EVEN>
+template <typename OFF, int EPI, bool SHORT, bool EVEN, bool MASK>
 __global__ void __launch_bounds__(kConvThreads, 1)
 conv_implicit_kernel(const __grid_constant__ CUtensorMap mapI0,
                      const __grid_constant__ CUtensorMap mapI1,
@@ -562,6 +557,10 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap mapI0,
         unsigned char* const stage_smem = epi_smem + (warp - 2) * 1024;
         unsigned stage = 0;
         const int epi_mask = epi_w - 1, kt8 = (kt + 7) >> 3 & epi_mask;
+        // plain rescale in 32-bit pieces: where the sums fit and the shift takes at least the low byte
+        const bool exact32 = EPI == EPI_INT && SHORT && !p.probe && sh >= 9 && sh <= 38;
+        const unsigned rmask8 = exact32 ? (1u << (sh - 8)) - 1u : 0u, rhalf8 = exact32 ? 1u << (sh - 9) : 0u;
+        unsigned smx = 0, smn = 0;                             // packed pairs: largest and smallest mantissa
         const bool probing = !EVEN && p.probe;
         const float z_lo = p.relu ? 0.0f : (probing ? -INFINITY : -32768.0f),
                     z_hi = probing ? INFINITY : 32767.0f;
@@ -584,21 +583,26 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap mapI0,
             // the eight that it loads and stores exist
             const bool live_img = EVEN || nb * 128 + quarter * 32 + lane < p.N;
             const int n_img = EVEN ? 8 : p.N - (nb * 128 + simg);
-            if (EPI != EPI_INT) {
-                // fp32 epilogue: the exact integer sum scaled to a real value, bias and residual
-                // added, ReLU, ONE quantisation with the output's exponent.  Eight columns at a
-                // time, loads first, then arithmetic, then stores: eight independent chains.  The
-                // warps that share a lane quarter take the 8-column pieces in turn.
-                // Instruction issue bounds it, so choices are made once per pixel or piece, sums
-                // are formed two at a time (fma.f32x2), and addresses once per pixel.
-                uint4 rq = make_uint4(0, 0, 0, 0);
+            if (EPI != EPI_INT || exact32) {
+                // Eight columns at a time, loads first, then arithmetic, then stores: eight independent
+                // chains.  The warps that share a lane quarter take the 8-column pieces in turn.
+                //   fused: the exact integer sum scaled to a real value in fp32, bias and residual added,
+                //   ReLU, ONE quantisation with the output's exponent; sums two at a time (fma.f32x2);
+                //   plain: the exact sum in 32-bit halves, rescaled with round to nearest even.
+                // Instruction issue bounds it, so choices are made once per pixel or piece, addresses
+                // once per pixel, and the statistic is taken on packed pairs.
+                uint4 rq = make_uint4(0, 0, 0, 0), mq = make_uint4(0, 0, 0, 0);
+                // residual and mask of a piece, fetched one piece ahead of its use
+                auto fetch = [&](OFF at) {
+                    if (EPI == EPI_RESIDUAL) rq = load8(p.residual + at, EVEN || p.vec, n_img);
+                    if (MASK) mq = load8(p.mask + at, EVEN || p.vec, n_img);
+                };
+                constexpr bool AHEAD = EPI == EPI_RESIDUAL || MASK;
                 OFF off;
                 bool inside = pixel(0, off);
                 off += (OFF)(ncol0 + scol) * ldc + (OFF)simg;
-                // the residual of the first piece is fetched while the tile is being multiplied
                 int c = (part & epi_mask) * 8;
-                if (EPI == EPI_RESIDUAL && inside && c < kt && (EVEN || c + scol < left))
-                    rq = load8(p.residual + off + (OFF)c * ldc, EVEN || p.vec, n_img);
+                if (AHEAD && inside && c < kt && (EVEN || c + scol < left)) fetch(off + (OFF)c * ldc);
                 if (ok && !mbar_wait(&tmem_full[buf], full_parity)) { atomicExch(fail_flag, 1); ok = false; }
                 tc_fence_after();
                 const unsigned lane_addr = tmem_base + buf * acc_cols + ((unsigned)(quarter * 32) << 16);
@@ -609,7 +613,8 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap mapI0,
                     const unsigned s_hi = tmem_ld1(lane_addr + bn + ncols + g);
                     const unsigned s_lo = tmem_ld1(lane_addr + 2 * bn + ncols + g);
                     tmem_ld_wait();
-                    const float fixf = 128.0f * (float)(int)(s_hi * 256u + s_lo);
+                    const int act_sum = (int)(s_hi * 256u + s_lo);
+                    const float fixf = 128.0f * (float)act_sum;
                     const unsigned long long fix2 = pack2(fixf, fixf);
                     const unsigned col0 = lane_addr + g * kt;
                     const bool here = inside && ok;
@@ -623,11 +628,12 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap mapI0,
                         const int live = left - c;
                         const OFF at = at_g + (OFF)c * ldc;
                         unsigned long long y[4];
-                        {
+                        if (EPI != EPI_INT) {
                             const ulonglong2 b0 = *reinterpret_cast<const ulonglong2*>(bias_s + c);
                             const ulonglong2 b1 = *reinterpret_cast<const ulonglong2*>(bias_s + c + 4);
                             y[0] = b0.x; y[1] = b0.y; y[2] = b1.x; y[3] = b1.y;
                         }
+                        const uint4 m_now = mq;
                         stage ^= 512;
                         if (EPI == EPI_RESIDUAL) {
                             *reinterpret_cast<uint4*>(stage_smem + stage + lane * 16) = rq;
@@ -637,7 +643,8 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap mapI0,
                             for (int j = 0; j < 4; ++j)
                                 y[j] = fma2(pack2((float)rs[64 * j], (float)rs[64 * j + 32]), s_res2, y[j]);
                             stage ^= 512;
-                            // the residual of the next piece, one piece ahead of its use
+                        }
+                        if (AHEAD) {
                             int cn = c + 8 * epi_w;
                             OFF offn = at_g;
                             const OFF keep = poff;
@@ -649,64 +656,96 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap mapI0,
                                 ahead = true;
                             }
                             poff = keep;
-                            if (in && cn < kt && (EVEN || cn + scol < left))
-                                rq = load8(p.residual + offn + (OFF)cn * ldc, EVEN || p.vec, n_img);
+                            if (in && cn < kt && (EVEN || cn + scol < left)) fetch(offn + (OFF)cn * ldc);
                         }
                         tmem_ld_wait();
                         if (!here) continue;
-                        if (SHORT) {
-                            // 256*HH + X fits 32 bits: two conversions a value instead of three
-#pragma unroll
-                            for (int j = 0; j < 4; ++j) {
-                                const unsigned long long t =
-                                    pack2((float)(int)((hh[2 * j] << 8) + xx[2 * j]),
-                                          (float)(int)((hh[2 * j + 1] << 8) + xx[2 * j + 1]));
-                                const unsigned long long l =
-                                    add2(pack2((float)(int)ll[2 * j], (float)(int)ll[2 * j + 1]), fix2);
-                                y[j] = fma2(fma2(t, k256, l), f_conv2, y[j]);
-                            }
-                        } else {
-                            // correctly rounded conversions instead of a 64-bit sum: the fp32
-                            // result is quantised to 16 bits right after
-#pragma unroll
-                            for (int j = 0; j < 4; ++j) {
-                                const unsigned long long l =
-                                    add2(pack2((float)(int)ll[2 * j], (float)(int)ll[2 * j + 1]), fix2);
-                                const unsigned long long x =
-                                    fma2(pack2((float)(int)xx[2 * j], (float)(int)xx[2 * j + 1]), k256, l);
-                                const unsigned long long h = pack2((float)(int)hh[2 * j], (float)(int)hh[2 * j + 1]);
-                                y[j] = fma2(fma2(h, k65536, x), f_conv2, y[j]);
-                            }
-                        }
-                        // in units of the output's step (see f_conv): ReLU and clamp, round to
-                        // nearest even by the magic-number add; the low 16 bits of the sum are the
-                        // mantissa.  (No NaN can arise: every term is finite.)
-                        float z[8];
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) unpack2(y[j], z[2 * j], z[2 * j + 1]);
-#pragma unroll
-                        for (int j = 0; j < 8; ++j) z[j] = fminf(fmaxf(z[j], z_lo), z_hi);
-                        if (EVEN || (live >= 8 && live_img)) {
-#pragma unroll
-                            for (int j = 0; j < 4; ++j) fstat = max3_abs(fstat, z[2 * j], z[2 * j + 1]);
-                        } else {
-#pragma unroll
-                            for (int j = 0; j < 8; ++j)
-                                if (j < live && live_img) fstat = fmaxf(fstat, fabsf(z[j]));
-                        }
-                        if (!EVEN && p.probe) { __syncwarp(); continue; }
                         unsigned short* so = reinterpret_cast<unsigned short*>(stage_smem + stage + lane * 2);
+                        if (EPI == EPI_INT) {
+                            // w = floor(sum / 256), r = sum mod 256; q = w / 2^(sh-8) to nearest, ties
+                            // (r = 0) to even
+                            const int fix = 128 * act_sum;
 #pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            float a, b;
-                            unpack2(add2(pack2(z[2 * j], z[2 * j + 1]), kmagic), a, b);
-                            so[64 * j] = (unsigned short)__float_as_uint(a);
-                            so[64 * j + 32] = (unsigned short)__float_as_uint(b);
+                            for (int j = 0; j < 8; ++j) {
+                                const int l = (int)ll[j] + fix, w = (int)(hh[j] << 8) + (int)xx[j] + (l >> 8);
+                                const unsigned rem = (unsigned)w & rmask8;
+                                int q = w >> (sh - 8);
+                                const unsigned odd = (unsigned)q & 1u;
+                                q += (rem > rhalf8 || (rem == rhalf8 && (odd | ((unsigned)l & 255u)))) ? 1 : 0;
+                                so[32 * j] = (unsigned short)max(-32768, min(32767, q));
+                            }
+                        } else {
+                            if (SHORT) {
+                                // 256*HH + X fits 32 bits: two conversions a value instead of three
+#pragma unroll
+                                for (int j = 0; j < 4; ++j) {
+                                    const unsigned long long t =
+                                        pack2((float)(int)((hh[2 * j] << 8) + xx[2 * j]),
+                                              (float)(int)((hh[2 * j + 1] << 8) + xx[2 * j + 1]));
+                                    const unsigned long long l =
+                                        add2(pack2((float)(int)ll[2 * j], (float)(int)ll[2 * j + 1]), fix2);
+                                    y[j] = fma2(fma2(t, k256, l), f_conv2, y[j]);
+                                }
+                            } else {
+                                // correctly rounded conversions instead of a 64-bit sum: the fp32
+                                // result is quantised to 16 bits right after
+#pragma unroll
+                                for (int j = 0; j < 4; ++j) {
+                                    const unsigned long long l =
+                                        add2(pack2((float)(int)ll[2 * j], (float)(int)ll[2 * j + 1]), fix2);
+                                    const unsigned long long x =
+                                        fma2(pack2((float)(int)xx[2 * j], (float)(int)xx[2 * j + 1]), k256, l);
+                                    const unsigned long long h = pack2((float)(int)hh[2 * j], (float)(int)hh[2 * j + 1]);
+                                    y[j] = fma2(fma2(h, k65536, x), f_conv2, y[j]);
+                                }
+                            }
+                            // in units of the output's step (see f_conv): ReLU and clamp, round to
+                            // nearest even by the magic-number add; the low 16 bits of the sum are the
+                            // mantissa.  (No NaN can arise: every term is finite.)
+                            float z[8];
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) unpack2(y[j], z[2 * j], z[2 * j + 1]);
+#pragma unroll
+                            for (int j = 0; j < 8; ++j) z[j] = fminf(fmaxf(z[j], z_lo), z_hi);
+                            if (!EVEN && p.probe) {
+                                // the largest |value| (kept where the mask is positive)
+                                if (MASK) {
+                                    *reinterpret_cast<uint4*>(stage_smem + stage + lane * 16) = m_now;
+                                    __syncwarp();
+#pragma unroll
+                                    for (int j = 0; j < 8; ++j) z[j] = (short)so[32 * j] > 0 ? z[j] : 0.0f;
+                                }
+#pragma unroll
+                                for (int j = 0; j < 8; ++j)
+                                    if (j < live && live_img) fstat = fmaxf(fstat, fabsf(z[j]));
+                                __syncwarp();
+                                continue;
+                            }
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) {
+                                float a, b;
+                                unpack2(add2(pack2(z[2 * j], z[2 * j + 1]), kmagic), a, b);
+                                so[64 * j] = (unsigned short)__float_as_uint(a);
+                                so[64 * j + 32] = (unsigned short)__float_as_uint(b);
+                            }
                         }
                         __syncwarp();
-                        const uint4 w = *reinterpret_cast<const uint4*>(stage_smem + stage + lane * 16);
+                        uint4 w = *reinterpret_cast<const uint4*>(stage_smem + stage + lane * 16);
+                        if (MASK) {
+                            w.x &= __vcmpgts2(m_now.x, 0u); w.y &= __vcmpgts2(m_now.y, 0u);
+                            w.z &= __vcmpgts2(m_now.z, 0u); w.w &= __vcmpgts2(m_now.w, 0u);
+                        }
                         if (EVEN || (scol < live && n_img > 0)) {
-                            if (p.out_planes) {
+                            if (!EVEN && n_img < 8) {
+                                // images beyond the batch count for nothing
+                                unsigned* v = reinterpret_cast<unsigned*>(&w);
+#pragma unroll
+                                for (int j = 0; j < 4; ++j)
+                                    v[j] &= (2 * j < n_img ? 0xffffu : 0u) | (2 * j + 1 < n_img ? 0xffff0000u : 0u);
+                            }
+                            smx = __vmaxs2(__vmaxs2(smx, w.x), __vmaxs2(__vmaxs2(w.y, w.z), w.w));
+                            smn = __vmins2(__vmins2(smn, w.x), __vmins2(__vmins2(w.y, w.z), w.w));
+                            if (EPI != EPI_INT && p.out_planes) {
                                 // (rows of the planes are padded to 16 images: all eight have a place)
                                 const OFF pat = EVEN ? at : poff_g + (OFF)c * ldc_p;
                                 *reinterpret_cast<uint2*>(p.out_planes + pat) =
@@ -715,8 +754,8 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap mapI0,
                                     make_uint2(__byte_perm(w.x, w.y, 0x6420), __byte_perm(w.z, w.w, 0x6420));
                             }
                             if (EVEN || p.vec) {
-                                if (p.write_i16) *reinterpret_cast<uint4*>((short*)p.O + at) = w;
-                            } else if (p.write_i16) {
+                                if (EPI == EPI_INT || p.write_i16) *reinterpret_cast<uint4*>((short*)p.O + at) = w;
+                            } else if (EPI == EPI_INT || p.write_i16) {
                                 const unsigned v[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll 1
                                 for (int j = 0; j < 8 && j < n_img; ++j)
@@ -730,8 +769,8 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap mapI0,
                         off += (OFF)(ncol0 + scol) * ldc + (OFF)simg;
                         c = start * 8;
                         // (a pixel in which this warp had no piece has fetched nothing ahead)
-                        if (EPI == EPI_RESIDUAL && !ahead && inside && c < kt && (EVEN || c + scol < left))
-                            rq = load8(p.residual + off + (OFF)c * ldc, EVEN || p.vec, n_img);
+                        if (AHEAD && !ahead && inside && c < kt && (EVEN || c + scol < left))
+                            fetch(off + (OFF)c * ldc);
                         ahead = false;
                     }
                 }
@@ -808,9 +847,8 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap mapI0,
             }
             if (lane == 0 && pmax) atomicMax(p.probe_out, pmax);
         } else {
-            // fused epilogue: the largest |value| before rounding (rounding is monotonic)
-            const int fs = (int)rintf(fstat);
-            stat = fs > stat ? fs : stat;
+            const int hi = max((int)(short)smx, (int)smx >> 16), lo = min((int)(short)smn, (int)smn >> 16);
+            stat = max(stat, max(hi, -lo));
             for (int o = 16; o > 0; o >>= 1) {
                 const int t = __shfl_xor_sync(0xffffffffu, stat, o);
                 stat = t > stat ? t : stat;
@@ -1151,7 +1189,8 @@ int implicit_tiles(const void* act_planes, const void* filt_planes, void* O, con
     p.NP = plane_pitch(g.N); p.ldc_planes = (long long)g.P * g.Q * p.NP;
     p.O = O; p.table = table; p.slotA = slotI; p.slotB = slotF; p.slotC = slotO;
     p.stats = stats; p.probe_out = probe_out; p.status = status; p.probe = probe;
-    p.vec = 0; p.bias = nullptr; p.residual = nullptr; p.slot_bias = p.slot_res = 0; p.relu = 0;
+    p.vec = ((uintptr_t)O & 15) == 0 && g.N % 8 == 0; p.mask = nullptr;
+    p.bias = nullptr; p.residual = nullptr; p.slot_bias = p.slot_res = 0; p.relu = 0;
     p.write_i16 = 1; p.out_planes = nullptr; p.out_plane_bytes = 0;
     if (epi) {
         B2_REQUIRE(!epi->bias || epi->slot_bias >= 0, "bias needs its scale slot");
@@ -1160,12 +1199,13 @@ int implicit_tiles(const void* act_planes, const void* filt_planes, void* O, con
         B2_REQUIRE(!epi->out_planes || ((uintptr_t)epi->out_planes & 15) == 0, "planes alignment");
         p.bias = epi->bias; p.slot_bias = epi->slot_bias;
         p.residual = epi->residual; p.slot_res = epi->slot_residual;
+        p.mask = epi->mask;
         p.relu = epi->relu ? 1 : 0;
         p.write_i16 = epi->write_int16 ? 1 : 0;
         p.out_planes = (unsigned char*)epi->out_planes;
         p.out_plane_bytes = (long long)epi->plane_bytes;
         B2_REQUIRE(!epi->out_planes || (epi->plane_bytes & 7) == 0, "planes alignment");
-        p.vec = (((uintptr_t)epi->residual | (epi->write_int16 ? (uintptr_t)O : 0)) & 15) == 0 &&
+        p.vec = (((uintptr_t)epi->residual | (uintptr_t)epi->mask | (epi->write_int16 ? (uintptr_t)O : 0)) & 15) == 0 &&
                 g.N % 8 == 0;
     }
     dim3 grid(p.num_tiles < 148 ? p.num_tiles : 148, s.ntn);
@@ -1186,24 +1226,27 @@ int implicit_tiles(const void* act_planes, const void* filt_planes, void* O, con
     cfg.attrs = attr; cfg.numAttrs = getenv("B2_CONV_NO_PDL") ? 0 : 1;
     typedef void (*Kernel)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const ConvTileParams);
     typedef unsigned long long U64;
+#define B2_TAILS(OFF, SHORT, EVEN)                                                               \
+    conv_implicit_kernel<OFF, EPI_FUSED, SHORT, EVEN, false>,                                    \
+        conv_implicit_kernel<OFF, EPI_RESIDUAL, SHORT, EVEN, false>,                             \
+        conv_implicit_kernel<OFF, EPI_FUSED, SHORT, EVEN, true>,                                 \
+        conv_implicit_kernel<OFF, EPI_RESIDUAL, SHORT, EVEN, true>
     static const Kernel kernels[] = {
-        conv_implicit_kernel<unsigned, EPI_INT, false, false>,
-        conv_implicit_kernel<unsigned, EPI_FUSED, false, false>,
-        conv_implicit_kernel<unsigned, EPI_RESIDUAL, false, false>,
-        conv_implicit_kernel<U64, EPI_INT, false, false>,
-        conv_implicit_kernel<U64, EPI_FUSED, false, false>,
-        conv_implicit_kernel<U64, EPI_RESIDUAL, false, false>,
-        conv_implicit_kernel<unsigned, EPI_FUSED, false, true>,
-        conv_implicit_kernel<unsigned, EPI_RESIDUAL, false, true>,
-        conv_implicit_kernel<unsigned, EPI_FUSED, true, true>,
-        conv_implicit_kernel<unsigned, EPI_RESIDUAL, true, true>};
+        conv_implicit_kernel<unsigned, EPI_INT, false, false, false>,
+        conv_implicit_kernel<unsigned, EPI_INT, true, false, false>,
+        conv_implicit_kernel<unsigned, EPI_INT, true, true, false>,
+        conv_implicit_kernel<U64, EPI_INT, false, false, false>,
+        B2_TAILS(unsigned, false, false), B2_TAILS(unsigned, false, true), B2_TAILS(unsigned, true, true),
+        B2_TAILS(U64, false, false)};
+#undef B2_TAILS
     // per product |HH| <= 2^14 and |X| <= 2^14 + 2^15
     const bool short_sum = (long long)g.C * g.R * g.S * ((1 << 22) + (1 << 16)) < (1LL << 31);
     const bool wide = (long long)g.K * p.ldc_planes >= (1LL << 32);
-    const bool even = epi && !wide && !probe && p.vec && g.N % 128 == 0 && g.K % 8 == 0 && s.kt % 8 == 0 &&
+    const bool even = !wide && !probe && p.vec && g.N % 128 == 0 && g.K % 8 == 0 && s.kt % 8 == 0 &&
                       g.K % s.kt == 0;
-    const int tail = !epi ? EPI_INT : p.residual ? EPI_RESIDUAL : EPI_FUSED;
-    const int which = even ? (short_sum ? 7 : 5) + tail : wide ? 3 + tail : tail;
+    const int tail = (p.mask ? 2 : 0) + (p.residual ? 1 : 0);
+    const int which = !epi ? (wide ? 3 : !short_sum ? 0 : even ? 2 : 1)
+                           : wide ? 16 + tail : !even ? 4 + tail : short_sum ? 12 + tail : 8 + tail;
     static bool attr_set = false;
     if (!attr_set) {
         for (size_t i = 0; i < sizeof(kernels) / sizeof(kernels[0]); ++i)

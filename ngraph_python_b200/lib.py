@@ -46,7 +46,7 @@ class ConvEpilogue(C.Structure):
     _fields_ = [("bias", C.c_void_p), ("slot_bias", C.c_int32),
                 ("residual", C.c_void_p), ("slot_residual", C.c_int32),
                 ("relu", C.c_int32), ("write_int16", C.c_int32),
-                ("out_planes", C.c_void_p), ("plane_bytes", C.c_size_t)]
+                ("out_planes", C.c_void_p), ("plane_bytes", C.c_size_t), ("mask", C.c_void_p)]
 
 
 class EwProgram(C.Structure):
