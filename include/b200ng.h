@@ -282,6 +282,14 @@ int b2_conv_fprop_scratch_bytes(int32_t flex, const b2_conv_dims* d, size_t* byt
 /* fp32 (3xTF32 on the tensor cores). */
 int b2_conv_fprop_f32(const float* I, const float* F, float* O, const b2_conv_dims* d,
                       void* scratch, size_t scratch_bytes, int32_t* status, void* stream);
+/* Kernels that the scratch-based entry points launch for a pass (0 forward, 1 input gradient, 2 filter
+ * gradient); 1: the operands are gathered and converted inside the product, no scratch needed. */
+int b2_conv_launches(int32_t flex, const b2_conv_dims* d, int32_t pass, int32_t* launches);
+/* With the layer's tail, where b2_conv_launches(0, d, 0) is 1: y = relu?(conv + bias[k] + residual);
+ * bias (K values) and residual (the output's layout) may be NULL. */
+int b2_conv_fprop_f32_fused(const float* I, const float* F, float* O, const b2_conv_dims* d,
+                            const float* bias, const float* residual, int32_t relu, int32_t* status,
+                            void* stream);
 /* flex16: exact integer sums, rescale/saturate/statistic as b2_gemm_flex16; probe as there. */
 int b2_conv_fprop_flex16(const int16_t* I, const int16_t* F, int16_t* O, const b2_conv_dims* d,
                          const b2_flex_scale* table, int32_t slotI, int32_t slotF, int32_t slotO,
@@ -291,11 +299,12 @@ int b2_conv_fprop_flex16(const int16_t* I, const int16_t* F, int16_t* O, const b
  * reads its streamed tensor (pass 0: the activations I; pass 1, the input gradient of a
  * convolution: the error tensor E) and the filters as byte planes -- high and low
  * bytes of the int16 mantissas, the streamed tensor in its own C,H,W,N (K,P,Q,N) order, every row
- * of N images padded to a multiple of 16 bytes, the low plane act_plane_bytes after the high
- * plane, 1024-byte aligned.  A fused elementwise kernel
+ * of N images padded to a multiple of 16 bytes, the low plane after the high plane at the next
+ * multiple of 1024 bytes, 1024-byte aligned; act_plane_bytes is the room to reserve for each.  A fused elementwise kernel
  * can emit such planes directly (B2_FLEX16_PLANES) and the filter planes of constant weights can
  * be built once, which leaves ONE launch per convolution.  `supported` is 0 where the plane path
- * does not apply (dilation, very large windows; pass 1: strides whose product exceeds 4);
+ * does not apply (dilation, very large windows; pass 1: strides whose product exceeds 4, strides
+ * with a batch that is no multiple of 128);
  * use b2_conv_fprop_flex16 / b2_conv_bprop_flex16 there.  `d` always describes the FORWARD
  * convolution.  No counterpart in the reference, whose kernels read int16 tensors directly. */
 enum b2_conv_pass { B2_CONV_FPROP = 0, B2_CONV_BPROP = 1 };

@@ -30,6 +30,7 @@
 //           kernel (deterministic, and exact for flex16: every slice is an exact integer).
 #include <cstdlib>
 
+#include "b2_direct.h"
 #include "b2_gemm_impl.cuh"
 
 namespace {
@@ -71,6 +72,47 @@ int geom_from(const b2_conv_dims* d, ConvGeom* g) {
 
 inline bool flat_depth(const ConvGeom& g) {
     return g.D == 1 && g.T == 1 && g.M == 1 && g.pad_d == 0;
+}
+
+// Whether a pass (0 forward, 1 input gradient) goes through the kernel that gathers and converts its
+// operands on the way into shared memory (b2_direct.cuh), and its arguments without the tensors.  It
+// does what the gather + GEMM path does, with one launch and without writing the unrolled planes
+// (8 bytes for each of the R*S copies of a value, and reading them again); the planes pay only where a
+// long list of output channels would have the gather repeated for every 128 of them.
+inline bool conv_goes_direct(int mode, const ConvGeom& g, int pass, b2_direct_args* out) {
+    if (!flat_depth(g) || getenv("B2_CONV_IM2COL")) return false;
+    const long long rows = pass ? (long long)g.H * g.W * g.N : (long long)g.P * g.Q * g.N;
+    const long long k = (long long)(pass ? g.K : g.C) * g.R * g.S;
+    if (rows >= (1LL << 31) - 256 || k > 32768) return false;
+    b2_direct_args d = {};
+    d.flex = mode == MODE_FLEX16;
+    d.a_kind = B2_OPERAND_GATHER;
+    d.M = (int)rows; d.N = pass ? g.C : g.K; d.K = (int)k;
+    d.b_kind = pass ? B2_OPERAND_K : B2_OPERAND_ROWS;
+    d.b_rs = pass ? (long long)g.R * g.S * g.K : 1;
+    d.b_ks = pass ? 1 : g.K;
+    d.g.channels = pass ? g.K : g.C; d.g.H = pass ? g.P : g.H; d.g.W = pass ? g.Q : g.W; d.g.N = g.N;
+    d.g.P = pass ? g.H : g.P; d.g.Q = pass ? g.W : g.Q; d.g.R = g.R; d.g.S = g.S;
+    d.g.pad_h = g.pad_h; d.g.pad_w = g.pad_w; d.g.str_h = g.str_h; d.g.str_w = g.str_w;
+    d.g.dil_h = g.dil_h; d.g.dil_w = g.dil_w; d.g.bprop = pass;
+    d.ldc = rows; d.colmajor = 1;
+    *out = d;
+    const long long cost = b2_direct_cost(d);
+    // the planes of the unrolled rows once out and once back (cycles at 5 TB/s), then the tile kernel
+    const Shapes s = shapes_for(mode, (int)rows, d.N, (int)k);
+    const long long planes = rows * s.Kp * s.esize * 4 / 2600;
+    const long long kb = (mode == MODE_FLEX16 ? 1430LL : 1100LL) * (128 + s.bn) / 256;
+    const long long tiles = (long long)(s.Mp / kBlockM) * (s.Np / s.bn);
+    return cost >= 0 &&
+           cost < 13000 + planes + (tiles + 147) / 148 * (3500 + (long long)(s.Kp * s.esize / kKBytes) * kb);
+}
+
+inline int launch_direct(b2_direct_args& d, const void* A, const void* B, void* C,
+                         const b2_flex_scale* table, int slotA, int slotB, int slotC, int* stats,
+                         unsigned long long* probe_out, int* status, int probe, cudaStream_t st) {
+    d.A = A; d.B = B; d.C = C; d.table = table; d.slotA = slotA; d.slotB = slotB; d.slotC = slotC;
+    d.stats = stats; d.probe_out = probe_out; d.status = status; d.probe = probe;
+    return b2_direct_launch(d, st);
 }
 
 // Gather + split.  Rows of the planes: r = ((m*P + p)*Q + q)*N + n ; columns:
@@ -1286,6 +1328,9 @@ int run_fprop(const T* I, const T* F, void* O, const b2_conv_dims* d, const b2_f
     if (implicit_ok(MODE, g))
         return run_fprop_implicit<T, MODE>(I, F, O, g, table, slotI, slotF, slotO, stats, scratch,
                                            scratch_bytes, probe_out, status, probe, st);
+    b2_direct_args direct;
+    if (conv_goes_direct(MODE, g, 0, &direct))
+        return launch_direct(direct, I, F, O, table, slotI, slotF, slotO, stats, probe_out, status, probe, st);
     const long long rows_ll = (long long)g.M * g.P * g.Q * g.N;
     B2_REQUIRE(rows_ll < (1LL << 31) - 256, "too many output positions");
     B2_REQUIRE((long long)g.C * g.T * g.R * g.S < (1LL << 24), "filter window too large");
@@ -1461,6 +1506,9 @@ int run_bprop(const T* E, const T* F, void* GI, const b2_conv_dims* d, const b2_
         return implicit_tiles(base, base + 2 * si.act_plane, GI, gb, si, table, slotE, slotF, slotG,
                               stats, probe_out, status, probe, st);
     }
+    b2_direct_args direct;
+    if (conv_goes_direct(MODE, g, 1, &direct))
+        return launch_direct(direct, E, F, GI, table, slotE, slotF, slotG, stats, probe_out, status, probe, st);
     const long long rows_ll = (long long)g.D * g.H * g.W * g.N;
     B2_REQUIRE(rows_ll < (1LL << 31) - 256 && (long long)g.K * g.M * g.P * g.Q * g.N < (1LL << 31) &&
                (long long)g.K * g.T * g.R * g.S < (1LL << 24), "tensor too large");
@@ -1873,13 +1921,39 @@ extern "C" int b2_conv_fprop_scratch_bytes(int32_t flex, const b2_conv_dims* d, 
     if (rc) return rc;
     B2_REQUIRE(bytes, "null argument");
     const int mode = flex ? MODE_FLEX16 : MODE_F32X3;
-    size_t need = shapes_for(mode, g.M * g.P * g.Q * g.N, g.K, g.C * g.T * g.R * g.S).bytes;
-    if (implicit_ok(mode, g)) {
-        const size_t alt = implicit_shape(g).bytes;
-        if (alt > need || !getenv("B2_CONV_IM2COL")) need = alt > need ? alt : need;
-    }
-    *bytes = need;
+    b2_direct_args direct;
+    *bytes = implicit_ok(mode, g) ? implicit_shape(g).bytes
+             : conv_goes_direct(mode, g, 0, &direct)
+                 ? 0 : shapes_for(mode, g.M * g.P * g.Q * g.N, g.K, g.C * g.T * g.R * g.S).bytes;
     return B2_OK;
+}
+
+extern "C" int b2_conv_launches(int32_t flex, const b2_conv_dims* d, int32_t pass, int32_t* launches) {
+    ConvGeom g;
+    int rc = geom_from(d, &g);
+    if (rc) return rc;
+    B2_REQUIRE(launches && pass >= 0 && pass <= 2, "bad argument");
+    const int mode = flex ? MODE_FLEX16 : MODE_F32X3;
+    ConvGeom gp;
+    b2_direct_args direct;
+    if (pass == 2)
+        *launches = update_implicit_shape(mode, g).ok || update_shape(mode, g).splits > 1 ? 4 : 3;
+    else
+        *launches = !(flex && pass_geom(g, pass, &gp)) && conv_goes_direct(mode, g, pass, &direct) ? 1 : 3;
+    return B2_OK;
+}
+
+extern "C" int b2_conv_fprop_f32_fused(const float* I, const float* F, float* O, const b2_conv_dims* d,
+                                       const float* bias, const float* residual, int32_t relu,
+                                       int32_t* status, void* stream) {
+    ConvGeom g;
+    int rc = geom_from(d, &g);
+    if (rc) return rc;
+    B2_REQUIRE(I && F && O, "null tensor");
+    b2_direct_args direct;
+    B2_REQUIRE(conv_goes_direct(MODE_F32X3, g, 0, &direct), "this convolution takes no fused tail");
+    direct.tail = 1; direct.bias = bias; direct.residual = residual; direct.relu = relu ? 1 : 0;
+    return launch_direct(direct, I, F, O, nullptr, 0, 0, 0, nullptr, nullptr, status, 0, (cudaStream_t)stream);
 }
 
 extern "C" int b2_conv_fprop_f32(const float* I, const float* F, float* O, const b2_conv_dims* d,
@@ -1907,12 +1981,21 @@ extern "C" int b2_conv_planes_info(const b2_conv_dims* d, int32_t pass, int32_t*
     int rc = geom_from(d, &f);
     if (rc) return rc;
     B2_REQUIRE(supported && act_plane_bytes && filter_planes_bytes, "null argument");
-    *supported = pass_geom(f, pass, &g) ? 1 : 0;
+    // The planes of a strided input gradient keep the contract that they have always had -- whole tiles
+    // of 128 images, room for the error tensor at the input's resolution -- although the tensor now lies
+    // undilated at the front of that room; other batches reach the tile kernel through
+    // b2_conv_bprop_flex16.
+    const bool strided = pass == 1 && (f.str_h > 1 || f.str_w > 1);
+    *supported = pass_geom(f, pass, &g) && !(strided && f.N % 128 != 0) ? 1 : 0;
     *act_plane_bytes = 0;
     *filter_planes_bytes = 0;
     if (*supported) {
         const ImplicitShape s = implicit_shape(g);
         *act_plane_bytes = s.act_plane;
+        if (strided) {
+            const size_t room = plane_size(f.K, f.H + 2 * f.pad_h - f.R + 1, f.W + 2 * f.pad_w - f.S + 1, f.N);
+            if (room > s.act_plane) *act_plane_bytes = room;
+        }
         *filter_planes_bytes = s.filt_bytes;
     }
     return B2_OK;
@@ -1981,13 +2064,11 @@ extern "C" int b2_conv_bprop_scratch_bytes(int32_t flex, const b2_conv_dims* d, 
     int rc = geom_from(d, &g);
     if (rc) return rc;
     B2_REQUIRE(bytes, "null argument");
-    size_t need = bprop_shape(flex ? MODE_FLEX16 : MODE_F32X3, g).bytes;
+    const int mode = flex ? MODE_FLEX16 : MODE_F32X3;
     ConvGeom gb;
-    if (flex && pass_geom(g, 1, &gb)) {
-        const size_t alt = implicit_shape(gb).bytes;
-        if (alt > need) need = alt;
-    }
-    *bytes = need;
+    b2_direct_args direct;
+    *bytes = flex && pass_geom(g, 1, &gb) ? implicit_shape(gb).bytes
+             : conv_goes_direct(mode, g, 1, &direct) ? 0 : bprop_shape(mode, g).bytes;
     return B2_OK;
 }
 

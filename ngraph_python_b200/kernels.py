@@ -79,7 +79,7 @@ class _PlaneUser(object):
     def _setup_planes(self, t, conv_pass, stream_arg, filter_arg):
         if not self.flex:
             return
-        ok, act_bytes, filt_bytes = lib.conv_planes_info(self.dims, conv_pass)
+        ok, _, filt_bytes = lib.conv_planes_info(self.dims, conv_pass)
         if not ok:
             return
         self.use_planes = True
@@ -89,7 +89,7 @@ class _PlaneUser(object):
         self.filter_bytes = filt_bytes
         self.in_views[filter_arg].buffer.watched = True
         buf = self.in_views[stream_arg].buffer
-        buf.plane_bytes = act_bytes
+        buf.plane_bytes = lib.plane_bytes(self.in_views[stream_arg].axes.lengths)
         # (planes whose rows of images are padded are written by the convolutions only)
         buf.plane_dense = self.dims.N % 16 == 0
         buf.plane_steps = getattr(buf, "plane_steps", []) + [self]
@@ -228,9 +228,9 @@ class ConvStep(_PlaneUser, _Step):
     launches = 3
 
     def __init__(self, index, op, t, epilogue=None):
-        """epilogue (flex16 implicit-GEMM path only): dict(out=<op whose tensor the step writes>,
+        """epilogue (where takes_conv_tail): dict(out=<op whose tensor the step writes>,
         bias=<op or None>, residual=<op or None>, relu=bool) -- the elementwise tail of the layer,
-        evaluated in the tile kernel's epilogue."""
+        evaluated in the convolution kernel's epilogue."""
         super(ConvStep, self).__init__(index, op)
         inputs, filters = op.args
         self.epi = epilogue
@@ -269,10 +269,11 @@ class ConvStep(_PlaneUser, _Step):
         self.out_views = [ov]
         self.flex = t.flex
         self.scratch_bytes = lib.conv_fprop_scratch_bytes(self.flex, d) + 1024
+        self.launches = lib.conv_launches(self.flex, d, lib.CONV_FPROP)
         self._setup_planes(t, lib.CONV_FPROP, 0, 1)
         if epilogue:
-            if not self.use_planes:
-                raise ValueError("a fused convolution epilogue needs the implicit-GEMM path")
+            if not (self.use_planes if self.flex else self.launches == 1):
+                raise ValueError("a fused convolution epilogue needs a kernel that takes one")
             self.probe_is_float = True
             self.write_int16 = True          # the planner clears it when only planes are read
             for key in ("bias", "residual"):
@@ -285,11 +286,21 @@ class ConvStep(_PlaneUser, _Step):
     def launch(self, t):
         if self.use_planes:
             return self._launch_planes(t)
-        iv, fv = self.in_views
+        iv, fv = self.in_views[:2]
         ov = self.out_views[0]
         raw = lib.raw()
         sp, sb = t._scratch_aligned()
         st = t.stream.cuda_stream
+        if self.epi:
+            extra = [self._ptr(v) for v in self.in_views[2:]]
+            bias = extra.pop(0) if self.epi.get("bias") is not None else None
+            residual = extra.pop(0) if self.epi.get("residual") is not None else None
+            lib.check(raw.b2_conv_fprop_f32_fused(self._ptr(iv), self._ptr(fv), self._ptr(ov),
+                                                  C.byref(self.dims), bias, residual,
+                                                  int(bool(self.epi.get("relu"))),
+                                                  t._status.data_ptr(), st))
+            t.kernel_launches += self.launches
+            return
         if not self.flex:
             lib.check(raw.b2_conv_fprop_f32(self._ptr(iv), self._ptr(fv), self._ptr(ov),
                                             C.byref(self.dims), sp, sb, t._status.data_ptr(), st))
@@ -304,6 +315,15 @@ class ConvStep(_PlaneUser, _Step):
                 t._table.data_ptr(), slots[0], slots[1], slots[2], t._stats.data_ptr(), sp, sb,
                 t._probe64.data_ptr(), t._status.data_ptr(), probe, st))
         self._flex_probe_then(t, ov.buffer, [iv.buffer, fv.buffer], call)
+
+
+def takes_conv_tail(fprop, t):
+    """Whether the forward convolution's kernel evaluates the layer's elementwise tail: the flex16
+    tile kernel, the fp32 kernel that gathers its operands."""
+    d = _conv_dims_of(fprop, t)
+    if t.flex:
+        return lib.conv_planes_info(d, lib.CONV_FPROP)[0]
+    return lib.conv_launches(False, d, lib.CONV_FPROP) == 1
 
 
 def _conv_dims_of(fprop, t):
@@ -352,6 +372,8 @@ class _ConvGradStep(_PlaneUser, _Step):
         sizer = lib.conv_bprop_scratch_bytes if self.what == "bprop" else \
             lib.conv_update_scratch_bytes
         self.scratch_bytes = sizer(self.flex, d) + 1024
+        self.launches = lib.conv_launches(
+            self.flex, d, lib.CONV_BPROP if self.what == "bprop" else lib.CONV_UPDATE)
         if self.what == "bprop":
             self._setup_planes(t, lib.CONV_BPROP, 0, 1)      # streamed: delta; filters: args[1]
 
@@ -394,7 +416,6 @@ class ConvUpdateStep(_ConvGradStep):
     """Filter gradient of a convolution: args (delta K,M,P,Q,N ; inputs C,D,H,W,N)."""
     kind = "conv_update"
     what = "update"
-    launches = 4                    # two operand kernels, the tile kernel, the slice sum
 
 
 class PoolStep(_Step):

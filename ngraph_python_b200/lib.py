@@ -124,6 +124,8 @@ def _load():
         "b2_gemm_flex16": (C.c_int, [vp, i64, i64, vp, i64, i64, vp, i64, i32, i32, i32, vp, i32,
                                      i32, i32, vp, vp, sz, vp, vp, i32, vp]),
         "b2_conv_fprop_scratch_bytes": (C.c_int, [i32, C.POINTER(ConvDims), C.POINTER(sz)]),
+        "b2_conv_launches": (C.c_int, [i32, C.POINTER(ConvDims), i32, C.POINTER(i32)]),
+        "b2_conv_fprop_f32_fused": (C.c_int, [vp, vp, vp, C.POINTER(ConvDims), vp, vp, i32, vp, vp]),
         "b2_conv_fprop_f32": (C.c_int, [vp, vp, vp, C.POINTER(ConvDims), vp, sz, vp, vp]),
         "b2_conv_fprop_flex16": (C.c_int, [vp, vp, vp, C.POINTER(ConvDims), vp, i32, i32, i32, vp,
                                            vp, sz, vp, vp, i32, vp]),
@@ -337,12 +339,26 @@ def conv_fprop_scratch_bytes(flex, dims):
     return n.value
 
 
-CONV_FPROP, CONV_BPROP = 0, 1
+CONV_FPROP, CONV_BPROP, CONV_UPDATE = 0, 1, 2
 RNG_UNIFORM, RNG_NORMAL = 0, 1
 
 
+def conv_launches(flex, dims, conv_pass):
+    n = C.c_int32()
+    check(_lib.b2_conv_launches(int(bool(flex)), C.byref(dims), conv_pass, C.byref(n)))
+    return n.value
+
+
+def plane_bytes(lengths):
+    """Offset of the low byte plane from the high one for a tensor of these extents (images last)."""
+    size = (lengths[-1] + 15) // 16 * 16
+    for n in lengths[:-1]:
+        size *= n
+    return (size + 1023) // 1024 * 1024
+
+
 def conv_planes_info(dims, conv_pass=CONV_FPROP):
-    """(supported, bytes of one plane of the streamed tensor, bytes of the filter planes)."""
+    """(supported, room for one plane of the streamed tensor, bytes of the filter planes)."""
     ok, a, f = C.c_int32(), C.c_size_t(), C.c_size_t()
     check(_lib.b2_conv_planes_info(C.byref(dims), conv_pass, C.byref(ok), C.byref(a), C.byref(f)))
     return bool(ok.value), a.value, f.value

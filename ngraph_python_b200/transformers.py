@@ -908,18 +908,18 @@ class _Planner(object):
             self.deferred.append(requant)
 
     def _find_conv_tails(self, ordered):
-        """flex16, implicit-GEMM convolutions: folds `+ bias[channel]`, `+ residual` and
+        """Convolutions whose kernel takes a tail: folds `+ bias[channel]`, `+ residual` and
         `maximum(., 0)` that follow a convolution -- each the only reader of the value before it
         -- into the convolution step (evaluated in the tile kernel's epilogue; the reference's
         kernels carry bias / relu flags for the same purpose, ngraph/transformers/gpu/conv.py)."""
         t = self.t
-        if not (t.flex and t.fuse and t.fuse_conv_tail):
+        if not (t.fuse and t.fuse_conv_tail):
             return
         for conv in ordered:
             if not isinstance(conv, ConvolutionOp):
                 continue
             try:
-                ok = lib.conv_planes_info(kernels._conv_dims_of(conv, t), lib.CONV_FPROP)[0]
+                ok = kernels.takes_conv_tail(conv, t)
             except Exception:
                 ok = False
             if not ok:
