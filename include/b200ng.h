@@ -193,7 +193,7 @@ int b2_flex_publish(int32_t* stats, int32_t n, const int32_t* status, int32_t* h
  * b2_call_outputs is b2_flex_publish with results: dst[k] (pinned host memory) <- bytes[k] bytes of
  * src[k], both 16-byte aligned.
  * b2_call_stage: the address at which the device can read `bytes` bytes of host memory at src:
- * src itself where it is page-locked, else `pinned`, to which they are copied.
+ * src itself where it is page-locked, else `pinned`, to which they are copied; NULL where that is NULL.
  * Replace FlexGPUDeviceTensor.__setitem__ / get and the per-kernel statistics read of the reference
  * (ngraph/transformers/flexgputransform.py:178-208, 347-371).
  * ------------------------------------------------------------------------------------------ */
@@ -312,6 +312,9 @@ int b2_conv_planes_info(const b2_conv_dims* d, int32_t pass, int32_t* supported,
                         size_t* act_plane_bytes, size_t* filter_planes_bytes);
 int b2_conv_split_activations(const int16_t* X, const b2_conv_dims* d, int32_t pass, void* planes,
                               void* stream);
+/* ... of any tensor of c x h x w x n mantissas. */
+int b2_conv_split_planes(const int16_t* X, int32_t c, int32_t h, int32_t w, int32_t n, void* planes,
+                         void* stream);
 int b2_conv_filter_planes(const int16_t* F, const b2_conv_dims* d, int32_t pass, void* planes,
                           void* stream);
 int b2_conv_flex16_planes(int32_t pass, const void* act_planes, const void* filter_planes,
@@ -364,6 +367,17 @@ int b2_conv_update_flex16(const int16_t* I, const int16_t* E, int16_t* U, const 
                           const b2_flex_scale* table, int32_t slotI, int32_t slotE, int32_t slotU,
                           int32_t* stats, void* scratch, size_t scratch_bytes, uint64_t* probe_out,
                           int32_t* status, int32_t probe, void* stream);
+/* The filter gradient from the byte planes of both tensors (laid out as b2_conv_planes_info says for
+ * the activations of pass 0 and the error tensor of pass 1), with the sum of the error tensor over
+ * (p,q,n) -- the bias gradient, quantised like an elementwise sum -- where bias_grad is not NULL.
+ * workspace: workspace_bytes, 1024-byte aligned, zero before the first call and left zero by every
+ * call.  probe: probe_out[0] for U, probe_out[1] for the bias (|sum of mantissas|). */
+int b2_conv_update_planes_info(const b2_conv_dims* d, int32_t* supported, size_t* workspace_bytes);
+int b2_conv_update_flex16_planes(const void* act_planes, const void* err_planes, int16_t* U,
+                                 int16_t* bias_grad, const b2_conv_dims* d, const b2_flex_scale* table,
+                                 int32_t slotI, int32_t slotE, int32_t slotU, int32_t slotB,
+                                 int32_t* stats, void* workspace, uint64_t* probe_out, int32_t* status,
+                                 int32_t probe, void* stream);
 /* Average pooling over H,W windows.  flex != 0: int16 in and out sharing one exponent
  * (ngraph/transformers/passes/flexpass.py:40-48); *stats_slot = max(*stats_slot, max |out|). */
 int b2_pool_avg_fprop(const void* I, void* O, int32_t flex, int32_t C, int32_t H, int32_t W,

@@ -233,7 +233,8 @@ extern "C" int b2_call_stage(const void* src, size_t bytes, void* pinned, const 
         return B2_OK;
     }
     (void)cudaGetLastError();                     // (not a CUDA address: no error of the caller's)
-    B2_REQUIRE(pinned, "pageable memory needs a pinned block to copy to");
+    *visible = nullptr;
+    if (!pinned) return B2_OK;                    // pageable, and no block to copy to
 #if defined(__x86_64__)
     static const bool avx2 = __builtin_cpu_supports("avx2");
     if (avx2 && ((uintptr_t)pinned & 31) == 0) copy_streaming(pinned, src, bytes);

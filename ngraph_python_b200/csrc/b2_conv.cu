@@ -907,47 +907,16 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap mapI0,
     if (threadIdx.x == 0 && *fail_flag && p.status) atomicExch(p.status, 1);
 }
 
-// activations -> two operand planes in the same C,H,W,N layout (elementwise)
-template <typename T, int MODE>
+// activations -> two operand planes in the same C,H,W,N layout, eight mantissas per thread: one 16-byte
+// load, two 8-byte stores
 __global__ void __launch_bounds__(256)
-split_same_layout_kernel(const T* __restrict__ src, long long n, void* __restrict__ plane0,
-                         void* __restrict__ plane1, unsigned lo_xor = 0) {
+split_same_layout_kernel(const short* __restrict__ src, long long n8, void* __restrict__ plane0,
+                         void* __restrict__ plane1) {
     const long long stride = (long long)gridDim.x * blockDim.x;
-    if (MODE == MODE_FLEX16 && (n & 7) == 0 && (((uintptr_t)src | (uintptr_t)plane0 |
-                                                  (uintptr_t)plane1) & 15) == 0) {
-        // eight mantissas per thread: one 16-byte load, two 8-byte stores
-        for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < n / 8; v += stride) {
-            const int4 w = __ldcs(reinterpret_cast<const int4*>(src) + v);
-            const unsigned x[4] = {(unsigned)w.x, (unsigned)w.y, (unsigned)w.z, (unsigned)w.w};
-            unsigned hi[2] = {0, 0}, lo[2] = {0, 0};
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                // each word holds two int16: low byte of each -> lo plane; (m - lo) >> 8 is just
-                // the high byte of the two's-complement pattern
-                const unsigned l2 = __byte_perm(x[j], 0, 0x4420);   // bytes 0 and 2
-                const unsigned h2 = __byte_perm(x[j], 0, 0x4431);   // bytes 1 and 3
-                lo[j >> 1] |= (l2 & 0xffffu) << (16 * (j & 1));
-                hi[j >> 1] |= (h2 & 0xffffu) << (16 * (j & 1));
-            }
-            reinterpret_cast<uint2*>(plane0)[v] = make_uint2(hi[0], hi[1]);
-            reinterpret_cast<uint2*>(plane1)[v] = make_uint2(lo[0] ^ lo_xor, lo[1] ^ lo_xor);
-        }
-        return;
-    }
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
-        if (MODE == MODE_FLEX16) {
-            const int m = (int)src[i];
-            const int lo = m & 0xff;
-            ((signed char*)plane0)[i] = (signed char)((m - lo) >> 8);
-            ((unsigned char*)plane1)[i] = (unsigned char)lo;
-        } else {
-            const float a = (float)src[i];
-            unsigned hb;
-            asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(hb) : "f"(a));
-            const float hi = __uint_as_float(hb);
-            ((float*)plane0)[i] = hi;
-            ((float*)plane1)[i] = a - hi;
-        }
+    for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < n8; v += stride) {
+        const uint4 w = __ldcs(reinterpret_cast<const uint4*>(src) + v);
+        reinterpret_cast<uint2*>(plane0)[v] = make_uint2(__byte_perm(w.x, w.y, 0x7531), __byte_perm(w.z, w.w, 0x7531));
+        reinterpret_cast<uint2*>(plane1)[v] = make_uint2(__byte_perm(w.x, w.y, 0x6420), __byte_perm(w.z, w.w, 0x6420));
     }
 }
 
@@ -982,8 +951,8 @@ int split_to_planes(const short* x, int c, int h, int w, int n, void* planes, si
     long long blocks = (units + 255) / 256;
     if (blocks > 148 * 16) blocks = 148 * 16;
     unsigned char* lo = (unsigned char*)planes + plane_bytes;
-    if (np == n)
-        split_same_layout_kernel<short, MODE_FLEX16><<<(unsigned)blocks, 256, 0, st>>>(x, rows * n, planes, lo);
+    if (np == n && ((uintptr_t)x & 15) == 0)
+        split_same_layout_kernel<<<(unsigned)blocks, 256, 0, st>>>(x, units, planes, lo);
     else
         split_padded_kernel<<<(unsigned)blocks, 256, 0, st>>>(x, rows, n, np, (unsigned char*)planes, lo);
     B2_CUDA(cudaGetLastError());
@@ -1535,29 +1504,55 @@ int run_bprop(const T* E, const T* F, void* GI, const b2_conv_dims* d, const b2_
 
 // ---- filter gradient on the tile kernel's operands ------------------------------------------------
 // U[(c,r,s), k] = sum over (p,q,n) of I[c, p*str-pad+r, q*str-pad+s, n] * E[k, p, q, n].
-// One k-block = one output pixel x 128 images.  Its A operand is the very box the forward kernel
-// loads (rows (c,r,s) of one channel chunk, 128 images along the row: K-major here), its B operand
-// the rows k of the error tensor's planes at that pixel.  A CTA owns a channel chunk, a tile of
-// filters and a range of k-blocks; two threads issue the products of alternate k-blocks into
-// accumulators of their own ([HH | Ah*El'] and [Al*Eh | LL], El' = El - 128 with the row sums of A
-// taken from a constant extra row of B), and the CTA writes its exact int64 sums as one slice of
-// partial[slice][C*R*S][K], which splitk_finish_kernel adds up, rescales and stores.
+// One k-block = a tile of gh x gw output pixels x 128 images.  Its A operand is the very box the forward
+// kernel loads (rows (c,h,w): the window under the tile for one channel chunk, images along the row:
+// K-major here), its B operand the rows (k, pixel) of the error tensor's planes; the product of window
+// row (h,w) with pixel (i,j) belongs to the tap (h - i*str, w - j*str), and the epilogue adds these up.
+// A CTA owns a channel chunk, a tile of filters and a range of k-blocks (a slice); both operands come as
+// (signed high, unsigned low) byte planes, four exact products HH | X | LL.  The CTAs of the other
+// slices add their 64-bit sums to the same accumulators with atomics -- whole numbers, so the order does
+// not matter -- and the last to arrive rescales, stores, and leaves the accumulators zero for the next
+// call: one launch, no partial sums in memory.  Four idle warps sum the error planes for the bias
+// gradient while the tensor core works on them (the chunks of one filter tile take the k-blocks in
+// turn).
+//
+// What bounds it: the bytes from L2 to the SMs and the tensor core about equally.  A window is read
+// once per tile instead of once per pixel: for 3x3 filters a tile of 2x2 pixels brings 16 rows a channel
+// instead of 36 and fills the 128 rows of the operand (8 channels x 16) where single pixels left 56 empty.
 struct UpdTileParams {
-    int Q, nblk, nkb;              // k-block kb = (p*Q + q)*nblk + nb
-    int pad_h, pad_w, str_h, str_w;
-    int cu, rs, C, K;              // channels per chunk, R*S
-    int ntn, kt, bn;               // filter tiles: kt filters each, bn = round_up(kt + 1, 16) rows
-    int per;                       // k-blocks per slice (grid.x)
-    int nstages, tmem_cols;
+    int tw, nblk, nkb;             // k-block kb = (tile_p*tw + tile_q)*nblk + nb
+    int off_h, off_w, step_h, step_w, str_h, str_w;
+    int gh, gw, wh, ww, R, S, cu, C, K, cchunks;
+    int ntn, kt, bn;               // filter tiles: kt filters x gh*gw pixels in bn rows
+    int per, nsplit;               // k-blocks per slice, slices (grid.x)
+    int ksteps, nstages, tmem_cols;
     unsigned box_a, box_b;         // bytes of one activation box, of one error box
-    long long* partial;
+    unsigned long long* acc;       // [C*R*S][K], then [K] for the bias: zero between calls
+    unsigned* arrived;             // [cchunks*ntn], then [ntn]: likewise
+    short *U, *bias;               // bias gradient: NULL where it is not wanted
+    const b2_flex_scale* table;
+    int slotI, slotE, slotU, slotB;
+    int* stats;
+    unsigned long long* probe_out; // probe: max |sum| of U, of the bias
     int* status;
+    int probe;
 };
 
 constexpr int kUpdThreads = 256;
 constexpr int kUpdMaxStages = 6;
+constexpr int kUpdMaxN = 160;                      // columns of one accumulator: three in 512
 constexpr int kUpdAPlane = 128 * kKBytes;          // 128 rows of 128 bytes
 constexpr int kUpdSmemFixed = 1024 + 512;
+
+// largest of a block's non-negative values, in thread 0's atomic
+template <typename V, typename F>
+__device__ __forceinline__ void update_max(V v, F put) {
+    for (int o = 16; o > 0; o >>= 1) {
+        const V t = __shfl_xor_sync(0xffffffffu, v, o);
+        v = t > v ? t : v;
+    }
+    if ((threadIdx.x & 31) == 0 && v) put(v);
+}
 
 __global__ void __launch_bounds__(kUpdThreads, 1)
 conv_update_kernel(const __grid_constant__ CUtensorMap mapI0, const __grid_constant__ CUtensorMap mapI1,
@@ -1566,45 +1561,32 @@ conv_update_kernel(const __grid_constant__ CUtensorMap mapI0, const __grid_const
     extern __shared__ unsigned char smem_raw[];
     unsigned char* ring = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     const int bn = p.bn, kt = p.kt;
-    const int b_bytes = 2 * bn * kKBytes;                   // [E_hi rows | E_lo' rows]
-    const int stage = 2 * kUpdAPlane + b_bytes;
-    unsigned long long* full_bar = (unsigned long long*)(ring + (size_t)p.nstages * stage);   // [2][max]
-    unsigned long long* empty_bar = full_bar + 2 * kUpdMaxStages;
-    unsigned long long* tmem_full = empty_bar + kUpdMaxStages;                               // [2]
-    unsigned* tmem_holder = (unsigned*)(tmem_full + 2);
+    const int b_plane = bn * kKBytes, stage = 2 * kUpdAPlane + 2 * b_plane;
+    unsigned long long* full_bar = (unsigned long long*)(ring + (size_t)p.nstages * stage);
+    unsigned long long* empty_bar = full_bar + kUpdMaxStages;
+    unsigned long long* tmem_full = empty_bar + kUpdMaxStages;
+    unsigned* tmem_holder = (unsigned*)(tmem_full + 1);
     int* fail_flag = (int*)(tmem_holder + 1);
+    unsigned* last = (unsigned*)(fail_flag + 1);                 // [2]
 
     const int warp = warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
     const int chunk = blockIdx.y / p.ntn, ktile = blockIdx.y - chunk * p.ntn;
     const int kb0 = blockIdx.x * p.per;
     int mine = p.nkb - kb0;
     if (mine > p.per) mine = p.per;
+    const int npix = p.gh * p.gw;
 
     if (threadIdx.x == 0) {
         prefetch_map(&mapI0); prefetch_map(&mapI1); prefetch_map(&mapE0); prefetch_map(&mapE1);
         for (int s = 0; s < kUpdMaxStages; ++s) {
-            mbar_init(&full_bar[s], 1); mbar_init(&full_bar[kUpdMaxStages + s], 1);
-            mbar_init(&empty_bar[s], 1);
+            mbar_init(&full_bar[s], 1);
+            mbar_init(&empty_bar[s], p.bias ? 5 : 1);
         }
-        mbar_init(&tmem_full[0], 1); mbar_init(&tmem_full[1], 1);
+        mbar_init(tmem_full, 1);
         *fail_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) tmem_alloc(tmem_holder, p.tmem_cols);
-    {
-        // rows kt .. bn-1 of both parts of every stage's B tile are constants the loads never
-        // touch: zero, except row kt of the low part, which is all ones (the row-sum column)
-        const int rows = bn - kt, units = p.nstages * 2 * rows * 8;        // 16-byte units
-        for (int i = threadIdx.x; i < units; i += kUpdThreads) {
-            const int u = i & 7, r = (i >> 3) % rows, part = ((i >> 3) / rows) & 1;
-            const int st = (i >> 3) / (2 * rows);
-            const unsigned v = (part == 1 && r == 0) ? 0x01010101u : 0u;
-            uint4* dst = (uint4*)(ring + (size_t)st * stage + 2 * kUpdAPlane +
-                                  (size_t)(part * bn + kt + r) * kKBytes) + u;
-            *dst = make_uint4(v, v, v, v);
-        }
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -1614,93 +1596,112 @@ conv_update_kernel(const __grid_constant__ CUtensorMap mapI0, const __grid_const
         if (elect_one()) {
             int s = 0;
             unsigned empty_parity = 1;
+            int nb = kb0 % p.nblk, pq = kb0 / p.nblk, q = pq % p.tw, pp = pq / p.tw;
             for (int i = 0; i < mine; ++i) {
-                const int kb = kb0 + i;
-                const int pq = kb / p.nblk, nb = kb - pq * p.nblk;
-                const int pp = pq / p.Q, q = pq - pp * p.Q;
-                unsigned long long* fb = full_bar + (i & 1) * kUpdMaxStages;
                 if (!mbar_wait_relaxed(&empty_bar[s], empty_parity)) { atomicExch(fail_flag, 1); break; }
                 unsigned char* sa = ring + (size_t)s * stage;
-                mbar_expect_tx(&fb[s], 2 * p.box_a + 2 * p.box_b);
-                tma_load_4d(sa, &mapI0, nb * 128, q * p.str_w - p.pad_w, pp * p.str_h - p.pad_h,
-                            chunk * p.cu, &fb[s]);
-                tma_load_4d(sa + kUpdAPlane, &mapI1, nb * 128, q * p.str_w - p.pad_w,
-                            pp * p.str_h - p.pad_h, chunk * p.cu, &fb[s]);
-                tma_load_2d(sa + 2 * kUpdAPlane, &mapE0, kb * 128, ktile * kt, &fb[s]);
-                tma_load_2d(sa + 2 * kUpdAPlane + bn * kKBytes, &mapE1, kb * 128, ktile * kt, &fb[s]);
+                mbar_expect_tx(&full_bar[s], 2 * p.box_a + 2 * p.box_b);
+                const int w0 = q * p.step_w + p.off_w, h0 = pp * p.step_h + p.off_h;
+                tma_load_4d(sa, &mapI0, nb * 128, w0, h0, chunk * p.cu, &full_bar[s]);
+                tma_load_4d(sa + kUpdAPlane, &mapI1, nb * 128, w0, h0, chunk * p.cu, &full_bar[s]);
+                unsigned char* sb = sa + 2 * kUpdAPlane;
+                tma_load_4d(sb, &mapE0, nb * 128, q * p.gw, pp * p.gh, ktile * kt, &full_bar[s]);
+                tma_load_4d(sb + b_plane, &mapE1, nb * 128, q * p.gw, pp * p.gh, ktile * kt, &full_bar[s]);
                 if (++s == p.nstages) { s = 0; empty_parity ^= 1u; }
+                if (++nb == p.nblk) {
+                    nb = 0;
+                    if (++q == p.tw) { q = 0; ++pp; }
+                }
             }
         }
-    } else if (warp == 1 || warp == 2) {
-        const int id = warp - 1;
+    } else if (warp == 1) {
         if (elect_one()) {
-            const unsigned id_s = make_idesc_n(2, 1, 1, 2 * bn), id_u = make_idesc_n(2, 0, 1, 2 * bn);
-            const unsigned acc = tmem_base + id * 4 * bn;
-            unsigned long long* fb = full_bar + id * kUpdMaxStages;
-            unsigned phase_bits = 0, accumulate = 0;
-            bool ok = true;
-            for (int i = id; i < mine && ok; i += 2) {
-                const int s = i % p.nstages;
-                if (!mbar_wait(&fb[s], (phase_bits >> s) & 1u)) { atomicExch(fail_flag, 1); ok = false; break; }
-                phase_bits ^= 1u << s;
+            const unsigned id_ss = make_idesc_n(2, 1, 1, bn), id_su = make_idesc_n(2, 1, 0, bn),
+                           id_us = make_idesc_n(2, 0, 1, bn), id_uu = make_idesc_n(2, 0, 0, bn);
+            const unsigned acc_x = tmem_base + bn, acc_l = tmem_base + 2 * bn;
+            const int ksteps = p.ksteps;
+            unsigned accumulate = 0, parity = 0;
+            int s = 0;
+            for (int i = 0; i < mine; ++i) {
+                if (!mbar_wait(&full_bar[s], parity)) { atomicExch(fail_flag, 1); break; }
                 tc_fence_after();
                 unsigned char* sa = ring + (size_t)s * stage;
                 const unsigned long long dAh = make_smem_desc(sa), dAl = make_smem_desc(sa + kUpdAPlane);
-                const unsigned long long dB = make_smem_desc(sa + 2 * kUpdAPlane);
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    tc_mma<MODE_FLEX16>(acc, dAh + 2 * k, dB + 2 * k, id_s, accumulate);            // HH | Ah*El'
-                    tc_mma<MODE_FLEX16>(acc + 2 * bn, dAl + 2 * k, dB + 2 * k, id_u, accumulate);   // Al*Eh | LL
+                const unsigned long long dBh = make_smem_desc(sa + 2 * kUpdAPlane);
+                const unsigned long long dBl = make_smem_desc(sa + 2 * kUpdAPlane + b_plane);
+                for (int k = 0; k < ksteps; ++k) {
+                    tc_mma<MODE_FLEX16>(tmem_base, dAh + 2 * k, dBh + 2 * k, id_ss, accumulate);
+                    tc_mma<MODE_FLEX16>(acc_x, dAh + 2 * k, dBl + 2 * k, id_su, accumulate);
+                    tc_mma<MODE_FLEX16>(acc_x, dAl + 2 * k, dBh + 2 * k, id_us, 1u);
+                    tc_mma<MODE_FLEX16>(acc_l, dAl + 2 * k, dBl + 2 * k, id_uu, accumulate);
                     accumulate = 1;
                 }
                 tc_commit(&empty_bar[s]);
+                if (++s == p.nstages) { s = 0; parity ^= 1u; }
             }
-            if (accumulate) tc_commit(&tmem_full[id]);
-            else mbar_arrive(&tmem_full[id]);          // no k-block of its own: nothing to wait for
+            tc_commit(tmem_full);
         }
-    } else if (warp >= 4) {
-        const int quarter = warp - 4;
-        const bool two = mine >= 2;                     // the second accumulator set holds sums
-        bool ok = mbar_wait_relaxed(&tmem_full[0], 0);
-        ok = mbar_wait_relaxed(&tmem_full[1], 0) && ok;
-        if (!ok) atomicExch(fail_flag, 1);
-        tc_fence_after();
-        const int row = quarter * 32 + lane;
-        const int cg = chunk * p.cu + row / p.rs;
-        const bool valid = ok && row < p.cu * p.rs && cg < p.C;
-        const unsigned a0 = tmem_base + ((unsigned)(quarter * 32) << 16), a1 = a0 + 4 * bn;
-        // (the loaded registers are only read after the wait)
-        const unsigned h0 = tmem_ld1(a0 + bn + kt), l0 = tmem_ld1(a0 + 3 * bn + kt);
-        unsigned h1 = 0, l1 = 0;
-        if (two) { h1 = tmem_ld1(a1 + bn + kt); l1 = tmem_ld1(a1 + 3 * bn + kt); }
-        tmem_ld_wait();
-        const long long s_hi = (long long)(int)h0 + (long long)(int)h1;
-        const long long s_lo = (long long)(int)l0 + (long long)(int)l1;
-        const long long fix = 128LL * (256LL * s_hi + s_lo);
-        long long* out = p.partial + ((long long)blockIdx.x * p.C * p.rs + (long long)chunk * p.cu * p.rs + row) * p.K +
-                         ktile * kt;
-        for (int c0 = 0; c0 < kt; c0 += 8) {
-            unsigned hh[8], x1[8], x2[8], ll[8];
-            tmem_ld8(a0 + c0, hh); tmem_ld8(a0 + bn + c0, x1);
-            tmem_ld8(a0 + 2 * bn + c0, x2); tmem_ld8(a0 + 3 * bn + c0, ll);
-            tmem_ld_wait();
-            long long v[8];
+    } else if (warp >= 4 && p.bias) {
+        // sums of the error rows: thread t takes the 16-byte units t, t + 128, ..., whose rows
+        // are t/8 + 16*m
+        const int t = threadIdx.x - 128;
+        constexpr int kMost = kUpdMaxN / 16;
+        int hi[kMost], lo[kMost];
 #pragma unroll
-            for (int j = 0; j < 8; ++j)
-                v[j] = ((long long)(int)hh[j] << 16) + (((long long)(int)x1[j] + (long long)(int)x2[j]) << 8) +
-                       (long long)(int)ll[j];
-            if (two) {
-                tmem_ld8(a1 + c0, hh); tmem_ld8(a1 + bn + c0, x1);
-                tmem_ld8(a1 + 2 * bn + c0, x2); tmem_ld8(a1 + 3 * bn + c0, ll);
-                tmem_ld_wait();
+        for (int m = 0; m < kMost; ++m) hi[m] = lo[m] = 0;
+        int s = 0, turn = 0;
+        unsigned parity = 0;
+        bool ok = true;
+        for (int i = 0; i < mine; ++i) {
+            if (ok && !mbar_wait_relaxed(&full_bar[s], parity)) { atomicExch(fail_flag, 1); ok = false; }
+            if (turn == chunk && ok) {
+                const unsigned char* sb = ring + (size_t)s * stage + 2 * kUpdAPlane + t * 16;
 #pragma unroll
-                for (int j = 0; j < 8; ++j)
-                    v[j] += ((long long)(int)hh[j] << 16) + (((long long)(int)x1[j] + (long long)(int)x2[j]) << 8) +
-                            (long long)(int)ll[j];
+                for (int m = 0; m < kMost; ++m) {
+                    if (m * 16 >= bn) break;
+                    const int4 h = *(const int4*)(sb + m * 2048);
+                    const uint4 l = *(const uint4*)(sb + b_plane + m * 2048);
+                    hi[m] = __dp4a(h.x, 0x01010101, hi[m]); lo[m] = (int)__dp4a(l.x, 0x01010101u, (unsigned)lo[m]);
+                    hi[m] = __dp4a(h.y, 0x01010101, hi[m]); lo[m] = (int)__dp4a(l.y, 0x01010101u, (unsigned)lo[m]);
+                    hi[m] = __dp4a(h.z, 0x01010101, hi[m]); lo[m] = (int)__dp4a(l.z, 0x01010101u, (unsigned)lo[m]);
+                    hi[m] = __dp4a(h.w, 0x01010101, hi[m]); lo[m] = (int)__dp4a(l.w, 0x01010101u, (unsigned)lo[m]);
+                }
             }
+            if (++turn == p.cchunks) turn = 0;
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&empty_bar[s]);
+            if (++s == p.nstages) { s = 0; parity ^= 1u; }
+        }
+#pragma unroll
+        for (int m = 0; m < kMost; ++m) {
+            if (m * 16 >= bn) break;
+            long long v = 256LL * hi[m] + lo[m];
+            for (int o = 1; o < 8; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+            const int row = (t >> 3) + 16 * m, k = ktile * kt + row / npix;
+            if ((t & 7) == 0 && row < kt * npix && k < p.K && ok && v)
+                atomicAdd(p.acc + (long long)p.C * p.R * p.S * p.K + k, (unsigned long long)v);
+        }
+    }
+    __syncwarp();
+    __syncthreads();                                  // (every reader is done with the ring)
+
+    // exact sums of this slice: tensor memory -> shared memory [row][column], then added up per tap
+    bool ok = mbar_wait_relaxed(tmem_full, 0);
+    if (!ok) atomicExch(fail_flag, 1);
+    tc_fence_after();
+    long long* red = (long long*)ring;
+    const int pitch = bn + 1;                         // odd: the 32 rows of a store fall into different banks
+    {
+        const int quarter = warp & 3, half = warp >> 2, row = quarter * 32 + lane;
+        const unsigned a0 = tmem_base + ((unsigned)(quarter * 32) << 16);
+        for (int c0 = half * 8; c0 < bn; c0 += 16) {
+            unsigned hh[8], xx[8], ll[8];
+            tmem_ld8(a0 + c0, hh); tmem_ld8(a0 + bn + c0, xx); tmem_ld8(a0 + 2 * bn + c0, ll);
+            tmem_ld_wait();
 #pragma unroll
             for (int j = 0; j < 8; ++j)
-                if (valid && c0 + j < kt && ktile * kt + c0 + j < p.K) out[c0 + j] = v[j] + fix;
+                red[row * pitch + c0 + j] =
+                    ((long long)(int)hh[j] << 16) + ((long long)(int)xx[j] << 8) + (long long)ll[j];
         }
     }
     tc_fence_before();
@@ -1709,108 +1710,211 @@ conv_update_kernel(const __grid_constant__ CUtensorMap mapI0, const __grid_const
         tc_fence_after();
         tmem_dealloc(tmem_base, p.tmem_cols);
     }
-    if (threadIdx.x == 0 && *fail_flag && p.status) atomicExch(p.status, 1);
+    ok = *fail_flag == 0;
+    const int rs = p.R * p.S, n_out = p.cu * rs * kt;
+    for (int i = threadIdx.x; i < n_out; i += kUpdThreads) {
+        const int k = i % kt, t = i / kt, tap = t % rs, c = t / rs, r = tap / p.S, s = tap - r * p.S;
+        const int cg = chunk * p.cu + c, kg = ktile * kt + k;
+        if (cg >= p.C || kg >= p.K || !ok) continue;
+        long long v = 0;
+        for (int a = 0; a < p.gh; ++a)
+            for (int b = 0; b < p.gw; ++b)
+                v += red[((c * p.wh + r + a * p.str_h) * p.ww + s + b * p.str_w) * pitch + k * npix + a * p.gw + b];
+        if (v) atomicAdd(p.acc + ((long long)cg * rs + tap) * p.K + kg, (unsigned long long)v);
+    }
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        unsigned* tile = p.arrived + blockIdx.y;
+        unsigned* col = p.arrived + p.cchunks * p.ntn + ktile;
+        last[0] = atomicAdd(tile, 1u) == (unsigned)p.nsplit - 1u;
+        if (last[0]) *tile = 0;
+        last[1] = p.bias && atomicAdd(col, 1u) == (unsigned)(p.nsplit * p.cchunks) - 1u;
+        if (last[1]) *col = 0;
+        if (*fail_flag && p.status) atomicExch(p.status, 1);
+    }
+    __syncthreads();
+    if (!last[0] && !last[1]) return;
+    __threadfence();
+    const float scale_e = p.table[p.slotE].scale;
+    if (last[0]) {
+        const int sh = -ilogbf(p.table[p.slotI].scale * scale_e * (p.probe ? 1.0f : p.table[p.slotU].inv_scale));
+        int stat = 0;
+        unsigned long long pmax = 0;
+        for (int i = threadIdx.x; i < n_out; i += kUpdThreads) {
+            const int k = i % kt, t = i / kt, tap = t % rs, cg = chunk * p.cu + t / rs, kg = ktile * kt + k;
+            if (cg >= p.C || kg >= p.K) continue;
+            const long long at = ((long long)cg * rs + tap) * p.K + kg;
+            const long long v = (long long)__ldcg(p.acc + at);
+            p.acc[at] = 0;
+            if (p.probe) {
+                const unsigned long long m = (unsigned long long)(v < 0 ? -v : v);
+                pmax = m > pmax ? m : pmax;
+            } else {
+                const int q = rescale_i64(v, sh), m = q < 0 ? -q : q;
+                stat = m > stat ? m : stat;
+                p.U[at] = (short)q;
+            }
+        }
+        if (p.probe) update_max(pmax, [&](unsigned long long m) { atomicMax(p.probe_out, m); });
+        else update_max(stat, [&](int m) { atomicMax(p.stats + p.slotU, m); });
+    }
+    if (last[1]) {
+        // an elementwise sum's quantisation: truncation toward zero
+        const int sh = -ilogbf(scale_e * (p.probe ? 1.0f : p.table[p.slotB].inv_scale));
+        int stat = 0;
+        unsigned long long pmax = 0;
+        for (int k = threadIdx.x; k < kt; k += kUpdThreads) {
+            const int kg = ktile * kt + k;
+            if (kg >= p.K) continue;
+            unsigned long long* at = p.acc + (long long)p.C * rs * p.K + kg;
+            const long long v = (long long)__ldcg(at);
+            *at = 0;
+            const unsigned long long m = (unsigned long long)(v < 0 ? -v : v);
+            if (p.probe) {
+                pmax = m > pmax ? m : pmax;
+                continue;
+            }
+            unsigned long long q = sh >= 63 ? 0 : sh >= 0 ? m >> sh : m >= 32768 || sh <= -16 ? (m ? 32768 : 0) : m << -sh;
+            const unsigned long long most = v < 0 ? 32768 : 32767;
+            q = q > most ? most : q;
+            stat = (int)q > stat ? (int)q : stat;
+            p.bias[kg] = (short)(v < 0 ? -(int)q : (int)q);
+        }
+        if (p.probe) update_max(pmax, [&](unsigned long long m) { atomicMax(p.probe_out + 1, m); });
+        else update_max(stat, [&](int m) { atomicMax(p.stats + p.slotB, m); });
+    }
 }
 
 struct UpdShape {
     bool ok;
-    int cu, cchunks, ntn, kt, bn, tmem_cols, nstages, smem, nkb, per, nsplit;
-    size_t act_plane, err_plane, partial_bytes, bytes;
+    int gh, gw, wh, ww, cu, cchunks, ntn, kt, bn, tmem_cols, ksteps, nstages, smem, tw, nblk, nkb, per, nsplit;
+    size_t act_plane, err_plane, acc_bytes;
+    long long cost;
 };
 
-UpdShape update_implicit_shape(int mode, const ConvGeom& g) {
-    UpdShape u;
-    u.ok = false;
-    const int rs = g.R * g.S;
-    const long long cols = (long long)g.P * g.Q * g.N;
-    if (mode != MODE_FLEX16 || g.N % 128 != 0 || g.dil_h != 1 || g.dil_w != 1 || rs > 128 ||
-        !flat_depth(g) ||
-        g.R > 256 || g.S > 256 || cols >= (1LL << 31) - 256 || getenv("B2_CONV_IM2COL"))
-        return u;
-    const int cu_max = 128 / rs;
+// Cycles of a k-block: the tensor core's rate, the shared memory its operands are read from, the
+// bytes from L2; measured constants.
+UpdShape update_shape_for(const ConvGeom& g, int gh, int gw) {
+    UpdShape u = {};
+    u.gh = gh; u.gw = gw; u.wh = (gh - 1) * g.str_h + g.R; u.ww = (gw - 1) * g.str_w + g.S;
+    const int win = u.wh * u.ww, npix = gh * gw;
+    const long long th = (g.P + gh - 1) / gh, nblk = image_blocks(g.N);
+    u.tw = (g.Q + gw - 1) / gw; u.nblk = (int)nblk;
+    if (win > 128 || th * u.tw * nblk >= (1LL << 30)) return u;
+    const int cu_max = 128 / win;
     u.cchunks = (g.C + cu_max - 1) / cu_max;
     u.cu = (g.C + u.cchunks - 1) / u.cchunks;
-    u.ntn = (g.K + 62) / 63;                       // two accumulator sets of 4*bn columns in 512
+    const int kt_max = kUpdMaxN / npix;
+    u.ntn = (g.K + kt_max - 1) / kt_max;
     u.kt = (g.K + u.ntn - 1) / u.ntn;
-    u.bn = round_up(u.kt + 1, 16);
+    u.bn = round_up(u.kt * npix, 16);
     u.tmem_cols = 32;
-    while (u.tmem_cols < 8 * u.bn) u.tmem_cols *= 2;
+    while (u.tmem_cols < 3 * u.bn) u.tmem_cols *= 2;
     const int stage = 2 * kUpdAPlane + 2 * u.bn * kKBytes;
     u.nstages = (kConvSmemMax - kUpdSmemFixed) / stage;
     if (u.nstages > kUpdMaxStages) u.nstages = kUpdMaxStages;
-    if (u.nstages < 2) return u;
+    if (u.nstages < 2 || (long long)u.cchunks * u.ntn > 65535) return u;
     u.smem = kUpdSmemFixed + u.nstages * stage;
-    u.nkb = (int)(cols / 128);
-    int slices = 148 / (u.cchunks * u.ntn);
-    if (slices < 1) slices = 1;
+    u.nkb = (int)(th * u.tw * nblk);
+    const int images = g.N < 128 ? g.N : 128;
+    u.ksteps = (images + 31) / 32;
+    const int cols = u.cchunks * u.ntn;
+    int slices = cols < 148 ? 148 / cols : 1;
     u.per = (u.nkb + slices - 1) / slices;
     if (u.per > 256) u.per = 256;                  // the int32 sums stay exact up to 32768 terms
     u.nsplit = (u.nkb + u.per - 1) / u.per;
-    u.act_plane = (((size_t)g.C * g.H * g.W * g.N) + 1023) / 1024 * 1024;
-    u.err_plane = (((size_t)g.K * cols) + 1023) / 1024 * 1024;
-    u.partial_bytes = (size_t)u.nsplit * g.C * rs * g.K * sizeof(long long);
-    u.bytes = 2 * u.act_plane + 2 * u.err_plane + align1k(u.partial_bytes);
+    const long long mma = 16LL * u.ksteps / 4 * (u.bn / 2 > 32 + u.bn / 4 ? u.bn / 2 : 32 + u.bn / 4);
+    const long long bytes = 2LL * images * (u.cu * win + u.kt * npix) / 56;
+    u.cost = ((long long)cols * u.nsplit + 147) / 148 * (u.per * ((mma > bytes ? mma : bytes) + 60) + 3000 + 40 * u.bn);
+    u.act_plane = plane_size(g.C, g.H, g.W, g.N);
+    u.err_plane = plane_size(g.K, g.P, g.Q, g.N);
+    u.acc_bytes = align1k((((size_t)g.C * g.R * g.S + 1) * g.K) * 8 + (size_t)(cols + u.ntn) * 4);
     u.ok = true;
     return u;
 }
 
-template <typename T, int MODE>
-int run_update_implicit(const T* I, const T* E, void* U, const ConvGeom& g, const UpdShape& u,
-                        const b2_flex_scale* table, int slotI, int slotE, int slotU, int* stats,
-                        void* scratch, size_t scratch_bytes, unsigned long long* probe_out,
-                        int* status, int probe, cudaStream_t st) {
+UpdShape update_implicit_shape(int mode, const ConvGeom& g) {
+    UpdShape best = {};
+    if (mode != MODE_FLEX16 || g.dil_h != 1 || g.dil_w != 1 || !flat_depth(g) || getenv("B2_CONV_IM2COL"))
+        return best;
+    for (int gh = 1; gh <= 2; ++gh)
+        for (int gw = 1; gw <= 2; ++gw) {
+            const UpdShape u = update_shape_for(g, gh, gw);
+            if (u.ok && (!best.ok || u.cost < best.cost)) best = u;
+        }
+    return best;
+}
+
+struct UpdOut {
+    void *U, *bias;
+    const b2_flex_scale* table;
+    int slotI, slotE, slotU, slotB;
+    int* stats;
+    unsigned long long* probe_out;
+    int* status;
+    int probe;
+};
+
+int run_update_planes(const void* act_planes, const void* err_planes, void* acc, const ConvGeom& g,
+                      const UpdShape& u, const UpdOut& o, cudaStream_t st) {
     int rc = get_encode();
     if (rc) return rc;
-    B2_REQUIRE(scratch && scratch_bytes >= u.bytes && ((uintptr_t)scratch & 1023) == 0,
-               "convolution update needs %zu bytes of 1024-byte aligned scratch, got %zu", u.bytes,
-               scratch_bytes);
-    unsigned char* base = (unsigned char*)scratch;
-    unsigned char* eplanes = base + 2 * u.act_plane;
-    long long* partial = (long long*)(eplanes + 2 * u.err_plane);
-    const long long n_act = (long long)g.C * g.H * g.W * g.N, n_err = (long long)g.K * g.P * g.Q * g.N;
-    long long blocks = (n_act / 8 + 255) / 256;
-    if (blocks > 148 * 16) blocks = 148 * 16;
-    split_same_layout_kernel<T, MODE><<<(unsigned)(blocks < 1 ? 1 : blocks), 256, 0, st>>>(
-        I, n_act, base, base + u.act_plane, 0u);
-    blocks = (n_err / 8 + 255) / 256;
-    if (blocks > 148 * 16) blocks = 148 * 16;
-    // the error tensor's low plane as signed bytes (low - 128): both of its planes then make one
-    // signed operand
-    split_same_layout_kernel<T, MODE><<<(unsigned)(blocks < 1 ? 1 : blocks), 256, 0, st>>>(
-        E, n_err, eplanes, eplanes + u.err_plane, 0x80808080u);
-    B2_CUDA(cudaGetLastError());
+    B2_REQUIRE((((uintptr_t)act_planes | (uintptr_t)err_planes | (uintptr_t)acc) & 1023) == 0,
+               "planes and workspace must be 1024-byte aligned");
+    unsigned char *I0 = (unsigned char*)act_planes, *E0 = (unsigned char*)err_planes;
+    ConvGeom e = g;
+    e.C = g.K; e.H = g.P; e.W = g.Q;
     CUtensorMap mI0, mI1, mE0, mE1;
-    if ((rc = make_map_4d(&mI0, base, g, u.cu, g.R, g.S))) return rc;
-    if ((rc = make_map_4d(&mI1, base + u.act_plane, g, u.cu, g.R, g.S))) return rc;
-    const int cols = g.P * g.Q * g.N;
-    if ((rc = make_map(&mE0, eplanes, g.K, cols, 1, u.kt))) return rc;
-    if ((rc = make_map(&mE1, eplanes + u.err_plane, g.K, cols, 1, u.kt))) return rc;
+    if ((rc = make_map_4d(&mI0, I0, g, u.cu, u.wh, u.ww))) return rc;
+    if ((rc = make_map_4d(&mI1, I0 + u.act_plane, g, u.cu, u.wh, u.ww))) return rc;
+    if ((rc = make_map_4d(&mE0, E0, e, u.kt, u.gh, u.gw))) return rc;
+    if ((rc = make_map_4d(&mE1, E0 + u.err_plane, e, u.kt, u.gh, u.gw))) return rc;
     UpdTileParams p;
-    p.Q = g.Q; p.nblk = g.N / 128; p.nkb = u.nkb;
-    p.pad_h = g.pad_h; p.pad_w = g.pad_w; p.str_h = g.str_h; p.str_w = g.str_w;
-    p.cu = u.cu; p.rs = g.R * g.S; p.C = g.C; p.K = g.K;
-    p.ntn = u.ntn; p.kt = u.kt; p.bn = u.bn; p.per = u.per;
-    p.nstages = u.nstages; p.tmem_cols = u.tmem_cols;
-    p.box_a = (unsigned)(u.cu * g.R * g.S * kKBytes); p.box_b = (unsigned)(u.kt * kKBytes);
-    p.partial = partial; p.status = status;
+    p.tw = u.tw; p.nblk = u.nblk; p.nkb = u.nkb;
+    p.off_h = -g.pad_h; p.off_w = -g.pad_w; p.step_h = u.gh * g.str_h; p.step_w = u.gw * g.str_w;
+    p.str_h = g.str_h; p.str_w = g.str_w;
+    p.gh = u.gh; p.gw = u.gw; p.wh = u.wh; p.ww = u.ww; p.R = g.R; p.S = g.S;
+    p.cu = u.cu; p.C = g.C; p.K = g.K; p.cchunks = u.cchunks;
+    p.ntn = u.ntn; p.kt = u.kt; p.bn = u.bn; p.per = u.per; p.nsplit = u.nsplit;
+    p.ksteps = u.ksteps; p.nstages = u.nstages; p.tmem_cols = u.tmem_cols;
+    p.box_a = (unsigned)(u.cu * u.wh * u.ww * kKBytes); p.box_b = (unsigned)(u.kt * u.gh * u.gw * kKBytes);
+    p.acc = (unsigned long long*)acc;
+    p.arrived = (unsigned*)(p.acc + ((size_t)g.C * g.R * g.S + 1) * g.K);
+    p.U = (short*)o.U; p.bias = (short*)o.bias; p.table = o.table;
+    p.slotI = o.slotI; p.slotE = o.slotE; p.slotU = o.slotU; p.slotB = o.slotB;
+    p.stats = o.stats; p.probe_out = o.probe_out; p.status = o.status; p.probe = o.probe;
     static bool attr_set = false;
     if (!attr_set) {
         B2_CUDA(cudaFuncSetAttribute(conv_update_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      kConvSmemMax));
         attr_set = true;
     }
-    dim3 grid(u.nsplit, u.cchunks * u.ntn);
-    conv_update_kernel<<<grid, kUpdThreads, u.smem, st>>>(mI0, mI1, mE0, mE1, p);
-    B2_CUDA(cudaGetLastError());
-    GemmParams gp;
-    const int rows = g.C * g.R * g.S;
-    fill_params(&gp, rows, g.K, g.K, U, 0, table, slotI, slotE, slotU, stats, probe_out, status, probe);
-    gp.partial = partial; gp.Mp = rows; gp.Np = g.K; gp.kb_per_split = u.per;
-    long long fb = ((long long)rows * g.K + 31) / 32;
-    if (fb > 148 * 16) fb = 148 * 16;
-    splitk_finish_kernel<MODE><<<(unsigned)fb, 256, 0, st>>>(gp, u.nsplit);
+    conv_update_kernel<<<dim3(u.nsplit, u.cchunks * u.ntn), kUpdThreads, u.smem, st>>>(mI0, mI1, mE0, mE1, p);
     B2_CUDA(cudaGetLastError());
     return B2_OK;
+}
+
+// from int16 tensors: whole tiles of 128 images, as the entry point's scratch has always been sized
+inline bool update_goes_in_planes(int mode, const ConvGeom& g, UpdShape* u) {
+    *u = update_implicit_shape(mode, g);
+    return u->ok && g.N % 128 == 0;
+}
+inline size_t update_planes_bytes(const UpdShape& u) { return 2 * u.act_plane + 2 * u.err_plane + u.acc_bytes; }
+
+int run_update_implicit(const short* I, const short* E, const ConvGeom& g, const UpdShape& u, const UpdOut& o,
+                        void* scratch, size_t scratch_bytes, cudaStream_t st) {
+    B2_REQUIRE(scratch && scratch_bytes >= update_planes_bytes(u) && ((uintptr_t)scratch & 1023) == 0,
+               "convolution update needs %zu bytes of 1024-byte aligned scratch, got %zu",
+               update_planes_bytes(u), scratch_bytes);
+    unsigned char* base = (unsigned char*)scratch;
+    unsigned char* eplanes = base + 2 * u.act_plane;
+    unsigned char* acc = eplanes + 2 * u.err_plane;
+    int rc = split_to_planes(I, g.C, g.H, g.W, g.N, base, u.act_plane, st);
+    if (rc) return rc;
+    if ((rc = split_to_planes(E, g.K, g.P, g.Q, g.N, eplanes, u.err_plane, st))) return rc;
+    B2_CUDA(cudaMemsetAsync(acc, 0, u.acc_bytes, st));
+    return run_update_planes(base, eplanes, acc, g, u, o, st);
 }
 
 template <typename T, int MODE>
@@ -1822,10 +1926,11 @@ int run_update(const T* I, const T* E, void* U, const b2_conv_dims* d, const b2_
     if (rc) return rc;
     B2_REQUIRE(I && E && U, "null tensor");
     {
-        const UpdShape u = update_implicit_shape(MODE, g);
-        if (u.ok)
-            return run_update_implicit<T, MODE>(I, E, U, g, u, table, slotI, slotE, slotU, stats,
-                                                scratch, scratch_bytes, probe_out, status, probe, st);
+        UpdShape u;
+        if (update_goes_in_planes(MODE, g, &u)) {
+            const UpdOut o = {U, nullptr, table, slotI, slotE, slotU, -1, stats, probe_out, status, probe};
+            return run_update_implicit((const short*)I, (const short*)E, g, u, o, scratch, scratch_bytes, st);
+        }
     }
     const long long kg_ll = (long long)g.M * g.P * g.Q * g.N;
     B2_REQUIRE(kg_ll < (1LL << 31) - 256 && (long long)g.C * g.D * g.H * g.W * g.N < (1LL << 31) &&
@@ -1936,8 +2041,9 @@ extern "C" int b2_conv_launches(int32_t flex, const b2_conv_dims* d, int32_t pas
     const int mode = flex ? MODE_FLEX16 : MODE_F32X3;
     ConvGeom gp;
     b2_direct_args direct;
+    UpdShape u;
     if (pass == 2)
-        *launches = update_implicit_shape(mode, g).ok || update_shape(mode, g).splits > 1 ? 4 : 3;
+        *launches = !update_goes_in_planes(mode, g, &u) && update_shape(mode, g).splits > 1 ? 4 : 3;
     else
         *launches = !(flex && pass_geom(g, pass, &gp)) && conv_goes_direct(mode, g, pass, &direct) ? 1 : 3;
     return B2_OK;
@@ -2009,6 +2115,12 @@ extern "C" int b2_conv_split_activations(const int16_t* X, const b2_conv_dims* d
     B2_REQUIRE(X && planes && pass_geom(f, pass, &g), "planes are not available for this convolution");
     return implicit_split_activations<short, MODE_FLEX16>(X, g, implicit_shape(g), planes,
                                                           (cudaStream_t)stream);
+}
+
+extern "C" int b2_conv_split_planes(const int16_t* X, int32_t c, int32_t h, int32_t w, int32_t n,
+                                    void* planes, void* stream) {
+    B2_REQUIRE(X && planes && c > 0 && h > 0 && w > 0 && n > 0 && ((uintptr_t)planes & 1023) == 0, "bad argument");
+    return split_to_planes(X, c, h, w, n, planes, plane_size(c, h, w, n), (cudaStream_t)stream);
 }
 
 extern "C" int b2_conv_filter_planes(const int16_t* F, const b2_conv_dims* d, int32_t pass,
@@ -2096,9 +2208,40 @@ extern "C" int b2_conv_update_scratch_bytes(int32_t flex, const b2_conv_dims* d,
     int rc = geom_from(d, &g);
     if (rc) return rc;
     B2_REQUIRE(bytes, "null argument");
-    const UpdShape u = update_implicit_shape(flex ? MODE_FLEX16 : MODE_F32X3, g);
-    *bytes = u.ok ? u.bytes : update_shape(flex ? MODE_FLEX16 : MODE_F32X3, g).bytes;
+    UpdShape u;
+    *bytes = update_goes_in_planes(flex ? MODE_FLEX16 : MODE_F32X3, g, &u)
+                 ? update_planes_bytes(u) : update_shape(flex ? MODE_FLEX16 : MODE_F32X3, g).bytes;
     return B2_OK;
+}
+
+extern "C" int b2_conv_update_planes_info(const b2_conv_dims* d, int32_t* supported, size_t* workspace_bytes) {
+    ConvGeom g;
+    int rc = geom_from(d, &g);
+    if (rc) return rc;
+    B2_REQUIRE(supported && workspace_bytes, "null argument");
+    const UpdShape u = update_implicit_shape(MODE_FLEX16, g);
+    *supported = u.ok ? 1 : 0;
+    *workspace_bytes = u.ok ? u.acc_bytes : 0;
+    return B2_OK;
+}
+
+extern "C" int b2_conv_update_flex16_planes(const void* act_planes, const void* err_planes, int16_t* U,
+                                            int16_t* bias_grad, const b2_conv_dims* d,
+                                            const b2_flex_scale* table, int32_t slotI, int32_t slotE,
+                                            int32_t slotU, int32_t slotB, int32_t* stats, void* workspace,
+                                            uint64_t* probe_out, int32_t* status, int32_t probe, void* stream) {
+    ConvGeom g;
+    int rc = geom_from(d, &g);
+    if (rc) return rc;
+    B2_REQUIRE(act_planes && err_planes && U && workspace, "null tensor");
+    B2_REQUIRE(table && slotI >= 0 && slotE >= 0 && slotU >= 0 && (!bias_grad || slotB >= 0),
+               "flex conv needs the scale table");
+    B2_REQUIRE(probe ? probe_out != nullptr : stats != nullptr, "missing statistics destination");
+    const UpdShape u = update_implicit_shape(MODE_FLEX16, g);
+    B2_REQUIRE(u.ok, "this filter gradient does not read planes");
+    const UpdOut o = {U, bias_grad, table, slotI, slotE, slotU, slotB, stats, (unsigned long long*)probe_out,
+                      status, probe ? 1 : 0};
+    return run_update_planes(act_planes, err_planes, workspace, g, u, o, (cudaStream_t)stream);
 }
 
 extern "C" int b2_conv_update_f32(const float* I, const float* E, float* U, const b2_conv_dims* d,

@@ -54,7 +54,7 @@ class _Step(object):
             t._probe64.zero_()
             call(1)
             t.kernel_launches += self.launches
-            imax = int(t._probe64.item())
+            imax = int(t._probe64[0].item())
             if getattr(self, "probe_is_float", False):
                 # fused epilogue: the kernel leaves the bit pattern of max |fp32 result|
                 real = float(np.array([imax & 0xffffffff], dtype=np.uint32).view(np.float32)[0])
@@ -68,11 +68,13 @@ class _Step(object):
 
 
 class _PlaneUser(object):
-    """flex16 convolution steps that can run on the implicit-GEMM tile kernel: the streamed
-    tensor (activations for the forward pass, the error tensor for the input gradient) is read as
-    two byte planes which its producer writes directly, and the filter planes are kept for as long
-    as the filters do not change -- one launch per convolution."""
+    """flex16 convolution steps that can run on the implicit-GEMM tile kernels: the streamed
+    tensors (activations, the error tensor) are read as two byte planes which their producer
+    writes directly -- or else the first step that reads them -- and the filter planes are kept for
+    as long as the filters do not change: one launch per convolution."""
     use_planes = False
+    plane_args = ()                 # indexes of the tensors read as planes in op.args / in_views
+    splits = ()                     # those that this step splits unless their producer has
     filter_planes = None
     filter_version = None
 
@@ -84,16 +86,34 @@ class _PlaneUser(object):
             return
         self.use_planes = True
         self.conv_pass = conv_pass
-        self.plane_arg = stream_arg          # index of the streamed tensor in op.args / in_views
         self.filter_arg = filter_arg
         self.filter_bytes = filt_bytes
         self.in_views[filter_arg].buffer.watched = True
-        buf = self.in_views[stream_arg].buffer
-        buf.plane_bytes = lib.plane_bytes(self.in_views[stream_arg].axes.lengths)
-        # (planes whose rows of images are padded are written by the convolutions only)
-        buf.plane_dense = self.dims.N % 16 == 0
-        buf.plane_steps = getattr(buf, "plane_steps", []) + [self]
+        self._read_planes((stream_arg,))
+
+    def _read_planes(self, args):
+        self.plane_args = self.splits = args
+        for k in args:
+            buf = self.in_views[k].buffer
+            buf.plane_bytes = lib.plane_bytes(self.in_views[k].axes.lengths)
+            # (planes whose rows of images are padded are written by the convolutions only)
+            buf.plane_dense = self.dims.N % 16 == 0
+            buf.plane_steps = getattr(buf, "plane_steps", []) + [self]
         self.launches = 1
+
+    def _planes(self, t, k):
+        """Address of the planes of argument k."""
+        v = self.in_views[k]
+        if k in self.splits and not v.buffer.planes_by_producer:
+            d = self.dims
+            lengths = (d.K, d.P, d.Q, d.N) if self.streams_errors(k) else (d.C, d.H, d.W, d.N)
+            lib.check(lib.raw().b2_conv_split_planes(self._ptr(v), *lengths, v.buffer.planes_ptr,
+                                                     t.stream.cuda_stream))
+            t.kernel_launches += 1
+        return v.buffer.planes_ptr
+
+    def streams_errors(self, k):
+        return False
 
     def allocate(self, t):
         if self.use_planes and self.filter_planes is None and not t.plan_only:
@@ -117,17 +137,21 @@ class _PlaneUser(object):
         if fbuf.last_write_step < 0 and self.filter_version != fbuf.version:
             self._build_filter_planes(t)
 
+    def _add_tail_views(self, t, epilogue):
+        for key in ("bias", "residual", "mask"):
+            if epilogue.get(key) is not None:
+                v = t._view_of(epilogue[key])
+                if not v.is_dense():
+                    raise ValueError("fused convolution %s must be a dense tensor" % key)
+                self.in_views.append(v)
+
     def _launch_planes(self, t):
-        xv, fv = self.in_views[self.plane_arg], self.in_views[self.filter_arg]
+        xv, fv = self.in_views[self.plane_args[0]], self.in_views[self.filter_arg]
         ov = self.out_views[0]
         raw = lib.raw()
         st = t.stream.cuda_stream
         xbuf, fbuf = xv.buffer, fv.buffer
-        planes_ptr = xbuf.planes_ptr
-        if not xbuf.planes_by_producer:
-            lib.check(raw.b2_conv_split_activations(self._ptr(xv), C.byref(self.dims),
-                                                    self.conv_pass, planes_ptr, st))
-            t.kernel_launches += 1
+        planes_ptr = self._planes(t, self.plane_args[0])
         if fbuf.last_write_step >= 0:
             self._build_filter_planes(t)     # filters written inside this computation
         else:
@@ -152,6 +176,9 @@ class _PlaneUser(object):
         if epi.get("residual") is not None:
             ce.residual = self._ptr(extra[k])
             ce.slot_residual = t._slot_for_read(extra[k].buffer, self)
+            k += 1
+        if epi.get("mask") is not None:
+            ce.mask = self._ptr(extra[k])
         ce.relu = int(bool(epi.get("relu")))
         obuf = ov.buffer
         ce.write_int16 = int(self.write_int16 or obuf.plane_bytes == 0)
@@ -276,12 +303,7 @@ class ConvStep(_PlaneUser, _Step):
                 raise ValueError("a fused convolution epilogue needs a kernel that takes one")
             self.probe_is_float = True
             self.write_int16 = True          # the planner clears it when only planes are read
-            for key in ("bias", "residual"):
-                if epilogue.get(key) is not None:
-                    v = t._view_of(epilogue[key])
-                    if not v.is_dense():
-                        raise ValueError("fused convolution %s must be a dense tensor" % key)
-                    self.in_views.append(v)
+            self._add_tail_views(t, epilogue)
 
     def launch(self, t):
         if self.use_planes:
@@ -317,10 +339,12 @@ class ConvStep(_PlaneUser, _Step):
         self._flex_probe_then(t, ov.buffer, [iv.buffer, fv.buffer], call)
 
 
-def takes_conv_tail(fprop, t):
-    """Whether the forward convolution's kernel evaluates the layer's elementwise tail: the flex16
-    tile kernel, the fp32 kernel that gathers its operands."""
+def takes_conv_tail(fprop, t, conv_pass=lib.CONV_FPROP):
+    """Whether the convolution's kernel evaluates the elementwise tail behind it: the flex16 tile
+    kernel, for the forward pass the fp32 kernel that gathers its operands."""
     d = _conv_dims_of(fprop, t)
+    if conv_pass != lib.CONV_FPROP:
+        return t.flex and lib.conv_planes_info(d, conv_pass)[0]
     if t.flex:
         return lib.conv_planes_info(d, lib.CONV_FPROP)[0]
     return lib.conv_launches(False, d, lib.CONV_FPROP) == 1
@@ -349,9 +373,13 @@ class _ConvGradStep(_PlaneUser, _Step):
     launches = 3
     what = None                     # "bprop" | "update"
 
-    def __init__(self, index, op, t):
+    def __init__(self, index, op, t, epilogue=None):
+        """epilogue (input gradient, where takes_conv_tail): dict(out, residual, mask) -- the sum
+        with another gradient and the mask of a ReLU behind it."""
         super(_ConvGradStep, self).__init__(index, op)
-        av, bv, ov = t._view_of(op.args[0]), t._view_of(op.args[1]), t._view_of(op)
+        self.epi = epilogue
+        av, bv = t._view_of(op.args[0]), t._view_of(op.args[1])
+        ov = t._view_of(epilogue["out"] if epilogue else op)
         for v in (av, bv):
             if not v.is_dense():
                 raise ValueError("Unhandled op: convolution %s operands must be dense tensors"
@@ -363,7 +391,11 @@ class _ConvGradStep(_PlaneUser, _Step):
                   "update": ((d.K, d.M, d.P, d.Q, d.N), (d.C, d.D, d.H, d.W, d.N),
                              (d.C, d.T, d.R, d.S, d.K))}[self.what]
         for v, shape in zip((av, bv, ov), expect):
-            if tuple(v.axes.lengths) != shape:
+            if v is ov and epilogue:
+                same = ov.is_dense() and [n for n in v.axes.lengths if n != 1] == [n for n in shape if n != 1]
+            else:
+                same = tuple(v.axes.lengths) == shape
+            if not same:
                 raise ValueError("convolution %s: tensor of shape %s where %s is expected"
                                  % (self.what, tuple(v.axes.lengths), shape))
         self.in_views = [av, bv]
@@ -376,11 +408,17 @@ class _ConvGradStep(_PlaneUser, _Step):
             self.flex, d, lib.CONV_BPROP if self.what == "bprop" else lib.CONV_UPDATE)
         if self.what == "bprop":
             self._setup_planes(t, lib.CONV_BPROP, 0, 1)      # streamed: delta; filters: args[1]
+        if epilogue:
+            if not self.use_planes:
+                raise ValueError("a fused convolution epilogue needs a kernel that takes one")
+            self.probe_is_float = True
+            self.write_int16 = True          # the planner clears it when only planes are read
+            self._add_tail_views(t, epilogue)
 
     def launch(self, t):
         if self.use_planes:
             return self._launch_planes(t)
-        av, bv = self.in_views           # (delta, filters) or (delta, inputs)
+        av, bv = self.in_views[:2]       # (delta, filters) or (delta, inputs)
         ov = self.out_views[0]
         raw = lib.raw()
         sp, sb = t._scratch_aligned()
@@ -405,6 +443,9 @@ class _ConvGradStep(_PlaneUser, _Step):
                           sp, sb, t._probe64.data_ptr(), t._status.data_ptr(), probe, st))
         self._flex_probe_then(t, ov.buffer, [first.buffer, second.buffer], call)
 
+    def streams_errors(self, k):
+        return k == 0
+
 
 class ConvBpropStep(_ConvGradStep):
     """Input gradient of a convolution: args (delta K,M,P,Q,N ; filters C,T,R,S,K)."""
@@ -416,6 +457,55 @@ class ConvUpdateStep(_ConvGradStep):
     """Filter gradient of a convolution: args (delta K,M,P,Q,N ; inputs C,D,H,W,N)."""
     kind = "conv_update"
     what = "update"
+    workspace = None
+
+    def __init__(self, index, op, t, bias_op=None):
+        """bias_op (where the gradient reads planes): the reduction that sums the delta over all
+        axes but the channels, evaluated in the same kernel."""
+        super(ConvUpdateStep, self).__init__(index, op, t)
+        self.reads_planes, self.workspace_bytes = False, 0
+        if self.flex:
+            self.reads_planes, self.workspace_bytes = lib.conv_update_planes_info(self.dims)
+        if self.reads_planes:
+            self.scratch_bytes = 0
+            self._read_planes((0, 1))
+        self.bias_op = bias_op
+        if bias_op is not None:
+            if not self.reads_planes:
+                raise ValueError("a fused bias gradient needs the kernel that reads planes")
+            self.out_views.append(t._view_of(bias_op))
+
+    def allocate(self, t):
+        if self.reads_planes and self.workspace is None and not t.plan_only:
+            self.workspace = t.torch.zeros((self.workspace_bytes + 1024,), dtype=t.torch.uint8,
+                                           device=t.device)
+            self.workspace_ptr = self.workspace.data_ptr() + (-self.workspace.data_ptr()) % 1024
+
+    def launch(self, t):
+        if not self.reads_planes:
+            return super(ConvUpdateStep, self).launch(t)
+        ev, iv = self.in_views
+        outs = [v.buffer for v in self.out_views]
+        errors, acts = self._planes(t, 0), self._planes(t, 1)
+        slot_i, slot_e = t._slot_for_read(iv.buffer, self), t._slot_for_read(ev.buffer, self)
+        bias = self.out_views[1] if self.bias_op is not None else None
+
+        def call(probe):
+            lib.check(lib.raw().b2_conv_update_flex16_planes(
+                acts, errors, self._ptr(self.out_views[0]), self._ptr(bias) if bias else None,
+                C.byref(self.dims), t._table.data_ptr(), slot_i, slot_e, outs[0].slot_write,
+                bias.buffer.slot_write if bias else -1, t._stats.data_ptr(), self.workspace_ptr,
+                t._probe64.data_ptr(), t._status.data_ptr(), probe, t.stream.cuda_stream))
+            t.kernel_launches += 1
+        if not all(b.entry.initialized for b in outs):
+            t._probe64.zero_()
+            call(1)
+            scales = (iv.buffer.entry.scale * ev.buffer.entry.scale, ev.buffer.entry.scale)
+            for b, most, scale in zip(outs, t._probe64.tolist(), scales):
+                if not b.entry.initialized:
+                    t._set_table_row(b.slot_write, b.entry.initialize_from_range(float(most) * scale))
+                    t._stats[b.slot_write:b.slot_write + 1].zero_()
+        call(0)
 
 
 class PoolStep(_Step):

@@ -132,6 +132,7 @@ def _load():
         "b2_conv_planes_info": (C.c_int, [C.POINTER(ConvDims), i32, C.POINTER(i32), C.POINTER(sz),
                                           C.POINTER(sz)]),
         "b2_conv_split_activations": (C.c_int, [vp, C.POINTER(ConvDims), i32, vp, vp]),
+        "b2_conv_split_planes": (C.c_int, [vp, i32, i32, i32, i32, vp, vp]),
         "b2_conv_filter_planes": (C.c_int, [vp, C.POINTER(ConvDims), i32, vp, vp]),
         "b2_conv_flex16_planes": (C.c_int, [i32, vp, vp, vp, C.POINTER(ConvDims), vp, i32, i32,
                                             i32, vp, vp, vp, i32, vp]),
@@ -142,6 +143,9 @@ def _load():
         "b2_conv_bprop_flex16": (C.c_int, [vp, vp, vp, C.POINTER(ConvDims), vp, i32, i32, i32, vp,
                                            vp, sz, vp, vp, i32, vp]),
         "b2_conv_update_scratch_bytes": (C.c_int, [i32, C.POINTER(ConvDims), C.POINTER(sz)]),
+        "b2_conv_update_planes_info": (C.c_int, [C.POINTER(ConvDims), C.POINTER(i32), C.POINTER(sz)]),
+        "b2_conv_update_flex16_planes": (C.c_int, [vp, vp, vp, vp, C.POINTER(ConvDims), vp, i32, i32, i32,
+                                                   i32, vp, vp, vp, vp, i32, vp]),
         "b2_conv_update_f32": (C.c_int, [vp, vp, vp, C.POINTER(ConvDims), vp, sz, vp, vp]),
         "b2_conv_update_flex16": (C.c_int, [vp, vp, vp, C.POINTER(ConvDims), vp, i32, i32, i32, vp,
                                             vp, sz, vp, vp, i32, vp]),
@@ -362,6 +366,13 @@ def conv_planes_info(dims, conv_pass=CONV_FPROP):
     ok, a, f = C.c_int32(), C.c_size_t(), C.c_size_t()
     check(_lib.b2_conv_planes_info(C.byref(dims), conv_pass, C.byref(ok), C.byref(a), C.byref(f)))
     return bool(ok.value), a.value, f.value
+
+
+def conv_update_planes_info(dims):
+    """(supported, bytes of the workspace)."""
+    ok, n = C.c_int32(), C.c_size_t()
+    check(_lib.b2_conv_update_planes_info(C.byref(dims), C.byref(ok), C.byref(n)))
+    return bool(ok.value), n.value
 
 
 def conv_bprop_scratch_bytes(flex, dims):

@@ -460,9 +460,12 @@ class _CallIO(object):
             # the driver's own pipelined copy
             t._stage(view, arr)
             return (buf.staging.data_ptr() if buf.flex else 0), arr
-        lib.check(lib.raw().b2_call_stage(
-            arr.__array_interface__["data"][0], arr.nbytes,
-            self._pinned_buffer(k) if arr.nbytes <= self.STAGED_MOST else None, self.visible))
+        # (the buffer is made only for an argument that needs it: pinning memory takes milliseconds)
+        address, stage = arr.__array_interface__["data"][0], lib.raw().b2_call_stage
+        have = self.pinned[k].data_ptr() if self.pinned[k] is not None else None
+        lib.check(stage(address, arr.nbytes, have, self.visible))
+        if not self.visible.value:
+            lib.check(stage(address, arr.nbytes, self._pinned_buffer(k), self.visible))
         return self.visible.value, arr
 
     def call(self, args):
@@ -504,7 +507,10 @@ class _Planner(object):
         self.consumers = collections.defaultdict(list)
         self.written_buffers = []
         self.conv_tails = {}       # ConvolutionOp -> dict(out, bias, residual, relu, ops)
-        self.conv_tail_of = {}     # absorbed elementwise op -> its ConvolutionOp
+        self.conv_tail_of = {}     # absorbed elementwise op -> its convolution
+        self.bias_sum_of = {}      # update_conv -> the sum of its delta that it evaluates as well
+        self.update_of = {}        # ... and the other way round
+        self.plane_split = {}      # buffer -> last step that splits it into planes
         self.deferred = []         # re-quantisations of reduced tensors, placed at first use
         self.arg_override = {}     # op -> value args after register forwarding
         self.comm_steps = []       # exchanges of this computation, in the order they are placed
@@ -664,7 +670,19 @@ class _Planner(object):
             buf.last_write_step = -1
             buf.last_read_step = -1
         self._find_conv_tails(ordered)
+        self._find_bias_sums(ordered)
         for op in ordered:
+            if op in self.update_of or op in self.bias_sum_of:
+                # a filter gradient and the bias gradient beside it: one step, where the first stands
+                update = self.update_of.get(op, op)
+                if update not in self.producer:
+                    if update is not op and not self._available(update.args):
+                        del self.update_of[self.bias_sum_of.pop(update)]
+                    else:
+                        self._place_other(update)
+                        continue
+                else:
+                    continue
             if op in self.conv_tail_of:
                 # part of a convolution layer's elementwise tail: the layer is placed, as one step,
                 # where its last op stands (every operand of the tail exists by then)
@@ -672,7 +690,7 @@ class _Planner(object):
                 if self.conv_tails[conv]["out"] is op:
                     self._place_other(conv)
                 continue
-            if isinstance(op, ConvolutionOp) and op in self.conv_tails:
+            if op in self.conv_tails:
                 continue
             if isinstance(op, (ElementWiseOp, ReductionOp, AssignOp)):
                 self._place_ew(op)
@@ -916,15 +934,17 @@ class _Planner(object):
         if not (t.fuse and t.fuse_conv_tail):
             return
         for conv in ordered:
-            if not isinstance(conv, ConvolutionOp):
+            forward = isinstance(conv, ConvolutionOp)
+            if not forward and not isinstance(conv, bprop_conv):
                 continue
             try:
-                ok = kernels.takes_conv_tail(conv, t)
+                ok = kernels.takes_conv_tail(conv, t) if forward else \
+                    kernels.takes_conv_tail(conv.fprop, t, lib.CONV_BPROP)
             except Exception:
                 ok = False
             if not ok:
                 continue
-            info = dict(out=None, bias=None, residual=None, relu=False, ops=[])
+            info = dict(out=None, bias=None, residual=None, mask=None, relu=False, ops=[])
             cur = conv
             chan = conv.axes[0].length
             while True:
@@ -947,8 +967,10 @@ class _Planner(object):
                 # axis of the result with a slice before the activation)
                 if [n for n in nxt.axes.lengths if n != 1] != [n for n in conv.axes.lengths if n != 1]:
                     break
+                if info["mask"] is not None:
+                    break
                 if nxt.opname == "add" and not info["relu"]:
-                    is_bias = (len(obase.axes) == 1 and obase.axes[0].length == chan and
+                    is_bias = (forward and len(obase.axes) == 1 and obase.axes[0].length == chan and
                                obase.axes[0] == nxt.axes[0] and not self._is_scalar_const(obase))
                     if ochain:
                         # a view of the other tensor that still walks it in memory order (the
@@ -964,7 +986,10 @@ class _Planner(object):
                         info["residual"] = other if ochain else obase
                     else:
                         break
-                elif nxt.opname == "maximum" and not info["relu"] and self._is_scalar_const(obase) \
+                elif nxt.opname == "mul" and not forward and not ochain and self._is_relu_mask(obase, nxt):
+                    info["mask"] = obase.args[0]
+                    info["ops"].append(obase)
+                elif nxt.opname == "maximum" and forward and not info["relu"] and self._is_scalar_const(obase) \
                         and float(np.asarray(obase.initial_value)) == 0.0:
                     info["relu"] = True
                 else:
@@ -977,6 +1002,57 @@ class _Planner(object):
                 for o in info["ops"]:
                     self.conv_tail_of[o] = conv
 
+    def _is_relu_mask(self, op, reader):
+        """`greater(activation, 0)` over a dense tensor, read by `reader` alone."""
+        if not isinstance(op, ElementWiseOp) or op.opname != "gt" or op in self.returned or \
+                op in self.conv_tail_of or op.axes != reader.axes:
+            return False
+        act, zero = op.args
+        zbase, _ = self._base_tensor(zero)
+        abase, _ = self._base_tensor(act)
+        if not self._is_scalar_const(zbase) or float(np.asarray(zbase.initial_value)) != 0.0 or \
+                isinstance(abase, AssignableTensorOp) or \
+                any(r is not reader for r in self.consumers.get(op, ()) if not isinstance(r, SequentialOp)):
+            return False
+        view = self.t._view_of(self._resolve(act))
+        return view.is_dense() and view.axes == reader.axes
+
+    def _find_bias_sums(self, ordered):
+        """flex16: the sum of a delta over everything but the channels, where a filter gradient
+        reads the same delta as byte planes -- its kernel has the delta at hand."""
+        t = self.t
+        if not (t.flex and t.fuse and t.fuse_conv_tail):
+            return
+        for op in ordered:
+            if not isinstance(op, update_conv):
+                continue
+            try:
+                if not lib.conv_update_planes_info(kernels._conv_dims_of(op.fprop, t))[0]:
+                    continue
+            except Exception:
+                continue
+            delta, _ = self._base_tensor(op.args[0])
+            if isinstance(delta, AssignableTensorOp):
+                continue
+            for r in self.consumers.get(delta, ()):
+                if not isinstance(r, ReductionOp) or r.redop != "sum" or r in self.update_of:
+                    continue
+                arg = r.args[0]
+                axes = [a for a in arg.axes if a.length != 1]
+                kept = [a for a in axes if a not in r.reduction_axes]
+                view = t._view_of(self._resolve(arg))
+                if len(r.axes) == 1 and len(kept) == 1 and axes and kept[0] is axes[0] and \
+                        kept[0].length == op.args[0].axes[0].length and r.axes[0] == kept[0] and \
+                        view.is_dense() and \
+                        [a.length for a in axes] == [n for n in op.args[0].axes.lengths if n != 1]:
+                    self.bias_sum_of[op] = r
+                    self.update_of[r] = op
+                    break
+
+    def _available(self, args):
+        return all(isinstance(b, AssignableTensorOp) or b in self.producer
+                   for b in (self._base_tensor(a)[0] for a in args))
+
     def _place_deferred_for(self, args):
         for a in args:
             base, _ = self._base_tensor(a)
@@ -986,10 +1062,10 @@ class _Planner(object):
 
     def _place_other(self, op):
         """Dense contractions and pooling: one step each, never fused with neighbours."""
-        tail = self.conv_tails.get(op) if isinstance(op, ConvolutionOp) else None
+        tail = self.conv_tails.get(op)
         reads = list(op.args)
         if tail:
-            reads += [x for x in (tail["bias"], tail["residual"]) if x is not None]
+            reads += [x for x in (tail["bias"], tail["residual"], tail["mask"]) if x is not None]
         self._place_deferred_for(reads)
         # Operands these kernels cannot take as they lie (a sliced or reordered view where a dense
         # tensor is needed; a dot operand that does not fold to two dimensions) are first copied
@@ -1049,15 +1125,13 @@ class _Planner(object):
             step = kernels.GemmStep(index, op, self.t)
         elif isinstance(op, ConvolutionOp):
             step = kernels.ConvStep(index, op, self.t, epilogue=tail)
-            if tail:
-                step.out_op = tail["out"]
-                self.producer[tail["out"]] = index
-                for o in tail["ops"]:
-                    self.producer[o] = index
         elif isinstance(op, bprop_conv):
-            step = kernels.ConvBpropStep(index, op, self.t)
+            step = kernels.ConvBpropStep(index, op, self.t, epilogue=tail)
         elif isinstance(op, update_conv):
-            step = kernels.ConvUpdateStep(index, op, self.t)
+            bias_op = self.bias_sum_of.get(op)
+            step = kernels.ConvUpdateStep(index, op, self.t, bias_op)
+            if bias_op is not None:
+                self.producer[bias_op] = index
         elif isinstance(op, PoolingOp):
             step = kernels.PoolStep(index, op, self.t)
         elif isinstance(op, BpropPoolOp):
@@ -1070,6 +1144,17 @@ class _Planner(object):
             step = kernels.RngStep(index, op, self.t)
         else:
             raise ValueError("Unhandled op: {}".format(op))
+        if tail:
+            step.out_op = tail["out"]
+            for o in tail["ops"]:
+                self.producer[o] = index
+        # byte planes that their producer does not write are made by the first step that reads them
+        for k in getattr(step, "plane_args", ()):
+            buf = step.in_views[k].buffer
+            if self.plane_split.get(buf, -1) > buf.last_write_step:
+                step.splits = tuple(i for i in step.splits if i != k)
+            else:
+                self.plane_split[buf] = index
         return step
 
     def _register_other(self, op, step, reads, tail):
@@ -1106,11 +1191,12 @@ class _Planner(object):
         buf = self.t._view_of(m).buffer
         steps = getattr(buf, "plane_steps", ())
         for c in readers:
+            c = self.update_of.get(c, c)
             st = [x for x in steps if x.op is c]
             if not st:
                 return False
             for i, a in enumerate(c.args):
-                if self._base_tensor(a)[0] is m and i != st[0].plane_arg:
+                if self._base_tensor(a)[0] is m and i not in st[0].plane_args:
                     return False
         return True
 
@@ -1719,7 +1805,7 @@ class B200Transformer(object):
         if self._status is None:
             self._status = torch.zeros((1,), dtype=torch.int32, device=self.device)
             self._status_host = torch.zeros((1,), dtype=torch.int32).pin_memory()
-            self._probe64 = torch.zeros((1,), dtype=torch.int64, device=self.device)
+            self._probe64 = torch.zeros((2,), dtype=torch.int64, device=self.device)
         if self.flex:
             n = max(self.flex_manager.n_slots + 64, 64)
             if self._table is None or self._table.shape[0] < n:
