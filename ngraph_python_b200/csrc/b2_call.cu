@@ -47,6 +47,7 @@ __global__ void __launch_bounds__(kThreads)
 k_call_inputs(const Inputs a, const b2_call_block* __restrict__ blk, b2_flex_scale* __restrict__ table,
               int* __restrict__ stats) {
     constexpr int kChunk = kThreads * kPerThread;
+    after_earlier_kernels();
     __shared__ int ismem[32];
     __shared__ const float* src_s[B2_CALL_MAX_INPUTS];
     __shared__ float inv_s[B2_CALL_MAX_INPUTS];
@@ -117,6 +118,7 @@ struct Outputs {
 __global__ void __launch_bounds__(kThreads)
 k_call_outputs(const Outputs o, int* __restrict__ stats, int n_stats, const int* __restrict__ status,
                int* __restrict__ host_stats, int* __restrict__ host_status) {
+    after_earlier_kernels();
     if (blockIdx.x == 0) {
         for (int i = threadIdx.x; i < n_stats; i += kThreads) {
             host_stats[i] = stats[i];
@@ -218,8 +220,8 @@ extern "C" int b2_call_outputs(const b2_call_output* outputs, int32_t n, int32_t
     long long grid = n == 0 ? 1 : 1 + (most / 16 + kThreads - 1) / kThreads;
     if (n && grid < 2) grid = 2;
     if (grid > 65) grid = 65;
-    k_call_outputs<<<(unsigned)grid, kThreads, 0, (cudaStream_t)stream>>>(o, stats, n_stats, status,
-                                                                          host_stats, host_status);
+    B2_CUDA(b2::launch_after(k_call_outputs, dim3((unsigned)grid), kThreads, 0, (cudaStream_t)stream, o, stats, n_stats, status,
+                                                                          host_stats, host_status));
     B2_CUDA(cudaGetLastError());
     return B2_OK;
 }

@@ -912,6 +912,7 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap mapI0,
 __global__ void __launch_bounds__(256)
 split_same_layout_kernel(const short* __restrict__ src, long long n8, void* __restrict__ plane0,
                          void* __restrict__ plane1) {
+    after_earlier_kernels();
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < n8; v += stride) {
         const uint4 w = __ldcs(reinterpret_cast<const uint4*>(src) + v);
@@ -924,6 +925,7 @@ split_same_layout_kernel(const short* __restrict__ src, long long n8, void* __re
 __global__ void __launch_bounds__(256)
 split_padded_kernel(const short* __restrict__ src, long long rows, int n, int np,
                     unsigned char* __restrict__ plane0, unsigned char* __restrict__ plane1) {
+    after_earlier_kernels();
     const int g8 = np / 8;
     const long long total = rows * g8, stride = (long long)gridDim.x * blockDim.x;
     for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < total; v += stride) {
@@ -952,9 +954,9 @@ int split_to_planes(const short* x, int c, int h, int w, int n, void* planes, si
     if (blocks > 148 * 16) blocks = 148 * 16;
     unsigned char* lo = (unsigned char*)planes + plane_bytes;
     if (np == n && ((uintptr_t)x & 15) == 0)
-        split_same_layout_kernel<<<(unsigned)blocks, 256, 0, st>>>(x, units, planes, lo);
+        B2_CUDA(b2::launch_after(split_same_layout_kernel, dim3((unsigned)blocks), 256, 0, st, x, units, planes, lo));
     else
-        split_padded_kernel<<<(unsigned)blocks, 256, 0, st>>>(x, rows, n, np, (unsigned char*)planes, lo);
+        B2_CUDA(b2::launch_after(split_padded_kernel, dim3((unsigned)blocks), 256, 0, st, x, rows, n, np, (unsigned char*)planes, lo));
     B2_CUDA(cudaGetLastError());
     return B2_OK;
 }
@@ -976,6 +978,7 @@ struct FilterLayout {
 template <typename T>
 __global__ void __launch_bounds__(256)
 filter_planes_kernel(const T* __restrict__ F, const FilterLayout f, unsigned char* __restrict__ planes) {
+    after_earlier_kernels();
     const int total = f.ntn * 2 * f.bn * f.kp, G = f.gh * f.gw, RS = f.R * f.S;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
         const int kc = i % f.kp;
@@ -1167,7 +1170,7 @@ int implicit_filter_planes(const T* F, const ConvGeom& g, const ImplicitShape& s
     const FilterLayout f = {g.C, g.R, g.S, g.K, s.cu, s.cchunks, s.kc_pad, s.ntn, s.bn, s.kt, s.kp,
                             s.gh, s.gw, g.str_h, g.str_w, s.wh, s.ww,
                             g.bprop, s.off_h, s.off_w, g.pad_h, g.pad_w};
-    filter_planes_kernel<T><<<(unsigned)fb, 256, 0, st>>>(F, f, (unsigned char*)planes);
+    B2_CUDA(b2::launch_after(filter_planes_kernel<T>, dim3((unsigned)fb), 256, 0, st, F, f, (unsigned char*)planes));
     B2_CUDA(cudaGetLastError());
     return B2_OK;
 }
@@ -1502,6 +1505,13 @@ int run_bprop(const T* E, const T* F, void* GI, const b2_conv_dims* d, const b2_
     return launch_on_planes<MODE>(base, s, p, st, t.splits, base + align1k(s.bytes));
 }
 
+// Division of numbers below 2^16 by a divisor up to 2^15: exact with a 32-bit reciprocal rounded up.
+struct FastDiv { unsigned d, m; };
+inline FastDiv fast_div(int d) { return {(unsigned)d, (unsigned)((0xffffffffULL + d) / d)}; }
+__device__ __forceinline__ int fast_quotient(const FastDiv& f, int x) {
+    return f.d == 1 ? x : (int)__umulhi((unsigned)x, f.m);
+}
+
 // ---- filter gradient on the tile kernel's operands ------------------------------------------------
 // U[(c,r,s), k] = sum over (p,q,n) of I[c, p*str-pad+r, q*str-pad+s, n] * E[k, p, q, n].
 // One k-block = a tile of gh x gw output pixels x 128 images.  Its A operand is the very box the forward
@@ -1519,12 +1529,17 @@ int run_bprop(const T* E, const T* F, void* GI, const b2_conv_dims* d, const b2_
 // What bounds it: the bytes from L2 to the SMs and the tensor core about equally.  A window is read
 // once per tile instead of once per pixel: for 3x3 filters a tile of 2x2 pixels brings 16 rows a channel
 // instead of 36 and fills the 128 rows of the operand (8 channels x 16) where single pixels left 56 empty.
+// Filter and bias gradient of a 16-channel 3x3 layer at batch 1024 24 us (46 with single pixels; 69
+// and a pass for the bias when the operands were split and the slices summed in launches of their own).
+// Clusters of slices that sum through distributed shared memory lost more than they saved: of four
+// CTAs with this much shared memory only 33 fit.
 struct UpdTileParams {
     int tw, nblk, nkb;             // k-block kb = (tile_p*tw + tile_q)*nblk + nb
     int off_h, off_w, step_h, step_w, str_h, str_w;
     int gh, gw, wh, ww, R, S, cu, C, K, cchunks;
     int ntn, kt, bn;               // filter tiles: kt filters x gh*gw pixels in bn rows
     int per, nsplit;               // k-blocks per slice, slices (grid.x)
+    FastDiv by_kt, by_rs, by_s;
     int ksteps, nstages, tmem_cols;
     unsigned box_a, box_b;         // bytes of one activation box, of one error box
     unsigned long long* acc;       // [C*R*S][K], then [K] for the bias: zero between calls
@@ -1538,11 +1553,11 @@ struct UpdTileParams {
     int probe;
 };
 
-constexpr int kUpdThreads = 256;
+constexpr int kUpdThreads = 512;
 constexpr int kUpdMaxStages = 6;
 constexpr int kUpdMaxN = 160;                      // columns of one accumulator: three in 512
 constexpr int kUpdAPlane = 128 * kKBytes;          // 128 rows of 128 bytes
-constexpr int kUpdSmemFixed = 1024 + 512;
+constexpr int kUpdSmemFixed = 1024 + 256 + kUpdMaxN * 8;
 
 // largest of a block's non-negative values, in thread 0's atomic
 template <typename V, typename F>
@@ -1568,6 +1583,7 @@ conv_update_kernel(const __grid_constant__ CUtensorMap mapI0, const __grid_const
     unsigned* tmem_holder = (unsigned*)(tmem_full + 1);
     int* fail_flag = (int*)(tmem_holder + 1);
     unsigned* last = (unsigned*)(fail_flag + 1);                 // [2]
+    long long* bias_sum = (long long*)((unsigned char*)full_bar + 256);           // [kt]
 
     const int warp = warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
     const int chunk = blockIdx.y / p.ntn, ktile = blockIdx.y - chunk * p.ntn;
@@ -1580,13 +1596,20 @@ conv_update_kernel(const __grid_constant__ CUtensorMap mapI0, const __grid_const
         prefetch_map(&mapI0); prefetch_map(&mapI1); prefetch_map(&mapE0); prefetch_map(&mapE1);
         for (int s = 0; s < kUpdMaxStages; ++s) {
             mbar_init(&full_bar[s], 1);
-            mbar_init(&empty_bar[s], p.bias ? 5 : 1);
+            mbar_init(&empty_bar[s], p.bias ? 6 : 2);
         }
-        mbar_init(tmem_full, 1);
+        mbar_init(tmem_full, 2);
         *fail_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 1) tmem_alloc(tmem_holder, p.tmem_cols);
+    for (int i = threadIdx.x; i < kt; i += kUpdThreads) bias_sum[i] = 0;
+    if (warp == 1) {
+        tmem_alloc(tmem_holder, p.tmem_cols);
+        // (not before this CTA holds its tensor memory, or it and the next kernel's could each wait for
+        // what the other has)
+        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    }
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -1614,34 +1637,39 @@ conv_update_kernel(const __grid_constant__ CUtensorMap mapI0, const __grid_const
                 }
             }
         }
-    } else if (warp == 1) {
+    } else if (warp == 1 || warp == 2) {
+        // two issuing threads, for different accumulators: HH and LL, X (one thread alone took 70
+        // cycles an instruction)
+        const bool cross = warp == 2;
         if (elect_one()) {
-            const unsigned id_ss = make_idesc_n(2, 1, 1, bn), id_su = make_idesc_n(2, 1, 0, bn),
-                           id_us = make_idesc_n(2, 0, 1, bn), id_uu = make_idesc_n(2, 0, 0, bn);
-            const unsigned acc_x = tmem_base + bn, acc_l = tmem_base + 2 * bn;
+            const unsigned id_h = make_idesc_n(2, 1, cross ? 0 : 1, bn), id_l = make_idesc_n(2, 0, cross ? 1 : 0, bn);
+            const unsigned acc_h = tmem_base + (cross ? bn : 0), acc_l = tmem_base + (cross ? bn : 2 * bn);
+            // matrix descriptors: only the low word (start address in 16-byte units) changes
+            const unsigned long long dsc = make_smem_desc(ring) & ~0x3fffULL;
+            const unsigned stage_units = (unsigned)(stage >> 4), a_units = kUpdAPlane >> 4,
+                           b_units = (unsigned)(b_plane >> 4), ring_at = (smem_u32(ring) >> 4) & 0x3FFF;
+            const unsigned bh = 2 * a_units + (cross ? b_units : 0), bl = 2 * a_units + (cross ? 0 : b_units);
             const int ksteps = p.ksteps;
-            unsigned accumulate = 0, parity = 0;
+            unsigned accumulate = 0, parity = 0, at = ring_at;
             int s = 0;
             for (int i = 0; i < mine; ++i) {
                 if (!mbar_wait(&full_bar[s], parity)) { atomicExch(fail_flag, 1); break; }
                 tc_fence_after();
-                unsigned char* sa = ring + (size_t)s * stage;
-                const unsigned long long dAh = make_smem_desc(sa), dAl = make_smem_desc(sa + kUpdAPlane);
-                const unsigned long long dBh = make_smem_desc(sa + 2 * kUpdAPlane);
-                const unsigned long long dBl = make_smem_desc(sa + 2 * kUpdAPlane + b_plane);
-                for (int k = 0; k < ksteps; ++k) {
-                    tc_mma<MODE_FLEX16>(tmem_base, dAh + 2 * k, dBh + 2 * k, id_ss, accumulate);
-                    tc_mma<MODE_FLEX16>(acc_x, dAh + 2 * k, dBl + 2 * k, id_su, accumulate);
-                    tc_mma<MODE_FLEX16>(acc_x, dAl + 2 * k, dBh + 2 * k, id_us, 1u);
-                    tc_mma<MODE_FLEX16>(acc_l, dAl + 2 * k, dBl + 2 * k, id_uu, accumulate);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    if (k >= ksteps) break;
+                    tc_mma<MODE_FLEX16>(acc_h, dsc | (at + 2 * k), dsc | (at + bh + 2 * k), id_h, accumulate);
+                    tc_mma<MODE_FLEX16>(acc_l, dsc | (at + a_units + 2 * k), dsc | (at + bl + 2 * k), id_l,
+                                        cross ? 1u : accumulate);
                     accumulate = 1;
                 }
                 tc_commit(&empty_bar[s]);
-                if (++s == p.nstages) { s = 0; parity ^= 1u; }
+                at += stage_units;
+                if (++s == p.nstages) { s = 0; parity ^= 1u; at = ring_at; }
             }
             tc_commit(tmem_full);
         }
-    } else if (warp >= 4 && p.bias) {
+    } else if (warp >= 4 && warp < 8 && p.bias) {
         // sums of the error rows: thread t takes the 16-byte units t, t + 128, ..., whose rows
         // are t/8 + 16*m
         const int t = threadIdx.x - 128;
@@ -1677,30 +1705,30 @@ conv_update_kernel(const __grid_constant__ CUtensorMap mapI0, const __grid_const
             if (m * 16 >= bn) break;
             long long v = 256LL * hi[m] + lo[m];
             for (int o = 1; o < 8; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-            const int row = (t >> 3) + 16 * m, k = ktile * kt + row / npix;
-            if ((t & 7) == 0 && row < kt * npix && k < p.K && ok && v)
-                atomicAdd(p.acc + (long long)p.C * p.R * p.S * p.K + k, (unsigned long long)v);
+            const int row = (t >> 3) + 16 * m;
+            if ((t & 7) == 0 && row < kt * npix && ok)
+                atomicAdd((unsigned long long*)bias_sum + row / npix, (unsigned long long)v);
         }
     }
     __syncwarp();
     __syncthreads();                                  // (every reader is done with the ring)
 
-    // exact sums of this slice: tensor memory -> shared memory [row][column], then added up per tap
+    // exact sums of this slice: tensor memory -> shared memory [row][column]
     bool ok = mbar_wait_relaxed(tmem_full, 0);
     if (!ok) atomicExch(fail_flag, 1);
     tc_fence_after();
     long long* red = (long long*)ring;
     const int pitch = bn + 1;                         // odd: the 32 rows of a store fall into different banks
     {
-        const int quarter = warp & 3, half = warp >> 2, row = quarter * 32 + lane;
+        const int quarter = warp & 3, row = quarter * 32 + lane;
         const unsigned a0 = tmem_base + ((unsigned)(quarter * 32) << 16);
-        for (int c0 = half * 8; c0 < bn; c0 += 16) {
+        for (int c0 = (warp >> 2) * 8; c0 < bn; c0 += 32) {
             unsigned hh[8], xx[8], ll[8];
             tmem_ld8(a0 + c0, hh); tmem_ld8(a0 + bn + c0, xx); tmem_ld8(a0 + 2 * bn + c0, ll);
             tmem_ld_wait();
 #pragma unroll
             for (int j = 0; j < 8; ++j)
-                red[row * pitch + c0 + j] =
+                red[row * pitch + c0 + j] = mine <= 0 ? 0 :
                     ((long long)(int)hh[j] << 16) + ((long long)(int)xx[j] << 8) + (long long)ll[j];
         }
     }
@@ -1712,16 +1740,41 @@ conv_update_kernel(const __grid_constant__ CUtensorMap mapI0, const __grid_const
     }
     ok = *fail_flag == 0;
     const int rs = p.R * p.S, n_out = p.cu * rs * kt;
-    for (int i = threadIdx.x; i < n_out; i += kUpdThreads) {
-        const int k = i % kt, t = i / kt, tap = t % rs, c = t / rs, r = tap / p.S, s = tap - r * p.S;
-        const int cg = chunk * p.cu + c, kg = ktile * kt + k;
-        if (cg >= p.C || kg >= p.K || !ok) continue;
+    unsigned long long* bias_acc = p.acc + (long long)p.C * rs * p.K + ktile * kt;
+    // ... added up per tap in shared memory, then onto the accumulators: rows of 16-byte multiples by bulk
+    // reductions (a 64-bit atomic takes its SM four cycles a value: 7500 cycles for a 64-channel tile,
+    // 1200 this way)
+    long long* sum = red + 128 * pitch;                          // (16-byte aligned: 128 is even)
+    const int rows = (p.C - chunk * p.cu < p.cu ? p.C - chunk * p.cu : p.cu) * rs;
+    const int width = p.K - ktile * kt < kt ? p.K - ktile * kt : kt;
+    const bool bulk = ((p.K | kt) & 1) == 0;
+    unsigned long long* acc = p.acc + (long long)chunk * p.cu * rs * p.K + ktile * kt;
+    for (int i = threadIdx.x; i < rows * kt && ok; i += kUpdThreads) {
+        const int t = fast_quotient(p.by_kt, i), k = i - t * kt, c = fast_quotient(p.by_rs, t), tap = t - c * rs;
+        const int r = fast_quotient(p.by_s, tap), s = tap - r * p.S;
+        const long long* at = red + ((c * p.wh + r) * p.ww + s) * pitch + k * npix;
         long long v = 0;
         for (int a = 0; a < p.gh; ++a)
-            for (int b = 0; b < p.gw; ++b)
-                v += red[((c * p.wh + r + a * p.str_h) * p.ww + s + b * p.str_w) * pitch + k * npix + a * p.gw + b];
-        if (v) atomicAdd(p.acc + ((long long)cg * rs + tap) * p.K + kg, (unsigned long long)v);
+            for (int b = 0; b < p.gw; ++b) v += at[(a * p.str_h * p.ww + b * p.str_w) * pitch + a * p.gw + b];
+        if (bulk) sum[i] = v;
+        else if (k < width && v) atomicAdd(acc + (long long)t * p.K + k, (unsigned long long)v);
     }
+    if (bulk) {
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncthreads();
+        const bool whole = kt == p.K;                     // then the tile is one piece
+        if (ok)
+            for (int t = threadIdx.x; t < (whole ? 1 : rows); t += kUpdThreads)
+                asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.u64 [%0], [%1], %2;"
+                             ::"l"(acc + (long long)t * p.K), "r"(smem_u32(sum + t * kt)),
+                               "r"((whole ? rows * kt : width) * 8) : "memory");
+        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+        asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+        asm volatile("fence.proxy.async.global;" ::: "memory");
+    }
+    if (p.bias)
+        for (int k = threadIdx.x; k < kt && ktile * kt + k < p.K; k += kUpdThreads)
+            if (bias_sum[k] && ok) atomicAdd(bias_acc + k, (unsigned long long)bias_sum[k]);
     __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -1741,19 +1794,28 @@ conv_update_kernel(const __grid_constant__ CUtensorMap mapI0, const __grid_const
         const int sh = -ilogbf(p.table[p.slotI].scale * scale_e * (p.probe ? 1.0f : p.table[p.slotU].inv_scale));
         int stat = 0;
         unsigned long long pmax = 0;
-        for (int i = threadIdx.x; i < n_out; i += kUpdThreads) {
-            const int k = i % kt, t = i / kt, tap = t % rs, cg = chunk * p.cu + t / rs, kg = ktile * kt + k;
-            if (cg >= p.C || kg >= p.K) continue;
-            const long long at = ((long long)cg * rs + tap) * p.K + kg;
-            const long long v = (long long)__ldcg(p.acc + at);
-            p.acc[at] = 0;
-            if (p.probe) {
-                const unsigned long long m = (unsigned long long)(v < 0 ? -v : v);
-                pmax = m > pmax ? m : pmax;
-            } else {
-                const int q = rescale_i64(v, sh), m = q < 0 ? -q : q;
-                stat = m > stat ? m : stat;
-                p.U[at] = (short)q;
+        constexpr int kBatch = 8;                         // loads in flight
+        for (int i0 = threadIdx.x; i0 < n_out; i0 += kBatch * kUpdThreads) {
+            long long at[kBatch], v[kBatch];
+#pragma unroll
+            for (int j = 0; j < kBatch; ++j) {
+                const int i = i0 + j * kUpdThreads, t = fast_quotient(p.by_kt, i), kg = ktile * kt + i - t * kt;
+                const long long row = (long long)chunk * p.cu * rs + t;
+                at[j] = i < n_out && row < (long long)p.C * rs && kg < p.K ? row * p.K + kg : -1;
+                v[j] = at[j] >= 0 ? (long long)__ldcg(p.acc + at[j]) : 0;
+            }
+#pragma unroll
+            for (int j = 0; j < kBatch; ++j) {
+                if (at[j] < 0) continue;
+                p.acc[at[j]] = 0;
+                if (p.probe) {
+                    const unsigned long long m = (unsigned long long)(v[j] < 0 ? -v[j] : v[j]);
+                    pmax = m > pmax ? m : pmax;
+                } else {
+                    const int q = rescale_i64(v[j], sh), m = q < 0 ? -q : q;
+                    stat = m > stat ? m : stat;
+                    p.U[at[j]] = (short)q;
+                }
             }
         }
         if (p.probe) update_max(pmax, [&](unsigned long long m) { atomicMax(p.probe_out, m); });
@@ -1764,12 +1826,9 @@ conv_update_kernel(const __grid_constant__ CUtensorMap mapI0, const __grid_const
         const int sh = -ilogbf(scale_e * (p.probe ? 1.0f : p.table[p.slotB].inv_scale));
         int stat = 0;
         unsigned long long pmax = 0;
-        for (int k = threadIdx.x; k < kt; k += kUpdThreads) {
-            const int kg = ktile * kt + k;
-            if (kg >= p.K) continue;
-            unsigned long long* at = p.acc + (long long)p.C * rs * p.K + kg;
-            const long long v = (long long)__ldcg(at);
-            *at = 0;
+        for (int k = threadIdx.x; k < kt && ktile * kt + k < p.K; k += kUpdThreads) {
+            const long long v = (long long)__ldcg(bias_acc + k);
+            bias_acc[k] = 0;
             const unsigned long long m = (unsigned long long)(v < 0 ? -v : v);
             if (p.probe) {
                 pmax = m > pmax ? m : pmax;
@@ -1779,7 +1838,7 @@ conv_update_kernel(const __grid_constant__ CUtensorMap mapI0, const __grid_const
             const unsigned long long most = v < 0 ? 32768 : 32767;
             q = q > most ? most : q;
             stat = (int)q > stat ? (int)q : stat;
-            p.bias[kg] = (short)(v < 0 ? -(int)q : (int)q);
+            p.bias[ktile * kt + k] = (short)(v < 0 ? -(int)q : (int)q);
         }
         if (p.probe) update_max(pmax, [&](unsigned long long m) { atomicMax(p.probe_out + 1, m); });
         else update_max(stat, [&](int m) { atomicMax(p.stats + p.slotB, m); });
@@ -1793,8 +1852,9 @@ struct UpdShape {
     long long cost;
 };
 
-// Cycles of a k-block: the tensor core's rate, the shared memory its operands are read from, the
-// bytes from L2; measured constants.
+// Cost in cycles, fitted to measured launches: a k-block takes what the tensor core needs for its
+// products, or its bytes from L2 at 56 a cycle; set-up, the sums' way to memory and the last CTA's work
+// take 8 us, and more with the columns and outputs of a tile.
 UpdShape update_shape_for(const ConvGeom& g, int gh, int gw) {
     UpdShape u = {};
     u.gh = gh; u.gw = gw; u.wh = (gh - 1) * g.str_h + g.R; u.ww = (gw - 1) * g.str_w + g.S;
@@ -1805,7 +1865,7 @@ UpdShape update_shape_for(const ConvGeom& g, int gh, int gw) {
     const int cu_max = 128 / win;
     u.cchunks = (g.C + cu_max - 1) / cu_max;
     u.cu = (g.C + u.cchunks - 1) / u.cchunks;
-    const int kt_max = kUpdMaxN / npix;
+    const int kt_max = npix == 1 ? 96 : kUpdMaxN / npix;
     u.ntn = (g.K + kt_max - 1) / kt_max;
     u.kt = (g.K + u.ntn - 1) / u.ntn;
     u.bn = round_up(u.kt * npix, 16);
@@ -1816,17 +1876,20 @@ UpdShape update_shape_for(const ConvGeom& g, int gh, int gw) {
     if (u.nstages > kUpdMaxStages) u.nstages = kUpdMaxStages;
     if (u.nstages < 2 || (long long)u.cchunks * u.ntn > 65535) return u;
     u.smem = kUpdSmemFixed + u.nstages * stage;
+    // (the ring holds the sums afterwards, by row and column and by output)
+    if (128 * (u.bn + 1) * 8 + u.cu * g.R * g.S * u.kt * 8 > u.nstages * stage) return u;
     u.nkb = (int)(th * u.tw * nblk);
     const int images = g.N < 128 ? g.N : 128;
     u.ksteps = (images + 31) / 32;
     const int cols = u.cchunks * u.ntn;
     int slices = cols < 148 ? 148 / cols : 1;
+    if (slices < (u.nkb + 255) / 256) slices = (u.nkb + 255) / 256;   // int32 sums: exact up to 32768 terms
     u.per = (u.nkb + slices - 1) / slices;
-    if (u.per > 256) u.per = 256;                  // the int32 sums stay exact up to 32768 terms
     u.nsplit = (u.nkb + u.per - 1) / u.per;
     const long long mma = 16LL * u.ksteps / 4 * (u.bn / 2 > 32 + u.bn / 4 ? u.bn / 2 : 32 + u.bn / 4);
     const long long bytes = 2LL * images * (u.cu * win + u.kt * npix) / 56;
-    u.cost = ((long long)cols * u.nsplit + 147) / 148 * (u.per * ((mma > bytes ? mma : bytes) + 60) + 3000 + 40 * u.bn);
+    u.cost = ((long long)cols * u.nsplit + 147) / 148 *
+             (u.per * ((mma > bytes ? mma : bytes) + 60) + 15500 + 48 * u.bn + 2LL * u.cu * g.R * g.S * u.kt);
     u.act_plane = plane_size(g.C, g.H, g.W, g.N);
     u.err_plane = plane_size(g.K, g.P, g.Q, g.N);
     u.acc_bytes = align1k((((size_t)g.C * g.R * g.S + 1) * g.K) * 8 + (size_t)(cols + u.ntn) * 4);
@@ -1877,6 +1940,7 @@ int run_update_planes(const void* act_planes, const void* err_planes, void* acc,
     p.gh = u.gh; p.gw = u.gw; p.wh = u.wh; p.ww = u.ww; p.R = g.R; p.S = g.S;
     p.cu = u.cu; p.C = g.C; p.K = g.K; p.cchunks = u.cchunks;
     p.ntn = u.ntn; p.kt = u.kt; p.bn = u.bn; p.per = u.per; p.nsplit = u.nsplit;
+    p.by_kt = fast_div(u.kt); p.by_rs = fast_div(g.R * g.S); p.by_s = fast_div(g.S);
     p.ksteps = u.ksteps; p.nstages = u.nstages; p.tmem_cols = u.tmem_cols;
     p.box_a = (unsigned)(u.cu * u.wh * u.ww * kKBytes); p.box_b = (unsigned)(u.kt * u.gh * u.gw * kKBytes);
     p.acc = (unsigned long long*)acc;
@@ -1890,8 +1954,8 @@ int run_update_planes(const void* act_planes, const void* err_planes, void* acc,
                                      kConvSmemMax));
         attr_set = true;
     }
-    conv_update_kernel<<<dim3(u.nsplit, u.cchunks * u.ntn), kUpdThreads, u.smem, st>>>(mI0, mI1, mE0, mE1, p);
-    B2_CUDA(cudaGetLastError());
+    B2_CUDA(b2::launch_after(conv_update_kernel, dim3(u.nsplit, u.cchunks * u.ntn), kUpdThreads, u.smem, st, mI0,
+                             mI1, mE0, mE1, p));
     return B2_OK;
 }
 
@@ -1966,6 +2030,7 @@ template <typename T, bool MAX>
 __global__ void __launch_bounds__(256)
 pool_kernel(const T* __restrict__ I, T* __restrict__ O, int C, int H, int W, int N, int P, int Q,
             int R, int S, int pad_h, int pad_w, int str_h, int str_w, int* stats) {
+    after_earlier_kernels();
     // a block takes 32 consecutive results (consecutive images: coalesced); its eight warps each
     // add every eighth element of the window, the eight partial sums are combined in warp order
     __shared__ float part[8][32];
@@ -2275,6 +2340,7 @@ pool_bprop_kernel(const T* __restrict__ E, const T* __restrict__ I, T* __restric
                   int W, int N, int P, int Q, int R, int S, int pad_h, int pad_w, int str_h,
                   int str_w, const b2_flex_scale* __restrict__ table, int slotE, int slotG,
                   int* stats, unsigned long long* probe_out, int probe) {
+    after_earlier_kernels();
     const long long total = (long long)C * H * W * N;
     const bool flex = sizeof(T) == 2;
     const float sE = flex ? table[slotE].scale : 1.0f;
@@ -2354,8 +2420,8 @@ int run_pool(bool is_max, const void* I, void* O, int32_t flex, int32_t C, int32
     if (blocks > 148 * 16) blocks = 148 * 16;
     cudaStream_t st = (cudaStream_t)stream;
 #define B2_POOL_LAUNCH(T, MAXV, STATS)                                                            \
-    pool_kernel<T, MAXV><<<(unsigned)blocks, 256, 0, st>>>((const T*)I, (T*)O, C, H, W, N, P, Q, R, \
-                                                          S, pad_h, pad_w, str_h, str_w, STATS)
+    B2_CUDA((b2::launch_after(pool_kernel<T, MAXV>, dim3((unsigned)blocks), 256, 0, st, (const T*)I, (T*)O, C, H, W, \
+                              N, P, Q, R, S, pad_h, pad_w, str_h, str_w, STATS)))
     if (flex) {
         if (is_max) B2_POOL_LAUNCH(short, true, stats_slot);
         else B2_POOL_LAUNCH(short, false, stats_slot);
@@ -2404,9 +2470,9 @@ extern "C" int b2_pool_bprop(const void* E, const void* I, void* GI, int32_t fle
     cudaStream_t st = (cudaStream_t)stream;
     unsigned long long* po = (unsigned long long*)probe_out;
 #define B2_PB_LAUNCH(T, MAXV)                                                                       \
-    pool_bprop_kernel<T, MAXV><<<(unsigned)blocks, 256, 0, st>>>(                                  \
-        (const T*)E, (const T*)I, (T*)GI, C, H, W, N, P, Q, R, S, pad_h, pad_w, str_h, str_w, table, \
-        slotE, slotGI, stats, po, probe ? 1 : 0)
+    B2_CUDA((b2::launch_after(pool_bprop_kernel<T, MAXV>, dim3((unsigned)blocks), 256, 0, st, (const T*)E, \
+                              (const T*)I, (T*)GI, C, H, W, N, P, Q, R, S, pad_h, pad_w, str_h, str_w, table, \
+                              slotE, slotGI, stats, po, probe ? 1 : 0)))
     if (flex) {
         if (is_max) B2_PB_LAUNCH(short, true);
         else B2_PB_LAUNCH(short, false);

@@ -36,6 +36,7 @@ struct ShuffleParams {
 template <typename T>
 __global__ void __launch_bounds__(256)
 dimshuffle_tiled_kernel(const T* __restrict__ src, T* __restrict__ dst, ShuffleParams p) {
+    after_earlier_kernels();
     __shared__ T tile[32][33];
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;      // 32 x 8
     const long long per_outer = p.tiles_x * p.tiles_y;
@@ -81,6 +82,7 @@ dimshuffle_tiled_kernel(const T* __restrict__ src, T* __restrict__ dst, ShuffleP
 template <typename T>
 __global__ void __launch_bounds__(256)
 dimshuffle_rows_kernel(const T* __restrict__ src, T* __restrict__ dst, ShuffleParams p) {
+    after_earlier_kernels();
     // threads along axis ax in chunks of 256; the other axes from the block index
     const long long chunks = p.tiles_x;
     const long long total = chunks * p.outer;
@@ -107,9 +109,9 @@ int launch(const void* src, void* dst, const ShuffleParams& p, cudaStream_t st) 
     const long long cap = 148LL * 32;
     const unsigned grid = (unsigned)(blocks < cap ? (blocks < 1 ? 1 : blocks) : cap);
     if (p.ay >= 0)
-        dimshuffle_tiled_kernel<T><<<grid, 256, 0, st>>>((const T*)src, (T*)dst, p);
+        B2_CUDA(b2::launch_after(dimshuffle_tiled_kernel<T>, dim3(grid), 256, 0, st, (const T*)src, (T*)dst, p));
     else
-        dimshuffle_rows_kernel<T><<<grid, 256, 0, st>>>((const T*)src, (T*)dst, p);
+        B2_CUDA(b2::launch_after(dimshuffle_rows_kernel<T>, dim3(grid), 256, 0, st, (const T*)src, (T*)dst, p));
     B2_CUDA(cudaGetLastError());
     return B2_OK;
 }

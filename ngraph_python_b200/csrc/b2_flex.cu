@@ -15,6 +15,7 @@ const int kThreads = 256;
 __global__ void __launch_bounds__(kThreads)
 k_host_quantize(const float* __restrict__ src, short* __restrict__ dst, long long n,
                 const b2_flex_scale* __restrict__ table, int slot, int* __restrict__ stats) {
+    after_earlier_kernels();
     __shared__ int ismem[32];
     const float inv = table[slot].inv_scale;
     int stat = 0;
@@ -32,6 +33,7 @@ k_host_quantize(const float* __restrict__ src, short* __restrict__ dst, long lon
 __global__ void __launch_bounds__(kThreads)
 k_dequantize(const short* __restrict__ src, float* __restrict__ dst, long long n,
              const b2_flex_scale* __restrict__ table, int slot) {
+    after_earlier_kernels();
     const float s = table[slot].scale;
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride)
@@ -62,8 +64,8 @@ extern "C" int b2_flex_host_quantize(const float* src, int16_t* dst, int64_t n,
                                      void* stream) {
     B2_REQUIRE(src && dst && table && stats && slot >= 0 && n >= 0, "bad argument");
     if (n == 0) return B2_OK;
-    k_host_quantize<<<grid_for(n), kThreads, 0, (cudaStream_t)stream>>>(src, dst, n, table, slot,
-                                                                       stats);
+    B2_CUDA(b2::launch_after(k_host_quantize, dim3(grid_for(n)), kThreads, 0, (cudaStream_t)stream, src, dst, n, table, slot,
+                                                                       stats));
     B2_CUDA(cudaGetLastError());
     return B2_OK;
 }
@@ -72,7 +74,7 @@ extern "C" int b2_flex_dequantize(const int16_t* src, float* dst, int64_t n,
                                   const b2_flex_scale* table, int32_t slot, void* stream) {
     B2_REQUIRE(src && dst && table && slot >= 0 && n >= 0, "bad argument");
     if (n == 0) return B2_OK;
-    k_dequantize<<<grid_for(n), kThreads, 0, (cudaStream_t)stream>>>(src, dst, n, table, slot);
+    B2_CUDA(b2::launch_after(k_dequantize, dim3(grid_for(n)), kThreads, 0, (cudaStream_t)stream, src, dst, n, table, slot));
     B2_CUDA(cudaGetLastError());
     return B2_OK;
 }

@@ -297,7 +297,13 @@ gemm_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constant__ C
         *fail_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 1) tmem_alloc(tmem_holder, kTmemCols);
+    if (warp == 1) {
+        tmem_alloc(tmem_holder, kTmemCols);
+        // (not before this CTA holds its tensor memory, or it and the next kernel's could each wait for
+        // what the other has)
+        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    }
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -542,6 +548,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constant__ C
 template <int MODE>
 __global__ void __launch_bounds__(256)
 splitk_finish_kernel(const GemmParams p, int splits) {
+    after_earlier_kernels();
     __shared__ long long part64[8][32];
     __shared__ float part32[8][32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -642,6 +649,7 @@ __global__ void __launch_bounds__(256)
 split_rows_kernel(const T* __restrict__ src, long long rs, int rows, int k, int rows_p, int kp,
                   void* __restrict__ plane0, void* __restrict__ plane1, unsigned lo_xor,
                   int* __restrict__ rowsum) {
+    after_earlier_kernels();
     constexpr int kPer = MODE == MODE_FLEX16 ? 16 : 4;
     const int upr = kp / kPer;                                   // units per row
     const long long idx = (long long)blockIdx.x * 256 + threadIdx.x;
@@ -709,6 +717,7 @@ __global__ void __launch_bounds__(256)
 split_cols_kernel(const T* __restrict__ src, long long cs, int rows, int k, int rows_p, int kp,
                   void* __restrict__ plane0, void* __restrict__ plane1, unsigned lo_xor,
                   int* __restrict__ rowsum) {
+    after_earlier_kernels();
     constexpr int kTileK = MODE == MODE_FLEX16 ? 64 : 32;
     constexpr int kPitch = MODE == MODE_FLEX16 ? 66 : 65;       // elements; odd word pitch
     __shared__ T tile[kTileK * kPitch];
@@ -794,6 +803,7 @@ __global__ void __launch_bounds__(256)
 split_planes_kernel(const T* __restrict__ src, long long rs, long long cs, int rows, int k,
                     int rows_p, int kp, void* __restrict__ plane0, void* __restrict__ plane1,
                     unsigned lo_xor, int* __restrict__ rowsum) {
+    after_earlier_kernels();
     __shared__ T tile[32][33];
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;     // 32 x 8
     const int r0 = blockIdx.y * 32, k0 = blockIdx.x * 32;
@@ -836,17 +846,17 @@ int split_operand(const T* src, long long rs, long long cs, int rows, int k, int
     const int vec = 16 / (int)sizeof(T);
     if (cs == 1 && base16 && rs % vec == 0) {
         const long long units = (long long)rows_p * (kp / (MODE == MODE_FLEX16 ? 16 : 4));
-        split_rows_kernel<T, MODE><<<(unsigned)((units + 255) / 256), 256, 0, st>>>(
-            src, rs, rows, k, rows_p, kp, plane0, plane1, lo_xor, rowsum);
+        B2_CUDA(b2::launch_after(split_rows_kernel<T, MODE>, dim3((unsigned)((units + 255) / 256)), 256, 0, st, 
+            src, rs, rows, k, rows_p, kp, plane0, plane1, lo_xor, rowsum));
     } else if (rs == 1 && base16 && cs % vec == 0) {
         const int tk = MODE == MODE_FLEX16 ? 64 : 32;
         dim3 g((kp + tk - 1) / tk, (rows_p + 63) / 64);
-        split_cols_kernel<T, MODE><<<g, 256, 0, st>>>(src, cs, rows, k, rows_p, kp, plane0, plane1,
-                                                     lo_xor, rowsum);
+        B2_CUDA(b2::launch_after(split_cols_kernel<T, MODE>, dim3(g), 256, 0, st, src, cs, rows, k, rows_p, kp, plane0, plane1,
+                                                     lo_xor, rowsum));
     } else {
         dim3 g((kp + 31) / 32, (rows_p + 31) / 32);
-        split_planes_kernel<T, MODE><<<g, 256, 0, st>>>(src, rs, cs, rows, k, rows_p, kp, plane0,
-                                                       plane1, lo_xor, rowsum);
+        B2_CUDA(b2::launch_after(split_planes_kernel<T, MODE>, dim3(g), 256, 0, st, src, rs, cs, rows, k, rows_p, kp, plane0,
+                                                       plane1, lo_xor, rowsum));
     }
     B2_CUDA(cudaGetLastError());
     return B2_OK;
@@ -918,8 +928,7 @@ int launch_tile(const CUtensorMap& mA0, const CUtensorMap& mA1, const CUtensorMa
         attr_set = true;
     }
     dim3 grid(s.Np / BN, s.Mp / kBlockM, splits);
-    gemm_kernel<MODE, BN><<<grid, kThreads, smem_bytes(BN), st>>>(mA0, mA1, mB0, mB1, p);
-    B2_CUDA(cudaGetLastError());
+    B2_CUDA(b2::launch_after(gemm_kernel<MODE, BN>, grid, kThreads, smem_bytes(BN), st, mA0, mA1, mB0, mB1, p));
     return B2_OK;
 }
 
@@ -986,7 +995,7 @@ int launch_on_planes(unsigned char* base, const Shapes& s, GemmParams p, cudaStr
     if (rc || !p.partial) return rc;
     long long blocks = ((long long)p.M * p.N + 31) / 32;
     if (blocks > 148 * 16) blocks = 148 * 16;
-    splitk_finish_kernel<MODE><<<(unsigned)blocks, 256, 0, st>>>(p, splits);
+    B2_CUDA(b2::launch_after(splitk_finish_kernel<MODE>, dim3((unsigned)blocks), 256, 0, st, p, splits));
     B2_CUDA(cudaGetLastError());
     return B2_OK;
 }

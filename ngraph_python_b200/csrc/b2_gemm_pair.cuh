@@ -136,7 +136,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constan
         asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;"
                      ::"r"(smem_u32(tmem_holder)), "r"(512) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     }
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     tc_fence_before();
     __syncthreads();
     pair_cluster_sync();
@@ -430,10 +432,12 @@ int launch_pair(unsigned char* base, const Shapes& s, GemmParams g, cudaStream_t
     cfg.blockDim = dim3(kPairThreads);
     cfg.dynamicSmemBytes = kPairSmem;
     cfg.stream = st;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = p.splits;
-    cfg.attrs = attr; cfg.numAttrs = 1;
+    cfg.attrs = attr; cfg.numAttrs = 2;
     B2_CUDA(cudaLaunchKernelEx(&cfg, gemm_pair_kernel<MODE>, mA0, mA1, mB0, mB1, p));
     return B2_OK;
 }
