@@ -908,6 +908,17 @@ class _Planner(object):
             sbuf.comm_key = id(sbuf)
             sbuf.entry = None
             t._buffers[staging] = sbuf
+            if t.comm.size == 1:
+                # nothing to exchange: the consumers read the gradient as it is stored, without the
+                # way through fp32 (a launch a tensor); the arena's plan stays what it is elsewhere
+                step = kernels.CommStep(index, op, t, None, sbuf)
+                step.reduce_func = op.reduce_func
+                t._alias[op] = src
+                self.consumers[src] = list(self.consumers[src]) + list(self.consumers.get(op, ()))
+                self.steps.append(step)
+                self.producer[op] = index
+                self.comm_steps.append(step)
+                return
             step = kernels.CommStep(index, op, t, src_view, sbuf)
             sbuf.last_write_step = index
             requant = ElementWiseOp("assign", (staging,))
