@@ -317,6 +317,14 @@ int b2_conv_split_planes(const int16_t* X, int32_t c, int32_t h, int32_t w, int3
                          void* stream);
 int b2_conv_filter_planes(const int16_t* F, const b2_conv_dims* d, int32_t pass, void* planes,
                           void* stream);
+/* ... of several convolutions at once, in as few launches as their arguments take. */
+typedef struct b2_conv_filter_job {
+    const int16_t* filters;
+    void* planes;
+    b2_conv_dims dims;
+    int32_t pass;
+} b2_conv_filter_job;
+int b2_conv_filter_planes_many(const b2_conv_filter_job* jobs, int32_t n, int32_t* launches, void* stream);
 int b2_conv_flex16_planes(int32_t pass, const void* act_planes, const void* filter_planes,
                           int16_t* out, const b2_conv_dims* d, const b2_flex_scale* table,
                           int32_t slotX, int32_t slotF, int32_t slotOut, int32_t* stats,

@@ -965,8 +965,9 @@ int split_to_planes(const short* x, int c, int h, int w, int n, void* planes, si
 // the high bytes of its output channels (rows 0..bn-1) and, behind them, the low bytes minus 128 as
 // signed bytes (rows bn..2bn-1).  A tile covers gh x gw output pixels: row g*kt + k holds output
 // channel k as pixel g sees it inside the common window of wh x ww taps (forward: shifted by
-// (g/gw)*str_h, (g%gw)*str_w; input gradient: the taps of its own residue modulo the stride, flipped); row gh*gw*kt + g is pixel g's sum column: 0 in the high half, +1 in the
-// low half on the taps of its own R x S window.  Everything else -- taps of the common window that
+// (g/gw)*str_h, (g%gw)*str_w; input gradient: the taps of its own residue modulo the stride, flipped);
+// row gh*gw*kt + g is pixel g's sum column: 0 in the high half, +1 in the low half on the taps of its
+// own R x S window.  Everything else -- taps of the common window that
 // are not the pixel's, channels beyond C, padding -- is zero in both halves, so it adds nothing
 // whatever the operand holds there.  The K positions of chunk cc start at cc*kc_pad and run over
 // (channel within the chunk, tap row, tap column).
@@ -975,12 +976,27 @@ struct FilterLayout {
     int bprop, off_h, off_w, pad_h, pad_w;
 };
 
-template <typename T>
+// Filters of several convolutions to a launch: a training step rebuilds the planes of every layer, 43
+// launches of 2 us for ResNet-20.
+constexpr int kFilterJobs = 32;                    // (the argument stays below 4 KB)
+struct FilterJobs {
+    int n, first[kFilterJobs + 1];                 // job j owns blocks first[j] .. first[j+1]-1
+    const short* F[kFilterJobs];
+    unsigned char* planes[kFilterJobs];
+    FilterLayout layout[kFilterJobs];
+};
+
 __global__ void __launch_bounds__(256)
-filter_planes_kernel(const T* __restrict__ F, const FilterLayout f, unsigned char* __restrict__ planes) {
+filter_planes_kernel(const __grid_constant__ FilterJobs jobs) {
     after_earlier_kernels();
+    int j = 0;
+    while (j + 1 < jobs.n && (int)blockIdx.x >= jobs.first[j + 1]) ++j;
+    const FilterLayout& f = jobs.layout[j];
+    const short* __restrict__ F = jobs.F[j];
+    unsigned char* __restrict__ planes = jobs.planes[j];
     const int total = f.ntn * 2 * f.bn * f.kp, G = f.gh * f.gw, RS = f.R * f.S;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+    const int stride = (jobs.first[j + 1] - jobs.first[j]) * (int)blockDim.x;
+    for (int i = ((int)blockIdx.x - jobs.first[j]) * (int)blockDim.x + threadIdx.x; i < total; i += stride) {
         const int kc = i % f.kp;
         const int r2 = (i / f.kp) % (2 * f.bn), tile = i / f.kp / (2 * f.bn);
         const bool low = r2 >= f.bn;
@@ -1160,19 +1176,31 @@ int implicit_split_activations(const T* I, const ConvGeom& g, const ImplicitShap
     return split_to_planes((const short*)I, g.C, g.H, g.W, g.N, planes, s.act_plane, st);
 }
 
-template <typename T, int MODE>
-int implicit_filter_planes(const T* F, const ConvGeom& g, const ImplicitShape& s, void* planes,
-                           cudaStream_t st) {
+int add_filter_job(FilterJobs* jobs, const void* F, const ConvGeom& g, const ImplicitShape& s, void* planes) {
     const long long n_f = (long long)s.ntn * 2 * s.bn * s.kp;
     B2_REQUIRE(n_f < (1LL << 30), "filter tensor too large");
     long long fb = (n_f + 255) / 256;
     if (fb > 148 * 8) fb = 148 * 8;
-    const FilterLayout f = {g.C, g.R, g.S, g.K, s.cu, s.cchunks, s.kc_pad, s.ntn, s.bn, s.kt, s.kp,
+    const int j = jobs->n++;
+    if (j == 0) jobs->first[0] = 0;
+    jobs->first[j + 1] = jobs->first[j] + (int)fb;
+    jobs->F[j] = (const short*)F; jobs->planes[j] = (unsigned char*)planes;
+    jobs->layout[j] = {g.C, g.R, g.S, g.K, s.cu, s.cchunks, s.kc_pad, s.ntn, s.bn, s.kt, s.kp,
                             s.gh, s.gw, g.str_h, g.str_w, s.wh, s.ww,
                             g.bprop, s.off_h, s.off_w, g.pad_h, g.pad_w};
-    B2_CUDA(b2::launch_after(filter_planes_kernel<T>, dim3((unsigned)fb), 256, 0, st, F, f, (unsigned char*)planes));
-    B2_CUDA(cudaGetLastError());
     return B2_OK;
+}
+
+int run_filter_jobs(const FilterJobs& jobs, cudaStream_t st) {
+    B2_CUDA(b2::launch_after(filter_planes_kernel, dim3((unsigned)jobs.first[jobs.n]), 256, 0, st, jobs));
+    return B2_OK;
+}
+
+int implicit_filter_planes(const void* F, const ConvGeom& g, const ImplicitShape& s, void* planes,
+                           cudaStream_t st) {
+    FilterJobs jobs = {};
+    int rc = add_filter_job(&jobs, F, g, s, planes);
+    return rc ? rc : run_filter_jobs(jobs, st);
 }
 
 int implicit_tiles(const void* act_planes, const void* filt_planes, void* O, const ConvGeom& g,
@@ -1284,7 +1312,7 @@ int run_fprop_implicit(const T* I, const T* F, void* O, const ConvGeom& g,
     unsigned char* base = (unsigned char*)scratch;
     int rc = implicit_split_activations<T, MODE>(I, g, s, base, st);
     if (rc) return rc;
-    if ((rc = implicit_filter_planes<T, MODE>(F, g, s, base + 2 * s.act_plane, st))) return rc;
+    if ((rc = implicit_filter_planes(F, g, s, base + 2 * s.act_plane, st))) return rc;
     return implicit_tiles(base, base + 2 * s.act_plane, O, g, s, table, slotI, slotF, slotO, stats,
                           probe_out, status, probe, st);
 }
@@ -1474,7 +1502,7 @@ int run_bprop(const T* E, const T* F, void* GI, const b2_conv_dims* d, const b2_
                    si.bytes, scratch_bytes);
         unsigned char* base = (unsigned char*)scratch;
         if ((rc = implicit_split_activations<T, MODE>(E, gb, si, base, st))) return rc;
-        if ((rc = implicit_filter_planes<T, MODE>(F, gb, si, base + 2 * si.act_plane, st))) return rc;
+        if ((rc = implicit_filter_planes(F, gb, si, base + 2 * si.act_plane, st))) return rc;
         return implicit_tiles(base, base + 2 * si.act_plane, GI, gb, si, table, slotE, slotF, slotG,
                               stats, probe_out, status, probe, st);
     }
@@ -2194,8 +2222,28 @@ extern "C" int b2_conv_filter_planes(const int16_t* F, const b2_conv_dims* d, in
     int rc = geom_from(d, &f);
     if (rc) return rc;
     B2_REQUIRE(F && planes && pass_geom(f, pass, &g), "planes are not available for this convolution");
-    return implicit_filter_planes<short, MODE_FLEX16>(F, g, implicit_shape(g), planes,
-                                                      (cudaStream_t)stream);
+    return implicit_filter_planes(F, g, implicit_shape(g), planes, (cudaStream_t)stream);
+}
+
+extern "C" int b2_conv_filter_planes_many(const b2_conv_filter_job* list, int32_t n, int32_t* launches,
+                                          void* stream) {
+    B2_REQUIRE(list && n > 0 && launches, "bad argument");
+    *launches = 0;
+    for (int i0 = 0; i0 < n; i0 += kFilterJobs) {
+        FilterJobs jobs = {};
+        for (int i = i0; i < n && i < i0 + kFilterJobs; ++i) {
+            ConvGeom f, g;
+            int rc = geom_from(&list[i].dims, &f);
+            if (rc) return rc;
+            B2_REQUIRE(list[i].filters && list[i].planes && pass_geom(f, list[i].pass, &g),
+                       "planes are not available for this convolution");
+            if ((rc = add_filter_job(&jobs, list[i].filters, g, implicit_shape(g), list[i].planes))) return rc;
+        }
+        int rc = run_filter_jobs(jobs, (cudaStream_t)stream);
+        if (rc) return rc;
+        ++*launches;
+    }
+    return B2_OK;
 }
 
 extern "C" int b2_conv_flex16_planes(int32_t pass, const void* act_planes,

@@ -75,6 +75,8 @@ class _PlaneUser(object):
     use_planes = False
     plane_args = ()                 # indexes of the tensors read as planes in op.args / in_views
     splits = ()                     # those that this step splits unless their producer has
+    planes_built_first = False      # the first of the convolutions builds the filter planes of all
+    joint_planes = None             # ... this one: the steps whose planes it builds
     filter_planes = None
     filter_version = None
 
@@ -128,10 +130,20 @@ class _PlaneUser(object):
         t.kernel_launches += 1
         self.filter_version = fv.buffer.version
 
+    def _build_joint_planes(self, t):
+        users = self.joint_planes
+        jobs = (lib.ConvFilterJob * len(users))()
+        for job, s in zip(jobs, users):
+            job.filters, job.planes = s._ptr(s.in_views[s.filter_arg]), s.filter_ptr
+            job.dims, job.conv_pass = s.dims, s.conv_pass
+        n = C.c_int32()
+        lib.check(lib.raw().b2_conv_filter_planes_many(jobs, len(users), C.byref(n), t.stream.cuda_stream))
+        t.kernel_launches += n.value
+
     def refresh(self, t):
         """Rebuilds the cached filter planes when the filters have changed since they were built
         (called before every launch, and before every replay of a captured step list)."""
-        if not self.use_planes:
+        if not self.use_planes or self.planes_built_first:
             return
         fbuf = self.in_views[self.filter_arg].buffer
         if fbuf.last_write_step < 0 and self.filter_version != fbuf.version:
@@ -152,7 +164,11 @@ class _PlaneUser(object):
         st = t.stream.cuda_stream
         xbuf, fbuf = xv.buffer, fv.buffer
         planes_ptr = self._planes(t, self.plane_args[0])
-        if fbuf.last_write_step >= 0:
+        if self.joint_planes:
+            self._build_joint_planes(t)
+        elif self.planes_built_first:
+            pass
+        elif fbuf.last_write_step >= 0:
             self._build_filter_planes(t)     # filters written inside this computation
         else:
             self.refresh(t)
@@ -191,6 +207,22 @@ class _PlaneUser(object):
                 C.byref(ce), t._stats.data_ptr(), t._probe64.data_ptr(), t._status.data_ptr(),
                 probe, st))
         self._flex_probe_then(t, obuf, [xbuf, fbuf], call)
+
+
+def join_filter_planes(steps):
+    """The filter planes of the convolutions whose filters this computation writes after reading
+    them (a training step): the first of them builds all, one launch per 32 layers."""
+    written, mine = set(), []
+    for s in steps:
+        if getattr(s, "filter_arg", None) is not None:
+            buf = s.in_views[s.filter_arg].buffer
+            if buf.last_write_step >= 0 and buf not in written:
+                mine.append(s)
+        written.update(s.output_buffers())
+    for s in mine:
+        s.planes_built_first = True
+    if mine:
+        mine[0].joint_planes = mine
 
 
 class GemmStep(_Step):

@@ -65,6 +65,10 @@ class ConvDims(C.Structure):
                  "pad_w", "str_d", "str_h", "str_w", "dil_d", "dil_h", "dil_w")]
 
 
+class ConvFilterJob(C.Structure):
+    _fields_ = [("filters", C.c_void_p), ("planes", C.c_void_p), ("dims", ConvDims), ("conv_pass", C.c_int32)]
+
+
 class FlexScale(C.Structure):
     _fields_ = [("scale", C.c_float), ("inv_scale", C.c_float)]
 
@@ -132,6 +136,7 @@ def _load():
         "b2_conv_planes_info": (C.c_int, [C.POINTER(ConvDims), i32, C.POINTER(i32), C.POINTER(sz),
                                           C.POINTER(sz)]),
         "b2_conv_split_activations": (C.c_int, [vp, C.POINTER(ConvDims), i32, vp, vp]),
+        "b2_conv_filter_planes_many": (C.c_int, [C.POINTER(ConvFilterJob), i32, C.POINTER(i32), vp]),
         "b2_conv_split_planes": (C.c_int, [vp, i32, i32, i32, i32, vp, vp]),
         "b2_conv_filter_planes": (C.c_int, [vp, C.POINTER(ConvDims), i32, vp, vp]),
         "b2_conv_flex16_planes": (C.c_int, [i32, vp, vp, vp, C.POINTER(ConvDims), vp, i32, i32,

@@ -182,6 +182,7 @@ class Computation(object):
         final = []
         for s in self.steps:
             final.extend(planner.finalize_step(s))     # (a step may bring copies that precede it)
+        kernels.join_filter_planes(final)
         self.steps = final
         self._comm_steps = planner.comm_steps
         # (a parameter the results do not depend on still gets its tensor: callers pass a value)
