@@ -2009,6 +2009,13 @@ int run_update_implicit(const short* I, const short* E, const ConvGeom& g, const
     return run_update_planes(base, eplanes, acc, g, u, o, st);
 }
 
+// the fp32 kernel that converts on the way in; its scratch, 0 where it does not take the problem
+inline size_t update_f32_scratch(int mode, const ConvGeom& g, b2_update_f32* d) {
+    if (mode != MODE_F32X3 || g.dil_h != 1 || g.dil_w != 1 || !flat_depth(g) || getenv("B2_CONV_IM2COL")) return 0;
+    *d = {g.C, g.H, g.W, g.N, g.K, g.R, g.S, g.P, g.Q, g.pad_h, g.pad_w, g.str_h, g.str_w};
+    return b2_update_f32_scratch(*d);
+}
+
 template <typename T, int MODE>
 int run_update(const T* I, const T* E, void* U, const b2_conv_dims* d, const b2_flex_scale* table,
                int slotI, int slotE, int slotU, int* stats, void* scratch, size_t scratch_bytes,
@@ -2023,6 +2030,12 @@ int run_update(const T* I, const T* E, void* U, const b2_conv_dims* d, const b2_
             const UpdOut o = {U, nullptr, table, slotI, slotE, slotU, -1, stats, probe_out, status, probe};
             return run_update_implicit((const short*)I, (const short*)E, g, u, o, scratch, scratch_bytes, st);
         }
+    }
+    b2_update_f32 f32;
+    if (const size_t need = update_f32_scratch(MODE, g, &f32)) {
+        B2_REQUIRE(scratch && scratch_bytes >= need && ((uintptr_t)scratch & 1023) == 0,
+                   "convolution update needs %zu bytes of 1024-byte aligned scratch, got %zu", need, scratch_bytes);
+        return b2_update_f32_launch(f32, (const float*)I, (const float*)E, (float*)U, scratch, status, st);
     }
     const long long kg_ll = (long long)g.M * g.P * g.Q * g.N;
     B2_REQUIRE(kg_ll < (1LL << 31) - 256 && (long long)g.C * g.D * g.H * g.W * g.N < (1LL << 31) &&
@@ -2135,8 +2148,9 @@ extern "C" int b2_conv_launches(int32_t flex, const b2_conv_dims* d, int32_t pas
     ConvGeom gp;
     b2_direct_args direct;
     UpdShape u;
+    b2_update_f32 f32;
     if (pass == 2)
-        *launches = !update_goes_in_planes(mode, g, &u) && update_shape(mode, g).splits > 1 ? 4 : 3;
+        *launches = update_f32_scratch(mode, g, &f32) ? 2 : !update_goes_in_planes(mode, g, &u) && update_shape(mode, g).splits > 1 ? 4 : 3;
     else
         *launches = !(flex && pass_geom(g, pass, &gp)) && conv_goes_direct(mode, g, pass, &direct) ? 1 : 3;
     return B2_OK;
@@ -2321,9 +2335,11 @@ extern "C" int b2_conv_update_scratch_bytes(int32_t flex, const b2_conv_dims* d,
     int rc = geom_from(d, &g);
     if (rc) return rc;
     B2_REQUIRE(bytes, "null argument");
+    const int mode = flex ? MODE_FLEX16 : MODE_F32X3;
     UpdShape u;
-    *bytes = update_goes_in_planes(flex ? MODE_FLEX16 : MODE_F32X3, g, &u)
-                 ? update_planes_bytes(u) : update_shape(flex ? MODE_FLEX16 : MODE_F32X3, g).bytes;
+    b2_update_f32 f32;
+    const size_t direct = update_f32_scratch(mode, g, &f32);
+    *bytes = update_goes_in_planes(mode, g, &u) ? update_planes_bytes(u) : direct ? direct : update_shape(mode, g).bytes;
     return B2_OK;
 }
 

@@ -14,7 +14,7 @@ pytestmark = pytest.mark.gpu
 CASES = [(3, 9, 7, 5, 17, 3, 3, 1, 1, 1, 1), (16, 8, 8, 100, 16, 3, 3, 1, 1, 1, 1),
          (5, 8, 9, 33, 40, 5, 5, 2, 2, 1, 1), (130, 5, 5, 20, 130, 3, 3, 2, 1, 2, 1),
          (2, 3, 40, 130, 9, 1, 31, 0, 1, 1, 1), (2, 3, 40, 130, 9, 1, 32, 0, 1, 1, 3),
-         (64, 8, 8, 1, 64, 3, 3, 1, 1, 1, 1), (33, 6, 6, 64, 32, 1, 1, 0, 2, 1, 1)]
+         (64, 8, 8, 1, 64, 3, 3, 1, 1, 1, 1), (20, 33, 31, 40, 70, 3, 2, 1, 1, 1, 1), (33, 6, 6, 64, 32, 1, 1, 0, 2, 1, 1)]
 
 
 @pytest.mark.parametrize("case", CASES)
@@ -52,6 +52,9 @@ def test_fp32_convolution_passes(case):
     gx = torch.nn.grad.conv2d_input(xn.shape, fn, en, stride=st, padding=pad, dilation=dil)
     close(run(raw.b2_conv_bprop_f32, lib.conv_bprop_scratch_bytes(False, d), (de, df), (Cc, H, W, N)),
           gx.permute(1, 2, 3, 0))
+    gf = torch.nn.grad.conv2d_weight(xn, fn.shape, en, stride=st, padding=pad, dilation=dil)
+    close(run(raw.b2_conv_update_f32, lib.conv_update_scratch_bytes(False, d), (dx, de), (Cc, R, S, K)),
+          gf.permute(1, 2, 3, 0))
     if launches != 1:
         return
     for bias, res, relu in ((db, de, 1), (db, None, 0), (None, de, 0)):
