@@ -364,6 +364,10 @@ int b2_conv_flex16_planes_fused(int32_t pass, const void* act_planes, const void
 int b2_conv_bprop_scratch_bytes(int32_t flex, const b2_conv_dims* d, size_t* bytes);
 int b2_conv_bprop_f32(const float* E, const float* F, float* GI, const b2_conv_dims* d,
                       void* scratch, size_t scratch_bytes, int32_t* status, void* stream);
+/* With the tail of back-propagation, where b2_conv_launches(0, d, 1) is 1: GI = conv + residual, times
+ * (mask > 0); both in the input's layout, either may be NULL. */
+int b2_conv_bprop_f32_fused(const float* E, const float* F, float* GI, const b2_conv_dims* d,
+                            const float* residual, const float* mask, int32_t* status, void* stream);
 int b2_conv_bprop_flex16(const int16_t* E, const int16_t* F, int16_t* GI, const b2_conv_dims* d,
                          const b2_flex_scale* table, int32_t slotE, int32_t slotF, int32_t slotGI,
                          int32_t* stats, void* scratch, size_t scratch_bytes, uint64_t* probe_out,

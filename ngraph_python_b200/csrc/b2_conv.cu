@@ -2165,7 +2165,7 @@ extern "C" int b2_conv_fprop_f32_fused(const float* I, const float* F, float* O,
     B2_REQUIRE(I && F && O, "null tensor");
     b2_direct_args direct;
     B2_REQUIRE(conv_goes_direct(MODE_F32X3, g, 0, &direct), "this convolution takes no fused tail");
-    direct.tail = 1; direct.bias = bias; direct.residual = residual; direct.relu = relu ? 1 : 0;
+    direct.bias = bias; direct.residual = residual; direct.relu = relu ? 1 : 0;
     return launch_direct(direct, I, F, O, nullptr, 0, 0, 0, nullptr, nullptr, status, 0, (cudaStream_t)stream);
 }
 
@@ -2328,6 +2328,18 @@ extern "C" int b2_conv_bprop_flex16(const int16_t* E, const int16_t* F, int16_t*
     return run_bprop<short, MODE_FLEX16>(E, F, GI, d, table, slotE, slotF, slotGI, stats, scratch,
                                          scratch_bytes, (unsigned long long*)probe_out, status,
                                          probe ? 1 : 0, (cudaStream_t)stream);
+}
+
+extern "C" int b2_conv_bprop_f32_fused(const float* E, const float* F, float* GI, const b2_conv_dims* d,
+                                       const float* residual, const float* mask, int32_t* status, void* stream) {
+    ConvGeom g;
+    int rc = geom_from(d, &g);
+    if (rc) return rc;
+    B2_REQUIRE(E && F && GI, "null tensor");
+    b2_direct_args direct;
+    B2_REQUIRE(conv_goes_direct(MODE_F32X3, g, 1, &direct), "this convolution takes no fused tail");
+    direct.residual = residual; direct.mask = mask;
+    return launch_direct(direct, E, F, GI, nullptr, 0, 0, 0, nullptr, nullptr, status, 0, (cudaStream_t)stream);
 }
 
 extern "C" int b2_conv_update_scratch_bytes(int32_t flex, const b2_conv_dims* d, size_t* bytes) {

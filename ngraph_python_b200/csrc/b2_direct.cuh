@@ -457,15 +457,10 @@ direct_kernel(const __grid_constant__ DirectParams p) {
     bool ok = true;
     int stat = 0;
     unsigned long long pmax = 0;
-    float fstat = 0.0f;
     int sh = 0;
-    float f_prod = 0.f, s_bias = 0.f, s_res = 0.f;
     if (MODE == MODE_FLEX16 && warp < 8) {
         const float q_out = a.probe ? 1.0f : a.table[a.slotC].inv_scale;
-        f_prod = a.table[a.slotA].scale * a.table[a.slotB].scale * q_out;
-        sh = -ilogbf(f_prod);
-        if (a.tail && a.bias) s_bias = a.table[a.slot_bias].scale * q_out;
-        if (a.tail && a.residual) s_res = a.table[a.slot_res].scale * q_out;
+        sh = -ilogbf(a.table[a.slotA].scale * a.table[a.slotB].scale * q_out);
     }
     auto finish = [&](int c0, Sum* v) {
         // eight results of one row: tail, rescale, statistics, store
@@ -480,16 +475,7 @@ direct_kernel(const __grid_constant__ DirectParams p) {
                 q[j] = 0;
                 if (j >= live) continue;
                 const long long x = (long long)v[j];
-                if (a.tail) {
-                    float y = (float)x * f_prod;
-                    if (a.bias) y += (float)((const short*)a.bias)[col + j] * s_bias;
-                    if (a.residual) y += (float)((const short*)a.residual)[at + j * dc] * s_res;
-                    if (a.relu) y = fmaxf(y, 0.0f);
-                    if (a.probe) { fstat = fmaxf(fstat, fabsf(y)); continue; }
-                    y = fminf(fmaxf(y, -32768.0f), 32767.0f);
-                    fstat = fmaxf(fstat, fabsf(y));
-                    q[j] = __float2int_rn(y);
-                } else if (a.probe) {
+                if (a.probe) {
                     const unsigned long long m = (unsigned long long)(x < 0 ? -x : x);
                     pmax = m > pmax ? m : pmax;
                 } else {
@@ -511,14 +497,32 @@ direct_kernel(const __grid_constant__ DirectParams p) {
                     if (j < live) out[j * dc] = (short)q[j];
             }
         } else {
-            float y[8];
+            // (one uniform branch per operand, its eight loads together)
+            float y[8], t[8];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                y[j] = (float)v[j];
-                if (j >= live || !a.tail) continue;
-                if (a.bias) y[j] += ((const float*)a.bias)[col + j];
-                if (a.residual) y[j] += ((const float*)a.residual)[at + j * dc];
-                if (a.relu) y[j] = y[j] < 0.0f ? 0.0f : y[j];      // (keeps NaN, as max(x, 0) does)
+            for (int j = 0; j < 8; ++j) y[j] = (float)v[j];
+            auto fetch = [&](const float* x, long long step) {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) t[j] = j < live ? __ldg(x + j * step) : 0.0f;
+            };
+            if (a.bias) {
+                fetch(a.bias + col, 1);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) y[j] += t[j];
+            }
+            if (a.residual) {
+                fetch(a.residual + at, dc);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) y[j] += t[j];
+            }
+            if (a.relu) {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) y[j] = y[j] < 0.0f ? 0.0f : y[j];      // (keeps NaN, as max(x, 0) does)
+            }
+            if (a.mask) {
+                fetch(a.mask + at, dc);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) y[j] *= t[j] > 0.0f ? 1.0f : 0.0f;     // (likewise)
             }
             float* out = (float*)a.C + at;
             if (!a.colmajor && live >= 8 && ((uintptr_t)out & 15) == 0) {
@@ -584,10 +588,6 @@ direct_kernel(const __grid_constant__ DirectParams p) {
         cluster_sync();                                           // peers may still be reading
     }
     if (MODE == MODE_FLEX16 && warp < 8) {
-        if (a.tail) {
-            if (a.probe) pmax = (unsigned long long)__float_as_uint(fstat);
-            else stat = (int)rintf(fstat);
-        }
         if (a.probe) {
             for (int o = 16; o > 0; o >>= 1) {
                 const unsigned long long t = __shfl_xor_sync(0xffffffffu, pmax, o);

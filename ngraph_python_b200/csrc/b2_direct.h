@@ -32,10 +32,10 @@ struct b2_direct_args {
     unsigned long long* probe_out;
     int* status;
     int probe;
-    // tail: y = relu?(product + bias[col] + residual), residual laid out as C; flex16: in fp32, one
-    // quantisation, the probe is the bit pattern of max |y|
-    int tail, relu, slot_bias, slot_res;
-    const void *bias, *residual;
+    // tail, fp32: y = relu?(product + bias[col] + residual), then 0 where mask (given) is not positive;
+    // residual and mask laid out as C
+    int relu;
+    const float *bias, *residual, *mask;
 };
 
 // Estimated cycles of a launch, negative where the kernel does not take the problem.

@@ -373,13 +373,11 @@ class ConvStep(_PlaneUser, _Step):
 
 def takes_conv_tail(fprop, t, conv_pass=lib.CONV_FPROP):
     """Whether the convolution's kernel evaluates the elementwise tail behind it: the flex16 tile
-    kernel, for the forward pass the fp32 kernel that gathers its operands."""
+    kernel, the fp32 kernel that gathers its operands."""
     d = _conv_dims_of(fprop, t)
-    if conv_pass != lib.CONV_FPROP:
-        return t.flex and lib.conv_planes_info(d, conv_pass)[0]
     if t.flex:
-        return lib.conv_planes_info(d, lib.CONV_FPROP)[0]
-    return lib.conv_launches(False, d, lib.CONV_FPROP) == 1
+        return lib.conv_planes_info(d, conv_pass)[0]
+    return lib.conv_launches(False, d, conv_pass) == 1
 
 
 def _conv_dims_of(fprop, t):
@@ -441,7 +439,7 @@ class _ConvGradStep(_PlaneUser, _Step):
         if self.what == "bprop":
             self._setup_planes(t, lib.CONV_BPROP, 0, 1)      # streamed: delta; filters: args[1]
         if epilogue:
-            if not self.use_planes:
+            if not (self.use_planes if self.flex else self.launches == 1):
                 raise ValueError("a fused convolution epilogue needs a kernel that takes one")
             self.probe_is_float = True
             self.write_int16 = True          # the planner clears it when only planes are read
@@ -461,6 +459,15 @@ class _ConvGradStep(_PlaneUser, _Step):
         else:
             first, second = bv, av       # I, E
             f32, f16 = raw.b2_conv_update_f32, raw.b2_conv_update_flex16
+        if self.epi:
+            extra = [self._ptr(v) for v in self.in_views[2:]]
+            residual = extra.pop(0) if self.epi.get("residual") is not None else None
+            mask = extra.pop(0) if self.epi.get("mask") is not None else None
+            lib.check(raw.b2_conv_bprop_f32_fused(self._ptr(first), self._ptr(second), self._ptr(ov),
+                                                  C.byref(self.dims), residual, mask,
+                                                  t._status.data_ptr(), st))
+            t.kernel_launches += self.launches
+            return
         if not self.flex:
             lib.check(f32(self._ptr(first), self._ptr(second), self._ptr(ov), C.byref(self.dims),
                           sp, sb, t._status.data_ptr(), st))

@@ -144,6 +144,7 @@ def _load():
         "b2_conv_flex16_planes_fused": (C.c_int, [i32, vp, vp, vp, C.POINTER(ConvDims), vp, i32, i32,
                                                   i32, C.POINTER(ConvEpilogue), vp, vp, vp, i32, vp]),
         "b2_conv_bprop_scratch_bytes": (C.c_int, [i32, C.POINTER(ConvDims), C.POINTER(sz)]),
+        "b2_conv_bprop_f32_fused": (C.c_int, [vp, vp, vp, C.POINTER(ConvDims), vp, vp, vp, vp]),
         "b2_conv_bprop_f32": (C.c_int, [vp, vp, vp, C.POINTER(ConvDims), vp, sz, vp, vp]),
         "b2_conv_bprop_flex16": (C.c_int, [vp, vp, vp, C.POINTER(ConvDims), vp, i32, i32, i32, vp,
                                            vp, sz, vp, vp, i32, vp]),

@@ -68,4 +68,15 @@ def test_fp32_convolution_passes(case):
         want = want + b.double()[:, None, None, None] if bias is not None else want
         want = want + e.double() if res is not None else want
         close(out.cpu().double(), want.clamp(min=0) if relu else want)
+    if lib.conv_launches(False, d, lib.CONV_BPROP) == 1:
+        other, act = torch.randn(x.shape, generator=g), torch.randn(x.shape, generator=g)
+        for res, mask in ((other, act), (None, act), (other, None)):
+            out = torch.full(x.shape, 7.0, device="cuda")
+            keep = [None if v is None else v.cuda() for v in (res, mask)]
+            lib.check(raw.b2_conv_bprop_f32_fused(
+                de.data_ptr(), df.data_ptr(), out.data_ptr(), C.byref(d),
+                *(None if v is None else v.data_ptr() for v in keep), status.data_ptr(), 0))
+            torch.cuda.synchronize()
+            want = gx.permute(1, 2, 3, 0) + (0 if res is None else res.double())
+            close(out.cpu().double(), want if mask is None else want * (mask > 0))
     assert int(status.item()) == 0
