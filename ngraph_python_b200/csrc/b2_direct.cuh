@@ -221,18 +221,18 @@ direct_kernel(const __grid_constant__ DirectParams p) {
         asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     }
     if (AK == B2_OPERAND_GATHER) {
-        // offset and tap of every column of this slice
+        // offset of every column of this slice and the bit of its tap (none beyond K)
         const b2_gather& g = a.g;
         const int RS = g.R * g.S;
         for (int i = threadIdx.x; i < nkb * KB; i += kDirThreads) {
             const int k = kb0 * KB + i;
-            int2 e = make_int2(0, 31);
+            int2 e = make_int2(0, 0);
             if (k < a.K) {
                 const int c = g.bprop ? k % g.channels : k / RS, rs = g.bprop ? k / g.channels : k % RS;
                 const int r = rs / g.S, s = rs - r * g.S;
                 const int dh = g.bprop ? -(r * g.dil_h / g.str_h) : r * g.dil_h;
                 const int dw = g.bprop ? -(s * g.dil_w / g.str_w) : s * g.dil_w;
-                e = make_int2(((c * g.H + dh) * g.W + dw) * g.N, rs);
+                e = make_int2(((c * g.H + dh) * g.W + dw) * g.N, (int)(1u << rs));
             }
             tab[i] = e;
         }
@@ -308,17 +308,19 @@ direct_kernel(const __grid_constant__ DirectParams p) {
 #pragma unroll
                 for (int i = 0; i < A_UNITS; ++i) {
                     const int kc = (a_c0 + a_cs * i) * PER;
+                    int4 pair_of;
 #pragma unroll
                     for (int j = 0; j < PER; ++j) {
                         unsigned v = 0;
                         long long o;
                         bool in0, in1 = false;
                         if (AK == B2_OPERAND_GATHER) {
-                            const int2 t = tab[kt + kc + j];
+                            // two entries to a load
+                            if (j % 2 == 0) pair_of = *(const int4*)(tab + kt + kc + j);
+                            const int2 t = j % 2 == 0 ? make_int2(pair_of.x, pair_of.y) : make_int2(pair_of.z, pair_of.w);
                             o = t.x;
-                            in0 = (mask[0] >> t.y) & 1u;
-                            if (GR == 2) in1 = (mask[GR - 1] >> t.y) & 1u;
-                            if (k0 + kc + j >= a.K) in0 = in1 = false;
+                            in0 = (mask[0] & (unsigned)t.y) != 0;
+                            if (GR == 2) in1 = (mask[GR - 1] & (unsigned)t.y) != 0;
                         } else {
                             o = (long long)(k0 + kc + j) * a.a_ks;
                             in0 = mask[0] && k0 + kc + j < a.K;
