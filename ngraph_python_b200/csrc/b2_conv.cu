@@ -74,37 +74,96 @@ inline bool flat_depth(const ConvGeom& g) {
     return g.D == 1 && g.T == 1 && g.M == 1 && g.pad_d == 0;
 }
 
-// Whether a pass (0 forward, 1 input gradient) goes through the kernel that gathers and converts its
-// operands on the way into shared memory (b2_direct.cuh), and its arguments without the tensors.  It
-// does what the gather + GEMM path does, with one launch and without writing the unrolled planes
-// (8 bytes for each of the R*S copies of a value, and reading them again); the planes pay only where a
-// long list of output channels would have the gather repeated for every 128 of them.
-inline bool conv_goes_direct(int mode, const ConvGeom& g, int pass, b2_direct_args* out) {
-    if (!flat_depth(g) || getenv("B2_CONV_IM2COL")) return false;
-    const long long rows = pass ? (long long)g.H * g.W * g.N : (long long)g.P * g.Q * g.N;
-    const long long k = (long long)(pass ? g.K : g.C) * g.R * g.S;
-    if (rows >= (1LL << 31) - 256 || k > 32768) return false;
+inline int floor_div(int a, int b) { return a >= 0 ? a / b : -((-a + b - 1) / b); }
+
+// One direction of a tile's window: output positions tile*g .. tile*g + g-1, filter extent r.
+//   forward:        input = out * str - pad + tap
+//   input gradient: error = (out + pad - tap) / str where that divides; g is a multiple of str, so every
+//                   tile has the same residues and steps g / str errors further
+inline void window(int bprop, int g, int r, int pad, int str, int* extent, int* off, int* step) {
+    if (!bprop) {
+        *extent = (g - 1) * str + r; *off = -pad; *step = g * str;
+    } else {
+        const int lo = -floor_div(-(pad - r + 1), str), hi = floor_div(g - 1 + pad, str);
+        *extent = hi - lo + 1 > 1 ? hi - lo + 1 : 1; *off = lo; *step = g / str;
+    }
+}
+
+// The arguments without the tensors of a pass (0 forward, 1 input gradient) for the kernel that gathers
+// and converts its operands on the way in (b2_direct.cuh), with gh x gw pixels to a row of the product;
+// false where a tile does not fit the convolution.  One pixel: every value of a window is gathered and
+// converted once per tap.  Several: the window they share is gathered once (2x2 pixels under 3x3
+// filters: 4 values a pixel and channel instead of 9) against filters padded with zeros, and as many
+// times fewer rows of the product fill the machine in one wave (16 channels, 32x32, batch 100: 800
+// tiles of 128 rows before).  The input gradient of a strided convolution needs tiles that are multiples
+// of the stride, in which every pixel finds its own residue class of taps.
+inline bool direct_args(int mode, const ConvGeom& g, int pass, int gh, int gw, b2_direct_args* out) {
+    const bool tiled = gh * gw > 1, strided = g.str_h > 1 || g.str_w > 1;
+    const int result = pass ? g.C : g.K, read = pass ? g.K : g.C;         // channels
+    const int rp = pass ? g.H : g.P, rq = pass ? g.W : g.Q;               // extents of the result
+    if (tiled && (g.dil_h != 1 || g.dil_w != 1 || result % 8 != 0)) return false;
+    if (pass && strided && (gh % g.str_h != 0 || gw % g.str_w != 0)) return false;
     b2_direct_args d = {};
     d.flex = mode == MODE_FLEX16;
     d.a_kind = B2_OPERAND_GATHER;
-    d.M = (int)rows; d.N = pass ? g.C : g.K; d.K = (int)k;
-    d.b_kind = pass ? B2_OPERAND_K : B2_OPERAND_ROWS;
-    d.b_rs = pass ? (long long)g.R * g.S * g.K : 1;
-    d.b_ks = pass ? 1 : g.K;
-    d.g.channels = pass ? g.K : g.C; d.g.H = pass ? g.P : g.H; d.g.W = pass ? g.Q : g.W; d.g.N = g.N;
-    d.g.P = pass ? g.H : g.P; d.g.Q = pass ? g.W : g.Q; d.g.R = g.R; d.g.S = g.S;
-    d.g.pad_h = g.pad_h; d.g.pad_w = g.pad_w; d.g.str_h = g.str_h; d.g.str_w = g.str_w;
-    d.g.dil_h = g.dil_h; d.g.dil_w = g.dil_w; d.g.bprop = pass;
-    d.ldc = rows; d.colmajor = 1;
+    b2_gather& t = d.g;
+    t.channels = read; t.H = pass ? g.P : g.H; t.W = pass ? g.Q : g.W; t.N = g.N;
+    t.P = (rp + gh - 1) / gh; t.Q = (rq + gw - 1) / gw;
+    t.channel_last = pass;
+    if (tiled) {
+        window(pass, gh, g.R, g.pad_h, g.str_h, &t.R, &t.off_h, &t.step_h);
+        window(pass, gw, g.S, g.pad_w, g.str_w, &t.S, &t.off_w, &t.step_w);
+        t.tap_h = t.tap_w = 1;
+        t.gh = gh; t.gw = gw; t.kt = result; t.out_p = rp; t.out_q = rq; t.fr = g.R; t.fs = g.S;
+        t.f0_h = pass ? g.pad_h - g.str_h * t.off_h : 0; t.f0_w = pass ? g.pad_w - g.str_w * t.off_w : 0;
+        t.f1_h = pass ? -g.str_h : 1; t.f1_w = pass ? -g.str_w : 1;
+        t.f2_h = pass ? 1 : -g.str_h; t.f2_w = pass ? 1 : -g.str_w;
+        d.b_kind = B2_OPERAND_FILTER;
+        d.b_rs = pass ? (long long)g.R * g.S * g.K : 1;
+        d.b_ks = pass ? 1 : (long long)g.R * g.S * g.K;
+    } else {
+        t.R = g.R; t.S = g.S; t.gh = t.gw = 1;
+        t.off_h = pass ? g.pad_h : -g.pad_h; t.off_w = pass ? g.pad_w : -g.pad_w;
+        t.step_h = g.str_h; t.step_w = g.str_w;
+        t.tap_h = pass ? -g.dil_h : g.dil_h; t.tap_w = pass ? -g.dil_w : g.dil_w;
+        d.b_kind = pass ? B2_OPERAND_K : B2_OPERAND_ROWS;
+        d.b_rs = pass ? (long long)g.R * g.S * g.K : 1;
+        d.b_ks = pass ? 1 : g.K;
+    }
+    const long long rows = (long long)t.P * t.Q * g.N, k = (long long)read * t.R * t.S;
+    if (rows >= (1LL << 31) - 256 || k > 32768 || (long long)result * g.R * g.S * read >= (1LL << 31)) return false;
+    d.M = (int)rows; d.N = gh * gw * result; d.K = (int)k;
+    d.ldc = (long long)rp * rq * g.N; d.colmajor = 1;
     *out = d;
-    const long long cost = b2_direct_cost(d);
+    return true;
+}
+
+// Whether a pass goes that way, with the best tile.  It does what the gather + GEMM path does, with one
+// launch and without writing the unrolled planes (8 bytes for each of the R*S copies of a value, and
+// reading them again); the planes pay only where a long list of output channels would have the gather
+// repeated for every 128 of them.
+inline bool conv_goes_direct(int mode, const ConvGeom& g, int pass, b2_direct_args* out) {
+    if (!flat_depth(g) || getenv("B2_CONV_IM2COL")) return false;
+    long long best = -1;
+    for (int a = 1; a <= 2; ++a)
+        for (int b = 1; b <= 2; ++b) {
+            b2_direct_args d;
+            if (!direct_args(mode, g, pass, pass ? a * g.str_h : a, pass ? b * g.str_w : b, &d)) continue;
+            const long long cost = b2_direct_cost(d);
+            if (cost < 0 || (best >= 0 && cost >= best)) continue;
+            best = cost;
+            *out = d;
+        }
+    if (best < 0) return false;
+    const long long rows = pass ? (long long)g.H * g.W * g.N : (long long)g.P * g.Q * g.N;
+    const long long k = (long long)(pass ? g.K : g.C) * g.R * g.S;
+    if (rows >= (1LL << 31) - 256) return true;
     // the planes of the unrolled rows once out and once back (cycles at 5 TB/s), then the tile kernel
-    const Shapes s = shapes_for(mode, (int)rows, d.N, (int)k);
+    const Shapes s = shapes_for(mode, (int)rows, pass ? g.C : g.K, (int)k);
     const long long planes = rows * s.Kp * s.esize * 4 / 2600;
     const long long kb = (mode == MODE_FLEX16 ? 1430LL : 1100LL) * (128 + s.bn) / 256;
     const long long tiles = (long long)(s.Mp / kBlockM) * (s.Np / s.bn);
-    return cost >= 0 &&
-           cost < 13000 + planes + (tiles + 147) / 148 * (3500 + (long long)(s.Kp * s.esize / kKBytes) * kb);
+    return best < 13000 + planes + (tiles + 147) / 148 * (3500 + (long long)(s.Kp * s.esize / kKBytes) * kb);
 }
 
 inline int launch_direct(b2_direct_args& d, const void* A, const void* B, void* C,
@@ -1047,21 +1106,6 @@ struct ImplicitShape {
     int gh, gw, wh, ww, off_h, off_w, step_h, step_w, tiles;
     size_t act_plane, filt_bytes, bytes;
 };
-
-inline int floor_div(int a, int b) { return a >= 0 ? a / b : -((-a + b - 1) / b); }
-
-// One direction of a tile's window: output positions tile*g .. tile*g + g-1, filter extent r.
-//   forward:        input = out * str - pad + tap
-//   input gradient: error = (out + pad - tap) / str where that divides; g is a multiple of str, so every
-//                   tile has the same residues and steps g / str errors further
-inline void window(int bprop, int g, int r, int pad, int str, int* extent, int* off, int* step) {
-    if (!bprop) {
-        *extent = (g - 1) * str + r; *off = -pad; *step = g * str;
-    } else {
-        const int lo = -floor_div(-(pad - r + 1), str), hi = floor_div(g - 1 + pad, str);
-        *extent = hi - lo + 1 > 1 ? hi - lo + 1 : 1; *off = lo; *step = g / str;
-    }
-}
 
 // the shape with tiles of gh x gw output pixels; nstages < 2 where it does not fit
 ImplicitShape implicit_shape_for(const ConvGeom& g, int gh, int gw) {

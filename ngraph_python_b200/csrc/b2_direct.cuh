@@ -39,6 +39,8 @@ __host__ __device__ constexpr int dir_tmem_cols(int mode, int bn) {
     return c;
 }
 
+__host__ __device__ inline bool filter_tiles(const b2_direct_args& a) { return a.b_kind == B2_OPERAND_FILTER; }
+
 struct DirectParams {
     b2_direct_args a;
     int num_kb, kb_per_split, splits;
@@ -201,6 +203,8 @@ direct_kernel(const __grid_constant__ DirectParams p) {
     unsigned* tmem_holder = (unsigned*)(tmem_full + 1);
     int* fail_flag = (int*)(tmem_holder + 1);
     int2* tab = (int2*)((unsigned char*)full_bar + 128);                          // [K of the slice] gather table
+    int2* ftab = tab + p.kb_per_split * KB;                                       // likewise, of the filters
+    const bool tiled = AK == B2_OPERAND_GATHER && filter_tiles(p.a);
 
     const int warp = warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
     const b2_direct_args& a = p.a;
@@ -226,15 +230,15 @@ direct_kernel(const __grid_constant__ DirectParams p) {
         const int RS = g.R * g.S;
         for (int i = threadIdx.x; i < nkb * KB; i += kDirThreads) {
             const int k = kb0 * KB + i;
-            int2 e = make_int2(0, 0);
+            int2 e = make_int2(0, 0), f = make_int2(0, 0x7fff7fff);       // (no filter has that tap)
             if (k < a.K) {
-                const int c = g.bprop ? k % g.channels : k / RS, rs = g.bprop ? k / g.channels : k % RS;
+                const int c = g.channel_last ? k % g.channels : k / RS, rs = g.channel_last ? k / g.channels : k % RS;
                 const int r = rs / g.S, s = rs - r * g.S;
-                const int dh = g.bprop ? -(r * g.dil_h / g.str_h) : r * g.dil_h;
-                const int dw = g.bprop ? -(s * g.dil_w / g.str_w) : s * g.dil_w;
-                e = make_int2(((c * g.H + dh) * g.W + dw) * g.N, (int)(1u << rs));
+                e = make_int2(((c * g.H + r * g.tap_h) * g.W + s * g.tap_w) * g.N, (int)(1u << rs));
+                f = make_int2(c * (int)a.b_ks, ((g.f0_h + g.f1_h * r) & 0xffff) << 16 | ((g.f0_w + g.f1_w * s) & 0xffff));
             }
             tab[i] = e;
+            if (tiled) ftab[i] = f;
         }
     }
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -270,24 +274,12 @@ direct_kernel(const __grid_constant__ DirectParams p) {
                     base = 0;
                     if (row < a.M) {
                         const int n = row % g.N, pq = row / g.N, q = pq % g.Q, pp = pq / g.Q;
-                        int h0, w0;
-                        if (g.bprop) {
-                            const int th = pp + g.pad_h, tw = q + g.pad_w;
-                            h0 = th / g.str_h; w0 = tw / g.str_w;
-                            for (int t = 0; t < g.R * g.S; ++t) {
-                                const int r = t / g.S * g.dil_h, s = t % g.S * g.dil_w;
-                                const int hh = h0 - r / g.str_h, ww = w0 - s / g.str_w;
-                                if (th >= r && tw >= s && (th - r) % g.str_h == 0 && (tw - s) % g.str_w == 0 &&
-                                    hh < g.H && ww < g.W)
-                                    mask[e] |= 1u << t;
-                            }
-                        } else {
-                            h0 = pp * g.str_h - g.pad_h; w0 = q * g.str_w - g.pad_w;
-                            for (int t = 0; t < g.R * g.S; ++t) {
-                                const int hh = h0 + t / g.S * g.dil_h, ww = w0 + t % g.S * g.dil_w;
+                        const int h0 = pp * g.step_h + g.off_h, w0 = q * g.step_w + g.off_w;
+                        for (int r = 0, t = 0; r < g.R; ++r)
+                            for (int s = 0; s < g.S; ++s, ++t) {
+                                const int hh = h0 + r * g.tap_h, ww = w0 + s * g.tap_w;
                                 if (hh >= 0 && hh < g.H && ww >= 0 && ww < g.W) mask[e] |= 1u << t;
                             }
-                        }
                         base = ((long long)h0 * g.W + w0) * g.N + n;
                     }
                 } else if (row < a.M) {
@@ -300,6 +292,20 @@ direct_kernel(const __grid_constant__ DirectParams p) {
         long long a_at[ATile::kKUnits], b_at[BTile::kKUnits];
         if (AK == B2_OPERAND_K) ATile::offsets_k(a_at, a.a_rs, m0, a.M, warp, lane);
         BTile::offsets_k(b_at, a.b_rs, n0, a.N, warp, lane);
+        // filter rows of this lane: channel's place in the filters and the pixel's share of the tap
+        constexpr int FR = BTile::kUnits * GR;
+        int f_at[FR], f_h[FR], f_w[FR];
+        if (AK == B2_OPERAND_GATHER && tiled) {
+            const b2_gather& g = a.g;
+#pragma unroll
+            for (int i = 0; i < FR; ++i) {
+                const int lr = (i / GR) * 32 * GR + GR * lane + i % GR, row = n0 + lr, pix = row / g.kt;
+                const int gy = pix / g.gw, gx = pix - gy * g.gw;
+                f_at[i] = (row - pix * g.kt) * (int)a.b_rs;
+                f_h[i] = lr < BN && row < a.N ? g.f2_h * gy : 1 << 20;
+                f_w[i] = g.f2_w * gx;
+            }
+        }
         auto load = [&](int kb, ATile& A, BTile& B) {
             const int kt = kb * KB, k0 = kb0 * KB + kt;
             if (AK == B2_OPERAND_K) {
@@ -340,7 +346,28 @@ direct_kernel(const __grid_constant__ DirectParams p) {
                     }
                 }
             }
-            if (a.b_kind == B2_OPERAND_K) {
+            if (AK == B2_OPERAND_GATHER && tiled) {
+                const b2_gather& g = a.g;
+                const int mult = (int)(g.channel_last ? a.g.channels : g.kt);     // filters: tap stride
+#pragma unroll
+                for (int j = 0; j < PER; ++j) {
+                    const int2 f = ftab[kt + warp * PER + j];
+                    const int th = f.y >> 16, tw = (short)f.y;
+#pragma unroll
+                    for (int i = 0; i < BTile::kUnits; ++i) {
+                        unsigned v = 0;
+#pragma unroll
+                        for (int e = 0; e < GR; ++e) {
+                            const int r = th + f_h[i * GR + e], s = tw + f_w[i * GR + e];
+                            if ((unsigned)r >= (unsigned)g.fr || (unsigned)s >= (unsigned)g.fs) continue;
+                            const int at = f.x + f_at[i * GR + e] + (r * g.fs + s) * mult;
+                            if (MODE == MODE_FLEX16) v |= (unsigned)__ldg((const unsigned short*)a.B + at) << (16 * e);
+                            else v = __float_as_uint(__ldg((const float*)a.B + at));
+                        }
+                        B.r[PER * i + j] = v;
+                    }
+                }
+            } else if (a.b_kind == B2_OPERAND_K) {
                 B.load_k(a.B, b_at, k0, a.K - k0, p.b_vec, lane);
             } else {
                 // chunk = warp, groups of 32 (64) rows
@@ -464,11 +491,26 @@ direct_kernel(const __grid_constant__ DirectParams p) {
         const float q_out = a.probe ? 1.0f : a.table[a.slotC].inv_scale;
         sh = -ilogbf(a.table[a.slotA].scale * a.table[a.slotB].scale * q_out);
     }
+    // tiles of several pixels: where the row's tile starts
+    int tile_p = 0, tile_q = 0;
+    long long tile_at = 0;
+    if (tiled) {
+        const int n = row % a.g.N, pq = row / a.g.N;
+        tile_p = pq / a.g.Q * a.g.gh; tile_q = pq % a.g.Q * a.g.gw;
+        tile_at = ((long long)tile_p * a.g.out_q + tile_q) * a.g.N + n;
+    }
     auto finish = [&](int c0, Sum* v) {
         // eight results of one row: tail, rescale, statistics, store
         if (row >= a.M) return;
-        const int col = n0 + c0, live = a.N - col;
-        const long long at = a.colmajor ? (long long)col * a.ldc + row : (long long)row * a.ldc + col;
+        int col = n0 + c0;
+        const int live = a.N - col;
+        long long at = a.colmajor ? (long long)col * a.ldc + row : (long long)row * a.ldc + col;
+        if (tiled) {
+            const int pix = col / a.g.kt, gy = pix / a.g.gw, gx = pix - gy * a.g.gw;
+            col -= pix * a.g.kt;
+            if (tile_p + gy >= a.g.out_p || tile_q + gx >= a.g.out_q) return;
+            at = (long long)col * a.ldc + tile_at + ((long long)gy * a.g.out_q + gx) * a.g.N;
+        }
         const long long dc = a.colmajor ? a.ldc : 1;
         if (MODE == MODE_FLEX16) {
             int q[8];
@@ -623,6 +665,8 @@ DirectShape direct_shape(const b2_direct_args& a) {
     // fp32: 16 k-blocks to a chain; flex16: exact int32 sums up to 32768 columns
     const int most = MODE == MODE_FLEX16 ? 256 : 16;
     DirectShape best = {0, 0, 0, -1};
+    // SMs that clusters of 1..8 CTAs of this shared memory fill (what cudaOccupancyMaxActiveClusters says)
+    static const int fit[9] = {0, 148, 148, 135, 132, 130, 132, 119, 120};
     const long long tm = (a.M + 127) / 128;
     for (int bn = 16; bn <= 128; bn *= 2) {
         if (bn > 16 && bn / 2 >= a.N) break;
@@ -630,18 +674,24 @@ DirectShape direct_shape(const b2_direct_args& a) {
         for (int want = 1; want <= 8 && want <= num_kb; ++want) {
             const int per = (num_kb + want - 1) / want, splits = (num_kb + per - 1) / per;
             if (splits != want || per > most) continue;
-            if (a.a_kind == B2_OPERAND_GATHER && 1152 + dir_ring_bytes(bn) + per * KB * 8 > 232448) continue;
+            const int tab = a.a_kind == B2_OPERAND_GATHER ? per * KB * (filter_tiles(a) ? 16 : 8) : 0;
+            if (1152 + dir_ring_bytes(bn) + tab > 232448) continue;
             // Measured on one B200 (cycles at 1.9 GHz): the producers set the pace, 7 (fp32) or 22
             // (flex16) cycles an operand row of a k-block when they keep an SM busy, and a k-block
-            // takes 1000 + 6 bn or 4000 cycles from load to commit when they do not; the two CTAs of
-            // an SM overlap.  Gathered rows cost their address and bounds.
+            // takes 1000 + 6 bn (gathered 2000 to 3500) or 4000 cycles from load to commit when they do
+            // not; the two CTAs of an SM overlap.  Gathered rows cost their address and bounds, filters as a tile's pixels see
+            // them the same, more where the lanes' rows lie apart; slices of their wide tiles 15000 more.
             const double ra = a.a_kind == B2_OPERAND_GATHER ? 1.5 : 1.0;
-            const long long pace = (long long)((128 * ra + bn) * (MODE == MODE_FLEX16 ? (bn == 128 ? 33 : 22) : 7));
-            const long long lat = MODE == MODE_FLEX16 ? 4000 : 1000 + 6 * bn;
-            const long long ctas = tiles * splits, slots = 148LL * (bn == 128 ? 1 : 2);
-            const long long together = ctas <= 148 || bn == 128 ? 1 : 2;
+            const double rb = !filter_tiles(a) ? 1.0 : a.g.channel_last ? 3.5 : 1.5;
+            const long long pace = (long long)((128 * ra + bn * rb) * (MODE == MODE_FLEX16 ? (bn == 128 ? 33 : 22) : 7));
+            const long long lat = MODE == MODE_FLEX16 ? 4000 : a.a_kind != B2_OPERAND_GATHER ? 1000 + 6 * bn
+                                  : bn >= 64 ? 3500 : 1600 + 25 * bn;
+            const long long ctas = tiles * splits, per_sm = bn == 128 || 1152 + dir_ring_bytes(bn) + tab > 115000 ? 1 : 2;
+            const long long slots = (long long)fit[splits] * per_sm;
+            const long long together = ctas <= 148 ? 1 : per_sm;
             const long long kb = together * pace > lat ? together * pace : lat;
-            const long long one = 7000 + per * kb + together * bn * (splits > 1 ? 24 : 12) + (splits > 1 ? 3000 : 0);
+            const long long one = 7000 + per * kb + together * bn * (splits > 1 ? 24 : 12) +
+                                  (splits == 1 ? 0 : filter_tiles(a) ? 18000 : 3000);
             const long long cost = (ctas + slots - 1) / slots * one;
             if (best.cost < 0 || cost < best.cost) best = {bn, splits, per, cost};
         }
@@ -656,11 +706,12 @@ int direct_launch_as(const DirectParams& p, cudaStream_t st) {
     const int red = p.splits > 1 ? BN * 128 * (MODE == MODE_FLEX16 ? 8 : 4) : 0;
     static_assert(dir_ring_bytes(BN) >= BN * 128 * 8, "the slices' sums are exchanged through the ring");
     (void)red;
-    const int smem = 1024 + ring + 128 + (AK == B2_OPERAND_GATHER ? p.kb_per_split * KB * 8 : 0);
+    const int smem = 1024 + ring + 128 +
+                     (AK == B2_OPERAND_GATHER ? p.kb_per_split * KB * (filter_tiles(p.a) ? 16 : 8) : 0);
     static bool attr_set = false;
     if (!attr_set) {
         B2_CUDA(cudaFuncSetAttribute(direct_kernel<MODE, BN, AK>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     1024 + ring + 128 + (AK == B2_OPERAND_GATHER ? kDirMaxK * 8 < 232448 - 1152 - ring ? kDirMaxK * 8 : 232448 - 1152 - ring : 0)));
+                                     AK == B2_OPERAND_GATHER ? 232448 : 1024 + ring + 128));
         attr_set = true;
     }
     cudaLaunchConfig_t cfg = {};
@@ -704,7 +755,7 @@ int direct_launch_mode(const b2_direct_args& a, cudaStream_t st) {
         return ((uintptr_t)x & 3) == 0 && a.g.N % 2 == 0;         // pairs of images of one pixel
     };
     p.a_vec = aligned(a.a_kind, a.A, a.a_rs, a.a_ks);
-    p.b_vec = aligned(a.b_kind, a.B, a.b_rs, a.b_ks);
+    p.b_vec = a.b_kind != B2_OPERAND_FILTER && aligned(a.b_kind, a.B, a.b_rs, a.b_ks);
     switch (s.bn) {
         case 16: return direct_launch_bn<MODE, 16>(p, st);
         case 32: return direct_launch_bn<MODE, 32>(p, st);

@@ -4,16 +4,23 @@
 #define B2_DIRECT_H
 #include "b2_common.h"
 
-// how an operand lies: K contiguous; rows contiguous; rows gathered from a C,H,W,N tensor
-enum { B2_OPERAND_K = 0, B2_OPERAND_ROWS = 1, B2_OPERAND_GATHER = 2 };
+// how an operand lies: K contiguous; rows contiguous; rows gathered from a C,H,W,N tensor; rows of
+// filters as the pixels of a tile see them
+enum { B2_OPERAND_K = 0, B2_OPERAND_ROWS = 1, B2_OPERAND_GATHER = 2, B2_OPERAND_FILTER = 3 };
 
-// Rows (p, q, n) of a convolution's unrolled input, or (h, w, n) of its error tensor: the value of
-// column k is x[base(row) + offset(k)] where tap(k) lies inside for that row, else zero.
+// Rows (tile, n) of a convolution: a tile is gh x gw pixels of the result and sees a window of R x S taps
+// of the tensor read, tap (th, tw) at (tile_p * step_h + off_h + th * tap_h, ...).  Columns (channel,
+// th, tw), or (th, tw, channel): the value there, or zero outside the tensor.
 struct b2_gather {
     int channels, H, W, N;           // the tensor read
-    int P, Q;                        // rows: pixel (p, q) of N images
-    int R, S, pad_h, pad_w, str_h, str_w, dil_h, dil_w;
-    int bprop;                       // columns (r, s, channel) of an input gradient, else (channel, r, s)
+    int P, Q;                        // tiles
+    int R, S, off_h, off_w, step_h, step_w, tap_h, tap_w;
+    int channel_last;                // order of the columns
+    // tiles of several pixels: column g * kt + k of the result is channel k of pixel g (kt a multiple of
+    // 8), the result is [kt][out_p][out_q][N]; its filter row has at tap (th, tw) the filter's tap
+    // r = f0_h + f1_h * th + f2_h * gy (s likewise) where that lies inside fr x fs, else zero.
+    int gh, gw, kt, out_p, out_q;
+    int fr, fs, f0_h, f0_w, f1_h, f1_w, f2_h, f2_w;
 };
 
 struct b2_direct_args {

@@ -14,7 +14,10 @@ pytestmark = pytest.mark.gpu
 CASES = [(3, 9, 7, 5, 17, 3, 3, 1, 1, 1, 1), (16, 8, 8, 100, 16, 3, 3, 1, 1, 1, 1),
          (5, 8, 9, 33, 40, 5, 5, 2, 2, 1, 1), (130, 5, 5, 20, 130, 3, 3, 2, 1, 2, 1),
          (2, 3, 40, 130, 9, 1, 31, 0, 1, 1, 1), (2, 3, 40, 130, 9, 1, 32, 0, 1, 1, 3),
-         (64, 8, 8, 1, 64, 3, 3, 1, 1, 1, 1), (20, 33, 31, 40, 70, 3, 2, 1, 1, 1, 1), (33, 6, 6, 64, 32, 1, 1, 0, 2, 1, 1)]
+         (64, 8, 8, 1, 64, 3, 3, 1, 1, 1, 1), (20, 33, 31, 40, 70, 3, 2, 1, 1, 1, 1), (33, 6, 6, 64, 32, 1, 1, 0, 2, 1, 1),
+         # tiles of several pixels with ragged edges: forward, both passes, a strided gradient
+         (3, 31, 33, 100, 16, 3, 3, 1, 1, 1, 1), (16, 31, 33, 250, 16, 3, 3, 1, 1, 1, 1),
+         (16, 31, 33, 100, 32, 3, 3, 1, 2, 1, 1)]
 
 
 @pytest.mark.parametrize("case", CASES)
