@@ -51,7 +51,9 @@ int b2_device_count(void);
 /* B2_FLEX16_PLANES (elementwise results only): the int16 mantissa is stored as two byte planes,
  * high bytes at the destination pointer and low bytes plane_bytes further -- the operand format
  * of the convolution entry points that take planes, so no separate split pass is needed. */
-enum b2_dtype { B2_F32 = 0, B2_FLEX16 = 1, B2_FLEX16_PLANES = 2 };
+/* B2_F32_AT (inputs only): the pointer given at launch is the address of a device word that holds the
+ * address of the values when the kernel runs, 16-byte aligned. */
+enum b2_dtype { B2_F32 = 0, B2_FLEX16 = 1, B2_FLEX16_PLANES = 2, B2_F32_AT = 3 };
 
 /* op codes: one per template of float_ew2.py:31-68 */
 enum b2_ew_opcode {
@@ -138,6 +140,18 @@ int b2_ew_scratch_bytes(const b2_ew_kernel* k, size_t* bytes);
 int b2_ew_launch(b2_ew_kernel* k, const void* const* in, void* const* out, const float* consts,
                  const b2_flex_scale* flex_table, int32_t* flex_stats, void* scratch,
                  size_t scratch_bytes, int32_t* status, int probe, void* stream);
+/* Programs of one and the same non-empty b2_ew_joint_source (no reductions, one row) in as few launches
+ * as their arguments take (one with pointers that are not 16-byte aligned goes by itself). */
+typedef struct b2_ew_launch_job {
+    b2_ew_kernel* kernel;
+    const void* const* in;
+    void* const* out;
+    const float* consts;
+} b2_ew_launch_job;
+int b2_ew_joint_source(const b2_ew_kernel* k, const char** source);
+int b2_ew_joint_prepare(b2_ew_kernel* first);   /* compiles what b2_ew_launch_many launches */
+int b2_ew_launch_many(const b2_ew_launch_job* jobs, int32_t n, const b2_flex_scale* flex_table,
+                      int32_t* flex_stats, int32_t* status, int32_t* launches, void* stream);
 /* The same launch for callers that cannot allocate (no counterpart in the reference, which
  * always allocates through pycuda).  Meant for hosts that gave the whole device to their own
  * arena at start-up, and for execution loops that must never reach cudaMalloc because it
@@ -190,6 +204,8 @@ int b2_flex_publish(int32_t* stats, int32_t n, const int32_t* status, int32_t* h
  * block lies in pinned host memory that the device can address and is read when the kernel runs, so
  * one recorded launch serves every call; so may be the arguments.  table_rows > 0 copies that many
  * rows of the block's scale table to `table` first.
+ * where, unless NULL: a device word that gets the address at which the values are to be read -- src for
+ * an argument marked in_place, which is then not copied (its reader does that: B2_F32_AT), else dst.
  * b2_call_outputs is b2_flex_publish with results: dst[k] (pinned host memory) <- bytes[k] bytes of
  * src[k], both 16-byte aligned.
  * b2_call_stage: the address at which the device can read `bytes` bytes of host memory at src:
@@ -199,12 +215,12 @@ int b2_flex_publish(int32_t* stats, int32_t n, const int32_t* status, int32_t* h
  * ------------------------------------------------------------------------------------------ */
 #define B2_CALL_MAX_INPUTS 16
 #define B2_CALL_MAX_OUTPUTS 16
-typedef struct b2_call_arg { const void* src; float inv_scale; int32_t reserved; } b2_call_arg;
+typedef struct b2_call_arg { const void* src; float inv_scale; int32_t in_place; } b2_call_arg;
 typedef struct b2_call_block {
     const b2_flex_scale* table; int32_t table_rows; int32_t reserved;
     b2_call_arg arg[B2_CALL_MAX_INPUTS];
 } b2_call_block;
-typedef struct b2_call_input { void* dst; int64_t n; int32_t flex_slot; int32_t reserved; } b2_call_input;
+typedef struct b2_call_input { void* dst; int64_t n; int32_t flex_slot; int32_t reserved; const void** where; } b2_call_input;
 typedef struct b2_call_output { const void* src; void* dst; int64_t bytes; } b2_call_output;
 int b2_call_inputs(const b2_call_input* inputs, int32_t n, const b2_call_block* block,
                    b2_flex_scale* table, int32_t* stats, void* stream);

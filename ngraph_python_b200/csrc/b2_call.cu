@@ -52,7 +52,11 @@ k_call_inputs(const Inputs a, const b2_call_block* __restrict__ blk, b2_flex_sca
     __shared__ const float* src_s[B2_CALL_MAX_INPUTS];
     __shared__ float inv_s[B2_CALL_MAX_INPUTS];
     if (threadIdx.x < a.n) {
-        src_s[threadIdx.x] = (const float*)blk->arg[threadIdx.x].src;
+        const float* src = (const float*)blk->arg[threadIdx.x].src;
+        const bool in_place = src && blk->arg[threadIdx.x].in_place && a.in[threadIdx.x].where;
+        src_s[threadIdx.x] = in_place ? nullptr : src;
+        if (blockIdx.x == 0 && a.in[threadIdx.x].where)
+            *a.in[threadIdx.x].where = in_place ? (const void*)src : a.in[threadIdx.x].dst;
         inv_s[threadIdx.x] = blk->arg[threadIdx.x].inv_scale;
     }
     // the scale table, when a row of it has changed

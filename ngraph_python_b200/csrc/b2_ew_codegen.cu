@@ -146,6 +146,10 @@ int compile_source(const std::string& src, bool has_finalize, Module** out) {
     return B2_OK;
 }
 
+const int kManyMost = 32;            // programs of one launch: 26 KB of arguments
+struct EwJobs { int n, first[kManyMost + 1]; EwArgs job[kManyMost]; };
+static_assert(sizeof(EwJobs) <= 32764, "the arguments of a kernel");
+
 // ---- code generation ------------------------------------------------------------------------
 const int kThreads = 256;
 const int kSMs = 148;
@@ -397,8 +401,17 @@ void emit_finalize(std::ostringstream& o, const b2_ew_program& p, bool probe) {
         o << "}\n";
     }
 
+// where input i lies: the pointer given, or (B2_F32_AT) what the word it points to holds by now, read once
+std::string input_pointer(const b2_ew_program& p, int i) {
+    std::ostringstream o;
+    if (p.in[i].dtype == B2_F32_AT) o << "at" << i;
+    else o << "(const " << ctype(p.in[i].dtype) << "*)p.in[" << i << "]";
+    return o.str();
+}
+
+// many: the kernel of b2_ew_launch_many, whose blocks find their program's arguments first
 int generate(const b2_ew_program& p, const Plan& pl, bool probe, std::string* out_src,
-             bool* has_finalize) {
+             bool* has_finalize, bool many = false) {
     std::ostringstream o;
     const int nres = p.n_out + p.n_red;
     const bool split = pl.nsplit > 1;
@@ -406,13 +419,26 @@ int generate(const b2_ew_program& p, const Plan& pl, bool probe, std::string* ou
     o << kDeviceHeader << "\n";
     o << "#define V " << pl.V << "\n#define THREADS " << kThreads << "\n#define GROUP "
       << pl.group << "\n#define NRED " << (p.n_red > 0 ? p.n_red : 1) << "\n";
-    o << "extern \"C\" __global__ void __launch_bounds__(THREADS, " << pl.minb << ") b2_ew_main(const b2_ew_args p) {\n";
+    if (many)
+        o << "struct b2_ew_jobs { int n, first[" << kManyMost + 1 << "]; b2_ew_args job[" << kManyMost << "]; };\n"
+          << "extern \"C\" __global__ void __launch_bounds__(THREADS, " << pl.minb
+          << ") b2_ew_main(const __grid_constant__ b2_ew_jobs jobs) {\n";
+    else
+        o << "extern \"C\" __global__ void __launch_bounds__(THREADS, " << pl.minb << ") b2_ew_main(const b2_ew_args p) {\n";
     o << "    __shared__ float smem[64];\n";
     // programmatic dependent launch: nothing above this line touches global memory; the next
     // kernel of the stream may be scheduled while this grid drains
     o << "    asm volatile(\"griddepcontrol.wait;\" ::: \"memory\");\n"
       << "    asm volatile(\"griddepcontrol.launch_dependents;\" ::: \"memory\");\n";
+    if (many)
+        o << "    int at_job = 0;\n"
+          << "    while (at_job + 1 < jobs.n && (int)blockIdx.x >= jobs.first[at_job + 1]) ++at_job;\n"
+          << "    const b2_ew_args& p = jobs.job[at_job];\n"
+          << "    const int first_block = jobs.first[at_job], end_block = jobs.first[at_job + 1];\n";
     emit_prologue(o, p, probe);
+    for (int i = 0; i < p.n_in; ++i)
+        if (p.in[i].dtype == B2_F32_AT)
+            o << "    const float* const at" << i << " = *(const float* const volatile*)p.in[" << i << "];\n";
 
     if (p.reduce_mode != B2_REDUCE_B) {
         o << "    const b2_i64 rows = p.A * p.B;\n"
@@ -423,8 +449,8 @@ int generate(const b2_ew_program& p, const Plan& pl, bool probe, std::string* ou
           << "        const b2_i64 a_idx = r / p.B, b_idx = r - a_idx * p.B;\n";
         for (int i = 0; i < p.n_in; ++i) {
             const char* ct = ctype(p.in[i].dtype);
-            o << "        const " << ct << "* in" << i << " = (const " << ct << "*)p.in[" << i
-              << "] + a_idx * p.in_sa[" << i << "] + b_idx * p.in_sb[" << i << "];\n";
+            o << "        const " << ct << "* in" << i << " = " << input_pointer(p, i)
+              << " + a_idx * p.in_sa[" << i << "] + b_idx * p.in_sb[" << i << "];\n";
             if (p.in[i].sc == 0) {
                 o << "        const float xb" << i << " = ";
                 if (p.in[i].dtype == B2_FLEX16) o << "s" << i << " * (float)";
@@ -541,8 +567,8 @@ int generate(const b2_ew_program& p, const Plan& pl, bool probe, std::string* ou
         o << "        for (b2_i64 b_idx = 0; b_idx < p.B; ++b_idx) {\n";
         for (int i = 0; i < p.n_in; ++i) {
             const char* ct = ctype(p.in[i].dtype);
-            o << "            const " << ct << "* in" << i << " = (const " << ct << "*)p.in[" << i
-              << "] + a_idx * p.in_sa[" << i << "] + b_idx * p.in_sb[" << i << "];\n";
+            o << "            const " << ct << "* in" << i << " = " << input_pointer(p, i)
+              << " + a_idx * p.in_sa[" << i << "] + b_idx * p.in_sb[" << i << "];\n";
             if (p.in[i].sc == 0) {
                 o << "            const float xb" << i << " = ";
                 if (p.in[i].dtype == B2_FLEX16) o << "s" << i << " * (float)";
@@ -606,6 +632,18 @@ int generate(const b2_ew_program& p, const Plan& pl, bool probe, std::string* ou
 
     if (split) emit_finalize(o, p, probe);
     *out_src = o.str();
+    if (many) {
+        // one row to a program: its blocks lie along x
+        auto put = [&](const char* what, const char* with) {
+            const size_t from = out_src->find("const b2_ew_args& p = jobs");
+            for (size_t i = from; (i = out_src->find(what, i)) != std::string::npos; i += strlen(with))
+                out_src->replace(i, strlen(what), with);
+        };
+        put("(b2_i64)blockIdx.x", "(b2_i64)((int)blockIdx.x - first_block)");
+        put("(b2_i64)gridDim.x", "(b2_i64)(end_block - first_block)");
+        put("(b2_i64)blockIdx.y", "(b2_i64)0");
+        put("(b2_i64)gridDim.y", "(b2_i64)1");
+    }
     return B2_OK;
 }
 
@@ -870,7 +908,9 @@ Plan make_plan(const b2_ew_program& p, bool want_vec) {
     // staged variant: full-size inputs go global -> shared by bulk async copies
     const char* env = getenv("B2_EW_STAGED");
     const bool allow = env && env[0] == '1';   // off by default: measured slower than plain loads
-    if (allow && pl.vec && p.reduce_mode != B2_REDUCE_B && pl.group == kThreads &&
+    bool at = false;
+    for (int i = 0; i < p.n_in; ++i) at |= p.in[i].dtype == B2_F32_AT;
+    if (allow && !at && pl.vec && p.reduce_mode != B2_REDUCE_B && pl.group == kThreads &&
         rows < (1LL << 30) && chunks < (1LL << 30)) {
         int bytes = 0;
         for (int i = 0; i < p.n_in; ++i)
@@ -909,6 +949,7 @@ struct b2_ew_kernel {
     b2_ew_program prog;
     // [vec?][probe?]
     Module* mod[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};
+    Module* many = nullptr;      // of its joint launches
     Plan plan[2];
     std::string src[2][2];
     bool can_vec = false;
@@ -947,7 +988,8 @@ int validate(const b2_ew_program& p) {
             B2_REQUIRE(p.out[k].redop >= B2_RED_SUM && p.out[k].redop <= B2_RED_ARGMIN, "bad redop");
     }
     for (int i = 0; i < p.n_in; ++i) {
-        B2_REQUIRE(p.in[i].dtype == B2_F32 || p.in[i].dtype == B2_FLEX16, "bad input dtype");
+        B2_REQUIRE(p.in[i].dtype == B2_F32 || p.in[i].dtype == B2_FLEX16 || p.in[i].dtype == B2_F32_AT,
+                   "bad input dtype");
         if (p.in[i].dtype == B2_FLEX16)
             B2_REQUIRE(p.in[i].flex_slot >= 0, "flex input %d has no slot", i);
     }
@@ -1078,7 +1120,7 @@ int check_launch(const b2_ew_kernel* k, const void* const* in, void* const* out,
     for (int i = 0; i < p.n_in; ++i) {
         B2_REQUIRE(in[i], "input %d is null", i);
         any_flex |= p.in[i].dtype == B2_FLEX16;
-        if (vec && p.in[i].sc == 1 && !aligned16(in[i])) vec = 0;
+        if (vec && p.in[i].sc == 1 && p.in[i].dtype != B2_F32_AT && !aligned16(in[i])) vec = 0;
     }
     for (int q = 0; q < nres; ++q) {
         B2_REQUIRE(out[q], "result %d is null", q);
@@ -1098,14 +1140,10 @@ size_t scratch_need(const b2_ew_kernel* k, int vec) {
         ? (size_t)pl.nsplit * (size_t)(p.A * p.B) * (size_t)p.n_red * sizeof(float) : 0;
 }
 
-int launch_variant(const b2_ew_kernel* k, int vec, const Module* m, const void* const* in,
-                   void* const* out, const float* consts, const b2_flex_scale* flex_table,
-                   int32_t* flex_stats, void* scratch, int32_t* status, unsigned fresh_mask,
-                   void* stream) {
-    const b2_ew_program& p = k->prog;
-    const Plan& pl = k->plan[vec];
+void fill_args(const b2_ew_program& p, const void* const* in, void* const* out, const float* consts,
+               const b2_flex_scale* flex_table, int32_t* flex_stats, int32_t* status, EwArgs* args) {
     const int nres = p.n_out + p.n_red;
-    EwArgs a;
+    EwArgs& a = *args;
     memset(&a, 0, sizeof(a));
     a.A = p.A; a.B = p.B; a.C = p.C;
     for (int i = 0; i < p.n_in; ++i) {
@@ -1122,8 +1160,18 @@ int launch_variant(const b2_ew_kernel* k, int vec, const Module* m, const void* 
     for (int i = 0; i < p.n_const; ++i) a.consts[i] = consts[i];
     a.flex_table = flex_table;
     a.flex_stats = flex_stats;
-    a.scratch = static_cast<float*>(scratch);
     a.status = status;
+}
+
+int launch_variant(const b2_ew_kernel* k, int vec, const Module* m, const void* const* in,
+                   void* const* out, const float* consts, const b2_flex_scale* flex_table,
+                   int32_t* flex_stats, void* scratch, int32_t* status, unsigned fresh_mask,
+                   void* stream) {
+    const b2_ew_program& p = k->prog;
+    const Plan& pl = k->plan[vec];
+    EwArgs a;
+    fill_args(p, in, out, consts, flex_table, flex_stats, status, &a);
+    a.scratch = static_cast<float*>(scratch);
     a.nsplit = pl.nsplit;
     a.fresh_mask = fresh_mask;
     void* params[] = {&a};
@@ -1155,6 +1203,75 @@ extern "C" int b2_ew_launch(b2_ew_kernel* k, const void* const* in, void* const*
                "split reduction needs %zu bytes of scratch, got %zu", need, scratch_bytes);
     return launch_variant(k, vec, k->mod[vec][probe], in, out, consts, flex_table, flex_stats,
                           scratch, status, fresh_mask, stream);
+}
+
+// ------------------------------------------------------------------------------------------------
+// Several programs of one source in one launch: the optimizer's updates of a network's tensors, each a
+// kernel of 2 us that a few blocks would do.
+// ------------------------------------------------------------------------------------------------
+namespace {
+bool goes_with_others(const b2_ew_kernel* k, int vec) {
+    const b2_ew_program& p = k->prog;
+    return p.reduce_mode == B2_REDUCE_NONE && p.A * p.B == 1 && !k->plan[vec].staged &&
+           k->plan[vec].grid.x <= 4 * kSMs;       // (larger ones fill the machine by themselves)
+}
+}  // namespace
+
+extern "C" int b2_ew_joint_source(const b2_ew_kernel* k, const char** source) {
+    B2_REQUIRE(k && source, "null argument");
+    const int vec = k->can_vec ? 1 : 0;
+    *source = goes_with_others(k, vec) ? k->src[vec][0].c_str() : "";
+    return B2_OK;
+}
+
+extern "C" int b2_ew_joint_prepare(b2_ew_kernel* first) {
+    B2_REQUIRE(first, "null argument");
+    if (first->many) return B2_OK;
+    const int vec = first->can_vec ? 1 : 0;
+    B2_REQUIRE(goes_with_others(first, vec), "this program is launched by itself");
+    std::string src;
+    bool has_final = false;
+    int rc = generate(first->prog, first->plan[vec], false, &src, &has_final, true);
+    return rc ? rc : compile_source(src, false, &first->many);
+}
+
+extern "C" int b2_ew_launch_many(const b2_ew_launch_job* list, int32_t n, const b2_flex_scale* flex_table,
+                                 int32_t* flex_stats, int32_t* status, int32_t* launches, void* stream) {
+    B2_REQUIRE(list && n > 0 && launches, "bad argument");
+    b2_ew_kernel* head = list[0].kernel;
+    int rc = b2_ew_joint_prepare(head);
+    if (rc) return rc;
+    const int vec = head->can_vec ? 1 : 0;
+    const Module* m = head->many;
+    *launches = 0;
+    static thread_local EwJobs jobs;
+    for (int i0 = 0; i0 < n; i0 += kManyMost) {
+        jobs.n = 0;
+        jobs.first[0] = 0;
+        for (int i = i0; i < n && i < i0 + kManyMost; ++i) {
+            const b2_ew_launch_job& j = list[i];
+            int v = 0;
+            if ((rc = check_launch(j.kernel, j.in, j.out, j.consts, flex_table, flex_stats, &v))) return rc;
+            if (v != vec) {                       // pointers that are not aligned: by itself
+                if ((rc = ensure_variant(j.kernel, v, 0))) return rc;
+                if ((rc = launch_variant(j.kernel, v, j.kernel->mod[v][0], j.in, j.out, j.consts, flex_table,
+                                         flex_stats, nullptr, status, 0u, stream))) return rc;
+                ++*launches;
+                continue;
+            }
+            B2_REQUIRE(j.kernel->src[v][0] == head->src[vec][0], "programs of different sources");
+            fill_args(j.kernel->prog, j.in, j.out, j.consts, flex_table, flex_stats, status, &jobs.job[jobs.n]);
+            jobs.job[jobs.n].nsplit = 1;
+            jobs.first[jobs.n + 1] = jobs.first[jobs.n] + (int)j.kernel->plan[v].grid.x;
+            ++jobs.n;
+        }
+        if (jobs.n == 0) continue;
+        void* params[] = {&jobs};
+        B2_CUDA(launch_main((const void*)m->main, dim3((unsigned)jobs.first[jobs.n]), params, 0,
+                            static_cast<cudaStream_t>(stream)));
+        ++*launches;
+    }
+    return B2_OK;
 }
 
 // ------------------------------------------------------------------------------------------------

@@ -10,7 +10,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(HERE, "libb200ng.so")
 
 EW_MAX_IN, EW_MAX_OUT, EW_MAX_CONST, EW_MAX_OPS = 12, 6, 16, 96
-F32, FLEX16, FLEX16_PLANES = 0, 1, 2
+F32, FLEX16, FLEX16_PLANES, F32_AT = 0, 1, 2, 3
 REDUCE_NONE, REDUCE_C, REDUCE_B = 0, 1, 2
 
 OPCODES = {
@@ -32,6 +32,11 @@ class EwTensor(C.Structure):
     _fields_ = [("dtype", C.c_int32), ("flex_slot", C.c_int32),
                 ("sa", C.c_int64), ("sb", C.c_int64), ("sc", C.c_int64),
                 ("plane_bytes", C.c_int64)]
+
+
+class EwLaunchJob(C.Structure):
+    _fields_ = [("kernel", C.c_void_p), ("inputs", C.c_void_p), ("results", C.c_void_p),
+                ("consts", C.c_void_p)]
 
 
 class EwOp(C.Structure):
@@ -77,7 +82,7 @@ CALL_MAX_INPUTS, CALL_MAX_OUTPUTS = 16, 16
 
 
 class CallArg(C.Structure):
-    _fields_ = [("src", C.c_void_p), ("inv_scale", C.c_float), ("reserved", C.c_int32)]
+    _fields_ = [("src", C.c_void_p), ("inv_scale", C.c_float), ("in_place", C.c_int32)]
 
 
 class CallBlock(C.Structure):
@@ -87,7 +92,7 @@ class CallBlock(C.Structure):
 
 class CallInput(C.Structure):
     _fields_ = [("dst", C.c_void_p), ("n", C.c_int64), ("flex_slot", C.c_int32),
-                ("reserved", C.c_int32)]
+                ("reserved", C.c_int32), ("where", C.c_void_p)]
 
 
 class CallOutput(C.Structure):
@@ -117,6 +122,9 @@ def _load():
         "b2_ew_scratch_bytes": (C.c_int, [vp, C.POINTER(sz)]),
         "b2_ew_launch": (C.c_int, [vp, C.POINTER(vp), C.POINTER(vp), C.POINTER(C.c_float), vp, vp,
                                    vp, sz, vp, C.c_int, vp]),
+        "b2_ew_joint_source": (C.c_int, [vp, C.POINTER(C.c_char_p)]),
+        "b2_ew_joint_prepare": (C.c_int, [vp]),
+        "b2_ew_launch_many": (C.c_int, [C.POINTER(EwLaunchJob), i32, vp, vp, vp, C.POINTER(i32), vp]),
         "b2_ew_launch_builtin_scratch": (C.c_int, [vp, C.POINTER(vp), C.POINTER(vp),
                                                    C.POINTER(C.c_float), vp, vp, vp, C.c_int, vp]),
         "b2_ew_source": (C.c_char_p, [vp]),
@@ -278,6 +286,22 @@ def ew_check(prog, vec=True, probe=False, want_source=False):
     return buf.value.decode() if buf else None
 
 
+def launch_many(jobs, flex_table=0, flex_stats=0, status=0, stream=0):
+    """jobs: (EwKernel, input pointers, result pointers, constants) of one joint_source(); returns the
+    number of launches."""
+    arr, keep = (EwLaunchJob * len(jobs))(), []
+    for a, (kernel, in_ptrs, out_ptrs, consts) in zip(arr, jobs):
+        ins = (C.c_void_p * max(1, len(in_ptrs)))(*in_ptrs)
+        outs = (C.c_void_p * max(1, len(out_ptrs)))(*out_ptrs)
+        cs = (C.c_float * EW_MAX_CONST)(*consts)
+        keep.append((ins, outs, cs))
+        a.kernel, a.inputs, a.results, a.consts = kernel.handle, C.addressof(ins), C.addressof(outs), \
+            C.addressof(cs)
+    n = C.c_int32()
+    check(_lib.b2_ew_launch_many(arr, len(jobs), flex_table, flex_stats, status, C.byref(n), stream))
+    return n.value
+
+
 class EwKernel(object):
     """A compiled fused kernel."""
 
@@ -294,6 +318,15 @@ class EwKernel(object):
 
     def source(self):
         return _lib.b2_ew_source(self.handle).decode()
+
+    def prepare_joint(self):
+        check(_lib.b2_ew_joint_prepare(self.handle))
+
+    def joint_source(self):
+        """What kernels of one joint launch have in common; empty for one that is launched alone."""
+        s = C.c_char_p()
+        check(_lib.b2_ew_joint_source(self.handle, C.byref(s)))
+        return s.value
 
     def launch(self, in_ptrs, out_ptrs, consts=(), flex_table=0, flex_stats=0, scratch=0,
                scratch_bytes=0, status=0, probe=False, stream=0):
@@ -329,6 +362,9 @@ class PlannedKernel(object):
 
     def source(self):
         return self._source
+
+    def joint_source(self):
+        return b""
 
 
 def gemm_scratch_bytes(flex, M, N, K):

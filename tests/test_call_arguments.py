@@ -1,0 +1,46 @@
+"""Large fp32 arguments of recorded calls: read where the caller's tensor lies by the kernel that uses
+them first, which stores them; later kernels, later calls with other kinds of arguments, unrecorded calls
+and the placeholder itself see the values of the last call."""
+import numpy as np
+import pytest
+
+import ngraph_python_b200 as ng
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("rows, cols", [(512, 512), (300, 1001), (1, 262144), (64, 4096)])
+def test_device_arguments_in_place(rows, cols):
+    import torch
+    A, B = ng.make_axis(rows, name="A"), ng.make_axis(cols, name="B")
+    x = ng.placeholder([A, B])
+    total = ng.sum(ng.exp(x) + x, reduction_axes=[B])
+    again = ng.sum(x, reduction_axes=[A])                    # another kernel reads x after it
+    t = ng.transformers.allocate_transformer("b200")
+    comp = t.computation([total, again], x)
+    other = t.computation(ng.sum(x * x, reduction_axes=[B]), x)
+    third = t.computation(ng.max(x, reduction_axes=[B]), x)
+
+    def check(value):
+        v = value.cpu().numpy() if isinstance(value, torch.Tensor) else value
+        v = v.astype(np.float64)
+        got = comp(value)
+        np.testing.assert_allclose(got[0], (np.exp(v) + v).sum(axis=1), rtol=2e-5, atol=1e-3)
+        np.testing.assert_allclose(got[1], v.sum(axis=0), rtol=2e-5, atol=1e-3)
+        np.testing.assert_array_equal(np.asarray(t.get_tensor_view_value(x)), v.astype(np.float32))
+        np.testing.assert_allclose(other(value), (v * v).sum(axis=1), rtol=2e-5, atol=1e-3)
+
+    def values(seed, extra=0):
+        g = torch.Generator(device="cuda").manual_seed(seed)
+        flat = torch.rand((rows * cols + extra,), device="cuda", generator=g)
+        return flat[extra:].reshape(rows, cols)
+    check(values(1))                                          # before recording
+    comp.capture(), other.capture()
+    check(values(2))
+    check(values(3, extra=1))                                 # not 16-byte aligned
+    check(np.random.RandomState(4).rand(rows, cols).astype(np.float32))
+    check(values(5).double())                                 # converted on the way
+    v = values(6)                                             # unrecorded, after recorded calls
+    np.testing.assert_array_equal(third(v), v.cpu().numpy().max(axis=1))
+    check(values(7))
+    t.close()
