@@ -23,7 +23,11 @@
 
 namespace {
 
-constexpr int kPairThreads = 320;
+// Epilogue warps.  flex16 fills tensor memory (HH | X1 | X2 | LL), so that a tile's epilogue holds up the
+// next tile's products: sixteen warps take half the time of eight.  fp32 overlaps the two, and its
+// sums want the registers.
+__host__ __device__ constexpr int pair_epi_warps(int mode) { return mode == MODE_FLEX16 ? 16 : 8; }
+__host__ __device__ constexpr int pair_threads(int mode) { return 64 + 32 * pair_epi_warps(mode); }
 constexpr int kPairStage = 48 * 1024;
 constexpr int kPairStages = 4;
 constexpr int kPairSmem = 1024 + kPairStages * kPairStage + 256;
@@ -102,7 +106,7 @@ __device__ __forceinline__ void pair_tile(const PairParams& p, int t, int& m, in
 }
 
 template <int MODE>
-__global__ void __launch_bounds__(kPairThreads, 1)
+__global__ void __launch_bounds__(pair_threads(MODE), 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constant__ CUtensorMap mapA1,
                  const __grid_constant__ CUtensorMap mapB0, const __grid_constant__ CUtensorMap mapB1,
                  const PairParams p) {
@@ -128,7 +132,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constan
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < kPairStages; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
-        for (int b = 0; b < 2; ++b) { mbar_init(&tmem_full[b], 1); mbar_init(&tmem_empty[b], 16); }
+        for (int b = 0; b < 2; ++b) { mbar_init(&tmem_full[b], 1); mbar_init(&tmem_empty[b], 2 * pair_epi_warps(MODE)); }
         *fail_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -228,10 +232,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constan
             }
         }
     } else {
-        // epilogue: lane quarter = warp % 4, columns of the two halves
+        // epilogue: lane quarter = warp % 4, a share of the columns each
         typedef typename std::conditional<MODE == MODE_FLEX16, long long, float>::type Sum;
         Sum* red = (Sum*)smem;                                    // [128 columns][128 rows], slices only
-        const int quarter = warp & 3, c_lo = ((warp - 2) >> 2) * 64;
+        constexpr int kGroups = pair_epi_warps(MODE) / 4, kCols = 128 / kGroups;
+        const int quarter = warp & 3, c_lo = ((warp - 2) >> 2) * kCols;
         const int lrow = quarter * 32 + lane;
         const unsigned lane_addr = tmem_base + ((unsigned)(quarter * 32) << 16);
         const unsigned empty0 = map_rank(&tmem_empty[0], leader), empty1 = map_rank(&tmem_empty[1], leader);
@@ -293,7 +298,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constan
                 if (ok && !mbar_wait(&tmem_full[0], chunk & 1)) { atomicExch(fail_flag, 1); ok = false; }
                 ++chunk;
                 tc_fence_after();
-                for (int c0 = c_lo; c0 < c_lo + 64; c0 += 8) {
+                for (int c0 = c_lo; c0 < c_lo + kCols; c0 += 8) {
                     unsigned hh[8], x1[8], x2[8], ll[8];
                     tmem_ld8(lane_addr + c0, hh);
                     tmem_ld8(lane_addr + 128 + c0, x1);
@@ -356,7 +361,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constan
             pair_tile(p, first, tm, tn);
             const int row = tm * 256 + side * 128 + lrow, n0 = tn * 128;
             const long long fix = MODE == MODE_FLEX16 && row < g.M ? 128LL * (long long)g.rowsum[row] : 0LL;
-            for (int c0 = (slice + ((warp - 2) >> 2) * p.splits) * 8; c0 < 128; c0 += 16 * p.splits) {
+            for (int c0 = (slice + ((warp - 2) >> 2) * p.splits) * 8; c0 < 128; c0 += 8 * kGroups * p.splits) {
                 Sum v[8];
 #pragma unroll
                 for (int j = 0; j < 8; ++j) v[j] = 0;
@@ -429,7 +434,7 @@ int launch_pair(unsigned char* base, const Shapes& s, GemmParams g, cudaStream_t
     cudaLaunchConfig_t cfg = {};
     const int pairs = p.splits > 1 || p.tiles < 74 ? p.tiles : 74;
     cfg.gridDim = dim3(2 * pairs, 1, p.splits);
-    cfg.blockDim = dim3(kPairThreads);
+    cfg.blockDim = dim3(pair_threads(MODE));
     cfg.dynamicSmemBytes = kPairSmem;
     cfg.stream = st;
     cudaLaunchAttribute attr[2];
