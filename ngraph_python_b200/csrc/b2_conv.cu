@@ -6,7 +6,10 @@
 // (gpu/pool.py:27-220, gpu/kernels/cuda/pooling.py:291-438).
 //
 // fprop:  O[K,M,P,Q,N] = sum_{c,t,r,s} F[C,T,R,S,K] * I[C,D,H,W,N]
-// is run as one GEMM on the tensor cores, O^T[(p,q,n), k] = Icol[(p,q,n),(c,r,s)] * F[(c,r,s), k]:
+// is run as one GEMM on the tensor cores, O^T[(p,q,n), k] = Icol[(p,q,n),(c,r,s)] * F[(c,r,s), k].  flex16
+// takes the tile kernel below (byte planes, windows fetched by TMA), fp32 and dilated filters the product
+// that gathers its operands on the way in (b2_direct.cuh); what neither takes (depth, large windows)
+// goes through memory:
 //   * a gather pre-pass writes the rows of Icol (one row per output pixel and image, the filter
 //     window unrolled along K, zero where the window hangs over the border) directly as the two
 //     operand planes the GEMM kernel streams with TMA (int8 hi/lo for flex16, tf32 hi/lo for
@@ -20,7 +23,8 @@
 //
 // The two training contractions (ConvBpropKernel / ConvUpdateKernel, gpu/conv.py:121-312,
 // FlexConvBpropKernel / FlexConvUpdateKernel, gpu/flex_conv.py:203-621; readable specification
-// ngraph/transformers/cpu/cpuengine.py:256-271 and :395-418) run on the same tile kernel:
+// ngraph/transformers/cpu/cpuengine.py:256-271 and :395-418) have the same three ways; through
+// memory:
 //   bprop:  gI^T[(h,w,n), c] = Ecol[(h,w,n),(k,r,s)] * F[(c,r,s),k] read as [(k,r,s)][c], where the
 //           gather takes E[k,p,q,n] with p = (h + pad - r*dil) / str when that division is exact
 //           and p lies inside the output, zero otherwise (the transposed, flipped convolution);
