@@ -14,6 +14,7 @@
 // 8192 x 16384 values: copy to a staging tensor 173 us + conversion 167 us before, one pass of
 // 6 bytes a value now.
 #include <cmath>
+#include <cstddef>
 #include <cstring>
 #if defined(__x86_64__)
 #include <immintrin.h>
@@ -52,12 +53,14 @@ k_call_inputs(const Inputs a, const b2_call_block* __restrict__ blk, b2_flex_sca
     __shared__ const float* src_s[B2_CALL_MAX_INPUTS];
     __shared__ float inv_s[B2_CALL_MAX_INPUTS];
     if (threadIdx.x < a.n) {
-        const float* src = (const float*)blk->arg[threadIdx.x].src;
-        const bool in_place = src && blk->arg[threadIdx.x].in_place && a.in[threadIdx.x].where;
+        // one 16-byte read over PCIe to a block and argument
+        const uint4 e = *reinterpret_cast<const uint4*>(&blk->arg[threadIdx.x]);
+        const float* src = (const float*)((unsigned long long)e.y << 32 | e.x);
+        const bool in_place = src && e.w && a.in[threadIdx.x].where;
         src_s[threadIdx.x] = in_place ? nullptr : src;
+        inv_s[threadIdx.x] = __uint_as_float(e.z);
         if (blockIdx.x == 0 && a.in[threadIdx.x].where)
             *a.in[threadIdx.x].where = in_place ? (const void*)src : a.in[threadIdx.x].dst;
-        inv_s[threadIdx.x] = blk->arg[threadIdx.x].inv_scale;
     }
     // the scale table, when a row of it has changed
     if (blockIdx.x == gridDim.x - 1 && table && blk->table_rows > 0) {
@@ -182,7 +185,9 @@ int largest_dec(double a) {
 
 extern "C" int b2_call_inputs(const b2_call_input* inputs, int32_t n, const b2_call_block* block,
                               b2_flex_scale* table, int32_t* stats, void* stream) {
-    B2_REQUIRE(n >= 0 && n <= B2_CALL_MAX_INPUTS && (n == 0 || inputs) && block, "bad argument");
+    static_assert(sizeof(b2_call_arg) == 16 && offsetof(b2_call_block, arg) % 16 == 0, "read as one word");
+    B2_REQUIRE(n >= 0 && n <= B2_CALL_MAX_INPUTS && (n == 0 || inputs) && block &&
+               ((uintptr_t)block & 15) == 0, "bad argument");
     Inputs a;
     a.n = n;
     long long chunks = 0, total = 0;
