@@ -10,8 +10,8 @@
 //   warp 8:    tensor memory, tcgen05.mma issue.
 // A k-block is 128 bytes of plane: 32 fp32 or 128 int16 values.
 //   fp32:   3xTF32.  B's planes lie behind one another and make one operand of 2*BN rows:
-//           A_hi x [B_hi | B_lo] -> [hh | x], A_lo x B_hi -> x.  The two sums are kept apart until the
-//           end; a chain runs over at most 16 k-blocks (the tensor core's fp32 sum truncates), longer
+//           A_hi x [B_hi | B_lo] -> [hh | x], A_lo x B_hi -> x.  Convolutions keep the two sums apart
+//           until the end, matrix products have one (see ONE_CHAIN); a chain runs over at most 16 k-blocks (the tensor core's fp32 sum truncates), longer
 //           K is cut into slices.
 //   flex16: four exact int8 products, HH | X | LL as in b2_gemm_impl.cuh.
 // Slices of K: the CTAs of a cluster (up to 8) take one each; partial sums meet in distributed shared
@@ -195,6 +195,10 @@ direct_kernel(const __grid_constant__ DirectParams p) {
     constexpr int KB = MODE == MODE_FLEX16 ? 128 : 32;            // columns of a k-block
     constexpr int PER = KB / 8;                                   // columns of a 16-byte chunk
     constexpr int kCols = dir_tmem_cols(MODE, BN);
+    // fp32 matrix products: one accumulator, the three products of a k-step in the order of the plane
+    // kernels, slices of whole chains -- the same rounding whichever kernel a size takes (a mask `x > 0`
+    // of a value near zero would otherwise change with the dispatch)
+    constexpr bool ONE_CHAIN = MODE == MODE_F32X3 && AK != B2_OPERAND_GATHER;
     typedef OperandTile<MODE, 128> ATile;
     typedef OperandTile<MODE, BN> BTile;
     unsigned long long* full_bar = (unsigned long long*)(smem + NST * STAGE);     // [NST]
@@ -464,6 +468,12 @@ direct_kernel(const __grid_constant__ DirectParams p) {
                     tc_mma<MODE>(tmem_base + BN, dA0 + adv, dB1 + adv, id_su, acc);          // X += ah*bl
                     tc_mma<MODE>(tmem_base + BN, dA1 + adv, dB0 + adv, id_us, 1u);           // X += al*bh
                     tc_mma<MODE>(tmem_base + 2 * BN, dA1 + adv, dB1 + adv, id_uu, acc);      // LL
+                } else if (ONE_CHAIN) {
+                    tc_mma<MODE>(tmem_base, dA0 + adv, dB0 + adv, id_t1, acc);               // hi*hi
+                    tc_mma<MODE>(tmem_base, a.colmajor ? dA1 + adv : dA0 + adv,
+                                 a.colmajor ? dB0 + adv : dB1 + adv, id_t1, 1u);
+                    tc_mma<MODE>(tmem_base, a.colmajor ? dA0 + adv : dA1 + adv,
+                                 a.colmajor ? dB1 + adv : dB0 + adv, id_t1, 1u);
                 } else {
                     tc_mma<MODE>(tmem_base, dA0 + adv, dB0 + adv, id_t2, acc);               // hh | x
                     tc_mma<MODE>(tmem_base + BN, dA1 + adv, dB0 + adv, id_t1, 1u);           // x += lo*hi
@@ -599,10 +609,12 @@ direct_kernel(const __grid_constant__ DirectParams p) {
             } else {
                 unsigned hh[8], xx[8];
                 tmem_ld8(lane_addr + c0, hh);
-                tmem_ld8(lane_addr + BN + c0, xx);
+                if (!ONE_CHAIN) tmem_ld8(lane_addr + BN + c0, xx);
                 tmem_ld_wait();
 #pragma unroll
-                for (int j = 0; j < 8; ++j) v[j] = (Sum)(__uint_as_float(hh[j]) + __uint_as_float(xx[j]));
+                for (int j = 0; j < 8; ++j)
+                    v[j] = ONE_CHAIN ? (Sum)__uint_as_float(hh[j])
+                                     : (Sum)(__uint_as_float(hh[j]) + __uint_as_float(xx[j]));
             }
             if (splits == 1) {
                 if (ok) finish(c0, v);
@@ -672,7 +684,8 @@ DirectShape direct_shape(const b2_direct_args& a) {
         if (bn > 16 && bn / 2 >= a.N) break;
         const long long tiles = tm * ((a.N + bn - 1) / bn);
         for (int want = 1; want <= 8 && want <= num_kb; ++want) {
-            const int per = (num_kb + want - 1) / want, splits = (num_kb + per - 1) / per;
+            const bool chains = MODE == MODE_F32X3 && a.a_kind != B2_OPERAND_GATHER && want > 1;
+            const int per = chains ? most : (num_kb + want - 1) / want, splits = (num_kb + per - 1) / per;
             if (splits != want || per > most) continue;
             const int tab = a.a_kind == B2_OPERAND_GATHER ? per * KB * (filter_tiles(a) ? 16 : 8) : 0;
             if (1152 + dir_ring_bytes(bn) + tab > 232448) continue;

@@ -27,9 +27,9 @@ inline long long plane_cost(int mode, const Shapes& s, int M, int N, int K) {
     const long long prepass = ((long long)M + N) * K * (mode == MODE_FLEX16 ? 4 : 12) / 2600;
     const long long num_kb = s.Kp / (kKBytes / s.esize);
     if (goes_in_pairs(s, M, pick_splits(mode, s, false))) {
-        const int tiles = ((M + 255) / 256) * ((N + 127) / 128), z = pair_splits(tiles, (int)num_kb);
+        const int tiles = ((M + 255) / 256) * ((N + 127) / 128), z = pair_splits(mode, tiles, (int)num_kb);
         const long long kb = mode == MODE_FLEX16 ? 1100 : 900;
-        return (mode == MODE_FLEX16 ? 20000 : 14000) + prepass + (long long)(tiles * z + 73) / 74 * (5000 + (num_kb + z - 1) / z * kb) + (z > 1 ? 2500 : 0);
+        return (mode == MODE_FLEX16 ? 20000 : 14000) + prepass + (long long)(tiles * z + 73) / 74 * (5000 + pair_slice(mode, (int)num_kb, z) * kb) + (z > 1 ? 2500 : 0);
     }
     const long long kb = (mode == MODE_FLEX16 ? 1430LL : 1100LL) * (128 + s.bn) / 256;
     const long long tiles = (long long)(s.Mp / kBlockM) * (s.Np / s.bn);

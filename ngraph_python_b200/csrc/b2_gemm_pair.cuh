@@ -218,8 +218,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constan
                             tc_mma_pair<MODE>(tmem_base + 256, dA1 + adv, dB0 + adv, id_u, acc);    // X2 | LL
                         } else {
                             tc_mma_pair<MODE>(acc0, dA0 + adv, dB0 + adv, id_t, acc);               // hi*hi
-                            tc_mma_pair<MODE>(acc0 + 128, dA0 + adv, dB1 + adv, id_t, acc);         // hi*lo
-                            tc_mma_pair<MODE>(acc0 + 128, dA1 + adv, dB0 + adv, id_t, 1u);          // lo*hi
+                            // (into one sum, in the single-SM kernel's order: the same rounding)
+                            tc_mma_pair<MODE>(acc0, dA0 + adv, dB1 + adv, id_t, 1u);                // hi*lo
+                            tc_mma_pair<MODE>(acc0, dA1 + adv, dB0 + adv, id_t, 1u);                // lo*hi
                         }
                     }
                     tc_commit_pair(&empty_bar[s], mask);
@@ -331,13 +332,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constan
                     tc_fence_after();
 #pragma unroll
                     for (int c0 = 0; c0 < 64; c0 += 16) {
-                        unsigned hh[16], xx[16];
-                        tmem_ld16(lane_addr + b * 256 + c_lo + c0, hh);
-                        tmem_ld16(lane_addr + b * 256 + 128 + c_lo + c0, xx);
+                        unsigned v[16];
+                        tmem_ld16(lane_addr + b * 256 + c_lo + c0, v);
                         tmem_ld_wait();
 #pragma unroll
-                        for (int j = 0; j < 16; ++j)
-                            sum[c0 + j] += (Sum)(__uint_as_float(hh[j]) + __uint_as_float(xx[j]));
+                        for (int j = 0; j < 16; ++j) sum[c0 + j] += (Sum)__uint_as_float(v[j]);
                     }
                     tc_fence_before();
                     __syncwarp();
@@ -400,11 +399,15 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constan
     if (threadIdx.x == 0 && *fail_flag && g.status) atomicExch(g.status, 1);
 }
 
-inline int pair_splits(int tiles, int num_kb) {
-    // pairs that would stand idle: 74 of them
+inline int pair_splits(int mode, int tiles, int num_kb) {
+    // pairs that would stand idle: 74 of them.  fp32 slices are whole chains of 16 k-blocks.
     int s = 1;
-    while (s < 4 && 2 * s * tiles <= 74 && num_kb / (2 * s) >= 4) s *= 2;
+    while (s < 4 && 2 * s * tiles <= 74 && (mode == MODE_FLEX16 ? num_kb / (2 * s) >= 4 : num_kb > 16 * s)) s *= 2;
     return s;
+}
+inline int pair_slice(int mode, int num_kb, int splits) {
+    const int per = (num_kb + splits - 1) / splits;
+    return mode == MODE_FLEX16 || splits == 1 ? per : (per + kChunkKb - 1) / kChunkKb * kChunkKb;
 }
 
 // The planes are in scratch, A's rows padded to 256 and B's to 128.
@@ -423,8 +426,8 @@ int launch_pair(unsigned char* base, const Shapes& s, GemmParams g, cudaStream_t
     p.g = g;
     p.g.num_kb = s.Kp / (kKBytes / s.esize);
     p.tm = (g.M + 255) / 256; p.tn = (g.N + 127) / 128; p.tiles = p.tm * p.tn;
-    p.splits = pair_splits(p.tiles, p.g.num_kb);
-    p.kb_per_split = (p.g.num_kb + p.splits - 1) / p.splits;
+    p.splits = pair_splits(MODE, p.tiles, p.g.num_kb);
+    p.kb_per_split = pair_slice(MODE, p.g.num_kb, p.splits);
     p.splits = (p.g.num_kb + p.kb_per_split - 1) / p.kb_per_split;
     static bool attr_set = false;
     if (!attr_set) {
