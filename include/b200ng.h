@@ -52,7 +52,8 @@ int b2_device_count(void);
  * high bytes at the destination pointer and low bytes plane_bytes further -- the operand format
  * of the convolution entry points that take planes, so no separate split pass is needed. */
 /* B2_F32_AT (inputs only): the pointer given at launch is the address of a device word that holds the
- * address of the values when the kernel runs, 16-byte aligned. */
+ * address of the values when the kernel runs, 16-byte aligned.  An fp32 result that is such an input's
+ * register, laid out as the input, is not stored where that address is the result's own. */
 enum b2_dtype { B2_F32 = 0, B2_FLEX16 = 1, B2_FLEX16_PLANES = 2, B2_F32_AT = 3 };
 
 /* op codes: one per template of float_ew2.py:31-68 */
@@ -140,6 +141,9 @@ int b2_ew_scratch_bytes(const b2_ew_kernel* k, size_t* bytes);
 int b2_ew_launch(b2_ew_kernel* k, const void* const* in, void* const* out, const float* consts,
                  const b2_flex_scale* flex_table, int32_t* flex_stats, void* scratch,
                  size_t scratch_bytes, int32_t* status, int probe, void* stream);
+/* Compiles and loads what b2_ew_launch with these pointers (probe 0) runs, so that a launch inside a
+ * stream capture compiles nothing. */
+int b2_ew_prepare(b2_ew_kernel* k, const void* const* in, void* const* out);
 /* Programs of one and the same non-empty b2_ew_joint_source (no reductions, one row) in as few launches
  * as their arguments take (one with pointers that are not 16-byte aligned goes by itself). */
 typedef struct b2_ew_launch_job {

@@ -295,9 +295,34 @@ void emit_loads(std::ostringstream& o, const b2_ew_program& p, const Plan& pl,
     }
 }
 
+// The B2_F32_AT input that result k stores as it was read, -1 where it stores something else.  Where the
+// word holds the result's own address the values are there already: such a result is not stored (put<k>,
+// decided once per block).  Storing them all the same costs 4 bytes a value: four arguments of 8192 x
+// 16384 fp32, three of them with such a result, 0.689 ms, and 0.433 without the stores.
+int stored_input(const b2_ew_program& p, int k) {
+    if (k >= p.n_out || p.out[k].reg >= p.n_in) return -1;
+    const int i = p.out[k].reg;
+    const b2_ew_tensor &in = p.in[i], &out = p.out[k].t;
+    return in.dtype == B2_F32_AT && out.dtype == B2_F32 && in.sa == out.sa && in.sb == out.sb && in.sc == out.sc ? i : -1;
+}
+
+void emit_store_always(std::ostringstream& o, const b2_ew_program& p, const Plan& pl, int k, bool probe,
+                       const std::string& ind);
+
 // Store of one elementwise output from y<k>[V].
 void emit_store(std::ostringstream& o, const b2_ew_program& p, const Plan& pl, int k, bool probe,
                 const std::string& ind) {
+    if (!probe && stored_input(p, k) >= 0) {
+        o << ind << "if (put" << k << ") {\n";
+        emit_store_always(o, p, pl, k, probe, ind + "    ");
+        o << ind << "}\n";
+    } else {
+        emit_store_always(o, p, pl, k, probe, ind);
+    }
+}
+
+void emit_store_always(std::ostringstream& o, const b2_ew_program& p, const Plan& pl, int k, bool probe,
+                       const std::string& ind) {
     const b2_ew_tensor& t = p.out[k].t;
     const bool flex = is_flex(t.dtype);
     const bool planes = t.dtype == B2_FLEX16_PLANES;
@@ -439,6 +464,9 @@ int generate(const b2_ew_program& p, const Plan& pl, bool probe, std::string* ou
     for (int i = 0; i < p.n_in; ++i)
         if (p.in[i].dtype == B2_F32_AT)
             o << "    const float* const at" << i << " = *(const float* const volatile*)p.in[" << i << "];\n";
+    for (int k = 0; k < p.n_out && !probe; ++k)
+        if (stored_input(p, k) >= 0)
+            o << "    const bool put" << k << " = at" << stored_input(p, k) << " != (const float*)p.out[" << k << "];\n";
 
     if (p.reduce_mode != B2_REDUCE_B) {
         o << "    const b2_i64 rows = p.A * p.B;\n"
@@ -1109,27 +1137,31 @@ cudaError_t launch_main(const void* func, dim3 grid, void** params, size_t dyn, 
 // What both launch entry points share: argument checks and the choice between the vector and the
 // scalar variant (decided by the pointers' alignment), then the argument block and the launches.
 namespace {
-int check_launch(const b2_ew_kernel* k, const void* const* in, void* const* out,
-                 const float* consts, const b2_flex_scale* flex_table, const int32_t* flex_stats,
-                 int* vec_out) {
+int variant_for(const b2_ew_kernel* k, const void* const* in, void* const* out, int* vec_out) {
     B2_REQUIRE(k && (in || k->prog.n_in == 0) && out, "null argument");
     const b2_ew_program& p = k->prog;
-    const int nres = p.n_out + p.n_red;
-    bool any_flex = false;
     int vec = k->can_vec ? 1 : 0;
     for (int i = 0; i < p.n_in; ++i) {
         B2_REQUIRE(in[i], "input %d is null", i);
-        any_flex |= p.in[i].dtype == B2_FLEX16;
         if (vec && p.in[i].sc == 1 && p.in[i].dtype != B2_F32_AT && !aligned16(in[i])) vec = 0;
     }
-    for (int q = 0; q < nres; ++q) {
+    for (int q = 0; q < p.n_out + p.n_red; ++q) {
         B2_REQUIRE(out[q], "result %d is null", q);
-        any_flex |= is_flex(p.out[q].t.dtype);
         if (vec && q < p.n_out && !aligned16(out[q])) vec = 0;
     }
+    *vec_out = vec;
+    return B2_OK;
+}
+
+int check_launch(const b2_ew_kernel* k, const void* const* in, void* const* out,
+                 const float* consts, const b2_flex_scale* flex_table, const int32_t* flex_stats,
+                 int* vec_out) {
+    const int rc = variant_for(k, in, out, vec_out);
+    if (rc) return rc;
+    const b2_ew_program& p = k->prog;
+    const bool any_flex = uses_flex(p);
     if (any_flex) B2_REQUIRE(flex_table && flex_stats, "flex tensors need a scale table and stats");
     B2_REQUIRE(p.n_const == 0 || consts, "constants missing");
-    *vec_out = vec;
     return B2_OK;
 }
 
@@ -1186,6 +1218,12 @@ int launch_variant(const b2_ew_kernel* k, int vec, const Module* m, const void* 
     return B2_OK;
 }
 }  // namespace
+
+extern "C" int b2_ew_prepare(b2_ew_kernel* k, const void* const* in, void* const* out) {
+    int vec = 0;
+    const int rc = variant_for(k, in, out, &vec);
+    return rc ? rc : ensure_variant(k, vec, 0);
+}
 
 extern "C" int b2_ew_launch(b2_ew_kernel* k, const void* const* in, void* const* out,
                             const float* consts, const b2_flex_scale* flex_table,

@@ -120,6 +120,7 @@ def _load():
         "b2_ew_check": (C.c_int, [C.POINTER(EwProgram), C.c_int, C.c_int, C.c_char_p, sz]),
         "b2_ew_compile": (C.c_int, [C.POINTER(EwProgram), C.POINTER(vp)]),
         "b2_ew_scratch_bytes": (C.c_int, [vp, C.POINTER(sz)]),
+        "b2_ew_prepare": (C.c_int, [vp, C.POINTER(vp), C.POINTER(vp)]),
         "b2_ew_launch": (C.c_int, [vp, C.POINTER(vp), C.POINTER(vp), C.POINTER(C.c_float), vp, vp,
                                    vp, sz, vp, C.c_int, vp]),
         "b2_ew_joint_source": (C.c_int, [vp, C.POINTER(C.c_char_p)]),
@@ -327,6 +328,11 @@ class EwKernel(object):
         s = C.c_char_p()
         check(_lib.b2_ew_joint_source(self.handle, C.byref(s)))
         return s.value
+
+    def prepare(self, in_ptrs, out_ptrs):
+        """Compiles what a launch with these pointers needs (a recording must not)."""
+        check(_lib.b2_ew_prepare(self.handle, (C.c_void_p * max(1, len(in_ptrs)))(*in_ptrs),
+                                 (C.c_void_p * max(1, len(out_ptrs)))(*out_ptrs)))
 
     def launch(self, in_ptrs, out_ptrs, consts=(), flex_table=0, flex_stats=0, scratch=0,
                scratch_bytes=0, status=0, probe=False, stream=0):

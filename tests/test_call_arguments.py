@@ -44,3 +44,25 @@ def test_device_arguments_in_place(rows, cols):
     np.testing.assert_array_equal(third(v), v.cpu().numpy().max(axis=1))
     check(values(7))
     t.close()
+
+
+def test_recorded_kernel_beside_an_unaligned_operand():
+    """The kernel of a recorded call is compiled before the recording, also where another operand's
+    address asks for the scalar variant."""
+    import torch
+    n = 1 << 18
+    A, whole = ng.make_axis(n, name="A"), ng.make_axis(n + 1, name="A")
+    w = np.random.RandomState(1).rand(n + 1).astype(np.float32)
+    x = ng.placeholder([A])
+    shifted = ng.cast_axes(ng.tensor_slice(ng.variable([whole], initial_value=w), (slice(1, None),)), [A])
+    t = ng.transformers.allocate_transformer("b200")
+    comp = t.computation(x * shifted, x)
+    comp(np.zeros(n, np.float32))
+    comp.capture()
+    step = [s for s in comp.steps if s.kind == "ew"][-1]
+    assert step.stores_argument and any(v.offset % 4 for v in step.in_views)
+    for seed in (2, 3):
+        v = torch.rand((n,), device="cuda", generator=torch.Generator(device="cuda").manual_seed(seed))
+        np.testing.assert_array_equal(comp(v), v.cpu().numpy() * w[1:])
+        np.testing.assert_array_equal(np.asarray(t.get_tensor_view_value(x)), v.cpu().numpy())
+    t.close()

@@ -66,3 +66,25 @@ def test_programs_compile(mode_dims, flex, vec, probe):
     assert "b2_ew_main" in src
     if mode == lib.REDUCE_C and Cn == 1 << 22:
         assert "b2_ew_finalize" in src
+
+
+@pytest.mark.parametrize("vec", (0, 1))
+@pytest.mark.parametrize("mode", (lib.REDUCE_NONE, lib.REDUCE_C, lib.REDUCE_B))
+def test_argument_in_place_is_not_stored_onto_itself(mode, vec):
+    """A result that stores an argument as it was read is stored only where the argument lies somewhere
+    else; a result in another layout, or of another register, always."""
+    A, B, Cn = 2, 6, 64
+    full, swapped = (B * Cn, Cn, 1), (Cn, A * Cn, 1)
+    ins = [dict(dtype=lib.F32_AT, strides=full), dict(dtype=lib.F32, strides=full)]
+    outs = [dict(dtype=lib.F32, strides=full, reg=2), dict(dtype=lib.F32, strides=full, reg=0),
+            dict(dtype=lib.F32, strides=swapped, reg=0), dict(dtype=lib.F32, strides=full, reg=1)]
+    red = {lib.REDUCE_NONE: [], lib.REDUCE_C: [(B, 1, 0)], lib.REDUCE_B: [(Cn, 0, 1)]}[mode]
+    reds = [dict(dtype=lib.F32, strides=st, reg=2, redop="sum") for st in red]
+    prog = lib.make_program((A, B, Cn), ins, [], [("mul", 0, 1)], outs, reds, mode)
+    src = lib.ew_check(prog, vec=bool(vec), want_source=True)
+    assert src.count("const bool put1 = at0 != (const float*)p.out[1];") == 1
+    assert re.findall(r"if \(put(\d)\)", src) == ["1"]
+    body = src[src.index("b2_ew_main"):]
+    stores = [m.start() for m in re.finditer(r"b2_st4_cs\(o1|o1\[\(c", body)]
+    assert len(stores) == 1 and body.rindex("if (put1) {", 0, stores[0]) > body.rindex("}", 0, stores[0])
+    assert "put" not in lib.ew_check(prog, vec=bool(vec), probe=True, want_source=True).split("b2_ew_main")[1]

@@ -42,6 +42,27 @@ def test_c2_is_one_kernel():
         comp(*[np.zeros((24, 2048), np.float32)] * 4)
 
 
+def test_arguments_are_in_place_unless_recorded():
+    """A call that is not recorded finds its arguments in their tensors: the kernel neither looks for
+    them nor stores them.  Only the program of a recorded call does, as many as it has results left."""
+    R, C = ng.make_axis(512, name="R"), ng.make_axis(1024, name="C")
+    x, a, b, c = ph = [ng.placeholder([R, C]) for _ in range(4)]
+    y = ng.tanh(a * x + b) * ng.sigmoid(c)
+    t = ng.transformers.allocate_transformer("b200", plan_only=True)
+    comp = t.computation([y, ng.sum(y, reduction_axes=[C]), ng.max(ng.absolute(y), reduction_axes=[C])], *ph)
+    t.initialize()
+    step, = comp.steps
+    plain, recorded = step.kernel.prog, step.recorded_program
+    assert (plain.n_in, plain.n_out, plain.n_red) == (4, 1, 2)
+    assert all(plain.inp[i].dtype == lib.F32 for i in range(4)) and len(step.out_targets) == 3
+    assert (recorded.n_in, recorded.n_out, recorded.n_red) == (4, 4, 2)
+    at = [i for i in range(4) if recorded.inp[i].dtype == lib.F32_AT]
+    assert at == list(step.stores_argument) == [recorded.out[k].reg for k in (1, 2, 3)]
+    assert [v.buffer for v, _ in step.recorded_targets[1:4]] == [step.in_views[i].buffer for i in at]
+    src = lib.ew_check(recorded, want_source=True)
+    assert len([1 for k in (1, 2, 3) if "if (put%d)" % k in src]) == 3
+
+
 def test_softmax_splits_at_reductions():
     """A value needed only after a whole reduction starts a new kernel (the reference's stage
     boundary, ngraph/transformers/gpu/float_ew2.py:553-612)."""
