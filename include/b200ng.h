@@ -267,7 +267,15 @@ int b2_gemm_scratch_bytes(int32_t flex, int32_t M, int32_t N, int32_t K, size_t*
  * planes and the tile kernel (K strides as below). */
 int b2_gemm_launches(int32_t flex, int64_t a_k_stride, int64_t b_k_stride, int32_t M, int32_t N,
                      int32_t K, int32_t* launches);
-/* fp32 via 3xTF32 (relative error ~2^-21). */
+/* Which kernel that is, and how it cuts the product: tile_n columns to a tile, K in `slices` parts that
+ * the CTAs or pairs of a cluster take, `waves` times as many clusters as the machine holds at once. */
+enum b2_gemm_kernel { B2_GEMM_DIRECT = 0, B2_GEMM_PAIRS = 1, B2_GEMM_TILES = 2 };
+typedef struct b2_gemm_plan_info { int32_t kernel, tile_n, slices, waves; } b2_gemm_plan_info;
+int b2_gemm_plan(int32_t flex, int64_t a_k_stride, int64_t b_k_stride, int32_t M, int32_t N, int32_t K,
+                 b2_gemm_plan_info* plan);
+/* fp32 via 3xTF32 (relative error ~2^-21).  Sums of K in chains of 512 products; up to K = 4096 every
+ * kernel adds the chains in order, so that a result does not depend on the number of rows and columns
+ * computed beside it. */
 int b2_gemm_f32(const float* A, int64_t a_row_stride, int64_t a_k_stride, const float* B,
                 int64_t b_k_stride, int64_t b_col_stride, float* C, int64_t ldc, int32_t M,
                 int32_t N, int32_t K, void* scratch, size_t scratch_bytes, int32_t* status,

@@ -13,6 +13,11 @@ long long b2_direct_cost(const b2_direct_args& a) {
     return a.flex ? direct_shape<MODE_FLEX16>(a).cost : direct_shape<MODE_F32X3>(a).cost;
 }
 
+void b2_direct_plan(const b2_direct_args& a, b2_gemm_plan_info* plan) {
+    const DirectShape s = a.flex ? direct_shape<MODE_FLEX16>(a) : direct_shape<MODE_F32X3>(a);
+    *plan = {B2_GEMM_DIRECT, s.bn, s.splits, s.waves};
+}
+
 int b2_direct_launch(const b2_direct_args& a, cudaStream_t st) {
     B2_REQUIRE(b2_direct_cost(a) >= 0, "problem outside the kernel's range");
     return a.flex ? b2_direct_launch_flex(a, st) : direct_launch_mode<MODE_F32X3>(a, st);

@@ -668,7 +668,7 @@ direct_kernel(const __grid_constant__ DirectParams p) {
 }
 
 // ---- host ------------------------------------------------------------------------------------
-struct DirectShape { int bn, splits, kb_per_split; long long cost; };
+struct DirectShape { int bn, splits, kb_per_split, waves; long long cost; };
 
 template <int MODE>
 DirectShape direct_shape(const b2_direct_args& a) {
@@ -676,9 +676,7 @@ DirectShape direct_shape(const b2_direct_args& a) {
     const int num_kb = (a.K + KB - 1) / KB;
     // fp32: 16 k-blocks to a chain; flex16: exact int32 sums up to 32768 columns
     const int most = MODE == MODE_FLEX16 ? 256 : 16;
-    DirectShape best = {0, 0, 0, -1};
-    // SMs that clusters of 1..8 CTAs of this shared memory fill (what cudaOccupancyMaxActiveClusters says)
-    static const int fit[9] = {0, 148, 148, 135, 132, 130, 132, 119, 120};
+    DirectShape best = {0, 0, 0, 0, -1};
     const long long tm = (a.M + 127) / 128;
     for (int bn = 16; bn <= 128; bn *= 2) {
         if (bn > 16 && bn / 2 >= a.N) break;
@@ -700,13 +698,13 @@ DirectShape direct_shape(const b2_direct_args& a) {
             const long long lat = MODE == MODE_FLEX16 ? 4000 : a.a_kind != B2_OPERAND_GATHER ? 1000 + 6 * bn
                                   : bn >= 64 ? 3500 : 1600 + 25 * bn;
             const long long ctas = tiles * splits, per_sm = bn == 128 || 1152 + dir_ring_bytes(bn) + tab > 115000 ? 1 : 2;
-            const long long slots = (long long)fit[splits] * per_sm;
+            const long long slots = (long long)kClusterCtas[splits] * per_sm;
             const long long together = ctas <= 148 ? 1 : per_sm;
             const long long kb = together * pace > lat ? together * pace : lat;
             const long long one = 7000 + per * kb + together * bn * (splits > 1 ? 24 : 12) +
                                   (splits == 1 ? 0 : filter_tiles(a) ? 18000 : 3000);
-            const long long cost = (ctas + slots - 1) / slots * one;
-            if (best.cost < 0 || cost < best.cost) best = {bn, splits, per, cost};
+            const long long waves = (ctas + slots - 1) / slots, cost = waves * one;
+            if (best.cost < 0 || cost < best.cost) best = {bn, splits, per, (int)waves, cost};
         }
     }
     return best;

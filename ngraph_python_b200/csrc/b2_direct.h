@@ -45,8 +45,13 @@ struct b2_direct_args {
     const float *bias, *residual, *mask;
 };
 
+// CTAs that the machine holds at once in clusters of 1..8 CTAs with an SM each (what
+// cudaOccupancyMaxActiveClusters says; a cluster does not cross a GPC).
+constexpr int kClusterCtas[9] = {0, 148, 148, 135, 132, 130, 132, 119, 120};
+
 // Estimated cycles of a launch, negative where the kernel does not take the problem.
 __attribute__((visibility("hidden"))) long long b2_direct_cost(const b2_direct_args& a);
+__attribute__((visibility("hidden"))) void b2_direct_plan(const b2_direct_args& a, b2_gemm_plan_info* plan);
 __attribute__((visibility("hidden"))) int b2_direct_launch(const b2_direct_args& a, cudaStream_t st);
 
 // fp32 filter gradient (b2_conv_update_f32.cu): no dilation, one depth.  Scratch 0: not taken.

@@ -123,6 +123,28 @@ extern "C" int b2_gemm_launches(int32_t flex, int64_t a_k_stride, int64_t b_k_st
     return B2_OK;
 }
 
+extern "C" int b2_gemm_plan(int32_t flex, int64_t a_k_stride, int64_t b_k_stride, int32_t M, int32_t N,
+                            int32_t K, b2_gemm_plan_info* plan) {
+    B2_REQUIRE(plan && M > 0 && N > 0 && K > 0, "bad argument");
+    const int mode = flex ? MODE_FLEX16 : MODE_F32X3;
+    b2_direct_args d;
+    if (gemm_goes_direct(mode, nullptr, 1, a_k_stride, nullptr, b_k_stride, 1, M, N, K, &d)) {
+        b2_direct_plan(d, plan);
+        return B2_OK;
+    }
+    const Shapes s = shapes_for(mode, M, N, K);
+    const int splits = pick_splits(mode, s, false), num_kb = s.Kp / (kKBytes / s.esize);
+    if (goes_in_pairs(s, M, splits)) {
+        const int tiles = ((M + 255) / 256) * ((N + 127) / 128), per = pair_slice(mode, num_kb, pair_splits(mode, tiles, num_kb));
+        const int z = (num_kb + per - 1) / per, clusters = kClusterCtas[2 * z] / (2 * z);
+        *plan = {B2_GEMM_PAIRS, 128, z, (tiles + clusters - 1) / clusters};
+    } else {
+        const long long tiles = (long long)(s.Mp / kBlockM) * (s.Np / s.bn) * splits;
+        *plan = {B2_GEMM_TILES, s.bn, splits, (int)((tiles + 147) / 148)};
+    }
+    return B2_OK;
+}
+
 extern "C" int b2_gemm_f32(const float* A, int64_t a_row_stride, int64_t a_k_stride, const float* B,
                            int64_t b_k_stride, int64_t b_col_stride, float* C, int64_t ldc,
                            int32_t M, int32_t N, int32_t K, void* scratch, size_t scratch_bytes,

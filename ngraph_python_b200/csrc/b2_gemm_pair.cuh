@@ -9,13 +9,21 @@
 // written, 64 (72) KB read.
 //   flex16: the merged operand [B_hi | B_lo'] of 256 rows is cut between the two SMs by plane:
 //           A_hi x [..] -> HH | X1,  A_lo x [..] -> X2 | LL   (512 columns of tensor memory, all of it)
-//   fp32:   hi*hi -> hh, hi*lo and lo*hi -> x, two buffers of [hh | x]; chains of 16 k-blocks, as there.
+//   fp32:   hi*hi, hi*lo and lo*hi into one sum, in the order of the other kernels; chains of 16
+//           k-blocks in two buffers, as there.
 //
 // Each CTA: warp 0 TMA producer (its loads complete on the leader's barrier), warp 1 tensor memory and,
 // in the leader, MMA issue; warps 2-9 epilogue.  Persistent over tiles, eight tiles of rows at a time
 // down the columns, so that the pairs in flight share panels in L2; the producer runs ahead into the
 // next tile while the epilogue drains the last.  Where there are fewer tiles than pairs, 2 or 4 pairs
-// of one cluster take slices of K and add up in distributed shared memory in slice order.
+// of one cluster take slices of K and add up in distributed shared memory in slice order.  In fp32 the
+// slices after the first keep up to four chains apart, each in tensor-memory columns of its own, and the
+// sum takes them one by one, so that it is rounded as the kernels round it that walk all of K: a value
+// near zero keeps its sign (a ReLU its mask) whatever kernel the number of rows and columns leads to.
+// Slices of more chains (K > 4096, which only this kernel and the single-SM one take) add their own first.
+// Against sums per slice: 1000 x 777 x 1500 32.8 -> 32.5 us, x 2048 34.5 -> 34.5, x 4096 59.7 -> 60.6,
+// 768 x 512 x 4096 34.6 -> 36.0 (eight chains handed over instead of four sums; 16-byte accesses to the
+// peers' memory, the sum of the first slice taken while it multiplies).
 #ifndef B2_GEMM_PAIR_CUH
 #define B2_GEMM_PAIR_CUH
 #include "b2_direct.h"
@@ -80,22 +88,46 @@ __device__ __forceinline__ void tc_mma_pair(unsigned tmem_d, unsigned long long 
 __host__ __device__ constexpr unsigned idesc_pair(unsigned dfmt, unsigned afmt, unsigned bfmt, unsigned n) {
     return (dfmt << 4) | (afmt << 7) | (bfmt << 10) | ((n >> 3) << 17) | ((256u >> 4) << 24);
 }
-__device__ __forceinline__ long long pair_ld(unsigned a, long long) {
-    long long v;
-    asm volatile("ld.shared::cluster.b64 %0, [%1];" : "=l"(v) : "r"(a) : "memory");
-    return v;
+// Eight columns of a row in the exchanged sums, fp32: two groups of four, rows behind one another, so that
+// a lane's share is two 16-byte accesses and a warp's is contiguous.
+__device__ __forceinline__ void put_piece(float* piece, int lrow, const float* v) {
+    *(float4*)(piece + lrow * 4) = make_float4(v[0], v[1], v[2], v[3]);
+    *(float4*)(piece + 512 + lrow * 4) = make_float4(v[4], v[5], v[6], v[7]);
 }
-__device__ __forceinline__ float pair_ld(unsigned a, float) {
-    float v;
-    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
-    return v;
+__device__ __forceinline__ void get_piece(const float* piece, int lrow, unsigned rank, float* v) {
+    const unsigned at = map_rank(piece + lrow * 4, rank);
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]) : "r"(at) : "memory");
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]) : "r"(at + 2048) : "memory");
+}
+__device__ __forceinline__ void put_piece(long long* piece, int lrow, const long long* v) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) piece[j * 128 + lrow] = v[j];
+}
+__device__ __forceinline__ void get_piece(const long long* piece, int lrow, unsigned rank, long long* v) {
+    const unsigned at = map_rank(piece + lrow, rank);
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+        asm volatile("ld.shared::cluster.b64 %0, [%1];" : "=l"(v[j]) : "r"(at + j * 1024) : "memory");
 }
 
 struct PairParams {
     GemmParams g;
     int tm, tn, tiles;             // 256-row and 128-column tiles
     int splits, kb_per_split;
+    int apart;                     // fp32: slices after the first hand out chains, not their sum ...
+    int apart_pieces, apart_inv;   // ... so many pieces of each; 32 / splits rounded up: i * inv >> 5 is i / splits, i < 16
 };
+
+constexpr int kOrderedKb = 8 * kChunkKb;   // up to here fp32 chains are added in order (K = 4096) ...
+constexpr int kApartChains = 4;            // ... which leaves a slice four at most, in 128 columns each
+// What slice z hands out of a chain: the pieces of eight columns that another slice finishes, one behind
+// the other.  Piece round * splits + owner is finished by slice `owner`; its place in slice z's memory:
+__host__ __device__ constexpr int apart_place(int round, int owner, int z, int splits) {
+    return round * (splits - 1) + owner - (owner > z ? 1 : 0);
+}
+static_assert(kApartChains * 12 * 8 * 128 * 4 <= kPairStages * kPairStage, "12 of 16 pieces fit the ring");
 
 // tile -> (row tile, column tile): bands of eight row tiles, down the columns
 __device__ __forceinline__ void pair_tile(const PairParams& p, int t, int& m, int& n) {
@@ -193,8 +225,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constan
             for (int t = first; t < p.tiles && ok; t += step) {
                 for (int kb = 0; kb < nkb && ok; ++kb) {
                     const int kin = MODE == MODE_FLEX16 ? kb : kb % kChunkKb;
-                    const int b = MODE == MODE_FLEX16 ? 0 : chunk & 1;
-                    if (kin == 0) {
+                    const bool apart = MODE != MODE_FLEX16 && p.apart && slice > 0;
+                    const int b = MODE == MODE_FLEX16 || apart ? 0 : chunk & 1;
+                    if (kin == 0 && !apart) {
                         // the accumulators of this chain must have been drained
                         const int use = MODE == MODE_FLEX16 ? chunk : chunk >> 1;
                         if (use > 0 && !mbar_wait(&tmem_empty[b], (use - 1) & 1)) {
@@ -208,7 +241,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constan
                     const unsigned long long dA0 = make_smem_desc(st), dA1 = make_smem_desc(st + kPlaneBytes);
                     const unsigned long long dB0 = make_smem_desc(st + 2 * kPlaneBytes);
                     const unsigned long long dB1 = make_smem_desc(st + 2 * kPlaneBytes + 64 * kKBytes);
-                    const unsigned acc0 = tmem_base + b * 256;
+                    const unsigned acc0 = tmem_base + (apart ? (kb / kChunkKb) * 128 : b * 256);
 #pragma unroll
                     for (int k = 0; k < 4; ++k) {
                         const unsigned long long adv = (unsigned long long)(2 * k);
@@ -225,7 +258,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constan
                     }
                     tc_commit_pair(&empty_bar[s], mask);
                     if (++s == kPairStages) { s = 0; parity ^= 1u; }
-                    if (kb == nkb - 1 || (MODE != MODE_FLEX16 && kin == kChunkKb - 1)) {
+                    if (kb == nkb - 1 || (MODE != MODE_FLEX16 && !apart && kin == kChunkKb - 1)) {
                         tc_commit_pair(&tmem_full[b], mask);
                         ++chunk;
                     }
@@ -235,7 +268,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constan
     } else {
         // epilogue: lane quarter = warp % 4, a share of the columns each
         typedef typename std::conditional<MODE == MODE_FLEX16, long long, float>::type Sum;
-        Sum* red = (Sum*)smem;                                    // [128 columns][128 rows], slices only
+        Sum* red = (Sum*)smem;                                    // 16 pieces (of every chain, apart), slices only
         constexpr int kGroups = pair_epi_warps(MODE) / 4, kCols = 128 / kGroups;
         const int quarter = warp & 3, c_lo = ((warp - 2) >> 2) * kCols;
         const int lrow = quarter * 32 + lane;
@@ -312,8 +345,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constan
                         v[j] = (Sum)(((long long)(int)hh[j] << 16) +
                                      (((long long)(int)x1[j] + (long long)(int)x2[j]) << 8) + (long long)(int)ll[j]);
                     if (p.splits > 1) {
-#pragma unroll
-                        for (int j = 0; j < 8; ++j) red[(c0 + j) * 128 + lrow] = v[j];
+                        put_piece(red + c0 * 128, lrow, v);
                     } else if (ok) {
                         finish(row, n0 + c0, fix, v);
                     }
@@ -321,6 +353,29 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constan
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) arrive_remote(empty0);
+            } else if (p.apart && slice > 0) {
+                // (one tile per cluster)  all products are done: the ring is free
+                if (ok && !mbar_wait(&tmem_full[0], 0)) { atomicExch(fail_flag, 1); ok = false; }
+                tc_fence_after();
+                const int pieces = p.apart_pieces;
+                for (int ch = 0; ch * kChunkKb < nkb; ++ch)
+#pragma unroll
+                    for (int half = 0; half < 2; ++half) {
+                        const int i0 = (c_lo >> 3) + 4 * half;
+                        unsigned v[32];
+                        tmem_ld16(lane_addr + ch * 128 + i0 * 8, v);
+                        tmem_ld16(lane_addr + ch * 128 + i0 * 8 + 16, v + 16);
+                        tmem_ld_wait();
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) {
+                            const int round = (i0 + u) * p.apart_inv >> 5, owner = i0 + u - round * p.splits;
+                            if (owner == slice) continue;
+                            Sum x[8];
+#pragma unroll
+                            for (int j = 0; j < 8; ++j) x[j] = (Sum)__uint_as_float(v[8 * u + j]);
+                            put_piece(red + (ch * pieces + apart_place(round, owner, slice, p.splits)) * 8 * 128, lrow, x);
+                        }
+                    }
             } else {
                 Sum sum[64];
 #pragma unroll
@@ -345,8 +400,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constan
 #pragma unroll
                 for (int c0 = 0; c0 < 64; c0 += 8) {
                     if (p.splits > 1) {
-#pragma unroll
-                        for (int j = 0; j < 8; ++j) red[(c_lo + c0 + j) * 128 + lrow] = sum[c0 + j];
+                        put_piece(red + (c_lo + c0) * 128, lrow, sum + c0);
                     } else if (ok) {
                         finish(row, n0 + c_lo + c0, 0, sum + c0);
                     }
@@ -360,14 +414,49 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constan
             pair_tile(p, first, tm, tn);
             const int row = tm * 256 + side * 128 + lrow, n0 = tn * 128;
             const long long fix = MODE == MODE_FLEX16 && row < g.M ? 128LL * (long long)g.rowsum[row] : 0LL;
-            for (int c0 = (slice + ((warp - 2) >> 2) * p.splits) * 8; c0 < 128; c0 += 8 * kGroups * p.splits) {
+            // piece round * splits + slice of eight columns
+            for (int round = (warp - 2) >> 2; round * p.splits + slice < 16; round += kGroups) {
+                const int c0 = (round * p.splits + slice) * 8;
                 Sum v[8];
+                if (MODE != MODE_FLEX16 && p.apart) {
+                    get_piece(red + c0 * 128, lrow, side, v);
+                    // the chains of the other slices, four at a time in flight
+                    const int per = p.kb_per_split / kChunkKb;
+                    const int chains = (g.num_kb - p.kb_per_split + kChunkKb - 1) / kChunkKb;
+                    int z = 1, ch = 0;
+                    for (int q = 0; q < chains; q += 4) {
+                        Sum x[4][8];
 #pragma unroll
-                for (int j = 0; j < 8; ++j) v[j] = 0;
-                for (int z = 0; z < p.splits; ++z) {
-                    const unsigned at = map_rank(red + c0 * 128 + lrow, 2 * z + side);
+                        for (int u = 0; u < 4; ++u) {
+                            if (q + u >= chains) break;
+                            if (z == slice) {
+                                unsigned y[8];
+                                tmem_ld8(lane_addr + ch * 128 + c0, y);
+                                tmem_ld_wait();
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) v[j] += pair_ld(at + j * 128 * (unsigned)sizeof(Sum), (Sum)0);
+                                for (int j = 0; j < 8; ++j) x[u][j] = (Sum)__uint_as_float(y[j]);
+                            } else {
+                                const int at = ch * p.apart_pieces + apart_place(round, slice, z, p.splits);
+                                get_piece(red + at * 8 * 128, lrow, 2 * z + side, x[u]);
+                            }
+                            if (++ch == per) { ch = 0; ++z; }
+                        }
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) {
+                            if (q + u >= chains) break;
+#pragma unroll
+                            for (int j = 0; j < 8; ++j) v[j] += x[u][j];
+                        }
+                    }
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) v[j] = 0;
+                    for (int z = 0; z < p.splits; ++z) {
+                        Sum x[8];
+                        get_piece(red + c0 * 128, lrow, 2 * z + side, x);
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) v[j] += x[j];
+                    }
                 }
                 if (ok) finish(row, n0 + c0, fix, v);
             }
@@ -429,6 +518,9 @@ int launch_pair(unsigned char* base, const Shapes& s, GemmParams g, cudaStream_t
     p.splits = pair_splits(MODE, p.tiles, p.g.num_kb);
     p.kb_per_split = pair_slice(MODE, p.g.num_kb, p.splits);
     p.splits = (p.g.num_kb + p.kb_per_split - 1) / p.kb_per_split;
+    p.apart_pieces = 16 - 16 / p.splits;
+    p.apart_inv = (32 + p.splits - 1) / p.splits;
+    p.apart = MODE != MODE_FLEX16 && p.splits > 1 && p.g.num_kb <= kOrderedKb;
     static bool attr_set = false;
     if (!attr_set) {
         B2_CUDA(cudaFuncSetAttribute(gemm_pair_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmem));

@@ -78,6 +78,11 @@ class FlexScale(C.Structure):
     _fields_ = [("scale", C.c_float), ("inv_scale", C.c_float)]
 
 
+class GemmPlan(C.Structure):
+    _fields_ = [(n, C.c_int32) for n in ("kernel", "tile_n", "slices", "waves")]
+
+
+GEMM_DIRECT, GEMM_PAIRS, GEMM_TILES = 0, 1, 2
 CALL_MAX_INPUTS, CALL_MAX_OUTPUTS = 16, 16
 
 
@@ -132,6 +137,7 @@ def _load():
         "b2_ew_launch_count": (C.c_int, [vp]),
         "b2_gemm_scratch_bytes": (C.c_int, [i32, i32, i32, i32, C.POINTER(sz)]),
         "b2_gemm_launches": (C.c_int, [i32, i64, i64, i32, i32, i32, C.POINTER(i32)]),
+        "b2_gemm_plan": (C.c_int, [i32, i64, i64, i32, i32, i32, C.POINTER(GemmPlan)]),
         "b2_gemm_f32": (C.c_int, [vp, i64, i64, vp, i64, i64, vp, i64, i32, i32, i32, vp, sz, vp,
                                   vp]),
         "b2_gemm_flex16": (C.c_int, [vp, i64, i64, vp, i64, i64, vp, i64, i32, i32, i32, vp, i32,
@@ -383,6 +389,13 @@ def gemm_launches(flex, a_k_stride, b_k_stride, M, N, K):
     n = C.c_int32()
     check(_lib.b2_gemm_launches(int(bool(flex)), a_k_stride, b_k_stride, M, N, K, C.byref(n)))
     return n.value
+
+
+def gemm_plan(flex, a_k_stride, b_k_stride, M, N, K):
+    """(kernel, columns of a tile, slices of K, waves of clusters) of a product."""
+    p = GemmPlan()
+    check(_lib.b2_gemm_plan(int(bool(flex)), a_k_stride, b_k_stride, M, N, K, C.byref(p)))
+    return p.kernel, p.tile_n, p.slices, p.waves
 
 
 def conv_fprop_scratch_bytes(flex, dims):

@@ -100,3 +100,41 @@ def test_products_for_pairs_of_sms(M, N, K, flex):
     from ngraph_python_b200 import lib
     assert lib.gemm_launches(flex, 1, N, M, N, K) > 1
     _run(torch, flex, "nn", M, N, K)
+
+
+SAME_BITS = {512: {(0, 1)}, 520: {(0, 2), (1, 2)}, 1024: {(0, 2)}, 1500: {(0, 3), (1, 2)},
+             2048: {(0, 4), (1, 2)}, 3000: {(0, 6), (1, 2), (1, 3)}, 4096: {(0, 8), (1, 2), (1, 4)}}
+
+
+@pytest.mark.parametrize("K", sorted(SAME_BITS))
+def test_fp32_rounding_does_not_depend_on_the_kernel(K):
+    """Rows and columns of a product that no slice cuts, computed again as smaller products: 1 to 8
+    chains, slices of one to four of them, either operand first, narrow and wide tiles."""
+    import torch
+    from ngraph_python_b200 import lib
+    M, N = 2304, 1152
+    g = torch.Generator(device="cuda").manual_seed(K)
+    A = torch.randn((M, K), device="cuda", generator=g)
+    B = torch.randn((K, N), device="cuda", generator=g)
+    A[3] = 0.0
+    A[7, 0::2], A[7, 1::2] = B[0::2, 5], -B[1::2, 5]            # a sum that nearly vanishes
+    status = torch.zeros((1,), dtype=torch.int32, device="cuda")
+
+    def product(m, n):
+        c = torch.full((m, n), 7.0, device="cuda")
+        nbytes = lib.gemm_scratch_bytes(False, m, n, K)
+        scratch = torch.empty((nbytes + 1024,), dtype=torch.uint8, device="cuda")
+        lib.check(lib.raw().b2_gemm_f32(A.data_ptr(), K, 1, B.data_ptr(), N, 1, c.data_ptr(), n, m, n, K,
+                                        scratch.data_ptr() + (-scratch.data_ptr()) % 1024, nbytes,
+                                        status.data_ptr(), 0))
+        torch.cuda.synchronize()
+        return c
+    assert lib.gemm_plan(False, 1, N, M, N, K)[:3] == (lib.GEMM_PAIRS, 128, 1)
+    whole, taken = product(M, N), set()
+    for m, n in ((40, 24), (24, 40), (128, 512), (512, 128), (1000, 777), (768, 512), (1024, 512), (1536, 512),
+                 (2304, 64), (65, 1152)):
+        kernel, _, slices, _ = lib.gemm_plan(False, 1, N, m, n, K)
+        taken.add((kernel, slices))
+        assert torch.equal(product(m, n).view(torch.int32), whole[:m, :n].contiguous().view(torch.int32)), (m, n)
+    assert SAME_BITS[K] <= taken
+    assert int(status.item()) == 0
