@@ -29,7 +29,8 @@ inline long long plane_cost(int mode, const Shapes& s, int M, int N, int K) {
     if (goes_in_pairs(s, M, pick_splits(mode, s, false))) {
         const int tiles = ((M + 255) / 256) * ((N + 127) / 128), z = pair_splits(mode, tiles, (int)num_kb);
         const long long kb = mode == MODE_FLEX16 ? 1100 : 900;
-        return (mode == MODE_FLEX16 ? 20000 : 14000) + prepass + (long long)(tiles * z + 73) / 74 * (5000 + pair_slice(mode, (int)num_kb, z) * kb) + (z > 1 ? 2500 : 0);
+        return (mode == MODE_FLEX16 ? 20000 : 14000) + prepass +
+               pair_waves(tiles, z) * (5000 + pair_slice(mode, (int)num_kb, z) * kb) + (z > 1 ? 2500 : 0);
     }
     const long long kb = (mode == MODE_FLEX16 ? 1430LL : 1100LL) * (128 + s.bn) / 256;
     const long long tiles = (long long)(s.Mp / kBlockM) * (s.Np / s.bn);
@@ -135,9 +136,8 @@ extern "C" int b2_gemm_plan(int32_t flex, int64_t a_k_stride, int64_t b_k_stride
     const Shapes s = shapes_for(mode, M, N, K);
     const int splits = pick_splits(mode, s, false), num_kb = s.Kp / (kKBytes / s.esize);
     if (goes_in_pairs(s, M, splits)) {
-        const int tiles = ((M + 255) / 256) * ((N + 127) / 128), per = pair_slice(mode, num_kb, pair_splits(mode, tiles, num_kb));
-        const int z = (num_kb + per - 1) / per, clusters = kClusterCtas[2 * z] / (2 * z);
-        *plan = {B2_GEMM_PAIRS, 128, z, (tiles + clusters - 1) / clusters};
+        const int tiles = ((M + 255) / 256) * ((N + 127) / 128), z = pair_splits(mode, tiles, num_kb);
+        *plan = {B2_GEMM_PAIRS, 128, z, (int)pair_waves(tiles, z)};
     } else {
         const long long tiles = (long long)(s.Mp / kBlockM) * (s.Np / s.bn) * splits;
         *plan = {B2_GEMM_TILES, s.bn, splits, (int)((tiles + 147) / 148)};

@@ -15,7 +15,7 @@
 // Each CTA: warp 0 TMA producer (its loads complete on the leader's barrier), warp 1 tensor memory and,
 // in the leader, MMA issue; warps 2-9 epilogue.  Persistent over tiles, eight tiles of rows at a time
 // down the columns, so that the pairs in flight share panels in L2; the producer runs ahead into the
-// next tile while the epilogue drains the last.  Where there are fewer tiles than pairs, 2 or 4 pairs
+// next tile while the epilogue drains the last.  Where there are fewer tiles than pairs, 2 to 4 pairs
 // of one cluster take slices of K and add up in distributed shared memory in slice order.  In fp32 the
 // slices after the first keep up to four chains apart, each in tensor-memory columns of its own, and the
 // sum takes them one by one, so that it is rounded as the kernels round it that walk all of K: a value
@@ -488,15 +488,24 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constan
     if (threadIdx.x == 0 && *fail_flag && g.status) atomicExch(g.status, 1);
 }
 
-inline int pair_splits(int mode, int tiles, int num_kb) {
-    // pairs that would stand idle: 74 of them.  fp32 slices are whole chains of 16 k-blocks.
-    int s = 1;
-    while (s < 4 && 2 * s * tiles <= 74 && (mode == MODE_FLEX16 ? num_kb / (2 * s) >= 4 : num_kb > 16 * s)) s *= 2;
-    return s;
-}
+// Clusters of `splits` pairs that the machine holds at once: 74, 33, 22, 15 (a cluster stays within a GPC)
+inline int pair_clusters(int splits) { return kClusterCtas[2 * splits] / (2 * splits); }
+inline long long pair_waves(int tiles, int splits) { return (tiles + pair_clusters(splits) - 1) / pair_clusters(splits); }
+// k-blocks of a slice; fp32 slices are whole chains
 inline int pair_slice(int mode, int num_kb, int splits) {
     const int per = (num_kb + splits - 1) / splits;
     return mode == MODE_FLEX16 || splits == 1 ? per : (per + kChunkKb - 1) / kChunkKb * kChunkKb;
+}
+// As many slices as leave every tile's cluster a place in the first wave: with one more a few clusters
+// would wait for all the others.  35 tiles, 1280 x 896 x 2048: 56.3 us in two slices, 48.2 in one (flex16
+// 39.7, 29.0); 16 tiles, 1024 x 512 x 4096: 57.2 us in four, 45.6 in three (flex16 43.8, 32.4).
+inline int pair_splits(int mode, int tiles, int num_kb) {
+    for (int s = 4; s > 1; --s) {
+        if (tiles > pair_clusters(s) || (mode == MODE_FLEX16 ? num_kb < 4 * s : num_kb <= kChunkKb * (s / 2))) continue;
+        const int per = pair_slice(mode, num_kb, s);
+        return (num_kb + per - 1) / per;
+    }
+    return 1;
 }
 
 // The planes are in scratch, A's rows padded to 256 and B's to 128.
@@ -517,7 +526,6 @@ int launch_pair(unsigned char* base, const Shapes& s, GemmParams g, cudaStream_t
     p.tm = (g.M + 255) / 256; p.tn = (g.N + 127) / 128; p.tiles = p.tm * p.tn;
     p.splits = pair_splits(MODE, p.tiles, p.g.num_kb);
     p.kb_per_split = pair_slice(MODE, p.g.num_kb, p.splits);
-    p.splits = (p.g.num_kb + p.kb_per_split - 1) / p.kb_per_split;
     p.apart_pieces = 16 - 16 / p.splits;
     p.apart_inv = (32 + p.splits - 1) / p.splits;
     p.apart = MODE != MODE_FLEX16 && p.splits > 1 && p.g.num_kb <= kOrderedKb;

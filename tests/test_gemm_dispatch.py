@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
 
 DIRECT = [(1, 1, 1), (3, 16, 31), (127, 17, 33), (129, 33, 127), (10, 256, 64), (64, 130, 129), (300, 40, 515),
           (65, 63, 1025), (257, 7, 2049)]
-PAIRS = [(4097, 4098, 32), (2049, 1200, 513), (1500, 1601, 1024), (700, 650, 6000)]
+PAIRS = [(4097, 4098, 32), (2049, 1200, 513), (1500, 1601, 1024), (700, 650, 6000), (500, 500, 6000), (1001, 900, 3001)]
 
 
 def _operands(torch, flex, layout, M, N, K, seed, offset=0):

@@ -171,3 +171,18 @@ def test_plane_entry_points_describe_the_dilated_error_tensor():
     small = lib.conv_update_scratch_bytes(True, dims(16, 32, 32, 128, 16, 3, 3, 1, 1)[0])
     odd_batch = lib.conv_update_scratch_bytes(True, dims(16, 32, 32, 96, 16, 3, 3, 1, 1)[0])
     assert small < odd_batch
+
+
+@pytest.mark.parametrize("flex", [False, True])
+def test_slices_of_a_product_fit_the_machine(flex):
+    """Clusters of slices never wait for a second wave: 33 of two pairs of SMs, 22 of three and 15 of
+    four are what the machine holds."""
+    taken = set()
+    for K in (544, 1024, 1500, 2048, 3000, 4096, 8192):
+        for m in range(1, 12):
+            for n in range(1, 12):
+                kernel, _, slices, waves = lib.gemm_plan(flex, 1, 128 * n, 256 * m, 128 * n, K)
+                if kernel == lib.GEMM_PAIRS and slices > 1:
+                    assert waves == 1 and m * n <= {2: 33, 3: 22, 4: 15}[slices], (K, m, n)
+                    taken.add(slices)
+    assert taken == {2, 3, 4}
