@@ -479,15 +479,15 @@ class _CallIO(object):
             arr = value
         else:
             arr = t._host_argument(view, value)
-        if arr.nbytes > self.STAGED_MOST and not torch.from_numpy(
-                arr if arr.flags.writeable else arr.copy()).is_pinned():
-            # the driver's own pipelined copy
-            t._stage(view, arr)
-            return (buf.staging.data_ptr() if buf.flex else 0), arr
         # (the buffer is made only for an argument that needs it: pinning memory takes milliseconds)
         address, stage = arr.__array_interface__["data"][0], lib.raw().b2_call_stage
-        have = self.pinned[k].data_ptr() if self.pinned[k] is not None else None
+        through_pinned = arr.nbytes <= self.STAGED_MOST
+        have = self.pinned[k].data_ptr() if through_pinned and self.pinned[k] is not None else None
         lib.check(stage(address, arr.nbytes, have, self.visible))
+        if not self.visible.value and not through_pinned:
+            # pageable: the driver's own pipelined copy
+            t._stage(view, arr)
+            return (buf.staging.data_ptr() if buf.flex else 0), arr
         if not self.visible.value:
             lib.check(stage(address, arr.nbytes, self._pinned_buffer(k), self.visible))
         return self.visible.value, arr
@@ -1955,8 +1955,7 @@ class B200Transformer(object):
                                           device=self.device)
             buf.staging.copy_(src, non_blocking=True)
             return
-        arr = self._host_argument(view, value)
-        src = torch.from_numpy(np.array(arr.reshape(-1), copy=not arr.flags.writeable))
+        src = self._host_tensor(self._host_argument(view, value))
         async_ok = src.is_pinned()
         if not buf.flex:
             buf.tensor.copy_(src, non_blocking=async_ok)
@@ -1964,6 +1963,14 @@ class B200Transformer(object):
         if buf.staging is None:
             buf.staging = torch.empty((max(buf.size, 1),), dtype=torch.float32, device=self.device)
         buf.staging.copy_(src, non_blocking=async_ok)
+
+    def _host_tensor(self, arr):
+        """A flat tensor over the memory of a contiguous fp32 array, to copy from.  (torch warns about
+        arrays that are read-only; nothing here writes to them.)"""
+        if not arr.flags.writeable and arr.nbytes:
+            memory = (ctypes.c_char * arr.nbytes).from_address(arr.__array_interface__["data"][0])
+            arr = np.frombuffer(memory, dtype=np.float32)
+        return self.torch.from_numpy(arr.reshape(-1))
 
     def _device_argument(self, view, value):
         """A tensor that already lives on the device (the reference's DeviceTensor.__setitem__

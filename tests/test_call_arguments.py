@@ -9,7 +9,7 @@ import ngraph_python_b200 as ng
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("rows, cols", [(512, 512), (300, 1001), (1, 262144), (64, 4096)])
+@pytest.mark.parametrize("rows, cols", [(512, 512), (300, 1001), (1, 262144), (64, 4096), (1200, 1024)])
 def test_device_arguments_in_place(rows, cols):
     import torch
     A, B = ng.make_axis(rows, name="A"), ng.make_axis(cols, name="B")
@@ -40,6 +40,11 @@ def test_device_arguments_in_place(rows, cols):
     check(values(3, extra=1))                                 # not 16-byte aligned
     check(np.random.RandomState(4).rand(rows, cols).astype(np.float32))
     check(values(5).double())                                 # converted on the way
+    for pinned in (False, True):
+        v = torch.rand((rows, cols), generator=torch.Generator().manual_seed(8))
+        v = (v.pin_memory() if pinned else v).numpy()
+        v.flags.writeable = False
+        check(v)
     v = values(6)                                             # unrecorded, after recorded calls
     np.testing.assert_array_equal(third(v), v.cpu().numpy().max(axis=1))
     check(values(7))
