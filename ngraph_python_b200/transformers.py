@@ -13,6 +13,7 @@ device raises.
 """
 import collections
 import ctypes
+import gc
 import math
 import numbers
 
@@ -336,6 +337,10 @@ class Computation(object):
                 if s.recorded_kernel is None:
                     s.recorded_kernel = lib.EwKernel(s.recorded_program)
                 s.recorded_kernel.prepare(*t._ew_pointers(s, recorded=True))
+        # A graph of an earlier computation that the collector finds now would be destroyed in the
+        # middle of the recording, which ends it with an error.
+        collecting = gc.isenabled()
+        gc.disable()
         try:
             for seg in segments:
                 if all(s.launches == 0 for s in seg["steps"]):
@@ -357,6 +362,8 @@ class Computation(object):
                         io_in_graph = True
                 seg["graph"] = g
         finally:
+            if collecting:
+                gc.enable()
             t._recording = t._recording_call = False
         per_call = t.kernel_launches - before
         self._graphs = [seg["graph"] for seg in segments]

@@ -274,3 +274,39 @@ def test_tracing_writes_a_chrome_trace(tmp_path, monkeypatch):
     assert {e["cat"] for e in trace} >= {"conv", "ew", "gemm"}
     ts = [e["ts"] for e in trace]
     assert ts == sorted(ts)
+
+
+def test_recording_beside_garbage_that_holds_graphs(monkeypatch):
+    """Computations that nothing refers to any more hold their graphs in cycles until the collector
+    runs; it must not run, and destroy them, while another computation is recorded."""
+    import gc
+    from ngraph_python_b200 import transformers
+
+    def computed(n):
+        A = ng.make_axis(n, name="A")
+        x = ng.placeholder([A])
+        comp = ng.transformers.allocate_transformer("b200").computation(
+            [ng.exp(x) + 1.0, ng.sum(x, reduction_axes=[A])], x)
+        comp(np.ones(n, np.float32))
+        return comp
+    place = transformers._CallIO.record_inputs
+
+    def collect_where_allowed(self):
+        place(self)
+        if gc.isenabled():
+            gc.collect()
+    before = gc.get_threshold()
+    try:
+        gc.set_threshold(1000000)            # the garbage is there until collect_where_allowed
+        comp = computed(3)
+        comp.capture()
+        cycle = [comp]
+        cycle.append(cycle)
+        del comp, cycle
+        comp = computed(5)
+        monkeypatch.setattr(transformers._CallIO, "record_inputs", collect_where_allowed)
+        comp.capture()
+        assert gc.isenabled()
+        np.testing.assert_allclose(comp(np.full(5, 2.0, np.float32))[1], 10.0)
+    finally:
+        gc.set_threshold(*before)
