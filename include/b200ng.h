@@ -125,6 +125,8 @@ int b2_ew_compile(const b2_ew_program* prog, b2_ew_kernel** out_kernel);
  * build-time check of a program.  `vec` asks for the 128-bit variant where the program allows
  * it; the generated source is copied to `source` when given. */
 int b2_ew_check(const b2_ew_program* prog, int vec, int probe, char* source, size_t source_cap);
+/* The same for the form that shares a launch with others (b2_ew_launch_many). */
+int b2_ew_check_joint(const b2_ew_program* prog, int vec, char* source, size_t source_cap);
 /* Bytes of caller-provided scratch a launch needs (0 for most programs; reductions of a few
  * very long rows are split across CTAs and combined from scratch). */
 int b2_ew_scratch_bytes(const b2_ew_kernel* k, size_t* bytes);

@@ -459,7 +459,11 @@ int generate(const b2_ew_program& p, const Plan& pl, bool probe, std::string* ou
         o << "    int at_job = 0;\n"
           << "    while (at_job + 1 < jobs.n && (int)blockIdx.x >= jobs.first[at_job + 1]) ++at_job;\n"
           << "    const b2_ew_args& p = jobs.job[at_job];\n"
-          << "    const int first_block = jobs.first[at_job], end_block = jobs.first[at_job + 1];\n";
+          // one row to a program: its blocks lie along x
+          << "    const b2_i64 block_x = (int)blockIdx.x - jobs.first[at_job], blocks_x = jobs.first[at_job + 1] - jobs.first[at_job];\n"
+          << "    const b2_i64 block_y = 0, blocks_y = 1;\n";
+    else
+        o << "    const b2_i64 block_x = blockIdx.x, blocks_x = gridDim.x, block_y = blockIdx.y, blocks_y = gridDim.y;\n";
     emit_prologue(o, p, probe);
     for (int i = 0; i < p.n_in; ++i)
         if (p.in[i].dtype == B2_F32_AT)
@@ -473,7 +477,7 @@ int generate(const b2_ew_program& p, const Plan& pl, bool probe, std::string* ou
           << "    const b2_i64 chunks = p.C / V;\n"
           << "    const int grp = threadIdx.x / GROUP, gl = threadIdx.x % GROUP;\n"
           << "    const int RPC = THREADS / GROUP;\n"
-          << "    for (b2_i64 r = (b2_i64)blockIdx.y * RPC + grp; r < rows; r += (b2_i64)gridDim.y * RPC) {\n"
+          << "    for (b2_i64 r = block_y * RPC + grp; r < rows; r += blocks_y * RPC) {\n"
           << "        const b2_i64 a_idx = r / p.B, b_idx = r - a_idx * p.B;\n";
         for (int i = 0; i < p.n_in; ++i) {
             const char* ct = ctype(p.in[i].dtype);
@@ -496,8 +500,8 @@ int generate(const b2_ew_program& p, const Plan& pl, bool probe, std::string* ou
               << ">();\n";
             if (is_arg(p.out[k].redop)) o << "        int idx" << k << " = 0x7fffffff;\n";
         }
-        o << "        b2_i64 j = (b2_i64)blockIdx.x * GROUP + gl;\n"
-          << "        const b2_i64 jstep = (b2_i64)gridDim.x * GROUP;\n";
+        o << "        b2_i64 j = block_x * GROUP + gl;\n"
+          << "        const b2_i64 jstep = blocks_x * GROUP;\n";
         for (int i = 0; i < p.n_in; ++i)
             if (prefetchable(p.in[i], pl))
                 o << "        " << raw_type(p.in[i].dtype, pl.V) << " w" << i << " = {}, n" << i
@@ -563,7 +567,7 @@ int generate(const b2_ew_program& p, const Plan& pl, bool probe, std::string* ou
             o << "        if (gl == 0) {\n";
             for (int k = p.n_out; k < nres; ++k) {
                 if (split) {
-                    o << "            p.scratch[((b2_i64)blockIdx.x * rows + r) * NRED + "
+                    o << "            p.scratch[(block_x * rows + r) * NRED + "
                       << (k - p.n_out) << "] = acc" << k << ";\n";
                 } else {
                     const std::string val = is_arg(p.out[k].redop)
@@ -580,9 +584,9 @@ int generate(const b2_ew_program& p, const Plan& pl, bool probe, std::string* ou
     } else {
         // REDUCE_B: threads run along C, every thread walks the B axis.
         o << "    const b2_i64 chunks = p.C / V;\n"
-          << "    for (b2_i64 a_idx = blockIdx.y; a_idx < p.A; a_idx += gridDim.y)\n"
-          << "    for (b2_i64 j = (b2_i64)blockIdx.x * THREADS + threadIdx.x; j < chunks; "
-             "j += (b2_i64)gridDim.x * THREADS) {\n"
+          << "    for (b2_i64 a_idx = block_y; a_idx < p.A; a_idx += blocks_y)\n"
+          << "    for (b2_i64 j = block_x * THREADS + threadIdx.x; j < chunks; "
+             "j += blocks_x * THREADS) {\n"
           << "        const b2_i64 c = j * V;\n";
         for (int k = p.n_out; k < nres; ++k) {
             o << "        float acc" << k << "[V];\n";
@@ -660,18 +664,6 @@ int generate(const b2_ew_program& p, const Plan& pl, bool probe, std::string* ou
 
     if (split) emit_finalize(o, p, probe);
     *out_src = o.str();
-    if (many) {
-        // one row to a program: its blocks lie along x
-        auto put = [&](const char* what, const char* with) {
-            const size_t from = out_src->find("const b2_ew_args& p = jobs");
-            for (size_t i = from; (i = out_src->find(what, i)) != std::string::npos; i += strlen(with))
-                out_src->replace(i, strlen(what), with);
-        };
-        put("(b2_i64)blockIdx.x", "(b2_i64)((int)blockIdx.x - first_block)");
-        put("(b2_i64)gridDim.x", "(b2_i64)(end_block - first_block)");
-        put("(b2_i64)blockIdx.y", "(b2_i64)0");
-        put("(b2_i64)gridDim.y", "(b2_i64)1");
-    }
     return B2_OK;
 }
 
@@ -1054,6 +1046,22 @@ extern "C" int b2_set_nvrtc_path(const char* path) {
     return B2_OK;
 }
 
+namespace {
+int check_source(const std::string& src, char* source, size_t source_cap) {
+    if (source && source_cap) {
+        strncpy(source, src.c_str(), source_cap - 1);
+        source[source_cap - 1] = '\0';
+    }
+    std::vector<char> cubin;
+    std::lock_guard<std::mutex> lock(g_mutex);
+    return nvrtc_compile(src, &cubin);
+}
+
+bool joint_form(const b2_ew_program& p, const Plan& pl) {
+    return p.reduce_mode == B2_REDUCE_NONE && p.A * p.B == 1 && !pl.staged;
+}
+}  // namespace
+
 extern "C" int b2_ew_check(const b2_ew_program* prog, int vec, int probe, char* source,
                            size_t source_cap) {
     B2_REQUIRE(prog, "null argument");
@@ -1064,17 +1072,19 @@ extern "C" int b2_ew_check(const b2_ew_program* prog, int vec, int probe, char* 
     bool has_final = false;
     rc = pl.staged ? generate_staged(*prog, pl, probe != 0, &src, &has_final)
                    : generate(*prog, pl, probe != 0, &src, &has_final);
+    return rc ? rc : check_source(src, source, source_cap);
+}
+
+extern "C" int b2_ew_check_joint(const b2_ew_program* prog, int vec, char* source, size_t source_cap) {
+    B2_REQUIRE(prog, "null argument");
+    int rc = validate(*prog);
     if (rc) return rc;
-    if (source && source_cap) {
-        strncpy(source, src.c_str(), source_cap - 1);
-        source[source_cap - 1] = '\0';
-    }
-    std::vector<char> cubin;
-    {
-        std::lock_guard<std::mutex> lock(g_mutex);
-        rc = nvrtc_compile(src, &cubin);
-    }
-    return rc;
+    const Plan pl = make_plan(*prog, vec != 0);
+    B2_REQUIRE(joint_form(*prog, pl), "this program is launched by itself");
+    std::string src;
+    bool has_final = false;
+    rc = generate(*prog, pl, false, &src, &has_final, true);
+    return rc ? rc : check_source(src, source, source_cap);
 }
 
 extern "C" int b2_ew_compile(const b2_ew_program* prog, b2_ew_kernel** out_kernel) {
@@ -1249,8 +1259,7 @@ extern "C" int b2_ew_launch(b2_ew_kernel* k, const void* const* in, void* const*
 // ------------------------------------------------------------------------------------------------
 namespace {
 bool goes_with_others(const b2_ew_kernel* k, int vec) {
-    const b2_ew_program& p = k->prog;
-    return p.reduce_mode == B2_REDUCE_NONE && p.A * p.B == 1 && !k->plan[vec].staged &&
+    return joint_form(k->prog, k->plan[vec]) &&
            k->plan[vec].grid.x <= 4 * kSMs;       // (larger ones fill the machine by themselves)
 }
 }  // namespace

@@ -123,6 +123,7 @@ def _load():
         "b2_device_count": (C.c_int, []),
         "b2_set_nvrtc_path": (C.c_int, [C.c_char_p]),
         "b2_ew_check": (C.c_int, [C.POINTER(EwProgram), C.c_int, C.c_int, C.c_char_p, sz]),
+        "b2_ew_check_joint": (C.c_int, [C.POINTER(EwProgram), C.c_int, C.c_char_p, sz]),
         "b2_ew_compile": (C.c_int, [C.POINTER(EwProgram), C.POINTER(vp)]),
         "b2_ew_scratch_bytes": (C.c_int, [vp, C.POINTER(sz)]),
         "b2_ew_prepare": (C.c_int, [vp, C.POINTER(vp), C.POINTER(vp)]),
@@ -287,9 +288,13 @@ def make_program(dims, inputs, consts, ops, outs, reds, reduce_mode):
     return p
 
 
-def ew_check(prog, vec=True, probe=False, want_source=False):
+def ew_check(prog, vec=True, probe=False, want_source=False, joint=False):
     buf = C.create_string_buffer(1 << 18) if want_source else None
-    check(_lib.b2_ew_check(C.byref(prog), int(vec), int(probe), buf, len(buf) if buf else 0))
+    size = len(buf) if buf else 0
+    if joint:
+        check(_lib.b2_ew_check_joint(C.byref(prog), int(vec), buf, size))
+    else:
+        check(_lib.b2_ew_check(C.byref(prog), int(vec), int(probe), buf, size))
     return buf.value.decode() if buf else None
 
 

@@ -88,3 +88,25 @@ def test_argument_in_place_is_not_stored_onto_itself(mode, vec):
     stores = [m.start() for m in re.finditer(r"b2_st4_cs\(o1|o1\[\(c", body)]
     assert len(stores) == 1 and body.rindex("if (put1) {", 0, stores[0]) > body.rindex("}", 0, stores[0])
     assert "put" not in lib.ew_check(prog, vec=bool(vec), probe=True, want_source=True).split("b2_ew_main")[1]
+
+
+@pytest.mark.parametrize("joint", (False, True))
+@pytest.mark.parametrize("vec", (0, 1))
+@pytest.mark.parametrize("mode", (lib.REDUCE_NONE, lib.REDUCE_C, lib.REDUCE_B))
+def test_a_block_finds_its_place_in_one_line(mode, vec, joint):
+    """Blocks of a joint launch belong to one program each: nothing but the line that says where a block
+    stands may look at the grid, in either form."""
+    if joint and mode != lib.REDUCE_NONE:
+        return
+    dims = (1, 1, 4096) if joint else (2, 6, 4096)
+    ins = [dict(dtype=lib.FLEX16, slot=0, strides=(6 * 4096, 4096, 1))]
+    outs = [dict(dtype=lib.F32, strides=(6 * 4096, 4096, 1), reg=1)]
+    reds = {lib.REDUCE_NONE: [], lib.REDUCE_C: [(6, 1, 0)], lib.REDUCE_B: [(4096, 0, 1)]}[mode]
+    reds = [dict(dtype=lib.F32, strides=st, reg=1, redop="sum") for st in reds]
+    prog = lib.make_program(dims, ins, [], [("exp", 0, None)], outs, reds, mode)
+    src = lib.ew_check(prog, vec=bool(vec), want_source=True, joint=joint)
+    main = src[src.index("b2_ew_main"):].split("b2_ew_finalize")[0]
+    lines = [line for line in main.splitlines() if "blockIdx" in line or "gridDim" in line]
+    assert len(lines) == (2 if joint else 1) and "block_x = " in lines[-1]
+    assert not joint or "jobs.first[at_job + 1]) ++at_job" in lines[0]
+    assert ("blocks_y = 1" in main) == joint
