@@ -2198,7 +2198,7 @@ extern "C" int b2_conv_launches(int32_t flex, const b2_conv_dims* d, int32_t pas
     UpdShape u;
     b2_update_f32 f32;
     if (pass == 2)
-        *launches = update_f32_scratch(mode, g, &f32) ? 2 : !update_goes_in_planes(mode, g, &u) && update_shape(mode, g).splits > 1 ? 4 : 3;
+        *launches = update_f32_scratch(mode, g, &f32) ? b2_update_f32_launches(f32) : !update_goes_in_planes(mode, g, &u) && update_shape(mode, g).splits > 1 ? 4 : 3;
     else
         *launches = !(flex && pass_geom(g, pass, &gp)) && conv_goes_direct(mode, g, pass, &direct) ? 1 : 3;
     return B2_OK;

@@ -7,7 +7,11 @@
 // rows (32 images: 128 contiguous bytes), split them into two tf32 planes and store them into a ring;
 // a ninth issues the products.  A slice of at most 16 k-blocks goes to each CTA (the tensor core's fp32
 // sum truncates: a longer chain would lose what 3xTF32 gains); its sums go to partial[slice], which
-// update_f32_finish_kernel adds in slice order.
+// update_f32_finish_kernel adds in slice order.  A slice's sums are a copy of the filters, and slices are
+// as many as the pixels and images ask for, so they go in rounds of what kScratchMost holds: 512 -> 512
+// channels, 3x3, 56x56 pixels of 256 images have 784 slices, 7.4 GB at once, in 28 rounds (of 11648 CTAs
+// each, 79 to an SM, so that the ends of the rounds cost little).  512 -> 512 channels, 3x3, 28x28 pixels
+// of 128 images: 10.59 ms with 1.8 GB of slices, 10.39 in seven rounds.
 //
 // What bounds it: the producers' issue slots, so a window is loaded once for up to four pixels.  The
 // unrolled planes and their product took 1.4 ms of a batch-128 training step of ResNet-14.
@@ -19,7 +23,7 @@ struct UpdF32Params {
     b2_update_f32 g;
     const float *I, *E;
     float* partial;                    // [slice][C*R*S][K]
-    int gh, gw, wh, ww, cu, ntn, kt, tw, nblk, nkb, per;
+    int gh, gw, wh, ww, cu, ntn, kt, tw, nblk, nkb, per, slice0;
     int vec;                           // rows start on 16-byte boundaries
     int* status;
 };
@@ -42,7 +46,7 @@ conv_update_f32_kernel(const __grid_constant__ UpdF32Params p) {
     const int warp = warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
     const b2_update_f32& g = p.g;
     const int chunk = blockIdx.y / p.ntn, ktile = blockIdx.y - chunk * p.ntn;
-    const int kb0 = blockIdx.x * p.per, nkb = min(p.per, p.nkb - kb0);
+    const int kb0 = (p.slice0 + blockIdx.x) * p.per, nkb = min(p.per, p.nkb - kb0);
     const int win = p.wh * p.ww, npix = p.gh * p.gw;
 
     if (threadIdx.x == 0) {
@@ -188,9 +192,9 @@ conv_update_f32_kernel(const __grid_constant__ UpdF32Params p) {
 }
 
 // Sum of the slices, in a fixed order: a block has 32 outputs, warp w adds the slices w, w+8, ... (four
-// loads in flight), then the eight sums are added in warp order.
+// loads in flight), then the eight sums are added in warp order.  add: to what earlier rounds left.
 __global__ void __launch_bounds__(256)
-update_f32_finish_kernel(const float* __restrict__ partial, float* __restrict__ U, int n, int slices) {
+update_f32_finish_kernel(const float* __restrict__ partial, float* __restrict__ U, int n, int slices, int add) {
     after_earlier_kernels();
     __shared__ float part[8][32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, i = blockIdx.x * 32 + lane;
@@ -211,11 +215,13 @@ update_f32_finish_kernel(const float* __restrict__ partial, float* __restrict__ 
     if (w == 0 && i < n) {
 #pragma unroll
         for (int j = 1; j < 8; ++j) v += part[j][lane];
-        U[i] = v;
+        U[i] = add ? U[i] + v : v;
     }
 }
 
-struct UpdF32Shape { bool ok; int gh, gw, wh, ww, cu, cchunks, ntn, kt, bn, tw, nblk, nkb, per, nsplit; long long cost; };
+const size_t kScratchMost = 256u << 20;
+
+struct UpdF32Shape { bool ok; int gh, gw, wh, ww, cu, cchunks, ntn, kt, bn, tw, nblk, nkb, per, nsplit, round; long long cost; };
 
 UpdF32Shape update_f32_shape_for(const b2_update_f32& g, int gh, int gw) {
     UpdF32Shape u = {};
@@ -240,7 +246,10 @@ UpdF32Shape update_f32_shape_for(const b2_update_f32& g, int gh, int gw) {
     slices *= (per + 15) / 16;
     u.per = (int)((nkb + slices - 1) / slices);
     u.nsplit = (int)((nkb + u.per - 1) / u.per);
-    if ((long long)u.nsplit * g.C * g.R * g.S * g.K >= (1LL << 31)) return u;
+    const long long filters = (long long)g.C * g.R * g.S * g.K;
+    if (u.nsplit * filters >= (1LL << 31)) return u;
+    const long long fit = (long long)(kScratchMost / 4) / filters;
+    u.round = fit < 1 ? 1 : fit < u.nsplit ? (int)fit : u.nsplit;
     // cycles: the producers' 7 a row of a k-block (two CTAs of an SM share them), the sums' way out
     const long long waves = (cols * u.nsplit + slots - 1) / slots;
     u.cost = waves * ((long long)u.per * (300 + 7 * (128 + u.bn) * (slots / 148)) + 6000 + 60 * u.bn) +
@@ -260,7 +269,7 @@ UpdF32Shape update_f32_shape(const b2_update_f32& g) {
 }
 
 template <int BN>
-int launch_update_f32(const UpdF32Params& p, const UpdF32Shape& u, cudaStream_t st) {
+int launch_update_f32(const UpdF32Params& p, const UpdF32Shape& u, int slices, cudaStream_t st) {
     static_assert(dir_ring_bytes(BN) >= 128 * (BN + 1) * 4, "the sums fit the ring");
     const int smem = 1024 + dir_ring_bytes(BN) + 128;
     static bool attr_set = false;
@@ -268,7 +277,7 @@ int launch_update_f32(const UpdF32Params& p, const UpdF32Shape& u, cudaStream_t 
         B2_CUDA(cudaFuncSetAttribute(conv_update_f32_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
         attr_set = true;
     }
-    B2_CUDA(b2::launch_after(conv_update_f32_kernel<BN>, dim3(u.nsplit, u.cchunks * u.ntn), kDirThreads, smem, st, p));
+    B2_CUDA(b2::launch_after(conv_update_f32_kernel<BN>, dim3(slices, u.cchunks * u.ntn), kDirThreads, smem, st, p));
     return B2_OK;
 }
 
@@ -276,7 +285,12 @@ int launch_update_f32(const UpdF32Params& p, const UpdF32Shape& u, cudaStream_t 
 
 size_t b2_update_f32_scratch(const b2_update_f32& g) {
     const UpdF32Shape u = update_f32_shape(g);
-    return u.ok ? (((size_t)u.nsplit * g.C * g.R * g.S * g.K * 4) + 1023) / 1024 * 1024 : 0;
+    return u.ok ? (((size_t)u.round * g.C * g.R * g.S * g.K * 4) + 1023) / 1024 * 1024 : 0;
+}
+
+int b2_update_f32_launches(const b2_update_f32& g) {
+    const UpdF32Shape u = update_f32_shape(g);
+    return !u.ok ? 0 : u.nsplit == 1 ? 1 : 2 * ((u.nsplit + u.round - 1) / u.round);
 }
 
 int b2_update_f32_launch(const b2_update_f32& g, const float* I, const float* E, float* U, void* scratch,
@@ -288,16 +302,19 @@ int b2_update_f32_launch(const b2_update_f32& g, const float* I, const float* E,
     p.gh = u.gh; p.gw = u.gw; p.wh = u.wh; p.ww = u.ww; p.cu = u.cu; p.ntn = u.ntn; p.kt = u.kt;
     p.tw = u.tw; p.nblk = u.nblk; p.nkb = u.nkb; p.per = u.per; p.status = status;
     p.vec = g.N % 4 == 0 && (((uintptr_t)I | (uintptr_t)E) & 15) == 0;
-    int rc;
-    switch (u.bn) {
-        case 16: rc = launch_update_f32<16>(p, u, st); break;
-        case 32: rc = launch_update_f32<32>(p, u, st); break;
-        case 64: rc = launch_update_f32<64>(p, u, st); break;
-        default: rc = launch_update_f32<128>(p, u, st); break;
-    }
-    if (rc || u.nsplit == 1) return rc;
     const int n = g.C * g.R * g.S * g.K;
-    B2_CUDA(b2::launch_after(update_f32_finish_kernel, dim3((n + 31) / 32), 256, 0, st, (const float*)scratch, U, n,
-                             u.nsplit));
+    for (p.slice0 = 0; p.slice0 < u.nsplit; p.slice0 += u.round) {
+        const int slices = u.nsplit - p.slice0 < u.round ? u.nsplit - p.slice0 : u.round;
+        int rc;
+        switch (u.bn) {
+            case 16: rc = launch_update_f32<16>(p, u, slices, st); break;
+            case 32: rc = launch_update_f32<32>(p, u, slices, st); break;
+            case 64: rc = launch_update_f32<64>(p, u, slices, st); break;
+            default: rc = launch_update_f32<128>(p, u, slices, st); break;
+        }
+        if (rc || u.nsplit == 1) return rc;
+        B2_CUDA(b2::launch_after(update_f32_finish_kernel, dim3((n + 31) / 32), 256, 0, st, (const float*)scratch, U, n,
+                                 slices, p.slice0 > 0 ? 1 : 0));
+    }
     return B2_OK;
 }

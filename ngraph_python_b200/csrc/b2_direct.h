@@ -57,6 +57,7 @@ __attribute__((visibility("hidden"))) int b2_direct_launch(const b2_direct_args&
 // fp32 filter gradient (b2_conv_update_f32.cu): no dilation, one depth.  Scratch 0: not taken.
 struct b2_update_f32 { int C, H, W, N, K, R, S, P, Q, pad_h, pad_w, str_h, str_w; };
 __attribute__((visibility("hidden"))) size_t b2_update_f32_scratch(const b2_update_f32& g);
+__attribute__((visibility("hidden"))) int b2_update_f32_launches(const b2_update_f32& g);
 __attribute__((visibility("hidden"))) int b2_update_f32_launch(const b2_update_f32& g, const float* I, const float* E,
                                                                float* U, void* scratch, int* status, cudaStream_t st);
 #endif  // B2_DIRECT_H

@@ -83,3 +83,34 @@ def test_fp32_convolution_passes(case):
             want = gx.permute(1, 2, 3, 0) + (0 if res is None else res.double())
             close(out.cpu().double(), want if mask is None else want * (mask > 0))
     assert int(status.item()) == 0
+
+
+def test_filter_gradient_in_rounds():
+    """More slices than the scratch holds at once: 28 copies of the filters fit, five rounds."""
+    import torch
+    Cc, side, N, K = 512, 32, 64, 512
+    d = lib.ConvDims()
+    for k, v in dict(C=Cc, D=1, H=side, W=side, N=N, K=K, T=1, R=3, S=3, M=1, P=side, Q=side, pad_h=1, pad_w=1,
+                     str_d=1, str_h=1, str_w=1, dil_d=1, dil_h=1, dil_w=1).items():
+        setattr(d, k, v)
+    size = lib.conv_update_scratch_bytes(False, d)
+    launches = lib.conv_launches(False, d, lib.CONV_UPDATE)
+    assert size <= 256 << 20 and launches == 10
+    g = torch.Generator(device="cuda").manual_seed(5)
+    x = torch.randn((Cc, side, side, N), device="cuda", generator=g)
+    e = torch.randn((K, side, side, N), device="cuda", generator=g)
+    scratch = torch.empty((size + 2048,), dtype=torch.uint8, device="cuda").fill_(77)
+    off = -scratch.data_ptr() % 1024
+    out = torch.full((Cc, 3, 3, K), 7.0, device="cuda")
+    status = torch.zeros((1,), dtype=torch.int32, device="cuda")
+    for _ in range(2):                               # the second call on what the first left
+        lib.check(lib.raw().b2_conv_update_f32(x.data_ptr(), e.data_ptr(), out.data_ptr(), C.byref(d),
+                                               scratch.data_ptr() + off, size, status.data_ptr(), 0))
+    torch.cuda.synchronize()
+    assert int(status.item()) == 0 and bool((scratch[off + size:] == 77).all())
+    padded = torch.nn.functional.pad(x.double(), (0, 0, 1, 1, 1, 1))
+    ed = e.double().reshape(K, -1)
+    for r in range(3):
+        for s in range(3):
+            want = padded[:, r:r + side, s:s + side].reshape(Cc, -1) @ ed.T
+            assert (out[:, r, s].double() - want).abs().max() <= 4e-6 * want.abs().max()

@@ -186,3 +186,23 @@ def test_slices_of_a_product_fit_the_machine(flex):
                     assert waves == 1 and m * n <= {2: 33, 3: 22, 4: 15}[slices], (K, m, n)
                     taken.add(slices)
     assert taken == {2, 3, 4}
+
+
+def _square_layer(C, K, side, N):
+    d = lib.ConvDims()
+    for k, v in dict(C=C, D=1, H=side, W=side, N=N, K=K, T=1, R=3, S=3, M=1, P=side, Q=side, pad_h=1, pad_w=1,
+                     str_d=1, str_h=1, str_w=1, dil_d=1, dil_h=1, dil_w=1).items():
+        setattr(d, k, v)
+    return d
+
+
+def test_filter_gradient_scratch_is_bounded():
+    """fp32 filter gradients hold 256 MB of slices at most, or one copy of larger filters, in as many
+    rounds as that takes; what fits is done in one."""
+    most = 256 << 20
+    for C, K, side, N, rounds in ((512, 512, 56, 256, 28), (512, 512, 14, 256, 4), (64, 64, 56, 256, 1), (3, 64, 224, 256, 1)):
+        d = _square_layer(C, K, side, N)
+        assert lib.conv_update_scratch_bytes(False, d) <= most
+        assert lib.conv_launches(False, d, lib.CONV_UPDATE) == 2 * rounds, (C, K, side, N)
+    d = _square_layer(3000, 3000, 14, 32)          # 324 MB of filters
+    assert lib.conv_update_scratch_bytes(False, d) < 4 * 9 * 3000 * 3000 + 1024
