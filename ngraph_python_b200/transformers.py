@@ -11,6 +11,7 @@ libb200ng.so; PyTorch only provides device memory, streams and pinned host buffe
 There is no CPU path: constructing the transformer without the shared library or without a CUDA
 device raises.
 """
+import bisect
 import collections
 import ctypes
 import gc
@@ -430,6 +431,10 @@ class _CallIO(object):
             if 4 * v.buffer.size <= 1 << 20:
                 self._pinned_buffer(k)
         self.visible = ctypes.c_void_p()
+        # what the computation writes: an argument that lies there is copied before anything runs
+        written = set(v.buffer for s in comp.steps for v in s.out_views)
+        written.update(v.buffer for v in views)
+        self.written = sorted((b.ptr(), b.ptr() + b.tensor.nbytes) for b in written)
         # results: small dense ones ride in the last node, the others are copied after it
         self.outputs, self.later, budget = [], [], self.RESULTS_MOST
         self.results = []               # (pinned array, view) or None, in the order of the returns
@@ -468,6 +473,11 @@ class _CallIO(object):
     def ready(self):
         """False while an argument has no exponent yet: its range has to be measured first."""
         return all(v.buffer.entry.initialized for v in self.flex_views)
+
+    def _stays_as_it_is(self, address, nbytes):
+        """Whether no kernel of the computation writes to this memory."""
+        at = bisect.bisect_left(self.written, (address + nbytes,))
+        return at == 0 or self.written[at - 1][1] <= address
 
     def _source(self, k, value):
         """(address the device can read argument k's fp32 values from, object to keep alive);
@@ -509,7 +519,9 @@ class _CallIO(object):
                 block.arg[k].src = address
                 # a device tensor is read where it lies by the kernel that uses it first, which
                 # also stores it
-                block.arg[k].in_place = address % 16 == 0 and isinstance(obj, t.torch.Tensor)
+                block.arg[k].in_place = (
+                    self.views[k].buffer.where is not None and isinstance(obj, t.torch.Tensor) and
+                    address % 16 == 0 and self._stays_as_it_is(address, obj.nbytes))
                 keep.append(obj)
             t._begin_call(comp, self)
             for k, v in enumerate(self.views):

@@ -71,3 +71,27 @@ def test_recorded_kernel_beside_an_unaligned_operand():
         np.testing.assert_array_equal(comp(v), v.cpu().numpy() * w[1:])
         np.testing.assert_array_equal(np.asarray(t.get_tensor_view_value(x)), v.cpu().numpy())
     t.close()
+
+
+def test_argument_that_the_computation_writes():
+    """The caller's tensor is what a kernel before the argument's first reader writes: the argument is
+    what the tensor held when the call was made, recorded or not."""
+    A, B = ng.make_axis(512, name="A"), ng.make_axis(512, name="B")
+    x = ng.placeholder([A, B])
+    y = ng.variable([A, B], initial_value=np.ones((512, 512), np.float32))
+    doubled = ng.assign(y, y * 2.0)
+    total = ng.sum(y, reduction_axes=[A, B])
+    t = ng.transformers.allocate_transformer("b200")
+    comp = t.computation(ng.sequential([doubled, total, x + total]), x)
+    comp(np.zeros((512, 512), np.float32))                    # y = 2
+    held = t.device_tensor(y).view.buffer.tensor
+    assert len([s for s in comp.steps if s.kind == "ew"]) > 1
+
+    def check(value):
+        np.testing.assert_array_equal(comp(held), np.full((512, 512), value + 2 * value * 512 * 512, np.float32))
+    check(2.0)
+    comp.capture()
+    check(4.0)
+    check(8.0)
+    assert comp.steps[-1].stores_argument
+    t.close()
