@@ -289,14 +289,14 @@ im2col_planes_kernel(const T* __restrict__ I, ConvGeom g, int rows, int kg, int 
 // ================================================================================================
 // Implicit GEMM (flex16): no unrolled copy of the input.
 //
-// For batches that are a multiple of 128 the tile kernel reads the activations straight from
-// their C,H,W,N layout.  A tile is one output pixel (p,q) x 128 images; its reduction runs over
-// chunks of `cu` input channels.  For every chunk ONE 4-d TMA box [cu channels][R][S][128 images]
-// per operand plane is fetched at (n0, q*str - pad, p*str - pad, c0): the whole filter window of
-// those channels in a single copy, zero fill outside the image doing the padding.  It lands in
-// shared memory as an MN-major (images contiguous) 128-byte-swizzled operand whose K rows are in
-// (channel, r, s) order -- the natural order of the C,R,S,K filter tensor -- padded to a multiple
-// of 32 rows (one MMA step).
+// The tile kernel reads the activations straight from their C,H,W,N layout, rows of images padded to 16
+// bytes (any batch; images beyond it are zero fill).  A tile is 1x1 to 2x2 output pixels x 128 images;
+// its reduction runs over chunks of `cu` input channels.  For every chunk ONE 4-d TMA box [cu channels]
+// [window][128 images] per operand plane is fetched: the window under all pixels of the tile in a single
+// copy, zero fill outside the image doing the padding.  It lands in shared memory as an MN-major (images
+// contiguous) 128-byte-swizzled operand whose K rows are in (channel, row, column of the window) order,
+// padded to a multiple of 32 rows (one MMA step).  Each pixel has columns of its own, whose filters stand
+// at its place in the window and are zero elsewhere.
 //
 // At 16..64 output channels an MMA's time is the read of its A operand from shared memory (4 KB
 // per instruction whatever N is), so the four byte products are folded into TWO instructions per
@@ -1193,8 +1193,8 @@ ImplicitShape implicit_shape(const ConvGeom& g) {
 
 // flex16 only: an MN-major tf32 operand needs the 32-byte-atom variant of the 128-byte swizzle
 // (both in the tensor map and in the matrix descriptor); with the plain 128-byte swizzle the
-// tensor core reads zeros.  fp32 convolutions therefore stay on the gather + K-major path, and so
-// do dilated filters and windows too large for two stages of shared memory.
+// tensor core reads zeros.  fp32 convolutions therefore gather K-major operands (direct_kernel, or the
+// unrolled planes), and so do dilated filters and windows too large for two stages of shared memory.
 bool implicit_ok(int mode, const ConvGeom& g) {
     if (mode != MODE_FLEX16 || g.dil_h != 1 || g.dil_w != 1 || getenv("B2_CONV_IM2COL")) return false;
     if (!flat_depth(g)) return false;

@@ -9,10 +9,10 @@
 //              into a ring of stages; afterwards the epilogue;
 //   warp 8:    tensor memory, tcgen05.mma issue.
 // A k-block is 128 bytes of plane: 32 fp32 or 128 int16 values.
-//   fp32:   3xTF32.  B's planes lie behind one another and make one operand of 2*BN rows:
-//           A_hi x [B_hi | B_lo] -> [hh | x], A_lo x B_hi -> x.  Convolutions keep the two sums apart
-//           until the end, matrix products have one (see ONE_CHAIN); a chain runs over at most 16 k-blocks (the tensor core's fp32 sum truncates), longer
-//           K is cut into slices.
+//   fp32:   3xTF32, in chains of at most 16 k-blocks (the tensor core's fp32 sum truncates); longer K
+//           is cut into slices.  Matrix products add hi*hi, hi*lo and lo*hi into one sum (see ONE_CHAIN).
+//           Convolutions keep two: B's planes lie behind one another and make one operand of 2*BN rows,
+//           A_hi x [B_hi | B_lo] -> [hh | x], A_lo x B_hi -> x.
 //   flex16: four exact int8 products, HH | X | LL as in b2_gemm_impl.cuh.
 // Slices of K: the CTAs of a cluster (up to 8) take one each; partial sums meet in distributed shared
 // memory, every CTA adds a share of the columns in slice order (deterministic, fp32 adds rounded to
@@ -56,26 +56,6 @@ __device__ __forceinline__ void dir_split_tf32(float a, float& hi, float& lo) {
 __device__ __forceinline__ unsigned swz(int row, int chunk) {
     return (unsigned)(row * 128 + ((chunk ^ (row & 7)) << 4));
 }
-__device__ __forceinline__ void cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ unsigned peer_addr(const void* p, int rank) {
-    unsigned r;
-    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_u32(p)), "r"(rank));
-    return r;
-}
-__device__ __forceinline__ long long ld_peer(unsigned a, long long) {
-    long long v;
-    asm volatile("ld.shared::cluster.b64 %0, [%1];" : "=l"(v) : "r"(a) : "memory");
-    return v;
-}
-__device__ __forceinline__ float ld_peer(unsigned a, float) {
-    float v;
-    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
-    return v;
-}
-
 // ---- operand tiles ---------------------------------------------------------------------------
 // Registers of one thread's share of an operand's k-block, loaded in one go so that all loads are
 // in flight together, and stored a k-block later.
@@ -634,7 +614,7 @@ direct_kernel(const __grid_constant__ DirectParams p) {
 #pragma unroll
                 for (int j = 0; j < 8; ++j) v[j] = 0;
                 for (int z = 0; z < splits; ++z) {
-                    const unsigned at = peer_addr(red + c0 * 128 + lrow, z);
+                    const unsigned at = map_rank(red + c0 * 128 + lrow, z);
 #pragma unroll
                     for (int j = 0; j < 8; ++j) v[j] += ld_peer(at + j * 128 * (unsigned)sizeof(Sum), (Sum)0);
                 }
@@ -713,10 +693,8 @@ DirectShape direct_shape(const b2_direct_args& a) {
 template <int MODE, int BN, int AK>
 int direct_launch_as(const DirectParams& p, cudaStream_t st) {
     const int KB = MODE == MODE_FLEX16 ? 128 : 32;
-    int ring = dir_ring_bytes(BN);
-    const int red = p.splits > 1 ? BN * 128 * (MODE == MODE_FLEX16 ? 8 : 4) : 0;
+    const int ring = dir_ring_bytes(BN);
     static_assert(dir_ring_bytes(BN) >= BN * 128 * 8, "the slices' sums are exchanged through the ring");
-    (void)red;
     const int smem = 1024 + ring + 128 +
                      (AK == B2_OPERAND_GATHER ? p.kb_per_split * KB * (filter_tiles(p.a) ? 16 : 8) : 0);
     static bool attr_set = false;

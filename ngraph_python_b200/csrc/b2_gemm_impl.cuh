@@ -38,7 +38,7 @@
 // padded to tile multiples, into caller-provided scratch.
 //
 // Every mbarrier wait is bounded; when one runs out the kernel records it in `status` and
-// finishes without hanging.  No cluster multicast is used anywhere.
+// finishes without hanging.  No load is multicast to a cluster.
 #ifndef B2_GEMM_IMPL_CUH
 #define B2_GEMM_IMPL_CUH
 #include <cuda.h>
@@ -190,6 +190,33 @@ __device__ __forceinline__ void tmem_ld8(unsigned taddr, unsigned* r) {
 }
 __device__ __forceinline__ void tmem_ld_wait() {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
+// ---- clusters --------------------------------------------------------------------------------------
+__device__ __forceinline__ unsigned cluster_rank() {
+    unsigned r;
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// the address at which CTA `rank` of the cluster has what this one has at p
+__device__ __forceinline__ unsigned map_rank(const void* p, unsigned rank) {
+    unsigned r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_u32(p)), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ long long ld_peer(unsigned a, long long) {
+    long long v;
+    asm volatile("ld.shared::cluster.b64 %0, [%1];" : "=l"(v) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ float ld_peer(unsigned a, float) {
+    float v;
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+    return v;
 }
 
 // Shared-memory matrix descriptor: K-major operand, 128-byte swizzle, rows of 128 B stored

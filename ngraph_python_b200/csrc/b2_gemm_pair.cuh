@@ -40,20 +40,6 @@ constexpr int kPairStage = 48 * 1024;
 constexpr int kPairStages = 4;
 constexpr int kPairSmem = 1024 + kPairStages * kPairStage + 256;
 
-__device__ __forceinline__ unsigned cluster_rank() {
-    unsigned r;
-    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ unsigned map_rank(const void* p, unsigned rank) {
-    unsigned r;
-    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_u32(p)), "r"(rank));
-    return r;
-}
-__device__ __forceinline__ void pair_cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 // completes on a barrier of the pair's leader
 __device__ __forceinline__ void tma_load_2d_pair(void* dst, const CUtensorMap* map, int x, int y, unsigned bar) {
     asm volatile(
@@ -88,8 +74,8 @@ __device__ __forceinline__ void tc_mma_pair(unsigned tmem_d, unsigned long long 
 __host__ __device__ constexpr unsigned idesc_pair(unsigned dfmt, unsigned afmt, unsigned bfmt, unsigned n) {
     return (dfmt << 4) | (afmt << 7) | (bfmt << 10) | ((n >> 3) << 17) | ((256u >> 4) << 24);
 }
-// Eight columns of a row in the exchanged sums, fp32: two groups of four, rows behind one another, so that
-// a lane's share is two 16-byte accesses and a warp's is contiguous.
+// Slices of K exchange their sums in pieces of eight columns x 128 rows.  fp32: two groups of four columns,
+// rows behind one another, so that a lane's share is two 16-byte accesses and a warp's is contiguous.
 __device__ __forceinline__ void put_piece(float* piece, int lrow, const float* v) {
     *(float4*)(piece + lrow * 4) = make_float4(v[0], v[1], v[2], v[3]);
     *(float4*)(piece + 512 + lrow * 4) = make_float4(v[4], v[5], v[6], v[7]);
@@ -105,11 +91,16 @@ __device__ __forceinline__ void put_piece(long long* piece, int lrow, const long
 #pragma unroll
     for (int j = 0; j < 8; ++j) piece[j * 128 + lrow] = v[j];
 }
-__device__ __forceinline__ void get_piece(const long long* piece, int lrow, unsigned rank, long long* v) {
+__device__ __forceinline__ void add_piece(const float* piece, int lrow, unsigned rank, float* v) {
+    float x[8];
+    get_piece(piece, lrow, rank, x);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] += x[j];
+}
+__device__ __forceinline__ void add_piece(const long long* piece, int lrow, unsigned rank, long long* v) {
     const unsigned at = map_rank(piece + lrow, rank);
 #pragma unroll
-    for (int j = 0; j < 8; ++j)
-        asm volatile("ld.shared::cluster.b64 %0, [%1];" : "=l"(v[j]) : "r"(at + j * 1024) : "memory");
+    for (int j = 0; j < 8; ++j) v[j] += ld_peer(at + j * 1024, 0LL);
 }
 
 struct PairParams {
@@ -177,7 +168,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constan
     asm volatile("griddepcontrol.wait;" ::: "memory");
     tc_fence_before();
     __syncthreads();
-    pair_cluster_sync();
+    cluster_sync();
     tc_fence_after();
     const unsigned tmem_base = (unsigned)warp_uniform((int)*tmem_holder);
 
@@ -409,7 +400,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constan
         }
         if (p.splits > 1) {
             // (one tile per cluster)  every slice adds a share of the column pieces
-            pair_cluster_sync();
+            cluster_sync();
             int tm, tn;
             pair_tile(p, first, tm, tn);
             const int row = tm * 256 + side * 128 + lrow, n0 = tn * 128;
@@ -418,7 +409,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constan
             for (int round = (warp - 2) >> 2; round * p.splits + slice < 16; round += kGroups) {
                 const int c0 = (round * p.splits + slice) * 8;
                 Sum v[8];
-                if (MODE != MODE_FLEX16 && p.apart) {
+                bool whole = true;                                // every slice hands out its sum
+                if constexpr (MODE != MODE_FLEX16) if (p.apart) {
+                    whole = false;
                     get_piece(red + c0 * 128, lrow, side, v);
                     // the chains of the other slices, four at a time in flight
                     const int per = p.kb_per_split / kChunkKb;
@@ -448,15 +441,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constan
                             for (int j = 0; j < 8; ++j) v[j] += x[u][j];
                         }
                     }
-                } else {
+                }
+                if (whole) {
 #pragma unroll
                     for (int j = 0; j < 8; ++j) v[j] = 0;
-                    for (int z = 0; z < p.splits; ++z) {
-                        Sum x[8];
-                        get_piece(red + c0 * 128, lrow, 2 * z + side, x);
-#pragma unroll
-                        for (int j = 0; j < 8; ++j) v[j] += x[j];
-                    }
+                    for (int z = 0; z < p.splits; ++z) add_piece(red + c0 * 128, lrow, 2 * z + side, v);
                 }
                 if (ok) finish(row, n0 + c0, fix, v);
             }
@@ -478,9 +467,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constan
         }
     }
     __syncwarp();
-    if (warp < 2 && p.splits > 1) pair_cluster_sync();             // (the epilogue's exchange)
+    if (warp < 2 && p.splits > 1) cluster_sync();             // (the epilogue's exchange)
     tc_fence_before();
-    pair_cluster_sync();               // nothing of the pair is still to be read or signalled
+    cluster_sync();               // nothing of the pair is still to be read or signalled
     if (warp == 1) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512) : "memory");
