@@ -1,6 +1,6 @@
 """The b200 transformer EXECUTING behind the reference's own API on a GPU.
 
-Graphs are built with the real `ngraph` package (the checker's copy under oracle/_ref, see
+Graphs are built with the real `ngraph` package (the copy under oracle/_ref, see
 oracle/make_ref.py), compiled by `ngraph.transformers.make_transformer_factory('b200')()` --
 the registration of ngraph/transformers/base.py:265-279, the computation protocol of
 base.py:94-136, 420-433 -- and run on the device; the same graph runs through the reference's
