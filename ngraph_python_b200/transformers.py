@@ -219,6 +219,8 @@ class Computation(object):
             t.initialize()
         if t.plan_only:
             raise lib.B200Error("a plan_only transformer cannot run computations")
+        if t.closed:        # (a recorded step list would run, on memory that is no longer its own)
+            raise lib.B200Error("the transformer has been closed")
         feed = kwargs.pop("feed_dict", None)
         if feed is not None:
             args = [feed[p] for p in self.parameters]

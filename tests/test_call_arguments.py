@@ -5,6 +5,7 @@ import numpy as np
 import pytest
 
 import ngraph_python_b200 as ng
+from ngraph_python_b200 import lib
 
 pytestmark = pytest.mark.gpu
 
@@ -95,3 +96,18 @@ def test_argument_that_the_computation_writes():
     check(8.0)
     assert comp.steps[-1].stores_argument
     t.close()
+
+
+def test_no_call_on_a_closed_transformer():
+    """A recorded step list holds the addresses of memory that the transformer has given back."""
+    A = ng.make_axis(64, name="A")
+    x = ng.placeholder([A])
+    t = ng.transformers.allocate_transformer("b200")
+    comp = t.computation(ng.exp(x), x)
+    comp(np.zeros(64, np.float32))
+    comp.capture()
+    launched = t.kernel_launches
+    t.close()
+    with pytest.raises(lib.B200Error, match="closed"):
+        comp(np.zeros(64, np.float32))
+    assert t.kernel_launches == launched
