@@ -103,7 +103,7 @@ def test_products_for_pairs_of_sms(M, N, K, flex):
 
 
 SAME_BITS = {512: {(0, 1)}, 520: {(0, 2), (1, 2)}, 1024: {(0, 2)}, 1500: {(0, 3), (1, 2)},
-             2048: {(0, 4), (1, 2)}, 3000: {(0, 6), (1, 2), (1, 3)}, 4096: {(0, 8), (1, 2), (1, 4)}}
+             2048: {(0, 4), (1, 2)}, 3000: {(0, 6), (1, 2), (1, 3)}, 4096: {(0, 8), (1, 2), (1, 3), (1, 4)}}
 
 
 @pytest.mark.parametrize("K", sorted(SAME_BITS))
