@@ -382,6 +382,32 @@ int b2_conv_flex16_planes_fused(int32_t pass, const void* act_planes, const void
                                 int32_t slotX, int32_t slotF, int32_t slotOut,
                                 const b2_conv_epilogue* epilogue, int32_t* stats,
                                 uint64_t* probe_out, int32_t* status, int32_t probe, void* stream);
+/* A run of flex16 convolution layers in one launch, for networks whose images fit into shared memory:
+ * layer l reads the chain's input (input = -1) or the result of layer `input`, adds bias and such a
+ * tensor (residual) as b2_conv_flex16_planes_fused does, bit for bit, and may be stored as an int16 K,P,Q,N tensor (out; NULL: only layers of the chain read it).
+ * Statistics go to slot_out of every layer.  The chain's input is an int16 C,H,W,N tensor (x) or, with
+ * x = NULL, its byte planes; pooled (K x N, or NULL) receives the averages of the last layer's images as
+ * b2_pool_avg_fprop makes them (up to 512 pixels).  b2_conv_chain_info says whether the layers can make a chain (strides of 1
+ * and 2, no dilation, output channels in multiples of 16 up to 112, activations of at least one image
+ * in shared memory, no tensor read at both strides) and the bytes of their filter planes, which
+ * b2_conv_chain_filters writes (16-byte aligned; again whenever the filters have changed). */
+#define B2_CONV_CHAIN_MAX 32
+#define B2_CONV_CHAIN_NONE (-2)       /* no residual */
+typedef struct b2_conv_chain_layer {
+    b2_conv_dims dims;
+    int32_t input, residual;
+    int32_t relu;
+    int32_t slot_in, slot_filters, slot_out, slot_bias, slot_residual;
+    const int16_t* filters;
+    const int16_t* bias;
+    int16_t* out;
+} b2_conv_chain_layer;
+int b2_conv_chain_info(const b2_conv_chain_layer* layers, int32_t n, int32_t* supported, size_t* filter_bytes);
+int b2_conv_chain_filters(const b2_conv_chain_layer* layers, int32_t n, void* filter_planes,
+                          int32_t* launches, void* stream);
+int b2_conv_chain_flex16(const b2_conv_chain_layer* layers, int32_t n, const int16_t* x, const void* x_planes,
+                         size_t plane_bytes, const void* filter_planes, const b2_flex_scale* table,
+                         int32_t* stats, int16_t* pooled, int32_t* status, void* stream);
 /* The two training contractions of a convolution whose forward pass has the dimensions `d`
  * (d always describes the FORWARD convolution: I is C,D,H,W,N, F is C,T,R,S,K, E is K,M,P,Q,N).
  * Replace ConvBpropKernel / ConvUpdateKernel (ngraph/transformers/gpu/conv.py:121-312) and

@@ -225,6 +225,147 @@ def join_filter_planes(steps):
         mine[0].joint_planes = mine
 
 
+class ConvChainStep(_Step):
+    """A run of convolution layers that a recorded call makes in one launch, with the activations between
+    them in shared memory.  `layers` describes them, `members` are the steps it stands for: outside
+    recorded calls (first writes, measuring launches) they run one by one, with the same bits."""
+    kind = "conv_chain"
+    launches = 1
+
+    def __init__(self, members, layers, nbytes, kept, pool=None):
+        """kept: results that somebody outside reads; pool: the averaging step behind the last layer,
+        where it takes whole images and reads them alone."""
+        super(ConvChainStep, self).__init__(members[0].index, members[0].op)
+        self.members, self.layers, self.nbytes = members, layers, nbytes
+        self.in_views = [v for s in members for v in s.in_views]
+        self.out_views = [v for s in members for v in s.out_views]
+        # results that only the run itself reads are not stored by it (int16 tensors that the members
+        # store when they run one by one)
+        self.unstored = set(s.out_views[0].buffer for s in members if s.write_int16) - kept
+        self.kept, self.pool = kept, pool
+        if pool is not None:
+            self.out_views += pool.out_views
+        self.planes = None
+        self.versions = None
+
+    def _filters(self):
+        return [s.in_views[s.filter_arg].buffer for s in self.members]
+
+    def refresh(self, t):
+        """Filter planes as the chain reads them, made again when filters have changed."""
+        versions = [b.version for b in self._filters()]
+        if versions == self.versions:
+            return
+        n = C.c_int32()
+        if self.planes is None:
+            self.planes = t.torch.zeros((self.nbytes,), dtype=t.torch.uint8, device=t.device)
+        lib.check(lib.raw().b2_conv_chain_filters(self._layers(t), len(self.members), self.planes.data_ptr(),
+                                                  C.byref(n), t.stream.cuda_stream))
+        t.kernel_launches += n.value
+        self.versions = versions
+
+    def _layers(self, t):
+        arr = (lib.ConvChainLayer * len(self.members))(*self.layers)
+        for a, s in zip(arr, self.members):
+            xv, fv, ov = s.in_views[0], s.in_views[1], s.out_views[0]
+            a.filters = s._ptr(fv)
+            a.slot_in, a.slot_filters = t._slot_for_read(xv.buffer, s), t._slot_for_read(fv.buffer, s)
+            a.slot_out, a.slot_bias, a.slot_residual = ov.buffer.slot_write, -1, -1
+            extra = list(s.in_views[2:])
+            if s.epi.get("bias") is not None:
+                v = extra.pop(0)
+                a.bias, a.slot_bias = s._ptr(v), t._slot_for_read(v.buffer, s)
+            if s.epi.get("residual") is not None:
+                a.slot_residual = t._slot_for_read(extra.pop(0).buffer, s)
+            a.out = s._ptr(ov) if ov.buffer in self.kept else None
+        return arr
+
+    def launch(self, t):
+        x = self.members[0].in_views[0]
+        planes = x.buffer.planes_ptr if x.buffer.planes_by_producer else None
+        lib.check(lib.raw().b2_conv_chain_flex16(
+            self._layers(t), len(self.members), None if planes else self._ptr(x), planes, x.buffer.plane_bytes,
+            self.planes.data_ptr(), t._table.data_ptr(), t._stats.data_ptr(),
+            self._ptr(self.pool.out_views[0]) if self.pool is not None else None, t._status.data_ptr(),
+            t.stream.cuda_stream))
+        t.kernel_launches += 1
+
+    def store_results(self, t):
+        """Results that recorded calls do not store, for a reader from outside any call."""
+        for s in self.members:
+            s.launch(t)
+        t._stats_clean = False           # (their statistics belong to the call that has been)
+
+
+def chain_convolutions(steps, returned, t):
+    """The step list with every run of convolution layers that fits one launch (b2_conv_chain_info)
+    replaced by a ConvChainStep.  A run is made of neighbouring steps; what they stream comes from the
+    run or, for its first layer's input, from int16 or byte planes that are complete before it; their
+    filters do not change inside the computation; and no step outside reads one of their results as byte
+    planes.  `returned`: buffers whose contents the computation returns."""
+    if not t.flex:
+        return list(steps)
+
+    def suits(s):
+        return (isinstance(s, ConvStep) and s.use_planes and s.epi is not None and
+                not s.planes_built_first and not s.joint_planes and s.splits in ((), (0,)) and
+                s.in_views[1].buffer.last_write_step < 0 and s.epi.get("mask") is None and
+                not s.out_views[0].buffer.persistent)
+
+    def chain_of(run):
+        made, layers = {}, []
+        first = run[0].in_views[0].buffer
+        for s in run:
+            layer = lib.ConvChainLayer()
+            layer.dims, layer.relu = s.dims, int(bool(s.epi.get("relu")))
+            x = s.in_views[0].buffer
+            layer.residual = lib.CHAIN_NONE
+            if x is not first and x not in made:
+                return None
+            layer.input = made.get(x, -1)
+            if s.epi.get("residual") is not None:
+                r = s.in_views[3 if s.epi.get("bias") is not None else 2].buffer
+                if r is not first and r not in made:
+                    return None
+                layer.residual = made.get(r, -1)
+            made[s.out_views[0].buffer] = len(layers)
+            layers.append(layer)
+        mine = set(run)
+        after = steps[steps.index(run[-1]) + 1] if steps.index(run[-1]) + 1 < len(steps) else None
+        pool = after if isinstance(after, PoolStep) and after.averages_images() and \
+            after.in_views[0].buffer is run[-1].out_views[0].buffer else None
+        mine.add(pool)
+        kept = set(b for b in made if b in returned)
+        for s in steps:
+            if s in mine:
+                continue
+            for k, v in enumerate(s.in_views):
+                if v.buffer in made or v.buffer is first:
+                    if k in getattr(s, "plane_args", ()):
+                        return None
+                    if v.buffer in made:
+                        kept.add(v.buffer)
+        ok, nbytes = lib.conv_chain_info(layers)
+        return ConvChainStep(list(run), layers, nbytes, kept, pool) if ok else None
+
+    out, i = [], 0
+    while i < len(steps):
+        end = i
+        while end < len(steps) and end - i < lib.CHAIN_MAX and suits(steps[end]):
+            end += 1
+        chain = None
+        while end - i >= 2 and chain is None:
+            chain = chain_of(steps[i:end])
+            end -= chain is None
+        if chain is None:
+            out.append(steps[i])
+            i += 1
+        else:
+            out.append(chain)
+            i = end + (chain.pool is not None)
+    return out
+
+
 class GemmStep(_Step):
     """C[M,N] = op(A)[M,K] * op(B)[K,N] for a DotOp."""
     kind = "gemm"
@@ -575,6 +716,12 @@ class PoolStep(_Step):
         self.in_views = [iv]
         self.out_views = [ov]
         self.flex = t.flex
+
+    def averages_images(self):
+        """Whether a result is the average of a whole channel of an image (of at most 512 pixels)."""
+        Cc, H, W, N, P, Q, R, S, pad_h, pad_w = self.args[:10]
+        return (self.flex and self.pool_op == "avg" and P == Q == 1 and (R, S) == (H, W) and
+                pad_h == pad_w == 0 and H * W <= 512)
 
     def output_buffers(self):
         return []          # no exponent of its own to manage

@@ -74,6 +74,17 @@ class ConvFilterJob(C.Structure):
     _fields_ = [("filters", C.c_void_p), ("planes", C.c_void_p), ("dims", ConvDims), ("conv_pass", C.c_int32)]
 
 
+CHAIN_MAX = 32                 # B2_CONV_CHAIN_MAX
+CHAIN_NONE = -2                # B2_CONV_CHAIN_NONE
+
+
+class ConvChainLayer(C.Structure):
+    _fields_ = [("dims", ConvDims), ("input", C.c_int32), ("residual", C.c_int32), ("relu", C.c_int32),
+                ("slot_in", C.c_int32), ("slot_filters", C.c_int32), ("slot_out", C.c_int32),
+                ("slot_bias", C.c_int32), ("slot_residual", C.c_int32),
+                ("filters", C.c_void_p), ("bias", C.c_void_p), ("out", C.c_void_p)]
+
+
 class FlexScale(C.Structure):
     _fields_ = [("scale", C.c_float), ("inv_scale", C.c_float)]
 
@@ -159,6 +170,9 @@ def _load():
                                             i32, vp, vp, vp, i32, vp]),
         "b2_conv_flex16_planes_fused": (C.c_int, [i32, vp, vp, vp, C.POINTER(ConvDims), vp, i32, i32,
                                                   i32, C.POINTER(ConvEpilogue), vp, vp, vp, i32, vp]),
+        "b2_conv_chain_info": (C.c_int, [C.POINTER(ConvChainLayer), i32, C.POINTER(i32), C.POINTER(sz)]),
+        "b2_conv_chain_filters": (C.c_int, [C.POINTER(ConvChainLayer), i32, vp, C.POINTER(i32), vp]),
+        "b2_conv_chain_flex16": (C.c_int, [C.POINTER(ConvChainLayer), i32, vp, vp, sz, vp, vp, vp, vp, vp, vp]),
         "b2_conv_bprop_scratch_bytes": (C.c_int, [i32, C.POINTER(ConvDims), C.POINTER(sz)]),
         "b2_conv_bprop_f32_fused": (C.c_int, [vp, vp, vp, C.POINTER(ConvDims), vp, vp, vp, vp]),
         "b2_conv_bprop_f32": (C.c_int, [vp, vp, vp, C.POINTER(ConvDims), vp, sz, vp, vp]),
@@ -432,6 +446,14 @@ def conv_planes_info(dims, conv_pass=CONV_FPROP):
     ok, a, f = C.c_int32(), C.c_size_t(), C.c_size_t()
     check(_lib.b2_conv_planes_info(C.byref(dims), conv_pass, C.byref(ok), C.byref(a), C.byref(f)))
     return bool(ok.value), a.value, f.value
+
+
+def conv_chain_info(layers):
+    """(whether the layers make a chain, bytes of their filter planes)."""
+    ok, n = C.c_int32(), C.c_size_t()
+    arr = (ConvChainLayer * len(layers))(*layers)
+    check(_lib.b2_conv_chain_info(arr, len(layers), C.byref(ok), C.byref(n)))
+    return bool(ok.value), n.value
 
 
 def conv_update_planes_info(dims):

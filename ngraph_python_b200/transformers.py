@@ -171,6 +171,7 @@ class Computation(object):
         self.executor = None
         self.launches_per_call = 0
         self._io = None             # argument and result handling of the recorded step list
+        self.chains = []            # runs of convolutions that recorded calls make in one launch
         self._comm_steps = []       # this computation's exchanges, in production order
         self._allreduce = None      # their arena and bucket plan (one per computation)
 
@@ -292,7 +293,11 @@ class Computation(object):
         if t.flex and any(not b.entry.initialized for b in self.written):
             raise lib.B200Error("run the computation once before capturing it")
         torch = t.torch
-        refreshable = [s for s in self.steps if hasattr(s, "refresh")]
+        steps = kernels.chain_convolutions(self.steps, set(v.buffer for v in self.return_views), t)
+        refreshable = [s for s in steps if hasattr(s, "refresh")]
+        self.chains = [s for s in steps if s.kind == "conv_chain"]
+        for s in self.chains:
+            s.refresh(t)
         ar = self._allreduce
         has_comm = any(s.kind == "comm" for s in self.steps) and ar is not None and ar.comm.size > 1
         in_graph = has_comm and getattr(ar.comm, "capturable", False)
@@ -306,7 +311,7 @@ class Computation(object):
             if cur is not None and cur["steps"]:
                 segments.append(cur)
             cur, made_here = None, set()
-        for s in self.steps:
+        for s in steps:
             needs = []
             if has_comm and s.kind != "comm":
                 needs = [v.buffer.comm_key for v in s.in_views
@@ -2441,6 +2446,10 @@ class DeviceTensor(object):
         return e.scale if e is not None else 1.0
 
     def get(self, tensor=None):
+        for comp in self.transformer.computations:
+            for chain in comp.chains:
+                if self.view.buffer in chain.unstored:
+                    chain.store_results(self.transformer)
         host = self.transformer._device_to_host(self.view)
         if tensor is None:
             return host
