@@ -389,7 +389,8 @@ int b2_conv_flex16_planes_fused(int32_t pass, const void* act_planes, const void
  * x = NULL, its byte planes; pooled (K x N, or NULL) receives the averages of the last layer's images as
  * b2_pool_avg_fprop makes them (up to 512 pixels).  b2_conv_chain_info says whether the layers can make a chain (strides of 1
  * and 2, no dilation, output channels in multiples of 16 up to 112, activations of at least one image
- * in shared memory, no tensor read at both strides) and the bytes of their filter planes, which
+ * in shared memory, no tensor read at both strides) that is faster than launches of their own -- `out` of
+ * every layer as it will be -- and gives the bytes of their filter planes, which
  * b2_conv_chain_filters writes (16-byte aligned; again whenever the filters have changed). */
 #define B2_CONV_CHAIN_MAX 32
 #define B2_CONV_CHAIN_NONE (-2)       /* no residual */

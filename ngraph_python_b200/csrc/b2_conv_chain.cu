@@ -20,6 +20,7 @@
 // The products are those of the tile kernel (high and low bytes, the filters' low byte stored minus 128,
 // its bias undone with the sum of the activations under the window), as two instructions per k-step:
 //     A_hi x [B_hi | B_lo' | sum] -> HH | X1 | S_hi        A_lo x [B_hi | B_lo' | sum] -> X2 | LL | S_lo
+// (B_hi and B_lo' by turns, eight output channels each),
 // each issued by a thread of its own (an MMA this small costs its issuer about as long as the tensor
 // pipe).  The epilogue evaluates the layer's tail with the arithmetic of the tile kernel, operation for
 // operation, so a network gives the same bits either way.  A thread has a pixel and 16 of its channels:
@@ -30,7 +31,11 @@
 // single pass over tiles is what makes taking over the memory of tensors that are no longer read safe;
 // plan() has the conditions.
 //
-// What bounds it: 256 images of ResNet-20 (128 CTAs of two images), 22 layers: see plan().
+// What bounds it: 256 images of ResNet-20 (128 CTAs of two images), 22 layers: 204 us one by one, 120 us
+// here.  Of these 60 are the chain of hand-overs (issue, full set, stored tile: 2.4 us a layer), 15 the
+// products beyond the first k-step of a tile, 13 the arithmetic of the epilogue and 34 the rest of it
+// (operands, tails, stores); a rolled epilogue is faster than an unrolled one (120 / 135 us), because a
+// warp that comes to a line of instructions after the others of its scheduler fetches it anew.
 #include <algorithm>
 #include <vector>
 
@@ -39,7 +44,7 @@
 namespace {
 
 constexpr int kLayersMost = B2_CONV_CHAIN_MAX;
-constexpr int kStepsMost = 36;               // k-steps of 32 bytes a layer may have (whole sixes)
+constexpr int kStepsMost = 36;               // k-steps of 32 bytes a layer may have
 constexpr int kTilesMost = 32;
 constexpr int kChannelsMost = 112;           // output channels: 2 * 112 + 16 columns an accumulator
 constexpr int kCtaThreads = 640;             // sixteen epilogue warps, one for the copies, three issuers
@@ -55,7 +60,7 @@ struct Place {
 };
 
 struct Layer {
-    unsigned step[kStepsMost];               // operand offset of a k-step | distance of its halves << 16
+    unsigned step[kStepsMost + 1];           // operand offset of a k-step | distance of its halves << 16
     int nk, a_base, a_row, sbo, plane;
     int trows, tcols, tiles;
     int filt, filt_units, prefetch;
@@ -106,13 +111,14 @@ __device__ __forceinline__ int least4(const unsigned* words) {
     return min(min(a, b), min(c, d));
 }
 // waits until the four warps of every slot have stored at least so many tiles; for ONE thread of a warp
-__device__ __forceinline__ bool stored(const unsigned* done, int4 e) {
+__device__ __forceinline__ bool stored(const unsigned* done, int4 e, unsigned pause = 20) {
     for (int i = 0; i < kWaitPolls; ++i) {
         const int a = least4(done) - e.x, b = least4(done + 4) - e.y, c = least4(done + 8) - e.z, d = least4(done + 12) - e.w;
         if (min(min(a, b), min(c, d)) >= 0) {
             asm volatile("fence.acq_rel.cta;" ::: "memory");
             return true;
         }
+        if (pause) __nanosleep(pause);           // (polling takes issue slots from the epilogue warps)
     }
     return false;
 }
@@ -121,6 +127,7 @@ __device__ __forceinline__ bool counted(const unsigned* word, unsigned e) {
         unsigned v;
         asm volatile("ld.acquire.cta.shared::cta.u32 %0, [%1];" : "=r"(v) : "r"(smem_u32(word)) : "memory");
         if ((int)(v - e) >= 0) return true;
+        __nanosleep(20);
     }
     return false;
 }
@@ -139,6 +146,20 @@ __device__ __forceinline__ int4 sets_after(int4 v, int n, int nsets) {
     else v.x += n;
     return v;
 }
+// A bounded wait that suspends for up to 0.1 ms at a time: many warps wait here, and a poll takes issue slots
+// from those that work.
+__device__ __forceinline__ bool bar_wait(unsigned long long* bar, unsigned parity) {
+    for (int i = 0; i < 1024; ++i) {
+        unsigned ok;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity), "r"(100000) : "memory");
+        if (ok) return true;
+    }
+    return false;
+}
 __device__ __forceinline__ void fence_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void epilogue_barrier() {
     asm volatile("bar.sync 1, %0;" ::"n"(kEpiWarps * 32) : "memory");
@@ -149,26 +170,42 @@ __device__ __forceinline__ unsigned tmem_ld1(unsigned taddr) {
     return r;
 }
 
-// Eight columns of an accumulator set to four pairs of mantissas.  The arithmetic of
-// conv_implicit_kernel's fused epilogue: same operations, same order; what differs is how the result is
-// quantised (rounded to nearest even and saturated by the conversions, the same values).  Instruction
-// issue bounds the epilogue, so nothing is packed and unpacked for the two-wide fp32 forms.
+__device__ __forceinline__ unsigned long long pack2(float a, float b) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+    unsigned long long r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
+    unsigned long long r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
+// Eight columns of an accumulator set (v1: HH | X1, v2: X2 | LL) to four pairs of mantissas.  The arithmetic
+// of conv_implicit_kernel's fused epilogue: same operations, same order; what differs is how the result is
+// quantised (rounded to nearest even and saturated by the conversions, the same values).
 template <bool SHORT>
-__device__ __forceinline__ void finish8(const unsigned* hh, const unsigned* x1, const unsigned* x2,
-                                        const unsigned* ll, float fix, float f, const float* y, unsigned* w) {
+__device__ __forceinline__ void finish8(const unsigned* v1, const unsigned* v2, unsigned long long fix,
+                                        unsigned long long f, const unsigned long long* y, unsigned* w) {
+    const unsigned long long k256 = pack2(256.0f, 256.0f), k65536 = pack2(65536.0f, 65536.0f);
 #pragma unroll
     for (int j = 0; j < 8; j += 2) {
-        int z[2];
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            const unsigned x = x1[j + i] + x2[j + i];
-            const float l = (float)(int)ll[j + i] + fix;
-            float v;
-            if (SHORT) v = fmaf((float)(int)((hh[j + i] << 8) + x), 256.0f, l);
-            else v = fmaf((float)(int)hh[j + i], 65536.0f, fmaf((float)(int)x, 256.0f, l));
-            z[i] = __float2int_rn(fmaf(v, f, y[j + i]));
-        }
-        asm("cvt.pack.sat.s16.s32 %0, %1, %2;" : "=r"(w[j >> 1]) : "r"(z[1]), "r"(z[0]));
+        const unsigned xa = v1[8 + j] + v2[j], xb = v1[9 + j] + v2[j + 1];
+        const unsigned long long l = add2(pack2((float)(int)v2[8 + j], (float)(int)v2[9 + j]), fix);
+        unsigned long long v;
+        if (SHORT)
+            v = fma2(pack2((float)(int)((v1[j] << 8) + xa), (float)(int)((v1[j + 1] << 8) + xb)), k256, l);
+        else
+            v = fma2(pack2((float)(int)v1[j], (float)(int)v1[j + 1]), k65536, fma2(pack2((float)(int)xa, (float)(int)xb), k256, l));
+        v = fma2(v, f, y[j >> 1]);
+        float p, q;
+        asm("mov.b64 {%0, %1}, %2;" : "=f"(p), "=f"(q) : "l"(v));
+        asm("cvt.pack.sat.s16.s32 %0, %1, %2;" : "=r"(w[j >> 1]) : "r"(__float2int_rn(q)), "r"(__float2int_rn(p)));
     }
 }
 
@@ -296,7 +333,7 @@ conv_chain_kernel(const __grid_constant__ Chain p) {
             // between them: half the lanes would go on without the other half, whatever the compiler takes
             // a load from one address to be.)
             int go = 1;
-            if (lane == 0) go = stored(done, e);
+            if (lane == 0) go = stored(done, e, 200);
             ok = __shfl_sync(0xffffffffu, go, 0) != 0;
             if (!ok) break;
             float* b = bias_s + (l & 1) * kChannelsMost;
@@ -316,7 +353,7 @@ conv_chain_kernel(const __grid_constant__ Chain p) {
         // what is in flight lands before the block ends, whatever has become of the other roles
         if (lane == 0) {
             for (int i = l > 2 ? l - 2 : 0; i < l; ++i)
-                if (!mbar_wait(&filt_full[i & 1], (i >> 1) & 1u)) ok = false;
+                if (!bar_wait(&filt_full[i & 1], (i >> 1) & 1u)) ok = false;
             if (!ok) atomicExch(fail_flag, 1);
         }
         __syncwarp();
@@ -343,31 +380,40 @@ conv_chain_kernel(const __grid_constant__ Chain p) {
                 bool first = true;
                 for (int t = split ? 0 : mine; t < tiles && (!split || mine < 2); t += split ? 1 : 3) {
                     const int tr = t / tcols, tc = t - tr * tcols, s = t & (nsets - 1);
+                    const unsigned d = tmem_base + (unsigned)(2 * s * n2);
+                    const unsigned a0 = a_base + (unsigned)(tr * a_row + tc * 8);
+                    const unsigned used = 16u * (unsigned)((s == 0 ? uses.x : s == 1 ? uses.y : s == 2 ? uses.z : uses.w) + t / nsets);
+                    unsigned b = b_lo, nxt = L.step[0], acc = 0;
                     if (coarse) {
-                        if (first) ok = stored(done, base);
-                    } else {
+                        if (first && ok) ok = stored(done, base);
+                    } else if (ok) {
                         // (the layer before has the same tiles)
                         const int er = tr + 1 < L.trows ? tr + 1 : tr, ec = tc + 1 < tcols ? tc + 1 : tc;
                         ok = stored(done, slots_after(prev, er * tcols + ec + 1, prev_sets));
                     }
-                    if (first && ok) ok = mbar_wait(&filt_full[l & 1], (l >> 1) & 1u);
+                    if (first && ok) ok = bar_wait(&filt_full[l & 1], (l >> 1) & 1u);
                     first = false;
-                    const unsigned used = 16u * (unsigned)((s == 0 ? uses.x : s == 1 ? uses.y : s == 2 ? uses.z : uses.w) + t / nsets);
                     if (!ok || !counted(&drained[s], used)) { ok = false; break; }
                     tc_fence_after();
-                    const unsigned d = tmem_base + (unsigned)(2 * s * n2);
-                    const unsigned a0 = a_base + (unsigned)(tr * a_row + tc * 8);
-                    unsigned b = b_lo;
-                    for (int k = 0; k < nk; k += 6) {
-                        unsigned st[6];
-#pragma unroll
-                        for (int i = 0; i < 6; ++i) st[i] = a0 + L.step[k + i];      // (the table is padded)
-#pragma unroll
-                        for (int i = 0; i < 6; ++i, b += b_step)
-                            if (k + i < nk) {
-                                if (!split || mine == 0) tc_mma<MODE_FLEX16>(d, a_hi | st[i], b_hi | b, id_hi | nbits, k + i > 0 ? 1u : 0u);
-                                if (!split || mine == 1) tc_mma<MODE_FLEX16>(d + n2, a_hi | (st[i] + plane), b_hi | b, id_lo | nbits, k + i > 0 ? 1u : 0u);
-                            }
+                    if (!split) {
+                        const unsigned ih = id_hi | nbits, il = id_lo | nbits, dl = d + n2;
+#pragma unroll 2
+                        for (int k = 0; k < nk; ++k, b += b_step) {
+                            const unsigned st = a0 + nxt;
+                            nxt = L.step[k + 1];                               // (the table has one to spare)
+                            tc_mma<MODE_FLEX16>(d, a_hi | st, b_hi | b, ih, acc);
+                            tc_mma<MODE_FLEX16>(dl, a_hi | (st + plane), b_hi | b, il, acc);
+                            acc = 1;
+                        }
+                    } else {
+                        const unsigned id = (mine ? id_lo : id_hi) | nbits, dd = d + mine * n2, aa = a0 + mine * plane;
+#pragma unroll 2
+                        for (int k = 0; k < nk; ++k, b += b_step) {
+                            const unsigned st = aa + nxt;
+                            nxt = L.step[k + 1];
+                            tc_mma<MODE_FLEX16>(dd, a_hi | st, b_hi | b, id, acc);
+                            acc = 1;
+                        }
                     }
                     if (!split) mbar_arrive(&tmem_full[s]);
                     tc_commit(&tmem_full[s]);
@@ -378,7 +424,7 @@ conv_chain_kernel(const __grid_constant__ Chain p) {
             }
             // nothing of this thread's is at work any more when the block ends, also where a wait ran out
             tc_commit(issued);
-            if (!mbar_wait(issued, 0)) ok = false;
+            if (!bar_wait(issued, 0)) ok = false;
             if (!ok) atomicExch(fail_flag, 1);
         }
     } else {
@@ -397,9 +443,9 @@ conv_chain_kernel(const __grid_constant__ Chain p) {
                 epilogue_barrier();
             }
             const int nsets = L.nsets, epi_w = 4 / nsets, set = slot / epi_w, part = slot - set * epi_w;
-            const int kt = L.K, n2 = L.n2, tiles = L.tiles, tcols = L.tcols, cgs = kt >> 4;
+            const int kt = L.K, n2 = L.n2, tiles = L.tiles, tcols = L.tcols;
             const float2 sc = scale_s[l];
-            const float f = sc.x, r = sc.y;
+            const unsigned long long f = pack2(sc.x, sc.x), r = pack2(sc.y, sc.y);
             const float* bias = bias_s + (l & 1) * kChannelsMost;
             const unsigned d1 = tmem_base + (unsigned)(2 * set * n2) + ((unsigned)(quarter * 32) << 16), d2 = d1 + n2;
             const bool has_res = L.has_res && img < n_img, has_out = L.has_out && img < n_img, short_sum = L.short_sum;
@@ -410,91 +456,70 @@ conv_chain_kernel(const __grid_constant__ Chain p) {
             const unsigned floor2 = L.relu ? 0u : 0x80008000u;
             short* const store = L.dst;
             unsigned smx = 0, smn = 0;                             // pairs: largest and smallest mantissa
+            int tr = set / tcols, tc = set - tr * tcols;
             for (int t = set; t < tiles; t += nsets) {
-                const int tr = t / tcols, tc = t - tr * tcols;
                 const int h = h0 + tr * (16 >> glog), q = q0 + tc * 8;
                 const bool live = h < P && q < Q && img < n_img;
                 uint4* const dst = reinterpret_cast<uint4*>(smem) + out_at + tr * out_tr + tc * out_tc;
                 const uint4* const rsd = reinterpret_cast<const uint4*>(smem) + res_at + tr * res_tr + tc * res_tc;
-                if (ok && !mbar_wait(&tmem_full[set], full_bits >> set & 1u)) { ok = false; atomicExch(fail_flag, 1); }
+                if (ok && !bar_wait(&tmem_full[set], full_bits >> set & 1u)) { ok = false; atomicExch(fail_flag, 1); }
                 full_bits ^= 1u << set;
                 tc_fence_after();
                 const unsigned s_hi = tmem_ld1(d1 + 2 * kt), s_lo = tmem_ld1(d2 + 2 * kt);
-                unsigned hh[2][8], x1[2][8], x2[2][8], ll[2][8];
-                auto load = [&](int half, int c) {
-                    tmem_ld8(d1 + c, hh[half]);
-                    tmem_ld8(d1 + kt + c, x1[half]);
-                    tmem_ld8(d2 + c, x2[half]);
-                    tmem_ld8(d2 + kt + c, ll[half]);
-                };
-                load(0, part * 16);                            // (a set's warps are never more than its channel groups)
-                for (int cg = part; cg < cgs; cg += epi_w) {
-                    unsigned hi[4], lo[4];
-                    uint4 rh = make_uint4(0, 0, 0, 0), rl = rh;
-                    if (has_res && live) {
-                        rh = rsd[cg * res_grp];
-                        rl = rsd[cg * res_grp + res_plane];
+                // eight channels at a time (rolled: the instructions of an unrolled tile would be fetched anew
+                // by every warp that comes to them)
+#pragma unroll 1
+                for (int c = part * 8; c < kt; c += epi_w * 8) {
+                    unsigned v1[16], v2[16], w[4];             // HH | X1, X2 | LL
+                    tmem_ld16(d1 + 2 * c, v1);
+                    tmem_ld16(d2 + 2 * c, v2);
+                    const ulonglong2 b0 = *reinterpret_cast<const ulonglong2*>(bias + c);
+                    const ulonglong2 b1 = *reinterpret_cast<const ulonglong2*>(bias + c + 4);
+                    unsigned long long y[4] = {b0.x, b0.y, b1.x, b1.y};
+                    if (has_res) {
+                        uint2 rh = make_uint2(0, 0), rl = rh;
+                        if (live) {
+                            const uint2* v = reinterpret_cast<const uint2*>(rsd + (c >> 4) * res_grp) + (c >> 3 & 1);
+                            rh = v[0];
+                            rl = v[2 * res_plane];
+                        }
+#pragma unroll
+                        for (int i = 0; i < 2; ++i) {
+                            const unsigned vh = i ? rh.y : rh.x, vl = i ? rl.y : rl.x;
+                            const unsigned a = __byte_perm(vl, vh, 0x5140), b = __byte_perm(vl, vh, 0x7362);
+                            y[2 * i] = fma2(pack2((float)(short)(a & 0xffffu), (float)((int)a >> 16)), r, y[2 * i]);
+                            y[2 * i + 1] = fma2(pack2((float)(short)(b & 0xffffu), (float)((int)b >> 16)), r, y[2 * i + 1]);
+                        }
                     }
                     tmem_ld_wait();
-                    load(1, cg * 16 + 8);
-                    const float fix = 128.0f * (float)(int)(s_hi * 256u + s_lo);
+                    if (c + epi_w * 8 >= kt) {                 // the set may be filled again
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) count_up(&drained[set], nsets);
+                    }
+                    const float fixf = 128.0f * (float)(int)(s_hi * 256u + s_lo);
+                    const unsigned long long fix = pack2(fixf, fixf);
+                    if (short_sum) finish8<true>(v1, v2, fix, f, y, w);
+                    else finish8<false>(v1, v2, fix, f, y, w);
 #pragma unroll
-                    for (int half = 0; half < 2; ++half) {
-                        const int c = cg * 16 + half * 8;
-                        unsigned w[4];
-                        float y[8];
-                        const float4 b0 = *reinterpret_cast<const float4*>(bias + c);
-                        const float4 b1 = *reinterpret_cast<const float4*>(bias + c + 4);
-                        y[0] = b0.x; y[1] = b0.y; y[2] = b0.z; y[3] = b0.w;
-                        y[4] = b1.x; y[5] = b1.y; y[6] = b1.z; y[7] = b1.w;
-                        if (has_res) {
-                            const unsigned vh[2] = {half ? rh.z : rh.x, half ? rh.w : rh.y},
-                                           vl[2] = {half ? rl.z : rl.x, half ? rl.w : rl.y};
-#pragma unroll
-                            for (int i = 0; i < 2; ++i) {
-                                // two mantissas to a word
-                                const unsigned a = __byte_perm(vl[i], vh[i], 0x5140), b = __byte_perm(vl[i], vh[i], 0x7362);
-                                y[4 * i] = fmaf((float)(short)(a & 0xffffu), r, y[4 * i]);
-                                y[4 * i + 1] = fmaf((float)((int)a >> 16), r, y[4 * i + 1]);
-                                y[4 * i + 2] = fmaf((float)(short)(b & 0xffffu), r, y[4 * i + 2]);
-                                y[4 * i + 3] = fmaf((float)((int)b >> 16), r, y[4 * i + 3]);
-                            }
-                        }
-                        if (half) {
-                            tmem_ld_wait();
-                            if (cg + epi_w < cgs) {
-                                load(0, (cg + epi_w) * 16);
-                            } else {
-                                // the set may be filled again
-                                tc_fence_before();
-                                __syncwarp();
-                                if (lane == 0) count_up(&drained[set], nsets);
-                            }
-                        }
-                        if (short_sum) finish8<true>(hh[half], x1[half], x2[half], ll[half], fix, f, y, w);
-                        else finish8<false>(hh[half], x1[half], x2[half], ll[half], fix, f, y, w);
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            w[j] = __vmaxs2(w[j], floor2);
-                            if (live) { smx = __vmaxs2(smx, w[j]); smn = __vmins2(smn, w[j]); }
-                        }
-#pragma unroll
-                        for (int j = 0; j < 2; ++j) {
-                            lo[half * 2 + j] = __byte_perm(w[2 * j], w[2 * j + 1], 0x6420);
-                            hi[half * 2 + j] = __byte_perm(w[2 * j], w[2 * j + 1], 0x7531);
-                        }
-                        if (store && live && ok)
-                            store8(store + ((long long)c * P * Q + h * Q + q) * p.N + n0 + img, (long long)P * Q * p.N, w[0], w[1], w[2], w[3]);
+                    for (int j = 0; j < 4; ++j) w[j] = __vmaxs2(w[j], floor2);
+                    if (live) {
+                        smx = __vmaxs2(__vmaxs2(smx, w[0]), __vmaxs2(__vmaxs2(w[1], w[2]), w[3]));
+                        smn = __vmins2(__vmins2(smn, w[0]), __vmins2(__vmins2(w[1], w[2]), w[3]));
                     }
                     if (has_out && live) {
-                        dst[cg * out_grp] = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-                        dst[cg * out_grp + out_plane] = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+                        uint2* v = reinterpret_cast<uint2*>(dst + (c >> 4) * out_grp) + (c >> 3 & 1);
+                        v[0] = make_uint2(__byte_perm(w[0], w[1], 0x7531), __byte_perm(w[2], w[3], 0x7531));
+                        v[2 * out_plane] = make_uint2(__byte_perm(w[0], w[1], 0x6420), __byte_perm(w[2], w[3], 0x6420));
                     }
+                    if (store && live && ok)
+                        store8(store + ((long long)c * P * Q + h * Q + q) * p.N + n0 + img, (long long)P * Q * p.N, w[0], w[1], w[2], w[3]);
                 }
                 fence_async();
                 __syncwarp();
                 ++stored_tiles;
                 if (lane == 0) publish(&done[slot * 4 + quarter], stored_tiles);
+                for (tc += nsets; tc >= tcols; ++tr) tc -= tcols;
             }
             // the sets of other warps: their phases of this layer
             for (int s = 0; s < nsets; ++s)
@@ -541,9 +566,10 @@ conv_chain_kernel(const __grid_constant__ Chain p) {
 }
 
 // ---- filters ---------------------------------------------------------------------------------------
-// Filters C,R,S,K -> per layer [chunk][row of 16 bytes]: rows 0..K-1 the high bytes of a chunk's 16 input
-// channels for output channel k, rows K..2K-1 their low bytes minus 128, row 2K ones (the sum of the
-// activations).  Channels beyond C, the chunk that pads an odd number and the rows up to n2 are zero.
+// Filters C,R,S,K -> per layer [chunk][row of 16 bytes]: for every eight output channels eight rows with the
+// high bytes of a chunk's 16 input channels and eight with their low bytes minus 128 (so that the epilogue
+// finds what it adds up side by side: a load of tensor memory costs about as much for eight columns as for
+// sixteen), row 2K ones (the sum of the activations).  Channels beyond C, the chunk that pads an odd number and the rows up to n2 are zero.
 struct FilterJob {
     const short* F;
     long long at;
@@ -568,9 +594,9 @@ chain_filters_kernel(const __grid_constant__ FilterJobList list, unsigned char* 
             if (row == 2 * f.K) {
                 v = 1;
             } else {
-                const int k = row < f.K ? row : row - f.K;
+                const int k = (row >> 4) * 8 + (row & 7);
                 const int m = (int)f.F[((long long)c * f.RS + (int)(id >> 8)) * f.K + k];
-                v = (unsigned char)(row < f.K ? m >> 8 : (m & 255) - 128);
+                v = (unsigned char)(row & 8 ? (m & 255) - 128 : m >> 8);
             }
         }
         d[i] = v;
@@ -821,9 +847,9 @@ bool plan_for(const b2_conv_chain_layer* in, int n, int glog, unsigned high, Cha
     return true;
 }
 
-// The plan of a chain: two images to a CTA where that leaves every SM at most one CTA fewer to run
-// (filters are read half as often, and the last stage's 64 pixels fill an instruction's rows), one where
-// the images would not reach all SMs otherwise, or where two do not fit.
+// The plan of a chain: two images to a CTA where one would make more CTAs than there are SMs (a layer of two
+// images takes 1.4 times one of one: filters are read once for both, and 64 pixels of each fill an
+// instruction's rows), one elsewhere, or where two do not fit.
 bool plan(const b2_conv_chain_layer* in, int n, Chain* out, std::vector<FilterJob>* jobs, size_t* filter_bytes) {
     if (n < 1 || n > kLayersMost) return false;
     for (int glog = in[0].dims.N > 148 ? 1 : 0; glog >= 0; --glog) {
@@ -845,6 +871,26 @@ bool plan(const b2_conv_chain_layer* in, int n, Chain* out, std::vector<FilterJo
     return false;
 }
 
+// Whether the chain is the faster way (microseconds, both sides as measured on ResNets of 10 to 22 layers, 8x8
+// to 32x32 pixels, 1 to 2048 images).  The chain: a start of 8, then per layer the hand-overs between its
+// roles and 0.25 a tile -- once per wave of 148 blocks --, and its stores of results that somebody outside
+// reads go to a line each.  One by one: 6 a launch and 1.46e-6 a result, in blocks of 128 images.  22 layers
+// of ResNet-20: 1 image 83 against 175, 100 images 85 / 159 (n = 64), 256 images 120 / 204, 300 images (two
+// waves) 234 / 429, 512 images 237 / 310, 2048 images 828 / 970; ten layers on 16x16 pixels, 1024 images
+// (four waves): 130 / 89, and two layers on 32x32 pixels, 256 images, the second stored: 38 / 21.
+bool faster(const b2_conv_chain_layer* in, const Chain& c) {
+    double chain = 8.0, stores = 0.0, apart = 0.0;
+    for (int l = 0; l < c.n; ++l) {
+        const b2_conv_dims& d = in[l].dims;
+        const double results = (double)d.K * d.P * d.Q;
+        chain += 3.2 + 0.25 * c.layer[l].tiles;
+        if (in[l].out) stores += 0.0006 * results * (1 << c.glog);
+        apart += 6.0 + 1.46e-6 * results * ((d.N + 127) / 128 * 128);
+    }
+    const int blocks = (c.N + (1 << c.glog) - 1) >> c.glog;
+    return (double)((blocks + 147) / 148) * (chain + stores) < apart;
+}
+
 }  // namespace
 
 extern "C" int b2_conv_chain_info(const b2_conv_chain_layer* layers, int32_t n, int32_t* supported,
@@ -853,7 +899,7 @@ extern "C" int b2_conv_chain_info(const b2_conv_chain_layer* layers, int32_t n, 
     std::vector<Chain> c(1);
     std::vector<FilterJob> jobs;
     *filter_bytes = 0;
-    *supported = plan(layers, n, &c[0], &jobs, filter_bytes) ? 1 : 0;
+    *supported = plan(layers, n, &c[0], &jobs, filter_bytes) && faster(layers, c[0]) ? 1 : 0;
     return B2_OK;
 }
 

@@ -246,14 +246,12 @@ class ConvChainStep(_Step):
         if pool is not None:
             self.out_views += pool.out_views
         self.planes = None
+        self.filters = [s.in_views[s.filter_arg].buffer for s in members]
         self.versions = None
-
-    def _filters(self):
-        return [s.in_views[s.filter_arg].buffer for s in self.members]
 
     def refresh(self, t):
         """Filter planes as the chain reads them, made again when filters have changed."""
-        versions = [b.version for b in self._filters()]
+        versions = [b.version for b in self.filters]
         if versions == self.versions:
             return
         n = C.c_int32()
@@ -345,6 +343,9 @@ def chain_convolutions(steps, returned, t):
                         return None
                     if v.buffer in made:
                         kept.add(v.buffer)
+        for layer, s in zip(layers, run):
+            if s.out_views[0].buffer in kept:
+                layer.out = 16               # (an address follows when there is one)
         ok, nbytes = lib.conv_chain_info(layers)
         return ConvChainStep(list(run), layers, nbytes, kept, pool) if ok else None
 

@@ -91,7 +91,7 @@ def test_results_inside_a_chain_are_there_for_who_asks():
     r = np.random.RandomState(2)
     x = ng.placeholder([ng.make_axis(5, name="C"), D, H, W, N])
     cur, mids, filters = x, [], []
-    for i in range(4):
+    for i in range(7):
         K, T = ng.make_axis(16, name="C"), ng.make_axis(1, name="T")
         Kt = ng.make_axis(16, name="K%d" % i)
         f = ng.variable([cur.axes[0], T, ng.make_axis(3, name="R%d" % i), ng.make_axis(3, name="S%d" % i), Kt],
@@ -103,10 +103,10 @@ def test_results_inside_a_chain_are_there_for_who_asks():
         mids.append(cur)
         filters.append(f)
     vals = [r.standard_normal((5, 1, 16, 16, 20)).astype(np.float32)]
-    outs = [mids[2], mids[3]]                        # the third result is returned, and read inside
+    outs = [mids[2], mids[6]]                        # the third result is returned, and read inside
     ref, _ = _run(outs, [x], vals, None)
     got, chains = _run(outs, [x], vals, 1, peek=[mids[1]])
-    assert chains == [4]
+    assert chains == [7]
     for a, b in zip(ref, got):
         for u, v in zip(a[:3], b[:3]):
             assert np.array_equal(u, v)
