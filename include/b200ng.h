@@ -53,8 +53,11 @@ int b2_device_count(void);
  * of the convolution entry points that take planes, so no separate split pass is needed. */
 /* B2_F32_AT (inputs only): the pointer given at launch is the address of a device word that holds the
  * address of the values when the kernel runs, 16-byte aligned.  An fp32 result that is such an input's
- * register, laid out as the input, is not stored where that address is the result's own. */
-enum b2_dtype { B2_F32 = 0, B2_FLEX16 = 1, B2_FLEX16_PLANES = 2, B2_F32_AT = 3 };
+ * register, laid out as the input, is not stored where that address is the result's own.
+ * B2_FLEX16_AT (likewise): where that address is the result's own -- a B2_FLEX16 result with the input's
+ * register, layout and slot, which there has to be -- it holds mantissas; elsewhere fp32 values, which
+ * the program sees as b2_flex_host_quantize would store them (and that result stores so). */
+enum b2_dtype { B2_F32 = 0, B2_FLEX16 = 1, B2_FLEX16_PLANES = 2, B2_F32_AT = 3, B2_FLEX16_AT = 4 };
 
 /* op codes: one per template of float_ew2.py:31-68 */
 enum b2_ew_opcode {
@@ -211,7 +214,8 @@ int b2_flex_publish(int32_t* stats, int32_t n, const int32_t* status, int32_t* h
  * one recorded launch serves every call; so may be the arguments.  table_rows > 0 copies that many
  * rows of the block's scale table to `table` first.
  * where, unless NULL: a device word that gets the address at which the values are to be read -- src for
- * an argument marked in_place, which is then not copied (its reader does that: B2_F32_AT), else dst.
+ * an argument marked in_place, which is then not copied (its reader does that: B2_F32_AT,
+ * B2_FLEX16_AT), else dst.
  * b2_call_outputs is b2_flex_publish with results: dst[k] (pinned host memory) <- bytes[k] bytes of
  * src[k], both 16-byte aligned.
  * b2_call_stage: the address at which the device can read `bytes` bytes of host memory at src:

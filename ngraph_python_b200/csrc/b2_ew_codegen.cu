@@ -233,7 +233,7 @@ inline bool is_flex(int dtype) { return dtype == B2_FLEX16 || dtype == B2_FLEX16
 
 // Emits the per-element body: registers for inputs/constants, the op list.
 bool uses_flex(const b2_ew_program& p) {
-    for (int i = 0; i < p.n_in; ++i) if (p.in[i].dtype == B2_FLEX16) return true;
+    for (int i = 0; i < p.n_in; ++i) if (p.in[i].dtype == B2_FLEX16 || p.in[i].dtype == B2_FLEX16_AT) return true;
     for (int k = 0; k < p.n_out + p.n_red; ++k) if (is_flex(p.out[k].t.dtype)) return true;
     return false;
 }
@@ -245,8 +245,8 @@ int emit_body(std::ostringstream& o, const b2_ew_program& p, const Plan& pl, boo
     for (int i = 0; i < p.n_in; ++i) {
         o << "            const float " << reg(i) << " = ";
         if (p.in[i].sc == 0) o << "xb" << i << ";\n";
-        else if (pl.vec && p.in[i].dtype == B2_FLEX16)
-            o << "b2_elem(w" << i << ", e, s" << i << ", bias" << i << ");\n";
+        else if (pl.vec && (p.in[i].dtype == B2_FLEX16 || p.in[i].dtype == B2_FLEX16_AT))
+            o << "b2_elem(" << (p.in[i].dtype == B2_FLEX16 ? "w" : "m") << i << ", e, s" << i << ", bias" << i << ");\n";
         else if (pl.vec) o << "b2_elem(w" << i << ", e, 1.0f, 0.0f);\n";
         else o << "x" << i << "[e];\n";
     }
@@ -270,7 +270,10 @@ bool prefetchable(const b2_ew_tensor& t, const Plan& pl) { return pl.vec && t.sc
 void emit_raw_loads(std::ostringstream& o, const b2_ew_program& p, const Plan& pl,
                     const std::string& prefix, const std::string& jexpr, const std::string& ind) {
     for (int i = 0; i < p.n_in; ++i)
-        if (prefetchable(p.in[i], pl))
+        if (prefetchable(p.in[i], pl) && p.in[i].dtype == B2_FLEX16_AT)
+            o << ind << "b2_ldraw_at(in" << i << " + (" << jexpr << ") * V, im" << i << " + (" << jexpr << ") * V, fp"
+              << i << ", " << prefix << i << ");\n";
+        else if (prefetchable(p.in[i], pl))
             o << ind << "b2_ldraw(in" << i << " + (" << jexpr << ") * V, " << prefix << i << ");\n";
 }
 
@@ -283,6 +286,15 @@ void emit_loads(std::ostringstream& o, const b2_ew_program& p, const Plan& pl,
         const bool flex = t.dtype == B2_FLEX16;
         if (t.sc == 0) {
             // broadcast along C: the scalar xb<i> is used directly
+        } else if (t.dtype == B2_FLEX16_AT && pl.vec) {
+            o << ind << "const float bias" << i << " = b2_i16_bias(s" << i << ");\n"
+              << ind << "const " << (pl.V == 8 ? "int4" : "int2") << " m" << i << " = b2_mantissas(w" << i << ", fp" << i
+              << ", q_in" << i << ");\n";
+        } else if (t.dtype == B2_FLEX16_AT) {
+            o << ind << "float x" << i << "[V];\n"
+              << ind << "_Pragma(\"unroll\") for (int e = 0; e < V; ++e) x" << i << "[e] = s" << i << " * (float)(fp" << i
+              << " ? b2_as_stored(in" << i << "[(c + e) * p.in_sc[" << i << "]], q_in" << i << ") : (int)im" << i
+              << "[(c + e) * p.in_sc[" << i << "]]);\n";
         } else if (pl.vec) {
             // converted lazily, element by element, inside the body (b2_elem)
             if (flex) o << ind << "const float bias" << i << " = b2_i16_bias(s" << i << ");\n";
@@ -295,7 +307,7 @@ void emit_loads(std::ostringstream& o, const b2_ew_program& p, const Plan& pl,
     }
 }
 
-// The B2_F32_AT input that result k stores as it was read, -1 where it stores something else.  Where the
+// The B2_F32_AT or B2_FLEX16_AT input that result k stores as it was read, -1 where it stores something else.  Where the
 // word holds the result's own address the values are there already: such a result is not stored (put<k>,
 // decided once per block).  Storing them all the same costs 4 bytes a value: four arguments of 8192 x
 // 16384 fp32, three of them with such a result, 0.689 ms, and 0.433 without the stores.
@@ -303,7 +315,16 @@ int stored_input(const b2_ew_program& p, int k) {
     if (k >= p.n_out || p.out[k].reg >= p.n_in) return -1;
     const int i = p.out[k].reg;
     const b2_ew_tensor &in = p.in[i], &out = p.out[k].t;
-    return in.dtype == B2_F32_AT && out.dtype == B2_F32 && in.sa == out.sa && in.sb == out.sb && in.sc == out.sc ? i : -1;
+    const bool same_kind = (in.dtype == B2_F32_AT && out.dtype == B2_F32) ||
+                           (in.dtype == B2_FLEX16_AT && out.dtype == B2_FLEX16 && in.flex_slot == out.flex_slot);
+    return same_kind && in.sa == out.sa && in.sb == out.sb && in.sc == out.sc ? i : -1;
+}
+
+// the result that stores the B2_FLEX16_AT input i, -1 without one
+int result_of(const b2_ew_program& p, int i) {
+    for (int k = 0; k < p.n_out; ++k)
+        if (stored_input(p, k) == i) return k;
+    return -1;
 }
 
 void emit_store_always(std::ostringstream& o, const b2_ew_program& p, const Plan& pl, int k, bool probe,
@@ -342,9 +363,18 @@ void emit_store_always(std::ostringstream& o, const b2_ew_program& p, const Plan
               << "[(c + e) * p.out_sc[" << k << "]] = y" << k << "[e];\n";
         return;
     }
-    o << ind << "{ int m[V];\n"
-      << ind << "  _Pragma(\"unroll\") for (int e = 0; e < V; ++e) { m[e] = b2_f32_to_i16(y" << k
-      << "[e] * q" << k << ", fstat" << k << "); }\n";
+    const int at = stored_input(p, k);
+    if (pl.vec && at >= 0) {                       // (an argument in place: its mantissas are at hand)
+        o << ind << "b2_st_words(o" << k << " + c, m" << at << ", pairs" << k << ");\n";
+        return;
+    }
+    if (pl.vec)
+        o << ind << "{ int m[V / 2];\n"
+          << ind << "  b2_to_words<V>(y" << k << ", q" << k << ", m, pairs" << k << ");\n";
+    else
+        o << ind << "{ int m[V];\n"
+          << ind << "  _Pragma(\"unroll\") for (int e = 0; e < V; ++e) { m[e] = b2_f32_to_i16(y" << k
+          << "[e] * q" << k << ", fstat" << k << "); }\n";
     if (planes && pl.vec)
         o << ind << "  b2_st" << pl.V << "_planes(o" << k << " + c, p.out_plane[" << k << "], m); }\n";
     else if (planes)
@@ -377,14 +407,17 @@ void emit_red_store(std::ostringstream& o, const b2_ew_program& p, int k, bool p
 void emit_prologue(std::ostringstream& o, const b2_ew_program& p, bool probe) {
     const int nres = p.n_out + p.n_red;
     for (int i = 0; i < p.n_in; ++i)
-        if (p.in[i].dtype == B2_FLEX16)
+        if (p.in[i].dtype == B2_FLEX16 || p.in[i].dtype == B2_FLEX16_AT) {
             o << "    const float s" << i << " = p.flex_table[p.in_slot[" << i << "]].scale;\n";
+            if (p.in[i].dtype == B2_FLEX16_AT)
+                o << "    const float q_in" << i << " = p.flex_table[p.in_slot[" << i << "]].inv_scale;\n";
+        }
     for (int k = 0; k < nres; ++k)
         if (is_flex(p.out[k].t.dtype)) {
             if (!probe)
                 o << "    const float q" << k << " = p.flex_table[p.out_slot[" << k
                   << "]].inv_scale;\n";
-            o << "    int stat" << k << " = 0;\n    float fstat" << k << " = 0.0f;\n";
+            o << "    int stat" << k << " = 0;\n    float fstat" << k << " = 0.0f;\n    b2_pairs pairs" << k << " = {0u, 0u};\n";
         }
     for (int i = 0; i < p.n_const; ++i)
         o << "    const float k" << i << " = p.consts[" << i << "];\n";
@@ -397,6 +430,29 @@ void emit_prologue(std::ostringstream& o, const b2_ew_program& p, bool probe) {
             o << "    const float rq" << k << " = p.flex_table[p.out_slot[" << k << "]].inv_scale;\n"
               << "    const float rs" << k << " = p.flex_table[p.out_slot[" << k << "]].scale;\n";
         }
+}
+
+// The statistics of the first `nstat` results: one barrier for all of them, a warp to each after it, one
+// atomic per block and result.  (One after the other, two barriers each, and with two more for every row
+// reduction they were 17 of 346 us of the flex16 kernel over 8192 x 16384 values.)
+void emit_stats(std::ostringstream& o, const b2_ew_program& p, int nstat) {
+    std::vector<int> ks;
+    for (int k = 0; k < nstat; ++k)
+        if (is_flex(p.out[k].t.dtype)) ks.push_back(k);
+    if (ks.empty()) return;
+    o << "    {\n        __shared__ int top[" << ks.size() << "][THREADS / 32];\n"
+      << "        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;\n";
+    for (size_t q = 0; q < ks.size(); ++q) {
+        const int k = ks[q];
+        o << "        { const int v = __reduce_max_sync(0xffffffffu, max(max(stat" << k << ", b2_pairs_to_int(pairs" << k
+          << ")), b2_stat_to_int(fstat" << k << "))); if (lane == 0) top[" << q << "][warp] = v; }\n";
+    }
+    o << "        __syncthreads();\n        if (warp < " << ks.size() << ") {\n"
+      << "            const int v = __reduce_max_sync(0xffffffffu, lane < THREADS / 32 ? top[warp][lane] : 0);\n"
+      << "            const int slot = ";
+    for (size_t q = 0; q + 1 < ks.size(); ++q) o << "warp == " << q << " ? p.out_slot[" << ks[q] << "] : ";
+    o << "p.out_slot[" << ks.back() << "];\n"
+      << "            if (lane == 0 && v > 0) atomicMax(p.flex_stats + slot, v);\n        }\n    }\n";
 }
 
 void emit_finalize(std::ostringstream& o, const b2_ew_program& p, bool probe) {
@@ -419,17 +475,14 @@ void emit_finalize(std::ostringstream& o, const b2_ew_program& p, bool probe) {
             o << "        }\n";
         }
         o << "    }\n";
-        for (int k = p.n_out; k < nres; ++k)
-            if (is_flex(p.out[k].t.dtype))
-                o << "    b2_block_stat(max(stat" << k << ", b2_stat_to_int(fstat" << k
-                  << ")), p.flex_stats + p.out_slot[" << k << "], reinterpret_cast<int*>(smem));\n";
+        emit_stats(o, p, nres);
         o << "}\n";
     }
 
-// where input i lies: the pointer given, or (B2_F32_AT) what the word it points to holds by now, read once
+// where input i lies: the pointer given, or (B2_F32_AT, B2_FLEX16_AT) what the word it points to holds by now, read once
 std::string input_pointer(const b2_ew_program& p, int i) {
     std::ostringstream o;
-    if (p.in[i].dtype == B2_F32_AT) o << "at" << i;
+    if (p.in[i].dtype == B2_F32_AT || p.in[i].dtype == B2_FLEX16_AT) o << "at" << i;
     else o << "(const " << ctype(p.in[i].dtype) << "*)p.in[" << i << "]";
     return o.str();
 }
@@ -466,12 +519,22 @@ int generate(const b2_ew_program& p, const Plan& pl, bool probe, std::string* ou
         o << "    const b2_i64 block_x = blockIdx.x, blocks_x = gridDim.x, block_y = blockIdx.y, blocks_y = gridDim.y;\n";
     emit_prologue(o, p, probe);
     for (int i = 0; i < p.n_in; ++i)
-        if (p.in[i].dtype == B2_F32_AT)
+        if (p.in[i].dtype == B2_F32_AT || p.in[i].dtype == B2_FLEX16_AT)
             o << "    const float* const at" << i << " = *(const float* const volatile*)p.in[" << i << "];\n";
     for (int k = 0; k < p.n_out && !probe; ++k)
         if (stored_input(p, k) >= 0)
             o << "    const bool put" << k << " = at" << stored_input(p, k) << " != (const float*)p.out[" << k << "];\n";
+    // B2_FLEX16_AT: fp32 values, or the mantissas where its result has them already
+    for (int i = 0; i < p.n_in; ++i)
+        if (p.in[i].dtype == B2_FLEX16_AT)
+            o << "    const bool fp" << i << " = at" << i << " != (const float*)p.out[" << result_of(p, i) << "];\n";
 
+    // rows of a block: the warps' shares meet behind one barrier a row (two sets in turn), then a warp adds
+    // up each reduction while the others start on the next row
+    bool meet = false;
+    if (p.reduce_mode == B2_REDUCE_C && pl.group != 32)
+        for (int k = p.n_out; k < nres; ++k) meet |= !is_arg(p.out[k].redop);
+    if (meet) o << "    __shared__ float share[2][NRED][THREADS / 32];\n    int turn = 0;\n";
     if (p.reduce_mode != B2_REDUCE_B) {
         o << "    const b2_i64 rows = p.A * p.B;\n"
           << "    const b2_i64 chunks = p.C / V;\n"
@@ -483,6 +546,8 @@ int generate(const b2_ew_program& p, const Plan& pl, bool probe, std::string* ou
             const char* ct = ctype(p.in[i].dtype);
             o << "        const " << ct << "* in" << i << " = " << input_pointer(p, i)
               << " + a_idx * p.in_sa[" << i << "] + b_idx * p.in_sb[" << i << "];\n";
+            if (p.in[i].dtype == B2_FLEX16_AT)
+                o << "        const short* im" << i << " = (const short*)at" << i << " + (in" << i << " - at" << i << ");\n";
             if (p.in[i].sc == 0) {
                 o << "        const float xb" << i << " = ";
                 if (p.in[i].dtype == B2_FLEX16) o << "s" << i << " * (float)";
@@ -559,27 +624,34 @@ int generate(const b2_ew_program& p, const Plan& pl, bool probe, std::string* ou
                     o << "        b2_block_reduce_arg<" << rn << ">(acc" << k << ", idx" << k
                       << ", smem);\n";
                 else
-                    o << "        acc" << k << " = b2_block_reduce<" << rn << ">(acc" << k
-                      << ", smem);\n";
+                    o << "        acc" << k << " = b2_warp_reduce<" << rn << ">(acc" << k << ");\n"
+                      << "        if ((threadIdx.x & 31) == 0) share[turn][" << (k - p.n_out) << "][threadIdx.x >> 5] = acc" << k << ";\n";
             }
         }
-        if (p.n_red > 0) {
-            o << "        if (gl == 0) {\n";
-            for (int k = p.n_out; k < nres; ++k) {
-                if (split) {
-                    o << "            p.scratch[(block_x * rows + r) * NRED + "
-                      << (k - p.n_out) << "] = acc" << k << ";\n";
-                } else {
-                    const std::string val = is_arg(p.out[k].redop)
-                                                ? "(float)idx" + std::to_string(k)
-                                                : "acc" + std::to_string(k);
-                    const std::string addr = "a_idx * p.out_sa[" + std::to_string(k) +
-                                             "] + b_idx * p.out_sb[" + std::to_string(k) + "]";
-                    emit_red_store(o, p, k, probe, val, addr, "            ");
-                }
+        if (meet) o << "        __syncthreads();\n";
+        for (int k = p.n_out; k < nres; ++k) {
+            const bool met = meet && !is_arg(p.out[k].redop);
+            if (met)
+                o << "        if (threadIdx.x >> 5 == " << (k - p.n_out) << ") {\n"
+                  << "            acc" << k << " = b2_warp_reduce<" << red_name(p.out[k].redop) << ">((threadIdx.x & 31) < THREADS / 32 ? share[turn]["
+                  << (k - p.n_out) << "][threadIdx.x & 31] : b2_red_init<" << red_name(p.out[k].redop) << ">());\n"
+                  << "            if ((threadIdx.x & 31) == 0) {\n";
+            else
+                o << "        {\n            if (gl == 0) {\n";
+            if (split) {
+                o << "                p.scratch[(block_x * rows + r) * NRED + "
+                  << (k - p.n_out) << "] = acc" << k << ";\n";
+            } else {
+                const std::string val = is_arg(p.out[k].redop)
+                                            ? "(float)idx" + std::to_string(k)
+                                            : "acc" + std::to_string(k);
+                const std::string addr = "a_idx * p.out_sa[" + std::to_string(k) +
+                                         "] + b_idx * p.out_sb[" + std::to_string(k) + "]";
+                emit_red_store(o, p, k, probe, val, addr, "                ");
             }
-            o << "        }\n";
+            o << "            }\n        }\n";
         }
+        if (meet) o << "        turn ^= 1;\n";
         o << "    }\n";
     } else {
         // REDUCE_B: threads run along C, every thread walks the B axis.
@@ -601,6 +673,8 @@ int generate(const b2_ew_program& p, const Plan& pl, bool probe, std::string* ou
             const char* ct = ctype(p.in[i].dtype);
             o << "            const " << ct << "* in" << i << " = " << input_pointer(p, i)
               << " + a_idx * p.in_sa[" << i << "] + b_idx * p.in_sb[" << i << "];\n";
+            if (p.in[i].dtype == B2_FLEX16_AT)
+                o << "            const short* im" << i << " = (const short*)at" << i << " + (in" << i << " - at" << i << ");\n";
             if (p.in[i].sc == 0) {
                 o << "            const float xb" << i << " = ";
                 if (p.in[i].dtype == B2_FLEX16) o << "s" << i << " * (float)";
@@ -653,13 +727,7 @@ int generate(const b2_ew_program& p, const Plan& pl, bool probe, std::string* ou
     }
     // flex statistics: one atomic per CTA and output.  In split mode the reduction outputs are
     // produced (and counted) by the finalize kernel.
-    {
-        const int nstat = split ? p.n_out : nres;
-        for (int k = 0; k < nstat; ++k)
-            if (is_flex(p.out[k].t.dtype))
-                o << "    b2_block_stat(max(stat" << k << ", b2_stat_to_int(fstat" << k
-                  << ")), p.flex_stats + p.out_slot[" << k << "], reinterpret_cast<int*>(smem));\n";
-    }
+    emit_stats(o, p, split ? p.n_out : nres);
     o << "}\n";
 
     if (split) emit_finalize(o, p, probe);
@@ -833,13 +901,7 @@ int generate_staged(const b2_ew_program& p, const Plan& pl, bool probe, std::str
       << "        }\n"
       << "    }\n"
       << "    if (timed_out && p.status) atomicExch(p.status, 1);\n";
-    {
-        const int nstat = split ? p.n_out : nres;
-        for (int k = 0; k < nstat; ++k)
-            if (is_flex(p.out[k].t.dtype))
-                o << "    b2_block_stat(max(stat" << k << ", b2_stat_to_int(fstat" << k
-                  << ")), p.flex_stats + p.out_slot[" << k << "], reinterpret_cast<int*>(smem));\n";
-    }
+    emit_stats(o, p, split ? p.n_out : nres);
     o << "}\n";
     if (split) emit_finalize(o, p, probe);
     *out_src = o.str();
@@ -866,7 +928,7 @@ bool vector_ok(const b2_ew_program& p, int V) {
 Plan make_plan(const b2_ew_program& p, bool want_vec) {
     Plan pl;
     bool any16 = false;
-    for (int i = 0; i < p.n_in; ++i) any16 |= p.in[i].dtype == B2_FLEX16;
+    for (int i = 0; i < p.n_in; ++i) any16 |= p.in[i].dtype == B2_FLEX16 || p.in[i].dtype == B2_FLEX16_AT;
     for (int k = 0; k < p.n_out; ++k) any16 |= is_flex(p.out[k].t.dtype);
     pl.V = 1;
     pl.vec = false;
@@ -929,7 +991,7 @@ Plan make_plan(const b2_ew_program& p, bool want_vec) {
     const char* env = getenv("B2_EW_STAGED");
     const bool allow = env && env[0] == '1';   // off by default: measured slower than plain loads
     bool at = false;
-    for (int i = 0; i < p.n_in; ++i) at |= p.in[i].dtype == B2_F32_AT;
+    for (int i = 0; i < p.n_in; ++i) at |= p.in[i].dtype == B2_F32_AT || p.in[i].dtype == B2_FLEX16_AT;
     if (allow && !at && pl.vec && p.reduce_mode != B2_REDUCE_B && pl.group == kThreads &&
         rows < (1LL << 30) && chunks < (1LL << 30)) {
         int bytes = 0;
@@ -1008,10 +1070,12 @@ int validate(const b2_ew_program& p) {
             B2_REQUIRE(p.out[k].redop >= B2_RED_SUM && p.out[k].redop <= B2_RED_ARGMIN, "bad redop");
     }
     for (int i = 0; i < p.n_in; ++i) {
-        B2_REQUIRE(p.in[i].dtype == B2_F32 || p.in[i].dtype == B2_FLEX16 || p.in[i].dtype == B2_F32_AT,
-                   "bad input dtype");
-        if (p.in[i].dtype == B2_FLEX16)
+        B2_REQUIRE(p.in[i].dtype == B2_F32 || p.in[i].dtype == B2_FLEX16 || p.in[i].dtype == B2_F32_AT ||
+                   p.in[i].dtype == B2_FLEX16_AT, "bad input dtype");
+        if (p.in[i].dtype == B2_FLEX16 || p.in[i].dtype == B2_FLEX16_AT)
             B2_REQUIRE(p.in[i].flex_slot >= 0, "flex input %d has no slot", i);
+        if (p.in[i].dtype == B2_FLEX16_AT)
+            B2_REQUIRE(p.in[i].sc != 0 && result_of(p, i) >= 0, "argument %d has no result that stores it", i);
     }
     return B2_OK;
 }
@@ -1153,7 +1217,7 @@ int variant_for(const b2_ew_kernel* k, const void* const* in, void* const* out, 
     int vec = k->can_vec ? 1 : 0;
     for (int i = 0; i < p.n_in; ++i) {
         B2_REQUIRE(in[i], "input %d is null", i);
-        if (vec && p.in[i].sc == 1 && p.in[i].dtype != B2_F32_AT && !aligned16(in[i])) vec = 0;
+        if (vec && p.in[i].sc == 1 && p.in[i].dtype != B2_F32_AT && p.in[i].dtype != B2_FLEX16_AT && !aligned16(in[i])) vec = 0;
     }
     for (int q = 0; q < p.n_out + p.n_red; ++q) {
         B2_REQUIRE(out[q], "result %d is null", q);

@@ -68,6 +68,32 @@ __device__ __forceinline__ float b2_requant(float v, float q, float s) {
     return (float)b2_f32_to_i16(v * q, unused) * s;
 }
 
+// The same for the vector forms: two values a word, converted (to int32, which rounds and makes NaN 0) and
+// packed with saturation -- 3.5 instructions a value with the statistic on packed pairs, where clamping,
+// the NaN test and the addition take 8.5.  The conversions are the one thing here that issues at an eighth
+// of a warp a cycle and scheduler: one a stored value is hidden, one a loaded value as well is not.
+__device__ __forceinline__ int b2_pack_sat(int lo, int hi) {
+    int r;
+    asm("cvt.pack.sat.s16.s32 %0, %1, %2;" : "=r"(r) : "r"(hi), "r"(lo));
+    return r;
+}
+struct b2_pairs { unsigned most, least; };             // largest and smallest mantissa of either half
+__device__ __forceinline__ void b2_follow(b2_pairs& s, int w) {
+    s.most = __vmaxs2(s.most, (unsigned)w);
+    s.least = __vmins2(s.least, (unsigned)w);
+}
+__device__ __forceinline__ int b2_pairs_to_int(const b2_pairs& s) {
+    const int hi = max((int)(short)s.most, (int)s.most >> 16), lo = min((int)(short)s.least, (int)s.least >> 16);
+    return max(hi, -lo);
+}
+template <int N> __device__ __forceinline__ void b2_to_words(const float* y, float q, int* w, b2_pairs& s) {
+#pragma unroll
+    for (int e = 0; e < N / 2; ++e) {
+        w[e] = b2_pack_sat(__float2int_rn(y[2 * e] * q), __float2int_rn(y[2 * e + 1] * q));
+        b2_follow(s, w[e]);
+    }
+}
+
 // two int16 mantissas packed in one 32-bit word -> two fp32 values times `scale`, exact:
 // (m ^ 0x8000) placed under the exponent of 2^23 is the float 2^23 + m + 32768.
 __device__ __forceinline__ void b2_i16x2_to_f32(unsigned w, float scale, float bias, float& lo,
@@ -108,6 +134,45 @@ __device__ __forceinline__ void b2_ldraw(const short* p, int4& w) {
 }
 __device__ __forceinline__ void b2_ldraw(const short* p, int2& w) {
     w = __ldcs(reinterpret_cast<const int2*>(p));
+}
+// An argument that is either fp32 values, to be stored as flex16, or the mantissas that are stored already
+// (the same for the whole grid): raw registers of the wider kind.
+__device__ __forceinline__ void b2_ldraw_at(const float* p, const short* m, bool fp, b2_f8& w) {
+    if (fp) {
+        b2_ldraw(p, w);
+    } else {
+        int4 t;
+        b2_ldraw(m, t);
+        w.a = make_float4(__int_as_float(t.x), __int_as_float(t.y), __int_as_float(t.z), __int_as_float(t.w));
+    }
+}
+__device__ __forceinline__ void b2_ldraw_at(const float* p, const short* m, bool fp, float4& w) {
+    if (fp) {
+        b2_ldraw(p, w);
+    } else {
+        int2 t;
+        b2_ldraw(m, t);
+        w.x = __int_as_float(t.x); w.y = __int_as_float(t.y);
+    }
+}
+// The mantissa a host write of x leaves in a flex16 tensor: x / step, clipped to int16 and truncated toward
+// zero (a NaN is clipped to the lowest).
+__device__ __forceinline__ int b2_as_stored(float x, float inv) {
+    return (int)fminf(fmaxf(x * inv, -32768.0f), 32767.0f);
+}
+// two of them in a word; the upper clip is the packing's
+__device__ __forceinline__ int b2_as_stored2(float x, float y, float inv) {
+    return b2_pack_sat((int)fmaxf(x * inv, -32768.0f), (int)fmaxf(y * inv, -32768.0f));
+}
+__device__ __forceinline__ int4 b2_mantissas(const b2_f8& w, bool fp, float inv) {
+    if (!fp)
+        return make_int4(__float_as_int(w.a.x), __float_as_int(w.a.y), __float_as_int(w.a.z), __float_as_int(w.a.w));
+    return make_int4(b2_as_stored2(w.a.x, w.a.y, inv), b2_as_stored2(w.a.z, w.a.w, inv),
+                     b2_as_stored2(w.b.x, w.b.y, inv), b2_as_stored2(w.b.z, w.b.w, inv));
+}
+__device__ __forceinline__ int2 b2_mantissas(const float4& w, bool fp, float inv) {
+    if (!fp) return make_int2(__float_as_int(w.x), __float_as_int(w.y));
+    return make_int2(b2_as_stored2(w.x, w.y, inv), b2_as_stored2(w.z, w.w, inv));
 }
 __device__ __forceinline__ void b2_cvt(const float4& w, float* v, float) {
     v[0] = w.x; v[1] = w.y; v[2] = w.z; v[3] = w.w;
@@ -154,38 +219,31 @@ __device__ __forceinline__ float b2_elem(const int2& w, int e, float scale, floa
     const int word = (e >> 1) == 0 ? w.x : w.y;
     return b2_elem_i16((unsigned)word, e & 1, scale, bias);
 }
-__device__ __forceinline__ int b2_pack_i16x2(int lo, int hi) {
-    return (int)__byte_perm((unsigned)lo, (unsigned)hi, 0x5410);
+// (w: the mantissas by twos)
+__device__ __forceinline__ void b2_st8_i16(short* p, const int* w) {
+    __stcs(reinterpret_cast<int4*>(p), make_int4(w[0], w[1], w[2], w[3]));
 }
-__device__ __forceinline__ void b2_st8_i16(short* p, const int* m) {
-    int4 t;
-    t.x = b2_pack_i16x2(m[0], m[1]);
-    t.y = b2_pack_i16x2(m[2], m[3]);
-    t.z = b2_pack_i16x2(m[4], m[5]);
-    t.w = b2_pack_i16x2(m[6], m[7]);
-    __stcs(reinterpret_cast<int4*>(p), t);
+__device__ __forceinline__ void b2_st4_i16(short* p, const int* w) {
+    __stcs(reinterpret_cast<int2*>(p), make_int2(w[0], w[1]));
 }
 // flex16 results stored as two byte planes (high bytes at p, low bytes `lo` bytes further): the
 // operand format of the convolution kernels, so that no separate split pass is needed
-__device__ __forceinline__ void b2_st8_planes(unsigned char* p, b2_i64 lo, const int* m) {
-    uint2 h, l;
-    const unsigned a = (unsigned)b2_pack_i16x2(m[0], m[1]), b = (unsigned)b2_pack_i16x2(m[2], m[3]);
-    const unsigned c = (unsigned)b2_pack_i16x2(m[4], m[5]), d = (unsigned)b2_pack_i16x2(m[6], m[7]);
-    h.x = __byte_perm(a, b, 0x7531); l.x = __byte_perm(a, b, 0x6420);
-    h.y = __byte_perm(c, d, 0x7531); l.y = __byte_perm(c, d, 0x6420);
-    __stcs(reinterpret_cast<uint2*>(p), h);
-    __stcs(reinterpret_cast<uint2*>(p + lo), l);
+__device__ __forceinline__ void b2_st8_planes(unsigned char* p, b2_i64 lo, const int* w) {
+    __stcs(reinterpret_cast<uint2*>(p), make_uint2(__byte_perm(w[0], w[1], 0x7531), __byte_perm(w[2], w[3], 0x7531)));
+    __stcs(reinterpret_cast<uint2*>(p + lo), make_uint2(__byte_perm(w[0], w[1], 0x6420), __byte_perm(w[2], w[3], 0x6420)));
 }
-__device__ __forceinline__ void b2_st4_planes(unsigned char* p, b2_i64 lo, const int* m) {
-    const unsigned a = (unsigned)b2_pack_i16x2(m[0], m[1]), b = (unsigned)b2_pack_i16x2(m[2], m[3]);
-    __stcs(reinterpret_cast<unsigned*>(p), __byte_perm(a, b, 0x7531));
-    __stcs(reinterpret_cast<unsigned*>(p + lo), __byte_perm(a, b, 0x6420));
+__device__ __forceinline__ void b2_st4_planes(unsigned char* p, b2_i64 lo, const int* w) {
+    __stcs(reinterpret_cast<unsigned*>(p), __byte_perm(w[0], w[1], 0x7531));
+    __stcs(reinterpret_cast<unsigned*>(p + lo), __byte_perm(w[0], w[1], 0x6420));
 }
-__device__ __forceinline__ void b2_st4_i16(short* p, const int* m) {
-    int2 t;
-    t.x = b2_pack_i16x2(m[0], m[1]);
-    t.y = b2_pack_i16x2(m[2], m[3]);
-    __stcs(reinterpret_cast<int2*>(p), t);
+// an argument's mantissas as read
+__device__ __forceinline__ void b2_st_words(short* p, const int4& w, b2_pairs& s) {
+    __stcs(reinterpret_cast<int4*>(p), w);
+    b2_follow(s, w.x); b2_follow(s, w.y); b2_follow(s, w.z); b2_follow(s, w.w);
+}
+__device__ __forceinline__ void b2_st_words(short* p, const int2& w, b2_pairs& s) {
+    __stcs(reinterpret_cast<int2*>(p), w);
+    b2_follow(s, w.x); b2_follow(s, w.y);
 }
 
 // ---- reductions across a warp / a CTA ---------------------------------------------------------

@@ -10,7 +10,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(HERE, "libb200ng.so")
 
 EW_MAX_IN, EW_MAX_OUT, EW_MAX_CONST, EW_MAX_OPS = 12, 6, 16, 96
-F32, FLEX16, FLEX16_PLANES, F32_AT = 0, 1, 2, 3
+F32, FLEX16, FLEX16_PLANES, F32_AT, FLEX16_AT = 0, 1, 2, 3, 4
 REDUCE_NONE, REDUCE_C, REDUCE_B = 0, 1, 2
 
 OPCODES = {

@@ -1311,11 +1311,12 @@ class _Planner(object):
 
     def _takes_argument(self, view, strides, dims):
         """Whether an elementwise kernel over dims = (A, B, C) may read this view from where the
-        caller's tensor lies: a large fp32 argument that nothing has read yet, every value of it
-        exactly once."""
+        caller's tensor lies: a large argument that nothing has read yet or writes, every value of it
+        exactly once (flex16: and that no convolution reads as byte planes)."""
         buf = view.buffer
         A, B, C = dims
-        return (not self.t.flex and buf in self.parameter_buffers and buf not in self.read_so_far and
+        return (buf.plane_bytes == 0 and buf.last_write_step < 0 and
+                buf in self.parameter_buffers and buf not in self.read_so_far and
                 4 * buf.size >= self.THROUGH_LEAST and view.is_dense() and A * B * C == buf.size and
                 strides[2] == 1 and (B == 1 or strides[1] == C) and (A == 1 or strides[0] == B * C))
 
@@ -1553,9 +1554,9 @@ class _Planner(object):
                              for k, d in enumerate(outs + reds)]
         step.stores_argument = []
         for i, (v, st) in enumerate(zip(in_views, abc[:n_in])):
-            # in a recorded call the first reader of a large fp32 argument reads it from wherever the
+            # in a recorded call the first reader of a large argument reads it from wherever the
             # caller has it and stores it on the way: a copy in front of the kernel reads it once more
-            # (512 MB: 173 us of a call of 640)
+            # (8192 x 16384 values, fp32: 173 us of a call of 640; flex16: 120 of 444)
             if self._takes_argument(v, st, dims) and \
                     len(outs) + len(reds) + len(step.stores_argument) < fusion.MAX_OUT:
                 step.stores_argument.append(i)
@@ -1564,9 +1565,9 @@ class _Planner(object):
             self.read_so_far.update(v.buffer for v in pre.in_views)
         prog = lib.make_program(dims, inputs, consts, ops, outs, reds, mode)
         if step.stores_argument:
-            at = [dict(d, dtype=lib.F32_AT) if i in step.stores_argument else d
-                  for i, d in enumerate(inputs)]
-            stores = [dict(dtype=lib.F32, strides=abc[i], slot=-1, reg=i) for i in step.stores_argument]
+            at = [dict(d, dtype=lib.FLEX16_AT if d["dtype"] == lib.FLEX16 else lib.F32_AT)
+                  if i in step.stores_argument else d for i, d in enumerate(inputs)]
+            stores = [dict(inputs[i], reg=i) for i in step.stores_argument]
             step.recorded_program = lib.make_program(dims, at, consts, ops, outs + stores, reds, mode)
         step.kernel = lib.PlannedKernel(prog, self.t.flex) if self.t.plan_only else lib.EwKernel(prog)
         step.in_views = in_views
