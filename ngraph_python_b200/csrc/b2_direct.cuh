@@ -2,12 +2,12 @@
 // launch, for problems where the pre-pass of the plane kernel (b2_gemm_impl.cuh) and its launches
 // cost as much as the product, and for convolutions that would otherwise be unrolled in memory.
 //
-// One CTA per 128 x BN tile (times a slice of K), 288 threads:
-//   warps 0-7: producers -- load a k-block of both operands from wherever it lies (K contiguous,
-//              rows contiguous, or rows gathered from a C,H,W,N tensor through a table of column
-//              offsets), split it into its two planes and store them K-major, 128-byte swizzled,
-//              into a ring of stages; afterwards the epilogue;
-//   warp 8:    tensor memory, tcgen05.mma issue.
+// One CTA per 128 x BN tile (times a slice of K), 288 or 544 threads:
+//   one or two groups of eight warps: producers -- load a k-block of both operands from wherever it
+//              lies (K contiguous, rows contiguous, or rows gathered from a C,H,W,N tensor through a
+//              table of column offsets), split it into its two planes and store them K-major, 128-byte
+//              swizzled, into a ring of stages, the groups by turns; the first group afterwards the epilogue;
+//   the last warp: tensor memory, tcgen05.mma issue.
 // A k-block is 128 bytes of plane: 32 fp32 or 128 int16 values.
 //   fp32:   3xTF32, in chains of at most 16 k-blocks (the tensor core's fp32 sum truncates); longer K
 //           is cut into slices.  Matrix products add hi*hi, hi*lo and lo*hi into one sum (see ONE_CHAIN).
@@ -20,7 +20,9 @@
 //
 // What bounds it: at the sizes it is chosen for, latency -- launch, first loads, one pass through the
 // ring, the exchange in the cluster -- so the split is taken to give every SM a CTA; for unrolled
-// convolutions the producers' issue slots.
+// convolutions the producers' issue slots.  The second group halves what a k-block waits for where an SM has
+// one CTA (one B200, one group -> two, us: fp32 512 x 128 x 784 16.7 -> 11.5, 600 x 600 x 600 24.5 -> 14.6,
+// flex16 512 x 128 x 784 11.0 -> 8.7, 905 x 380 x 611 24.1 -> 15.0; 20 % of it over 38 sizes).
 #ifndef B2_DIRECT_CUH
 #define B2_DIRECT_CUH
 #include "b2_direct.h"
@@ -30,9 +32,14 @@ namespace {
 
 constexpr int kDirThreads = 288;
 constexpr int kDirMaxK = 4608;            // columns of the gather table
-__host__ __device__ constexpr int dir_stages(int bn) { return bn == 128 ? 3 : 2; }
+// groups: producers in groups of eight warps, each with a k-block of its own; more than one only where every
+// SM has a single CTA, which then has the shared memory for a deeper ring
+__host__ __device__ constexpr int dir_stages(int bn, int groups = 1) {
+    return groups > 1 ? (bn >= 64 ? 3 : 4) : bn == 128 ? 3 : 2;
+}
+__host__ __device__ constexpr int dir_threads(int groups) { return groups * 256 + 32; }
 __host__ __device__ constexpr int dir_stage_bytes(int bn) { return 2 * (128 + bn) * 128; }
-__host__ __device__ constexpr int dir_ring_bytes(int bn) { return dir_stages(bn) * dir_stage_bytes(bn); }
+__host__ __device__ constexpr int dir_ring_bytes(int bn, int groups = 1) { return dir_stages(bn, groups) * dir_stage_bytes(bn); }
 __host__ __device__ constexpr int dir_tmem_cols(int mode, int bn) {
     int need = (mode == MODE_FLEX16 ? 3 : 2) * bn, c = 32;
     while (c < need) c *= 2;
@@ -166,12 +173,12 @@ struct OperandTile {
     }
 };
 
-template <int MODE, int BN, int AK>
-__global__ void __launch_bounds__(kDirThreads, (BN == 128 ? 1 : 2))
+template <int MODE, int BN, int AK, int G>
+__global__ void __launch_bounds__(dir_threads(G), (BN == 128 || G > 1 ? 1 : 2))
 direct_kernel(const __grid_constant__ DirectParams p) {
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    constexpr int NST = dir_stages(BN), STAGE = dir_stage_bytes(BN);
+    constexpr int NST = dir_stages(BN, G), STAGE = dir_stage_bytes(BN), MMA_WARP = 8 * G;
     constexpr int KB = MODE == MODE_FLEX16 ? 128 : 32;            // columns of a k-block
     constexpr int PER = KB / 8;                                   // columns of a 16-byte chunk
     constexpr int kCols = dir_tmem_cols(MODE, BN);
@@ -190,7 +197,8 @@ direct_kernel(const __grid_constant__ DirectParams p) {
     int2* ftab = tab + p.kb_per_split * KB;                                       // likewise, of the filters
     const bool tiled = AK == B2_OPERAND_GATHER && filter_tiles(p.a);
 
-    const int warp = warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
+    // (warp: within its group of eight)
+    const int wid = warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31, group = wid >> 3, warp = wid & 7;
     const b2_direct_args& a = p.a;
     const int m0 = blockIdx.y * 128, n0 = blockIdx.x * BN;
     const int rank = blockIdx.z, kb0 = rank * p.kb_per_split;
@@ -202,7 +210,7 @@ direct_kernel(const __grid_constant__ DirectParams p) {
         *fail_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 8) {
+    if (wid == MMA_WARP) {
         tmem_alloc(tmem_holder, kCols);
         // the next kernel may start its set-up now: not before this CTA holds its tensor memory, or
         // the two could each wait for what the other has
@@ -212,7 +220,7 @@ direct_kernel(const __grid_constant__ DirectParams p) {
         // offset of every column of this slice and the bit of its tap (none beyond K)
         const b2_gather& g = a.g;
         const int RS = g.R * g.S;
-        for (int i = threadIdx.x; i < nkb * KB; i += kDirThreads) {
+        for (int i = threadIdx.x; i < nkb * KB; i += dir_threads(G)) {
             const int k = kb0 * KB + i;
             int2 e = make_int2(0, 0), f = make_int2(0, 0x7fff7fff);       // (no filter has that tap)
             if (k < a.K) {
@@ -231,7 +239,7 @@ direct_kernel(const __grid_constant__ DirectParams p) {
     tc_fence_after();
     const unsigned tmem_base = (unsigned)warp_uniform((int)*tmem_holder);
 
-    if (warp < 8) {
+    if (wid < MMA_WARP) {
         // ---- producers
         // fp32 loads a k-block ahead; a flex16 k-block is 128 columns, few of them make a problem, and a
         // second set of registers would spill
@@ -355,24 +363,30 @@ direct_kernel(const __grid_constant__ DirectParams p) {
                 B.load_k(a.B, b_at, k0, a.K - k0, p.b_vec, lane);
             } else {
                 // chunk = warp, groups of 32 (64) rows
+                const bool whole = k0 + KB <= a.K;
+                const char* from = (const char*)a.B + (n0 + lane + (long long)(k0 + warp * PER) * a.b_ks) * 4;
 #pragma unroll
                 for (int i = 0; i < BTile::kUnits; ++i) {
-                    const int lr = MODE == MODE_FLEX16 ? i * 64 + 2 * lane : i * 32 + lane, row = n0 + lr;
+                    if (MODE != MODE_FLEX16) {
+                        const bool there = i * 32 + lane < BN && n0 + i * 32 + lane < a.N;
+                        const float* s = (const float*)from + i * 32;
+#pragma unroll
+                        for (int j = 0; j < PER; ++j, s += a.b_ks)
+                            B.r[PER * i + j] = there && (whole || k0 + warp * PER + j < a.K) ? __float_as_uint(__ldg(s)) : 0u;
+                        continue;
+                    }
+                    const int lr = i * 64 + 2 * lane, row = n0 + lr;
                     const bool in0 = lr < BN && row < a.N, in1 = lr + 1 < BN && row + 1 < a.N;
 #pragma unroll
                     for (int j = 0; j < PER; ++j) {
                         const int k = k0 + warp * PER + j;
                         unsigned v = 0;
                         if (k < a.K) {
-                            if (MODE == MODE_FLEX16) {
-                                const unsigned short* s = (const unsigned short*)a.B + row + (long long)k * a.b_ks;
-                                if (p.b_vec && in1) v = __ldg((const unsigned*)s);
-                                else {
-                                    if (in0) v = __ldg(s);
-                                    if (in1) v |= (unsigned)__ldg(s + 1) << 16;
-                                }
-                            } else if (in0) {
-                                v = __float_as_uint(__ldg((const float*)a.B + row + (long long)k * a.b_ks));
+                            const unsigned short* s = (const unsigned short*)a.B + row + (long long)k * a.b_ks;
+                            if (p.b_vec && in1) v = __ldg((const unsigned*)s);
+                            else {
+                                if (in0) v = __ldg(s);
+                                if (in1) v |= (unsigned)__ldg(s + 1) << 16;
                             }
                         }
                         B.r[PER * i + j] = v;
@@ -406,24 +420,25 @@ direct_kernel(const __grid_constant__ DirectParams p) {
                 }
             }
         };
-        if (AHEAD) load(0, ta[0], tb[0]);
-        int s = 0;
+        if (AHEAD && group < nkb) load(group, ta[0], tb[0]);
+        int s = group % NST;
         unsigned parity = 1;
         bool ok = true;
         auto put = [&](int kb, ATile& A, BTile& B, ATile& An, BTile& Bn) {
             if (!AHEAD) load(kb, A, B);
-            else if (kb + 1 < nkb) load(kb + 1, An, Bn);          // in flight while this one is stored
+            else if (kb + G < nkb) load(kb + G, An, Bn);          // in flight while this one is stored
             if (ok && !mbar_wait(&empty_bar[s], parity)) { atomicExch(fail_flag, 1); ok = false; }
             store(s, A, B);
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncwarp();
             if (lane == 0) mbar_arrive(&full_bar[s]);
-            if (++s == NST) { s = 0; parity ^= 1u; }
+            s += G;
+            if (s >= NST) { s -= NST; parity ^= 1u; }
         };
         constexpr int kNext = AHEAD ? 1 : 0;
-        for (int kb = 0; kb < nkb; kb += 2) {
+        for (int kb = group; kb < nkb; kb += 2 * G) {
             put(kb, ta[0], tb[0], ta[kNext], tb[kNext]);
-            if (kb + 1 < nkb) put(kb + 1, ta[kNext], tb[kNext], ta[0], tb[0]);
+            if (kb + G < nkb) put(kb + G, ta[kNext], tb[kNext], ta[0], tb[0]);
         }
     } else if (elect_one()) {
         // ---- MMA issue
@@ -477,7 +492,7 @@ direct_kernel(const __grid_constant__ DirectParams p) {
     int stat = 0;
     unsigned long long pmax = 0;
     int sh = 0;
-    if (MODE == MODE_FLEX16 && warp < 8) {
+    if (MODE == MODE_FLEX16 && wid < 8) {
         const float q_out = a.probe ? 1.0f : a.table[a.slotC].inv_scale;
         sh = -ilogbf(a.table[a.slotA].scale * a.table[a.slotB].scale * q_out);
     }
@@ -569,7 +584,7 @@ direct_kernel(const __grid_constant__ DirectParams p) {
             }
         }
     };
-    if (warp < 8) {
+    if (wid < 8) {
         ok = mbar_wait(tmem_full, 0);
         if (!ok) atomicExch(fail_flag, 1);
         tc_fence_after();
@@ -606,24 +621,37 @@ direct_kernel(const __grid_constant__ DirectParams p) {
     }
     if (splits > 1) {
         cluster_sync();
-        if (warp < 8) {
+        if (wid < 8) {
             // this CTA's share of the pieces: every splits-th, dealt to the warps of a quarter
             for (int c0 = (rank + half * splits) * 8; c0 < BN; c0 += 16 * splits) {
                 if (n0 + c0 >= a.N) break;
                 Sum v[8];
 #pragma unroll
                 for (int j = 0; j < 8; ++j) v[j] = 0;
-                for (int z = 0; z < splits; ++z) {
-                    const unsigned at = map_rank(red + c0 * 128 + lrow, z);
+                // (a peer's values take about 700 cycles: those of several slices come together)
+                constexpr int Z = MODE == MODE_FLEX16 ? 2 : 4;
+                for (int z0 = 0; z0 < splits; z0 += Z) {
+                    Sum t[Z][8];
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) v[j] += ld_peer(at + j * 128 * (unsigned)sizeof(Sum), (Sum)0);
+                    for (int z = 0; z < Z; ++z) {
+                        if (z0 + z >= splits) break;
+                        const unsigned at = map_rank(red + c0 * 128 + lrow, z0 + z);
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) t[z][j] = ld_peer(at + j * 128 * (unsigned)sizeof(Sum), (Sum)0);
+                    }
+#pragma unroll
+                    for (int z = 0; z < Z; ++z) {
+                        if (z0 + z >= splits) break;
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) v[j] += t[z][j];
+                    }
                 }
                 if (ok) finish(c0, v);
             }
         }
         cluster_sync();                                           // peers may still be reading
     }
-    if (MODE == MODE_FLEX16 && warp < 8) {
+    if (MODE == MODE_FLEX16 && wid < 8) {
         if (a.probe) {
             for (int o = 16; o > 0; o >>= 1) {
                 const unsigned long long t = __shfl_xor_sync(0xffffffffu, pmax, o);
@@ -640,7 +668,7 @@ direct_kernel(const __grid_constant__ DirectParams p) {
     }
     tc_fence_before();
     __syncthreads();
-    if (warp == 8) {
+    if (wid == MMA_WARP) {
         tc_fence_after();
         tmem_dealloc(tmem_base, kCols);
     }
@@ -648,7 +676,7 @@ direct_kernel(const __grid_constant__ DirectParams p) {
 }
 
 // ---- host ------------------------------------------------------------------------------------
-struct DirectShape { int bn, splits, kb_per_split, waves; long long cost; };
+struct DirectShape { int bn, splits, kb_per_split, waves, groups; long long cost; };
 
 template <int MODE>
 DirectShape direct_shape(const b2_direct_args& a) {
@@ -656,7 +684,7 @@ DirectShape direct_shape(const b2_direct_args& a) {
     const int num_kb = (a.K + KB - 1) / KB;
     // fp32: 16 k-blocks to a chain; flex16: exact int32 sums up to 32768 columns
     const int most = MODE == MODE_FLEX16 ? 256 : 16;
-    DirectShape best = {0, 0, 0, 0, -1};
+    DirectShape best = {0, 0, 0, 0, 1, -1};
     const long long tm = (a.M + 127) / 128;
     for (int bn = 16; bn <= 128; bn *= 2) {
         if (bn > 16 && bn / 2 >= a.N) break;
@@ -672,40 +700,54 @@ DirectShape direct_shape(const b2_direct_args& a) {
             // takes 1000 + 6 bn (gathered 2000 to 3500) or 4000 cycles from load to commit when they do
             // not; the two CTAs of an SM overlap.  Gathered rows cost their address and bounds, filters as a tile's pixels see
             // them the same, more where the lanes' rows lie apart; slices of their wide tiles 15000 more.
-            const double ra = a.a_kind == B2_OPERAND_GATHER ? 1.5 : 1.0;
-            const double rb = !filter_tiles(a) ? 1.0 : a.g.channel_last ? 3.5 : 1.5;
+            // Rows along K that do not start on 16-byte boundaries are loaded value by value: twice (flex16)
+            // and 1.5 times (fp32) the producers' instructions, and 6000 cycles a k-block at the least.
+            const int vec = MODE == MODE_FLEX16 ? 8 : 4;
+            const bool a_single = a.a_kind == B2_OPERAND_K && a.a_rs % vec != 0;
+            const bool b_single = a.b_kind == B2_OPERAND_K && a.b_rs % vec != 0;
+            const double single = MODE == MODE_FLEX16 ? 2.0 : 1.5;
+            const double ra = a.a_kind == B2_OPERAND_GATHER ? 1.5 : a_single ? single : 1.0;
+            const double rb = filter_tiles(a) ? (a.g.channel_last ? 3.5 : 1.5) : b_single ? single : 1.0;
             const long long pace = (long long)((128 * ra + bn * rb) * (MODE == MODE_FLEX16 ? (bn == 128 ? 33 : 22) : 7));
-            const long long lat = MODE == MODE_FLEX16 ? 4000 : a.a_kind != B2_OPERAND_GATHER ? 1000 + 6 * bn
-                                  : bn >= 64 ? 3500 : 1600 + 25 * bn;
+            const long long lat = MODE == MODE_FLEX16 ? (a_single || b_single ? 6000 : 4000)
+                                  : a.a_kind != B2_OPERAND_GATHER ? 1000 + 6 * bn : bn >= 64 ? 3500 : 1600 + 25 * bn;
             const long long ctas = tiles * splits, per_sm = bn == 128 || 1152 + dir_ring_bytes(bn) + tab > 115000 ? 1 : 2;
-            const long long slots = (long long)kClusterCtas[splits] * per_sm;
             const long long together = ctas <= 148 ? 1 : per_sm;
-            const long long kb = together * pace > lat ? together * pace : lat;
+            // Two groups of producers where each SM has one CTA anyway and a k-block for both: a k-block then
+            // takes 65 % (flex16) or 60 % of the cycles (fp32 512 x 128 x 512: 1470 -> 820).  With more CTAs than
+            // SMs two of them on an SM do the same (flex16 1500 x 200 x 900 in 144 CTAs of two groups, clusters
+            // of three, where 135 find an SM: 26.4 us, 22.5 with one group).  Tiles of 128 columns would spill.
+            const int groups = ctas <= kClusterCtas[splits] && per > 1 && bn < 128 &&
+                               1152 + dir_ring_bytes(bn, 2) + tab <= 232448 ? 2 : 1;
+            long long kb = together * pace > lat ? together * pace : lat;
+            if (groups == 2) kb = kb * (MODE == MODE_FLEX16 ? 65 : 60) / 100;
+            const long long slots = (long long)kClusterCtas[splits] * (groups == 2 ? 1 : per_sm);
+            // (the exchange of slices: 700 and 500 a slice)
             const long long one = 7000 + per * kb + together * bn * (splits > 1 ? 24 : 12) +
-                                  (splits == 1 ? 0 : filter_tiles(a) ? 18000 : 3000);
+                                  (splits == 1 ? 0 : filter_tiles(a) ? 18000 : 700 + 500 * splits);
             const long long waves = (ctas + slots - 1) / slots, cost = waves * one;
-            if (best.cost < 0 || cost < best.cost) best = {bn, splits, per, (int)waves, cost};
+            if (best.cost < 0 || cost < best.cost) best = {bn, splits, per, (int)waves, groups, cost};
         }
     }
     return best;
 }
 
-template <int MODE, int BN, int AK>
+template <int MODE, int BN, int AK, int G>
 int direct_launch_as(const DirectParams& p, cudaStream_t st) {
     const int KB = MODE == MODE_FLEX16 ? 128 : 32;
-    const int ring = dir_ring_bytes(BN);
-    static_assert(dir_ring_bytes(BN) >= BN * 128 * 8, "the slices' sums are exchanged through the ring");
+    const int ring = dir_ring_bytes(BN, G);
+    static_assert(dir_ring_bytes(BN, G) >= BN * 128 * 8, "the slices' sums are exchanged through the ring");
     const int smem = 1024 + ring + 128 +
                      (AK == B2_OPERAND_GATHER ? p.kb_per_split * KB * (filter_tiles(p.a) ? 16 : 8) : 0);
     static bool attr_set = false;
     if (!attr_set) {
-        B2_CUDA(cudaFuncSetAttribute(direct_kernel<MODE, BN, AK>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        B2_CUDA(cudaFuncSetAttribute(direct_kernel<MODE, BN, AK, G>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      AK == B2_OPERAND_GATHER ? 232448 : 1024 + ring + 128));
         attr_set = true;
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((p.a.N + BN - 1) / BN, (p.a.M + 127) / 128, p.splits);
-    cfg.blockDim = dim3(kDirThreads);
+    cfg.blockDim = dim3(dir_threads(G));
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cudaLaunchAttribute attr[2];
@@ -715,16 +757,16 @@ int direct_launch_as(const DirectParams& p, cudaStream_t st) {
     attr[1].val.clusterDim.x = 1; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = p.splits;
     cfg.attrs = attr;
     cfg.numAttrs = p.splits > 1 ? 2 : 1;
-    B2_CUDA(cudaLaunchKernelEx(&cfg, direct_kernel<MODE, BN, AK>, p));
+    B2_CUDA(cudaLaunchKernelEx(&cfg, direct_kernel<MODE, BN, AK, G>, p));
     return B2_OK;
 }
 
-template <int MODE, int BN>
+template <int MODE, int BN, int G>
 int direct_launch_bn(const DirectParams& p, cudaStream_t st) {
     switch (p.a.a_kind) {
-        case B2_OPERAND_K: return direct_launch_as<MODE, BN, B2_OPERAND_K>(p, st);
-        case B2_OPERAND_ROWS: return direct_launch_as<MODE, BN, B2_OPERAND_ROWS>(p, st);
-        default: return direct_launch_as<MODE, BN, B2_OPERAND_GATHER>(p, st);
+        case B2_OPERAND_K: return direct_launch_as<MODE, BN, B2_OPERAND_K, G>(p, st);
+        case B2_OPERAND_ROWS: return direct_launch_as<MODE, BN, B2_OPERAND_ROWS, G>(p, st);
+        default: return direct_launch_as<MODE, BN, B2_OPERAND_GATHER, G>(p, st);
     }
 }
 
@@ -745,11 +787,18 @@ int direct_launch_mode(const b2_direct_args& a, cudaStream_t st) {
     };
     p.a_vec = aligned(a.a_kind, a.A, a.a_rs, a.a_ks);
     p.b_vec = a.b_kind != B2_OPERAND_FILTER && aligned(a.b_kind, a.B, a.b_rs, a.b_ks);
+    if (s.groups == 2) {
+        switch (s.bn) {
+            case 16: return direct_launch_bn<MODE, 16, 2>(p, st);
+            case 32: return direct_launch_bn<MODE, 32, 2>(p, st);
+            default: return direct_launch_bn<MODE, 64, 2>(p, st);
+        }
+    }
     switch (s.bn) {
-        case 16: return direct_launch_bn<MODE, 16>(p, st);
-        case 32: return direct_launch_bn<MODE, 32>(p, st);
-        case 64: return direct_launch_bn<MODE, 64>(p, st);
-        default: return direct_launch_bn<MODE, 128>(p, st);
+        case 16: return direct_launch_bn<MODE, 16, 1>(p, st);
+        case 32: return direct_launch_bn<MODE, 32, 1>(p, st);
+        case 64: return direct_launch_bn<MODE, 64, 1>(p, st);
+        default: return direct_launch_bn<MODE, 128, 1>(p, st);
     }
 }
 
