@@ -220,6 +220,7 @@ int b2_flex_publish(int32_t* stats, int32_t n, const int32_t* status, int32_t* h
  * src[k], both 16-byte aligned.
  * b2_call_stage: the address at which the device can read `bytes` bytes of host memory at src:
  * src itself where it is page-locked, else `pinned`, to which they are copied; NULL where that is NULL.
+ * b2_call_wait returns when all that was launched on the device's stream has ended.
  * Replace FlexGPUDeviceTensor.__setitem__ / get and the per-kernel statistics read of the reference
  * (ngraph/transformers/flexgputransform.py:178-208, 347-371).
  * ------------------------------------------------------------------------------------------ */
@@ -236,6 +237,7 @@ int b2_call_inputs(const b2_call_input* inputs, int32_t n, const b2_call_block* 
                    b2_flex_scale* table, int32_t* stats, void* stream);
 int b2_call_outputs(const b2_call_output* outputs, int32_t n, int32_t* stats, int32_t n_stats,
                     const int32_t* status, int32_t* host_stats, int32_t* host_status, void* stream);
+int b2_call_wait(int32_t device, void* stream);
 int b2_call_stage(const void* src, size_t bytes, void* pinned, const void** visible);
 /* Exponent bookkeeping of a whole call over the state arrays of all entries (one row per entry; the
  * rule is ngraph_python_b200/flex.py's, FlexEntry.begin_write / end_write).

@@ -235,6 +235,16 @@ extern "C" int b2_call_outputs(const b2_call_output* outputs, int32_t n, int32_t
     return B2_OK;
 }
 
+extern "C" int b2_call_wait(int32_t device, void* stream) {
+    int current = device;
+    B2_CUDA(cudaGetDevice(&current));
+    if (current != device) B2_CUDA(cudaSetDevice(device));         // (stream 0 is the current device's)
+    const cudaError_t e = cudaStreamSynchronize((cudaStream_t)stream);
+    if (current != device) cudaSetDevice(current);
+    B2_CUDA(e);
+    return B2_OK;
+}
+
 extern "C" int b2_call_stage(const void* src, size_t bytes, void* pinned, const void** visible) {
     B2_REQUIRE(src && visible, "null argument");
     cudaPointerAttributes at;

@@ -698,8 +698,9 @@ DirectShape direct_shape(const b2_direct_args& a) {
             // Measured on one B200 (cycles at 1.9 GHz): the producers set the pace, 7 (fp32) or 22
             // (flex16) cycles an operand row of a k-block when they keep an SM busy, and a k-block
             // takes 1000 + 6 bn (gathered 2000 to 3500) or 4000 cycles from load to commit when they do
-            // not; the two CTAs of an SM overlap.  Gathered rows cost their address and bounds, filters as a tile's pixels see
-            // them the same, more where the lanes' rows lie apart; slices of their wide tiles 15000 more.
+            // not; the two CTAs of an SM overlap.  Gathered rows cost their address and bounds, filters as
+            // a tile's pixels see them the same, more where the lanes' rows lie apart; slices of their wide
+            // tiles 15000 more.
             // Rows along K that do not start on 16-byte boundaries are loaded value by value: twice (flex16)
             // and 1.5 times (fp32) the producers' instructions, and 6000 cycles a k-block at the least.
             const int vec = MODE == MODE_FLEX16 ? 8 : 4;

@@ -140,10 +140,14 @@ class _PlaneUser(object):
         lib.check(lib.raw().b2_conv_filter_planes_many(jobs, len(users), C.byref(n), t.stream.cuda_stream))
         t.kernel_launches += n.value
 
+    def kept_planes(self):
+        """Whether `refresh` can have anything to do."""
+        return self.use_planes and not self.planes_built_first
+
     def refresh(self, t):
         """Rebuilds the cached filter planes when the filters have changed since they were built
         (called before every launch, and before every replay of a captured step list)."""
-        if not self.use_planes or self.planes_built_first:
+        if not self.kept_planes():
             return
         fbuf = self.in_views[self.filter_arg].buffer
         if fbuf.last_write_step < 0 and self.filter_version != fbuf.version:
@@ -248,6 +252,9 @@ class ConvChainStep(_Step):
         self.planes = None
         self.filters = [s.in_views[s.filter_arg].buffer for s in members]
         self.versions = None
+
+    def kept_planes(self):
+        return True
 
     def refresh(self, t):
         """Filter planes as the chain reads them, made again when filters have changed."""

@@ -294,7 +294,7 @@ class Computation(object):
             raise lib.B200Error("run the computation once before capturing it")
         torch = t.torch
         steps = kernels.chain_convolutions(self.steps, set(v.buffer for v in self.return_views), t)
-        refreshable = [s for s in steps if hasattr(s, "refresh")]
+        refreshable = [s for s in steps if hasattr(s, "refresh") and s.kept_planes()]
         self.chains = [s for s in steps if s.kind == "conv_chain"]
         for s in self.chains:
             s.refresh(t)
@@ -428,8 +428,11 @@ class _CallIO(object):
         self.comp, self.views = comp, views
         self.lengths = [tuple(v.axes.lengths) for v in views]
         self.flex_views = [v for v in views if v.buffer.flex]
+        self.flex_buffers = [v.buffer for v in self.flex_views]
         self.block_mem = torch.zeros((ctypes.sizeof(lib.CallBlock),), dtype=torch.uint8).pin_memory()
         self.block = lib.CallBlock.from_address(self.block_mem.data_ptr())
+        self.args = [(k, v.buffer, self.block.arg[k], v.buffer.where is not None)
+                     for k, v in enumerate(views)]
         self.table_rows = t._table_host.shape[0] if t.flex else 0
         if t.flex:
             self.block.table = t._table_host.data_ptr()
@@ -444,7 +447,7 @@ class _CallIO(object):
         self.written = sorted((b.ptr(), b.ptr() + b.tensor.nbytes) for b in written)
         # results: small dense ones ride in the last node, the others are copied after it
         self.outputs, self.later, budget = [], [], self.RESULTS_MOST
-        self.results = []               # (pinned array, view) or None, in the order of the returns
+        self.results = []               # (pinned array, buffer) or None, in the order of the returns
         for v in comp.return_views:
             buf = v.buffer
             n = max(buf.size, 1) * (2 if buf.flex else 4)
@@ -454,7 +457,8 @@ class _CallIO(object):
                 budget -= n
                 host = torch.empty((max(buf.size, 1),), dtype=buf.tensor.dtype).pin_memory()
                 self.outputs.append((buf.ptr(), host.data_ptr(), n))
-                self.results.append((host, v))
+                # (as a caller sees it: copied, or scaled, when the call has ended)
+                self.results.append((host.numpy().reshape(v.axes.lengths), buf))
             else:
                 self.results.append(None)
 
@@ -493,6 +497,9 @@ class _CallIO(object):
         buf = view.buffer
         torch = t.torch
         if isinstance(value, torch.Tensor) and value.is_cuda:
+            if value.dtype is torch.float32 and value.device == t.device and \
+                    value.shape == self.lengths[k] and value.is_contiguous():
+                return value.data_ptr(), value
             src = t._device_argument(view, value)
             if src.device == t.device:
                 return src.data_ptr(), src
@@ -520,31 +527,33 @@ class _CallIO(object):
         t, comp, block = self.t, self.comp, self.block
         keep = []
         try:
-            for k, value in enumerate(args):
-                self.views[k].buffer.version += 1
+            for (k, buf, arg, read_in_place), value in zip(self.args, args):
+                buf.version += 1
                 address, obj = self._source(k, value)
-                block.arg[k].src = address
+                arg.src = address
                 # a device tensor is read where it lies by the kernel that uses it first, which
                 # also stores it
-                block.arg[k].in_place = (
-                    self.views[k].buffer.where is not None and isinstance(obj, t.torch.Tensor) and
+                arg.in_place = (
+                    read_in_place and isinstance(obj, t.torch.Tensor) and
                     address % 16 == 0 and self._stays_as_it_is(address, obj.nbytes))
                 keep.append(obj)
             t._begin_call(comp, self)
-            for k, v in enumerate(self.views):
-                if v.buffer.flex:
-                    block.arg[k].inv_scale = math.ldexp(1.0, v.buffer.entry.dec)
-                    t._inputs_written.append(v.buffer)
+            for k, buf, arg, _ in self.args:
+                if buf.flex:
+                    arg.inv_scale = math.ldexp(1.0, buf.entry.dec)
+            if self.flex_buffers:
+                t._inputs_written = list(self.flex_buffers)
             comp.executor()
             pending = [None if r is not None else t._device_to_host_async(v)
                        for r, v in zip(self.results, comp.return_views)]
             t._end_call(comp)
         finally:
-            for k in range(len(args)):
-                block.arg[k].src = None
+            for _, _, arg, _ in self.args:
+                arg.src = None
             block.table_rows = 0
-        return comp._results([t._finish_host(p or r)
-                              for p, r in zip(pending, self.results)])
+        return comp._results([
+            t._finish_host(p) if r is None else t._as_result(*r)
+            for p, r in zip(pending, self.results)])
 
 
 # ---------------------------------------------------------------------------------------------
@@ -2098,13 +2107,13 @@ class B200Transformer(object):
         (DeviceTensor.get, gputransform.py:710-744; flex: int16 * scale,
         flexgputransform.py:178-181)."""
         pinned, view = pending
-        host = pinned.numpy().reshape(view.axes.lengths)
-        if view.buffer.flex:
-            return host.astype(np.float64) * view.buffer.entry.scale
-        host = host.copy()
-        if host.shape == ():
-            return host[()]
-        return host
+        return self._as_result(pinned.numpy().reshape(view.axes.lengths), view.buffer)
+
+    @staticmethod
+    def _as_result(host, buf):
+        if buf.flex:
+            return np.multiply(host, buf.entry.scale, dtype=np.float64)
+        return host.copy() if host.shape else host[()]
 
     def _device_to_host(self, view):
         """DeviceTensor.get (gputransform.py:710-744); flex: int16 * scale
@@ -2295,7 +2304,8 @@ class B200Transformer(object):
         exchanging = self._allreduce is not None and self.comm.size > 1
         if exchanging:
             self._allreduce.finish()        # CommError instead of an endless synchronisation
-        torch.cuda.current_stream(self.device).synchronize()
+        device = self.device.index
+        lib.check(lib.raw().b2_call_wait(device, torch._C._cuda_getCurrentRawStream(device)))
         if exchanging:
             self._allreduce.after_sync()
         watched = getattr(comp, "_watched", None)
@@ -2317,34 +2327,31 @@ class B200Transformer(object):
         stats = self._stats_host.numpy()
         steady = getattr(comp, "_steady", None)
         if steady is not None and steady[0] == self._flex_epoch and \
-                len(self._inputs_written) == steady[3] and np.array_equal(stats[steady[1]], steady[2]):
+                len(self._inputs_written) == steady[3] and stats[steady[1]].tobytes() == steady[2]:
             # the same maxima as after the previous call, with every history window already full
             # of them: every entry would make the choice it made before
             return
         self._flex_epoch += 1
         fm = self.flex_manager
-        for b in self._inputs_written:
-            b.entry.end_write(int(stats[b.slot]))
-        arrays = getattr(comp, "_flex_written_arrays", None)
-        if arrays is None:
-            ids = np.array([b.entry.i for b in comp.written], dtype=np.int64)
-            arrays = (ids, np.array([b.slot_write for b in comp.written], dtype=np.int64),
-                      len(set(ids.tolist())) == len(ids))
-            comp._flex_written_arrays = arrays
-        ids, slots, distinct = arrays
+        inputs = self._inputs_written
+        cached = getattr(comp, "_flex_written_arrays", None)
+        if cached is None or cached[0] != inputs:
+            # (the arguments written this call, then what the computation writes)
+            both = [(b.entry.i, b.slot) for b in inputs] + [(b.entry.i, b.slot_write) for b in comp.written]
+            ids = np.array([i for i, _ in both], dtype=np.int64)
+            cached = comp._flex_written_arrays = (
+                list(inputs), ids, np.array([k for _, k in both], dtype=np.int64),
+                len(set(ids.tolist())) == len(ids))
+        _, ids, slots, distinct = cached
         if distinct:
-            settled = fm.end_call(ids, slots, stats)   # all written tensors in one native pass
+            settled = fm.end_call(ids, slots, stats)   # all tensors in one native pass
         else:
-            for b in comp.written:                     # an entry written twice: one at a time
+            for b in inputs:                           # an entry written twice: one at a time
+                b.entry.end_write(int(stats[b.slot]))
+            for b in comp.written:
                 b.entry.end_write(int(stats[b.slot_write]))
             settled = fm.settled(ids)
-        in_ids = np.array([b.entry.i for b in self._inputs_written], dtype=np.int64)
-        if settled and fm.settled(in_ids):
-            idx = np.concatenate([np.array([b.slot for b in self._inputs_written], dtype=np.int64),
-                                  slots])
-            comp._steady = (self._flex_epoch, idx, stats[idx].copy(), len(self._inputs_written))
-        else:
-            comp._steady = None
+        comp._steady = (self._flex_epoch, slots, stats[slots].tobytes(), len(inputs)) if settled else None
 
     # ---- launching -------------------------------------------------------------------------------
     def _ew_pointers(self, step, recorded=False):
