@@ -75,6 +75,7 @@ class _PlaneUser(object):
     use_planes = False
     plane_args = ()                 # indexes of the tensors read as planes in op.args / in_views
     splits = ()                     # those that this step splits unless their producer has
+    filters_change = False          # the computation writes the filters, or takes them as an argument
     planes_built_first = False      # the first of the convolutions builds the filter planes of all
     joint_planes = None             # ... this one: the steps whose planes it builds
     filter_planes = None
@@ -142,7 +143,7 @@ class _PlaneUser(object):
 
     def kept_planes(self):
         """Whether `refresh` can have anything to do."""
-        return self.use_planes and not self.planes_built_first
+        return self.use_planes and not self.planes_built_first and not self.filters_change
 
     def refresh(self, t):
         """Rebuilds the cached filter planes when the filters have changed since they were built
@@ -150,7 +151,7 @@ class _PlaneUser(object):
         if not self.kept_planes():
             return
         fbuf = self.in_views[self.filter_arg].buffer
-        if fbuf.last_write_step < 0 and self.filter_version != fbuf.version:
+        if self.filter_version != fbuf.version:
             self._build_filter_planes(t)
 
     def _add_tail_views(self, t, epilogue):
@@ -172,8 +173,8 @@ class _PlaneUser(object):
             self._build_joint_planes(t)
         elif self.planes_built_first:
             pass
-        elif fbuf.last_write_step >= 0:
-            self._build_filter_planes(t)     # filters written inside this computation
+        elif self.filters_change:
+            self._build_filter_planes(t)
         else:
             self.refresh(t)
         slots = (t._slot_for_read(xbuf, self), t._slot_for_read(fbuf, self), ov.buffer.slot_write)
@@ -213,13 +214,15 @@ class _PlaneUser(object):
         self._flex_probe_then(t, obuf, [xbuf, fbuf], call)
 
 
-def join_filter_planes(steps):
-    """The filter planes of the convolutions whose filters this computation writes after reading
+def join_filter_planes(steps, arguments):
+    """Which convolutions of a computation make their filter planes in every call: those whose filters it
+    writes or receives (`arguments`).  The filter planes of the convolutions whose filters this computation writes after reading
     them (a training step): the first of them builds all, one launch per 32 layers."""
     written, mine = set(), []
     for s in steps:
         if getattr(s, "filter_arg", None) is not None:
             buf = s.in_views[s.filter_arg].buffer
+            s.filters_change = buf.last_write_step >= 0 or buf in arguments
             if buf.last_write_step >= 0 and buf not in written:
                 mine.append(s)
         written.update(s.output_buffers())
@@ -314,7 +317,7 @@ def chain_convolutions(steps, returned, t):
     def suits(s):
         return (isinstance(s, ConvStep) and s.use_planes and s.epi is not None and
                 not s.planes_built_first and not s.joint_planes and s.splits in ((), (0,)) and
-                s.in_views[1].buffer.last_write_step < 0 and s.epi.get("mask") is None and
+                not s.filters_change and s.epi.get("mask") is None and
                 not s.out_views[0].buffer.persistent)
 
     def chain_of(run):

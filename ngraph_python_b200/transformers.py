@@ -198,7 +198,7 @@ class Computation(object):
         planner.parameter_buffers = set(t._view_of(p).buffer for p in self.parameters)
         for s in self.steps:
             final.extend(planner.finalize_step(s))     # (a step may bring copies that precede it)
-        kernels.join_filter_planes(final)
+        kernels.join_filter_planes(final, planner.parameter_buffers)
         if t.comm.size == 1:      # (elsewhere every update starts when its gradient is there)
             _join_launches(final)
         self.steps = final
