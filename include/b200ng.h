@@ -355,12 +355,21 @@ int b2_conv_filter_planes(const int16_t* F, const b2_conv_dims* d, int32_t pass,
                           void* stream);
 /* ... of several convolutions at once, in as few launches as their arguments take. */
 typedef struct b2_conv_filter_job {
-    const int16_t* filters;
+    const void* filters;
     void* planes;
     b2_conv_dims dims;
     int32_t pass;
 } b2_conv_filter_job;
 int b2_conv_filter_planes_many(const b2_conv_filter_job* jobs, int32_t n, int32_t* launches, void* stream);
+/* fp32 convolutions (pass 0 forward, 1 input gradient) with the filters laid out beforehand, as the stages of
+ * the kernel that gathers its operands hold them: bytes of that (0: this one takes none), the launches that
+ * make it for several convolutions (job.filters: fp32; planes on 128-byte boundaries), and the pass with the
+ * tails of b2_conv_fprop_f32_fused and b2_conv_bprop_f32_fused. */
+int b2_conv_filter_tiles_info(const b2_conv_dims* d, int32_t pass, size_t* bytes);
+int b2_conv_filter_tiles(const b2_conv_filter_job* jobs, int32_t n, int32_t* launches, void* stream);
+int b2_conv_f32_tiles(int32_t pass, const float* X, const void* filter_tiles, float* O, const b2_conv_dims* d,
+                      const float* bias, const float* residual, int32_t relu, const float* mask, int32_t* status,
+                      void* stream);
 int b2_conv_flex16_planes(int32_t pass, const void* act_planes, const void* filter_planes,
                           int16_t* out, const b2_conv_dims* d, const b2_flex_scale* table,
                           int32_t slotX, int32_t slotF, int32_t slotOut, int32_t* stats,

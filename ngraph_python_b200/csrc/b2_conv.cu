@@ -170,6 +170,29 @@ inline bool conv_goes_direct(int mode, const ConvGeom& g, int pass, b2_direct_ar
     return best < 13000 + planes + (tiles + 147) / 148 * (3500 + (long long)(s.Kp * s.esize / kKBytes) * kb);
 }
 
+// The same with the filters' rows made beforehand (b2_direct_stage_filters), for fp32 convolutions that go
+// direct: false where a launch would take no less time (what the kernel's cost rule says for both; a row of
+// filters costs its producers as much as a gathered one, or more).  With only the gathered rows to make, tiles
+// of six pixels pay: 16 channels at 32x32, batch 100, 12.8 us against 16.7 for four, as they lie 20.2.
+inline bool conv_goes_staged(const ConvGeom& g, int pass, b2_direct_args* out) {
+    b2_direct_args d;
+    if (!conv_goes_direct(MODE_F32X3, g, pass, &d)) return false;
+    long long best = b2_direct_cost(d);
+    bool found = false;
+    for (int a = 1; a <= 4; ++a)
+        for (int b = 1; b <= 4; ++b) {
+            if (!direct_args(MODE_F32X3, g, pass, pass ? a * g.str_h : a, pass ? b * g.str_w : b, &d)) continue;
+            d.staged = &d;                        // (there will be such)
+            const long long cost = b2_direct_cost(d);
+            if (cost < 0 || cost >= best) continue;
+            best = cost;
+            found = true;
+            *out = d;
+            out->staged = out;
+        }
+    return found;
+}
+
 inline int launch_direct(b2_direct_args& d, const void* A, const void* B, void* C,
                          const b2_flex_scale* table, int slotA, int slotB, int slotC, int* stats,
                          unsigned long long* probe_out, int* status, int probe, cudaStream_t st) {
@@ -2215,6 +2238,55 @@ extern "C" int b2_conv_fprop_f32_fused(const float* I, const float* F, float* O,
     B2_REQUIRE(conv_goes_direct(MODE_F32X3, g, 0, &direct), "this convolution takes no fused tail");
     direct.bias = bias; direct.residual = residual; direct.relu = relu ? 1 : 0;
     return launch_direct(direct, I, F, O, nullptr, 0, 0, 0, nullptr, nullptr, status, 0, (cudaStream_t)stream);
+}
+
+extern "C" int b2_conv_filter_tiles_info(const b2_conv_dims* d, int32_t pass, size_t* bytes) {
+    ConvGeom g;
+    int rc = geom_from(d, &g);
+    if (rc) return rc;
+    B2_REQUIRE(bytes && (pass == 0 || pass == 1), "bad argument");
+    b2_direct_args direct;
+    *bytes = conv_goes_staged(g, pass, &direct) ? b2_direct_staged_bytes(direct) : 0;
+    return B2_OK;
+}
+
+extern "C" int b2_conv_filter_tiles(const b2_conv_filter_job* jobs, int32_t n, int32_t* launches, void* stream) {
+    B2_REQUIRE(jobs && n >= 0 && launches, "bad argument");
+    *launches = 0;
+    for (int32_t at = 0; at < n; at += kStageJobs) {
+        b2_stage_job list[kStageJobs];
+        const int m = n - at < kStageJobs ? n - at : kStageJobs;
+        for (int j = 0; j < m; ++j) {
+            const b2_conv_filter_job& job = jobs[at + j];
+            ConvGeom g;
+            int rc = geom_from(&job.dims, &g);
+            if (rc) return rc;
+            B2_REQUIRE(job.filters && job.planes && ((uintptr_t)job.planes & 127) == 0 && (job.pass == 0 || job.pass == 1),
+                       "bad argument");
+            B2_REQUIRE(conv_goes_staged(g, job.pass, &list[j].a), "this convolution takes no filter tiles");
+            list[j].a.staged = list[j].staged = job.planes;
+            list[j].filters = (const float*)job.filters;
+        }
+        int count = 0;
+        const int rc = b2_direct_stage_filters(list, m, &count, (cudaStream_t)stream);
+        if (rc) return rc;
+        *launches += count;
+    }
+    return B2_OK;
+}
+
+extern "C" int b2_conv_f32_tiles(int32_t pass, const float* X, const void* filter_tiles, float* O, const b2_conv_dims* d,
+                                 const float* bias, const float* residual, int32_t relu, const float* mask,
+                                 int32_t* status, void* stream) {
+    ConvGeom g;
+    int rc = geom_from(d, &g);
+    if (rc) return rc;
+    B2_REQUIRE(X && filter_tiles && O && status && (pass == 0 || pass == 1), "bad argument");
+    b2_direct_args direct;
+    B2_REQUIRE(conv_goes_staged(g, pass, &direct), "this convolution takes no filter tiles");
+    direct.staged = filter_tiles;
+    direct.bias = bias; direct.residual = residual; direct.relu = relu ? 1 : 0; direct.mask = mask;
+    return launch_direct(direct, X, nullptr, O, nullptr, 0, 0, 0, nullptr, nullptr, status, 0, (cudaStream_t)stream);
 }
 
 extern "C" int b2_conv_fprop_f32(const float* I, const float* F, float* O, const b2_conv_dims* d,

@@ -22,3 +22,90 @@ int b2_direct_launch(const b2_direct_args& a, cudaStream_t st) {
     B2_REQUIRE(b2_direct_cost(a) >= 0, "problem outside the kernel's range");
     return a.flex ? b2_direct_launch_flex(a, st) : direct_launch_mode<MODE_F32X3>(a, st);
 }
+
+// ---- filters as the stages hold them ------------------------------------------------------------
+// The rows of the filters that the pixels of a tile see are the same in every tile, and making them costs
+// a producer more than the rows it gathers (a lane's rows lie apart, each with its own tap): here each is
+// made once, in the order n tile, k-block, plane, row, 128-byte swizzled, and the kernel copies a
+// k-block's 2 * bn * 128 bytes as they are.  Bound by launch latency (a network's filters are some MB).
+namespace {
+
+struct StageLayout {
+    const float* F;
+    unsigned char* out;
+    long long b_rs, b_ks;
+    b2_gather g;
+    int N, K, bn, num_kb, ntn, tiled;
+};
+struct StageJobs {
+    int n, first[kStageJobs + 1];                 // job j owns blocks first[j] .. first[j+1]-1
+    StageLayout layout[kStageJobs];
+};
+static_assert(sizeof(StageJobs) <= 4096, "kernel argument");
+
+__global__ void __launch_bounds__(256)
+stage_filters_kernel(const __grid_constant__ StageJobs jobs) {
+    after_earlier_kernels();
+    int j = 0;
+    while (j + 1 < jobs.n && (int)blockIdx.x >= jobs.first[j + 1]) ++j;
+    const StageLayout& f = jobs.layout[j];
+    const b2_gather& g = f.g;
+    const int RS = g.R * g.S, total = f.ntn * f.num_kb * 8 * f.bn;
+    const int stride = (jobs.first[j + 1] - jobs.first[j]) * (int)blockDim.x;
+    for (int i = ((int)blockIdx.x - jobs.first[j]) * (int)blockDim.x + threadIdx.x; i < total; i += stride) {
+        const int lr = i % f.bn, chunk = i / f.bn % 8, block = i / f.bn / 8, kb = block % f.num_kb;
+        const int row = block / f.num_kb * f.bn + lr;
+        const int pix = f.tiled ? row / g.kt : 0, gy = f.tiled ? pix / g.gw : 0, gx = f.tiled ? pix - gy * g.gw : 0;
+        float4 h, l;
+        float *hp = (float*)&h, *lp = (float*)&l;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int k = kb * 32 + chunk * 4 + q;
+            float v = 0.0f;
+            if (row < f.N && k < f.K) {
+                if (f.tiled) {
+                    const int c = g.channel_last ? k % g.channels : k / RS, rs = g.channel_last ? k / g.channels : k % RS;
+                    const int th = rs / g.S, tw = rs - th * g.S;
+                    const int r = g.f0_h + g.f1_h * th + g.f2_h * gy, s = g.f0_w + g.f1_w * tw + g.f2_w * gx;
+                    if (r >= 0 && r < g.fr && s >= 0 && s < g.fs)
+                        v = __ldg(f.F + c * f.b_ks + (row - pix * g.kt) * f.b_rs +
+                                  (long long)(r * g.fs + s) * (g.channel_last ? g.channels : g.kt));
+                } else {
+                    v = __ldg(f.F + row * f.b_rs + k * f.b_ks);
+                }
+            }
+            dir_split_tf32(v, hp[q], lp[q]);
+        }
+        unsigned char* out = f.out + (long long)block * (2 * f.bn * 128) + swz(lr, chunk);
+        *(float4*)out = h;
+        *(float4*)(out + f.bn * 128) = l;
+    }
+}
+
+}  // namespace
+
+size_t b2_direct_staged_bytes(const b2_direct_args& a) {
+    const DirectShape s = direct_shape<MODE_F32X3>(a);
+    return (size_t)((a.N + s.bn - 1) / s.bn) * ((a.K + 31) / 32) * (2 * s.bn * 128);
+}
+
+int b2_direct_stage_filters(const b2_stage_job* list, int n, int* launches, cudaStream_t st) {
+    *launches = 0;
+    for (int at = 0; at < n; at += kStageJobs) {
+        StageJobs jobs = {};
+        jobs.n = n - at < kStageJobs ? n - at : kStageJobs;
+        for (int j = 0; j < jobs.n; ++j) {
+            const b2_direct_args& a = list[at + j].a;
+            const DirectShape s = direct_shape<MODE_F32X3>(a);
+            const int ntn = (a.N + s.bn - 1) / s.bn, num_kb = (a.K + 31) / 32;
+            jobs.layout[j] = {list[at + j].filters, (unsigned char*)list[at + j].staged, a.b_rs, a.b_ks, a.g,
+                              a.N, a.K, s.bn, num_kb, ntn, filter_tiles(a)};
+            const long long blocks = ((long long)ntn * num_kb * 8 * s.bn + 255) / 256;
+            jobs.first[j + 1] = jobs.first[j] + (int)(blocks < 148 * 4 ? blocks : 148 * 4);
+        }
+        B2_CUDA(b2::launch_after(stage_filters_kernel, dim3(jobs.first[jobs.n]), 256, 0, st, jobs));
+        B2_CUDA(cudaGetLastError());
+        ++*launches;
+    }
+    return B2_OK;
+}

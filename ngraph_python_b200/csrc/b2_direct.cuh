@@ -7,7 +7,8 @@
 //              lies (K contiguous, rows contiguous, or rows gathered from a C,H,W,N tensor through a
 //              table of column offsets), split it into its two planes and store them K-major, 128-byte
 //              swizzled, into a ring of stages, the groups by turns; the first group afterwards the epilogue;
-//   the last warp: tensor memory, tcgen05.mma issue.
+//   one warp:  tensor memory, tcgen05.mma issue;
+//   one more where B lies ready as the stages hold it: its copies.
 // A k-block is 128 bytes of plane: 32 fp32 or 128 int16 values.
 //   fp32:   3xTF32, in chains of at most 16 k-blocks (the tensor core's fp32 sum truncates); longer K
 //           is cut into slices.  Matrix products add hi*hi, hi*lo and lo*hi into one sum (see ONE_CHAIN).
@@ -23,6 +24,10 @@
 // convolutions the producers' issue slots.  The second group halves what a k-block waits for where an SM has
 // one CTA (one B200, one group -> two, us: fp32 512 x 128 x 784 16.7 -> 11.5, 600 x 600 x 600 24.5 -> 14.6,
 // flex16 512 x 128 x 784 11.0 -> 8.7, 905 x 380 x 611 24.1 -> 15.0; 20 % of it over 38 sizes).
+// Unrolled convolutions whose filters were laid out beforehand leave the producers only the gathered rows, and
+// tiles of more pixels pay (batch 100, forward / input gradient, us: 16 channels at 32x32 20.2 -> 12.8 / 25.1 ->
+// 12.8, 32 at 16x16 14.6 -> 12.0 / 23.3 -> 12.0, 64 at 8x8 14.3 -> 11.7 / 14.2 -> 11.7); the filters' way from L2 to
+// every SM, 256 bytes a row and k-block, then bounds the widest tiles.
 #ifndef B2_DIRECT_CUH
 #define B2_DIRECT_CUH
 #include "b2_direct.h"
@@ -37,7 +42,7 @@ constexpr int kDirMaxK = 4608;            // columns of the gather table
 __host__ __device__ constexpr int dir_stages(int bn, int groups = 1) {
     return groups > 1 ? (bn >= 64 ? 3 : 4) : bn == 128 ? 3 : 2;
 }
-__host__ __device__ constexpr int dir_threads(int groups) { return groups * 256 + 32; }
+__host__ __device__ constexpr int dir_threads(int groups, bool staged = false) { return groups * 256 + (staged ? 64 : 32); }
 __host__ __device__ constexpr int dir_stage_bytes(int bn) { return 2 * (128 + bn) * 128; }
 __host__ __device__ constexpr int dir_ring_bytes(int bn, int groups = 1) { return dir_stages(bn, groups) * dir_stage_bytes(bn); }
 __host__ __device__ constexpr int dir_tmem_cols(int mode, int bn) {
@@ -47,6 +52,10 @@ __host__ __device__ constexpr int dir_tmem_cols(int mode, int bn) {
 }
 
 __host__ __device__ inline bool filter_tiles(const b2_direct_args& a) { return a.b_kind == B2_OPERAND_FILTER; }
+
+__host__ __device__ inline int dir_table_bytes(const b2_direct_args& a, int columns) {
+    return a.a_kind != B2_OPERAND_GATHER ? 0 : columns * (filter_tiles(a) && !a.staged ? 16 : 8);
+}
 
 struct DirectParams {
     b2_direct_args a;
@@ -173,8 +182,8 @@ struct OperandTile {
     }
 };
 
-template <int MODE, int BN, int AK, int G>
-__global__ void __launch_bounds__(dir_threads(G), (BN == 128 || G > 1 ? 1 : 2))
+template <int MODE, int BN, int AK, int G, bool STAGED>
+__global__ void __launch_bounds__(dir_threads(G, STAGED), (BN == 128 || G > 1 ? 1 : 2))
 direct_kernel(const __grid_constant__ DirectParams p) {
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -196,6 +205,7 @@ direct_kernel(const __grid_constant__ DirectParams p) {
     int2* tab = (int2*)((unsigned char*)full_bar + 128);                          // [K of the slice] gather table
     int2* ftab = tab + p.kb_per_split * KB;                                       // likewise, of the filters
     const bool tiled = AK == B2_OPERAND_GATHER && filter_tiles(p.a);
+    const bool ftiled = tiled && !STAGED;                         // the producers make the rows of the filters
 
     // (warp: within its group of eight)
     const int wid = warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31, group = wid >> 3, warp = wid & 7;
@@ -205,7 +215,7 @@ direct_kernel(const __grid_constant__ DirectParams p) {
     const int nkb = min(p.kb_per_split, p.num_kb - kb0);
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < NST; ++s) { mbar_init(&full_bar[s], 8); mbar_init(&empty_bar[s], 1); }
+        for (int s = 0; s < NST; ++s) { mbar_init(&full_bar[s], STAGED ? 9 : 8); mbar_init(&empty_bar[s], 1); }
         mbar_init(tmem_full, 1);
         *fail_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -220,7 +230,7 @@ direct_kernel(const __grid_constant__ DirectParams p) {
         // offset of every column of this slice and the bit of its tap (none beyond K)
         const b2_gather& g = a.g;
         const int RS = g.R * g.S;
-        for (int i = threadIdx.x; i < nkb * KB; i += dir_threads(G)) {
+        for (int i = threadIdx.x; i < nkb * KB; i += dir_threads(G, STAGED)) {
             const int k = kb0 * KB + i;
             int2 e = make_int2(0, 0), f = make_int2(0, 0x7fff7fff);       // (no filter has that tap)
             if (k < a.K) {
@@ -230,7 +240,7 @@ direct_kernel(const __grid_constant__ DirectParams p) {
                 f = make_int2(c * (int)a.b_ks, ((g.f0_h + g.f1_h * r) & 0xffff) << 16 | ((g.f0_w + g.f1_w * s) & 0xffff));
             }
             tab[i] = e;
-            if (tiled) ftab[i] = f;
+            if (ftiled) ftab[i] = f;
         }
     }
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -283,11 +293,11 @@ direct_kernel(const __grid_constant__ DirectParams p) {
         }
         long long a_at[ATile::kKUnits], b_at[BTile::kKUnits];
         if (AK == B2_OPERAND_K) ATile::offsets_k(a_at, a.a_rs, m0, a.M, warp, lane);
-        BTile::offsets_k(b_at, a.b_rs, n0, a.N, warp, lane);
+        if (!STAGED) BTile::offsets_k(b_at, a.b_rs, n0, a.N, warp, lane);
         // filter rows of this lane: channel's place in the filters and the pixel's share of the tap
         constexpr int FR = BTile::kUnits * GR;
         int f_at[FR], f_h[FR], f_w[FR];
-        if (AK == B2_OPERAND_GATHER && tiled) {
+        if (AK == B2_OPERAND_GATHER && ftiled) {
             const b2_gather& g = a.g;
 #pragma unroll
             for (int i = 0; i < FR; ++i) {
@@ -338,7 +348,9 @@ direct_kernel(const __grid_constant__ DirectParams p) {
                     }
                 }
             }
-            if (AK == B2_OPERAND_GATHER && tiled) {
+            if (STAGED) {
+                // (the copying warp brings B)
+            } else if (AK == B2_OPERAND_GATHER && ftiled) {
                 const b2_gather& g = a.g;
                 const int mult = (int)(g.channel_last ? a.g.channels : g.kt);     // filters: tap stride
 #pragma unroll
@@ -408,7 +420,8 @@ direct_kernel(const __grid_constant__ DirectParams p) {
                         ATile::store_f4(st, st + 128 * 128, swz(a_lr, a_c0 + a_cs * i), A.r + PER * i);
                 }
             }
-            if (a.b_kind == B2_OPERAND_K) {
+            if (STAGED) {
+            } else if (a.b_kind == B2_OPERAND_K) {
                 B.store_k(b0, b0 + BN * 128, warp, lane);
             } else {
 #pragma unroll
@@ -439,6 +452,26 @@ direct_kernel(const __grid_constant__ DirectParams p) {
         for (int kb = group; kb < nkb; kb += 2 * G) {
             put(kb, ta[0], tb[0], ta[kNext], tb[kNext]);
             if (kb + G < nkb) put(kb + G, ta[kNext], tb[kNext], ta[0], tb[0]);
+        }
+    } else if (STAGED && wid > MMA_WARP) {
+        if (elect_one()) {
+            // ---- copies of B: one to a k-block, in the order of n tiles and k-blocks
+            constexpr unsigned bytes = 2 * BN * 128;
+            const char* src = (const char*)a.staged + ((long long)blockIdx.x * p.num_kb + kb0) * bytes;
+            int s = 0, n = 0;
+            unsigned parity = 1;
+            for (; n < nkb; ++n) {
+                if (!mbar_wait(&empty_bar[s], parity)) { atomicExch(fail_flag, 1); break; }
+                mbar_expect_tx(&full_bar[s], bytes);
+                asm volatile(
+                    "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                    ::"r"(smem_u32(smem + s * STAGE + 2 * 128 * 128)), "l"(src + (long long)n * bytes), "r"(bytes),
+                      "r"(smem_u32(&full_bar[s])) : "memory");
+                if (++s == NST) { s = 0; parity ^= 1u; }
+            }
+            // what is in flight lands before the block ends, whatever has become of the other roles
+            for (int i = n > NST ? n - NST : 0; i < n; ++i)
+                if (!mbar_wait(&full_bar[i % NST], (i / NST) & 1)) { atomicExch(fail_flag, 1); break; }
         }
     } else if (elect_one()) {
         // ---- MMA issue
@@ -693,7 +726,7 @@ DirectShape direct_shape(const b2_direct_args& a) {
             const bool chains = MODE == MODE_F32X3 && a.a_kind != B2_OPERAND_GATHER && want > 1;
             const int per = chains ? most : (num_kb + want - 1) / want, splits = (num_kb + per - 1) / per;
             if (splits != want || per > most) continue;
-            const int tab = a.a_kind == B2_OPERAND_GATHER ? per * KB * (filter_tiles(a) ? 16 : 8) : 0;
+            const int tab = dir_table_bytes(a, per * KB);
             if (1152 + dir_ring_bytes(bn) + tab > 232448) continue;
             // Measured on one B200 (cycles at 1.9 GHz): the producers set the pace, 7 (fp32) or 22
             // (flex16) cycles an operand row of a k-block when they keep an SM busy, and a k-block
@@ -707,11 +740,15 @@ DirectShape direct_shape(const b2_direct_args& a) {
             const bool a_single = a.a_kind == B2_OPERAND_K && a.a_rs % vec != 0;
             const bool b_single = a.b_kind == B2_OPERAND_K && a.b_rs % vec != 0;
             const double single = MODE == MODE_FLEX16 ? 2.0 : 1.5;
-            const double ra = a.a_kind == B2_OPERAND_GATHER ? 1.5 : a_single ? single : 1.0;
-            const double rb = filter_tiles(a) ? (a.g.channel_last ? 3.5 : 1.5) : b_single ? single : 1.0;
+            const double ra = a.a_kind == B2_OPERAND_GATHER ? (a.staged ? 1.25 : 1.5) : a_single ? single : 1.0;
+            const double rb = a.staged ? 0.0 : filter_tiles(a) ? (a.g.channel_last ? 3.5 : 1.5) : b_single ? single : 1.0;
             const long long pace = (long long)((128 * ra + bn * rb) * (MODE == MODE_FLEX16 ? (bn == 128 ? 33 : 22) : 7));
             const long long lat = MODE == MODE_FLEX16 ? (a_single || b_single ? 6000 : 4000)
-                                  : a.a_kind != B2_OPERAND_GATHER ? 1000 + 6 * bn : bn >= 64 ? 3500 : 1600 + 25 * bn;
+                                  : a.a_kind != B2_OPERAND_GATHER ? 1000 + 6 * bn
+                                  : a.staged ? (bn == 128 ? 1500 : 1700 + 6 * bn) : bn >= 64 ? 3500 : 1600 + 25 * bn;
+            // staged filters: 256 bytes a row and k-block from L2 to every SM (128 rows: 1580 cycles with one
+            // group of producers or two)
+            const long long copies = a.staged ? 25 * bn / 2 : 0;
             const long long ctas = tiles * splits, per_sm = bn == 128 || 1152 + dir_ring_bytes(bn) + tab > 115000 ? 1 : 2;
             const long long together = ctas <= 148 ? 1 : per_sm;
             // Two groups of producers where each SM has one CTA anyway and a k-block for both: a k-block then
@@ -722,10 +759,11 @@ DirectShape direct_shape(const b2_direct_args& a) {
                                1152 + dir_ring_bytes(bn, 2) + tab <= 232448 ? 2 : 1;
             long long kb = together * pace > lat ? together * pace : lat;
             if (groups == 2) kb = kb * (MODE == MODE_FLEX16 ? 65 : 60) / 100;
+            if (kb < together * copies) kb = together * copies;
             const long long slots = (long long)kClusterCtas[splits] * (groups == 2 ? 1 : per_sm);
             // (the exchange of slices: 700 and 500 a slice)
             const long long one = 7000 + per * kb + together * bn * (splits > 1 ? 24 : 12) +
-                                  (splits == 1 ? 0 : filter_tiles(a) ? 18000 : 700 + 500 * splits);
+                                  (splits == 1 ? 0 : filter_tiles(a) && !a.staged ? 18000 : 700 + 500 * splits);
             const long long waves = (ctas + slots - 1) / slots, cost = waves * one;
             if (best.cost < 0 || cost < best.cost) best = {bn, splits, per, (int)waves, groups, cost};
         }
@@ -733,22 +771,21 @@ DirectShape direct_shape(const b2_direct_args& a) {
     return best;
 }
 
-template <int MODE, int BN, int AK, int G>
+template <int MODE, int BN, int AK, int G, bool STAGED = false>
 int direct_launch_as(const DirectParams& p, cudaStream_t st) {
     const int KB = MODE == MODE_FLEX16 ? 128 : 32;
     const int ring = dir_ring_bytes(BN, G);
     static_assert(dir_ring_bytes(BN, G) >= BN * 128 * 8, "the slices' sums are exchanged through the ring");
-    const int smem = 1024 + ring + 128 +
-                     (AK == B2_OPERAND_GATHER ? p.kb_per_split * KB * (filter_tiles(p.a) ? 16 : 8) : 0);
+    const int smem = 1024 + ring + 128 + dir_table_bytes(p.a, p.kb_per_split * KB);
     static bool attr_set = false;
     if (!attr_set) {
-        B2_CUDA(cudaFuncSetAttribute(direct_kernel<MODE, BN, AK, G>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        B2_CUDA(cudaFuncSetAttribute(direct_kernel<MODE, BN, AK, G, STAGED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      AK == B2_OPERAND_GATHER ? 232448 : 1024 + ring + 128));
         attr_set = true;
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((p.a.N + BN - 1) / BN, (p.a.M + 127) / 128, p.splits);
-    cfg.blockDim = dim3(dir_threads(G));
+    cfg.blockDim = dim3(dir_threads(G, STAGED));
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cudaLaunchAttribute attr[2];
@@ -758,12 +795,14 @@ int direct_launch_as(const DirectParams& p, cudaStream_t st) {
     attr[1].val.clusterDim.x = 1; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = p.splits;
     cfg.attrs = attr;
     cfg.numAttrs = p.splits > 1 ? 2 : 1;
-    B2_CUDA(cudaLaunchKernelEx(&cfg, direct_kernel<MODE, BN, AK, G>, p));
+    B2_CUDA(cudaLaunchKernelEx(&cfg, direct_kernel<MODE, BN, AK, G, STAGED>, p));
     return B2_OK;
 }
 
 template <int MODE, int BN, int G>
 int direct_launch_bn(const DirectParams& p, cudaStream_t st) {
+    if constexpr (MODE == MODE_F32X3)
+        if (p.a.staged) return direct_launch_as<MODE, BN, B2_OPERAND_GATHER, G, true>(p, st);
     switch (p.a.a_kind) {
         case B2_OPERAND_K: return direct_launch_as<MODE, BN, B2_OPERAND_K, G>(p, st);
         case B2_OPERAND_ROWS: return direct_launch_as<MODE, BN, B2_OPERAND_ROWS, G>(p, st);
@@ -775,6 +814,8 @@ template <int MODE>
 int direct_launch_mode(const b2_direct_args& a, cudaStream_t st) {
     const DirectShape s = direct_shape<MODE>(a);
     B2_REQUIRE(s.cost >= 0, "K is too long for this kernel");
+    B2_REQUIRE(!a.staged || (MODE == MODE_F32X3 && a.a_kind == B2_OPERAND_GATHER && ((uintptr_t)a.staged & 127) == 0),
+               "staged filters: of gathered fp32 products, on 128-byte boundaries");
     DirectParams p;
     p.a = a;
     const int KB = MODE == MODE_FLEX16 ? 128 : 32, vec = MODE == MODE_FLEX16 ? 8 : 4;

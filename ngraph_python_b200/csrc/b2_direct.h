@@ -27,6 +27,8 @@ struct b2_direct_args {
     int flex;
     int a_kind, b_kind;
     const void *A, *B;
+    // gathered fp32 rows: B's k-blocks as the kernel's stages hold them (b2_direct_stage_filters), or NULL
+    const void* staged;
     long long a_rs, a_ks, b_rs, b_ks;   // element strides: A[row * a_rs + k * a_ks]; rows of B are columns of C
     int M, N, K;
     b2_gather g;
@@ -46,12 +48,21 @@ struct b2_direct_args {
 };
 
 // CTAs that the machine holds at once in clusters of 1..8 CTAs with an SM each (what
-// cudaOccupancyMaxActiveClusters says; a cluster does not cross a GPC).
-constexpr int kClusterCtas[9] = {0, 148, 148, 135, 132, 130, 132, 119, 120};
+// cudaOccupancyMaxActiveClusters says; a cluster does not cross a GPC, and which SMs of it work differs
+// from one machine to the next: 119 in clusters of seven on one, 105 on another).
+constexpr int kClusterCtas[9] = {0, 148, 148, 135, 132, 130, 132, 105, 120};
 
 // Estimated cycles of a launch, negative where the kernel does not take the problem.
 __attribute__((visibility("hidden"))) long long b2_direct_cost(const b2_direct_args& a);
 __attribute__((visibility("hidden"))) void b2_direct_plan(const b2_direct_args& a, b2_gemm_plan_info* plan);
+// `staged` operands: bytes, and the kernel that makes those of n products (fewest launches; `launches`
+// counts them).  Whether a product has its operand staged changes its shape, so `staged` is set (to
+// anything) for b2_direct_cost, b2_direct_plan and here alike.
+constexpr int kStageJobs = 16;
+struct b2_stage_job { b2_direct_args a; const float* filters; void* staged; };
+__attribute__((visibility("hidden"))) size_t b2_direct_staged_bytes(const b2_direct_args& a);
+__attribute__((visibility("hidden"))) int b2_direct_stage_filters(const b2_stage_job* jobs, int n, int* launches,
+                                                                  cudaStream_t st);
 __attribute__((visibility("hidden"))) int b2_direct_launch(const b2_direct_args& a, cudaStream_t st);
 
 // fp32 filter gradient (b2_conv_update_f32.cu): no dilation, one depth.  Scratch 0: not taken.

@@ -71,8 +71,10 @@ class _PlaneUser(object):
     """flex16 convolution steps that can run on the implicit-GEMM tile kernels: the streamed
     tensors (activations, the error tensor) are read as two byte planes which their producer
     writes directly -- or else the first step that reads them -- and the filter planes are kept for
-    as long as the filters do not change: one launch per convolution."""
+    as long as the filters do not change: one launch per convolution.  fp32: the filters as the
+    kernel that gathers its operands holds them (`tiles`), kept likewise."""
     use_planes = False
+    tiles = False
     plane_args = ()                 # indexes of the tensors read as planes in op.args / in_views
     splits = ()                     # those that this step splits unless their producer has
     filters_change = False          # the computation writes the filters, or takes them as an argument
@@ -82,17 +84,22 @@ class _PlaneUser(object):
     filter_version = None
 
     def _setup_planes(self, t, conv_pass, stream_arg, filter_arg):
-        if not self.flex:
-            return
-        ok, _, filt_bytes = lib.conv_planes_info(self.dims, conv_pass)
+        if self.flex:
+            ok, _, filt_bytes = lib.conv_planes_info(self.dims, conv_pass)
+        else:
+            filt_bytes = lib.conv_filter_tiles_info(self.dims, conv_pass)
+            ok = filt_bytes > 0
         if not ok:
             return
-        self.use_planes = True
         self.conv_pass = conv_pass
         self.filter_arg = filter_arg
         self.filter_bytes = filt_bytes
         self.in_views[filter_arg].buffer.watched = True
-        self._read_planes((stream_arg,))
+        if self.flex:
+            self.use_planes = True
+            self._read_planes((stream_arg,))
+        else:
+            self.tiles = True
 
     def _read_planes(self, args):
         self.plane_args = self.splits = args
@@ -119,31 +126,48 @@ class _PlaneUser(object):
         return False
 
     def allocate(self, t):
-        if self.use_planes and self.filter_planes is None and not t.plan_only:
+        if (self.use_planes or self.tiles) and self.filter_planes is None and not t.plan_only:
             self.filter_planes = t.torch.zeros((self.filter_bytes + 1024,), dtype=t.torch.uint8,
                                                device=t.device)
             self.filter_ptr = self.filter_planes.data_ptr() + (-self.filter_planes.data_ptr()) % 1024
 
     def _build_filter_planes(self, t):
         fv = self.in_views[self.filter_arg]
+        if self.tiles:
+            self._build_tiles(t, [self])
+            self.filter_version = fv.buffer.version
+            return
         lib.check(lib.raw().b2_conv_filter_planes(self._ptr(fv), C.byref(self.dims), self.conv_pass,
                                                   self.filter_ptr, t.stream.cuda_stream))
         t.kernel_launches += 1
         self.filter_version = fv.buffer.version
 
-    def _build_joint_planes(self, t):
-        users = self.joint_planes
+    @staticmethod
+    def _build_tiles(t, users):
+        jobs, n = _PlaneUser._filter_jobs(users), C.c_int32()
+        lib.check(lib.raw().b2_conv_filter_tiles(jobs, len(users), C.byref(n), t.stream.cuda_stream))
+        t.kernel_launches += n.value
+
+    @staticmethod
+    def _filter_jobs(users):
         jobs = (lib.ConvFilterJob * len(users))()
         for job, s in zip(jobs, users):
             job.filters, job.planes = s._ptr(s.in_views[s.filter_arg]), s.filter_ptr
             job.dims, job.conv_pass = s.dims, s.conv_pass
-        n = C.c_int32()
+        return jobs
+
+    def _build_joint_planes(self, t):
+        users = self.joint_planes
+        if self.tiles:
+            self._build_tiles(t, users)
+            return
+        jobs, n = self._filter_jobs(users), C.c_int32()
         lib.check(lib.raw().b2_conv_filter_planes_many(jobs, len(users), C.byref(n), t.stream.cuda_stream))
         t.kernel_launches += n.value
 
     def kept_planes(self):
         """Whether `refresh` can have anything to do."""
-        return self.use_planes and not self.planes_built_first and not self.filters_change
+        return (self.use_planes or self.tiles) and not self.planes_built_first and not self.filters_change
 
     def refresh(self, t):
         """Rebuilds the cached filter planes when the filters have changed since they were built
@@ -162,13 +186,8 @@ class _PlaneUser(object):
                     raise ValueError("fused convolution %s must be a dense tensor" % key)
                 self.in_views.append(v)
 
-    def _launch_planes(self, t):
-        xv, fv = self.in_views[self.plane_args[0]], self.in_views[self.filter_arg]
-        ov = self.out_views[0]
-        raw = lib.raw()
-        st = t.stream.cuda_stream
-        xbuf, fbuf = xv.buffer, fv.buffer
-        planes_ptr = self._planes(t, self.plane_args[0])
+    def _current_filter_planes(self, t):
+        fbuf = self.in_views[self.filter_arg].buffer
         if self.joint_planes:
             self._build_joint_planes(t)
         elif self.planes_built_first:
@@ -177,6 +196,26 @@ class _PlaneUser(object):
             self._build_filter_planes(t)
         else:
             self.refresh(t)
+
+    def _launch_tiles(self, t):
+        self._current_filter_planes(t)
+        epi = getattr(self, "epi", None) or {}
+        extra = [self._ptr(v) for v in self.in_views[2:]]
+        tail = [extra.pop(0) if epi.get(k) is not None else None for k in ("bias", "residual", "mask")]
+        lib.check(lib.raw().b2_conv_f32_tiles(
+            self.conv_pass, self._ptr(self.in_views[1 - self.filter_arg]), self.filter_ptr,
+            self._ptr(self.out_views[0]), C.byref(self.dims), tail[0], tail[1], int(bool(epi.get("relu"))),
+            tail[2], t._status.data_ptr(), t.stream.cuda_stream))
+        t.kernel_launches += self.launches
+
+    def _launch_planes(self, t):
+        xv, fv = self.in_views[self.plane_args[0]], self.in_views[self.filter_arg]
+        ov = self.out_views[0]
+        raw = lib.raw()
+        st = t.stream.cuda_stream
+        xbuf, fbuf = xv.buffer, fv.buffer
+        planes_ptr = self._planes(t, self.plane_args[0])
+        self._current_filter_planes(t)
         slots = (t._slot_for_read(xbuf, self), t._slot_for_read(fbuf, self), ov.buffer.slot_write)
         epi = getattr(self, "epi", None)
         if epi is None:
@@ -492,6 +531,8 @@ class ConvStep(_PlaneUser, _Step):
     def launch(self, t):
         if self.use_planes:
             return self._launch_planes(t)
+        if self.tiles:
+            return self._launch_tiles(t)
         iv, fv = self.in_views[:2]
         ov = self.out_views[0]
         raw = lib.raw()
@@ -600,6 +641,8 @@ class _ConvGradStep(_PlaneUser, _Step):
     def launch(self, t):
         if self.use_planes:
             return self._launch_planes(t)
+        if self.tiles:
+            return self._launch_tiles(t)
         av, bv = self.in_views[:2]       # (delta, filters) or (delta, inputs)
         ov = self.out_views[0]
         raw = lib.raw()

@@ -165,6 +165,9 @@ def _load():
         "b2_conv_split_activations": (C.c_int, [vp, C.POINTER(ConvDims), i32, vp, vp]),
         "b2_conv_filter_planes_many": (C.c_int, [C.POINTER(ConvFilterJob), i32, C.POINTER(i32), vp]),
         "b2_conv_split_planes": (C.c_int, [vp, i32, i32, i32, i32, vp, vp]),
+        "b2_conv_filter_tiles_info": (C.c_int, [C.POINTER(ConvDims), i32, C.POINTER(sz)]),
+        "b2_conv_filter_tiles": (C.c_int, [C.POINTER(ConvFilterJob), i32, C.POINTER(i32), vp]),
+        "b2_conv_f32_tiles": (C.c_int, [i32, vp, vp, vp, C.POINTER(ConvDims), vp, vp, i32, vp, vp, vp]),
         "b2_conv_filter_planes": (C.c_int, [vp, C.POINTER(ConvDims), i32, vp, vp]),
         "b2_conv_flex16_planes": (C.c_int, [i32, vp, vp, vp, C.POINTER(ConvDims), vp, i32, i32,
                                             i32, vp, vp, vp, i32, vp]),
@@ -447,6 +450,13 @@ def conv_planes_info(dims, conv_pass=CONV_FPROP):
     ok, a, f = C.c_int32(), C.c_size_t(), C.c_size_t()
     check(_lib.b2_conv_planes_info(C.byref(dims), conv_pass, C.byref(ok), C.byref(a), C.byref(f)))
     return bool(ok.value), a.value, f.value
+
+
+def conv_filter_tiles_info(dims, conv_pass):
+    """Bytes of the filters as the fp32 kernel's stages hold them; 0 where it takes them as they lie."""
+    n = C.c_size_t()
+    check(_lib.b2_conv_filter_tiles_info(C.byref(dims), conv_pass, C.byref(n)))
+    return n.value
 
 
 def conv_chain_info(layers):
