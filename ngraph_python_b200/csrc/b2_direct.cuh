@@ -13,7 +13,11 @@
 //   fp32:   3xTF32, in chains of at most 16 k-blocks (the tensor core's fp32 sum truncates); longer K
 //           is cut into slices.  Matrix products add hi*hi, hi*lo and lo*hi into one sum (see ONE_CHAIN).
 //           Convolutions keep two: B's planes lie behind one another and make one operand of 2*BN rows,
-//           A_hi x [B_hi | B_lo] -> [hh | x], A_lo x B_hi -> x.
+//           A_hi x [B_hi | B_lo] -> [hh | x], A_lo x B_hi -> x.  Where tiles of many pixels stretch a sum
+//           over more k-blocks, between the zeros of their filters (staged ones), even and odd k-blocks have
+//           a pair each: against 64 bits, 22-layer networks' shapes at batch 1 to 1000, no error is larger
+//           than with one pair and filters as they lie, most are half (16 channels at 32x32 5.0e-7 -> 2.9e-7
+//           of the result's root mean square), for one percent of the time.
 //   flex16: four exact int8 products, HH | X | LL as in b2_gemm_impl.cuh.
 // Slices of K: the CTAs of a cluster (up to 8) take one each; partial sums meet in distributed shared
 // memory, every CTA adds a share of the columns in slice order (deterministic, fp32 adds rounded to
@@ -25,8 +29,8 @@
 // one CTA (one B200, one group -> two, us: fp32 512 x 128 x 784 16.7 -> 11.5, 600 x 600 x 600 24.5 -> 14.6,
 // flex16 512 x 128 x 784 11.0 -> 8.7, 905 x 380 x 611 24.1 -> 15.0; 20 % of it over 38 sizes).
 // Unrolled convolutions whose filters were laid out beforehand leave the producers only the gathered rows, and
-// tiles of more pixels pay (batch 100, forward / input gradient, us: 16 channels at 32x32 20.2 -> 12.8 / 25.1 ->
-// 12.8, 32 at 16x16 14.6 -> 12.0 / 23.3 -> 12.0, 64 at 8x8 14.3 -> 11.7 / 14.2 -> 11.7); the filters' way from L2 to
+// tiles of more pixels pay (batch 100, forward / input gradient, us: 16 channels at 32x32 20.2 -> 12.9 / 25.1 ->
+// 12.9, 32 at 16x16 14.6 -> 12.1 / 23.3 -> 12.2, 64 at 8x8 14.3 -> 12.1 / 14.2 -> 12.1); the filters' way from L2 to
 // every SM, 256 bytes a row and k-block, then bounds the widest tiles.
 #ifndef B2_DIRECT_CUH
 #define B2_DIRECT_CUH
@@ -45,8 +49,8 @@ __host__ __device__ constexpr int dir_stages(int bn, int groups = 1) {
 __host__ __device__ constexpr int dir_threads(int groups, bool staged = false) { return groups * 256 + (staged ? 64 : 32); }
 __host__ __device__ constexpr int dir_stage_bytes(int bn) { return 2 * (128 + bn) * 128; }
 __host__ __device__ constexpr int dir_ring_bytes(int bn, int groups = 1) { return dir_stages(bn, groups) * dir_stage_bytes(bn); }
-__host__ __device__ constexpr int dir_tmem_cols(int mode, int bn) {
-    int need = (mode == MODE_FLEX16 ? 3 : 2) * bn, c = 32;
+__host__ __device__ constexpr int dir_tmem_cols(int mode, int bn, bool staged = false) {
+    int need = (mode == MODE_FLEX16 ? 3 : staged ? 4 : 2) * bn, c = 32;
     while (c < need) c *= 2;
     return c;
 }
@@ -190,7 +194,7 @@ direct_kernel(const __grid_constant__ DirectParams p) {
     constexpr int NST = dir_stages(BN, G), STAGE = dir_stage_bytes(BN), MMA_WARP = 8 * G;
     constexpr int KB = MODE == MODE_FLEX16 ? 128 : 32;            // columns of a k-block
     constexpr int PER = KB / 8;                                   // columns of a 16-byte chunk
-    constexpr int kCols = dir_tmem_cols(MODE, BN);
+    constexpr int kCols = dir_tmem_cols(MODE, BN, STAGED);
     // fp32 matrix products: one accumulator, the three products of a k-step in the order of the plane
     // kernels, slices of whole chains -- the same rounding whichever kernel a size takes (a mask `x > 0`
     // of a value near zero would otherwise change with the dispatch)
@@ -487,10 +491,11 @@ direct_kernel(const __grid_constant__ DirectParams p) {
             const unsigned long long dA0 = make_smem_desc(st), dA1 = make_smem_desc(st + 128 * 128);
             const unsigned long long dB0 = make_smem_desc(st + 2 * 128 * 128);
             const unsigned long long dB1 = make_smem_desc(st + 2 * 128 * 128 + BN * 128);
+            const unsigned sums = tmem_base + (STAGED && (kb & 1) ? 2 * BN : 0);
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
                 const unsigned long long adv = (unsigned long long)(2 * k);
-                const unsigned acc = (kb > 0 || k > 0) ? 1u : 0u;
+                const unsigned acc = (kb > (STAGED ? 1 : 0) || k > 0) ? 1u : 0u;
                 if (MODE == MODE_FLEX16) {
                     tc_mma<MODE>(tmem_base, dA0 + adv, dB0 + adv, id_ss, acc);               // HH
                     tc_mma<MODE>(tmem_base + BN, dA0 + adv, dB1 + adv, id_su, acc);          // X += ah*bl
@@ -503,8 +508,8 @@ direct_kernel(const __grid_constant__ DirectParams p) {
                     tc_mma<MODE>(tmem_base, a.colmajor ? dA0 + adv : dA1 + adv,
                                  a.colmajor ? dB1 + adv : dB0 + adv, id_t1, 1u);
                 } else {
-                    tc_mma<MODE>(tmem_base, dA0 + adv, dB0 + adv, id_t2, acc);               // hh | x
-                    tc_mma<MODE>(tmem_base + BN, dA1 + adv, dB0 + adv, id_t1, 1u);           // x += lo*hi
+                    tc_mma<MODE>(sums, dA0 + adv, dB0 + adv, id_t2, acc);                    // hh | x
+                    tc_mma<MODE>(sums + BN, dA1 + adv, dB0 + adv, id_t1, 1u);                // x += lo*hi
                 }
             }
             tc_commit(&empty_bar[s]);
@@ -635,10 +640,21 @@ direct_kernel(const __grid_constant__ DirectParams p) {
                 for (int j = 0; j < 8; ++j)
                     v[j] = (Sum)(((long long)(int)hh[j] << 16) + ((long long)(int)xx[j] << 8) + (long long)(int)ll[j]);
             } else {
-                unsigned hh[8], xx[8];
+                unsigned hh[8], xx[8], h1[8], x1[8];
                 tmem_ld8(lane_addr + c0, hh);
                 if (!ONE_CHAIN) tmem_ld8(lane_addr + BN + c0, xx);
+                if (STAGED && nkb > 1) {
+                    tmem_ld8(lane_addr + 2 * BN + c0, h1);
+                    tmem_ld8(lane_addr + 3 * BN + c0, x1);
+                }
                 tmem_ld_wait();
+                if (STAGED && nkb > 1) {
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        hh[j] = __float_as_uint(__uint_as_float(hh[j]) + __uint_as_float(h1[j]));
+                        xx[j] = __float_as_uint(__uint_as_float(xx[j]) + __uint_as_float(x1[j]));
+                    }
+                }
 #pragma unroll
                 for (int j = 0; j < 8; ++j)
                     v[j] = ONE_CHAIN ? (Sum)__uint_as_float(hh[j])
