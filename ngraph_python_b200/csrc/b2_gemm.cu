@@ -21,7 +21,7 @@ inline bool goes_in_pairs(const Shapes& s, int M, int splits) {
     return s.bn == 128 && M > kBlockM && splits == 1;
 }
 
-// Cycles of the plane path: two pre-pass launches (and a memset), their traffic, and the tile kernel at
+// Cycles of the plane path: the pre-pass launch (flex16 with a memset), its traffic, and the tile kernel at
 // the cycles measured for a k-block.
 inline long long plane_cost(int mode, const Shapes& s, int M, int N, int K) {
     const long long prepass = ((long long)M + N) * K * (mode == MODE_FLEX16 ? 4 : 12) / 2600;
@@ -29,12 +29,12 @@ inline long long plane_cost(int mode, const Shapes& s, int M, int N, int K) {
     if (goes_in_pairs(s, M, pick_splits(mode, s, false))) {
         const int tiles = ((M + 255) / 256) * ((N + 127) / 128), z = pair_splits(mode, tiles, (int)num_kb);
         const long long kb = mode == MODE_FLEX16 ? 1100 : 900;
-        return (mode == MODE_FLEX16 ? 20000 : 14000) + prepass +
+        return (mode == MODE_FLEX16 ? 17500 : 12500) + prepass +
                pair_waves(tiles, z) * (5000 + pair_slice(mode, (int)num_kb, z) * kb) + (z > 1 ? 2500 : 0);
     }
     const long long kb = (mode == MODE_FLEX16 ? 1430LL : 1100LL) * (128 + s.bn) / 256;
     const long long tiles = (long long)(s.Mp / kBlockM) * (s.Np / s.bn);
-    return (mode == MODE_FLEX16 ? 20000 : 13000) + prepass + (tiles + 147) / 148 * (3500 + num_kb * kb);
+    return (mode == MODE_FLEX16 ? 17500 : 11500) + prepass + (tiles + 147) / 148 * (3500 + num_kb * kb);
 }
 
 // Whether a product takes the kernel that converts its operands on the way in (one launch), and its
@@ -88,12 +88,12 @@ int run_gemm(const T* A, long long a_rs, long long a_cs, const T* B, long long b
     if (MODE == MODE_FLEX16) {
         rowsum = (int*)(base + s.rowsum_off);
         lo_xor = 0x80;
-        B2_CUDA(cudaMemsetAsync(rowsum, 0, (size_t)s.Mp * sizeof(int), st));
     }
-    int rc = split_operand<T, MODE>(A, a_rs, a_cs, M, K, s.Mp, s.Kp, A0, A1, 0, rowsum, st);
-    if (rc) return rc;
+    const SplitJob ja = split_job<T, MODE>(A, a_rs, a_cs, M, K, s.Mp, s.Kp, A0, A1, 0, rowsum);
+    if (rowsum && ja.way != kSplitRowSums) B2_CUDA(cudaMemsetAsync(rowsum, 0, (size_t)s.Mp * sizeof(int), st));
     // op(B)^T: rows = N, element (n, k) = B[k * b_ks + n * b_ns]
-    rc = split_operand<T, MODE>(B, b_ns, b_ks, N, K, s.Np, s.Kp, B0, B1, lo_xor, nullptr, st);
+    const SplitJob jb = split_job<T, MODE>(B, b_ns, b_ks, N, K, s.Np, s.Kp, B0, B1, lo_xor, nullptr);
+    const int rc = split_operands<T, MODE>(ja, jb, st);
     if (rc) return rc;
     GemmParams p;
     p.M = M; p.N = N; p.num_kb = 0;
@@ -120,7 +120,7 @@ extern "C" int b2_gemm_launches(int32_t flex, int64_t a_k_stride, int64_t b_k_st
     const int mode = flex ? MODE_FLEX16 : MODE_F32X3;
     b2_direct_args d;
     *launches = gemm_goes_direct(mode, nullptr, 1, a_k_stride, nullptr, b_k_stride, 1, M, N, K, &d) ? 1
-                : pick_splits(mode, shapes_for(mode, M, N, K), false) > 1 ? 4 : 3;
+                : pick_splits(mode, shapes_for(mode, M, N, K), false) > 1 ? 3 : 2;
     return B2_OK;
 }
 

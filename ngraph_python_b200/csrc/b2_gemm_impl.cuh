@@ -651,11 +651,26 @@ splitk_finish_kernel(const GemmParams p, int splits) {
 // ---- pre-pass: operand planes, K-major, zero padded ---------------------------------------------
 // src element (r, k) of op(X) is src[r * rs + k * cs]; planes are [rows_p][kp] with kp contiguous.
 //   flex16: plane0 = high byte (signed), plane1 = low byte XOR lo_xor (lo_xor = 0x80 stores the
-//           signed byte lo - 128); rowsum (optional) accumulates sum_k of the int16 values per row.
+//           signed byte lo - 128); rowsum (optional): sum_k of the int16 values per row, stored where
+//           a row has its own warps (kSplitRowSums), else added to what is there.
 //   fp32:   plane0 = value rounded to tf32, plane1 = remainder.
-// Three kernels: K contiguous with 16-byte aligned rows (vector loads, no staging), rows contiguous
+// Three ways: K contiguous with 16-byte aligned rows (vector loads, no staging), rows contiguous
 // with aligned columns (64x64 / 64x32 tiles transposed through shared memory, vector loads and
-// stores), and a 32x32-tile kernel without any alignment requirement.
+// stores), and 32x32 tiles without any alignment requirement.  One launch takes both operands of a product,
+// each its own way: up to some thousand rows a pre-pass is its launch (fp32 1000 x 777 x 1500: 29.8 -> 28.8 us
+// with the product; flex16, where a memset had to clear the row sums as well, 38.6 -> 35.3, 1536 x 1536 x 1536
+// 24.4 -> 22.7).
+enum { kSplitRows, kSplitRowSums, kSplitCols, kSplitAny };
+struct SplitJob {
+    const void* src;
+    long long rs, cs;
+    int rows, k, rows_p, kp;
+    void *plane0, *plane1;
+    unsigned lo_xor;
+    int* rowsum;
+    int way, across, blocks;             // blocks, `across` of them along K
+};
+struct SplitJobs { SplitJob a, b; };     // (b.blocks == 0: one operand)
 
 __device__ __forceinline__ void tf32_split(float a, float& hi, float& lo) {
     unsigned hb;
@@ -670,23 +685,14 @@ __device__ __forceinline__ void add_rowsum(int* rowsum, int r, int rows, int v, 
     if ((threadIdx.x & (group - 1)) == 0 && r < rows && v != 0) atomicAdd(rowsum + r, v);
 }
 
-// K contiguous: one thread = 16 int16 (two 16-byte loads) or 4 floats of one row
+// K contiguous: a unit is 16 int16 (two 16-byte loads) or 4 floats of one row; the sum of its values
 template <typename T, int MODE>
-__global__ void __launch_bounds__(256)
-split_rows_kernel(const T* __restrict__ src, long long rs, int rows, int k, int rows_p, int kp,
-                  void* __restrict__ plane0, void* __restrict__ plane1, unsigned lo_xor,
-                  int* __restrict__ rowsum) {
-    after_earlier_kernels();
-    constexpr int kPer = MODE == MODE_FLEX16 ? 16 : 4;
-    const int upr = kp / kPer;                                   // units per row
-    const long long idx = (long long)blockIdx.x * 256 + threadIdx.x;
-    const bool live = idx < (long long)rows_p * upr;
-    const int r = live ? (int)(idx / upr) : rows_p;
-    const int kk = live ? (int)(idx % upr) * kPer : 0;
+__device__ __forceinline__ int split_unit(const T* __restrict__ src, long long rs, int rows, int k, int kp, int r,
+                                          int kk, void* __restrict__ plane0, void* __restrict__ plane1, unsigned lo_xor) {
     const long long o = (long long)r * kp + kk;
     if (MODE == MODE_FLEX16) {
         unsigned w[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-        if (live && r < rows) {
+        if (r < rows) {
             const short* sp = (const short*)src + (long long)r * rs + kk;
             if (kk + 16 <= k) {
                 const int4 a = __ldg((const int4*)sp), b = __ldg((const int4*)sp + 1);
@@ -706,18 +712,12 @@ split_rows_kernel(const T* __restrict__ src, long long rs, int rows, int k, int 
             sum += ((int)(w[2 * j] << 16) >> 16) + ((int)w[2 * j] >> 16) +
                    ((int)(w[2 * j + 1] << 16) >> 16) + ((int)w[2 * j + 1] >> 16);
         }
-        if (live) {
-            *(int4*)((unsigned char*)plane0 + o) = make_int4(hi[0], hi[1], hi[2], hi[3]);
-            *(int4*)((unsigned char*)plane1 + o) = make_int4(lo[0], lo[1], lo[2], lo[3]);
-        }
-        if (rowsum) {
-            const int r0 = __shfl_sync(0xffffffffu, r, 0);
-            if (__all_sync(0xffffffffu, r == r0)) add_rowsum(rowsum, r, rows, sum, 32);
-            else if (r < rows && sum != 0) atomicAdd(rowsum + r, sum);
-        }
+        *(int4*)((unsigned char*)plane0 + o) = make_int4(hi[0], hi[1], hi[2], hi[3]);
+        *(int4*)((unsigned char*)plane1 + o) = make_int4(lo[0], lo[1], lo[2], lo[3]);
+        return sum;
     } else {
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (live && r < rows) {
+        if (r < rows) {
             const float* sp = (const float*)src + (long long)r * rs + kk;
             if (kk + 4 <= k) v = __ldg((const float4*)sp);
             else {
@@ -729,27 +729,24 @@ split_rows_kernel(const T* __restrict__ src, long long rs, int rows, int k, int 
         float4 h, l;
         tf32_split(v.x, h.x, l.x); tf32_split(v.y, h.y, l.y);
         tf32_split(v.z, h.z, l.z); tf32_split(v.w, h.w, l.w);
-        if (live) {
-            *(float4*)((float*)plane0 + o) = h;
-            *(float4*)((float*)plane1 + o) = l;
-        }
+        *(float4*)((float*)plane0 + o) = h;
+        *(float4*)((float*)plane1 + o) = l;
+        return 0;
     }
 }
 
 // rows contiguous in the source (element (r, k) at src[k * cs + r]): tiles of 64 rows x 64 k
 // (flex16) or 64 rows x 32 k (fp32) are read with 16-byte loads along r, transposed through shared
 // memory and written with 16- / 32-byte stores along k.
+template <int MODE> constexpr int kSplitTileK = MODE == MODE_FLEX16 ? 64 : 32;
+template <int MODE> constexpr int kSplitPitch = MODE == MODE_FLEX16 ? 66 : 65;       // elements; odd word pitch
 template <typename T, int MODE>
-__global__ void __launch_bounds__(256)
-split_cols_kernel(const T* __restrict__ src, long long cs, int rows, int k, int rows_p, int kp,
-                  void* __restrict__ plane0, void* __restrict__ plane1, unsigned lo_xor,
-                  int* __restrict__ rowsum) {
-    after_earlier_kernels();
-    constexpr int kTileK = MODE == MODE_FLEX16 ? 64 : 32;
-    constexpr int kPitch = MODE == MODE_FLEX16 ? 66 : 65;       // elements; odd word pitch
-    __shared__ T tile[kTileK * kPitch];
+__device__ __forceinline__ void split_cols(const T* __restrict__ src, long long cs, int rows, int k, int rows_p, int kp,
+                                           void* __restrict__ plane0, void* __restrict__ plane1, unsigned lo_xor,
+                                           int* __restrict__ rowsum, int bx, int by, T* tile) {
+    constexpr int kTileK = kSplitTileK<MODE>, kPitch = kSplitPitch<MODE>;
     const int tid = threadIdx.x;
-    const int r0 = blockIdx.y * 64, k0 = blockIdx.x * kTileK;
+    const int r0 = by * 64, k0 = bx * kTileK;
     if (MODE == MODE_FLEX16) {
         // load: 8 rows per thread per k; 8 threads cover 64 rows, 32 k per pass
         for (int i = 0; i < 2; ++i) {
@@ -826,24 +823,25 @@ split_cols_kernel(const T* __restrict__ src, long long cs, int rows, int k, int 
 // no alignment requirement: 32x32 tiles through shared memory so that both the read and the write
 // are coalesced whichever of rs / cs is 1.
 template <typename T, int MODE>
-__global__ void __launch_bounds__(256)
-split_planes_kernel(const T* __restrict__ src, long long rs, long long cs, int rows, int k,
-                    int rows_p, int kp, void* __restrict__ plane0, void* __restrict__ plane1,
-                    unsigned lo_xor, int* __restrict__ rowsum) {
-    after_earlier_kernels();
-    __shared__ T tile[32][33];
+__device__ __forceinline__ void split_any(const T* __restrict__ src, long long rs, long long cs, int rows, int k,
+                                          int rows_p, int kp, void* __restrict__ plane0, void* __restrict__ plane1,
+                                          unsigned lo_xor, int* __restrict__ rowsum, int bx, int by, T (*tile)[33]) {
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;     // 32 x 8
-    const int r0 = blockIdx.y * 32, k0 = blockIdx.x * 32;
+    const int r0 = by * 32, k0 = bx * 32;
     const bool k_contig = (cs == 1);
-    for (int i = ty; i < 32; i += 8) {
+    T v[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
         // read so that the contiguous source direction runs along tx
-        const int r = k_contig ? r0 + i : r0 + tx;
+        const int i = ty + 8 * q, r = k_contig ? r0 + i : r0 + tx;
         const int kk = k_contig ? k0 + tx : k0 + i;
-        T v = 0;
-        if (r < rows && kk < k) v = src[(long long)r * rs + (long long)kk * cs];
-        if (k_contig) tile[i][tx] = v; else tile[tx][i] = v;
+        v[q] = r < rows && kk < k ? __ldg(src + (long long)r * rs + (long long)kk * cs) : (T)0;
     }
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+        if (k_contig) tile[ty + 8 * q][tx] = v[q]; else tile[tx][ty + 8 * q] = v[q];
     __syncthreads();
+#pragma unroll
     for (int i = ty; i < 32; i += 8) {
         const int r = r0 + i, kk = k0 + tx;
         const T v = tile[i][tx];
@@ -865,28 +863,80 @@ split_planes_kernel(const T* __restrict__ src, long long rs, long long cs, int r
     }
 }
 
-// Picks the pre-pass kernel for one operand.
+template <typename T, int MODE>
+__global__ void __launch_bounds__(256)
+split_kernel(const __grid_constant__ SplitJobs jobs) {
+    after_earlier_kernels();
+    __shared__ alignas(16) T tile[kSplitTileK<MODE> * kSplitPitch<MODE>];
+    static_assert(kSplitTileK<MODE> * kSplitPitch<MODE> >= 32 * 33, "one array for both");
+    const bool second = (int)blockIdx.x >= jobs.a.blocks;
+    const SplitJob& j = second ? jobs.b : jobs.a;
+    const int block = (int)blockIdx.x - (second ? jobs.a.blocks : 0);
+    const T* src = (const T*)j.src;
+    constexpr int kPer = MODE == MODE_FLEX16 ? 16 : 4;
+    if (j.way == kSplitRows) {
+        const int upr = j.kp / kPer;                             // units per row
+        const long long idx = (long long)block * 256 + threadIdx.x;
+        if (idx < (long long)j.rows_p * upr)
+            split_unit<T, MODE>(src, j.rs, j.rows, j.k, j.kp, (int)(idx / upr), (int)(idx % upr) * kPer, j.plane0, j.plane1,
+                                j.lo_xor);
+    } else if (j.way == kSplitRowSums) {
+        // four warps to a row (one: 2173 rows of 2728 values leave an SM 16 warps, 39.2 us with the product
+        // instead of 31.6)
+        const int warp = threadIdx.x >> 5, r = block * 2 + (warp >> 2);
+        int sum = 0;
+        for (int kk = (threadIdx.x & 127) * kPer; kk < j.kp; kk += 128 * kPer)
+            sum += split_unit<T, MODE>(src, j.rs, j.rows, j.k, j.kp, r, kk, j.plane0, j.plane1, j.lo_xor);
+        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        int* part = (int*)tile;
+        if ((threadIdx.x & 31) == 0) part[warp] = sum;
+        __syncthreads();
+        if ((threadIdx.x & 127) == 0) j.rowsum[r] = part[warp] + part[warp + 1] + part[warp + 2] + part[warp + 3];
+    } else if (j.way == kSplitCols) {
+        split_cols<T, MODE>(src, j.cs, j.rows, j.k, j.rows_p, j.kp, j.plane0, j.plane1, j.lo_xor, j.rowsum,
+                            block % j.across, block / j.across, tile);
+    } else {
+        split_any<T, MODE>(src, j.rs, j.cs, j.rows, j.k, j.rows_p, j.kp, j.plane0, j.plane1, j.lo_xor, j.rowsum,
+                           block % j.across, block / j.across, (T(*)[33])tile);
+    }
+}
+
+// How an operand is split.
+template <typename T, int MODE>
+SplitJob split_job(const T* src, long long rs, long long cs, int rows, int k, int rows_p, int kp, void* plane0,
+                   void* plane1, unsigned lo_xor, int* rowsum) {
+    const bool base16 = ((uintptr_t)src & 15) == 0;
+    const int vec = 16 / (int)sizeof(T);
+    SplitJob j = {src, rs, cs, rows, k, rows_p, kp, plane0, plane1, lo_xor, rowsum, kSplitAny, 1, 0};
+    if (cs == 1 && base16 && rs % vec == 0) {
+        const long long units = (long long)rows_p * (kp / (MODE == MODE_FLEX16 ? 16 : 4));
+        j.way = rowsum ? kSplitRowSums : kSplitRows;
+        j.blocks = rowsum ? rows_p / 2 : (int)((units + 255) / 256);
+    } else if (rs == 1 && base16 && cs % vec == 0) {
+        j.way = kSplitCols;
+        j.across = (kp + kSplitTileK<MODE> - 1) / kSplitTileK<MODE>;
+        j.blocks = j.across * ((rows_p + 63) / 64);
+    } else {
+        j.across = (kp + 31) / 32;
+        j.blocks = j.across * ((rows_p + 31) / 32);
+    }
+    return j;
+}
+
+template <typename T, int MODE>
+int split_operands(const SplitJob& a, const SplitJob& b, cudaStream_t st) {
+    B2_REQUIRE((long long)a.blocks + b.blocks < (1LL << 31), "operands too large");
+    const SplitJobs jobs = {a, b};
+    B2_CUDA(b2::launch_after(split_kernel<T, MODE>, dim3((unsigned)(a.blocks + b.blocks)), 256, 0, st, jobs));
+    B2_CUDA(cudaGetLastError());
+    return B2_OK;
+}
+
 template <typename T, int MODE>
 int split_operand(const T* src, long long rs, long long cs, int rows, int k, int rows_p, int kp,
                   void* plane0, void* plane1, unsigned lo_xor, int* rowsum, cudaStream_t st) {
-    const bool base16 = ((uintptr_t)src & 15) == 0;
-    const int vec = 16 / (int)sizeof(T);
-    if (cs == 1 && base16 && rs % vec == 0) {
-        const long long units = (long long)rows_p * (kp / (MODE == MODE_FLEX16 ? 16 : 4));
-        B2_CUDA(b2::launch_after(split_rows_kernel<T, MODE>, dim3((unsigned)((units + 255) / 256)), 256, 0, st, 
-            src, rs, rows, k, rows_p, kp, plane0, plane1, lo_xor, rowsum));
-    } else if (rs == 1 && base16 && cs % vec == 0) {
-        const int tk = MODE == MODE_FLEX16 ? 64 : 32;
-        dim3 g((kp + tk - 1) / tk, (rows_p + 63) / 64);
-        B2_CUDA(b2::launch_after(split_cols_kernel<T, MODE>, dim3(g), 256, 0, st, src, cs, rows, k, rows_p, kp, plane0, plane1,
-                                                     lo_xor, rowsum));
-    } else {
-        dim3 g((kp + 31) / 32, (rows_p + 31) / 32);
-        B2_CUDA(b2::launch_after(split_planes_kernel<T, MODE>, dim3(g), 256, 0, st, src, rs, cs, rows, k, rows_p, kp, plane0,
-                                                       plane1, lo_xor, rowsum));
-    }
-    B2_CUDA(cudaGetLastError());
-    return B2_OK;
+    return split_operands<T, MODE>(split_job<T, MODE>(src, rs, cs, rows, k, rows_p, kp, plane0, plane1, lo_xor, rowsum),
+                                   SplitJob(), st);
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*,
