@@ -21,20 +21,21 @@ inline bool goes_in_pairs(const Shapes& s, int M, int splits) {
     return s.bn == 128 && M > kBlockM && splits == 1;
 }
 
-// Cycles of the plane path: the pre-pass launch (flex16 with a memset), its traffic, and the tile kernel at
-// the cycles measured for a k-block.
+// Cycles of the plane path: the pre-pass launch, its traffic, and the tile kernel at the cycles measured for a
+// k-block.  (2500 cycles less, for the launch that two operands share, sends products the wrong way: flex16
+// 2165 x 116 x 1878 22 us direct, 34 on planes, 1121 x 705 x 489 23 and 29; fp32 942 x 2897 x 54 24 and 27.)
 inline long long plane_cost(int mode, const Shapes& s, int M, int N, int K) {
     const long long prepass = ((long long)M + N) * K * (mode == MODE_FLEX16 ? 4 : 12) / 2600;
     const long long num_kb = s.Kp / (kKBytes / s.esize);
     if (goes_in_pairs(s, M, pick_splits(mode, s, false))) {
         const int tiles = ((M + 255) / 256) * ((N + 127) / 128), z = pair_splits(mode, tiles, (int)num_kb);
         const long long kb = mode == MODE_FLEX16 ? 1100 : 900;
-        return (mode == MODE_FLEX16 ? 17500 : 12500) + prepass +
+        return (mode == MODE_FLEX16 ? 20000 : 14000) + prepass +
                pair_waves(tiles, z) * (5000 + pair_slice(mode, (int)num_kb, z) * kb) + (z > 1 ? 2500 : 0);
     }
     const long long kb = (mode == MODE_FLEX16 ? 1430LL : 1100LL) * (128 + s.bn) / 256;
     const long long tiles = (long long)(s.Mp / kBlockM) * (s.Np / s.bn);
-    return (mode == MODE_FLEX16 ? 17500 : 11500) + prepass + (tiles + 147) / 148 * (3500 + num_kb * kb);
+    return (mode == MODE_FLEX16 ? 20000 : 13000) + prepass + (tiles + 147) / 148 * (3500 + num_kb * kb);
 }
 
 // Whether a product takes the kernel that converts its operands on the way in (one launch), and its
@@ -55,7 +56,15 @@ inline bool gemm_goes_direct(int mode, const void* A, long long a_rs, long long 
     const long long plane = plane_cost(mode, shapes_for(mode, M, N, K), M, N, K);
     const bool swap = ct >= 0 && (cd < 0 || ct < cd);
     *out = swap ? t : d;
-    const long long best = swap ? ct : cd;
+    long long best = swap ? ct : cd;
+    // Both operands contiguous along their rows take longer than the direct kernel's own choice of a shape has to
+    // know: fp32 638 x 937 x 631 26 us against 20 on planes, 383 x 3300 x 1440 47 and 39 (two k-blocks or less
+    // don't: 1869 x 1337 x 46 20 and 26); flex16 an odd number of values apart, loaded one by one, 249 x 1831 x
+    // 3065 75 and 41, 745 x 913 x 1135 65 and 31.  (With one of the two along K: 236 x 339 x 3450 26 and 33.)
+    if (d.a_kind == B2_OPERAND_ROWS && d.b_kind == B2_OPERAND_ROWS) {
+        if (mode == MODE_F32X3) best += K > 64 ? best / 6 : 0;
+        else if (K > 128 && out->a_ks % 2 != 0) best += best / 2;
+    }
     return best >= 0 && best < plane;
 }
 
