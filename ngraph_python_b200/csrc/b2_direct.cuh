@@ -13,11 +13,11 @@
 //   fp32:   3xTF32, in chains of at most 16 k-blocks (the tensor core's fp32 sum truncates); longer K
 //           is cut into slices.  Matrix products add hi*hi, hi*lo and lo*hi into one sum (see ONE_CHAIN).
 //           Convolutions keep two: B's planes lie behind one another and make one operand of 2*BN rows,
-//           A_hi x [B_hi | B_lo] -> [hh | x], A_lo x B_hi -> x.  Where tiles of many pixels stretch a sum
-//           over more k-blocks, between the zeros of their filters (staged ones), even and odd k-blocks have
-//           a pair each: against 64 bits, 22-layer networks' shapes at batch 1 to 1000, no error is larger
-//           than with one pair and filters as they lie, most are half (16 channels at 32x32 5.0e-7 -> 2.9e-7
-//           of the result's root mean square), for one percent of the time.
+//           A_hi x [B_hi | B_lo] -> [hh | x], A_lo x B_hi -> x.  The sum in tensor memory loses
+//           bits with every k-block, so the k-blocks go by turns to two pairs, or four where tensor memory has room,
+//           which are added to nearest at the end: against 64 bits, the shapes of the 22-layer networks at
+//           batch 1 to 1000, most errors are half of what they are with one pair (16 channels at 32x32,
+//           batch 100, 5.0e-7 -> 2.9e-7 of the result's root mean square), for one percent of the time.
 //   flex16: four exact int8 products, HH | X | LL as in b2_gemm_impl.cuh.
 // Slices of K: the CTAs of a cluster (up to 8) take one each; partial sums meet in distributed shared
 // memory, every CTA adds a share of the columns in slice order (deterministic, fp32 adds rounded to
@@ -49,8 +49,8 @@ __host__ __device__ constexpr int dir_stages(int bn, int groups = 1) {
 __host__ __device__ constexpr int dir_threads(int groups, bool staged = false) { return groups * 256 + (staged ? 64 : 32); }
 __host__ __device__ constexpr int dir_stage_bytes(int bn) { return 2 * (128 + bn) * 128; }
 __host__ __device__ constexpr int dir_ring_bytes(int bn, int groups = 1) { return dir_stages(bn, groups) * dir_stage_bytes(bn); }
-__host__ __device__ constexpr int dir_tmem_cols(int mode, int bn, bool staged = false) {
-    int need = (mode == MODE_FLEX16 ? 3 : staged ? 4 : 2) * bn, c = 32;
+__host__ __device__ constexpr int dir_tmem_cols(int mode, int bn, int pairs = 1) {
+    int need = (mode == MODE_FLEX16 ? 3 : 2 * pairs) * bn, c = 32;
     while (c < need) c *= 2;
     return c;
 }
@@ -194,7 +194,8 @@ direct_kernel(const __grid_constant__ DirectParams p) {
     constexpr int NST = dir_stages(BN, G), STAGE = dir_stage_bytes(BN), MMA_WARP = 8 * G;
     constexpr int KB = MODE == MODE_FLEX16 ? 128 : 32;            // columns of a k-block
     constexpr int PER = KB / 8;                                   // columns of a 16-byte chunk
-    constexpr int kCols = dir_tmem_cols(MODE, BN, STAGED);
+    constexpr int PAIRS = MODE == MODE_F32X3 && AK == B2_OPERAND_GATHER ? (BN <= 32 || (BN == 64 && G > 1) ? 4 : 2) : 1;
+    constexpr int kCols = dir_tmem_cols(MODE, BN, PAIRS);
     // fp32 matrix products: one accumulator, the three products of a k-step in the order of the plane
     // kernels, slices of whole chains -- the same rounding whichever kernel a size takes (a mask `x > 0`
     // of a value near zero would otherwise change with the dispatch)
@@ -491,11 +492,11 @@ direct_kernel(const __grid_constant__ DirectParams p) {
             const unsigned long long dA0 = make_smem_desc(st), dA1 = make_smem_desc(st + 128 * 128);
             const unsigned long long dB0 = make_smem_desc(st + 2 * 128 * 128);
             const unsigned long long dB1 = make_smem_desc(st + 2 * 128 * 128 + BN * 128);
-            const unsigned sums = tmem_base + (STAGED && (kb & 1) ? 2 * BN : 0);
+            const unsigned sums = tmem_base + kb % PAIRS * 2 * BN;
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
                 const unsigned long long adv = (unsigned long long)(2 * k);
-                const unsigned acc = (kb > (STAGED ? 1 : 0) || k > 0) ? 1u : 0u;
+                const unsigned acc = (kb >= PAIRS || k > 0) ? 1u : 0u;
                 if (MODE == MODE_FLEX16) {
                     tc_mma<MODE>(tmem_base, dA0 + adv, dB0 + adv, id_ss, acc);               // HH
                     tc_mma<MODE>(tmem_base + BN, dA0 + adv, dB1 + adv, id_su, acc);          // X += ah*bl
@@ -640,19 +641,21 @@ direct_kernel(const __grid_constant__ DirectParams p) {
                 for (int j = 0; j < 8; ++j)
                     v[j] = (Sum)(((long long)(int)hh[j] << 16) + ((long long)(int)xx[j] << 8) + (long long)(int)ll[j]);
             } else {
-                unsigned hh[8], xx[8], h1[8], x1[8];
+                unsigned hh[8], xx[8];
                 tmem_ld8(lane_addr + c0, hh);
                 if (!ONE_CHAIN) tmem_ld8(lane_addr + BN + c0, xx);
-                if (STAGED && nkb > 1) {
-                    tmem_ld8(lane_addr + 2 * BN + c0, h1);
-                    tmem_ld8(lane_addr + 3 * BN + c0, x1);
-                }
                 tmem_ld_wait();
-                if (STAGED && nkb > 1) {
+#pragma unroll
+                for (int q = 1; q < PAIRS; ++q) {
+                    if (q >= nkb) break;
+                    unsigned h[8], x[8];
+                    tmem_ld8(lane_addr + q * 2 * BN + c0, h);
+                    tmem_ld8(lane_addr + q * 2 * BN + BN + c0, x);
+                    tmem_ld_wait();
 #pragma unroll
                     for (int j = 0; j < 8; ++j) {
-                        hh[j] = __float_as_uint(__uint_as_float(hh[j]) + __uint_as_float(h1[j]));
-                        xx[j] = __float_as_uint(__uint_as_float(xx[j]) + __uint_as_float(x1[j]));
+                        hh[j] = __float_as_uint(__uint_as_float(hh[j]) + __uint_as_float(h[j]));
+                        xx[j] = __float_as_uint(__uint_as_float(xx[j]) + __uint_as_float(x[j]));
                     }
                 }
 #pragma unroll
