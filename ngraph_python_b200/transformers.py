@@ -1318,13 +1318,16 @@ class _Planner(object):
 
     THROUGH_LEAST = 1 << 20         # bytes
 
-    def _takes_argument(self, view, strides, dims):
-        """Whether an elementwise kernel over dims = (A, B, C) may read this view from where the
-        caller's tensor lies: a large argument that nothing has read yet or writes, every value of it
-        exactly once (flex16: and that no convolution reads as byte planes)."""
+    def _takes_argument(self, view, strides, dims, in_views):
+        """Whether an elementwise kernel over dims = (A, B, C) that reads in_views may read this one of
+        them from where the caller's tensor lies: a large argument that nothing has read yet or writes,
+        every value of it exactly once (flex16: and that no convolution reads as byte planes).  Read
+        through a second view, the argument's own memory would be read by some blocks while others store
+        what they have read there."""
         buf = view.buffer
         A, B, C = dims
-        return (buf.plane_bytes == 0 and buf.last_write_step < 0 and
+        return (sum(v.buffer is buf for v in in_views) == 1 and
+                buf.plane_bytes == 0 and buf.last_write_step < 0 and
                 buf in self.parameter_buffers and buf not in self.read_so_far and
                 4 * buf.size >= self.THROUGH_LEAST and view.is_dense() and A * B * C == buf.size and
                 strides[2] == 1 and (B == 1 or strides[1] == C) and (A == 1 or strides[0] == B * C))
@@ -1562,16 +1565,16 @@ class _Planner(object):
         step.requant_deps = [dep.get(d["reg"], 0) & ~(1 << k if k < len(outs) else 0)
                              for k, d in enumerate(outs + reds)]
         step.stores_argument = []
+        for pre in pre_steps:               # (copies that run in front of the kernel)
+            self.read_so_far.update(v.buffer for v in pre.in_views)
         for i, (v, st) in enumerate(zip(in_views, abc[:n_in])):
             # in a recorded call the first reader of a large argument reads it from wherever the
             # caller has it and stores it on the way: a copy in front of the kernel reads it once more
             # (8192 x 16384 values, fp32: 173 us of a call of 640; flex16: 120 of 444)
-            if self._takes_argument(v, st, dims) and \
+            if self._takes_argument(v, st, dims, in_views) and \
                     len(outs) + len(reds) + len(step.stores_argument) < fusion.MAX_OUT:
                 step.stores_argument.append(i)
         self.read_so_far.update(v.buffer for v in in_views)
-        for pre in pre_steps:
-            self.read_so_far.update(v.buffer for v in pre.in_views)
         prog = lib.make_program(dims, inputs, consts, ops, outs, reds, mode)
         if step.stores_argument:
             at = [dict(d, dtype=lib.FLEX16_AT if d["dtype"] == lib.FLEX16 else lib.F32_AT)
