@@ -40,6 +40,11 @@ class _Step(object):
         self.in_views = []
 
     def output_buffers(self):
+        """The tensors whose exponents this step manages."""
+        return [v.buffer for v in self.out_views]
+
+    def writes(self):
+        """Every tensor whose memory this step changes, with an exponent of its own or not."""
         return [v.buffer for v in self.out_views]
 
     def _ptr(self, v):
@@ -1014,6 +1019,9 @@ class CommStep(_Step):
 
     def output_buffers(self):
         return []
+
+    def writes(self):
+        return [self.arena_buffer]
 
     def launch(self, t):
         if self.src_view is not None:

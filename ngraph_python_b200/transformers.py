@@ -140,6 +140,10 @@ class EwStep(object):
     def output_buffers(self):
         return [v.buffer for v in self.out_views]
 
+    def writes(self):
+        """Every tensor whose memory the kernel changes, arguments that it stores included."""
+        return [v.buffer for v in self.out_views] + [v.buffer for v, _ in self.recorded_targets]
+
     @property
     def launches(self):
         return 0 if self.led else self.kernel.launches
@@ -1603,10 +1607,9 @@ def _join_launches(steps):
     leaders = {}          # source -> (leader, buffers read and written by the steps since)
     for s in steps:
         reads = set(v.buffer for v in s.in_views)
-        writes = set(s.output_buffers())
+        writes = set(s.writes())
         source = b""
         if s.kind == "ew":
-            writes.update(v.buffer for v, _ in s.recorded_targets)
             # (one that stores arguments has a launch of its own: recorded, it is another program)
             if not s.stores_argument and all(v.offset == 0 for v in s.in_views) and \
                     all(v.offset == 0 for v, _ in s.out_targets):
