@@ -2357,6 +2357,11 @@ class B200Transformer(object):
             for b in comp.written:
                 b.entry.end_write(int(stats[b.slot_write]))
             settled = fm.settled(ids)
+        # Tensors written in place are read by other computations through the row that held their
+        # exponent before the call.
+        for b in comp.written:
+            if b.slot != b.slot_write and not getattr(b, "shares_entry", False):
+                self._set_table_row_host(b.slot, b.entry.dec)
         comp._steady = (self._flex_epoch, slots, stats[slots].tobytes(), len(inputs)) if settled else None
 
     # ---- launching -------------------------------------------------------------------------------
