@@ -82,7 +82,7 @@ class _PlaneUser(object):
     tiles = False
     plane_args = ()                 # indexes of the tensors read as planes in op.args / in_views
     splits = ()                     # those that this step splits unless their producer has
-    filters_change = False          # the computation writes the filters, or takes them as an argument
+    filters_change = False          # the computation makes the filters, or takes them as an argument
     planes_built_first = False      # the first of the convolutions builds the filter planes of all
     joint_planes = None             # ... this one: the steps whose planes it builds
     filter_planes = None
@@ -260,16 +260,18 @@ class _PlaneUser(object):
 
 def join_filter_planes(steps, arguments):
     """Which convolutions of a computation make their filter planes in every call: those whose filters it
-    writes or receives (`arguments`).  The filter planes of the convolutions whose filters this computation writes after reading
-    them (a training step): the first of them builds all, one launch per 32 layers."""
+    writes, computes or copies itself, or receives (`arguments`).  The filter planes of the convolutions
+    whose filters this computation writes after reading them (a training step): the first of them builds
+    all, one launch per 32 layers."""
+    made = set(b for s in steps for b in s.writes())
     written, mine = set(), []
     for s in steps:
         if getattr(s, "filter_arg", None) is not None:
             buf = s.in_views[s.filter_arg].buffer
-            s.filters_change = buf.last_write_step >= 0 or buf in arguments
+            s.filters_change = buf in made or buf in arguments
             if buf.last_write_step >= 0 and buf not in written:
                 mine.append(s)
-        written.update(s.output_buffers())
+        written.update(s.writes())
     for s in mine:
         s.planes_built_first = True
     if mine:

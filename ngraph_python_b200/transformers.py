@@ -215,6 +215,7 @@ class Computation(object):
                 s.allocate(t)
         self.launches_per_call = builtin_sum(s.launches for s in self.steps)
         self.written = planner.written_buffers
+        self.touched = list(dict.fromkeys(b for s in self.steps for b in s.writes()))
         self.executor = self._run_steps
 
     # ---- run -----------------------------------------------------------------------------
@@ -2317,7 +2318,7 @@ class B200Transformer(object):
         watched = getattr(comp, "_watched", None)
         if watched is None:
             # (the tensors whose changes somebody follows: convolution filters with cached planes)
-            watched = comp._watched = [b for b in comp.written if getattr(b, "watched", False)]
+            watched = comp._watched = [b for b in comp.touched if getattr(b, "watched", False)]
             self._status_np = self._status_host.numpy()
         for b in watched:
             b.version += 1
