@@ -99,7 +99,7 @@ class _PlaneUser(object):
         self.conv_pass = conv_pass
         self.filter_arg = filter_arg
         self.filter_bytes = filt_bytes
-        self.in_views[filter_arg].buffer.watched = True
+        self.in_views[filter_arg].buffer.watched = True     # (what is kept follows its version)
         if self.flex:
             self.use_planes = True
             self._read_planes((stream_arg,))
@@ -301,6 +301,13 @@ class ConvChainStep(_Step):
         self.planes = None
         self.filters = [s.in_views[s.filter_arg].buffer for s in members]
         self.versions = None
+        # what a reader of unstored results has to know: tensors made by the run and before it, the rows of
+        # the scale table that stand for them, and the state of all that at the end of the last call
+        self.results = [s.out_views[0].buffer for s in members]
+        self.reads = [b for b in dict.fromkeys(v.buffer for v in self.in_views) if b not in self.results]
+        self.rows = sorted(set(r for b in self.reads + self.results for r in (b.slot, b.slot_write)))
+        self.open = False            # the last call's results are not all stored
+        self.clock = self.epoch = self.exponents = None
 
     def kept_planes(self):
         return True
@@ -344,10 +351,33 @@ class ConvChainStep(_Step):
             t.stream.cuda_stream))
         t.kernel_launches += 1
 
-    def store_results(self, t):
-        """Results that recorded calls do not store, for a reader from outside any call."""
+    def called(self, t):
+        """A recorded call has ended."""
+        self.open, self.clock = True, t._clock
+        if self.epoch != t._flex_epoch:
+            self.epoch, self.exponents = t._flex_epoch, t._dec_uploaded[self.rows]
+
+    def store_result(self, t, buf):
+        """For a reader from outside any call: `buf` as the last call made it, if that was a call of this
+        run which did not store it."""
+        if not self.open or buf not in self.unstored or buf.version > self.clock:
+            return
+        changed = [b.name for b in self.reads if b.version > self.clock]
+        if changed or (t._dec_uploaded[self.rows] != self.exponents).any():
+            raise lib.B200Error(
+                "the recorded call did not store %s, and %s changed since: read it before that, return it from "
+                "the computation, or take its device_tensor before capture()"
+                % (buf.name, ", ".join(changed) + (" have" if len(changed) > 1 else " has") if changed else
+                   "the exponents of the tensors that it follows from have"))
+        # the layers one by one write all their results: those that are stored, or that somebody else has
+        # written since, stay as they are
+        others = [b for b in self.results if b not in self.unstored or b.version > self.clock]
+        saved = [(b, b.tensor.clone()) for b in others]
         for s in self.members:
             s.launch(t)
+        for b, values in saved:
+            b.tensor.copy_(values)
+        self.open = False
         t._stats_clean = False           # (their statistics belong to the call that has been)
 
 
@@ -355,8 +385,9 @@ def chain_convolutions(steps, returned, t):
     """The step list with every run of convolution layers that fits one launch (b2_conv_chain_info)
     replaced by a ConvChainStep.  A run is made of neighbouring steps; what they stream comes from the
     run or, for its first layer's input, from int16 or byte planes that are complete before it; their
-    filters do not change inside the computation; and no step outside reads one of their results as byte
-    planes.  `returned`: buffers whose contents the computation returns."""
+    filters do not change inside the computation, nor does anything else that they read behind them; and no
+    step outside reads one of their results as byte planes.  `returned`: buffers whose contents are wanted
+    after a call."""
     if not t.flex:
         return list(steps)
 
@@ -389,6 +420,9 @@ def chain_convolutions(steps, returned, t):
         pool = after if isinstance(after, PoolStep) and after.averages_images() and \
             after.in_views[0].buffer is run[-1].out_views[0].buffer else None
         mine.add(pool)
+        behind = set(b for s in steps[steps.index(run[-1]) + 1:] for b in s.writes())
+        if any(v.buffer in behind for s in run for v in s.in_views):
+            return None                      # (results that are not stored could not be made again)
         kept = set(b for b in made if b in returned)
         for s in steps:
             if s in mine:

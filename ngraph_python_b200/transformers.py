@@ -60,7 +60,11 @@ class Buffer(object):
         self.planes = None          # torch uint8 allocation holding both planes
         self.planes_ptr = 0         # 1024-byte aligned start of the high plane
         self.planes_by_producer = False   # the kernel that writes the tensor writes the planes
-        self.version = 0            # bumped whenever the contents change
+        # Moves whenever the contents change, to the transformer's clock of then (in calls of computations:
+        # of arguments, and of tensors that are `watched`).
+        self.version = 0
+        self.held = False           # somebody has asked for a DeviceTensor of it
+        self.watched = False        # some step keeps what follows from the contents
         # planning state (per computation build)
         self.where = None           # device word: address of the values in a recorded call
         self.last_write_step = -1
@@ -176,6 +180,8 @@ class Computation(object):
         self.launches_per_call = 0
         self._io = None             # argument and result handling of the recorded step list
         self.chains = []            # runs of convolutions that recorded calls make in one launch
+        self._replayed = ()         # runs of layers that this call has launched
+        self._watched = None        # what calls write of the tensors that somebody follows
         self._comm_steps = []       # this computation's exchanges, in production order
         self._allreduce = None      # their arena and bucket plan (one per computation)
 
@@ -298,11 +304,20 @@ class Computation(object):
         if t.flex and any(not b.entry.initialized for b in self.written):
             raise lib.B200Error("run the computation once before capturing it")
         torch = t.torch
-        steps = kernels.chain_convolutions(self.steps, set(v.buffer for v in self.return_views), t)
+        # (results that somebody holds a tensor of are stored like those that are returned)
+        asked = set(b for b in t._buffers.values() if b.held)
+        steps = kernels.chain_convolutions(self.steps, asked.union(v.buffer for v in self.return_views), t)
         refreshable = [s for s in steps if hasattr(s, "refresh") and s.kept_planes()]
-        self.chains = [s for s in steps if s.kind == "conv_chain"]
-        for s in self.chains:
+        # (of an earlier recording: what it left unstored can still be made)
+        t._chains = [c for c in t._chains if c not in self.chains or c.open]
+        self.chains = chains = [s for s in steps if s.kind == "conv_chain"]
+        t._chains.extend(chains)
+        for s in chains:
             s.refresh(t)
+            for b in s.reads + s.results:
+                b.watched = True
+        for c in t.computations if chains else ():
+            c._watched = None
         ar = self._allreduce
         has_comm = any(s.kind == "comm" for s in self.steps) and ar is not None and ar.comm.size > 1
         in_graph = has_comm and getattr(ar.comm, "capturable", False)
@@ -397,6 +412,7 @@ class Computation(object):
             if in_graph:
                 ar.graph_launched(t.stream)
             t.kernel_launches += per_call
+            self._replayed = chains
             if io_in_graph:
                 t._io_done = True
                 t._stats_clean = t.flex
@@ -533,7 +549,7 @@ class _CallIO(object):
         keep = []
         try:
             for (k, buf, arg, read_in_place), value in zip(self.args, args):
-                buf.version += 1
+                t._changed(buf)
                 address, obj = self._source(k, value)
                 arg.src = address
                 # a device tensor is read where it lies by the kernel that uses it first, which
@@ -1716,6 +1732,7 @@ class B200Transformer(object):
     transformer_name = "b200"
     default_rtol = 1e-05
     default_atol = 1e-08
+    _clock = 0                      # moves with every change of a tensor that somebody may follow
 
     def __init__(self, device_id=0, flex=False, fixed_point=False, flex_verbose=False,
                  plan_only=False, fuse=True, **kwargs):
@@ -1751,6 +1768,7 @@ class B200Transformer(object):
         self._io_done = False       # the replayed graph has already queued the call's read-back
         self._stats_clean = False   # ... and left the statistics array cleared
         self._flex_epoch = 0        # moves whenever any exponent bookkeeping may have changed
+        self._chains = []           # runs of layers whose results may be asked for
         self._buffers = collections.OrderedDict()   # op -> Buffer
         self._views = {}
         self.finalized = False
@@ -1979,13 +1997,18 @@ class B200Transformer(object):
                                              dtype=self.torch.uint8, device=self.device)
 
     # ---- host <-> device -----------------------------------------------------------------------
+    def _changed(self, buf):
+        """The contents of `buf` are about to be something else, or are it already."""
+        self._clock += 1
+        buf.version = self._clock
+
     def _stage(self, view, value):
         """The copy half of a host write: the fp32 values go to the device (for a flex16 tensor
         into its staging buffer).  Depends on nothing else of a call, so a computation starts
         these copies before its exponent bookkeeping."""
         torch = self.torch
         buf = view.buffer
-        buf.version += 1
+        self._changed(buf)
         if not view.is_dense():
             raise ValueError("host writes need a dense tensor")
         if isinstance(value, torch.Tensor) and value.is_cuda:
@@ -2150,6 +2173,7 @@ class B200Transformer(object):
         v = self._view_of(as_op(op))
         if v.buffer.tensor is None:
             raise ValueError("no computation of this transformer uses %r" % (op,))
+        v.buffer.held = True
         return DeviceTensor(self, v)
 
     def get_tensor_view_value(self, op, host_tensor=None):
@@ -2204,7 +2228,7 @@ class B200Transformer(object):
                            src_strides, list(view.strides), self.stream.cuda_stream)
             self.kernel_launches += 1
         self.stream.synchronize()
-        buf.version += 1
+        self._changed(buf)
 
     # ---- flex bookkeeping ------------------------------------------------------------------------
     def _set_table_row(self, slot, dec):
@@ -2315,13 +2339,19 @@ class B200Transformer(object):
         lib.check(lib.raw().b2_call_wait(device, torch._C._cuda_getCurrentRawStream(device)))
         if exchanging:
             self._allreduce.after_sync()
-        watched = getattr(comp, "_watched", None)
+        watched = comp._watched
         if watched is None:
-            # (the tensors whose changes somebody follows: convolution filters with cached planes)
-            watched = comp._watched = [b for b in comp.touched if getattr(b, "watched", False)]
+            # (the tensors whose changes somebody follows: convolution filters with cached planes, tensors
+            # of runs of layers)
+            watched = comp._watched = [b for b in comp.touched if b.watched]
             self._status_np = self._status_host.numpy()
-        for b in watched:
-            b.version += 1
+        if watched:
+            self._clock += 1
+            for b in watched:
+                b.version = self._clock
+        for c in comp._replayed:
+            c.called(self)
+        comp._replayed = ()
         if self._status_np[0] != 0:
             self._status.zero_()
             raise lib.B200Error("a device-side wait ran out during the computation")
@@ -2450,6 +2480,11 @@ class DeviceTensor(object):
         w.get()                      # numpy copy of the whole tensor
         w[2:5, :, 0].get()           # a window: slices and integers per axis, Ellipsis
         w[...] = array               # whole tensor; w[1:3] = 0.5 fills a window
+
+    Recorded calls (Computation.capture) of flex16 convolutions do not store results that only a run of
+    layers reads.  They are made when they are read here, from what the call had: once an argument, a
+    filter or an exponent of the run has changed that is an error.  A tensor that was asked for before
+    capture() is stored by every call.
     """
 
     def __init__(self, transformer, view):
@@ -2466,10 +2501,7 @@ class DeviceTensor(object):
         return e.scale if e is not None else 1.0
 
     def get(self, tensor=None):
-        for comp in self.transformer.computations:
-            for chain in comp.chains:
-                if self.view.buffer in chain.unstored:
-                    chain.store_results(self.transformer)
+        self._store()
         host = self.transformer._device_to_host(self.view)
         if tensor is None:
             return host
@@ -2512,7 +2544,15 @@ class DeviceTensor(object):
         return DeviceTensor(self.transformer, View(v.buffer, axes, strides, offset))
 
     def __setitem__(self, key, value):
-        self.transformer._write_view(self.__getitem__(key).view, value)
+        window = self.__getitem__(key)
+        if not window.view.is_dense():
+            window._store()              # (the rest of the tensor stays as it is)
+        self.transformer._write_view(window.view, value)
+
+    def _store(self):
+        """A result inside a run of layers that its last call did not store is made now."""
+        for chain in self.transformer._chains:
+            chain.store_result(self.transformer, self.view.buffer)
 
 
 # ---------------------------------------------------------------------------------------------
