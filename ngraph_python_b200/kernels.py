@@ -111,6 +111,7 @@ class _PlaneUser(object):
         for k in args:
             buf = self.in_views[k].buffer
             buf.plane_bytes = lib.plane_bytes(self.in_views[k].axes.lengths)
+            buf.plane_images = self.in_views[k].axes.lengths[-1]
             # (planes whose rows of images are padded are written by the convolutions only)
             buf.plane_dense = self.dims.N % 16 == 0
             buf.plane_steps = getattr(buf, "plane_steps", []) + [self]
@@ -292,9 +293,9 @@ class ConvChainStep(_Step):
         self.members, self.layers, self.nbytes = members, layers, nbytes
         self.in_views = [v for s in members for v in s.in_views]
         self.out_views = [v for s in members for v in s.out_views]
-        # results that only the run itself reads are not stored by it (int16 tensors that the members
-        # store when they run one by one)
-        self.unstored = set(s.out_views[0].buffer for s in members if s.write_int16) - kept
+        # results that only the run itself reads are not stored by it (as int16 tensors or byte planes,
+        # which the members store when they run one by one)
+        self.unstored = set(s.out_views[0].buffer for s in members) - kept
         self.kept, self.pool = kept, pool
         if pool is not None:
             self.out_views += pool.out_views
@@ -354,6 +355,8 @@ class ConvChainStep(_Step):
     def called(self, t):
         """A recorded call has ended."""
         self.open, self.clock = True, t._clock
+        for b in self.kept:
+            b.int16_at = b.version
         if self.epoch != t._flex_epoch:
             self.epoch, self.exponents = t._flex_epoch, t._dec_uploaded[self.rows]
 
@@ -372,6 +375,8 @@ class ConvChainStep(_Step):
         # the layers one by one write all their results: those that are stored, or that somebody else has
         # written since, stay as they are
         others = [b for b in self.results if b not in self.unstored or b.version > self.clock]
+        for b in others:
+            b.join_planes()
         saved = [(b, b.tensor.clone()) for b in others]
         for s in self.members:
             s.launch(t)

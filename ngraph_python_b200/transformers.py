@@ -59,7 +59,10 @@ class Buffer(object):
         self.plane_bytes = 0        # bytes of one plane (0: no planes wanted)
         self.planes = None          # torch uint8 allocation holding both planes
         self.planes_ptr = 0         # 1024-byte aligned start of the high plane
+        self.plane_images = 0       # images to a row of a plane, padded to 16
         self.planes_by_producer = False   # the kernel that writes the tensor writes the planes
+        self.bytes_only = False     # some computation writes the planes and not the int16 tensor
+        self.int16_at = 0           # `version` that the int16 tensor holds (where bytes_only)
         # Moves whenever the contents change, to the transformer's clock of then (in calls of computations:
         # of arguments, and of tensors that are `watched`).
         self.version = 0
@@ -72,6 +75,20 @@ class Buffer(object):
 
     def ptr(self):
         return self.tensor.data_ptr()
+
+    def join_planes(self):
+        """Brings the int16 tensor up to date where only the planes are (queued on the current stream)."""
+        if not self.bytes_only or self.int16_at >= self.version:
+            return
+        row = (self.plane_images + 15) // 16 * 16
+        rows = self.size // self.plane_images
+        start = self.planes_ptr - self.planes.data_ptr()
+        high, low = [self.planes[at:at + rows * row].view(rows, row)[:, :self.plane_images]
+                     for at in (start, start + self.plane_bytes)]
+        tensor = self.tensor.view(rows, self.plane_images)
+        tensor.copy_(high)
+        tensor.mul_(256).add_(low)          # (a high byte of 128 or more wraps to its negative value)
+        self.int16_at = self.version
 
 
 class View(object):
@@ -182,6 +199,8 @@ class Computation(object):
         self.chains = []            # runs of convolutions that recorded calls make in one launch
         self._replayed = ()         # runs of layers that this call has launched
         self._watched = None        # what calls write of the tensors that somebody follows
+        self._int16 = []            # those of them that other computations may write as byte planes alone
+        self.bytes_only = set()     # what this one writes as byte planes alone
         self._comm_steps = []       # this computation's exchanges, in production order
         self._allreduce = None      # their arena and bucket plan (one per computation)
 
@@ -1335,7 +1354,14 @@ class _Planner(object):
             if buf.plane_bytes > 0:
                 buf.planes_by_producer = True
                 step.write_int16 = not self._only_plane_readers(step.out_op)
+                if not step.write_int16:
+                    self._planes_alone(buf)
         return [step]
+
+    def _planes_alone(self, buf):
+        """This computation writes the byte planes of `buf` and not the int16 tensor."""
+        buf.bytes_only = buf.watched = True
+        self.comp.bytes_only.add(buf)
 
     THROUGH_LEAST = 1 << 20         # bytes
 
@@ -1568,7 +1594,9 @@ class _Planner(object):
                     outs.append(pd)
                     out_targets.append((v, True))
                     buf.planes_by_producer = True
-                if not (wants and self._only_plane_readers(m)):
+                if wants and self._only_plane_readers(m):
+                    self._planes_alone(buf)
+                else:
                     result_index[m] = len(outs)
                     outs.append(d)
                     out_targets.append((v, False))
@@ -2000,7 +2028,7 @@ class B200Transformer(object):
     def _changed(self, buf):
         """The contents of `buf` are about to be something else, or are it already."""
         self._clock += 1
-        buf.version = self._clock
+        buf.version = buf.int16_at = self._clock
 
     def _stage(self, view, value):
         """The copy half of a host write: the fp32 values go to the device (for a flex16 tensor
@@ -2344,11 +2372,14 @@ class B200Transformer(object):
             # (the tensors whose changes somebody follows: convolution filters with cached planes, tensors
             # of runs of layers)
             watched = comp._watched = [b for b in comp.touched if b.watched]
+            comp._int16 = [b for b in watched if b.bytes_only and b not in comp.bytes_only]
             self._status_np = self._status_host.numpy()
         if watched:
             self._clock += 1
             for b in watched:
                 b.version = self._clock
+            for b in comp._int16:
+                b.int16_at = self._clock
         for c in comp._replayed:
             c.called(self)
         comp._replayed = ()
@@ -2550,9 +2581,11 @@ class DeviceTensor(object):
         self.transformer._write_view(window.view, value)
 
     def _store(self):
-        """A result inside a run of layers that its last call did not store is made now."""
+        """What the last call has not stored as it is read here is made now: a result inside a run of layers,
+        an int16 tensor of which only convolutions read, as byte planes."""
         for chain in self.transformer._chains:
             chain.store_result(self.transformer, self.view.buffer)
+        self.view.buffer.join_planes()
 
 
 # ---------------------------------------------------------------------------------------------

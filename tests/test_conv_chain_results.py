@@ -96,7 +96,7 @@ def test_refused_once_something_has_changed(change):
         assert np.array_equal(net.get(k), steps.get(k))
     for n in (steps, net):
         n.infer(n.values(9, 0.5))
-    for k in (1, 2, 3, 5):                                   # and the next call has all its results
+    for k in (0, 1, 2, 3, 4, 5):                             # and the next call has all its results
         assert np.array_equal(net.get(k), steps.get(k)), k
 
 
@@ -106,14 +106,14 @@ def test_one_result_leaves_the_others():
     for n in (steps, net):                                   # (windows keep their tensor's exponent)
         n.t.device_tensor(n.mids[5])[:9] = 0.125
         n.t.device_tensor(n.mids[2])[3:5] = 0.25
-    for k in (1, 3, 2, 5, 1):
+    for k in (1, 3, 0, 2, 4, 5, 1):
         assert np.array_equal(net.get(k), steps.get(k)), k
 
 
 @pytest.mark.gpu
 def test_inner_results_then_returned_ones():
     steps, net = _pair()
-    for k in (1, 5, 2, 3):
+    for k in (1, 0, 5, 2, 3, 4):
         assert np.array_equal(net.get(k), steps.get(k)), k
     _write_filter(net)                                       # (all were made before)
     assert np.array_equal(net.get(1), steps.get(1))
