@@ -366,6 +366,11 @@ int b2_conv_filter_planes_many(const b2_conv_filter_job* jobs, int32_t n, int32_
  * make it for several convolutions (job.filters: fp32; planes on 128-byte boundaries), and the pass with the
  * tails of b2_conv_fprop_f32_fused and b2_conv_bprop_f32_fused. */
 int b2_conv_filter_tiles_info(const b2_conv_dims* d, int32_t pass, size_t* bytes);
+/* How an fp32 pass gathers its operands, with filters as they lie or laid out (tiles): pixels to a row of the
+ * product, columns to a tile, slices of K, its k-blocks of 32 columns and those that go into one sum; all zero
+ * where it does not. */
+typedef struct b2_conv_plan_info { int32_t tile_h, tile_w, tile_n, slices, blocks, in_one_sum; } b2_conv_plan_info;
+int b2_conv_f32_plan(const b2_conv_dims* d, int32_t pass, int32_t tiles, b2_conv_plan_info* plan);
 int b2_conv_filter_tiles(const b2_conv_filter_job* jobs, int32_t n, int32_t* launches, void* stream);
 int b2_conv_f32_tiles(int32_t pass, const float* X, const void* filter_tiles, float* O, const b2_conv_dims* d,
                       const float* bias, const float* residual, int32_t relu, const float* mask, int32_t* status,

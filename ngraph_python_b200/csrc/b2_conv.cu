@@ -142,32 +142,68 @@ inline bool direct_args(int mode, const ConvGeom& g, int pass, int gh, int gw, b
     return true;
 }
 
+// Cycles of the gather + GEMM path: the planes of the unrolled rows once out and once back (at 5 TB/s), then
+// the tile kernel.
+inline long long unrolled_cost(int mode, const ConvGeom& g, int pass) {
+    const long long rows = pass ? (long long)g.H * g.W * g.N : (long long)g.P * g.Q * g.N;
+    const long long k = (long long)(pass ? g.K : g.C) * g.R * g.S;
+    if (rows >= (1LL << 31) - 256) return 1LL << 62;
+    const Shapes s = shapes_for(mode, (int)rows, pass ? g.C : g.K, (int)k);
+    const long long planes = rows * s.Kp * s.esize * 4 / 2600;
+    const long long kb = (mode == MODE_FLEX16 ? 1430LL : 1100LL) * (128 + s.bn) / 256;
+    const long long tiles = (long long)(s.Mp / kBlockM) * (s.Np / s.bn);
+    return 13000 + planes + (tiles + 147) / 148 * (3500 + (long long)(s.Kp * s.esize / kKBytes) * kb);
+}
+
+// fp32: what a shape and tile of a pass may add up, whichever is taken: the k-blocks in one sum
+// (b2_direct_args::longest), and where one block holds all of K no more than that one (further sums are added to
+// nearest, which is nothing beside the blocks' loss but is something beside none: 16 -> 32 channels 1x1 at stride
+// 2, batch 384, in three blocks of a 1x3 tile 1.09e-7 of the result's root mean square against 64 bits, 1.00e-7 in
+// one).  An unrolled product adds chains of 16.
+struct SumBound {
+    int longest;
+    bool one_block;
+    bool allows(const b2_direct_args& d) const { return !one_block || d.K <= 32; }
+};
+
+inline SumBound sum_bound(int mode, const ConvGeom& g, int pass) {
+    if (mode != MODE_F32X3) return {0, false};                    // (exact)
+    long long best = -1;
+    SumBound bound = {0, false};
+    for (int a = 1; a <= 2; ++a)
+        for (int b = 1; b <= 2; ++b) {
+            b2_direct_args d;
+            int n = 0;
+            if (!direct_args(mode, g, pass, pass ? a * g.str_h : a, pass ? b * g.str_w : b, &d)) continue;
+            const long long cost = b2_direct_longest(d, &n);
+            if (cost < 0 || (best >= 0 && cost >= best)) continue;
+            best = cost;
+            bound = {n, d.K <= 32};
+        }
+    if (best >= 0 && best < unrolled_cost(mode, g, pass)) return bound;
+    const int blocks = ((pass ? g.K : g.C) * g.R * g.S + 31) / 32;
+    return {blocks < 16 ? blocks : 16, blocks == 1};
+}
+
 // Whether a pass goes that way, with the best tile.  It does what the gather + GEMM path does, with one
 // launch and without writing the unrolled planes (8 bytes for each of the R*S copies of a value, and
 // reading them again); the planes pay only where a long list of output channels would have the gather
 // repeated for every 128 of them.
 inline bool conv_goes_direct(int mode, const ConvGeom& g, int pass, b2_direct_args* out) {
     if (!flat_depth(g) || getenv("B2_CONV_IM2COL")) return false;
+    const SumBound bound = sum_bound(mode, g, pass);
     long long best = -1;
     for (int a = 1; a <= 2; ++a)
         for (int b = 1; b <= 2; ++b) {
             b2_direct_args d;
-            if (!direct_args(mode, g, pass, pass ? a * g.str_h : a, pass ? b * g.str_w : b, &d)) continue;
+            if (!direct_args(mode, g, pass, pass ? a * g.str_h : a, pass ? b * g.str_w : b, &d) || !bound.allows(d)) continue;
+            d.longest = bound.longest;
             const long long cost = b2_direct_cost(d);
             if (cost < 0 || (best >= 0 && cost >= best)) continue;
             best = cost;
             *out = d;
         }
-    if (best < 0) return false;
-    const long long rows = pass ? (long long)g.H * g.W * g.N : (long long)g.P * g.Q * g.N;
-    const long long k = (long long)(pass ? g.K : g.C) * g.R * g.S;
-    if (rows >= (1LL << 31) - 256) return true;
-    // the planes of the unrolled rows once out and once back (cycles at 5 TB/s), then the tile kernel
-    const Shapes s = shapes_for(mode, (int)rows, pass ? g.C : g.K, (int)k);
-    const long long planes = rows * s.Kp * s.esize * 4 / 2600;
-    const long long kb = (mode == MODE_FLEX16 ? 1430LL : 1100LL) * (128 + s.bn) / 256;
-    const long long tiles = (long long)(s.Mp / kBlockM) * (s.Np / s.bn);
-    return best < 13000 + planes + (tiles + 147) / 148 * (3500 + (long long)(s.Kp * s.esize / kKBytes) * kb);
+    return best >= 0 && best < unrolled_cost(mode, g, pass);
 }
 
 // The same with the filters' rows made beforehand (b2_direct_stage_filters), for fp32 convolutions that go
@@ -178,10 +214,12 @@ inline bool conv_goes_staged(const ConvGeom& g, int pass, b2_direct_args* out) {
     b2_direct_args d;
     if (!conv_goes_direct(MODE_F32X3, g, pass, &d)) return false;
     long long best = b2_direct_cost(d);
+    const SumBound bound = sum_bound(MODE_F32X3, g, pass);
     bool found = false;
     for (int a = 1; a <= 4; ++a)
         for (int b = 1; b <= 4; ++b) {
-            if (!direct_args(MODE_F32X3, g, pass, pass ? a * g.str_h : a, pass ? b * g.str_w : b, &d)) continue;
+            if (!direct_args(MODE_F32X3, g, pass, pass ? a * g.str_h : a, pass ? b * g.str_w : b, &d) || !bound.allows(d)) continue;
+            d.longest = bound.longest;
             d.staged = &d;                        // (there will be such)
             const long long cost = b2_direct_cost(d);
             if (cost < 0 || cost >= best) continue;
@@ -2248,6 +2286,20 @@ extern "C" int b2_conv_fprop_f32_fused(const float* I, const float* F, float* O,
     B2_REQUIRE(conv_goes_direct(MODE_F32X3, g, 0, &direct), "this convolution takes no fused tail");
     direct.bias = bias; direct.residual = residual; direct.relu = relu ? 1 : 0;
     return launch_direct(direct, I, F, O, nullptr, 0, 0, 0, nullptr, nullptr, status, 0, (cudaStream_t)stream);
+}
+
+extern "C" int b2_conv_f32_plan(const b2_conv_dims* d, int32_t pass, int32_t tiles, b2_conv_plan_info* plan) {
+    ConvGeom g;
+    int rc = geom_from(d, &g);
+    if (rc) return rc;
+    B2_REQUIRE(plan && (pass == 0 || pass == 1), "bad argument");
+    *plan = {};
+    b2_direct_args a;
+    if (!(tiles ? conv_goes_staged(g, pass, &a) : conv_goes_direct(MODE_F32X3, g, pass, &a))) return B2_OK;
+    b2_gemm_plan_info p;
+    b2_direct_plan(a, &p);
+    *plan = {a.g.gh, a.g.gw, p.tile_n, p.slices, (a.K + 31) / 32, b2_direct_in_one_sum(a)};
+    return B2_OK;
 }
 
 extern "C" int b2_conv_filter_tiles_info(const b2_conv_dims* d, int32_t pass, size_t* bytes) {

@@ -3,14 +3,31 @@
 
 __attribute__((visibility("hidden"))) int b2_direct_launch_flex(const b2_direct_args& a, cudaStream_t st);
 
-long long b2_direct_cost(const b2_direct_args& a) {
+static bool within_range(const b2_direct_args& a) {
     if (a.a_kind == B2_OPERAND_GATHER) {
         const b2_gather& g = a.g;
         const long long elems = (long long)g.channels * g.H * g.W * g.N;
-        if (g.R * g.S > 31 || a.K > kDirMaxK || elems >= (1LL << 31)) return -1;
+        if (g.R * g.S > 31 || a.K > kDirMaxK || elems >= (1LL << 31)) return false;
     }
-    if ((long long)(a.M + 127) / 128 > 65535) return -1;           // grid.y
+    return (long long)(a.M + 127) / 128 <= 65535;                  // grid.y
+}
+
+long long b2_direct_cost(const b2_direct_args& a) {
+    if (!within_range(a)) return -1;
     return a.flex ? direct_shape<MODE_FLEX16>(a).cost : direct_shape<MODE_F32X3>(a).cost;
+}
+
+long long b2_direct_longest(const b2_direct_args& a, int* longest) {
+    if (!within_range(a)) return -1;
+    const DirectShape s = direct_shape<MODE_F32X3>(a, true);
+    *longest = s.kb_per_split;
+    return s.cost;
+}
+
+int b2_direct_in_one_sum(const b2_direct_args& a) {
+    const DirectShape s = direct_shape<MODE_F32X3>(a);
+    const int pairs = dir_pairs(s.bn, s.groups);
+    return (s.kb_per_split + pairs - 1) / pairs;
 }
 
 void b2_direct_plan(const b2_direct_args& a, b2_gemm_plan_info* plan) {

@@ -17,7 +17,10 @@
 //           bits with every k-block, so the k-blocks go by turns to two pairs, or four where tensor memory has room,
 //           which are added to nearest at the end: against 64 bits, the shapes of the 22-layer networks at
 //           batch 1 to 1000, most errors are half of what they are with one pair (16 channels at 32x32,
-//           batch 100, 5.0e-7 -> 2.9e-7 of the result's root mean square), for one percent of the time.
+//           batch 100, 5.0e-7 -> 2.9e-7 of the result's root mean square), for one percent of the time.  No shape may
+//           put more k-blocks into one sum than with one pair (b2_direct_args::longest): of 336 random layers and
+//           passes the errors against 64 bits are 0.70 of those with one pair (geometric mean), none larger by more than 3 %
+//           (of K of 75); without that bound 54 of 8010 shapes had longer sums and up to 1.3 times the error.
 //   flex16: four exact int8 products, HH | X | LL as in b2_gemm_impl.cuh.
 // Slices of K: the CTAs of a cluster (up to 8) take one each; partial sums meet in distributed shared
 // memory, every CTA adds a share of the columns in slice order (deterministic, fp32 adds rounded to
@@ -54,6 +57,9 @@ __host__ __device__ constexpr int dir_tmem_cols(int mode, int bn, int pairs = 1)
     while (c < need) c *= 2;
     return c;
 }
+
+// gathered fp32 rows: pairs of sums that the k-blocks go to by turns
+__host__ __device__ constexpr int dir_pairs(int bn, int groups) { return bn <= 32 || (bn == 64 && groups > 1) ? 4 : 2; }
 
 __host__ __device__ inline bool filter_tiles(const b2_direct_args& a) { return a.b_kind == B2_OPERAND_FILTER; }
 
@@ -194,7 +200,7 @@ direct_kernel(const __grid_constant__ DirectParams p) {
     constexpr int NST = dir_stages(BN, G), STAGE = dir_stage_bytes(BN), MMA_WARP = 8 * G;
     constexpr int KB = MODE == MODE_FLEX16 ? 128 : 32;            // columns of a k-block
     constexpr int PER = KB / 8;                                   // columns of a 16-byte chunk
-    constexpr int PAIRS = MODE == MODE_F32X3 && AK == B2_OPERAND_GATHER ? (BN <= 32 || (BN == 64 && G > 1) ? 4 : 2) : 1;
+    constexpr int PAIRS = MODE == MODE_F32X3 && AK == B2_OPERAND_GATHER ? dir_pairs(BN, G) : 1;
     constexpr int kCols = dir_tmem_cols(MODE, BN, PAIRS);
     // fp32 matrix products: one accumulator, the three products of a k-step in the order of the plane
     // kernels, slices of whole chains -- the same rounding whichever kernel a size takes (a mask `x > 0`
@@ -730,8 +736,10 @@ direct_kernel(const __grid_constant__ DirectParams p) {
 // ---- host ------------------------------------------------------------------------------------
 struct DirectShape { int bn, splits, kb_per_split, waves, groups; long long cost; };
 
+// `plain`: the shape of a kernel with one group of producers and one pair of sums, for what it adds up in
+// one go (see b2_direct_args::longest).
 template <int MODE>
-DirectShape direct_shape(const b2_direct_args& a) {
+DirectShape direct_shape(const b2_direct_args& a, bool plain = false) {
     const int KB = MODE == MODE_FLEX16 ? 128 : 32;
     const int num_kb = (a.K + KB - 1) / KB;
     // fp32: 16 k-blocks to a chain; flex16: exact int32 sums up to 32768 columns
@@ -774,15 +782,16 @@ DirectShape direct_shape(const b2_direct_args& a) {
             // takes 65 % (flex16) or 60 % of the cycles (fp32 512 x 128 x 512: 1470 -> 820).  With more CTAs than
             // SMs two of them on an SM do the same (flex16 1500 x 200 x 900 in 144 CTAs of two groups, clusters
             // of three, where 135 find an SM: 26.4 us, 22.5 with one group).  Tiles of 128 columns would spill.
-            const int groups = ctas <= kClusterCtas[splits] && per > 1 && bn < 128 &&
+            const int groups = !plain && ctas <= kClusterCtas[splits] && per > 1 && bn < 128 &&
                                1152 + dir_ring_bytes(bn, 2) + tab <= 232448 ? 2 : 1;
+            if (a.longest > 0 && !plain && (per + dir_pairs(bn, groups) - 1) / dir_pairs(bn, groups) > a.longest) continue;
             long long kb = together * pace > lat ? together * pace : lat;
             if (groups == 2) kb = kb * (MODE == MODE_FLEX16 ? 65 : 60) / 100;
             if (kb < together * copies) kb = together * copies;
             const long long slots = (long long)kClusterCtas[splits] * (groups == 2 ? 1 : per_sm);
             // (the exchange of slices: 700 and 500 a slice)
             const long long one = 7000 + per * kb + together * bn * (splits > 1 ? 24 : 12) +
-                                  (splits == 1 ? 0 : filter_tiles(a) && !a.staged ? 18000 : 700 + 500 * splits);
+                                  (splits == 1 ? 0 : filter_tiles(a) && !a.staged ? 18000 : plain ? 3000 : 700 + 500 * splits);
             const long long waves = (ctas + slots - 1) / slots, cost = waves * one;
             if (best.cost < 0 || cost < best.cost) best = {bn, splits, per, (int)waves, groups, cost};
         }

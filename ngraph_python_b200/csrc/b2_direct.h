@@ -29,6 +29,11 @@ struct b2_direct_args {
     const void *A, *B;
     // gathered fp32 rows: B's k-blocks as the kernel's stages hold them (b2_direct_stage_filters), or NULL
     const void* staged;
+    // Gathered fp32 rows: the most k-blocks that may go into one sum (0: any).  The tensor core's sum loses
+    // bits with every one, and a cheaper shape is not to lose more than callers of a layer have had: the bound
+    // is what the shape of one group of producers and one pair of sums, filters as they lie, adds up in one go
+    // (b2_direct_longest).
+    int longest;
     long long a_rs, a_ks, b_rs, b_ks;   // element strides: A[row * a_rs + k * a_ks]; rows of B are columns of C
     int M, N, K;
     b2_gather g;
@@ -54,6 +59,10 @@ constexpr int kClusterCtas[9] = {0, 148, 148, 135, 132, 130, 132, 105, 120};
 
 // Estimated cycles of a launch, negative where the kernel does not take the problem.
 __attribute__((visibility("hidden"))) long long b2_direct_cost(const b2_direct_args& a);
+// The same for one group of producers and one pair of sums, and the k-blocks that then go into one sum.
+__attribute__((visibility("hidden"))) long long b2_direct_longest(const b2_direct_args& a, int* longest);
+// ... that do so in the shape taken.
+__attribute__((visibility("hidden"))) int b2_direct_in_one_sum(const b2_direct_args& a);
 __attribute__((visibility("hidden"))) void b2_direct_plan(const b2_direct_args& a, b2_gemm_plan_info* plan);
 // `staged` operands: bytes, and the kernel that makes those of n products (fewest launches; `launches`
 // counts them).  Whether a product has its operand staged changes its shape, so `staged` is set (to

@@ -93,6 +93,10 @@ class GemmPlan(C.Structure):
     _fields_ = [(n, C.c_int32) for n in ("kernel", "tile_n", "slices", "waves")]
 
 
+class ConvPlan(C.Structure):
+    _fields_ = [(n, C.c_int32) for n in ("tile_h", "tile_w", "tile_n", "slices", "blocks", "in_one_sum")]
+
+
 GEMM_DIRECT, GEMM_PAIRS, GEMM_TILES = 0, 1, 2
 CALL_MAX_INPUTS, CALL_MAX_OUTPUTS = 16, 16
 
@@ -165,6 +169,7 @@ def _load():
         "b2_conv_split_activations": (C.c_int, [vp, C.POINTER(ConvDims), i32, vp, vp]),
         "b2_conv_filter_planes_many": (C.c_int, [C.POINTER(ConvFilterJob), i32, C.POINTER(i32), vp]),
         "b2_conv_split_planes": (C.c_int, [vp, i32, i32, i32, i32, vp, vp]),
+        "b2_conv_f32_plan": (C.c_int, [C.POINTER(ConvDims), i32, i32, C.POINTER(ConvPlan)]),
         "b2_conv_filter_tiles_info": (C.c_int, [C.POINTER(ConvDims), i32, C.POINTER(sz)]),
         "b2_conv_filter_tiles": (C.c_int, [C.POINTER(ConvFilterJob), i32, C.POINTER(i32), vp]),
         "b2_conv_f32_tiles": (C.c_int, [i32, vp, vp, vp, C.POINTER(ConvDims), vp, vp, i32, vp, vp, vp]),
@@ -450,6 +455,13 @@ def conv_planes_info(dims, conv_pass=CONV_FPROP):
     ok, a, f = C.c_int32(), C.c_size_t(), C.c_size_t()
     check(_lib.b2_conv_planes_info(C.byref(dims), conv_pass, C.byref(ok), C.byref(a), C.byref(f)))
     return bool(ok.value), a.value, f.value
+
+
+def conv_f32_plan(dims, conv_pass, tiles):
+    """ConvPlan of an fp32 pass, or None where it does not gather its operands (so)."""
+    p = ConvPlan()
+    check(_lib.b2_conv_f32_plan(C.byref(dims), conv_pass, int(tiles), C.byref(p)))
+    return p if p.tile_n else None
 
 
 def conv_filter_tiles_info(dims, conv_pass):
