@@ -210,6 +210,11 @@ inline bool conv_goes_direct(int mode, const ConvGeom& g, int pass, b2_direct_ar
 // direct: false where a launch would take no less time (what the kernel's cost rule says for both; a row of
 // filters costs its producers as much as a gathered one, or more).  With only the gathered rows to make, tiles
 // of six pixels pay: 16 channels at 32x32, batch 100, 12.8 us against 16.7 for four, as they lie 20.2.
+//
+// Infinities and NaN: a row of the product holds the whole window of its tile, and a value outside a pixel's own
+// taps meets zeros of that pixel's filters.  An infinity or NaN therefore makes every result of its image NaN that
+// stands in a tile whose window covers it: up to 2x2 pixels with filters as they lie, 4x4 here (times the stride in
+// an input gradient), beside those whose taps see it.  One-pixel tiles reach no further than the taps.
 inline bool conv_goes_staged(const ConvGeom& g, int pass, b2_direct_args* out) {
     b2_direct_args d;
     if (!conv_goes_direct(MODE_F32X3, g, pass, &d)) return false;
