@@ -60,20 +60,15 @@ C2_ROWS, C2_COLS = 8192, 16384
 FALLBACK_HBM_GBS = 6650.0
 FALLBACK_BF16_TFLOPS = 1590.0
 INT8_DATASHEET_TOPS = 4500.0
-# dram__bytes_read.sum + dram__bytes_write.sum per full-size launch, scaled from the ncu capture
-# of a quarter-size launch (2048 rows): see profiles/ew_c2_flex16.md and profiles/ew_c2_fp32.md
+# dram__bytes_read.sum + dram__bytes_write.sum per full-size launch, scaled from an ncu capture of a
+# quarter-size launch (2048 rows)
 NCU_TRAFFIC_BYTES = {"c2_flex16": 4 * (268457728 + 39549952), "c2_fp32": 4 * (536940544 + 107399680)}
-# the same two counters summed over the 22 convolution launches of one batch-256 flex16 pass
-# (profiles/conv_resnet20_flex16.md).  ncu flushes the caches before every launch it measures, so
-# this counts as DRAM reads what the real sequence finds in L2, and no write reaches DRAM within
-# its launch: an upper bound on the reads of the timed pass, not its traffic to the byte.
-NCU_CONV_TRAFFIC_BYTES = {"resnet20_flex16": 154123008}
+# the same counters of the one launch that holds the 22 convolutions of a flex16 pass of 256 images, caches
+# flushed in front of it: the images' byte planes, filters and biases; nothing that it writes leaves L2 meanwhile
+NCU_CONV_TRAFFIC_BYTES = {("resnet20_flex16", 256, 1): 2321408}
 
 RESNET_N = 256
-# algorithmic figures per 256-image batch: 21.03 GFLOP; minimal layer I/O of the 22 convolutions
-# (inputs 58 458 112 + outputs 55 574 528 + filters 270 512 elements)
-RESNET_FLOP_PER_IMG = 82.1e6
-RESNET_CONV_ELEMS_PER_256 = 58458112 + 55574528 + 270512
+RESNET_FLOP_PER_IMG = 82.1e6     # of the 22 convolutions
 TRAIN_PARAM_BYTES = 1084648      # fp32 gradients exchanged per step (no batch norm, no biases)
 REFERENCE_NETWORK = ("reference examples/resnet/resnet.py BuildResnet('cifar10', 20, False, 3, "
                      "batch_norm=False), built with the reference's ngraph")
@@ -181,6 +176,7 @@ class ClockSampler(object):
 class Timer(object):
     """CUDA-event timing of `repeats` loops of `steps` calls, barrier + synchronize on both sides
     of every loop, max over ranks per loop."""
+    FLUSH_BYTES = 256 << 20         # (L2: 126 MB)
 
     def __init__(self, torch, dist):
         self.torch, self.dist = torch, dist
@@ -191,6 +187,27 @@ class Timer(object):
         if self.dist is not None:
             self.dist.barrier()
         self.torch.cuda.synchronize()
+
+    def flushed(self, fn, steps, repeats, host=False):
+        """`loops` for work that fits in L2: a buffer larger than L2 is written in front of every call, and
+        the calls are timed one by one.  host: the call's own work on the host is part of it (the device
+        is idle when it starts)."""
+        torch = self.torch
+        buf = torch.empty((self.FLUSH_BYTES,), dtype=torch.uint8, device="cuda")
+        events = [[torch.cuda.Event(enable_timing=True) for _ in range(2)] for _ in range(steps)]
+        out = []
+        for _ in range(max(1, repeats)):
+            self.barrier()
+            for ev0, ev1 in events:
+                buf.zero_()
+                if host:
+                    torch.cuda.synchronize()
+                ev0.record(self.stream)
+                fn()
+                ev1.record(self.stream)
+            self.barrier()
+            out.append(sum(ev0.elapsed_time(ev1) for ev0, ev1 in events))
+        return self._slowest(out)
 
     def loops(self, fn, steps, repeats):
         torch = self.torch
@@ -204,8 +221,11 @@ class Timer(object):
             ev1.record(self.stream)
             self.barrier()
             out.append(ev0.elapsed_time(ev1))
+        return self._slowest(out)
+
+    def _slowest(self, out):
         if self.dist is not None:
-            tt = torch.tensor(out, dtype=torch.float64, device="cuda")
+            tt = self.torch.tensor(out, dtype=self.torch.float64, device="cuda")
             self.dist.all_reduce(tt, op=self.dist.ReduceOp.MAX)
             out = [float(v) for v in tt.tolist()]
         return out
@@ -482,6 +502,16 @@ def check_parity(got, want, flex):
     return report
 
 
+def conv_step_bytes(step):
+    """What a launch of a convolution step cannot do without: each tensor it reads and each one it stores,
+    once.  A run of layers keeps the activations between them in shared memory."""
+    if step.kind == "conv_chain":
+        bufs = step.reads + list(step.kept) + ([step.pool.out_views[0].buffer] if step.pool is not None else [])
+    else:
+        bufs = [v.buffer for v in step.in_views + step.out_views]
+    return sum(b.size * (2 if b.flex else 4) for b in bufs)
+
+
 def run_resnet(args, rank, world, torch, dist, local):
     flex = args.workload == "resnet20_flex16"
     n = args.batch
@@ -513,25 +543,27 @@ def run_resnet(args, rank, world, torch, dist, local):
     sampler = ClockSampler(local)
     timer.barrier()
     sampler.start()
-    loop_ms = timer.loops(step_resident, args.steps, args.repeats)
+    loop_ms = timer.flushed(step_resident, args.steps, args.repeats, host=True)
     sampler.keep_loaded(step_resident, torch.cuda.synchronize)
-    replay_ms = timer.loops(comp.executor, args.steps, args.repeats)
-    # the 22 convolution launches alone, back to back, as a CUDA graph of their own: every tensor
+    replay_ms = timer.flushed(comp.executor, args.steps, args.repeats)
+    # the convolution launches of a pass alone, back to back, as a CUDA graph of their own: every tensor
     # they read is still in place from the last pass
-    conv_steps = [s for s in comp.steps if s.kind == "conv"]
+    conv_steps = [s for s in (comp.recorded or comp.steps) if s.kind in ("conv", "conv_chain")]
+    conv_launches = sum(s.launches for s in conv_steps)
+    conv_bytes = sum(conv_step_bytes(s) for s in conv_steps)
 
     def convs_only():
         for s in conv_steps:
             t._launch_step(s)
-    conv_fn, conv_src = convs_only, "CUDA events around the 22 convolution steps launched one by one"
+    conv_fn, conv_src = convs_only, "CUDA events around the convolution launches of a pass, one by one"
     if not args.no_graph:
         torch.cuda.synchronize()
         g = torch.cuda.CUDAGraph()
         with torch.cuda.graph(g):
             convs_only()
         conv_fn = g.replay
-        conv_src = "CUDA events around a replayed graph of the 22 convolution steps alone"
-    conv_loops = timer.loops(conv_fn, args.steps, args.repeats)
+        conv_src = "CUDA events around a replayed graph of the convolution launches of a pass alone"
+    conv_loops = timer.flushed(conv_fn, args.steps, args.repeats)
     # end to end
     for _ in range(2):
         net.call(host)
@@ -544,20 +576,28 @@ def run_resnet(args, rank, world, torch, dist, local):
     ms_step = statistics.median(loop_ms) / args.steps
     replay_step = statistics.median(replay_ms) / args.steps
     conv_ms = statistics.median(conv_loops) / args.steps
-    peak, which = peaks()
     item = 2 if flex else 4
-    conv_bytes = RESNET_CONV_ELEMS_PER_256 * item * n / 256.0
-    conv_gbs = conv_bytes / (conv_ms * 1e-3) / 1e9
+    # the slower of what the launches move and what they multiply, at the measured rates
+    hbm, which = peaks()
+    bf16, _ = tensor_peak()
+    tensor = bf16 * 2 if flex else bf16 / 2
+    tensor_ops = RESNET_FLOP_PER_IMG * n * (4 if flex else 3)
+    if conv_bytes / (hbm * 1e9) >= tensor_ops / (tensor * 1e12):
+        bound, achieved, peak, unit = "hbm", conv_bytes / (conv_ms * 1e-3) / 1e9, hbm, "GB/s"
+    else:
+        bound, achieved, peak = "tensor", tensor_ops / (conv_ms * 1e-3) / 1e12, tensor
+        unit = "TOPS (int8)" if flex else "TFLOP/s (tf32)"
+        which += " bf16 x 2 as int8 stand-in" if flex else " bf16 / 2 as tf32 stand-in"
+    layers = sum(len(s.members) if s.kind == "conv_chain" else 1 for s in conv_steps)
     cfg = resnet_config(args.workload, n, world, net.frontend)
     cfg.update({"replicas": world,
                 "transformer": "ngraph.transformers.make_transformer_factory('b200') (plug-in)"
                                if net.graph is not None else "ngraph_python_b200.transformers",
-                "l2": "L2 flushed by the run itself: each pass streams >126 MB of activations and "
-                      "operand planes",
-                "steps_per_pass": len(comp.steps), "cuda_graph": not args.no_graph,
+                "l2": "flushed: %d MB written between passes, outside the timed intervals"
+                      % (Timer.FLUSH_BYTES >> 20),
+                "steps_per_pass": len(comp.recorded or comp.steps), "cuda_graph": not args.no_graph,
                 "value_includes": "per-call exponent bookkeeping, graph replay, statistics and "
                                   "status read-back with one stream synchronisation"})
-    traffic = NCU_CONV_TRAFFIC_BYTES.get(args.workload)
     line = {
         "metric": "ResNet-20 %s inference img/s" % ("flex16" if flex else "fp32"),
         "value": round(world * n / (ms_step * 1e-3), 1), "unit": "img/s", "n_gpus": world,
@@ -577,16 +617,15 @@ def run_resnet(args, rank, world, torch, dist, local):
                 "h2d_bytes_per_step": int(host.nbytes), "d2h_bytes_per_step": int(10 * n * item),
                 "steps": e2e_steps, "ms_per_step": round(e2e_ms / e2e_steps, 3)},
         "gpu_launches": launches_per_step * args.steps,
-        "roofline": {"bound": "hbm", "kernel": "the 22 convolution steps of a pass (tcgen05 tile "
-                     "kernel with fused tails)" if flex else "the 22 convolution steps of a pass",
-                     "achieved": round(conv_gbs, 1), "peak": peak,
-                     "unit": "GB/s", "frac": round(conv_gbs / peak, 4),
-                     "traffic": int(traffic * n / 256.0) if traffic else None,
+        "roofline": {"bound": bound, "kernel": "the convolutions of a pass with their fused tails",
+                     "achieved": round(achieved, 1), "peak": round(peak, 1), "unit": unit,
+                     "frac": round(achieved / peak, 4),
+                     "traffic": NCU_CONV_TRAFFIC_BYTES.get((args.workload, n, conv_launches)),
                      "peak_source": which, "algorithmic_bytes_per_launch": int(conv_bytes),
-                     "launch": "one pass = 22 kernel launches", "ms": round(conv_ms, 4),
-                     "ms_source": conv_src},
-        "tensor_TOPS_algorithmic": round(RESNET_FLOP_PER_IMG * n * (4 if flex else 3)
-                                         / (conv_ms * 1e-3) / 1e12, 2),
+                     "launch": "one pass = %d kernel launch%s, %d convolutions"
+                               % (conv_launches, "" if conv_launches == 1 else "es", layers),
+                     "ms": round(conv_ms, 4), "ms_source": conv_src},
+        "tensor_TOPS_algorithmic": round(tensor_ops / (conv_ms * 1e-3) / 1e12, 2),
         "parity": parity,
     }
     net.close()
@@ -807,7 +846,8 @@ def measure_training(args, rank, world, torch, dist, local, flex, steps, repeats
                      "frac": round(tops / tpeak, 4), "traffic": None,
                      "peak_source": which + (" bf16 x 2 as int8 stand-in" if flex else
                                              " bf16 / 2 as tf32 stand-in"),
-                     "ms": round(conv_ms, 4)},
+                     "ms": round(conv_ms, 4),
+                     "ms_source": "CUDA events around every step, launched one by one, gaps included"},
         "step_time_ms_by_kind": {k: round(v[0] / passes, 4) for k, v in kinds.items()},
         "allreduce_algorithmic_bytes_per_gpu": int(2 * (world - 1) / world * TRAIN_PARAM_BYTES),
         "loss_first_steps": [round(v, 5) for v in losses], "loss_last": round(last, 5),

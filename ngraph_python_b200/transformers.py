@@ -196,7 +196,8 @@ class Computation(object):
         self.executor = None
         self.launches_per_call = 0
         self._io = None             # argument and result handling of the recorded step list
-        self.chains = []            # runs of convolutions that recorded calls make in one launch
+        self.recorded = None        # the steps that a recorded call launches, once capture() has been called
+        self.chains = []            # ... and the runs of convolutions among them, a launch each
         self._replayed = ()         # runs of layers that this call has launched
         self._watched = None        # what calls write of the tensors that somebody follows
         self._int16 = []            # those of them that other computations may write as byte planes alone
@@ -329,6 +330,7 @@ class Computation(object):
         refreshable = [s for s in steps if hasattr(s, "refresh") and s.kept_planes()]
         # (of an earlier recording: what it left unstored can still be made)
         t._chains = [c for c in t._chains if c not in self.chains or c.open]
+        self.recorded = steps
         self.chains = chains = [s for s in steps if s.kind == "conv_chain"]
         t._chains.extend(chains)
         for s in chains:
