@@ -248,12 +248,16 @@ int b2_call_stage(const void* src, size_t bytes, void* pinned, const void** visi
  *          the next exponents.  undecided[0..*n_undecided) lists the k whose choice lies so close to
  *          a boundary that it needs exactly rounded sums; *settled: every entry has seen the same
  *          maximum for longer than its history window and keeps its exponent.
+ *   rows written: row slot_read[k] gets the exponent that ids[k] was written with, for calls that read it
+ *          and do not write it.
  * Replace manage_before_computation / manage_after_computation (flexgputransform.py:347-371). */
 #define B2_FLEX_HISTORY 16
 typedef struct b2_flex_state {
     int64_t *dec, *pending; uint8_t* initialized; int64_t* overflows;
     double* hist; int64_t *hist_len, *hist_pos; double* run_value; int64_t *run_length, *run_choice;
 } b2_flex_state;
+int b2_flex_rows_written(const b2_flex_state* s, int32_t n, const int64_t* ids, const int64_t* slot_read,
+                         int64_t* uploaded, b2_flex_scale* host_table, int32_t* changed);
 int b2_flex_begin_call(const b2_flex_state* s, int32_t n, const int64_t* ids,
                        const int64_t* slot_write, const int64_t* slot_read, int64_t* uploaded,
                        b2_flex_scale* host_table, int32_t* changed);

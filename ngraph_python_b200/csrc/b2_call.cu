@@ -267,19 +267,21 @@ extern "C" int b2_call_stage(const void* src, size_t bytes, void* pinned, const 
     return B2_OK;
 }
 
+static int set_row(int64_t slot, int64_t dec, int64_t* uploaded, b2_flex_scale* host_table) {
+    if (uploaded[slot] == dec) return 0;
+    uploaded[slot] = dec;
+    host_table[slot].scale = std::ldexp(1.0f, (int)-dec);
+    host_table[slot].inv_scale = std::ldexp(1.0f, (int)dec);
+    return 1;
+}
+
 extern "C" int b2_flex_begin_call(const b2_flex_state* s, int32_t n, const int64_t* ids,
                                   const int64_t* slot_write, const int64_t* slot_read,
                                   int64_t* uploaded, b2_flex_scale* host_table, int32_t* changed) {
     B2_REQUIRE(s && n >= 0 && (n == 0 || (ids && slot_write && slot_read)) && uploaded && host_table &&
                changed, "null argument");
     int ch = 0;
-    auto row = [&](int64_t slot, int64_t dec) {
-        if (uploaded[slot] == dec) return;
-        uploaded[slot] = dec;
-        host_table[slot].scale = std::ldexp(1.0f, (int)-dec);
-        host_table[slot].inv_scale = std::ldexp(1.0f, (int)dec);
-        ch = 1;
-    };
+    auto row = [&](int64_t slot, int64_t dec) { ch |= set_row(slot, dec, uploaded, host_table); };
     for (int32_t k = 0; k < n; ++k) {
         const int64_t i = ids[k], stored = s->dec[i];
         if (s->initialized[i] && s->pending[i] >= 0) {
@@ -289,6 +291,15 @@ extern "C" int b2_flex_begin_call(const b2_flex_state* s, int32_t n, const int64
         row(slot_write[k], s->dec[i]);
         if (slot_read[k] != slot_write[k]) row(slot_read[k], stored);
     }
+    *changed = ch;
+    return B2_OK;
+}
+
+extern "C" int b2_flex_rows_written(const b2_flex_state* s, int32_t n, const int64_t* ids, const int64_t* slot_read,
+                                    int64_t* uploaded, b2_flex_scale* host_table, int32_t* changed) {
+    B2_REQUIRE(s && n >= 0 && (n == 0 || (ids && slot_read)) && uploaded && host_table && changed, "null argument");
+    int ch = 0;
+    for (int32_t k = 0; k < n; ++k) ch |= set_row(slot_read[k], s->dec[ids[k]], uploaded, host_table);
     *changed = ch;
     return B2_OK;
 }

@@ -220,6 +220,17 @@ class FlexManager(object):
             slots_read.ctypes.data, uploaded.ctypes.data, table.ctypes.data, changed))
         return bool(changed.value)
 
+    def rows_written(self, ids, slots_read, uploaded, table):
+        """The rows through which others read the tensors of `ids`, after a call that wrote them; `uploaded`
+        and `table` as for begin_call.  True when a row changed."""
+        import ctypes
+        from . import lib
+        changed = ctypes.c_int32(0)
+        lib.check(lib.raw().b2_flex_rows_written(
+            self._native_state(), len(ids), ids.ctypes.data, slots_read.ctypes.data, uploaded.ctypes.data,
+            table.ctypes.data, changed))
+        return bool(changed.value)
+
     def _native_state(self):
         """The arrays as the native library takes them."""
         if self._state is None:

@@ -223,6 +223,7 @@ def _load():
         "b2_call_outputs": (C.c_int, [C.POINTER(CallOutput), i32, vp, i32, vp, vp, vp, vp]),
         "b2_call_wait": (C.c_int, [i32, vp]),
         "b2_call_stage": (C.c_int, [vp, sz, vp, C.POINTER(vp)]),
+        "b2_flex_rows_written": (C.c_int, [C.POINTER(FlexState), i32, vp, vp, vp, vp, C.POINTER(i32)]),
         "b2_flex_begin_call": (C.c_int, [C.POINTER(FlexState), i32, vp, vp, vp, vp, vp,
                                          C.POINTER(i32)]),
         "b2_flex_end_call": (C.c_int, [C.POINTER(FlexState), i32, vp, vp, vp, vp, C.POINTER(i32),

@@ -1798,6 +1798,7 @@ class B200Transformer(object):
         self._io_done = False       # the replayed graph has already queued the call's read-back
         self._stats_clean = False   # ... and left the statistics array cleared
         self._flex_epoch = 0        # moves whenever any exponent bookkeeping may have changed
+        self._epoch_at_begin = 0    # ... as it was when the running call began to adopt exponents
         self._chains = []           # runs of layers whose results may be asked for
         self._buffers = collections.OrderedDict()   # op -> Buffer
         self._views = {}
@@ -2304,6 +2305,7 @@ class B200Transformer(object):
                 self._stats.zero_()
             return
         comp._steady = None
+        self._epoch_at_begin = self._flex_epoch
         # Only tensors this computation writes (or receives from the host) can adopt a new exponent
         # here; every other tensor's table rows were brought up to date by the call that wrote it.
         bufs = getattr(comp, "_flex_bufs", None)
@@ -2365,10 +2367,7 @@ class B200Transformer(object):
         exchanging = self._allreduce is not None and self.comm.size > 1
         if exchanging:
             self._allreduce.finish()        # CommError instead of an endless synchronisation
-        device = self.device.index
-        lib.check(lib.raw().b2_call_wait(device, torch._C._cuda_getCurrentRawStream(device)))
-        if exchanging:
-            self._allreduce.after_sync()
+        # (while the device is still at work)
         watched = comp._watched
         if watched is None:
             # (the tensors whose changes somebody follows: convolution filters with cached planes, tensors
@@ -2385,6 +2384,10 @@ class B200Transformer(object):
         for c in comp._replayed:
             c.called(self)
         comp._replayed = ()
+        device = self.device.index
+        lib.check(lib.raw().b2_call_wait(device, torch._C._cuda_getCurrentRawStream(device)))
+        if exchanging:
+            self._allreduce.after_sync()
         if self._status_np[0] != 0:
             self._status.zero_()
             raise lib.B200Error("a device-side wait ran out during the computation")
@@ -2401,6 +2404,7 @@ class B200Transformer(object):
             # the same maxima as after the previous call, with every history window already full
             # of them: every entry would make the choice it made before
             return
+        moved = self._flex_epoch != self._epoch_at_begin      # (some exponent did in this call)
         self._flex_epoch += 1
         fm = self.flex_manager
         inputs = self._inputs_written
@@ -2421,11 +2425,17 @@ class B200Transformer(object):
             for b in comp.written:
                 b.entry.end_write(int(stats[b.slot_write]))
             settled = fm.settled(ids)
-        # Tensors written in place are read by other computations through the row that held their
-        # exponent before the call.
-        for b in comp.written:
-            if b.slot != b.slot_write and not getattr(b, "shares_entry", False):
-                self._set_table_row_host(b.slot, b.entry.dec)
+        if moved:
+            # Tensors written in place are read by other computations through the row that held their
+            # exponent before the call.
+            rows = getattr(comp, "_rows_written", None)
+            if rows is None:
+                both = [(b.entry.i, b.slot) for b in comp.written
+                        if b.slot != b.slot_write and not getattr(b, "shares_entry", False)]
+                rows = comp._rows_written = np.array(both, dtype=np.int64).reshape(-1, 2).T.copy()
+            if fm.rows_written(rows[0], rows[1], self._dec_uploaded, self._table_np):
+                self._flex_epoch += 1
+                self._table_dirty = True
         comp._steady = (self._flex_epoch, slots, stats[slots].tobytes(), len(inputs)) if settled else None
 
     # ---- launching -------------------------------------------------------------------------------
