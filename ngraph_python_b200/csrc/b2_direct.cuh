@@ -20,7 +20,7 @@
 //           batch 100, 5.0e-7 -> 2.9e-7 of the result's root mean square), for one percent of the time.  No shape may
 //           put more k-blocks into one sum than with one pair (b2_direct_args::longest): of 336 random layers and
 //           passes the errors against 64 bits are 0.70 of those with one pair (geometric mean), none larger by more than 3 %
-//           (of K of 75); without that bound 54 of 8010 shapes had longer sums and up to 1.3 times the error.
+//           (of K of 75); without that bound 54 of 8010 shapes had longer sums and up to 1.4 times the error.
 //   flex16: four exact int8 products, HH | X | LL as in b2_gemm_impl.cuh.
 // Slices of K: the CTAs of a cluster (up to 8) take one each; partial sums meet in distributed shared
 // memory, every CTA adds a share of the columns in slice order (deterministic, fp32 adds rounded to

@@ -353,10 +353,13 @@ class ConvChainStep(_Step):
         t.kernel_launches += 1
 
     def called(self, t):
-        """A recorded call has ended."""
+        """A recorded call has been launched."""
         self.open, self.clock = True, t._clock
         for b in self.kept:
             b.int16_at = b.version
+
+    def keep_exponents(self, t):
+        """... and its exponents are settled."""
         if self.epoch != t._flex_epoch:
             self.epoch, self.exponents = t._flex_epoch, t._dec_uploaded[self.rows]
 
@@ -365,6 +368,8 @@ class ConvChainStep(_Step):
         run which did not store it."""
         if not self.open or buf not in self.unstored or buf.version > self.clock:
             return
+        if t.closed:
+            raise lib.B200Error("the transformer has been closed")
         changed = [b.name for b in self.reads if b.version > self.clock]
         if changed or (t._dec_uploaded[self.rows] != self.exponents).any():
             raise lib.B200Error(

@@ -484,7 +484,7 @@ class _CallIO(object):
                 self._pinned_buffer(k)
         self.visible = ctypes.c_void_p()
         # what the computation writes: an argument that lies there is copied before anything runs
-        written = set(v.buffer for s in comp.steps for v in s.out_views)
+        written = set(b for s in comp.steps for b in s.writes())
         written.update(v.buffer for v in views)
         self.written = sorted((b.ptr(), b.ptr() + b.tensor.nbytes) for b in written)
         # results: small dense ones ride in the last node, the others are copied after it
@@ -2381,9 +2381,9 @@ class B200Transformer(object):
                 b.version = self._clock
             for b in comp._int16:
                 b.int16_at = self._clock
-        for c in comp._replayed:
+        ran, comp._replayed = comp._replayed, ()
+        for c in ran:
             c.called(self)
-        comp._replayed = ()
         device = self.device.index
         lib.check(lib.raw().b2_call_wait(device, torch._C._cuda_getCurrentRawStream(device)))
         if exchanging:
@@ -2393,6 +2393,8 @@ class B200Transformer(object):
             raise lib.B200Error("a device-side wait ran out during the computation")
         if self.flex:
             self._end_call_flex(comp)
+        for c in ran:
+            c.keep_exponents(self)
 
     def _end_call_flex(self, comp):
         """Exponent bookkeeping after a call (manage_after_computation, flexgputransform.py:

@@ -165,3 +165,12 @@ def test_no_layer_of_a_run_whose_bias_the_computation_changes_behind_it():
         steps = kernels.chain_convolutions(net.infer.steps, set(v.buffer for v in net.infer.return_views), net.t)
         read = [v.buffer for s in steps if s.kind == "conv_chain" for v in s.in_views]
         assert read and (net.t._view_of(net.biases[1]).buffer in read) != behind
+
+
+@pytest.mark.gpu
+def test_no_results_of_a_closed_transformer():
+    _, net = _pair()
+    tensor = net.t.device_tensor(net.mids[1])
+    net.t.close()
+    with pytest.raises(lib.B200Error, match="closed"):
+        tensor.get()
