@@ -221,15 +221,19 @@ class FlexManager(object):
         return bool(changed.value)
 
     def rows_written(self, ids, slots_read, uploaded, table):
-        """The rows through which others read the tensors of `ids`, after a call that wrote them; `uploaded`
-        and `table` as for begin_call.  True when a row changed."""
+        """A function that sets the rows through which others read the tensors of `ids`, to be called when a
+        call that wrote them has ended; `uploaded` and `table` as for begin_call.  It returns True when a row
+        changed.  (The arrays and their addresses are looked up here, once.)"""
         import ctypes
         from . import lib
-        changed = ctypes.c_int32(0)
-        lib.check(lib.raw().b2_flex_rows_written(
-            self._native_state(), len(ids), ids.ctypes.data, slots_read.ctypes.data, uploaded.ctypes.data,
-            table.ctypes.data, changed))
-        return bool(changed.value)
+        arrays = (ids, slots_read, uploaded, table)
+        at = [a.ctypes.data for a in arrays]
+        changed, call, n = ctypes.c_int32(0), lib.raw().b2_flex_rows_written, len(ids)
+
+        def run(keep=arrays):
+            lib.check(call(self._native_state(), n, at[0], at[1], at[2], at[3], changed))
+            return changed.value != 0
+        return run
 
     def _native_state(self):
         """The arrays as the native library takes them."""

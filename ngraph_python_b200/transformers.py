@@ -202,6 +202,7 @@ class Computation(object):
         self._watched = None        # what calls write of the tensors that somebody follows
         self._int16 = []            # those of them that other computations may write as byte planes alone
         self.bytes_only = set()     # what this one writes as byte planes alone
+        self._rows_written = None, None   # flex16: (scale table, what sets the rows of tensors written in place)
         self._comm_steps = []       # this computation's exchanges, in production order
         self._allreduce = None      # their arena and bucket plan (one per computation)
 
@@ -568,9 +569,10 @@ class _CallIO(object):
     def call(self, args):
         t, comp, block = self.t, self.comp, self.block
         keep = []
+        t._clock = clock = t._clock + 1
         try:
             for (k, buf, arg, read_in_place), value in zip(self.args, args):
-                t._changed(buf)
+                buf.version = clock
                 address, obj = self._source(k, value)
                 arg.src = address
                 # a device tensor is read where it lies by the kernel that uses it first, which
@@ -2381,9 +2383,11 @@ class B200Transformer(object):
                 b.version = self._clock
             for b in comp._int16:
                 b.int16_at = self._clock
-        ran, comp._replayed = comp._replayed, ()
-        for c in ran:
-            c.called(self)
+        ran = comp._replayed
+        if ran:
+            comp._replayed = ()
+            for c in ran:
+                c.called(self)
         device = self.device.index
         lib.check(lib.raw().b2_call_wait(device, torch._C._cuda_getCurrentRawStream(device)))
         if exchanging:
@@ -2430,12 +2434,14 @@ class B200Transformer(object):
         if moved:
             # Tensors written in place are read by other computations through the row that held their
             # exponent before the call.
-            rows = getattr(comp, "_rows_written", None)
-            if rows is None:
+            table, rows_written = comp._rows_written
+            if table is not self._table_np:
                 both = [(b.entry.i, b.slot) for b in comp.written
                         if b.slot != b.slot_write and not getattr(b, "shares_entry", False)]
-                rows = comp._rows_written = np.array(both, dtype=np.int64).reshape(-1, 2).T.copy()
-            if fm.rows_written(rows[0], rows[1], self._dec_uploaded, self._table_np):
+                ids, slots_read = np.array(both, dtype=np.int64).reshape(-1, 2).T.copy()
+                rows_written = fm.rows_written(ids, slots_read, self._dec_uploaded, self._table_np)
+                comp._rows_written = self._table_np, rows_written
+            if rows_written():
                 self._flex_epoch += 1
                 self._table_dirty = True
         comp._steady = (self._flex_epoch, slots, stats[slots].tobytes(), len(inputs)) if settled else None
