@@ -216,6 +216,10 @@ int b2_flex_publish(int32_t* stats, int32_t n, const int32_t* status, int32_t* h
  * where, unless NULL: a device word that gets the address at which the values are to be read -- src for
  * an argument marked in_place, which is then not copied (its reader does that: B2_F32_AT,
  * B2_FLEX16_AT), else dst.
+ * b2_call_take does the same in front of the step list instead of inside it: the block (any host memory)
+ * is read by the call itself, and pageable[k], unless pageable or that is NULL, is host memory that is first copied
+ * to the pinned block at arg[k].src, in pieces that the device reads while the next is copied.
+ * *launches gets how many kernels that took (none where there is nothing to copy).
  * b2_call_outputs is b2_flex_publish with results: dst[k] (pinned host memory) <- bytes[k] bytes of
  * src[k], both 16-byte aligned.
  * b2_call_stage: the address at which the device can read `bytes` bytes of host memory at src:
@@ -235,6 +239,8 @@ typedef struct b2_call_input { void* dst; int64_t n; int32_t flex_slot; int32_t 
 typedef struct b2_call_output { const void* src; void* dst; int64_t bytes; } b2_call_output;
 int b2_call_inputs(const b2_call_input* inputs, int32_t n, const b2_call_block* block,
                    b2_flex_scale* table, int32_t* stats, void* stream);
+int b2_call_take(const b2_call_input* inputs, int32_t n, const b2_call_block* block, const void* const* pageable,
+                 b2_flex_scale* table, int32_t* stats, int32_t* launches, int32_t device, void* stream);
 int b2_call_outputs(const b2_call_output* outputs, int32_t n, int32_t* stats, int32_t n_stats,
                     const int32_t* status, int32_t* host_stats, int32_t* host_status, void* stream);
 int b2_call_wait(int32_t device, void* stream);

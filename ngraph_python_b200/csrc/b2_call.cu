@@ -6,13 +6,20 @@
 // kernel and manage_before / manage_after_computation per tensor (flexgputransform.py:347-371) --
 // by one kernel at each end of a recorded step list and one pass over plain arrays on the host.
 //
-// k_call_inputs is the first node of a recorded step list.  The addresses of a call's arguments
-// stand in a block of pinned host memory that it reads; the values are read from wherever they lie
-// (the caller's own device tensor, the caller's pinned array, or the pinned block into which
-// b2_call_stage copied pageable memory) and stored once, quantised where the tensor is flex16.
-// Bound by what it reads: PCIe for host arguments, HBM for device tensors.  A flex16 argument of
-// 8192 x 16384 values: copy to a staging tensor 173 us + conversion 167 us before, one pass of
-// 6 bytes a value now.
+// k_call_inputs takes the arguments in.  The values are read from wherever they lie (the caller's own
+// device tensor, the caller's pinned array, or the pinned block into which pageable memory was
+// copied) and stored once, quantised where the tensor is flex16.  Bound by what it reads: PCIe for host
+// arguments, HBM for device tensors.  A flex16 argument of 8192 x 16384 values: copy to a staging
+// tensor 173 us + conversion 167 us before, one pass of 6 bytes a value now.
+//
+// b2_call_take launches it in front of a recorded step list: addresses and scales are launch parameters,
+// only what is to be copied has blocks, and it runs while the launch of the graph is on its way (8 to
+// 10 us from the call to the first node); pageable memory goes through the pinned block in pieces, each
+// read by the device while the host copies the next.  As the graph's first node (b2_call_inputs) every block
+// reads its addresses from pinned memory first, 1184 of them where nothing is copied.  A call, first node ->
+// in front, one B200: 333 x 1001 flex16 values from the device 50 -> 34 us; 8192 x 16384 read in place by
+// their kernel, flex16 / fp32 373 -> 355 / 538 -> 515 us; 400 KB pageable and 22 launches 157 -> 149 us; 3 MB
+// pinned and a run of layers 248 -> 244 us.  (The last results' stores, below, are part of that.)
 #include <cmath>
 #include <cstddef>
 #include <cstring>
@@ -34,6 +41,14 @@ struct Inputs {
     int n;
     b2_call_input in[B2_CALL_MAX_INPUTS];
     long long first_chunk[B2_CALL_MAX_INPUTS + 1];
+    // as of b2_call_take (else they stand in the block):
+    const void* src[B2_CALL_MAX_INPUTS];      // nothing to copy where null
+    float inv[B2_CALL_MAX_INPUTS];
+    int n_words;                              // device words for addresses: where[i] <- address[i]
+    const void** where[B2_CALL_MAX_INPUTS];
+    const void* address[B2_CALL_MAX_INPUTS];
+    const b2_flex_scale* rows;                // rows of the scale table
+    int n_rows;
 };
 
 __device__ __forceinline__ short quant1(float x, float inv, int& stat) {
@@ -52,7 +67,17 @@ k_call_inputs(const Inputs a, const b2_call_block* __restrict__ blk, b2_flex_sca
     __shared__ int ismem[32];
     __shared__ const float* src_s[B2_CALL_MAX_INPUTS];
     __shared__ float inv_s[B2_CALL_MAX_INPUTS];
-    if (threadIdx.x < a.n) {
+    if (!blk) {
+        if (threadIdx.x < a.n) {
+            src_s[threadIdx.x] = (const float*)a.src[threadIdx.x];
+            inv_s[threadIdx.x] = a.inv[threadIdx.x];
+        }
+        // (the last block has the fewest values to copy)
+        if (blockIdx.x == gridDim.x - 1) {
+            if (threadIdx.x < a.n_words) *a.where[threadIdx.x] = a.address[threadIdx.x];
+            for (int i = threadIdx.x; i < a.n_rows; i += kThreads) table[i] = a.rows[i];
+        }
+    } else if (threadIdx.x < a.n) {
         // one 16-byte read over PCIe to a block and argument
         const uint4 e = *reinterpret_cast<const uint4*>(&blk->arg[threadIdx.x]);
         const float* src = (const float*)((unsigned long long)e.y << 32 | e.x);
@@ -63,7 +88,7 @@ k_call_inputs(const Inputs a, const b2_call_block* __restrict__ blk, b2_flex_sca
             *a.in[threadIdx.x].where = in_place ? (const void*)src : a.in[threadIdx.x].dst;
     }
     // the scale table, when a row of it has changed
-    if (blockIdx.x == gridDim.x - 1 && table && blk->table_rows > 0) {
+    if (blk && blockIdx.x == gridDim.x - 1 && table && blk->table_rows > 0) {
         const b2_flex_scale* h = blk->table;
         for (int i = threadIdx.x; i < blk->table_rows; i += kThreads) table[i] = h[i];
     }
@@ -115,35 +140,55 @@ k_call_inputs(const Inputs a, const b2_call_block* __restrict__ blk, b2_flex_sca
     if (a.n && a.in[cur].flex_slot >= 0) b2_block_stat(stat, stats + a.in[cur].flex_slot, ismem);
 }
 
+// chunks of the inputs, and the launch: values a thread takes by how much there is in all
+cudaError_t launch_inputs(Inputs& a, const b2_call_block* block, b2_flex_scale* table, int* stats, cudaStream_t st) {
+    long long chunks = 0, total = 0;
+    for (int i = 0; i < a.n; ++i) total += a.in[i].n;
+    const bool brief = total < 148LL * 2 * kThreads * kPerLong;
+    const int kChunk = kThreads * (brief ? kPerShort : kPerLong);
+    for (int i = 0; i < a.n; ++i) {
+        a.first_chunk[i] = chunks;
+        chunks += (a.in[i].n + kChunk - 1) / kChunk;
+    }
+    a.first_chunk[a.n] = chunks;
+    const unsigned grid = (unsigned)(chunks < 1 ? 1 : chunks > 148 * 8 ? 148 * 8 : chunks);
+    if (brief) k_call_inputs<kPerShort><<<grid, kThreads, 0, st>>>(a, block, table, stats);
+    else k_call_inputs<kPerLong><<<grid, kThreads, 0, st>>>(a, block, table, stats);
+    return cudaGetLastError();
+}
+
 struct Outputs {
     int n;
     b2_call_output out[B2_CALL_MAX_OUTPUTS];
+    int first_block[B2_CALL_MAX_OUTPUTS + 1];
 };
 
 // End of a call: results, flex statistics and status word into pinned host memory the device can
-// address, statistics cleared.  Block 0 takes statistics and status, the others the results.
+// address, statistics cleared.  Block 0 takes statistics and status, the others 4 KB of a result each:
+// bound by one read and one posted write over PCIe (blocks that went through the results one after another
+// waited for every read: five results and ten blocks 6.9 -> 5.1 us, seven blocks 7.2 -> 4.0 us).
 __global__ void __launch_bounds__(kThreads)
 k_call_outputs(const Outputs o, int* __restrict__ stats, int n_stats, const int* __restrict__ status,
                int* __restrict__ host_stats, int* __restrict__ host_status) {
     after_earlier_kernels();
     if (blockIdx.x == 0) {
+        const int word = threadIdx.x == 0 && status ? *status : 0;
         for (int i = threadIdx.x; i < n_stats; i += kThreads) {
             host_stats[i] = stats[i];
             stats[i] = 0;
         }
-        if (threadIdx.x == 0 && status) *host_status = *status;
+        if (threadIdx.x == 0 && status) *host_status = word;
     } else {
-        const long long first = (long long)(blockIdx.x - 1) * kThreads + threadIdx.x;
-        const long long stride = (long long)(gridDim.x - 1) * kThreads;
-        for (int k = 0; k < o.n; ++k) {
-            const long long n16 = o.out[k].bytes >> 4;       // (allocations are 16-byte aligned)
-            const uint4* s = reinterpret_cast<const uint4*>(o.out[k].src);
-            uint4* d = reinterpret_cast<uint4*>(o.out[k].dst);
-            for (long long i = first; i < n16; i += stride) d[i] = s[i];
-            const long long tail = (n16 << 4) + first * 2;   // (elements are 2 or 4 bytes)
-            if (tail < o.out[k].bytes)
-                *(unsigned short*)((char*)o.out[k].dst + tail) = *(const unsigned short*)((const char*)o.out[k].src + tail);
-        }
+        int k = 0;
+        while ((int)blockIdx.x - 1 >= o.first_block[k + 1]) ++k;
+        const long long at = ((long long)((int)blockIdx.x - 1 - o.first_block[k]) * kThreads + threadIdx.x) * 16;
+        const long long left = o.out[k].bytes - at;
+        const char* s = (const char*)o.out[k].src + at;       // (allocations are 16-byte aligned)
+        char* d = (char*)o.out[k].dst + at;
+        if (left >= 16) *reinterpret_cast<uint4*>(d) = *reinterpret_cast<const uint4*>(s);
+        else
+            for (int i = 0; i < left; i += 2)                  // (elements are 2 or 4 bytes)
+                *(unsigned short*)(d + i) = *(const unsigned short*)(s + i);
     }
 }
 
@@ -188,25 +233,84 @@ extern "C" int b2_call_inputs(const b2_call_input* inputs, int32_t n, const b2_c
     static_assert(sizeof(b2_call_arg) == 16 && offsetof(b2_call_block, arg) % 16 == 0, "read as one word");
     B2_REQUIRE(n >= 0 && n <= B2_CALL_MAX_INPUTS && (n == 0 || inputs) && block &&
                ((uintptr_t)block & 15) == 0, "bad argument");
-    Inputs a;
+    Inputs a = {};
     a.n = n;
-    long long chunks = 0, total = 0;
-    for (int i = 0; i < n; ++i) total += inputs[i].n;
-    const bool brief = total < 148LL * 2 * kThreads * kPerLong;
-    const int kChunk = kThreads * (brief ? kPerShort : kPerLong);
     for (int i = 0; i < n; ++i) {
         B2_REQUIRE(inputs[i].dst && inputs[i].n >= 0 && (inputs[i].flex_slot < 0 || stats), "bad argument");
         a.in[i] = inputs[i];
-        a.first_chunk[i] = chunks;
-        chunks += (inputs[i].n + kChunk - 1) / kChunk;
     }
-    a.first_chunk[n] = chunks;
-    long long grid = chunks < 1 ? 1 : chunks > 148 * 8 ? 148 * 8 : chunks;
-    if (brief)
-        k_call_inputs<kPerShort><<<(unsigned)grid, kThreads, 0, (cudaStream_t)stream>>>(a, block, table, stats);
-    else
-        k_call_inputs<kPerLong><<<(unsigned)grid, kThreads, 0, (cudaStream_t)stream>>>(a, block, table, stats);
-    B2_CUDA(cudaGetLastError());
+    B2_CUDA(launch_inputs(a, block, table, stats, (cudaStream_t)stream));
+    return B2_OK;
+}
+
+namespace {
+void copy_to_pinned(void* pinned, const void* src, size_t bytes) {
+#if defined(__x86_64__)
+    static const bool avx2 = __builtin_cpu_supports("avx2");
+    if (avx2 && ((uintptr_t)pinned & 31) == 0) return copy_streaming(pinned, src, bytes);
+#endif
+    memcpy(pinned, src, bytes);
+}
+}  // namespace
+
+extern "C" int b2_call_take(const b2_call_input* inputs, int32_t n, const b2_call_block* block,
+                            const void* const* pageable, b2_flex_scale* table, int32_t* stats, int32_t* launches,
+                            int32_t device, void* stream) {
+    B2_REQUIRE(n >= 0 && n <= B2_CALL_MAX_INPUTS && (n == 0 || inputs) && block && launches, "bad argument");
+    B2_REQUIRE(block->table_rows <= 0 || (table && block->table), "rows without a table");
+    *launches = 0;
+    int current = device;
+    B2_CUDA(cudaGetDevice(&current));
+    const struct Back {                                        // (stream 0 is the current device's)
+        int to, from;
+        Back(int t, int f) : to(t), from(f) { if (to != from) cudaSetDevice(from); }
+        ~Back() { if (to != from) cudaSetDevice(to); }
+    } back(current, device);
+    // A piece of pageable memory: the host copies about 20 GB/s and a launch costs it 2 us, PCIe brings
+    // 50 GB/s: less than 192 KB (10 us of copying, 4 of reading) is not worth another launch.
+    const long long least = 48 << 10;                          // values
+    Inputs a = {};
+    a.rows = block->table;
+    a.n_rows = block->table_rows > 0 ? block->table_rows : 0;
+    for (int k = 0; k < n; ++k) {
+        B2_REQUIRE(inputs[k].dst && inputs[k].n >= 0 && (inputs[k].flex_slot < 0 || stats), "bad argument");
+        const void* src = block->arg[k].src;
+        if (!inputs[k].where) continue;
+        // (where there is nothing to copy the values are in their place)
+        a.where[a.n_words] = inputs[k].where;
+        a.address[a.n_words++] = src && block->arg[k].in_place ? src : inputs[k].dst;
+    }
+    auto add = [&](const b2_call_input& in, const b2_call_arg& arg, long long first, long long count) {
+        a.in[a.n] = in;
+        a.in[a.n].n = count;
+        a.in[a.n].dst = (char*)in.dst + first * (in.flex_slot >= 0 ? 2 : 4);
+        a.src[a.n] = (const float*)arg.src + first;
+        a.inv[a.n++] = arg.inv_scale;
+    };
+    auto launch = [&]() -> cudaError_t {
+        const cudaError_t e = launch_inputs(a, nullptr, table, stats, (cudaStream_t)stream);
+        ++*launches;
+        a.n = a.n_words = a.n_rows = 0;
+        return e;
+    };
+    for (int pass = 0; pass < 2; ++pass)                       // pageable memory last
+        for (int k = 0; k < n; ++k) {
+            const b2_call_arg& arg = block->arg[k];
+            const bool staged = pageable && pageable[k];
+            if (!arg.src || (arg.in_place && inputs[k].where) || staged != (pass == 1)) continue;
+            if (!staged) { add(inputs[k], arg, 0, inputs[k].n); continue; }
+            const long long count = inputs[k].n;
+            long long piece = count / 4 / 4096 * 4096;
+            if (piece < least) piece = least;
+            for (long long at = 0; at < count; at += piece) {
+                const long long now = count - at < piece + piece / 2 ? count - at : piece;
+                copy_to_pinned((float*)arg.src + at, (const float*)pageable[k] + at, (size_t)now * 4);
+                add(inputs[k], arg, at, now);
+                if (at + now < count) { B2_CUDA(launch()); continue; }
+                break;
+            }
+        }
+    if (a.n || a.n_words || a.n_rows) B2_CUDA(launch());
     return B2_OK;
 }
 
@@ -218,17 +322,17 @@ extern "C" int b2_call_outputs(const b2_call_output* outputs, int32_t n, int32_t
     B2_REQUIRE((status == nullptr) == (host_status == nullptr), "status source and destination go together");
     Outputs o;
     o.n = n;
-    long long most = 0;
+    o.first_block[0] = 0;
     for (int i = 0; i < n; ++i) {
         B2_REQUIRE(outputs[i].src && outputs[i].dst && outputs[i].bytes >= 0 &&
                    (((uintptr_t)outputs[i].src | (uintptr_t)outputs[i].dst) & 15) == 0,
                    "results must be 16-byte aligned");
+        const long long blocks = (outputs[i].bytes + kThreads * 16 - 1) / (kThreads * 16);
+        B2_REQUIRE(o.first_block[i] + blocks < (1 << 30), "results too large");
         o.out[i] = outputs[i];
-        if (outputs[i].bytes > most) most = outputs[i].bytes;
+        o.first_block[i + 1] = o.first_block[i] + (int)blocks;
     }
-    long long grid = n == 0 ? 1 : 1 + (most / 16 + kThreads - 1) / kThreads;
-    if (n && grid < 2) grid = 2;
-    if (grid > 65) grid = 65;
+    const int grid = 1 + o.first_block[n];
     B2_CUDA(b2::launch_after(k_call_outputs, dim3((unsigned)grid), kThreads, 0, (cudaStream_t)stream, o, stats, n_stats, status,
                                                                           host_stats, host_status));
     B2_CUDA(cudaGetLastError());
@@ -256,13 +360,7 @@ extern "C" int b2_call_stage(const void* src, size_t bytes, void* pinned, const 
     (void)cudaGetLastError();                     // (not a CUDA address: no error of the caller's)
     *visible = nullptr;
     if (!pinned) return B2_OK;                    // pageable, and no block to copy to
-#if defined(__x86_64__)
-    static const bool avx2 = __builtin_cpu_supports("avx2");
-    if (avx2 && ((uintptr_t)pinned & 31) == 0) copy_streaming(pinned, src, bytes);
-    else memcpy(pinned, src, bytes);
-#else
-    memcpy(pinned, src, bytes);
-#endif
+    copy_to_pinned(pinned, src, bytes);
     *visible = pinned;
     return B2_OK;
 }

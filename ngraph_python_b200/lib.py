@@ -220,6 +220,7 @@ def _load():
         "b2_absmax_bits_f32": (C.c_int, [vp, i64, vp, vp]),
         "b2_flex_publish": (C.c_int, [vp, i32, vp, vp, vp, vp]),
         "b2_call_inputs": (C.c_int, [C.POINTER(CallInput), i32, vp, vp, vp, vp]),
+        "b2_call_take": (C.c_int, [vp, i32, vp, vp, vp, vp, vp, i32, vp]),
         "b2_call_outputs": (C.c_int, [C.POINTER(CallOutput), i32, vp, i32, vp, vp, vp, vp]),
         "b2_call_wait": (C.c_int, [i32, vp]),
         "b2_call_stage": (C.c_int, [vp, sz, vp, C.POINTER(vp)]),

@@ -378,7 +378,7 @@ class Computation(object):
         t._allreduce = self._allreduce
         if t._allreduce is not None:
             t._allreduce.begin_call()
-        t._recording_call = False        # set once the graph's first node places the arguments
+        t._recording_call = False        # set once a launch in front of the graph places the arguments
         t._recording = has_comm          # comm steps and waits: kernels only, no NCCL, no bookkeeping
         io_in_graph = False
         io = _CallIO.of(self, exchanged_apart=has_comm)
@@ -398,7 +398,7 @@ class Computation(object):
                 g = torch.cuda.CUDAGraph()
                 with torch.cuda.graph(g):
                     if io is not None and seg is segments[0]:
-                        io.record_inputs()       # the call's arguments are the first node
+                        io.record_inputs()       # the call's arguments are there before the first node
                         t._recording_call = True
                     for s in seg["steps"]:
                         t._launch_step(s)
@@ -447,10 +447,9 @@ builtin_sum = sum
 
 # ---------------------------------------------------------------------------------------------
 class _CallIO(object):
-    """Arguments and results of a recorded step list: its first node reads the arguments from
-    wherever they lie and its last one stores small results into pinned memory, so that a call is
-    one graph launch and one synchronisation.  Per argument the host only writes an address into a
-    pinned block; pageable memory is first copied to a pinned buffer."""
+    """Arguments and results of a recorded step list: a launch in front of it reads the arguments from
+    wherever they lie, pageable memory through a pinned buffer, and its last node stores small results
+    into pinned memory, so that a call is two launches and one synchronisation."""
 
     STAGED_MOST = 4 << 20       # pageable arguments up to this size go through a pinned buffer
     RESULTS_MOST = 1 << 20      # results up to this many bytes are stored by the last node
@@ -472,8 +471,10 @@ class _CallIO(object):
         self.lengths = [tuple(v.axes.lengths) for v in views]
         self.flex_views = [v for v in views if v.buffer.flex]
         self.flex_buffers = [v.buffer for v in self.flex_views]
-        self.block_mem = torch.zeros((ctypes.sizeof(lib.CallBlock),), dtype=torch.uint8).pin_memory()
-        self.block = lib.CallBlock.from_address(self.block_mem.data_ptr())
+        self.block = lib.CallBlock()
+        self.inputs = (lib.CallInput * max(1, len(views)))()
+        self.pageable = (ctypes.c_void_p * max(1, len(views)))()     # ... arguments, while a call takes them in
+        self.launches = ctypes.c_int32()
         self.args = [(k, v.buffer, self.block.arg[k], v.buffer.where is not None)
                      for k, v in enumerate(views)]
         self.table_rows = t._table_host.shape[0] if t.flex else 0
@@ -512,17 +513,23 @@ class _CallIO(object):
         return self.pinned[k].data_ptr()
 
     def record_inputs(self):
+        """What the launch that takes the arguments in is told about their tensors."""
         t = self.t
-        ins = (lib.CallInput * max(1, len(self.views)))()
+        ins = self.inputs
         for k, v in enumerate(self.views):
             ins[k].dst, ins[k].n = v.buffer.ptr(), v.buffer.size
             ins[k].flex_slot = v.buffer.slot if v.buffer.flex else -1
             ins[k].where = v.buffer.where.data_ptr() if v.buffer.where is not None else None
-        lib.check(lib.raw().b2_call_inputs(
-            ins, len(self.views), self.block_mem.data_ptr(),
-            t._table.data_ptr() if t.flex else None, t._stats.data_ptr() if t.flex else None,
-            t.stream.cuda_stream))
-        t.kernel_launches += 1
+        device = t.device.index
+        fixed = (ctypes.addressof(ins), len(self.views), ctypes.addressof(self.block), ctypes.addressof(self.pageable),
+                 t._table.data_ptr() if t.flex else None, t._stats.data_ptr() if t.flex else None,
+                 ctypes.addressof(self.launches), device)
+        take, stream_of = lib.raw().b2_call_take, t.torch._C._cuda_getCurrentRawStream
+
+        def taken():
+            lib.check(take(*fixed, stream_of(device)))
+            t.kernel_launches += self.launches.value
+        self.take = taken
 
     def ready(self):
         """False while an argument has no exponent yet: its range has to be measured first."""
@@ -556,14 +563,14 @@ class _CallIO(object):
         # (the buffer is made only for an argument that needs it: pinning memory takes milliseconds)
         address, stage = arr.__array_interface__["data"][0], lib.raw().b2_call_stage
         through_pinned = arr.nbytes <= self.STAGED_MOST
-        have = self.pinned[k].data_ptr() if through_pinned and self.pinned[k] is not None else None
-        lib.check(stage(address, arr.nbytes, have, self.visible))
+        lib.check(stage(address, arr.nbytes, None, self.visible))
         if not self.visible.value and not through_pinned:
             # pageable: the driver's own pipelined copy
             t._stage(view, arr)
             return (buf.staging.data_ptr() if buf.flex else 0), arr
         if not self.visible.value:
-            lib.check(stage(address, arr.nbytes, self._pinned_buffer(k), self.visible))
+            self.pageable[k] = address
+            return self._pinned_buffer(k), arr
         return self.visible.value, arr
 
     def call(self, args):
@@ -587,13 +594,18 @@ class _CallIO(object):
                     arg.inv_scale = math.ldexp(1.0, buf.entry.dec)
             if self.flex_buffers:
                 t._inputs_written = list(self.flex_buffers)
-            comp.executor()
-            pending = [None if r is not None else t._device_to_host_async(v)
-                       for r, v in zip(self.results, comp.return_views)]
+            self.take()
+            try:
+                comp.executor()
+                pending = [None if r is not None else t._device_to_host_async(v)
+                           for r, v in zip(self.results, comp.return_views)]
+            except BaseException:
+                t.stream.synchronize()         # (the arguments may still be being read)
+                raise
             t._end_call(comp)
         finally:
-            for _, _, arg, _ in self.args:
-                arg.src = None
+            for k, _, arg, _ in self.args:
+                arg.src = self.pageable[k] = None
             block.table_rows = 0
         return comp._results([
             t._finish_host(p) if r is None else t._as_result(*r)
@@ -1795,7 +1807,7 @@ class B200Transformer(object):
         self._inputs_written = []
         self._allreduce = None      # exchange state of the computation that ran last
         self._recording = False     # a CUDA graph segment is being recorded
-        self._recording_call = False   # ... behind the node that places a call's arguments
+        self._recording_call = False   # ... behind the launch that places a call's arguments
         self.tracer = None
         self._io_done = False       # the replayed graph has already queued the call's read-back
         self._stats_clean = False   # ... and left the statistics array cleared
@@ -2282,8 +2294,7 @@ class B200Transformer(object):
             self._table_dirty = True
 
     def _begin_call(self, comp, io=None):
-        """io: the recorded step list's argument handling; its first node then uploads the scale
-        table."""
+        """io: the recorded step list's argument handling, which then uploads the scale table."""
         self._ensure_scratch()
         self._allreduce = comp._allreduce
         if self._allreduce is not None:
