@@ -1,6 +1,7 @@
 // Tensor-core product with the operands converted on the way in: C[M,N] = A[M,K] * B[N,K]^T in one
 // launch, for problems where the pre-pass of the plane kernel (b2_gemm_impl.cuh) and its launches
-// cost as much as the product, and for convolutions that would otherwise be unrolled in memory.
+// cost as much as the product, and for convolutions that would otherwise be unrolled in memory.  (Matrix products
+// of more than a few k-blocks: b2_stream.cuh.)
 //
 // One CTA per 128 x BN tile (times a slice of K), 288 or 544 threads:
 //   one or two groups of eight warps: producers -- load a k-block of both operands from wherever it
@@ -29,8 +30,7 @@
 // What bounds it: at the sizes it is chosen for, latency -- launch, first loads, one pass through the
 // ring, the exchange in the cluster -- so the split is taken to give every SM a CTA; for unrolled
 // convolutions the producers' issue slots.  The second group halves what a k-block waits for where an SM has
-// one CTA (one B200, one group -> two, us: fp32 512 x 128 x 784 16.7 -> 11.5, 600 x 600 x 600 24.5 -> 14.6,
-// flex16 512 x 128 x 784 11.0 -> 8.7, 905 x 380 x 611 24.1 -> 15.0; 20 % of it over 38 sizes).
+// one CTA (one B200, one group -> two, us: fp32 512 x 128 x 784 16.7 -> 11.5, 600 x 600 x 600 24.5 -> 14.6).
 // Unrolled convolutions whose filters were laid out beforehand leave the producers only the gathered rows, and
 // tiles of more pixels pay (batch 100, forward / input gradient, us: 16 channels at 32x32 20.2 -> 12.9 / 25.1 ->
 // 12.9, 32 at 16x16 14.6 -> 12.1 / 23.3 -> 12.2, 64 at 8x8 14.3 -> 12.1 / 14.2 -> 12.1); the filters' way from L2 to
@@ -831,6 +831,11 @@ template <int MODE, int BN, int G>
 int direct_launch_bn(const DirectParams& p, cudaStream_t st) {
     if constexpr (MODE == MODE_F32X3)
         if (p.a.staged) return direct_launch_as<MODE, BN, B2_OPERAND_GATHER, G, true>(p, st);
+    // (flex16 matrix products come here with one k-block: one group)
+    if constexpr (MODE == MODE_FLEX16 && G > 1) {
+        B2_REQUIRE(p.a.a_kind == B2_OPERAND_GATHER, "a product of several k-blocks");
+        return direct_launch_as<MODE, BN, B2_OPERAND_GATHER, G>(p, st);
+    }
     switch (p.a.a_kind) {
         case B2_OPERAND_K: return direct_launch_as<MODE, BN, B2_OPERAND_K, G>(p, st);
         case B2_OPERAND_ROWS: return direct_launch_as<MODE, BN, B2_OPERAND_ROWS, G>(p, st);

@@ -74,6 +74,12 @@ __attribute__((visibility("hidden"))) int b2_direct_stage_filters(const b2_stage
                                                                   cudaStream_t st);
 __attribute__((visibility("hidden"))) int b2_direct_launch(const b2_direct_args& a, cudaStream_t st);
 
+// Matrix products of operands as they lie (b2_stream.cuh): whether it takes one rather than the kernel above, and likewise.
+__attribute__((visibility("hidden"))) bool b2_product_streams(const b2_direct_args& a);
+__attribute__((visibility("hidden"))) long long b2_stream_cost(const b2_direct_args& a);
+__attribute__((visibility("hidden"))) void b2_stream_plan(const b2_direct_args& a, b2_gemm_plan_info* plan);
+__attribute__((visibility("hidden"))) int b2_stream_launch(const b2_direct_args& a, cudaStream_t st);
+
 // fp32 filter gradient (b2_conv_update_f32.cu): no dilation, one depth.  Scratch 0: not taken.
 struct b2_update_f32 { int C, H, W, N, K, R, S, P, Q, pad_h, pad_w, str_h, str_w; };
 __attribute__((visibility("hidden"))) size_t b2_update_f32_scratch(const b2_update_f32& g);

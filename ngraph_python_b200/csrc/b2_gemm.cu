@@ -52,16 +52,20 @@ inline bool gemm_goes_direct(int mode, const void* A, long long a_rs, long long 
     t.A = d.B; t.a_rs = d.b_rs; t.a_ks = d.b_ks; t.a_kind = d.b_kind;
     t.B = d.A; t.b_rs = d.a_rs; t.b_ks = d.a_ks; t.b_kind = d.a_kind;
     t.M = N; t.N = M; t.colmajor = 1;
-    const long long cd = b2_direct_cost(d), ct = b2_direct_cost(t);
+    const bool streams = b2_product_streams(d);                   // (the same for C's transpose)
+    const long long cd = streams ? b2_stream_cost(d) : b2_direct_cost(d), ct = streams ? b2_stream_cost(t) : b2_direct_cost(t);
     const long long plane = plane_cost(mode, shapes_for(mode, M, N, K), M, N, K);
     const bool swap = ct >= 0 && (cd < 0 || ct < cd);
     *out = swap ? t : d;
     long long best = swap ? ct : cd;
+    // (near the line the planes are the faster ones: flex16 2692 x 688 x 640 16.4 us, 18.2 in one launch, 500 x 500 x 6000
+    // transposed 19.6 and 21.3)
+    if (streams && mode == MODE_FLEX16) best += best / 8;
     // Both operands contiguous along their rows take longer than the direct kernel's own choice of a shape has to
     // know: fp32 638 x 937 x 631 26 us against 20 on planes, 383 x 3300 x 1440 47 and 39 (two k-blocks or less
     // don't: 1869 x 1337 x 46 20 and 26); flex16 an odd number of values apart, loaded one by one, 249 x 1831 x
     // 3065 75 and 41, 745 x 913 x 1135 65 and 31.  (With one of the two along K: 236 x 339 x 3450 26 and 33.)
-    if (d.a_kind == B2_OPERAND_ROWS && d.b_kind == B2_OPERAND_ROWS) {
+    if (!streams && d.a_kind == B2_OPERAND_ROWS && d.b_kind == B2_OPERAND_ROWS) {
         if (mode == MODE_F32X3) best += K > 64 ? best / 6 : 0;
         else if (K > 128 && out->a_ks % 2 != 0) best += best / 2;
     }
@@ -81,7 +85,7 @@ int run_gemm(const T* A, long long a_rs, long long a_cs, const T* B, long long b
         d.C = C; d.ldc = ldc; d.table = table; d.slotC = slotC;
         d.slotA = d.colmajor ? slotB : slotA; d.slotB = d.colmajor ? slotA : slotB;
         d.stats = stats; d.probe_out = probe_out; d.status = status; d.probe = probe;
-        return b2_direct_launch(d, st);
+        return b2_product_streams(d) ? b2_stream_launch(d, st) : b2_direct_launch(d, st);
     }
     const Shapes s = shapes_for(MODE, M, N, K);
     const int splits = pick_splits(MODE, s, false);     // > 1 only for flex16 with K > 32768
@@ -128,7 +132,7 @@ extern "C" int b2_gemm_launches(int32_t flex, int64_t a_k_stride, int64_t b_k_st
     B2_REQUIRE(launches && M > 0 && N > 0 && K > 0, "bad argument");
     const int mode = flex ? MODE_FLEX16 : MODE_F32X3;
     b2_direct_args d;
-    *launches = gemm_goes_direct(mode, nullptr, 1, a_k_stride, nullptr, b_k_stride, 1, M, N, K, &d) ? 1
+    *launches = gemm_goes_direct(mode, nullptr, a_k_stride == 1 ? K : 1, a_k_stride, nullptr, b_k_stride, b_k_stride == 1 ? K : 1, M, N, K, &d) ? 1
                 : pick_splits(mode, shapes_for(mode, M, N, K), false) > 1 ? 3 : 2;
     return B2_OK;
 }
@@ -138,8 +142,9 @@ extern "C" int b2_gemm_plan(int32_t flex, int64_t a_k_stride, int64_t b_k_stride
     B2_REQUIRE(plan && M > 0 && N > 0 && K > 0, "bad argument");
     const int mode = flex ? MODE_FLEX16 : MODE_F32X3;
     b2_direct_args d;
-    if (gemm_goes_direct(mode, nullptr, 1, a_k_stride, nullptr, b_k_stride, 1, M, N, K, &d)) {
-        b2_direct_plan(d, plan);
+    if (gemm_goes_direct(mode, nullptr, a_k_stride == 1 ? K : 1, a_k_stride, nullptr, b_k_stride, b_k_stride == 1 ? K : 1, M, N, K, &d)) {
+        if (b2_product_streams(d)) b2_stream_plan(d, plan);
+        else b2_direct_plan(d, plan);
         return B2_OK;
     }
     const Shapes s = shapes_for(mode, M, N, K);
