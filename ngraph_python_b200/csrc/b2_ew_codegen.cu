@@ -160,6 +160,7 @@ struct Plan {
     int nsplit = 1;     // CTAs sharing one row (REDUCE_C)
     dim3 grid;
     bool vec = false;
+    bool ragged = false;     // vectors although rows do not start and end on one
     bool prefetch = false;   // load step j+1 into spare registers before computing step j
     int minb = 1;            // __launch_bounds__ second argument (CTAs per SM to fit registers for)
     bool staged = false;     // inputs travel global -> shared by cp.async.bulk, STAGES deep
@@ -266,9 +267,35 @@ const char* raw_type(int dtype, int V) {
 }
 bool prefetchable(const b2_ew_tensor& t, const Plan& pl) { return pl.vec && t.sc != 0; }
 
+// a tensor that has every element of the iteration space, "" without one
+std::string full_tensor(const b2_ew_program& p) {
+    for (int i = 0; i < p.n_in; ++i)
+        if (p.in[i].sc == 1) return "in[" + std::to_string(i) + "]";
+    for (int k = 0; k < p.n_out; ++k)
+        if (p.out[k].t.sc == 1) return "out[" + std::to_string(k) + "]";
+    return "";
+}
+
 // Issues the raw vector loads of step `jexpr` into registers <prefix><i>.
 void emit_raw_loads(std::ostringstream& o, const b2_ew_program& p, const Plan& pl,
                     const std::string& prefix, const std::string& jexpr, const std::string& ind) {
+    if (pl.ragged) {
+        // the vectors at the two ends of a row: element by element
+        o << ind << "if (there == (1u << V) - 1u) {\n";
+        for (int some = 0; some < 2; ++some) {
+            if (some) o << ind << "} else {\n";
+            for (int i = 0; i < p.n_in; ++i) {
+                if (!prefetchable(p.in[i], pl)) continue;
+                const bool at = p.in[i].dtype == B2_FLEX16_AT;
+                o << ind << "    " << (at ? "b2_ldraw_at" : "b2_ldraw") << (some ? "_some" : "") << "(in" << i << " + c";
+                if (at) o << ", im" << i << " + c, fp" << i;
+                if (some) o << ", there";
+                o << ", " << prefix << i << ");\n";
+            }
+        }
+        o << ind << "}\n";
+        return;
+    }
     for (int i = 0; i < p.n_in; ++i)
         if (prefetchable(p.in[i], pl) && p.in[i].dtype == B2_FLEX16_AT)
             o << ind << "b2_ldraw_at(in" << i << " + (" << jexpr << ") * V, im" << i << " + (" << jexpr << ") * V, fp"
@@ -354,6 +381,7 @@ void emit_store_always(std::ostringstream& o, const b2_ew_program& p, const Plan
         return;
     }
     if (!flex) {
+        if (pl.ragged) o << ind << "if (there != (1u << V) - 1u) b2_st_some<V>(o" << k << " + c, y" << k << ", there);\n" << ind << "else {\n";
         if (pl.vec)
             for (int h = 0; h < pl.V / 4; ++h)
                 o << ind << "b2_st4_cs(o" << k << " + c + " << 4 * h << ", y" << k << " + "
@@ -361,9 +389,11 @@ void emit_store_always(std::ostringstream& o, const b2_ew_program& p, const Plan
         else
             o << ind << "_Pragma(\"unroll\") for (int e = 0; e < V; ++e) o" << k
               << "[(c + e) * p.out_sc[" << k << "]] = y" << k << "[e];\n";
+        if (pl.ragged) o << ind << "}\n";
         return;
     }
     const int at = stored_input(p, k);
+    if (pl.ragged && at >= 0) o << ind << "if (there != (1u << V) - 1u) b2_st_words_some(o" << k << " + c, m" << at << ", pairs" << k << ", there);\n" << ind << "else\n";
     if (pl.vec && at >= 0) {                       // (an argument in place: its mantissas are at hand)
         o << ind << "b2_st_words(o" << k << " + c, m" << at << ", pairs" << k << ");\n";
         return;
@@ -375,6 +405,7 @@ void emit_store_always(std::ostringstream& o, const b2_ew_program& p, const Plan
         o << ind << "{ int m[V];\n"
           << ind << "  _Pragma(\"unroll\") for (int e = 0; e < V; ++e) { m[e] = b2_f32_to_i16(y" << k
           << "[e] * q" << k << ", fstat" << k << "); }\n";
+    if (pl.ragged) o << ind << "  if (there != (1u << V) - 1u) b2_st_some<V>(o" << k << " + c, m, there); else\n";
     if (planes && pl.vec)
         o << ind << "  b2_st" << pl.V << "_planes(o" << k << " + c, p.out_plane[" << k << "], m); }\n";
     else if (planes)
@@ -537,11 +568,18 @@ int generate(const b2_ew_program& p, const Plan& pl, bool probe, std::string* ou
     if (meet) o << "    __shared__ float share[2][NRED][THREADS / 32];\n    int turn = 0;\n";
     if (p.reduce_mode != B2_REDUCE_B) {
         o << "    const b2_i64 rows = p.A * p.B;\n"
-          << "    const b2_i64 chunks = p.C / V;\n"
+          << (pl.ragged ? "" : "    const b2_i64 chunks = p.C / V;\n")
           << "    const int grp = threadIdx.x / GROUP, gl = threadIdx.x % GROUP;\n"
           << "    const int RPC = THREADS / GROUP;\n"
           << "    for (b2_i64 r = block_y * RPC + grp; r < rows; r += blocks_y * RPC) {\n"
           << "        const b2_i64 a_idx = r / p.B, b_idx = r - a_idx * p.B;\n";
+        if (pl.ragged) {
+            // every full tensor's row starts `ahead` elements behind a vector
+            const std::string f = full_tensor(p);
+            o << "        const int ahead = (int)((a_idx * p." << f.substr(0, f.find('[')) << "_sa" << f.substr(f.find('[')) << " + b_idx * p."
+              << f.substr(0, f.find('[')) << "_sb" << f.substr(f.find('[')) << ") & (V - 1));\n"
+              << "        const b2_i64 chunks = (ahead + p.C + V - 1) / V;\n";
+        }
         for (int i = 0; i < p.n_in; ++i) {
             const char* ct = ctype(p.in[i].dtype);
             o << "        const " << ct << "* in" << i << " = " << input_pointer(p, i)
@@ -577,7 +615,11 @@ int generate(const b2_ew_program& p, const Plan& pl, bool probe, std::string* ou
             o << "        }\n";
         }
         o << "        for (; j < chunks; j += jstep) {\n"
-          << "            const b2_i64 c = j * V;\n";
+          << "            const b2_i64 c = j * V" << (pl.ragged ? " - ahead" : "") << ";\n";
+        if (pl.ragged)
+            o << "            unsigned there = (1u << V) - 1u;\n"
+              << "            if (c < 0) there &= there << (int)-c;\n"
+              << "            if (c + V > p.C) there &= (1u << (int)(p.C - c)) - 1u;\n";
         if (pl.prefetch) {
             o << "            if (j + jstep < chunks) {\n";
             emit_raw_loads(o, p, pl, "n", "j + jstep", "                ");
@@ -587,6 +629,12 @@ int generate(const b2_ew_program& p, const Plan& pl, bool probe, std::string* ou
         }
         emit_loads(o, p, pl, "            ");
         for (int k = 0; k < p.n_out; ++k) o << "            float y" << k << "[V];\n";
+        // Sums of few lanes: a vector's values by twos first, so that what a lane adds one after another is a value per
+        // vector (against 64 bits, eight sizes, rows of 121 to 13233: 0.97 of the error of one value to a thread and a
+        // block to a row, geometric mean; the largest 1.04, 8.6e-8 -> 8.9e-8).
+        auto by_twos = [&](int k) { return p.out[k].redop == B2_RED_SUM && (pl.ragged || (pl.vec && pl.group == 32 && p.C / pl.V > 64)); };
+        for (int k = p.n_out; k < nres; ++k)
+            if (by_twos(k)) o << "            float v" << k << "[V];\n";
         o << "            _Pragma(\"unroll\") for (int e = 0; e < V; ++e) {\n";
         {
             std::ostringstream body;
@@ -594,9 +642,14 @@ int generate(const b2_ew_program& p, const Plan& pl, bool probe, std::string* ou
             o << body.str();
         }
         for (int k = 0; k < p.n_out; ++k)
-            o << "            y" << k << "[e] = " << reg(p.out[k].reg) << ";\n";
+            o << "            y" << k << "[e] = " << (pl.ragged ? "!(there >> e & 1u) ? 0.0f : " : "") << reg(p.out[k].reg) << ";\n";
         for (int k = p.n_out; k < nres; ++k) {
             const int op = p.out[k].redop;
+            if (by_twos(k)) {
+                o << "            v" << k << "[e] = " << (pl.ragged ? "!(there >> e & 1u) ? 0.0f : " : "") << reg(p.out[k].reg) << ";\n";
+                continue;
+            }
+            if (pl.ragged) o << "            if (there >> e & 1u)\n";
             if (is_arg(op))
                 o << "            b2_arg_comb<" << red_name(op) << ">(acc" << k << ", idx" << k
                   << ", " << reg(p.out[k].reg) << ", (int)(c + e));\n";
@@ -605,6 +658,11 @@ int generate(const b2_ew_program& p, const Plan& pl, bool probe, std::string* ou
                   << ", " << reg(p.out[k].reg) << ");\n";
         }
         o << "            }\n";
+        for (int k = p.n_out; k < nres; ++k)
+            if (by_twos(k))
+                o << "            _Pragma(\"unroll\") for (int h = V / 2; h > 0; h /= 2)\n"
+                  << "                _Pragma(\"unroll\") for (int e = 0; e < h; ++e) v" << k << "[e] += v" << k << "[e + h];\n"
+                  << "            acc" << k << " += v" << k << "[0];\n";
         for (int k = 0; k < p.n_out; ++k) emit_store(o, p, pl, k, probe, "            ");
         if (pl.prefetch)
             for (int i = 0; i < p.n_in; ++i)
@@ -925,6 +983,25 @@ bool vector_ok(const b2_ew_program& p, int V) {
     return true;
 }
 
+// Rows of full tensors that are the same distance apart start on the same place within a vector: all of a row but its
+// ends is read and stored in vectors though its length or distance is no multiple of one.  Not worth it for rows whose
+// ends are much of them, nor for so little work that one value to a thread keeps the machine half empty.  One
+// B200, us a launch, one value to a thread -> vectors: flex16 333 x 1001 13.0 -> 6.5, 8192 x 16383
+// 995 -> 392, 7013 x 73 35.4 -> 17.0, 8192 x 3001 209 -> 114, fp32 1500 x 16001 206 -> 108, 4415 x 121 21.6 -> 7.5.
+bool ragged_ok(const b2_ew_program& p) {
+    const b2_ew_tensor* full = nullptr;
+    auto ok = [&](const b2_ew_tensor& t) {
+        if (t.sc == 0) return true;
+        if (t.sc != 1 || t.dtype == B2_FLEX16_PLANES) return false;
+        if (!full) full = &t;
+        return t.sa == full->sa && t.sb == full->sb;
+    };
+    if (p.reduce_mode == B2_REDUCE_B) return false;
+    for (int i = 0; i < p.n_in; ++i) if (!ok(p.in[i])) return false;
+    for (int k = 0; k < p.n_out; ++k) if (p.out[k].t.sc != 1 || !ok(p.out[k].t)) return false;
+    return full && p.C >= 64 && (long long)p.A * p.B * p.C >= 64 * 1024;
+}
+
 Plan make_plan(const b2_ew_program& p, bool want_vec) {
     Plan pl;
     bool any16 = false;
@@ -935,9 +1012,10 @@ Plan make_plan(const b2_ew_program& p, bool want_vec) {
     if (want_vec) {
         if (any16 && vector_ok(p, 8)) { pl.V = 8; pl.vec = true; }
         else if (vector_ok(p, 4)) { pl.V = 4; pl.vec = true; }
+        else if (ragged_ok(p)) { pl.V = any16 ? 8 : 4; pl.vec = pl.ragged = true; }
     }
     const long long rows = p.A * p.B;
-    const long long chunks = p.C / pl.V;
+    const long long chunks = (p.C + (pl.ragged ? pl.V : 0)) / pl.V;
     const int wave = kSMs * 8;
     if (p.reduce_mode == B2_REDUCE_NONE) {
         long long gx = (chunks + kThreads - 1) / kThreads;
@@ -952,7 +1030,11 @@ Plan make_plan(const b2_ew_program& p, bool want_vec) {
     } else if (p.reduce_mode == B2_REDUCE_C) {
         bool has_arg = false;
         for (int k = p.n_out; k < p.n_out + p.n_red; ++k) has_arg |= is_arg(p.out[k].redop);
-        if (chunks <= 64) {
+        // A warp to a row where that gives the machine warps enough: no barrier between a row and the next, and short
+        // rows do not leave most of a block idle (one B200, us a launch, a block to a row -> a warp: flex16 6709 x 930
+        // 59.0 -> 35.4, 1000 x 800 7.9 -> 6.8, 2551 x 2254 39.2 -> 33.9, 8192 x 3001 114 -> 107; fp32 4222 x 336 13.5 ->
+        // 6.8).
+        if (chunks <= 64 || (rows >= 1000 && chunks <= 512)) {
             pl.group = 32;
             long long gy = (rows + 7) / 8;
             if (gy > 65535) gy = 65535;
@@ -979,7 +1061,7 @@ Plan make_plan(const b2_ew_program& p, bool want_vec) {
     }
     {
         const char* pf = getenv("B2_EW_PREFETCH");
-        pl.prefetch = pf && pf[0] == '1';
+        pl.prefetch = pf && pf[0] == '1' && !pl.ragged;
     }
     {
         const char* mb = getenv("B2_EW_MINB");
@@ -992,7 +1074,7 @@ Plan make_plan(const b2_ew_program& p, bool want_vec) {
     const bool allow = env && env[0] == '1';   // off by default: measured slower than plain loads
     bool at = false;
     for (int i = 0; i < p.n_in; ++i) at |= p.in[i].dtype == B2_F32_AT || p.in[i].dtype == B2_FLEX16_AT;
-    if (allow && !at && pl.vec && p.reduce_mode != B2_REDUCE_B && pl.group == kThreads &&
+    if (allow && !at && pl.vec && !pl.ragged && p.reduce_mode != B2_REDUCE_B && pl.group == kThreads &&
         rows < (1LL << 30) && chunks < (1LL << 30)) {
         int bytes = 0;
         for (int i = 0; i < p.n_in; ++i)

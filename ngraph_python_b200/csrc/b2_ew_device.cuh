@@ -174,6 +174,54 @@ __device__ __forceinline__ int2 b2_mantissas(const float4& w, bool fp, float inv
     if (!fp) return make_int2(__float_as_int(w.x), __float_as_int(w.y));
     return make_int2(b2_as_stored2(w.x, w.y, inv), b2_as_stored2(w.z, w.w, inv));
 }
+// Vectors at the ends of rows that do not start or end on a vector: bit e of `there` says that element e belongs to
+// the row.  Others are not touched and count as zero.
+__device__ __forceinline__ float b2_some(const float* p, int e, unsigned there) { return there >> e & 1u ? p[e] : 0.0f; }
+__device__ __forceinline__ int b2_some2(const short* p, int e, unsigned there) {
+    const unsigned lo = there >> e & 1u ? (unsigned short)p[e] : 0u, hi = there >> (e + 1) & 1u ? (unsigned short)p[e + 1] : 0u;
+    return (int)(lo | hi << 16);
+}
+__device__ __forceinline__ void b2_ldraw_some(const float* p, unsigned there, float4& w) {
+    w = make_float4(b2_some(p, 0, there), b2_some(p, 1, there), b2_some(p, 2, there), b2_some(p, 3, there));
+}
+__device__ __forceinline__ void b2_ldraw_some(const float* p, unsigned there, b2_f8& w) {
+    b2_ldraw_some(p, there, w.a);
+    b2_ldraw_some(p + 4, there >> 4, w.b);
+}
+__device__ __forceinline__ void b2_ldraw_some(const short* p, unsigned there, int2& w) {
+    w = make_int2(b2_some2(p, 0, there), b2_some2(p, 2, there));
+}
+__device__ __forceinline__ void b2_ldraw_some(const short* p, unsigned there, int4& w) {
+    w = make_int4(b2_some2(p, 0, there), b2_some2(p, 2, there), b2_some2(p, 4, there), b2_some2(p, 6, there));
+}
+__device__ __forceinline__ void b2_ldraw_at_some(const float* p, const short* m, bool fp, unsigned there, b2_f8& w) {
+    if (fp) {
+        b2_ldraw_some(p, there, w);
+    } else {
+        int4 t;
+        b2_ldraw_some(m, there, t);
+        w.a = make_float4(__int_as_float(t.x), __int_as_float(t.y), __int_as_float(t.z), __int_as_float(t.w));
+    }
+}
+__device__ __forceinline__ void b2_ldraw_at_some(const float* p, const short* m, bool fp, unsigned there, float4& w) {
+    if (fp) {
+        b2_ldraw_some(p, there, w);
+    } else {
+        int2 t;
+        b2_ldraw_some(m, there, t);
+        w.x = __int_as_float(t.x); w.y = __int_as_float(t.y);
+    }
+}
+template <int N> __device__ __forceinline__ void b2_st_some(float* p, const float* v, unsigned there) {
+#pragma unroll
+    for (int e = 0; e < N; ++e)
+        if (there >> e & 1u) p[e] = v[e];
+}
+template <int N> __device__ __forceinline__ void b2_st_some(short* p, const int* w, unsigned there) {
+#pragma unroll
+    for (int e = 0; e < N; ++e)
+        if (there >> e & 1u) p[e] = (short)(w[e >> 1] >> 16 * (e & 1));
+}
 __device__ __forceinline__ void b2_cvt(const float4& w, float* v, float) {
     v[0] = w.x; v[1] = w.y; v[2] = w.z; v[3] = w.w;
 }
@@ -243,6 +291,16 @@ __device__ __forceinline__ void b2_st_words(short* p, const int4& w, b2_pairs& s
 }
 __device__ __forceinline__ void b2_st_words(short* p, const int2& w, b2_pairs& s) {
     __stcs(reinterpret_cast<int2*>(p), w);
+    b2_follow(s, w.x); b2_follow(s, w.y);
+}
+__device__ __forceinline__ void b2_st_words_some(short* p, const int4& w, b2_pairs& s, unsigned there) {
+    const int m[4] = {w.x, w.y, w.z, w.w};
+    b2_st_some<8>(p, m, there);
+    b2_follow(s, w.x); b2_follow(s, w.y); b2_follow(s, w.z); b2_follow(s, w.w);
+}
+__device__ __forceinline__ void b2_st_words_some(short* p, const int2& w, b2_pairs& s, unsigned there) {
+    const int m[2] = {w.x, w.y};
+    b2_st_some<4>(p, m, there);
     b2_follow(s, w.x); b2_follow(s, w.y);
 }
 
