@@ -14,6 +14,7 @@ static bool within_range(const b2_direct_args& a) {
 
 long long b2_direct_cost(const b2_direct_args& a) {
     if (!within_range(a)) return -1;
+    if (b2_gather_streams(a)) return b2_gather_plan(a).cost;
     return a.flex ? direct_shape<MODE_FLEX16>(a).cost : direct_shape<MODE_F32X3>(a).cost;
 }
 
@@ -24,19 +25,35 @@ long long b2_direct_longest(const b2_direct_args& a, int* longest) {
     return s.cost;
 }
 
+long long b2_direct_own_cost(const b2_direct_args& a, int* in_one_sum) {
+    if (!within_range(a)) return -1;
+    const DirectShape s = direct_shape<MODE_F32X3>(a);
+    if (s.cost < 0) return -1;
+    const int pairs = dir_pairs(s.bn, s.groups);
+    *in_one_sum = (s.kb_per_split + pairs - 1) / pairs;
+    return s.cost;
+}
+
 int b2_direct_in_one_sum(const b2_direct_args& a) {
+    if (b2_gather_streams(a)) return b2_gather_plan(a).in_one_sum;
     const DirectShape s = direct_shape<MODE_F32X3>(a);
     const int pairs = dir_pairs(s.bn, s.groups);
     return (s.kb_per_split + pairs - 1) / pairs;
 }
 
 void b2_direct_plan(const b2_direct_args& a, b2_gemm_plan_info* plan) {
+    if (b2_gather_streams(a)) {
+        const b2_gather_info s = b2_gather_plan(a);
+        *plan = {B2_GEMM_DIRECT, s.bn, s.splits, s.waves};
+        return;
+    }
     const DirectShape s = a.flex ? direct_shape<MODE_FLEX16>(a) : direct_shape<MODE_F32X3>(a);
     *plan = {B2_GEMM_DIRECT, s.bn, s.splits, s.waves};
 }
 
 int b2_direct_launch(const b2_direct_args& a, cudaStream_t st) {
     B2_REQUIRE(b2_direct_cost(a) >= 0, "problem outside the kernel's range");
+    if (b2_gather_streams(a)) return b2_gather_launch(a, st);
     return a.flex ? b2_direct_launch_flex(a, st) : direct_launch_mode<MODE_F32X3>(a, st);
 }
 
@@ -52,7 +69,7 @@ struct StageLayout {
     unsigned char* out;
     long long b_rs, b_ks;
     b2_gather g;
-    int N, K, bn, num_kb, ntn, tiled;
+    int N, K, bn, num_kb, ntn, tiled, turned;       // turned: see b2_gather_info
 };
 struct StageJobs {
     int n, first[kStageJobs + 1];                 // job j owns blocks first[j] .. first[j+1]-1
@@ -94,16 +111,21 @@ stage_filters_kernel(const __grid_constant__ StageJobs jobs) {
             dir_split_tf32(v, hp[q], lp[q]);
         }
         unsigned char* out = f.out + (long long)block * (2 * f.bn * 128) + swz(lr, chunk);
-        *(float4*)out = h;
-        *(float4*)(out + f.bn * 128) = l;
+        const bool turn = f.turned && (kb / f.turned & 1);
+        *(float4*)out = turn ? l : h;
+        *(float4*)(out + f.bn * 128) = turn ? h : l;
     }
 }
 
 }  // namespace
 
+static int staged_tile(const b2_direct_args& a) {
+    return b2_gather_streams(a) ? b2_gather_plan(a).bn : direct_shape<MODE_F32X3>(a).bn;
+}
+
 size_t b2_direct_staged_bytes(const b2_direct_args& a) {
-    const DirectShape s = direct_shape<MODE_F32X3>(a);
-    return (size_t)((a.N + s.bn - 1) / s.bn) * ((a.K + 31) / 32) * (2 * s.bn * 128);
+    const int bn = staged_tile(a);
+    return (size_t)((a.N + bn - 1) / bn) * ((a.K + 31) / 32) * (2 * bn * 128);
 }
 
 int b2_direct_stage_filters(const b2_stage_job* list, int n, int* launches, cudaStream_t st) {
@@ -113,11 +135,10 @@ int b2_direct_stage_filters(const b2_stage_job* list, int n, int* launches, cuda
         jobs.n = n - at < kStageJobs ? n - at : kStageJobs;
         for (int j = 0; j < jobs.n; ++j) {
             const b2_direct_args& a = list[at + j].a;
-            const DirectShape s = direct_shape<MODE_F32X3>(a);
-            const int ntn = (a.N + s.bn - 1) / s.bn, num_kb = (a.K + 31) / 32;
+            const int bn = staged_tile(a), ntn = (a.N + bn - 1) / bn, num_kb = (a.K + 31) / 32;
             jobs.layout[j] = {list[at + j].filters, (unsigned char*)list[at + j].staged, a.b_rs, a.b_ks, a.g,
-                              a.N, a.K, s.bn, num_kb, ntn, filter_tiles(a)};
-            const long long blocks = ((long long)ntn * num_kb * 8 * s.bn + 255) / 256;
+                              a.N, a.K, bn, num_kb, ntn, filter_tiles(a), b2_gather_streams(a) ? b2_gather_plan(a).turned : 0};
+            const long long blocks = ((long long)ntn * num_kb * 8 * bn + 255) / 256;
             jobs.first[j + 1] = jobs.first[j] + (int)(blocks < 148 * 4 ? blocks : 148 * 4);
         }
         B2_CUDA(b2::launch_after(stage_filters_kernel, dim3(jobs.first[jobs.n]), 256, 0, st, jobs));

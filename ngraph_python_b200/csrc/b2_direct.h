@@ -61,6 +61,8 @@ constexpr int kClusterCtas[9] = {0, 148, 148, 135, 132, 130, 132, 105, 120};
 __attribute__((visibility("hidden"))) long long b2_direct_cost(const b2_direct_args& a);
 // The same for one group of producers and one pair of sums, and the k-blocks that then go into one sum.
 __attribute__((visibility("hidden"))) long long b2_direct_longest(const b2_direct_args& a, int* longest);
+// Cost in that kernel also where the one of b2_gather.cu would take the product, and the k-blocks in one sum.
+__attribute__((visibility("hidden"))) long long b2_direct_own_cost(const b2_direct_args& a, int* in_one_sum);
 // ... that do so in the shape taken.
 __attribute__((visibility("hidden"))) int b2_direct_in_one_sum(const b2_direct_args& a);
 __attribute__((visibility("hidden"))) void b2_direct_plan(const b2_direct_args& a, b2_gemm_plan_info* plan);
@@ -79,6 +81,14 @@ __attribute__((visibility("hidden"))) bool b2_product_streams(const b2_direct_ar
 __attribute__((visibility("hidden"))) long long b2_stream_cost(const b2_direct_args& a);
 __attribute__((visibility("hidden"))) void b2_stream_plan(const b2_direct_args& a, b2_gemm_plan_info* plan);
 __attribute__((visibility("hidden"))) int b2_stream_launch(const b2_direct_args& a, cudaStream_t st);
+
+// Gathered products whose filters are laid out beforehand (b2_gather.cu): whether it takes one rather than the kernel
+// above, its cost and shape (tile, slices, waves, k-blocks in one sum), and the launch.  K-block n has its planes in the
+// other order where `turned` is not 0 and n / turned odd.
+struct b2_gather_info { long long cost; int bn, splits, waves, in_one_sum, turned; };
+__attribute__((visibility("hidden"))) bool b2_gather_streams(const b2_direct_args& a);
+__attribute__((visibility("hidden"))) b2_gather_info b2_gather_plan(const b2_direct_args& a);
+__attribute__((visibility("hidden"))) int b2_gather_launch(const b2_direct_args& a, cudaStream_t st);
 
 // fp32 filter gradient (b2_conv_update_f32.cu): no dilation, one depth.  Scratch 0: not taken.
 struct b2_update_f32 { int C, H, W, N, K, R, S, P, Q, pad_h, pad_w, str_h, str_w; };
