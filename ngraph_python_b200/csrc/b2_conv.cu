@@ -218,35 +218,32 @@ inline bool conv_goes_direct(int mode, const ConvGeom& g, int pass, b2_direct_ar
 inline bool conv_goes_staged(const ConvGeom& g, int pass, b2_direct_args* out) {
     b2_direct_args d;
     if (!conv_goes_direct(MODE_F32X3, g, pass, &d)) return false;
-    const long long unstaged = b2_direct_cost(d);
+    long long best = b2_direct_cost(d);
     const SumBound bound = sum_bound(MODE_F32X3, g, pass);
-    auto search = [&](bool own, int longest, long long best, int* in_one_sum) {
+    auto search = [&](bool own, int longest) {
         bool found = false;
         for (int a = 1; a <= 4; ++a)
             for (int b = 1; b <= 4; ++b) {
                 if (!direct_args(MODE_F32X3, g, pass, pass ? a * g.str_h : a, pass ? b * g.str_w : b, &d) || !bound.allows(d)) continue;
                 d.longest = longest;
                 d.staged = &d;                    // (there will be such)
-                int n = 0;
-                const long long cost = own ? b2_direct_own_cost(d, &n) : b2_direct_cost(d);
+                d.staged_own = own;
+                const long long cost = b2_direct_cost(d);
                 if (cost < 0 || cost >= best) continue;
                 best = cost;
                 found = true;
-                if (own) { *in_one_sum = n; continue; }
                 *out = d;
                 out->staged = out;
             }
         return found;
     };
-    int longest = bound.longest;
-    if (g.N % 4 == 0) {
-        // The kernel of b2_gather.cu does not put more k-blocks into one sum than the one of b2_direct.cuh, in the tile and
-        // shape that it would take (against 64 bits, 160 layers and passes, batch 4 to 256: 0.976 of its
-        // error, geometric mean, the largest 1.07; without the bound 1.02 and 1.64).
-        b2_direct_own_cost(d, &longest);
-        search(true, bound.longest, unstaged, &longest);
-    }
-    return search(false, longest, unstaged, nullptr);
+    // The kernel of b2_gather.cu, where it takes less, does not put more k-blocks into one sum than the one of
+    // b2_direct.cuh in the tile and shape that it would take (against 64 bits, 172 layers and passes, batch 4 to 256:
+    // 0.998 of its error, geometric mean, the largest 1.08; without the bound 1.02 and 1.64).
+    b2_direct_args without = d;
+    const bool own = search(true, bound.longest);
+    const bool gathers = g.N % 4 == 0 && search(false, b2_direct_in_one_sum(own ? *out : without));
+    return own || gathers;
 }
 
 inline int launch_direct(b2_direct_args& d, const void* A, const void* B, void* C,

@@ -25,15 +25,6 @@ long long b2_direct_longest(const b2_direct_args& a, int* longest) {
     return s.cost;
 }
 
-long long b2_direct_own_cost(const b2_direct_args& a, int* in_one_sum) {
-    if (!within_range(a)) return -1;
-    const DirectShape s = direct_shape<MODE_F32X3>(a);
-    if (s.cost < 0) return -1;
-    const int pairs = dir_pairs(s.bn, s.groups);
-    *in_one_sum = (s.kb_per_split + pairs - 1) / pairs;
-    return s.cost;
-}
-
 int b2_direct_in_one_sum(const b2_direct_args& a) {
     if (b2_gather_streams(a)) return b2_gather_plan(a).in_one_sum;
     const DirectShape s = direct_shape<MODE_F32X3>(a);

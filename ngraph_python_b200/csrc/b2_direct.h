@@ -29,6 +29,7 @@ struct b2_direct_args {
     const void *A, *B;
     // gathered fp32 rows: B's k-blocks as the kernel's stages hold them (b2_direct_stage_filters), or NULL
     const void* staged;
+    int staged_own;                  // ... for the kernel of b2_direct.cuh, whatever b2_gather.cu makes of it
     // Gathered fp32 rows: the most k-blocks that may go into one sum (0: any).  The tensor core's sum loses
     // bits with every one, and a cheaper shape is not to lose more than callers of a layer have had: the bound
     // is what the shape of one group of producers and one pair of sums, filters as they lie, adds up in one go
@@ -61,8 +62,6 @@ constexpr int kClusterCtas[9] = {0, 148, 148, 135, 132, 130, 132, 105, 120};
 __attribute__((visibility("hidden"))) long long b2_direct_cost(const b2_direct_args& a);
 // The same for one group of producers and one pair of sums, and the k-blocks that then go into one sum.
 __attribute__((visibility("hidden"))) long long b2_direct_longest(const b2_direct_args& a, int* longest);
-// Cost in that kernel also where the one of b2_gather.cu would take the product, and the k-blocks in one sum.
-__attribute__((visibility("hidden"))) long long b2_direct_own_cost(const b2_direct_args& a, int* in_one_sum);
 // ... that do so in the shape taken.
 __attribute__((visibility("hidden"))) int b2_direct_in_one_sum(const b2_direct_args& a);
 __attribute__((visibility("hidden"))) void b2_direct_plan(const b2_direct_args& a, b2_gemm_plan_info* plan);

@@ -511,7 +511,7 @@ int gather_launch_bn(const GatherParams& p, cudaStream_t st) {
 
 // Images of a pixel in fours: sixteen bytes a copy.
 bool b2_gather_streams(const b2_direct_args& a) {
-    return a.staged && !a.flex && a.a_kind == B2_OPERAND_GATHER && a.colmajor && a.g.N % 4 == 0;
+    return a.staged && !a.staged_own && !a.flex && a.a_kind == B2_OPERAND_GATHER && a.colmajor && a.g.N % 4 == 0;
 }
 
 b2_gather_info b2_gather_plan(const b2_direct_args& a) {
