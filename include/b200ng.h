@@ -282,7 +282,8 @@ int b2_flex_end_call(const b2_flex_state* s, int32_t n, const int64_t* ids, cons
  * ------------------------------------------------------------------------------------------ */
 int b2_gemm_scratch_bytes(int32_t flex, int32_t M, int32_t N, int32_t K, size_t* bytes);
 /* Kernels one product launches: 1 where its operands are converted on the way in, else the operand
- * planes and the tile kernel (K strides as below, operands dense along the other side). */
+ * planes and the tile kernel (K strides as below; for rows along K that start anywhere: where they start on
+ * sixteen bytes some more products take one launch). */
 int b2_gemm_launches(int32_t flex, int64_t a_k_stride, int64_t b_k_stride, int32_t M, int32_t N,
                      int32_t K, int32_t* launches);
 /* Which kernel that is, and how it cuts the product: tile_n columns to a tile, K in `slices` parts that

@@ -42,7 +42,7 @@ inline long long plane_cost(int mode, const Shapes& s, int M, int N, int K) {
 // arguments: the cheaper of C and its transpose, so that a product with few rows does not pad them to
 // a whole tile.
 inline bool gemm_goes_direct(int mode, const void* A, long long a_rs, long long a_cs, const void* B,
-                             long long b_ks, long long b_ns, int M, int N, int K, b2_direct_args* out) {
+                             long long b_ks, long long b_ns, int M, int N, int K, b2_direct_args* out, bool may_stream = true) {
     b2_direct_args d = {};
     d.flex = mode == MODE_FLEX16;
     d.A = A; d.a_rs = a_rs; d.a_ks = a_cs; d.a_kind = a_cs == 1 ? B2_OPERAND_K : B2_OPERAND_ROWS;
@@ -52,15 +52,15 @@ inline bool gemm_goes_direct(int mode, const void* A, long long a_rs, long long 
     t.A = d.B; t.a_rs = d.b_rs; t.a_ks = d.b_ks; t.a_kind = d.b_kind;
     t.B = d.A; t.b_rs = d.a_rs; t.b_ks = d.a_ks; t.b_kind = d.a_kind;
     t.M = N; t.N = M; t.colmajor = 1;
-    const bool streams = b2_product_streams(d);                   // (the same for C's transpose)
+    const bool streams = may_stream && b2_product_streams(d);     // (the same for C's transpose)
     const long long cd = streams ? b2_stream_cost(d) : b2_direct_cost(d), ct = streams ? b2_stream_cost(t) : b2_direct_cost(t);
     const long long plane = plane_cost(mode, shapes_for(mode, M, N, K), M, N, K);
     const bool swap = ct >= 0 && (cd < 0 || ct < cd);
     *out = swap ? t : d;
     long long best = swap ? ct : cd;
-    // (near the line the planes are the faster ones: flex16 2692 x 688 x 640 16.4 us, 18.2 in one launch, 500 x 500 x 6000
-    // transposed 19.6 and 21.3)
-    if (streams && mode == MODE_FLEX16) best += best / 8;
+    // (many k-blocks in few slices: flex16 500 x 500 x 6000, the second operand along K, 19.7 us on planes, 21.6 in one
+    // launch)
+    if (streams && mode == MODE_FLEX16 && K > 4096 && M > 256 && N > 256) best += best / 8;
     // Both operands contiguous along their rows take longer than the direct kernel's own choice of a shape has to
     // know: fp32 638 x 937 x 631 26 us against 20 on planes, 383 x 3300 x 1440 47 and 39 (two k-blocks or less
     // don't: 1869 x 1337 x 46 20 and 26); flex16 an odd number of values apart, loaded one by one, 249 x 1831 x
@@ -80,18 +80,22 @@ int run_gemm(const T* A, long long a_rs, long long a_cs, const T* B, long long b
     B2_REQUIRE(A && B && C && M > 0 && N > 0 && K > 0, "bad GEMM argument");
     B2_REQUIRE(a_rs == 1 || a_cs == 1, "A must be contiguous along M or K");
     B2_REQUIRE(b_ks == 1 || b_ns == 1, "B must be contiguous along K or N");
+    const Shapes s = shapes_for(MODE, M, N, K);
+    const size_t need = gemm_scratch_need(MODE, s);
+    const bool room = scratch && scratch_bytes >= need && ((uintptr_t)scratch & 1023) == 0;
     b2_direct_args d;
-    if (gemm_goes_direct(MODE, A, a_rs, a_cs, B, b_ks, b_ns, M, N, K, &d)) {
+    // (what needs scratch does not change with the kernels' measurements: without it one launch takes what
+    // b2_direct.cuh's kernel would be chosen for)
+    if (!room)
+        B2_REQUIRE(gemm_goes_direct(MODE, A, a_rs, a_cs, B, b_ks, b_ns, M, N, K, &d, false),
+                   "GEMM needs %zu bytes of 1024-byte aligned scratch, got %zu", need, scratch_bytes);
+    if (gemm_goes_direct(MODE, A, a_rs, a_cs, B, b_ks, b_ns, M, N, K, &d) || !room) {
         d.C = C; d.ldc = ldc; d.table = table; d.slotC = slotC;
         d.slotA = d.colmajor ? slotB : slotA; d.slotB = d.colmajor ? slotA : slotB;
         d.stats = stats; d.probe_out = probe_out; d.status = status; d.probe = probe;
         return b2_product_streams(d) ? b2_stream_launch(d, st) : b2_direct_launch(d, st);
     }
-    const Shapes s = shapes_for(MODE, M, N, K);
     const int splits = pick_splits(MODE, s, false);     // > 1 only for flex16 with K > 32768
-    const size_t need = gemm_scratch_need(MODE, s);
-    B2_REQUIRE(scratch && scratch_bytes >= need && ((uintptr_t)scratch & 1023) == 0,
-               "GEMM needs %zu bytes of 1024-byte aligned scratch, got %zu", need, scratch_bytes);
     unsigned char* base = (unsigned char*)scratch;
     const size_t a_plane = (size_t)s.Mp * s.Kp * s.esize, b_plane = (size_t)s.Np * s.Kp * s.esize;
     void* A0 = base; void* A1 = base + a_plane;
@@ -132,7 +136,7 @@ extern "C" int b2_gemm_launches(int32_t flex, int64_t a_k_stride, int64_t b_k_st
     B2_REQUIRE(launches && M > 0 && N > 0 && K > 0, "bad argument");
     const int mode = flex ? MODE_FLEX16 : MODE_F32X3;
     b2_direct_args d;
-    *launches = gemm_goes_direct(mode, nullptr, a_k_stride == 1 ? K : 1, a_k_stride, nullptr, b_k_stride, b_k_stride == 1 ? K : 1, M, N, K, &d) ? 1
+    *launches = gemm_goes_direct(mode, nullptr, 1, a_k_stride, nullptr, b_k_stride, 1, M, N, K, &d) ? 1
                 : pick_splits(mode, shapes_for(mode, M, N, K), false) > 1 ? 3 : 2;
     return B2_OK;
 }
@@ -142,7 +146,7 @@ extern "C" int b2_gemm_plan(int32_t flex, int64_t a_k_stride, int64_t b_k_stride
     B2_REQUIRE(plan && M > 0 && N > 0 && K > 0, "bad argument");
     const int mode = flex ? MODE_FLEX16 : MODE_F32X3;
     b2_direct_args d;
-    if (gemm_goes_direct(mode, nullptr, a_k_stride == 1 ? K : 1, a_k_stride, nullptr, b_k_stride, b_k_stride == 1 ? K : 1, M, N, K, &d)) {
+    if (gemm_goes_direct(mode, nullptr, 1, a_k_stride, nullptr, b_k_stride, 1, M, N, K, &d)) {
         if (b2_product_streams(d)) b2_stream_plan(d, plan);
         else b2_direct_plan(d, plan);
         return B2_OK;

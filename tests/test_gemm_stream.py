@@ -25,3 +25,20 @@ def test_many_results_of_one_k_block():
     import torch
     _run(torch, True, "nn", 1501, 701, 100)
     _run(torch, True, "tn", 1500, 600, 128)
+
+
+def test_products_without_scratch():
+    """What one launch did without scratch it still does; what needed it is refused."""
+    import torch
+    from ngraph_python_b200 import lib
+    status = torch.zeros((1,), dtype=torch.int32, device="cuda")
+    for M, N, K, taken in ((64, 130, 129, True), (512, 128, 784, True), (300, 40, 2048, True), (4097, 4098, 32, False)):
+        a, b = torch.randn((M, K), device="cuda"), torch.randn((K, N), device="cuda")
+        c = torch.zeros((M, N), device="cuda")
+        rc = lib.raw().b2_gemm_f32(a.data_ptr(), K, 1, b.data_ptr(), N, 1, c.data_ptr(), N, M, N, K, None, 0,
+                                   status.data_ptr(), 0)
+        torch.cuda.synchronize()
+        assert (rc == 0) == taken
+        if taken:
+            torch.testing.assert_close(c.double(), a.double() @ b.double(), rtol=1e-4, atol=1e-5 * K ** 0.5 * 4)
+    assert int(status.item()) == 0
