@@ -19,8 +19,8 @@
 // What bounds it: chains of instructions.  Start and first columns 4400 cycles, a k-block 700 to 1000 (a slot of tensor
 // memory is filled, announced, multiplied and given back in 1400, there are two or three), the epilogue 2000 for eight
 // columns of a warp; without any loads of A or B the launches take 0.89 of their time, with a quarter of the MMAs 0.90.
-// One B200, fp32 ResNet-20, kernels of b2_direct.cuh -> this one, us: 22 layers at batch 100 266 -> 235 (a call 354 ->
-// 300), forward and input gradients at batch 256 1000 -> 860; of its epilogue the one with a branch a term took 1.4 times
+// One B200, fp32 ResNet-20, kernels of b2_direct.cuh -> this one, us: 22 layers at batch 100 266 -> 239 (a call 341 ->
+// 294), forward and input gradients at batch 256 1000 -> 875; of its epilogue the one with a branch a term took 1.4 times
 // as long in training.
 #include "b2_stream.cuh"
 
