@@ -422,6 +422,8 @@ class Computation(object):
         def replay():
             for s in refreshable:
                 s.refresh(t)          # cached operand planes of tensors that changed since
+            if self._io is not None:
+                self._io.before_replay()
             for seg in segments:
                 for k in seg["wait"]:
                     ar.wait_for(k)
@@ -475,6 +477,7 @@ class _CallIO(object):
         self.inputs = (lib.CallInput * max(1, len(views)))()
         self.pageable = (ctypes.c_void_p * max(1, len(views)))()     # ... arguments, while a call takes them in
         self.launches = ctypes.c_int32()
+        self.taken = False          # this call's arguments are in, addresses of those read in place included
         self.args = [(k, v.buffer, self.block.arg[k], v.buffer.where is not None)
                      for k, v in enumerate(views)]
         self.table_rows = t._table_host.shape[0] if t.flex else 0
@@ -529,7 +532,15 @@ class _CallIO(object):
         def taken():
             lib.check(take(*fixed, stream_of(device)))
             t.kernel_launches += self.launches.value
+            self.taken = True
         self.take = taken
+
+    def before_replay(self):
+        """The step list is about to run.  Not by a call with arguments of its own: what is read in place are
+        the arguments' tensors, not those of a caller who is gone."""
+        if not self.taken and any(read_in_place for _, _, _, read_in_place in self.args):
+            self.take()             # (no argument has an address: the tensors' own)
+        self.taken = False
 
     def ready(self):
         """False while an argument has no exponent yet: its range has to be measured first."""
@@ -607,6 +618,7 @@ class _CallIO(object):
             for k, _, arg, _ in self.args:
                 arg.src = self.pageable[k] = None
             block.table_rows = 0
+            self.taken = False
         return comp._results([
             t._finish_host(p) if r is None else t._as_result(*r)
             for p, r in zip(pending, self.results)])
