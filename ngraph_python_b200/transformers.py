@@ -605,12 +605,14 @@ class _CallIO(object):
                     arg.inv_scale = math.ldexp(1.0, buf.entry.dec)
             if self.flex_buffers:
                 t._inputs_written = list(self.flex_buffers)
-            self.take()
             try:
+                self.take()                    # (one launch or several)
                 comp.executor()
                 pending = [None if r is not None else t._device_to_host_async(v)
                            for r, v in zip(self.results, comp.return_views)]
             except BaseException:
+                if block.table_rows:
+                    t._table_dirty = True      # (the scale rows may not be there)
                 t.stream.synchronize()         # (the arguments may still be being read)
                 raise
             t._end_call(comp)
