@@ -219,7 +219,9 @@ int b2_flex_publish(int32_t* stats, int32_t n, const int32_t* status, int32_t* h
  * b2_call_take does the same in front of the step list instead of inside it: the block (any host memory)
  * is read by the call itself, and pageable[k], unless pageable or that is NULL, is host memory that is first copied
  * to the pinned block at arg[k].src, in pieces that the device reads while the next is copied.
- * *launches gets how many kernels that took (none where there is nothing to copy).
+ * *launches gets how many kernels that took (none where there is nothing to copy and no word or row to set).
+ * holds, unless NULL: a host word with what `where` holds, kept by b2_call_take alone (NULL in it: not known); a
+ * device word that holds its address already is not written again.
  * b2_call_outputs is b2_flex_publish with results: dst[k] (pinned host memory) <- bytes[k] bytes of
  * src[k], both 16-byte aligned.
  * b2_call_stage: the address at which the device can read `bytes` bytes of host memory at src:
@@ -235,7 +237,7 @@ typedef struct b2_call_block {
     const b2_flex_scale* table; int32_t table_rows; int32_t reserved;
     b2_call_arg arg[B2_CALL_MAX_INPUTS];
 } b2_call_block;
-typedef struct b2_call_input { void* dst; int64_t n; int32_t flex_slot; int32_t reserved; const void** where; } b2_call_input;
+typedef struct b2_call_input { void* dst; int64_t n; int32_t flex_slot; int32_t reserved; const void** where; const void** holds; } b2_call_input;
 typedef struct b2_call_output { const void* src; void* dst; int64_t bytes; } b2_call_output;
 int b2_call_inputs(const b2_call_input* inputs, int32_t n, const b2_call_block* block,
                    b2_flex_scale* table, int32_t* stats, void* stream);

@@ -16,10 +16,11 @@
 // only what is to be copied has blocks, and it runs while the launch of the graph is on its way (8 to
 // 10 us from the call to the first node); pageable memory goes through the pinned block in pieces, each
 // read by the device while the host copies the next.  As the graph's first node (b2_call_inputs) every block
-// reads its addresses from pinned memory first, 1184 of them where nothing is copied.  A call, first node ->
-// in front, one B200: 333 x 1001 flex16 values from the device 50 -> 34 us; 8192 x 16384 read in place by
-// their kernel, flex16 / fp32 373 -> 355 / 538 -> 515 us; 400 KB pageable and 22 launches 157 -> 149 us; 3 MB
-// pinned and a run of layers 248 -> 244 us.  (The last results' stores, below, are part of that.)
+// reads its addresses from pinned memory first, and the host has one launch less: the better way for few
+// values (16 x 64 fp32 18.7 us a call, 21.2 in front).  A call, first node -> in front, one B200 under a host
+// that launches slowly / quickly: 128 x 1000 fp32 values from the device 35 -> 24 / 26 -> 23 us, 400 KB pageable
+// and 22 launches 149 -> 141, 3 MB pinned and a run of layers 249 -> 241 / 239 -> 242; 8192 x 16384 read in
+// place by their kernel, flex16 / fp32 373 -> 355 / 538 -> 515.
 #include <cmath>
 #include <cstddef>
 #include <cstring>
@@ -157,6 +158,18 @@ cudaError_t launch_inputs(Inputs& a, const b2_call_block* block, b2_flex_scale* 
     return cudaGetLastError();
 }
 
+// Words alone: few parameters, which the host writes sooner (333 x 1001 values from another device tensor in every call
+// 26.3 us with the launch above, 25.7 with this one, 22.8 where the word holds the address already).
+struct Words {
+    static constexpr int kMost = 4;
+    int n;
+    const void** where[kMost];
+    const void* address[kMost];
+};
+__global__ void k_call_words(const Words w) {
+    if (threadIdx.x < w.n) *w.where[threadIdx.x] = w.address[threadIdx.x];
+}
+
 struct Outputs {
     int n;
     b2_call_output out[B2_CALL_MAX_OUTPUTS];
@@ -270,6 +283,7 @@ extern "C" int b2_call_take(const b2_call_input* inputs, int32_t n, const b2_cal
     // 50 GB/s: less than 192 KB (10 us of copying, 4 of reading) is not worth another launch.
     const long long least = 48 << 10;                          // values
     Inputs a = {};
+    const void** holds[B2_CALL_MAX_INPUTS];
     a.rows = block->table;
     a.n_rows = block->table_rows > 0 ? block->table_rows : 0;
     for (int k = 0; k < n; ++k) {
@@ -277,8 +291,14 @@ extern "C" int b2_call_take(const b2_call_input* inputs, int32_t n, const b2_cal
         const void* src = block->arg[k].src;
         if (!inputs[k].where) continue;
         // (where there is nothing to copy the values are in their place)
+        const void* address = src && block->arg[k].in_place ? src : inputs[k].dst;
+        if (inputs[k].holds) {
+            if (*inputs[k].holds == address) continue;
+            *inputs[k].holds = nullptr;                        // (until the launch is on its way)
+        }
         a.where[a.n_words] = inputs[k].where;
-        a.address[a.n_words++] = src && block->arg[k].in_place ? src : inputs[k].dst;
+        a.address[a.n_words] = address;
+        holds[a.n_words++] = inputs[k].holds;
     }
     auto add = [&](const b2_call_input& in, const b2_call_arg& arg, long long first, long long count) {
         a.in[a.n] = in;
@@ -288,8 +308,18 @@ extern "C" int b2_call_take(const b2_call_input* inputs, int32_t n, const b2_cal
         a.inv[a.n++] = arg.inv_scale;
     };
     auto launch = [&]() -> cudaError_t {
-        const cudaError_t e = launch_inputs(a, nullptr, table, stats, (cudaStream_t)stream);
+        cudaError_t e;
+        if (a.n || a.n_rows || a.n_words > Words::kMost) {
+            e = launch_inputs(a, nullptr, table, stats, (cudaStream_t)stream);
+        } else {
+            Words w = {a.n_words};
+            for (int i = 0; i < w.n; ++i) { w.where[i] = a.where[i]; w.address[i] = a.address[i]; }
+            k_call_words<<<1, 32, 0, (cudaStream_t)stream>>>(w);
+            e = cudaGetLastError();
+        }
         ++*launches;
+        for (int i = 0; i < a.n_words && e == cudaSuccess; ++i)
+            if (holds[i]) *holds[i] = a.address[i];
         a.n = a.n_words = a.n_rows = 0;
         return e;
     };

@@ -112,7 +112,7 @@ class CallBlock(C.Structure):
 
 class CallInput(C.Structure):
     _fields_ = [("dst", C.c_void_p), ("n", C.c_int64), ("flex_slot", C.c_int32),
-                ("reserved", C.c_int32), ("where", C.c_void_p)]
+                ("reserved", C.c_int32), ("where", C.c_void_p), ("holds", C.c_void_p)]
 
 
 class CallOutput(C.Structure):

@@ -70,6 +70,7 @@ class Buffer(object):
         self.watched = False        # some step keeps what follows from the contents
         # planning state (per computation build)
         self.where = None           # device word: address of the values in a recorded call
+        self.where_holds = None     # ... what it holds, as far as the host knows
         self.last_write_step = -1
         self.last_read_step = -1
 
@@ -378,7 +379,7 @@ class Computation(object):
         t._allreduce = self._allreduce
         if t._allreduce is not None:
             t._allreduce.begin_call()
-        t._recording_call = False        # set once a launch in front of the graph places the arguments
+        t._recording_call = False        # set once it is settled what places the arguments
         t._recording = has_comm          # comm steps and waits: kernels only, no NCCL, no bookkeeping
         io_in_graph = False
         io = _CallIO.of(self, exchanged_apart=has_comm)
@@ -398,7 +399,7 @@ class Computation(object):
                 g = torch.cuda.CUDAGraph()
                 with torch.cuda.graph(g):
                     if io is not None and seg is segments[0]:
-                        io.record_inputs()       # the call's arguments are there before the first node
+                        io.record_inputs()       # the call's arguments are there before the first step
                         t._recording_call = True
                     for s in seg["steps"]:
                         t._launch_step(s)
@@ -449,12 +450,18 @@ builtin_sum = sum
 
 # ---------------------------------------------------------------------------------------------
 class _CallIO(object):
-    """Arguments and results of a recorded step list: a launch in front of it reads the arguments from
-    wherever they lie, pageable memory through a pinned buffer, and its last node stores small results
-    into pinned memory, so that a call is two launches and one synchronisation."""
+    """Arguments and results of a recorded step list: its first node, or a launch in front of it, reads the
+    arguments from wherever they lie, pageable memory through a pinned buffer, and its last node stores small
+    results into pinned memory, so that a call is one or two launches and one synchronisation."""
 
     STAGED_MOST = 4 << 20       # pageable arguments up to this size go through a pinned buffer
     RESULTS_MOST = 1 << 20      # results up to this many bytes are stored by the last node
+    # Arguments of this many bytes together have a launch in front of the step list, which begins while that is on its
+    # way; fewer are taken in by its first node, sooner than another launch.  One B200, us a call, first node / in front
+    # under a host that launches quickly, then one that launches slowly: 16 x 64 fp32 values from the device 18.2 / 21.5 and
+    # 20.2 / 22.8, 64 x 256 21.7 / 23.4 and 24.4 / 22.8; ResNet of one block, flex16, pinned, one image 81 / 86 and
+    # 83 / 88, sixteen (192 KB) 94 / 98 and 104 / 97; 128 x 1000 fp32 values from the device 26 / 23 and 36 / 24.
+    IN_FRONT_LEAST = 128 << 10
 
     @classmethod
     def of(cls, comp, exchanged_apart):
@@ -473,7 +480,13 @@ class _CallIO(object):
         self.lengths = [tuple(v.axes.lengths) for v in views]
         self.flex_views = [v for v in views if v.buffer.flex]
         self.flex_buffers = [v.buffer for v in self.flex_views]
-        self.block = lib.CallBlock()
+        self.in_front = (sum(4 * v.buffer.size for v in views) >= self.IN_FRONT_LEAST or
+                         any(v.buffer.where is not None for v in views))
+        # (read by the launch in front, or when the step list runs)
+        self.block_mem = torch.zeros((ctypes.sizeof(lib.CallBlock),), dtype=torch.uint8)
+        if not self.in_front:
+            self.block_mem = self.block_mem.pin_memory()
+        self.block = lib.CallBlock.from_address(self.block_mem.data_ptr())
         self.inputs = (lib.CallInput * max(1, len(views)))()
         self.pageable = (ctypes.c_void_p * max(1, len(views)))()     # ... arguments, while a call takes them in
         self.launches = ctypes.c_int32()
@@ -516,13 +529,21 @@ class _CallIO(object):
         return self.pinned[k].data_ptr()
 
     def record_inputs(self):
-        """What the launch that takes the arguments in is told about their tensors."""
+        """The step list's first node, or what the launch in front of it is told about the arguments' tensors."""
         t = self.t
         ins = self.inputs
         for k, v in enumerate(self.views):
             ins[k].dst, ins[k].n = v.buffer.ptr(), v.buffer.size
             ins[k].flex_slot = v.buffer.slot if v.buffer.flex else -1
-            ins[k].where = v.buffer.where.data_ptr() if v.buffer.where is not None else None
+            if v.buffer.where is not None:
+                ins[k].where, ins[k].holds = v.buffer.where.data_ptr(), ctypes.addressof(v.buffer.where_holds)
+        if not self.in_front:
+            lib.check(lib.raw().b2_call_inputs(
+                ins, len(self.views), ctypes.addressof(self.block), t._table.data_ptr() if t.flex else None,
+                t._stats.data_ptr() if t.flex else None, t.stream.cuda_stream))
+            t.kernel_launches += 1
+            self.take = lambda: None
+            return
         device = t.device.index
         fixed = (ctypes.addressof(ins), len(self.views), ctypes.addressof(self.block), ctypes.addressof(self.pageable),
                  t._table.data_ptr() if t.flex else None, t._stats.data_ptr() if t.flex else None,
@@ -538,7 +559,7 @@ class _CallIO(object):
     def before_replay(self):
         """The step list is about to run.  Not by a call with arguments of its own: what is read in place are
         the arguments' tensors, not those of a caller who is gone."""
-        if not self.taken and any(read_in_place for _, _, _, read_in_place in self.args):
+        if self.in_front and not self.taken and any(read_in_place for _, _, _, read_in_place in self.args):
             self.take()             # (no argument has an address: the tensors' own)
         self.taken = False
 
@@ -580,8 +601,12 @@ class _CallIO(object):
             t._stage(view, arr)
             return (buf.staging.data_ptr() if buf.flex else 0), arr
         if not self.visible.value:
-            self.pageable[k] = address
-            return self._pinned_buffer(k), arr
+            pinned = self._pinned_buffer(k)
+            if self.in_front:
+                self.pageable[k] = address             # (copied while the device reads what is there)
+            else:
+                lib.check(stage(address, arr.nbytes, pinned, self.visible))
+            return pinned, arr
         return self.visible.value, arr
 
     def call(self, args):
@@ -1821,7 +1846,7 @@ class B200Transformer(object):
         self._inputs_written = []
         self._allreduce = None      # exchange state of the computation that ran last
         self._recording = False     # a CUDA graph segment is being recorded
-        self._recording_call = False   # ... behind the launch that places a call's arguments
+        self._recording_call = False   # ... behind what places a call's arguments
         self.tracer = None
         self._io_done = False       # the replayed graph has already queued the call's read-back
         self._stats_clean = False   # ... and left the statistics array cleared
@@ -2026,6 +2051,7 @@ class B200Transformer(object):
                 b = s.in_views[i].buffer
                 if b.where is None:
                     b.where = torch.tensor([b.ptr()], dtype=torch.int64, device=self.device)
+                    b.where_holds = ctypes.c_void_p(b.ptr())
         for op, b in self._buffers.items():
             if b.plane_bytes > 0 and b.planes is None:
                 b.planes = torch.zeros((2 * b.plane_bytes + 1024,), dtype=torch.uint8,

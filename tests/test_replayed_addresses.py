@@ -13,7 +13,7 @@ from ngraph_python_b200 import transformers
 def test_addresses_are_set_unless_the_call_has(taken, in_place, sets):
     io = transformers._CallIO.__new__(transformers._CallIO)
     io.args = [(0, None, types.SimpleNamespace(src=None), False), (1, None, types.SimpleNamespace(src=None), in_place)]
-    io.taken, calls = taken, []
+    io.in_front, io.taken, calls = True, taken, []
 
     def take():
         assert all(arg.src is None for _, _, arg, _ in io.args)
