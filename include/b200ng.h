@@ -384,6 +384,12 @@ int b2_conv_filter_tiles_info(const b2_conv_dims* d, int32_t pass, size_t* bytes
  * where it does not. */
 typedef struct b2_conv_plan_info { int32_t tile_h, tile_w, tile_n, slices, blocks, in_one_sum; } b2_conv_plan_info;
 int b2_conv_f32_plan(const b2_conv_dims* d, int32_t pass, int32_t tiles, b2_conv_plan_info* plan);
+/* With filters laid out: which kernel that is (0: none; B2_CONV_GATHER keeps A's planes in tensor memory), the k-blocks
+ * in one of its sums of large terms (hi x hi; in_one_sum) and in one of small terms, and what the sums lose to the tensor
+ * core's rounding, in units that compare shapes of one layer and pass, beside the other kernel's shape for it (not less). */
+enum { B2_CONV_DIRECT = 1, B2_CONV_GATHER = 2 };
+typedef struct b2_conv_sums_info { int32_t kernel, large, small, reserved; double loss, other_loss; } b2_conv_sums_info;
+int b2_conv_f32_sums(const b2_conv_dims* d, int32_t pass, b2_conv_sums_info* sums);
 int b2_conv_filter_tiles(const b2_conv_filter_job* jobs, int32_t n, int32_t* launches, void* stream);
 int b2_conv_f32_tiles(int32_t pass, const float* X, const void* filter_tiles, float* O, const b2_conv_dims* d,
                       const float* bias, const float* residual, int32_t relu, const float* mask, int32_t* status,

@@ -189,9 +189,10 @@ inline SumBound sum_bound(int mode, const ConvGeom& g, int pass) {
 // launch and without writing the unrolled planes (8 bytes for each of the R*S copies of a value, and
 // reading them again); the planes pay only where a long list of output channels would have the gather
 // repeated for every 128 of them.
-inline bool conv_goes_direct(int mode, const ConvGeom& g, int pass, b2_direct_args* out) {
+inline bool conv_goes_direct(int mode, const ConvGeom& g, int pass, b2_direct_args* out, SumBound* bound_out = nullptr) {
     if (!flat_depth(g) || getenv("B2_CONV_IM2COL")) return false;
     const SumBound bound = sum_bound(mode, g, pass);
+    if (bound_out) *bound_out = bound;
     long long best = -1;
     for (int a = 1; a <= 2; ++a)
         for (int b = 1; b <= 2; ++b) {
@@ -215,35 +216,57 @@ inline bool conv_goes_direct(int mode, const ConvGeom& g, int pass, b2_direct_ar
 // taps meets zeros of that pixel's filters.  An infinity or NaN therefore makes every result of its image NaN that
 // stands in a tile whose window covers it: up to 2x2 pixels with filters as they lie, 4x4 here (times the stride in
 // an input gradient), beside those whose taps see it.  One-pixel tiles reach no further than the taps.
-inline bool conv_goes_staged(const ConvGeom& g, int pass, b2_direct_args* out) {
-    b2_direct_args d;
-    if (!conv_goes_direct(MODE_F32X3, g, pass, &d)) return false;
-    long long best = b2_direct_cost(d);
-    const SumBound bound = sum_bound(MODE_F32X3, g, pass);
-    auto search = [&](bool own, int longest) {
-        bool found = false;
-        for (int a = 1; a <= 4; ++a)
-            for (int b = 1; b <= 4; ++b) {
-                if (!direct_args(MODE_F32X3, g, pass, pass ? a * g.str_h : a, pass ? b * g.str_w : b, &d) || !bound.allows(d)) continue;
-                d.longest = longest;
-                d.staged = &d;                    // (there will be such)
-                d.staged_own = own;
-                const long long cost = b2_direct_cost(d);
-                if (cost < 0 || cost >= best) continue;
-                best = cost;
-                found = true;
-                *out = d;
-                out->staged = out;
-            }
-        return found;
-    };
-    // The kernel of b2_gather.cu, where it takes less, does not put more k-blocks into one sum than the one of
-    // b2_direct.cuh in the tile and shape that it would take (against 64 bits, 172 layers and passes, batch 4 to 256:
-    // 0.998 of its error, geometric mean, the largest 1.08; without the bound 1.02 and 1.64).
-    b2_direct_args without = d;
-    const bool own = search(true, bound.longest);
-    const bool gathers = g.N % 4 == 0 && search(false, b2_direct_in_one_sum(own ? *out : without));
-    return own || gathers;
+// `other`, unless NULL: what it would be without the kernel of b2_gather.cu.
+inline bool conv_goes_staged(const ConvGeom& g, int pass, b2_direct_args* out, b2_direct_args* other = nullptr) {
+    SumBound bound;
+    if (!conv_goes_direct(MODE_F32X3, g, pass, out, &bound)) return false;
+    long long best = b2_direct_cost(*out);
+    b2_direct_args tile[16];
+    int n = 0;
+    bool found = false;
+    for (int a = 1; a <= 4; ++a)
+        for (int b = 1; b <= 4; ++b) {
+            b2_direct_args& d = tile[n];
+            if (!direct_args(MODE_F32X3, g, pass, pass ? a * g.str_h : a, pass ? b * g.str_w : b, &d) || !bound.allows(d)) continue;
+            ++n;
+            d.longest = bound.longest;
+            d.staged = out;                       // (there will be such)
+            d.staged_own = 1;
+            const long long cost = b2_direct_cost(d);
+            if (cost < 0 || cost >= best) continue;
+            best = cost;
+            found = true;
+            *out = d;
+        }
+    if (other) *other = *out;
+    if (g.N % 4 != 0) return found;
+    // The kernel of b2_gather.cu, where it takes less.  It does not put more k-blocks into one sum of large terms (hi x
+    // hi) than the one of b2_direct.cuh in the tile and shape that it would take, and its sums do not lose more: k-blocks
+    // alone do not say it, those of 64 -> 64 channels at 8x8, batch 100, in tiles of one pixel are dense where a quarter
+    // of 1x2 pixels' are zeros, in five slices of three and two (input gradient 2.04e-7 -> 2.18e-7 against 64 bits in two
+    // slices of three and two; 32 -> 8 channels at 24x7, batch 220, 1.92e-7 -> 2.59e-7).  Shorter sums until that holds.
+    // Sums of small terms have up to twice as many k-blocks as the large ones; they lose 2^-11 of what those do.
+    const int longest = b2_direct_in_one_sum(*out);
+    long long cost[16];
+    double limit = -1;
+    for (int i = 0; i < n; ++i) {
+        tile[i].longest = longest;
+        tile[i].staged_own = 0;
+        cost[i] = b2_direct_cost(tile[i]);
+    }
+    for (;;) {
+        int i = -1;
+        for (int j = 0; j < n; ++j)
+            if (cost[j] >= 0 && cost[j] < best && (i < 0 || cost[j] < cost[i])) i = j;
+        if (i < 0) return found;
+        if (limit < 0) limit = b2_direct_loss(*out) * (1 + 1e-9);
+        if (b2_direct_loss(tile[i]) <= limit) {
+            *out = tile[i];
+            return true;
+        }
+        tile[i].longest = b2_direct_in_one_sum(tile[i]) - 1;
+        cost[i] = tile[i].longest > 0 ? b2_direct_cost(tile[i]) : -1;
+    }
 }
 
 inline int launch_direct(b2_direct_args& d, const void* A, const void* B, void* C,
@@ -2338,6 +2361,21 @@ extern "C" int b2_conv_f32_plan(const b2_conv_dims* d, int32_t pass, int32_t til
     b2_gemm_plan_info p;
     b2_direct_plan(a, &p);
     *plan = {a.g.gh, a.g.gw, p.tile_n, p.slices, (a.K + 31) / 32, b2_direct_in_one_sum(a)};
+    return B2_OK;
+}
+
+extern "C" int b2_conv_f32_sums(const b2_conv_dims* d, int32_t pass, b2_conv_sums_info* sums) {
+    ConvGeom g;
+    int rc = geom_from(d, &g);
+    if (rc) return rc;
+    B2_REQUIRE(sums && (pass == 0 || pass == 1), "bad argument");
+    *sums = {};
+    b2_direct_args a, other;
+    if (!conv_goes_staged(g, pass, &a, &other)) return B2_OK;
+    const int large = b2_direct_in_one_sum(a);
+    const bool gathers = b2_gather_streams(a);
+    *sums = {gathers ? B2_CONV_GATHER : B2_CONV_DIRECT, large, gathers ? b2_gather_plan(a).small : large, 0, b2_direct_loss(a),
+             b2_direct_loss(other)};
     return B2_OK;
 }
 

@@ -1,4 +1,5 @@
 // Dispatch of the kernel with operands converted on the way in; the fp32 half of it.
+#include <cmath>
 #include "b2_direct.cuh"
 
 __attribute__((visibility("hidden"))) int b2_direct_launch_flex(const b2_direct_args& a, cudaStream_t st);
@@ -30,6 +31,46 @@ int b2_direct_in_one_sum(const b2_direct_args& a) {
     const DirectShape s = direct_shape<MODE_F32X3>(a);
     const int pairs = dir_pairs(s.bn, s.groups);
     return (s.kb_per_split + pairs - 1) / pairs;
+}
+
+double b2_direct_loss(const b2_direct_args& a) {
+    const b2_gather& g = a.g;
+    int per, splits, sums;
+    if (b2_gather_streams(a)) {
+        const b2_gather_info s = b2_gather_plan(a);
+        per = s.kb_per_split; splits = s.splits; sums = s.sums;
+    } else {
+        const DirectShape s = direct_shape<MODE_F32X3>(a);
+        per = s.kb_per_split; splits = s.splits; sums = dir_pairs(s.bn, s.groups);
+    }
+    const int taps = g.R * g.S, pixels = filter_tiles(a) ? g.gh * g.gw : 1;
+    double lost = 0;
+    for (int pixel = 0; pixel < pixels; ++pixel) {
+        unsigned char seen[32];                   // (taps <= 31)
+        for (int t = 0; t < taps; ++t) {
+            const int r = g.f0_h + g.f1_h * (t / g.S) + g.f2_h * (pixel / g.gw), s = g.f0_w + g.f1_w * (t % g.S) + g.f2_w * (pixel % g.gw);
+            seen[t] = !filter_tiles(a) || (r >= 0 && r < g.fr && s >= 0 && s < g.fs);
+        }
+        int tap = 0, channel = 0;                 // of the next column
+        for (int z = 0; z < splits; ++z) {
+            double sum[4] = {}, steps[4] = {};    // a sum's squared size; what its steps have cut off
+            for (int kb = z * per; kb < (z + 1) * per && kb * 32 < a.K; ++kb)
+                for (int step = 0; step < 4; ++step) {
+                    int n = 0;
+                    for (int k = kb * 32 + step * 8, end = k + 8; k < end && k < a.K; ++k) {
+                        n += seen[tap];
+                        if (g.channel_last) { if (++channel == g.channels) { channel = 0; ++tap; } }
+                        else if (++tap == taps) tap = 0;
+                    }
+                    if (!n) continue;
+                    const int i = (kb - z * per) % sums;
+                    sum[i] += n;
+                    steps[i] += sqrt(sum[i]);
+                }
+            for (int i = 0; i < sums; ++i) lost += steps[i] * steps[i];
+        }
+    }
+    return lost / pixels;
 }
 
 void b2_direct_plan(const b2_direct_args& a, b2_gemm_plan_info* plan) {

@@ -516,8 +516,9 @@ bool b2_gather_streams(const b2_direct_args& a) {
 
 b2_gather_info b2_gather_plan(const b2_direct_args& a) {
     const GatherShape s = gather_shape(a);
-    const int sums = gat_sums(s.bn);
-    return {s.cost, s.bn, s.splits, s.waves, (s.kb_per_split + sums - 1) / sums, gat_issuers(s.bn)};
+    const int sums = gat_sums(s.bn), issuers = gat_issuers(s.bn);
+    return {s.cost, s.bn, s.splits, s.waves, s.kb_per_split, sums, (s.kb_per_split + sums - 1) / sums,
+            (s.kb_per_split + issuers - 1) / issuers, issuers};
 }
 
 int b2_gather_launch(const b2_direct_args& a, cudaStream_t st) {

@@ -97,6 +97,12 @@ class ConvPlan(C.Structure):
     _fields_ = [(n, C.c_int32) for n in ("tile_h", "tile_w", "tile_n", "slices", "blocks", "in_one_sum")]
 
 
+class ConvSums(C.Structure):
+    _fields_ = ([(n, C.c_int32) for n in ("kernel", "large", "small", "reserved")] +
+                [(n, C.c_double) for n in ("loss", "other_loss")])
+
+
+CONV_DIRECT, CONV_GATHER = 1, 2
 GEMM_DIRECT, GEMM_PAIRS, GEMM_TILES = 0, 1, 2
 CALL_MAX_INPUTS, CALL_MAX_OUTPUTS = 16, 16
 
@@ -170,6 +176,7 @@ def _load():
         "b2_conv_filter_planes_many": (C.c_int, [C.POINTER(ConvFilterJob), i32, C.POINTER(i32), vp]),
         "b2_conv_split_planes": (C.c_int, [vp, i32, i32, i32, i32, vp, vp]),
         "b2_conv_f32_plan": (C.c_int, [C.POINTER(ConvDims), i32, i32, C.POINTER(ConvPlan)]),
+        "b2_conv_f32_sums": (C.c_int, [C.POINTER(ConvDims), i32, C.POINTER(ConvSums)]),
         "b2_conv_filter_tiles_info": (C.c_int, [C.POINTER(ConvDims), i32, C.POINTER(sz)]),
         "b2_conv_filter_tiles": (C.c_int, [C.POINTER(ConvFilterJob), i32, C.POINTER(i32), vp]),
         "b2_conv_f32_tiles": (C.c_int, [i32, vp, vp, vp, C.POINTER(ConvDims), vp, vp, i32, vp, vp, vp]),
@@ -464,6 +471,13 @@ def conv_f32_plan(dims, conv_pass, tiles):
     p = ConvPlan()
     check(_lib.b2_conv_f32_plan(C.byref(dims), conv_pass, int(tiles), C.byref(p)))
     return p if p.tile_n else None
+
+
+def conv_f32_sums(dims, conv_pass):
+    """ConvSums of an fp32 pass with its filters laid out, or None where it takes none."""
+    s = ConvSums()
+    check(_lib.b2_conv_f32_sums(C.byref(dims), conv_pass, C.byref(s)))
+    return s if s.kernel else None
 
 
 def conv_filter_tiles_info(dims, conv_pass):
