@@ -746,13 +746,18 @@ DirectShape direct_shape(const b2_direct_args& a, bool plain = false) {
     const int most = MODE == MODE_FLEX16 ? 256 : 16;
     DirectShape best = {0, 0, 0, 0, 1, -1};
     const long long tm = (a.M + 127) / 128;
+    int per_of[9] = {};                                           // k-blocks of a slice, 0: not so many slices
+    for (int want = 1; want <= 8 && want <= num_kb; ++want) {
+        const bool chains = MODE == MODE_F32X3 && a.a_kind != B2_OPERAND_GATHER && want > 1;
+        const int per = chains ? most : (num_kb + want - 1) / want;
+        if ((num_kb + per - 1) / per == want && per <= most) per_of[want] = per;
+    }
     for (int bn = 16; bn <= 128; bn *= 2) {
         if (bn > 16 && bn / 2 >= a.N) break;
         const long long tiles = tm * ((a.N + bn - 1) / bn);
-        for (int want = 1; want <= 8 && want <= num_kb; ++want) {
-            const bool chains = MODE == MODE_F32X3 && a.a_kind != B2_OPERAND_GATHER && want > 1;
-            const int per = chains ? most : (num_kb + want - 1) / want, splits = (num_kb + per - 1) / per;
-            if (splits != want || per > most) continue;
+        for (int splits = 1; splits <= 8; ++splits) {
+            const int per = per_of[splits];
+            if (!per) continue;
             const int tab = dir_table_bytes(a, per * KB);
             if (1152 + dir_ring_bytes(bn) + tab > 232448) continue;
             // Measured on one B200 (cycles at 1.9 GHz): the producers set the pace, 7 (fp32) or 22
@@ -792,6 +797,7 @@ DirectShape direct_shape(const b2_direct_args& a, bool plain = false) {
             // (the exchange of slices: 700 and 500 a slice)
             const long long one = 7000 + per * kb + together * bn * (splits > 1 ? 24 : 12) +
                                   (splits == 1 ? 0 : filter_tiles(a) && !a.staged ? 18000 : plain ? 3000 : 700 + 500 * splits);
+            if (best.cost >= 0 && one >= best.cost) continue;
             const long long waves = (ctas + slots - 1) / slots, cost = waves * one;
             if (best.cost < 0 || cost < best.cost) best = {bn, splits, per, (int)waves, groups, cost};
         }

@@ -462,17 +462,23 @@ GatherShape gather_shape(const b2_direct_args& a) {
     GatherShape best = {0, 0, 0, 0, -1};
     const long long tm = (a.M + 127) / 128;
     if (tm > 65535) return best;
+    int per_of[9] = {};                                           // k-blocks of a slice, 0: not so many slices
+    for (int want = 1; want <= 8 && want <= num_kb; ++want) {
+        const int per = (num_kb + want - 1) / want;
+        if ((want - 1) * per < num_kb) per_of[want] = per;
+    }
     for (int bn : {16, 32, 64, 96, 128}) {
         if (bn > 16 && (bn == 96 ? 64 : bn / 2) >= a.N) break;
         const long long tiles = tm * ((a.N + bn - 1) / bn);
-        for (int want = 1; want <= 8 && want <= num_kb; ++want) {
-            const int per = (num_kb + want - 1) / want, splits = (num_kb + per - 1) / per;
-            if (splits != want || gather_smem(bn, per) > 232448 - 1024) continue;
+        const int kb = bn <= 64 ? 520 : 6 * bn + 30;
+        for (int splits = 1; splits <= 8; ++splits) {
+            const int per = per_of[splits];
+            if (!per || gather_smem(bn, per) > 232448 - 1024) continue;
             if (a.longest > 0 && (per + gat_sums(bn) - 1) / gat_sums(bn) > a.longest) continue;
-            const long long kb = bn <= 64 ? 520 : 6 * bn + 30;
+            const long long one = 7500 + per * kb + 30 * bn + (splits == 1 ? 0 : 3000 + 10 * bn);
+            if (best.cost >= 0 && one >= best.cost) continue;
             const long long ctas = tiles * splits, slots = kClusterCtas[splits], waves = (ctas + slots - 1) / slots;
-            const long long cost = waves * (7500 + per * kb + 30 * bn + (splits == 1 ? 0 : 3000 + 10 * bn));
-            if (best.cost < 0 || cost < best.cost) best = {bn, splits, per, (int)waves, cost};
+            if (best.cost < 0 || waves * one < best.cost) best = {bn, splits, per, (int)waves, waves * one};
         }
     }
     return best;
