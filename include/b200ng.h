@@ -284,16 +284,19 @@ int b2_flex_end_call(const b2_flex_state* s, int32_t n, const int64_t* ids, cons
  * ------------------------------------------------------------------------------------------ */
 int b2_gemm_scratch_bytes(int32_t flex, int32_t M, int32_t N, int32_t K, size_t* bytes);
 /* Kernels one product launches: 1 where its operands are converted on the way in, else the operand
- * planes and the tile kernel (K strides as below; for rows along K that start anywhere: where they start on
- * sixteen bytes some more products take one launch). */
+ * planes and the tile kernel (K strides as below, operands dense along the other side). */
 int b2_gemm_launches(int32_t flex, int64_t a_k_stride, int64_t b_k_stride, int32_t M, int32_t N,
                      int32_t K, int32_t* launches);
 /* Which kernel that is, and how it cuts the product: tile_n columns to a tile, K in `slices` parts that
  * the CTAs or pairs of a cluster take, `waves` times as many clusters as the machine holds at once. */
-enum b2_gemm_kernel { B2_GEMM_DIRECT = 0, B2_GEMM_PAIRS = 1, B2_GEMM_TILES = 2 };
+enum b2_gemm_kernel { B2_GEMM_DIRECT = 0, B2_GEMM_PAIRS = 1, B2_GEMM_TILES = 2, B2_GEMM_STREAM = 3 };
 typedef struct b2_gemm_plan_info { int32_t kernel, tile_n, slices, waves; } b2_gemm_plan_info;
 int b2_gemm_plan(int32_t flex, int64_t a_k_stride, int64_t b_k_stride, int32_t M, int32_t N, int32_t K,
                  b2_gemm_plan_info* plan);
+/* Both for strides as a product is called with (b2_gemm_plan has B2_GEMM_DIRECT for either kernel that takes one launch;
+ * here B2_GEMM_STREAM is the one with A's planes in tensor memory). */
+int b2_gemm_route(int32_t flex, int64_t a_row_stride, int64_t a_k_stride, int64_t b_k_stride, int64_t b_col_stride,
+                  int32_t M, int32_t N, int32_t K, b2_gemm_plan_info* plan, int32_t* launches);
 /* fp32 via 3xTF32 (relative error ~2^-21).  Sums of K in chains of 512 products; up to K = 4096 every
  * kernel adds the chains in order, so that a result does not depend on the number of rows and columns
  * computed beside it. */

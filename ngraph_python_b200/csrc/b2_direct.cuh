@@ -837,9 +837,10 @@ template <int MODE, int BN, int G>
 int direct_launch_bn(const DirectParams& p, cudaStream_t st) {
     if constexpr (MODE == MODE_F32X3)
         if (p.a.staged) return direct_launch_as<MODE, BN, B2_OPERAND_GATHER, G, true>(p, st);
-    // (flex16 matrix products come here with one k-block: one group)
+    // (flex16 matrix products of several k-blocks come here with both operands along K)
     if constexpr (MODE == MODE_FLEX16 && G > 1) {
-        B2_REQUIRE(p.a.a_kind == B2_OPERAND_GATHER, "a product of several k-blocks");
+        B2_REQUIRE(p.a.a_kind != B2_OPERAND_ROWS, "a product of several k-blocks");
+        if (p.a.a_kind == B2_OPERAND_K) return direct_launch_as<MODE, BN, B2_OPERAND_K, G>(p, st);
         return direct_launch_as<MODE, BN, B2_OPERAND_GATHER, G>(p, st);
     }
     switch (p.a.a_kind) {

@@ -38,9 +38,29 @@ inline long long plane_cost(int mode, const Shapes& s, int M, int N, int K) {
     return (mode == MODE_FLEX16 ? 20000 : 13000) + prepass + (tiles + 147) / 148 * (3500 + num_kb * kb);
 }
 
-// Whether a product takes the kernel that converts its operands on the way in (one launch), and its
-// arguments: the cheaper of C and its transpose, so that a product with few rows does not pad them to
-// a whole tile.
+// The same for flex16 products that the kernel of b2_stream.cuh may take instead, with what the rule above leaves out:
+// results that are stored one by one, operands that do not start their lines on sixteen bytes (7053 x 271 x 336 takes 50
+// us on planes, 5282 x 5707 x 137 318).
+inline long long plane_cost_measured(const b2_direct_args& d, long long plane) {
+    const long long results = (long long)d.M * d.N;
+    return plane + 3000 + results * (d.N % 8 == 0 ? 0 : d.N % 4 == 0 ? 9 : 16) / 1000 +
+           (b2_product_even(d) ? 0 : ((long long)d.M + d.N) * d.K * 2 / 1000);
+}
+
+// A product in one launch: the kernel that takes least for it, and C or its transpose -- so that a product with few rows
+// does not pad them to a whole tile.  `out` gets its arguments; whether that takes less than the planes.
+//
+// Both kernels and the planes measured side by side on one B200, 1900 products of 1 to 8192 rows, columns and K in all
+// three layouts:
+//   fp32, the cheaper of b2_stream.cuh's cost and b2_direct.cuh's, which is short by 1.4 where both operands are
+//     contiguous along their rows and by 1.05 elsewhere (512 x 128 x 512 8.6 us against 10.7, 1784 x 508 x 952
+//     transposed 31.6 and 23.9, 1489 x 605 x 176 13.3 and 12.7), of 129 to 1024 columns or narrow results, and where no
+//     line has to be shifted out of words that its neighbour shares (99 x 1347 x 2389 19.3 and 17.0).
+//   flex16, b2_stream.cuh's, 1.36 times as fast (geometric mean), but
+//     for one k-block and many results, where the other's two CTAs an SM hide the epilogue (2929 x 567 x 122 22.5 and 16.2);
+//     for one k-block and few results whose operands lie along K off sixteen bytes (7 x 128 x 31 4.9 and 4.1);
+//     for narrow results with many k-blocks to a CTA, both operands along K and on sixteen bytes (78 x 3096 x 3360 21.7
+//     and 17.9, 4396 x 44 x 5248 21.0 and 18.5).
 inline bool gemm_goes_direct(int mode, const void* A, long long a_rs, long long a_cs, const void* B,
                              long long b_ks, long long b_ns, int M, int N, int K, b2_direct_args* out, bool may_stream = true) {
     b2_direct_args d = {};
@@ -52,20 +72,50 @@ inline bool gemm_goes_direct(int mode, const void* A, long long a_rs, long long 
     t.A = d.B; t.a_rs = d.b_rs; t.a_ks = d.b_ks; t.a_kind = d.b_kind;
     t.B = d.A; t.b_rs = d.a_rs; t.b_ks = d.a_ks; t.b_kind = d.a_kind;
     t.M = N; t.N = M; t.colmajor = 1;
-    const bool streams = may_stream && b2_product_streams(d);     // (the same for C's transpose)
-    const long long cd = streams ? b2_stream_cost(d) : b2_direct_cost(d), ct = streams ? b2_stream_cost(t) : b2_direct_cost(t);
-    const long long plane = plane_cost(mode, shapes_for(mode, M, N, K), M, N, K);
-    const bool swap = ct >= 0 && (cd < 0 || ct < cd);
-    *out = swap ? t : d;
-    long long best = swap ? ct : cd;
-    // (many k-blocks in few slices: flex16 500 x 500 x 6000, the second operand along K, 19.7 us on planes, 21.6 in one
-    // launch)
-    if (streams && mode == MODE_FLEX16 && K > 4096 && M > 256 && N > 256) best += best / 8;
+    const bool by_rows = d.a_kind == B2_OPERAND_ROWS && d.b_kind == B2_OPERAND_ROWS;
+    const bool along_k = d.a_kind == B2_OPERAND_K && d.b_kind == B2_OPERAND_K, even = b2_product_even(d);
+    const long long plane = plane_cost(mode, shapes_for(mode, M, N, K), M, N, K), results = (long long)M * N;
+    auto cheaper = [&](long long cd, long long ct) {
+        const bool swap = ct >= 0 && (cd < 0 || ct < cd);
+        *out = swap ? t : d;
+        return swap ? ct : cd;
+    };
+    long long stream = -1;
+    if (may_stream && mode == MODE_FLEX16) {
+        const bool few = along_k && !even && M <= 64 && results < 4096;
+        if (K > 128 || (!few && results < (by_rows || along_k ? 900000 : 400000))) {
+            // (near each other C itself is the faster: 178 x 2 x 46 transposed 4.2 and 4.7 us)
+            const long long ct = b2_stream_cost(t);
+            stream = cheaper(b2_stream_cost(d), ct < 0 ? ct : ct + 1000);
+            out->streams = 1;
+            if (along_k && even && K > 128 && stream >= 0 && (M <= 192 || N <= 192)) {
+                const b2_direct_args streamed = *out;
+                b2_gemm_plan_info plan;
+                b2_stream_plan(streamed, &plan);
+                const long long direct = cheaper(b2_direct_cost(d), b2_direct_cost(t));
+                const int per = ((K + 127) / 128 + plan.slices - 1) / plan.slices;
+                if (direct < 0 || per < 14 || direct >= stream + stream * 2 / 9) *out = streamed;
+            }
+            // (many k-blocks in few slices: flex16 500 x 500 x 6000, the second operand along K, 19.7 us on planes, 21.6
+            // in one launch)
+            if (K > 4096 && M > 256 && N > 256) return stream >= 0 && stream + stream / 8 < plane;
+            return stream >= 0 && stream < (K > 128 ? plane_cost_measured(d, plane) : plane);
+        }
+    } else if (may_stream && K > 128 && (K <= 1024 || M <= 32 || N <= 32) && (by_rows || even)) {
+        stream = cheaper(b2_stream_cost(d), b2_stream_cost(t));
+    }
+    const b2_direct_args streamed = *out;
+    long long best = cheaper(b2_direct_cost(d), b2_direct_cost(t));
+    if (stream >= 0 && stream < plane && (best < 0 || stream <= best + (by_rows ? best * 2 / 5 : best / 20))) {
+        *out = streamed;
+        out->streams = 1;
+        return true;
+    }
     // Both operands contiguous along their rows take longer than the direct kernel's own choice of a shape has to
     // know: fp32 638 x 937 x 631 26 us against 20 on planes, 383 x 3300 x 1440 47 and 39 (two k-blocks or less
     // don't: 1869 x 1337 x 46 20 and 26); flex16 an odd number of values apart, loaded one by one, 249 x 1831 x
     // 3065 75 and 41, 745 x 913 x 1135 65 and 31.  (With one of the two along K: 236 x 339 x 3450 26 and 33.)
-    if (!streams && d.a_kind == B2_OPERAND_ROWS && d.b_kind == B2_OPERAND_ROWS) {
+    if (by_rows) {
         if (mode == MODE_F32X3) best += K > 64 ? best / 6 : 0;
         else if (K > 128 && out->a_ks % 2 != 0) best += best / 2;
     }
@@ -93,7 +143,7 @@ int run_gemm(const T* A, long long a_rs, long long a_cs, const T* B, long long b
         d.C = C; d.ldc = ldc; d.table = table; d.slotC = slotC;
         d.slotA = d.colmajor ? slotB : slotA; d.slotB = d.colmajor ? slotA : slotB;
         d.stats = stats; d.probe_out = probe_out; d.status = status; d.probe = probe;
-        return b2_product_streams(d) ? b2_stream_launch(d, st) : b2_direct_launch(d, st);
+        return d.streams ? b2_stream_launch(d, st) : b2_direct_launch(d, st);
     }
     const int splits = pick_splits(MODE, s, false);     // > 1 only for flex16 with K > 32768
     unsigned char* base = (unsigned char*)scratch;
@@ -131,36 +181,46 @@ extern "C" int b2_gemm_scratch_bytes(int32_t flex, int32_t M, int32_t N, int32_t
     return B2_OK;
 }
 
-extern "C" int b2_gemm_launches(int32_t flex, int64_t a_k_stride, int64_t b_k_stride, int32_t M,
-                                int32_t N, int32_t K, int32_t* launches) {
-    B2_REQUIRE(launches && M > 0 && N > 0 && K > 0, "bad argument");
+extern "C" int b2_gemm_route(int32_t flex, int64_t a_rs, int64_t a_cs, int64_t b_ks, int64_t b_ns, int32_t M, int32_t N,
+                             int32_t K, b2_gemm_plan_info* plan, int32_t* launches) {
+    B2_REQUIRE(plan && launches && M > 0 && N > 0 && K > 0, "bad argument");
+    B2_REQUIRE((a_rs == 1 || a_cs == 1) && (b_ks == 1 || b_ns == 1), "operands are contiguous along one of their sides");
     const int mode = flex ? MODE_FLEX16 : MODE_F32X3;
     b2_direct_args d;
-    *launches = gemm_goes_direct(mode, nullptr, 1, a_k_stride, nullptr, b_k_stride, 1, M, N, K, &d) ? 1
-                : pick_splits(mode, shapes_for(mode, M, N, K), false) > 1 ? 3 : 2;
+    if (gemm_goes_direct(mode, nullptr, a_rs, a_cs, nullptr, b_ks, b_ns, M, N, K, &d)) {
+        *launches = 1;
+        if (d.streams) {
+            b2_stream_plan(d, plan);
+            plan->kernel = B2_GEMM_STREAM;
+        } else {
+            b2_direct_plan(d, plan);
+        }
+        return B2_OK;
+    }
+    const Shapes s = shapes_for(mode, M, N, K);
+    const int splits = pick_splits(mode, s, false);
+    *launches = splits > 1 ? 3 : 2;
+    if (goes_in_pairs(s, M, splits)) {
+        const int tiles = ((M + 255) / 256) * ((N + 127) / 128), z = pair_splits(mode, tiles, (int)(s.Kp / (kKBytes / s.esize)));
+        *plan = {B2_GEMM_PAIRS, 128, z, (int)pair_waves(tiles, z)};
+    } else {
+        *plan = {B2_GEMM_TILES, s.bn, splits, (int)(((long long)(s.Mp / kBlockM) * (s.Np / s.bn) * splits + 147) / 148)};
+    }
     return B2_OK;
+}
+
+extern "C" int b2_gemm_launches(int32_t flex, int64_t a_k_stride, int64_t b_k_stride, int32_t M,
+                                int32_t N, int32_t K, int32_t* launches) {
+    b2_gemm_plan_info plan;
+    return b2_gemm_route(flex, a_k_stride == 1 ? K : 1, a_k_stride, b_k_stride, b_k_stride == 1 ? K : 1, M, N, K, &plan, launches);
 }
 
 extern "C" int b2_gemm_plan(int32_t flex, int64_t a_k_stride, int64_t b_k_stride, int32_t M, int32_t N,
                             int32_t K, b2_gemm_plan_info* plan) {
-    B2_REQUIRE(plan && M > 0 && N > 0 && K > 0, "bad argument");
-    const int mode = flex ? MODE_FLEX16 : MODE_F32X3;
-    b2_direct_args d;
-    if (gemm_goes_direct(mode, nullptr, 1, a_k_stride, nullptr, b_k_stride, 1, M, N, K, &d)) {
-        if (b2_product_streams(d)) b2_stream_plan(d, plan);
-        else b2_direct_plan(d, plan);
-        return B2_OK;
-    }
-    const Shapes s = shapes_for(mode, M, N, K);
-    const int splits = pick_splits(mode, s, false), num_kb = s.Kp / (kKBytes / s.esize);
-    if (goes_in_pairs(s, M, splits)) {
-        const int tiles = ((M + 255) / 256) * ((N + 127) / 128), z = pair_splits(mode, tiles, num_kb);
-        *plan = {B2_GEMM_PAIRS, 128, z, (int)pair_waves(tiles, z)};
-    } else {
-        const long long tiles = (long long)(s.Mp / kBlockM) * (s.Np / s.bn) * splits;
-        *plan = {B2_GEMM_TILES, s.bn, splits, (int)((tiles + 147) / 148)};
-    }
-    return B2_OK;
+    int32_t launches;
+    const int rc = b2_gemm_route(flex, a_k_stride == 1 ? K : 1, a_k_stride, b_k_stride, b_k_stride == 1 ? K : 1, M, N, K, plan, &launches);
+    if (rc == B2_OK && plan->kernel == B2_GEMM_STREAM) plan->kernel = B2_GEMM_DIRECT;
+    return rc;
 }
 
 extern "C" int b2_gemm_f32(const float* A, int64_t a_row_stride, int64_t a_k_stride, const float* B,

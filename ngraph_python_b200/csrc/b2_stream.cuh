@@ -20,7 +20,7 @@
 //
 // What bounds it: latency at the smallest sizes, then shared memory's 128 bytes a clock.  An instruction of few
 // columns reads 4 KB of A from shared memory in 39 cycles and writes next to nothing; from tensor memory it takes 9
-// (N = 16) to 64 (N = 128, the tensor pipe's own rate).  A k-block then takes 480 + 9 BN (fp32) or 900 + 16 BN
+// (N = 16) to 64 (N = 128, the tensor pipe's own rate).  A k-block then takes 370 + 9 BN (fp32) or 900 + 16 BN
 // (flex16) cycles, which is instruction issue: copies, conversion and the issue of its twelve or sixteen MMAs.  One
 // B200, the kernel of b2_direct.cuh -> this one, us: fp32 512 x 128 x 512 10.7 -> 8.6, by columns 13.6 -> 10.0; flex16
 // 512 x 128 x 784 8.8 -> 7.6, 300 x 50 x 300 9.6 -> 6.5, 187 x 131 x 31 12.4 -> 6.8 (a result is a chain of a hundred
@@ -534,7 +534,7 @@ stream_kernel(const __grid_constant__ StreamParams p) {
                 Sum v[U];
 #pragma unroll
                 for (int u = 0; u < U; ++u) v[u] = 0;
-                constexpr int Z = FLEX ? 8 / U : 8 / U;
+                constexpr int Z = 8 / U;
                 for (int i0 = 0; i0 < total; i0 += Z) {
                     Sum t[Z][U];
 #pragma unroll
@@ -623,17 +623,21 @@ StreamShape stream_shape(const b2_direct_args& a) {
             const int chains = MODE == MODE_FLEX16 ? 1 : (per + most - 1) / most;
             if (splits != want || (MODE == MODE_FLEX16 ? per > most : chains > chains_most)) continue;
             if (splits > 1 && chains * bn * 128 * (MODE == MODE_FLEX16 ? 8 : 4) > 200 * 1024) continue;
-            // Measured on one B200 (cycles at 1.9 GHz, 290 products, all their shapes; the rule is within 11 % of them,
-            // root mean square): lines off sixteen bytes cost their converters a shift, A by columns the loads of a
-            // column each.
+            // Measured on one B200 (cycles at 1.9 GHz, 1060 flex16 and 250 fp32 products, each in two shapes; the rule is
+            // within 7 and 5 % of them, root mean square): lines off sixteen bytes cost their converters a shift, operands
+            // by columns the loads of a column each; results by rows that are stored one by one go to as many lines
+            // as there are rows; flex16 takes longer where every SM is busy.
             const long long ctas = tiles * splits, slots = kClusterCtas[splits], waves = (ctas + slots - 1) / slots;
+            const int rows = a.M < 128 ? a.M : 128, live = bn < a.N ? bn : a.N, busy = ctas < 148 ? (int)ctas : 148;
+            const int alone = a.colmajor || (splits == 1 && a.N % 4 == 0) ? 0 : rows * live / splits;
+            const bool a_rows = a.a_kind == B2_OPERAND_ROWS, b_rows = a.b_kind == B2_OPERAND_ROWS;
             long long one, kb;
             if (MODE == MODE_FLEX16) {
-                kb = 900 + 16 * bn + (even ? 0 : 470 + 6 * bn) + (a.a_kind == B2_OPERAND_K ? 0 : 130);
-                one = 6600 + per * kb + 84 * bn + (splits == 1 ? 0 : 1800 + 19 * bn);
+                kb = 900 + 16 * bn + (even ? 0 : 470 + 6 * bn) + (a_rows ? 130 : 0);
+                one = 5000 + per * kb + 84 * bn + (splits > 1 ? 1800 + 19 * bn + 5 * alone / 3 : alone) + 20 * busy - (waves > 1 ? 2300 : 0);
             } else {
-                kb = 480 + 9 * bn + (even ? 0 : 220 + 2 * bn) + (a.a_kind == B2_OPERAND_K ? 0 : 45);
-                one = 5800 + per * kb + 43 * bn + (splits == 1 ? 0 : 2800 + 4 * bn * splits);
+                kb = 370 + 9 * bn + (even ? 0 : 155) + (a_rows ? 140 : 0) + (b_rows ? 3 * bn / 2 : 0);
+                one = 6400 + per * kb + 57 * bn + (splits > 1 ? 3100 : 0) + 2 * alone / 3 - (waves > 1 ? 1300 : 0);
             }
             const long long cost = waves * one;
             if (best.cost < 0 || cost < best.cost) best = {bn, splits, per, (int)waves, cost};

@@ -103,7 +103,7 @@ class ConvSums(C.Structure):
 
 
 CONV_DIRECT, CONV_GATHER = 1, 2
-GEMM_DIRECT, GEMM_PAIRS, GEMM_TILES = 0, 1, 2
+GEMM_DIRECT, GEMM_PAIRS, GEMM_TILES, GEMM_STREAM = 0, 1, 2, 3
 CALL_MAX_INPUTS, CALL_MAX_OUTPUTS = 16, 16
 
 
@@ -159,6 +159,7 @@ def _load():
         "b2_ew_launch_count": (C.c_int, [vp]),
         "b2_gemm_scratch_bytes": (C.c_int, [i32, i32, i32, i32, C.POINTER(sz)]),
         "b2_gemm_launches": (C.c_int, [i32, i64, i64, i32, i32, i32, C.POINTER(i32)]),
+        "b2_gemm_route": (C.c_int, [i32, i64, i64, i64, i64, i32, i32, i32, C.POINTER(GemmPlan), C.POINTER(i32)]),
         "b2_gemm_plan": (C.c_int, [i32, i64, i64, i32, i32, i32, C.POINTER(GemmPlan)]),
         "b2_gemm_f32": (C.c_int, [vp, i64, i64, vp, i64, i64, vp, i64, i32, i32, i32, vp, sz, vp,
                                   vp]),
@@ -433,6 +434,15 @@ def gemm_plan(flex, a_k_stride, b_k_stride, M, N, K):
     p = GemmPlan()
     check(_lib.b2_gemm_plan(int(bool(flex)), a_k_stride, b_k_stride, M, N, K, C.byref(p)))
     return p.kernel, p.tile_n, p.slices, p.waves
+
+
+def gemm_route(flex, a_strides, b_strides, M, N, K):
+    """(kernel, columns of a tile, slices of K, waves of clusters, launches) of a product called with these strides:
+    (row, K) of the first operand, (K, column) of the second."""
+    p, n = GemmPlan(), C.c_int32()
+    check(_lib.b2_gemm_route(int(bool(flex)), a_strides[0], a_strides[1], b_strides[0], b_strides[1], M, N, K, C.byref(p),
+                             C.byref(n)))
+    return p.kernel, p.tile_n, p.slices, p.waves, n.value
 
 
 def conv_fprop_scratch_bytes(flex, dims):
