@@ -497,7 +497,7 @@ class GemmStep(_Step):
         self.out_views = [t._view_of(op)]
         self.flex = t.flex
         self.scratch_bytes = lib.gemm_scratch_bytes(self.flex, self.M, self.N, self.K) + 1024
-        self.launches = lib.gemm_launches(self.flex, a_cs, b_ks, self.M, self.N, self.K)
+        self.launches = lib.gemm_route(self.flex, self.a_str, self.b_str, self.M, self.N, self.K)[-1]
 
     def launch(self, t):
         xv, yv = self.in_views

@@ -5,6 +5,7 @@ import random
 
 import pytest
 
+import ngraph_python_b200 as ng
 from ngraph_python_b200 import lib
 from tests.test_gemm_dispatch import _run
 
@@ -59,3 +60,19 @@ def test_queries_without_row_strides_mean_dense_operands():
 def test_results(flex, layout, M, N, K, kernel):
     import torch
     _run(torch, flex, layout, M, N, K)
+
+
+@pytest.mark.parametrize("extra", [0, 1])
+def test_a_steps_launches_are_those_of_its_strides(extra):
+    """Rows further apart than they are long, off sixteen bytes: on planes, where dense ones take one launch."""
+    M, N, K = 1000, 480, 1360
+    A, B, W = ng.make_axis(M, name="A"), ng.make_axis(N, name="B"), ng.make_axis(K + extra, name="W")
+    x = ng.placeholder([A, W])
+    rows = ng.tensor_slice(x, [slice(None), slice(0, K)], axes=ng.make_axes([A, ng.make_axis(K, name="K")])) if extra else x
+    y = ng.placeholder([rows.axes[1], B])
+    t = ng.transformers.allocate_transformer("b200", plan_only=True)
+    comp = t.computation(ng.dot(rows, y), x, y)
+    t.initialize()
+    step, = [s for s in comp.steps if s.kind == "gemm"]
+    assert step.a_str == (K + extra, 1)
+    assert step.launches == 1 + extra == lib.gemm_route(False, step.a_str, step.b_str, M, N, K)[-1]
