@@ -247,6 +247,8 @@ inline bool conv_goes_staged(const ConvGeom& g, int pass, b2_direct_args* out, b
     // slices of three and two; 32 -> 8 channels at 24x7, batch 220, 1.92e-7 -> 2.59e-7).  Shorter sums until that holds.
     // Sums of small terms have up to twice as many k-blocks as the large ones; they lose 2^-11 of what those do.
     const int longest = b2_direct_in_one_sum(*out);
+    b2_gemm_plan_info plan;
+    b2_direct_plan(*out, &plan);
     long long cost[16];
     double limit = -1;
     for (int i = 0; i < n; ++i) {
@@ -259,6 +261,12 @@ inline bool conv_goes_staged(const ConvGeom& g, int pass, b2_direct_args* out, b
         for (int j = 0; j < n; ++j)
             if (cost[j] >= 0 && cost[j] < best && (i < 0 || cost[j] < cost[i])) i = j;
         if (i < 0) return found;
+        // The same shape in more than one wave: two of the other kernel's CTAs share an SM and take less than its rule says
+        // (3 <- 16 channels 3x3 at 32x32, batch 128, 28.9 us, 38.8 in this one; 32 <- 16 at stride 2, batch 200, 17.3 and 20.1).
+        if (plan.waves > 1 && plan.tile_n < 128 && tile[i].g.gh == out->g.gh && tile[i].g.gw == out->g.gw && cost[i] > best - best / 5) {
+            const b2_gather_info own = b2_gather_plan(tile[i]);
+            if (own.bn == plan.tile_n && own.splits == plan.slices) return found;
+        }
         if (limit < 0) limit = b2_direct_loss(*out) * (1 + 1e-9);
         if (b2_direct_loss(tile[i]) <= limit) {
             *out = tile[i];

@@ -88,3 +88,12 @@ def test_device_cases_reach_the_kernel():
 @pytest.mark.parametrize("shift", [0, 1])
 def test_widest_tiles(case, shift):
     _both_passes(case, shift)
+
+
+@pytest.mark.parametrize("layer, bprop, kernel", [
+    ((3, 32, 32, 16, 3, 1, 128), 1, lib.CONV_DIRECT), ((16, 32, 32, 32, 3, 2, 200), 1, lib.CONV_DIRECT),
+    ((8, 14, 35, 24, 5, 1, 480), 0, lib.CONV_DIRECT), ((16, 32, 32, 16, 3, 1, 100), 0, lib.CONV_GATHER),
+    ((64, 8, 8, 64, 3, 1, 256), 1, lib.CONV_GATHER), ((24, 16, 35, 56, 3, 2, 144), 1, lib.CONV_GATHER)])
+def test_kernel_of_a_layer(layer, bprop, kernel):
+    """Several waves in the shape that the other kernel has, two CTAs of it to an SM: that one (measured)."""
+    assert lib.conv_f32_sums(_dims(*layer), bprop).kernel == kernel
