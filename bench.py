@@ -597,7 +597,9 @@ def run_resnet(args, rank, world, torch, dist, local):
                       % (Timer.FLUSH_BYTES >> 20),
                 "steps_per_pass": len(comp.recorded or comp.steps), "cuda_graph": not args.no_graph,
                 "value_includes": "per-call exponent bookkeeping, graph replay, statistics and "
-                                  "status read-back with one stream synchronisation"})
+                                  "status read-back with one stream synchronisation; the images are in "
+                                  "their tensor: the launch that takes a call's arguments in counts in "
+                                  "e2e alone"})
     line = {
         "metric": "ResNet-20 %s inference img/s" % ("flex16" if flex else "fp32"),
         "value": round(world * n / (ms_step * 1e-3), 1), "unit": "img/s", "n_gpus": world,

@@ -3,9 +3,9 @@
 // the same for matrix products, b2_direct.cuh the rows of the columns' table and what a tile is).
 //
 // One CTA per 128 x BN tile (times a slice of K), 864 threads:
-//   eight warps copy a k-block's 32 columns: 128 rows each, sixteen bytes a copy (four images of a pixel; four bytes
-//             where the images of a pixel are no multiple of four or the tensor does not start on sixteen bytes),
-//             zeros where the tap lies outside; in two groups that take the k-blocks by turns;
+//   eight warps copy a k-block's 32 columns: 128 rows each, sixteen bytes a copy (four images of a pixel: other numbers
+//             of images stay with b2_direct.cuh; four bytes a copy where the tensor does not start on sixteen), zeros
+//             where the tap lies outside; in two groups that take the k-blocks by turns;
 //   two groups of eight warps convert, the k-blocks by turns: a lane is a row, a warp has half of its columns, converted
 //             by the time the slot in tensor memory is free; afterwards all sixteen are the epilogue (bias, residual,
 //             ReLU, mask);
@@ -19,9 +19,9 @@
 // What bounds it: chains of instructions.  Start and first columns 4400 cycles, a k-block 700 to 1000 (a slot of tensor
 // memory is filled, announced, multiplied and given back in 1400, there are two or three), the epilogue 2000 for eight
 // columns of a warp; without any loads of A or B the launches take 0.89 of their time, with a quarter of the MMAs 0.90.
-// One B200, fp32 ResNet-20, kernels of b2_direct.cuh -> this one, us: 22 layers at batch 100 266 -> 239 (a call 341 ->
-// 294), forward and input gradients at batch 256 1000 -> 875; of its epilogue the one with a branch a term took 1.4 times
-// as long in training.
+// One B200, fp32 ResNet-20, kernels of b2_direct.cuh -> this one, us: 22 layers at batch 100 266 -> 239, forward and
+// input gradients at batch 256 1000 -> 875; of its epilogue the one with a branch a term took 1.4 times as long in
+// training.
 #include "b2_stream.cuh"
 
 namespace {
@@ -510,7 +510,7 @@ int gather_launch_as(const GatherParams& p, cudaStream_t st) {
 
 template <int BN>
 int gather_launch_bn(const GatherParams& p, cudaStream_t st) {
-    return p.a.g.N % 4 == 0 && ((uintptr_t)p.a.A & 15) == 0 ? gather_launch_as<BN, true>(p, st) : gather_launch_as<BN, false>(p, st);
+    return ((uintptr_t)p.a.A & 15) == 0 ? gather_launch_as<BN, true>(p, st) : gather_launch_as<BN, false>(p, st);
 }
 
 }  // namespace
