@@ -983,12 +983,37 @@ bool vector_ok(const b2_ew_program& p, int V) {
     return true;
 }
 
+// A row to a warp, where that gives the machine warps enough, each with its row's loads under way: no barrier between a
+// row and the next, and short rows do not leave most of a block idle.  Fewer and longer rows are faster by blocks; how
+// many and how long depends on what a row takes besides the sums.  One B200, 212 sizes, us a launch, a block to a
+// row -> a warp: four tensors read, one stored, two reductions, flex16 7972 x 868 32.4 -> 19.1, 2900 x 728 12.0 -> 8.0, 2094 x 1446
+// 15.6 -> 13.9, but 1000 x 4096 11.0 -> 19.1, 3000 x 3001 30.6 -> 42.5; fp32 6167 x 384 18.4 -> 8.7, but 3370 x 937 19.7 -> 24.6,
+// 6621 x 1680 38.7 -> 41.4.  Two read and one sum, flex16 2340 x 2784 9.4 -> 7.9, but 1079 x 2464 5.3 -> 5.9; fp32 2775 x 1624
+// 9.3 -> 5.4, 1024 x 2048 4.4 -> 3.7, but 1000 x 4096 5.5 -> 6.7, 1024 x 1999 5.6 -> 7.2.  (One value to a thread: short rows alone, a
+// lane's sum would have more terms than a thread's of a block.)
+int full_tensors(const b2_ew_program& p) {
+    int n = p.n_out;
+    for (int i = 0; i < p.n_in; ++i) n += p.in[i].sc != 0;
+    return n;
+}
+bool warp_to_row(const b2_ew_program& p, long long rows, long long chunks, int V, bool ragged) {
+    if (chunks <= 64) return true;
+    if (V == 1 || rows < 1000) return false;
+    if (full_tensors(p) > 3) return chunks <= (rows >= 6000 ? 288 : rows >= 2000 ? 192 : 128);
+    if (V == 8) return chunks <= (rows < 2000 ? 220 : ragged ? 240 : rows < 4000 ? 360 : 512);
+    if (!ragged) return chunks <= (rows < 2000 && full_tensors(p) > 2 ? 256 : 512);
+    return chunks <= (rows >= 2000 ? 450 : 300);
+}
+
 // Rows of full tensors that are the same distance apart start on the same place within a vector: all of a row but its
 // ends is read and stored in vectors though its length or distance is no multiple of one.  Not worth it for rows whose
-// ends are much of them, nor for so little work that one value to a thread keeps the machine half empty.  One
+// ends are much of them, nor for so little work that one value to a thread keeps the machine half empty: reductions of less
+// than 70 k values (fp32 63 x 1041 3.7 -> 5.0), in few rows of a warp 96 k (187 x 439 3.6 -> 5.4), of few long rows with many
+// tensors (20 x 15001 flex16 6.3 -> 7.1), and of fp32 rows to a block where little else is done (1010 x 4001 6.9 -> 7.8, 766 x
+// 11787 14.1 -> 17.9; rows that would be cut over blocks are: 293 x 2767 5.0 -> 3.4).  One
 // B200, us a launch, one value to a thread -> vectors: flex16 333 x 1001 13.0 -> 6.5, 8192 x 16383
 // 995 -> 392, 7013 x 73 35.4 -> 17.0, 8192 x 3001 209 -> 114, fp32 1500 x 16001 206 -> 108, 4415 x 121 21.6 -> 7.5.
-bool ragged_ok(const b2_ew_program& p) {
+bool ragged_ok(const b2_ew_program& p, int V) {
     const b2_ew_tensor* full = nullptr;
     auto ok = [&](const b2_ew_tensor& t) {
         if (t.sc == 0) return true;
@@ -999,7 +1024,14 @@ bool ragged_ok(const b2_ew_program& p) {
     if (p.reduce_mode == B2_REDUCE_B) return false;
     for (int i = 0; i < p.n_in; ++i) if (!ok(p.in[i])) return false;
     for (int k = 0; k < p.n_out; ++k) if (p.out[k].t.sc != 1 || !ok(p.out[k].t)) return false;
-    return full && p.C >= 64 && (long long)p.A * p.B * p.C >= 64 * 1024;
+    const long long rows = (long long)p.A * p.B;
+    if (!full || p.C < 64 || rows * p.C < 64 * 1024) return false;
+    if (p.reduce_mode != B2_REDUCE_C) return true;
+    const long long chunks = (p.C + V) / V;
+    const bool warp = warp_to_row(p, rows, chunks, V, true);
+    if (V == 4 && rows >= 2 * kSMs && full_tensors(p) <= 2 && !warp) return false;
+    if (full_tensors(p) > 3 && rows < 32 && p.C >= 4096) return false;
+    return rows * p.C >= (!warp ? 70 : rows < 400 ? 96 : 64) * 1024;
 }
 
 Plan make_plan(const b2_ew_program& p, bool want_vec) {
@@ -1012,7 +1044,7 @@ Plan make_plan(const b2_ew_program& p, bool want_vec) {
     if (want_vec) {
         if (any16 && vector_ok(p, 8)) { pl.V = 8; pl.vec = true; }
         else if (vector_ok(p, 4)) { pl.V = 4; pl.vec = true; }
-        else if (ragged_ok(p)) { pl.V = any16 ? 8 : 4; pl.vec = pl.ragged = true; }
+        else if (ragged_ok(p, any16 ? 8 : 4)) { pl.V = any16 ? 8 : 4; pl.vec = pl.ragged = true; }
     }
     const long long rows = p.A * p.B;
     const long long chunks = (p.C + (pl.ragged ? pl.V : 0)) / pl.V;
@@ -1030,11 +1062,7 @@ Plan make_plan(const b2_ew_program& p, bool want_vec) {
     } else if (p.reduce_mode == B2_REDUCE_C) {
         bool has_arg = false;
         for (int k = p.n_out; k < p.n_out + p.n_red; ++k) has_arg |= is_arg(p.out[k].redop);
-        // A warp to a row where that gives the machine warps enough: no barrier between a row and the next, and short
-        // rows do not leave most of a block idle (one B200, us a launch, a block to a row -> a warp: flex16 6709 x 930
-        // 59.0 -> 35.4, 1000 x 800 7.9 -> 6.8, 2551 x 2254 39.2 -> 33.9, 8192 x 3001 114 -> 107; fp32 4222 x 336 13.5 ->
-        // 6.8).
-        if (chunks <= 64 || (rows >= 1000 && chunks <= 512)) {
+        if (warp_to_row(p, rows, chunks, pl.V, pl.ragged)) {
             pl.group = 32;
             long long gy = (rows + 7) / 8;
             if (gy > 65535) gy = 65535;
@@ -1043,9 +1071,12 @@ Plan make_plan(const b2_ew_program& p, bool want_vec) {
             pl.group = kThreads;
             long long gy = rows > 65535 ? 65535 : rows;
             pl.nsplit = 1;
-            if (!has_arg && rows < 2 * kSMs && chunks >= 8LL * kThreads) {
+            // (vectors of few ragged rows where much is done: shorter parts, as many as one value to a thread had; elsewhere the
+            // second launch costs more than it gives: fp32 60 x 6114 7.8 -> 6.6 us, but flex16 108 x 6669 7.2 -> 9.2)
+            const bool shorter = pl.ragged && rows <= 64 && full_tensors(p) > 3;
+            if (!has_arg && rows < 2 * kSMs && chunks >= (shorter ? 4LL : 8LL) * kThreads) {
                 long long want = (4LL * kSMs + rows - 1) / rows;
-                long long maxs = chunks / (4LL * kThreads);
+                long long maxs = chunks / ((shorter ? 1LL : 4LL) * kThreads);
                 long long ns = want < maxs ? want : maxs;
                 if (ns > 1024) ns = 1024;
                 if (ns > 1) pl.nsplit = (int)ns;
