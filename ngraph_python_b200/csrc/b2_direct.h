@@ -41,7 +41,8 @@ struct b2_direct_args {
     void* C;
     long long ldc;
     int colmajor;                    // C[col * ldc + row] instead of C[row * ldc + col]
-    int streams;                     // matrix products: for the kernel of b2_stream.cuh
+    int streams;                     // matrix products: for the kernel of b2_stream.cuh, in the shape that its cost is of
+    struct { int bn, splits, kb_per_split, waves; } stream;
     const b2_flex_scale* table;
     int slotA, slotB, slotC;
     int* stats;
@@ -85,8 +86,7 @@ __attribute__((visibility("hidden"))) int b2_direct_launch(const b2_direct_args&
 // Matrix products of operands as they lie (b2_stream.cuh): likewise; whether all lines of both start on sixteen bytes
 // if the operands do.
 __attribute__((visibility("hidden"))) bool b2_product_even(const b2_direct_args& a);
-__attribute__((visibility("hidden"))) long long b2_stream_cost(const b2_direct_args& a);
-__attribute__((visibility("hidden"))) void b2_stream_plan(const b2_direct_args& a, b2_gemm_plan_info* plan);
+__attribute__((visibility("hidden"))) long long b2_stream_cost(b2_direct_args& a);            // (sets a.stream)
 __attribute__((visibility("hidden"))) int b2_stream_launch(const b2_direct_args& a, cudaStream_t st);
 
 // Gathered products whose filters are laid out beforehand (b2_gather.cu): whether it takes one rather than the kernel

@@ -88,13 +88,12 @@ inline bool gemm_goes_direct(int mode, const void* A, long long a_rs, long long 
             const long long ct = b2_stream_cost(t);
             stream = cheaper(b2_stream_cost(d), ct < 0 ? ct : ct + 1000);
             out->streams = 1;
-            if (along_k && even && K > 128 && stream >= 0 && (M <= 192 || N <= 192)) {
-                const b2_direct_args streamed = *out;
-                b2_gemm_plan_info plan;
-                b2_stream_plan(streamed, &plan);
-                const long long direct = cheaper(b2_direct_cost(d), b2_direct_cost(t));
-                const int per = ((K + 127) / 128 + plan.slices - 1) / plan.slices;
-                if (direct < 0 || per < 14 || direct >= stream + stream * 2 / 9) *out = streamed;
+            if (along_k && even && K > 13 * 128 && stream >= 0 && (M <= 192 || N <= 192)) {
+                if (out->stream.kb_per_split >= 14) {
+                    const b2_direct_args streamed = *out;
+                    const long long direct = cheaper(b2_direct_cost(d), b2_direct_cost(t));
+                    if (direct < 0 || direct >= stream + stream * 2 / 9) *out = streamed;
+                }
             }
             // (many k-blocks in few slices: flex16 500 x 500 x 6000, the second operand along K, 19.7 us on planes, 21.6
             // in one launch)
@@ -190,8 +189,7 @@ extern "C" int b2_gemm_route(int32_t flex, int64_t a_rs, int64_t a_cs, int64_t b
     if (gemm_goes_direct(mode, nullptr, a_rs, a_cs, nullptr, b_ks, b_ns, M, N, K, &d)) {
         *launches = 1;
         if (d.streams) {
-            b2_stream_plan(d, plan);
-            plan->kernel = B2_GEMM_STREAM;
+            *plan = {B2_GEMM_STREAM, d.stream.bn, d.stream.splits, d.stream.waves};
         } else {
             b2_direct_plan(d, plan);
         }

@@ -8,15 +8,10 @@ bool b2_product_even(const b2_direct_args& a) {
     return str_even(nullptr, a.a_kind, a.a_rs, a.a_ks, size) && str_even(nullptr, a.b_kind, a.b_rs, a.b_ks, size);
 }
 
-static StreamShape shape_of(const b2_direct_args& a) {
-    return a.flex ? stream_shape<MODE_FLEX16>(a) : stream_shape<MODE_F32X3>(a);
-}
-
-long long b2_stream_cost(const b2_direct_args& a) { return shape_of(a).cost; }
-
-void b2_stream_plan(const b2_direct_args& a, b2_gemm_plan_info* plan) {
-    const StreamShape s = shape_of(a);
-    *plan = {B2_GEMM_DIRECT, s.bn, s.splits, s.waves};
+long long b2_stream_cost(b2_direct_args& a) {
+    const StreamShape s = a.flex ? stream_shape<MODE_FLEX16>(a) : stream_shape<MODE_F32X3>(a);
+    a.stream = {s.bn, s.splits, s.kb_per_split, s.waves};
+    return s.cost;
 }
 
 int b2_stream_launch(const b2_direct_args& a, cudaStream_t st) {

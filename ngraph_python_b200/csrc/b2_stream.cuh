@@ -609,6 +609,12 @@ StreamShape stream_shape(const b2_direct_args& a) {
     if (tm > 65535) return best;
     const int size = MODE == MODE_FLEX16 ? 2 : 4;
     const bool even = str_even(nullptr, a.a_kind, a.a_rs, a.a_ks, size) && str_even(nullptr, a.b_kind, a.b_rs, a.b_ks, size);
+    int per_of[9] = {};                                           // k-blocks of a slice, 0: not so many slices
+    for (int want = 1; want <= 8 && want <= num_kb; ++want) {
+        int per = (num_kb + want - 1) / want;
+        if (MODE != MODE_FLEX16 && want > 1) per = (per + most - 1) / most * most;
+        if ((num_kb + per - 1) / per == want && (MODE != MODE_FLEX16 || per <= most)) per_of[want] = per;
+    }
     for (int bn = 16; bn <= 128; bn *= 2) {
         if (bn > 16 && bn / 2 >= a.N) break;
         const long long tiles = tm * ((a.N + bn - 1) / bn);
@@ -616,12 +622,9 @@ StreamShape stream_shape(const b2_direct_args& a) {
         // 2680 38.1 -> 25.4 us), else one: slices of more are no faster than pairs on planes (1000 x 777 x 1500 31.4 and
         // 28.4).
         const int chains_most = MODE == MODE_FLEX16 || a.N > 32 ? 1 : (512 - str_slots(bn) * 64) / bn;
-        for (int want = 1; want <= 8 && want <= num_kb; ++want) {
-            int per = (num_kb + want - 1) / want;
-            if (MODE != MODE_FLEX16 && want > 1) per = (per + most - 1) / most * most;
-            const int splits = (num_kb + per - 1) / per;
-            const int chains = MODE == MODE_FLEX16 ? 1 : (per + most - 1) / most;
-            if (splits != want || (MODE == MODE_FLEX16 ? per > most : chains > chains_most)) continue;
+        for (int splits = 1; splits <= 8; ++splits) {
+            const int per = per_of[splits], chains = MODE == MODE_FLEX16 ? 1 : (per + most - 1) / most;
+            if (!per || chains > chains_most) continue;
             if (splits > 1 && chains * bn * 128 * (MODE == MODE_FLEX16 ? 8 : 4) > 200 * 1024) continue;
             // Measured on one B200 (cycles at 1.9 GHz, 1060 flex16 and 250 fp32 products, each in two shapes; the rule is
             // within 7 and 5 % of them, root mean square): lines off sixteen bytes cost their converters a shift, operands
@@ -694,8 +697,8 @@ int stream_launch_bn(StreamParams& p, bool even, cudaStream_t st) {
 
 template <int MODE>
 int stream_launch_mode(const b2_direct_args& a, cudaStream_t st) {
-    const StreamShape s = stream_shape<MODE>(a);
-    B2_REQUIRE(s.cost >= 0, "K is too long for this kernel");
+    const auto& s = a.stream;
+    B2_REQUIRE(s.bn > 0, "a product without a shape");
     StreamParams p;
     p.a = a;
     const int KB = MODE == MODE_FLEX16 ? 128 : 32, size = MODE == MODE_FLEX16 ? 2 : 4;
